@@ -116,8 +116,9 @@ int asca_gemm(asca_ctx* ctx, int mode, int64_t M, int64_t N, int64_t K, const vo
     p.accumulate = accumulate;
     p.group_dim = gemm::GROUP_NONE;
     p.epi = gemm::EPI_NONE;
+    p.mode = mode;
     const int bf = dtype == ASCA_BF16;
-    ASCA_CUDA(ctx, gemm::launch<float>(p, mode, bf, bf, 0, ctx->stream));
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, p, bf, bf));
     ctx->launches++;
     return ASCA_OK;
 }

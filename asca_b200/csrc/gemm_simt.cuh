@@ -1,18 +1,28 @@
-// f32-accurate SIMT GEMM (FFMA, f32 accumulate) with optional row gather / scatter maps and
+// f32-accurate SIMT products (FFMA, f32 accumulate) with optional row gather / scatter maps and
 // expert grouping. It is the exact-mode (1e-5) engine behind asca_matmul / asca_gemm and the
 // grouped expert products of the hash-MoE; operands may be f32 or bf16 and are widened to f32
 // on the way into shared memory.
 //
-// Tiling: 128 x 128 x 16 per CTA, 256 threads, 8 x 8 outputs per thread held in registers;
-// operands are staged in shared memory k-major ([k][m] and [k][n]) so the inner product reads
-// two float4 per operand per k. The next k-slab is prefetched into registers while the current
-// one is multiplied.
+// One launch takes up to four independent products of any operand form (a training step's products
+// are microseconds long: what is launched together is paid for once), in one of three tile shapes:
+//   128 x 128 x 16                256 threads x (8 x 8)    large products: FFMA issue bound
+//    64 x  64 x 32  4 k-groups of  64 threads x (8 x 8)    a few hundred rows and up
+//    32 x  32 x 64  8 k-groups of  32 threads x (4 x 8)    latency bound: few tiles, short k
+// and a k-split over the CTAs of a cluster (1, 2, 4 or 8): the partial tiles stay in shared memory
+// and are added across the cluster in rank order, so a weight gradient over thousands of rows with
+// a handful of output tiles fills the GPU without a scratch buffer or a second launch. Results do
+// not depend on scheduling. plan() picks tile shape and split from the launch's tiles and slabs.
+//
+// Operands go to shared memory with cp.async, STAGES slabs deep. What bounds the
+// inner loop is the 128 bytes a cycle that shared memory returns to an SM's registers, broadcast or
+// not: an 8 x 8 thread tile needs 64 bytes for 64 FFMAs (both limits met at once), a 4 x 4 tile twice
+// that. Hence the k-groups: a small CTA tile keeps the large thread tile, and its warps divide k.
 #pragma once
 #include "common.cuh"
 
-namespace gemm {
+#include <algorithm>
 
-constexpr int BM = 128, BN = 128, BK = 16, THREADS = 256, PAD = 4;
+namespace gemm {
 
 enum { EPI_NONE = 0, EPI_SILU = 1, EPI_SILU_BWD = 2 };
 enum { GROUP_NONE = 0, GROUP_M = 1, GROUP_K = 2 };
@@ -38,7 +48,7 @@ struct Params {
     const int32_t* offsets;
     int n_groups;
     int group_dim;
-    int64_t a_gstride, b_gstride, c_gstride, bias_gstride;
+    int64_t b_gstride, c_gstride, bias_gstride;
     // epilogue: EPI_SILU writes the pre-activation to C and silu to C2 (type TC2);
     // EPI_SILU_BWD multiplies by silu'(aux[row][col]) (aux rows follow the logical row).
     int epi;
@@ -46,33 +56,44 @@ struct Params {
     int64_t ldaux;
     void* C2;
     int64_t ldc2;
+    int mode;               // ASCA_NN / ASCA_TN / ASCA_NT
+    int64_t total_rows;     // grouped: token rows over all groups (bounds the grid and the k range)
+    // a second operand pair with its own k, added to the same result (ungrouped, no maps)
+    const void* A2;
+    const void* B2;
+    int64_t lda2, ldb2;
+    int K2;
+    // TN: the column sums of B (a bias gradient) beside the product; with A null, the sums alone (f32, K rows of B)
+    float* colsum;
+    int64_t colsum_gstride;
 };
 
-template <typename T>
-__device__ __forceinline__ void load4(const T* p, bool vec_ok, int valid, float out[4]);
+constexpr int MAX_PROBLEMS = 4;
+constexpr int THREADS = 256;
 
-template <>
-__device__ __forceinline__ void load4<float>(const float* p, bool vec_ok, int valid, float out[4]) {
-    if (vec_ok && valid == 4) {
-        float4 v = *reinterpret_cast<const float4*>(p);
-        out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) out[j] = j < valid ? p[j] : 0.0f;
-    }
-}
-template <>
-__device__ __forceinline__ void load4<__nv_bfloat16>(const __nv_bfloat16* p, bool vec_ok, int valid, float out[4]) {
-    if (vec_ok && valid == 4) {
-        uint2 raw = *reinterpret_cast<const uint2*>(p);
-        __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162*>(&raw.x);
-        __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&raw.y);
-        out[0] = __low2float(a); out[1] = __high2float(a); out[2] = __low2float(b); out[3] = __high2float(b);
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) out[j] = j < valid ? __bfloat162float(p[j]) : 0.0f;
-    }
-}
+struct Multi {
+    Params p[MAX_PROBLEMS];
+    int tile0[MAX_PROBLEMS + 1];   // first tile of each problem
+    int n, split;
+};
+
+template <int BM_, int BN_, int BK_, int TM_, int TN_, int KG_, int STAGES_>
+struct Cfg {
+    static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = TM_, TN = TN_, KG = KG_, STAGES = STAGES_;
+    static constexpr int THR_M = BM / TM, THR_N = BN / TN;
+    static_assert(THR_M * THR_N * KG == THREADS && TM % 4 == 0 && TN % 4 == 0 && BK % (4 * KG) == 0, "tile shape");
+    // row pitches: 16-byte aligned, 8 consecutive rows start in 8 different bank groups
+    static constexpr bool TRANSPOSE = KG == 1;   // operands along k are transposed on their way into shared memory
+    static constexpr int A_FLOATS = BM * (BK + 4) > BK * (BM + 8) ? BM * (BK + 4) : BK * (BM + 8);
+    static constexpr int B_FLOATS = BN * (BK + 4) > BK * (BN + 8) ? BN * (BK + 4) : BK * (BN + 8);
+    static constexpr int STAGE_FLOATS = A_FLOATS + B_FLOATS;
+    static constexpr int RED_FLOATS = KG * (BM * BN + BN);   // partial tiles + column sums, over the (finished) stages
+    static constexpr int SMEM_FLOATS = STAGES * STAGE_FLOATS > RED_FLOATS ? STAGES * STAGE_FLOATS : RED_FLOATS;
+    static constexpr size_t SMEM = (size_t)SMEM_FLOATS * 4;
+};
+using CfgL = Cfg<128, 128, 16, 8, 8, 1, 3>;
+using CfgM = Cfg<64, 64, 32, 8, 8, 4, 3>;
+using CfgS = Cfg<32, 32, 64, 4, 8, 8, 3>;
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float silu_grad_f(float p) {
@@ -80,50 +101,271 @@ __device__ __forceinline__ float silu_grad_f(float p) {
     return sg * (1.0f + p * (1.0f - sg));
 }
 
-// MODE: ASCA_NN / ASCA_TN / ASCA_NT as in the public header.
-template <int MODE, typename TA, typename TB, typename TC2>
-__global__ void __launch_bounds__(THREADS) gemm_kernel(Params p) {
-    __shared__ float As[BK][BM + PAD];
-    __shared__ float Bs[BK][BN + PAD];
-    __shared__ int sh_group[4];
+// two independent FFMAs in one instruction (the rounding of two scalar ones, half the issue slots)
+__device__ __forceinline__ void fma2(float2& d, const float2& a, const float2& b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+}
+
+// Four elements of a row into shared memory, the first `valid` of them from p and zeros behind.
+__device__ __forceinline__ void stage4(float* dst, const float* p, bool vec_ok, int valid) {
+    const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst);
+    if (vec_ok) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(p), "r"(valid * 4) : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s + 4 * j), "l"(j < valid ? p + j : p), "r"(j < valid ? 4 : 0)
+                         : "memory");
+    }
+}
+__device__ __forceinline__ void stage4(float* dst, const __nv_bfloat16* p, bool vec_ok, int valid) {
+    float4 v = make_float4(0, 0, 0, 0);
+    if (vec_ok && valid == 4) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(p);
+        const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+        v = make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+    } else {
+        if (valid > 0) v.x = __bfloat162float(p[0]);
+        if (valid > 1) v.y = __bfloat162float(p[1]);
+        if (valid > 2) v.z = __bfloat162float(p[2]);
+        if (valid > 3) v.w = __bfloat162float(p[3]);
+    }
+    *reinterpret_cast<float4*>(dst) = v;
+}
+
+__device__ __forceinline__ void stage1(float* dst, const float* p, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(p), "r"(valid ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void stage1(float* dst, const __nv_bfloat16* p, bool valid) { *dst = valid ? __bfloat162float(*p) : 0.0f; }
+
+// One operand's slabs on their way into shared memory, laid out as in memory: [row][k] where k is contiguous there (ALONG_K;
+// row = output row or column of the tile), [k][row] otherwise. A thread copies CH runs of four elements per slab.
+template <typename T, int ROWS, int BK, bool ALONG_K>
+struct Stager {
+    static constexpr int LD = (ALONG_K ? BK : ROWS) + 4, CH = ROWS * BK / 4 / THREADS;
+    static constexpr int RUNS = (ALONG_K ? BK : ROWS) / 4, STEP = THREADS / RUNS;   // runs per memory row; rows covered by one pass
+    static_assert(CH >= 1 && THREADS % RUNS == 0, "tile shape");
+    const T* ptr[ALONG_K ? CH : 1];   // ALONG_K: this thread's runs at k = 0 of the slab sequence; else its run of memory row 0
+    const int32_t* idx;               // !ALONG_K: memory row of each k, from the group's first row
+    int64_t ld;
+    int K, next_row[ALONG_K ? 1 : CH];
+    int valid_rows;                   // !ALONG_K: elements of the run that exist; ALONG_K: bit c: row of run c exists
+    bool vec;
+
+    // row0: first tile row; n: rows that exist; idx_base: logical position of the first row (ALONG_K) or of k = 0
+    __device__ __forceinline__ void init(const T* b, int64_t ld_, int row0, int n, int K_, const int32_t* idx_, int64_t idx_base) {
+        const int tid = threadIdx.x;
+        K = K_;
+        vec = (ld_ & 3) == 0 && (reinterpret_cast<uintptr_t>(b) & (sizeof(T) * 4 - 1)) == 0;
+        if (ALONG_K) {
+            valid_rows = 0;
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                const int r = row0 + tid / RUNS + c * STEP;
+                if (r < n) valid_rows |= 1 << c;
+                ptr[c] = b + (r < n ? (idx_ ? (int64_t)idx_[idx_base + r] : idx_base + r) : 0) * ld_;
+            }
+        } else {
+            const int r = row0 + (tid % RUNS) * 4;
+            valid_rows = max(0, min(4, n - r));
+            ptr[0] = b + (valid_rows ? r : 0) + (idx_ ? 0 : idx_base * ld_);
+            idx = idx_ ? idx_ + idx_base : nullptr;
+            ld = ld_;
+        }
+    }
+    // !ALONG_K with a row map: the memory rows of the slab starting at k0 (asked for a slab ahead of the copy)
+    __device__ __forceinline__ void look_up(int k0) {
+        if (!ALONG_K && idx) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                const int k = k0 + (int)threadIdx.x / RUNS + c * STEP;
+                next_row[ALONG_K ? 0 : c] = k < K ? idx[k] : 0;
+            }
+        }
+    }
+    __device__ __forceinline__ void put(float* dst, int k0) {
+        const int tid = threadIdx.x, first = tid / RUNS, run = tid % RUNS;
+        float* d = dst + first * LD + run * 4;
+        if (ALONG_K) {
+            const int k = k0 + run * 4, left = K - k, valid = left < 0 ? 0 : (left > 4 ? 4 : left), at = left > 0 ? k : 0;
+#pragma unroll
+            for (int c = 0; c < CH; ++c) stage4(d + c * STEP * LD, ptr[c] + at, vec, (valid_rows >> c & 1) ? valid : 0);
+        } else {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                const int k = k0 + first + c * STEP;
+                const bool ok = k < K;
+                stage4(d + c * STEP * LD, ptr[0] + (int64_t)(ok ? (idx ? next_row[ALONG_K ? 0 : c] : k) : 0) * ld, vec, ok ? valid_rows : 0);
+            }
+        }
+    }
+};
+
+template <typename TC2>
+__device__ __forceinline__ void emit(const Params& p, float* crow, const float* bias, int64_t lr, int n, float v) {
+    if (bias) v += bias[n];
+    if (p.epi == EPI_SILU_BWD) v *= silu_grad_f(p.aux[lr * p.ldaux + n]);
+    if (p.accumulate) v += crow[n];
+    crow[n] = v;
+    if (p.epi == EPI_SILU) reinterpret_cast<TC2*>(p.C2)[lr * p.ldc2 + n] = from_f32<TC2>(silu_f(v));
+}
+
+// four columns n .. n + 3 of one row, 16-byte accesses (row pitches and pointers allow them: vec4_ok)
+template <typename TC2>
+__device__ __forceinline__ bool vec4_ok(const Params& p, const float* C, const float* bias) {
+    int64_t pitch = p.ldc;
+    uintptr_t at = reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias);
+    if (p.epi == EPI_SILU_BWD) pitch |= p.ldaux, at |= reinterpret_cast<uintptr_t>(p.aux);
+    if (p.epi == EPI_SILU) pitch |= p.ldc2, at |= reinterpret_cast<uintptr_t>(p.C2);
+    return ((pitch & 3) | (at & 15)) == 0;
+}
+template <typename TC2>
+__device__ __forceinline__ void emit4(const Params& p, float* crow, const float* bias, int64_t lr, int n, float4 v) {
+    if (bias) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + n);
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+    }
+    if (p.epi == EPI_SILU_BWD) {
+        const float4 x = *reinterpret_cast<const float4*>(p.aux + lr * p.ldaux + n);
+        v.x *= silu_grad_f(x.x); v.y *= silu_grad_f(x.y); v.z *= silu_grad_f(x.z); v.w *= silu_grad_f(x.w);
+    }
+    if (p.accumulate) {
+        const float4 c = *reinterpret_cast<const float4*>(crow + n);
+        v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
+    }
+    *reinterpret_cast<float4*>(crow + n) = v;
+    if (p.epi == EPI_SILU) {
+        TC2* c2 = reinterpret_cast<TC2*>(p.C2) + lr * p.ldc2 + n;
+        const float s[4] = {silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w)};
+        if (sizeof(TC2) == 4) {
+            *reinterpret_cast<float4*>(c2) = make_float4(s[0], s[1], s[2], s[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c2[j] = from_f32<TC2>(s[j]);
+        }
+    }
+}
+
+// Column sums alone: 8 columns (one sector) of all rows per CTA, 32 rows a pass, 8 passes in flight, a fixed tree.
+__device__ __forceinline__ void colsum_tile(const Params& p, int tile, float* smem) {
+    const float* B = reinterpret_cast<const float*>(p.B);
+    const int tid = threadIdx.x, c = tile * 8 + (tid & 7), w = tid >> 3;
+    float acc = 0.0f;
+    if (c < p.N) {
+        int r = w;
+        for (; r + 224 < p.K; r += 256) {
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = B[(int64_t)(r + 32 * i) * p.ldb + c];
+            acc += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+        }
+        for (; r < p.K; r += 32) acc += B[(int64_t)r * p.ldb + c];
+    }
+    smem[w * 8 + (tid & 7)] = acc;
+    __syncthreads();
+    if (tid < 8 && c < p.N) {
+        float t = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t += smem[i * 8 + tid];
+        p.colsum[c] = p.accumulate ? p.colsum[c] + t : t;
+    }
+}
+
+// Values of T rows at k of a staged operand.
+template <int T, bool ALONG_K, class Of>
+__device__ __forceinline__ void read_rows(const float* s, int ld, int k, const Of& of, float (&v)[T]) {
+    if (ALONG_K) {
+#pragma unroll
+        for (int i = 0; i < T; ++i) v[i] = s[of(i) * ld + k];
+    } else {
+#pragma unroll
+        for (int i = 0; i < T; i += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(s + k * ld + of(i));
+            v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+        }
+    }
+}
+
+// The same for an operand that is contiguous along k, transposed to [k][row] by the copy: a warp takes 8 rows x 4 k at a time
+// (pitch ROWS + 8: 32 different banks). The largest tile shape reads its operands along the rows in every form, since
+// reading 16 values one by one costs it more issue slots than the 4-byte copies do.
+template <typename T, int ROWS, int BK>
+struct TransposingStager {
+    static constexpr int CH = ROWS * BK / THREADS, KB = BK / 4, WR = 8 / KB * 8;
+    const T* base;
+    int64_t ld;
+    int K, kl, row[CH];   // memory rows of this thread's elements, -1: none
+    __device__ __forceinline__ void init(const T* b, int64_t ld_, int row0, int n, int K_, const int32_t* idx, int64_t idx_base) {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        base = b; ld = ld_; K = K_;
+        kl = (w % KB) * 4 + (lane >> 3);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const int r = row0 + w / KB * 8 + (lane & 7) + c * WR;
+            row[c] = r < n ? (int)(idx ? (int64_t)idx[idx_base + r] : idx_base + r) : -1;
+        }
+    }
+    __device__ __forceinline__ void look_up(int) {}
+    __device__ __forceinline__ void put(float* dst, int k0) {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        float* d = dst + kl * (ROWS + 8) + w / KB * 8 + (lane & 7);
+        const T* p = base + (k0 + kl < K ? k0 + kl : 0);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) stage1(d + c * WR, p + (int64_t)max(row[c], 0) * ld, row[c] >= 0 && k0 + kl < K);
+    }
+};
+template <class C, typename T, int ROWS, bool ALONG_K, bool TR = C::TRANSPOSE && ALONG_K>
+struct StagerOf {
+    using type = Stager<T, ROWS, C::BK, ALONG_K>;
+};
+template <class C, typename T, int ROWS, bool ALONG_K>
+struct StagerOf<C, T, ROWS, ALONG_K, true> {
+    using type = TransposingStager<T, ROWS, C::BK>;
+};
+
+template <class C, int MODE, typename TA, typename TB, typename TC2>
+__device__ __forceinline__ void tile_product(const Params& p, int tile, int rank, int split, float* smem, int* sh_group) {
+    constexpr int BM = C::BM, BN = C::BN, BK = C::BK, TM = C::TM, TN = C::TN, KG = C::KG, STAGES = C::STAGES;
+    constexpr bool A_KC = !C::TRANSPOSE && MODE != ASCA_TN, B_KC = !C::TRANSPOSE && MODE == ASCA_NT;   // along k in shared memory
+    constexpr int LDA = A_KC ? BK + 4 : BM + (C::TRANSPOSE && MODE != ASCA_TN ? 8 : 4),
+                  LDB = B_KC ? BK + 4 : BN + (C::TRANSPOSE && MODE == ASCA_NT ? 8 : 4);
 
     int M = p.M, N = p.N, K = p.K;
-    int tile_m, tile_n;
-    int64_t row_base = 0;   // logical row offset of this group (GROUP_M) or k offset (GROUP_K)
     const TA* A = reinterpret_cast<const TA*>(p.A);
     const TB* B = reinterpret_cast<const TB*>(p.B);
-    float* C = p.C;
+    float* Cp = p.C;
     const float* bias = p.bias;
-    const int tiles_n = (N + BN - 1) / BN;
-
-    if (p.group_dim == GROUP_NONE) {
-        tile_n = blockIdx.x % tiles_n;
-        tile_m = blockIdx.x / tiles_n;
-    } else {
-        // locate (group, tile) for this CTA: warp 0 scans the per-group tile counts
-        if (threadIdx.x < 32) {
-            const int lane = threadIdx.x;
+    float* colsum = p.colsum;
+    const int tiles_n = (N + BN - 1) / BN, tid = threadIdx.x;
+    int64_t row_base = 0;   // logical row offset of this group (GROUP_M) or its k offset (GROUP_K)
+    int g = 0, t = tile;
+    if (p.group_dim != GROUP_NONE) {
+        // locate (group, tile): warp 0 scans the per-group tile counts
+        if (tid < 32) {
+            const int lane = tid;
             int found_g = -1, found_t = 0, base = 0;
             for (int g0 = 0; g0 < p.n_groups && found_g < 0; g0 += 32) {
-                int g = g0 + lane;
+                const int gi = g0 + lane;
                 int cnt = 0;
-                if (g < p.n_groups) {
-                    int n_g = p.offsets[g + 1] - p.offsets[g];
+                if (gi < p.n_groups) {
+                    const int n_g = p.offsets[gi + 1] - p.offsets[gi];
                     cnt = p.group_dim == GROUP_M ? ((n_g + BM - 1) / BM) * tiles_n : ((M + BM - 1) / BM) * tiles_n;
                 }
                 int inc = cnt;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    int n = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += n;
+                    const int x = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += x;
                 }
-                int start = base + inc - cnt;
-                bool mine = (int)blockIdx.x >= start && (int)blockIdx.x < start + cnt;
-                unsigned m = __ballot_sync(0xffffffffu, mine);
+                const int start = base + inc - cnt;
+                const unsigned m = __ballot_sync(0xffffffffu, tile >= start && tile < start + cnt);
                 if (m) {
-                    int src = __ffs(m) - 1;
-                    found_g = __shfl_sync(0xffffffffu, g, src);
-                    found_t = (int)blockIdx.x - __shfl_sync(0xffffffffu, start, src);
+                    const int src = __ffs(m) - 1;
+                    found_g = __shfl_sync(0xffffffffu, gi, src);
+                    found_t = tile - __shfl_sync(0xffffffffu, start, src);
                 }
                 base += __shfl_sync(0xffffffffu, inc, 31);
             }
@@ -133,11 +375,9 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(Params p) {
             }
         }
         __syncthreads();
-        const int g = sh_group[0];
-        if (g < 0) return;  // surplus CTA of the upper-bound grid
-        const int t = sh_group[1];
-        tile_n = t % tiles_n;
-        tile_m = t / tiles_n;
+        g = sh_group[0];
+        if (g < 0) return;   // surplus tile of the upper-bound grid (every CTA of its cluster returns here)
+        t = sh_group[1];
         const int lo = p.offsets[g], n_g = p.offsets[g + 1] - lo;
         row_base = lo;
         if (p.group_dim == GROUP_M) {
@@ -145,194 +385,330 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(Params p) {
             B += (int64_t)g * p.b_gstride;
         } else {
             K = n_g;
-            C += (int64_t)g * p.c_gstride;
+            Cp += (int64_t)g * p.c_gstride;
+            if (colsum) colsum += (int64_t)g * p.colsum_gstride;
         }
         if (bias) bias += (int64_t)g * p.bias_gstride;
-        (void)A;
     }
-
+    const int tile_n = t % tiles_n, tile_m = t / tiles_n;
     const int m0 = tile_m * BM, n0 = tile_n * BN;
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
+    const int64_t m_base = p.group_dim == GROUP_M ? row_base : 0, k_base = p.group_dim == GROUP_K ? row_base : 0;
+    const bool want_cs = MODE == ASCA_TN && colsum && tile_m == 0;
 
-    // ---- global -> register staging descriptors
-    // "k-contiguous" operand (A in NN/NT, B in NT): thread loads rows r = tid/4 + {0,64},
-    // 4 consecutive k at kq = (tid%4)*4. "row-contiguous" operand (A in TN, B in NN/TN):
-    // thread loads k rows kr = tid/32 + {0,8}, 4 consecutive columns at (tid%32)*4.
-    constexpr bool A_KCONT = (MODE != ASCA_TN);
-    constexpr bool B_KCONT = (MODE == ASCA_NT);
-    const bool a_vec = ((p.lda & 3) == 0) && ((reinterpret_cast<uintptr_t>(A) & (sizeof(TA) * 4 - 1)) == 0);
-    const bool b_vec = ((p.ldb & 3) == 0) && ((reinterpret_cast<uintptr_t>(B) & (sizeof(TB) * 4 - 1)) == 0);
-
-    float ra[2][4], rb[2][4];
-    int64_t a_row_off[2];  // element offset of the memory row this thread reads (k-contiguous A)
-    bool a_row_ok[2];
-    int64_t b_row_off[2];
-    bool b_row_ok[2];
-    if (A_KCONT) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            int m = m0 + (tid >> 2) + h * 64;
-            a_row_ok[h] = m < M;
-            int64_t lr = row_base * (p.group_dim == GROUP_M) + m;
-            int64_t mr = a_row_ok[h] ? (p.a_idx ? (int64_t)p.a_idx[lr] : lr) : 0;
-            a_row_off[h] = mr * p.lda;
-        }
-    }
-    if (B_KCONT) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            int n = n0 + (tid >> 2) + h * 64;
-            b_row_ok[h] = n < N;
-            b_row_off[h] = (int64_t)(b_row_ok[h] ? n : 0) * p.ldb;
-        }
-    }
-
-    auto fetch = [&](int k0) {
-        if (A_KCONT) {
-            const int kq = k0 + (tid & 3) * 4;
-            const int valid = K - kq < 0 ? 0 : (K - kq > 4 ? 4 : K - kq);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                load4<TA>(A + a_row_off[h] + kq, a_vec, a_row_ok[h] ? valid : 0, ra[h]);
-        } else {  // TN: A memory is (K x M); rows are k (token rows under GROUP_K)
-            const int mc = m0 + (tid & 31) * 4;
-            const int valid = M - mc < 0 ? 0 : (M - mc > 4 ? 4 : M - mc);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                int k = k0 + (tid >> 5) + h * 8;
-                bool ok = k < K;
-                int64_t lr = row_base * (p.group_dim == GROUP_K) + k;
-                int64_t mr = ok ? (p.a_idx ? (int64_t)p.a_idx[lr] : lr) : 0;
-                load4<TA>(A + mr * p.lda + mc, a_vec, ok ? valid : 0, ra[h]);
-            }
-        }
-        if (B_KCONT) {
-            const int kq = k0 + (tid & 3) * 4;
-            const int valid = K - kq < 0 ? 0 : (K - kq > 4 ? 4 : K - kq);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                load4<TB>(B + b_row_off[h] + kq, b_vec, b_row_ok[h] ? valid : 0, rb[h]);
-        } else {  // B memory is (K x N)
-            const int nc = n0 + (tid & 31) * 4;
-            const int valid = N - nc < 0 ? 0 : (N - nc > 4 ? 4 : N - nc);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                int k = k0 + (tid >> 5) + h * 8;
-                bool ok = k < K;
-                int64_t lr = (MODE == ASCA_TN ? row_base * (p.group_dim == GROUP_K) : 0) + k;
-                int64_t mr = ok ? ((MODE == ASCA_TN && p.b_idx) ? (int64_t)p.b_idx[lr] : lr) : 0;
-                load4<TB>(B + mr * p.ldb + nc, b_vec, ok ? valid : 0, rb[h]);
-            }
-        }
+    typename StagerOf<C, TA, BM, MODE != ASCA_TN>::type sa;
+    typename StagerOf<C, TB, BN, MODE == ASCA_NT>::type sb;
+    sa.init(A, p.lda, m0, M, K, p.a_idx, MODE != ASCA_TN ? m_base : k_base);
+    sb.init(B, p.ldb, n0, N, K, MODE == ASCA_TN ? p.b_idx : nullptr, MODE == ASCA_TN ? k_base : 0);
+    const int slabs1 = (K + BK - 1) / BK, slabs = slabs1 + (p.K2 + BK - 1) / BK;
+    const int s_lo = (int)((int64_t)slabs * rank / split), s_hi = (int)((int64_t)slabs * (rank + 1) / split);
+    int staged = s_lo;   // next slab to stage
+    auto second = [&]() {   // from here on the slabs come from the second operand pair
+        sa.init(reinterpret_cast<const TA*>(p.A2), p.lda2, m0, M, p.K2, nullptr, 0);
+        sb.init(reinterpret_cast<const TB*>(p.B2), p.ldb2, n0, N, p.K2, nullptr, 0);
     };
-    auto stash = [&]() {
-        if (A_KCONT) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) As[(tid & 3) * 4 + j][(tid >> 2) + h * 64] = ra[h][j];
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float4*>(&As[(tid >> 5) + h * 8][(tid & 31) * 4]) =
-                    make_float4(ra[h][0], ra[h][1], ra[h][2], ra[h][3]);
+    if (p.K2 > 0 && s_lo > slabs1) second();
+    sa.look_up(s_lo * BK);
+    sb.look_up(s_lo * BK);
+    auto stage_next = [&]() {
+        if (staged < s_hi) {
+            if (p.K2 > 0 && staged == slabs1) second();
+            const int k0 = (staged >= slabs1 ? staged - slabs1 : staged) * BK;
+            float* As = smem + ((staged - s_lo) % STAGES) * C::STAGE_FLOATS;
+            sa.put(As, k0);
+            sb.put(As + C::A_FLOATS, k0);
+            ++staged;
+            sa.look_up(k0 + BK);
+            sb.look_up(k0 + BK);
         }
-        if (B_KCONT) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) Bs[(tid & 3) * 4 + j][(tid >> 2) + h * 64] = rb[h][j];
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float4*>(&Bs[(tid >> 5) + h * 8][(tid & 31) * 4]) =
-                    make_float4(rb[h][0], rb[h][1], rb[h][2], rb[h][3]);
-        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    const int kg = tid / (C::THR_M * C::THR_N), tt = tid % (C::THR_M * C::THR_N);
+    const int tn = tt % C::THR_N, tm = tt / C::THR_N;
+    // this thread's output rows and columns: interleaved where the operand is read along k (the lanes of a phase then read
+    // rows a pitch apart: no bank conflict), groups of four where it is read along the row
+    auto m_of = [&](int i) { return A_KC ? tm + C::THR_M * i : (i >> 2) * (BM * 4 / TM) + tm * 4 + (i & 3); };
+    auto n_of = [&](int j) { return B_KC ? tn + C::THR_N * j : (j >> 2) * (BN * 4 / TN) + tn * 4 + (j & 3); };
 
-    if (K > 0) {
-        fetch(0);
-        for (int k0 = 0; k0 < K; k0 += BK) {
-            __syncthreads();
-            stash();
-            __syncthreads();
-            if (k0 + BK < K) fetch(k0 + BK);
+    float2 acc[TM][TN / 2];   // columns (j, j + 1)
 #pragma unroll
-            for (int kk = 0; kk < BK; ++kk) {
-                float a[8], b[8];
-                float4 t;
-                t = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-                a[0] = t.x; a[1] = t.y; a[2] = t.z; a[3] = t.w;
-                t = *reinterpret_cast<const float4*>(&As[kk][64 + ty * 4]);
-                a[4] = t.x; a[5] = t.y; a[6] = t.z; a[7] = t.w;
-                t = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-                b[0] = t.x; b[1] = t.y; b[2] = t.z; b[3] = t.w;
-                t = *reinterpret_cast<const float4*>(&Bs[kk][64 + tx * 4]);
-                b[4] = t.x; b[5] = t.y; b[6] = t.z; b[7] = t.w;
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    float cs[TN];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    for (int j = 0; j < TN; ++j) cs[j] = 0.0f;
+
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) stage_next();
+    for (int slab = s_lo; slab < s_hi; ++slab) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();   // the slab has landed for every thread, and the stage filled next is no longer being read
+        stage_next();
+        const float* As = smem + ((slab - s_lo) % STAGES) * C::STAGE_FLOATS;
+        const float* Bs = As + C::A_FLOATS;
+        // the operands of the next k are read while this one is multiplied; the k-groups take turns four k wide
+        float a[2][TM], b[2][TN];
+        auto read = [&](int kk) {
+            const int k = ((kk >> 2) * KG + kg) * 4 + (kk & 3);
+            read_rows<TM, A_KC>(As, LDA, k, m_of, a[kk & 1]);
+            read_rows<TN, B_KC>(Bs, LDB, k, n_of, b[kk & 1]);
+        };
+        read(0);
+#pragma unroll
+        for (int kk = 0; kk < BK / KG; ++kk) {
+            if (kk + 1 < BK / KG) read(kk + 1);
+            if (MODE == ASCA_TN && want_cs) {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) cs[j] += b[kk & 1][j];
             }
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) {
+                    const float2 bb = make_float2(b[kk & 1][2 * j], b[kk & 1][2 * j + 1]);
+                    if (B_KC) {   // (the two columns come from separate loads: pairing them would cost moves)
+                        acc[i][j].x = fmaf(a[kk & 1][i], bb.x, acc[i][j].x);
+                        acc[i][j].y = fmaf(a[kk & 1][i], bb.y, acc[i][j].y);
+                    } else {
+                        fma2(acc[i][j], make_float2(a[kk & 1][i], a[kk & 1][i]), bb);
+                    }
+                }
         }
     }
+    auto value = [&](int i, int j) -> float { return (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x; };
 
-    // ---- epilogue
-    TC2* C2 = reinterpret_cast<TC2*>(p.C2);
+    const bool vec = vec4_ok<TC2>(p, Cp, bias);
+    if (KG == 1 && split == 1 && !want_cs) {   // straight from the registers
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-        if (m >= M) continue;
-        const int64_t lr = row_base * (p.group_dim == GROUP_M) + m;
-        const int64_t cr = p.c_idx ? (int64_t)p.c_idx[lr] : lr;
-        float* crow = C + cr * p.ldc;
+        for (int i = 0; i < TM; ++i) {
+            const int m = m0 + m_of(i);
+            if (m >= M) continue;
+            const int64_t lr = m_base + m;
+            float* crow = Cp + (p.c_idx ? (int64_t)p.c_idx[lr] : lr) * p.ldc;
+            if (!B_KC && vec) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-            if (n >= N) continue;
-            float v = acc[i][j];
-            if (bias) v += bias[n];
-            if (p.epi == EPI_SILU_BWD) v *= silu_grad_f(p.aux[lr * p.ldaux + n]);
-            if (p.accumulate) v += crow[n];
-            crow[n] = v;
-            if (p.epi == EPI_SILU) C2[lr * p.ldc2 + n] = from_f32<TC2>(silu_f(v));
+                for (int j = 0; j < TN; j += 4)
+                    if (n0 + n_of(j) + 3 < N)
+                        emit4<TC2>(p, crow, bias, lr, n0 + n_of(j), make_float4(value(i, j), value(i, j + 1), value(i, j + 2), value(i, j + 3)));
+                    else
+                        for (int jj = 0; jj < 3; ++jj)
+                            if (n0 + n_of(j) + jj < N) emit<TC2>(p, crow, bias, lr, n0 + n_of(j) + jj, jj == 0 ? value(i, j) : jj == 1 ? value(i, j + 1) : value(i, j + 2));
+                continue;
+            }
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int n = n0 + n_of(j);
+                if (n < N) emit<TC2>(p, crow, bias, lr, n, value(i, j));
+            }
         }
+        return;
+    }
+    // partial tiles to shared memory, added over the cluster's CTAs and their k-groups in order
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // the stages are free
+    float* red = smem;
+    float* red_cs = smem + KG * BM * BN;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        float* row = red + kg * BM * BN + m_of(i) * BN;
+        if (B_KC) {
+#pragma unroll
+            for (int j = 0; j < TN; ++j) row[n_of(j)] = value(i, j);
+        } else {
+#pragma unroll
+            for (int j = 0; j < TN; j += 4)
+                *reinterpret_cast<float4*>(row + n_of(j)) = make_float4(value(i, j), value(i, j + 1), value(i, j + 2), value(i, j + 3));
+        }
+    }
+    if (want_cs && tm == 0) {
+#pragma unroll
+        for (int j = 0; j < TN; ++j) red_cs[kg * BN + n_of(j)] = cs[j];
+    }
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(smem);
+    if (split > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    else __syncthreads();
+    // v + the KG values at off, off + stride, ... (floats) of every CTA, in order
+    auto add_all = [&](float4 v, int off, int stride) -> float4 {
+        for (int r = 0; r < split; ++r) {
+            float4 x[KG];
+            uint32_t at;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(r));
+#pragma unroll
+            for (int q = 0; q < KG; ++q)
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(x[q].x), "=f"(x[q].y), "=f"(x[q].z), "=f"(x[q].w) : "r"(at + (uint32_t)(off + q * stride) * 4));
+#pragma unroll
+            for (int q = 0; q < KG; ++q) v.x += x[q].x, v.y += x[q].y, v.z += x[q].z, v.w += x[q].w;
+        }
+        return v;
+    };
+    const int rows = BM / split;   // this CTA finishes its share of the tile's rows
+    for (int e = tid; e < rows * BN / 4; e += THREADS) {
+        const int mi = rank * rows + e / (BN / 4), ni = e % (BN / 4) * 4, m = m0 + mi, n = n0 + ni;
+        if (m >= M || n >= N) continue;
+        const float4 v = add_all(make_float4(0.0f, 0.0f, 0.0f, 0.0f), mi * BN + ni, BM * BN);
+        const int64_t lr = m_base + m;
+        float* crow = Cp + (p.c_idx ? (int64_t)p.c_idx[lr] : lr) * p.ldc;
+        if (vec && n + 3 < N) {
+            emit4<TC2>(p, crow, bias, lr, n, v);
+        } else {
+            emit<TC2>(p, crow, bias, lr, n, v.x);
+            if (n + 1 < N) emit<TC2>(p, crow, bias, lr, n + 1, v.y);
+            if (n + 2 < N) emit<TC2>(p, crow, bias, lr, n + 2, v.z);
+            if (n + 3 < N) emit<TC2>(p, crow, bias, lr, n + 3, v.w);
+        }
+    }
+    if (want_cs && rank == 0 && tid < BN / 4) {
+        const float4 v = add_all(make_float4(0.0f, 0.0f, 0.0f, 0.0f), KG * BM * BN + tid * 4, BN);
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (n0 + tid * 4 + j < N) {
+                float* o = colsum + n0 + tid * 4 + j;
+                *o = p.accumulate ? *o + x[j] : x[j];
+            }
+    }
+    if (split > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");   // peers may still read
+}
+
+// MODE: the operand form of every problem of the launch, or ANY_MODE (mixed forms; costs registers).
+constexpr int ANY_MODE = -1;
+template <class C, int MODE, typename TA, typename TB, typename TC2>
+__global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const __grid_constant__ Multi mp) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int sh_group[2];
+    const int split = mp.split, tile = blockIdx.x / split, rank = blockIdx.x % split;
+    int i = 0;
+#pragma unroll
+    for (int q = 1; q < MAX_PROBLEMS; ++q)
+        if (q < mp.n && tile >= mp.tile0[q]) i = q;
+    const Params& p = mp.p[i];
+    const int t = tile - mp.tile0[i];
+    const int mode = MODE == ANY_MODE ? p.mode : MODE;
+    if (mode == ASCA_TN && p.A == nullptr) {
+        if (rank == 0) colsum_tile(p, t, smem);
+    } else if (mode == ASCA_NN) {
+        tile_product<C, ASCA_NN, TA, TB, TC2>(p, t, rank, split, smem, sh_group);
+    } else if (mode == ASCA_TN) {
+        tile_product<C, ASCA_TN, TA, TB, TC2>(p, t, rank, split, smem, sh_group);
+    } else {
+        tile_product<C, ASCA_NT, TA, TB, TC2>(p, t, rank, split, smem, sh_group);
     }
 }
 
-// Number of CTAs for a launch (upper bound for GROUP_M: every group can add one ragged tile).
-inline int64_t grid_size(const Params& p, int64_t total_token_rows) {
-    const int64_t tn = (p.N + BN - 1) / BN;
-    if (p.group_dim == GROUP_NONE) return ((p.M + BM - 1) / BM) * tn;
-    if (p.group_dim == GROUP_M) return (total_token_rows / BM + p.n_groups) * tn;
-    return (int64_t)p.n_groups * ((p.M + BM - 1) / BM) * tn;
+// Tiles of one problem (upper bound for GROUP_M: every group can add one ragged tile).
+template <class C>
+inline int64_t tiles_of(const Params& p) {
+    if (p.mode == ASCA_TN && !p.A) return (p.N + 7) / 8;
+    const int64_t tn = (p.N + C::BN - 1) / C::BN, tm = std::max<int64_t>(1, (p.M + C::BM - 1) / C::BM);
+    if (p.group_dim == GROUP_NONE) return tm * tn;
+    if (p.group_dim == GROUP_M) return (p.total_rows / C::BM + p.n_groups) * tn;
+    return (int64_t)p.n_groups * tm * tn;
 }
 
+template <class C, int MODE, typename TA, typename TB, typename TC2>
+inline cudaError_t launch_mode(asca_ctx* ctx, Multi& m, int split) {
+    int64_t tiles = 0;
+    for (int i = 0; i < m.n; ++i) {
+        m.tile0[i] = (int)tiles;
+        tiles += tiles_of<C>(m.p[i]);
+    }
+    m.tile0[m.n] = (int)tiles;
+    m.split = split;
+    if (tiles == 0) return cudaSuccess;
+    auto kern = gemm_kernel<C, MODE, TA, TB, TC2>;
+    if (C::SMEM > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * split));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)split;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = split > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, (const Multi)m);
+}
+
+template <class C, typename TA, typename TB, typename TC2>
+inline cudaError_t launch_cfg(asca_ctx* ctx, Multi& m, int split) {
+    for (int i = 1; i < m.n; ++i)
+        if (m.p[i].mode != m.p[0].mode) return launch_mode<C, ANY_MODE, TA, TB, TC2>(ctx, m, split);
+    if (m.p[0].mode == ASCA_NN) return launch_mode<C, ASCA_NN, TA, TB, TC2>(ctx, m, split);
+    if (m.p[0].mode == ASCA_TN) return launch_mode<C, ASCA_TN, TA, TB, TC2>(ctx, m, split);
+    return launch_mode<C, ASCA_NT, TA, TB, TC2>(ctx, m, split);
+}
+
+// Estimated microseconds of a launch, from the measured time of a slab on an SM (CTAs that share an SM add their slabs: the
+// kernel is bound by its own issue, not by latency), of a CTA's prologue and epilogue, and of a launch. Measured on B200,
+// back to back in a graph: 64 x 64 tiles 1.0 us a slab (2048 x 576 x 192: 16 us = 28 TFLOP/s; 8192-long
+// weight gradients with the k-split 65 us, 272 without), 32 x 32 tiles 0.81 us (2048 x 64 x 64: 3.5 us), 128 x 128 tiles
+// 1.6 us (4096^3: 2.7 - 2.9 ms = 47 - 51 TFLOP/s). A k-split pays for the cluster's two barriers and the exchange.
+struct Shape {
+    double slab, cta, cta_split, launch;
+};
+template <class C>
+inline double estimate(const Multi& m, int split, int n_sm, const Shape& c) {
+    double ctas = 0.0, slabs = 0.0, longest = 0.0;
+    for (int i = 0; i < m.n; ++i) {
+        const Params& p = m.p[i];
+        if (p.mode == ASCA_TN && !p.A) continue;
+        const double tn = (p.N + C::BN - 1) / C::BN, groups = p.group_dim == GROUP_NONE ? 1 : p.n_groups;
+        const double mean = (double)p.total_rows / groups;   // token rows of a group
+        const double tm = std::ceil((p.group_dim == GROUP_M ? mean : (double)p.M) / C::BM);
+        const double k = (p.group_dim == GROUP_K ? mean : (double)p.K) + p.K2;
+        const double t = groups * tm * tn, s = std::max(1.0, std::ceil(k / C::BK) / split);
+        ctas += t * split;
+        slabs += t * split * s;
+        longest = std::max(longest, s);
+    }
+    if (ctas == 0.0) return c.launch;
+    const double rounds = std::ceil(ctas / n_sm);
+    return c.launch + std::max(rounds * slabs / ctas, longest) * c.slab + rounds * (split > 1 ? c.cta_split : c.cta);
+}
+
+inline void plan(const asca_ctx* ctx, const Multi& m, int& shape, int& split) {
+    const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    double best = 1e300;
+    shape = split = 1;
+    for (int s = 1; s <= 8; s *= 2) {
+        const double e[3] = {s > 1 ? 1e300 : estimate<CfgL>(m, s, n_sm, {1.6, 7.0, 0.0, 3.3}),
+                             estimate<CfgM>(m, s, n_sm, {1.0, 0.8, 3.8, 3.3}), estimate<CfgS>(m, s, n_sm, {0.81, 0.8, 2.3, 2.6})};
+        for (int c = 0; c < 3; ++c)
+            if (e[c] < best) {
+                best = e[c];
+                shape = c;
+                split = s;
+            }
+    }
+}
+
+// One launch of up to MAX_PROBLEMS f32 products.
+inline cudaError_t launch_f32(asca_ctx* ctx, Multi& m) {
+    int shape, split;
+    plan(ctx, m, shape, split);
+    if (shape == 0) return launch_cfg<CfgL, float, float, float>(ctx, m, split);
+    if (shape == 1) return launch_cfg<CfgM, float, float, float>(ctx, m, split);
+    return launch_cfg<CfgS, float, float, float>(ctx, m, split);
+}
+
+// One product with operands of either type. bf16 operands come here only where the tensor-core kernels cannot take the
+// shape (odd pitches, few columns), so they have the middle tile shape alone.
 template <typename TC2 = float>
-inline cudaError_t launch(const Params& p, int mode, int a_bf16, int b_bf16, int64_t total_token_rows,
-                          cudaStream_t s) {
-    const int64_t g = grid_size(p, total_token_rows);
-    if (g <= 0) return cudaSuccess;
-    dim3 grid((unsigned)g), block(THREADS);
-#define ASCA_GEMM_CASE(MD, TA_, TB_) gemm_kernel<MD, TA_, TB_, TC2><<<grid, block, 0, s>>>(p)
-#define ASCA_GEMM_MODE(MD)                                                       \
-    if (!a_bf16 && !b_bf16) ASCA_GEMM_CASE(MD, float, float);                    \
-    else if (a_bf16 && b_bf16) ASCA_GEMM_CASE(MD, __nv_bfloat16, __nv_bfloat16); \
-    else if (a_bf16) ASCA_GEMM_CASE(MD, __nv_bfloat16, float);                   \
-    else ASCA_GEMM_CASE(MD, float, __nv_bfloat16)
-    if (mode == ASCA_NN) { ASCA_GEMM_MODE(ASCA_NN); }
-    else if (mode == ASCA_TN) { ASCA_GEMM_MODE(ASCA_TN); }
-    else { ASCA_GEMM_MODE(ASCA_NT); }
-#undef ASCA_GEMM_MODE
-#undef ASCA_GEMM_CASE
-    return cudaGetLastError();
+inline cudaError_t launch(asca_ctx* ctx, const Params& p, int a_bf16, int b_bf16) {
+    Multi m{};
+    m.p[0] = p;
+    m.n = 1;
+    if (!a_bf16 && !b_bf16) return launch_f32(ctx, m);
+    if (a_bf16 && b_bf16) return launch_cfg<CfgM, __nv_bfloat16, __nv_bfloat16, TC2>(ctx, m, 1);
+    if (a_bf16) return launch_cfg<CfgM, __nv_bfloat16, float, TC2>(ctx, m, 1);
+    return launch_cfg<CfgM, float, __nv_bfloat16, TC2>(ctx, m, 1);
 }
 
 }  // namespace gemm

@@ -12,36 +12,8 @@ bool asca_tc_enabled();  // gemm.cu
 
 namespace {
 
-// Column sums of a (rows x cols) f32 matrix, optionally per expert segment of the permuted
-// order and optionally through a row map. Deterministic: each CTA owns 32 columns of one
-// segment and reduces rows in a fixed order. out[g*out_gstride + c].
-__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ src, int64_t ld,
-                                                     const int32_t* __restrict__ row_idx,
-                                                     const int32_t* __restrict__ offsets, int64_t rows_total,
-                                                     int cols, float* __restrict__ out, int64_t out_gstride, int accumulate) {
-    __shared__ float part[8][33];
-    const int g = blockIdx.y;
-    const int64_t lo = offsets ? offsets[g] : 0, hi = offsets ? offsets[g + 1] : rows_total;
-    const int c = blockIdx.x * 32 + (threadIdx.x & 31);
-    const int w = threadIdx.x >> 5;
-    float acc = 0.0f;
-    if (c < cols)
-        for (int64_t r = lo + w; r < hi; r += 8) {
-            int64_t mr = row_idx ? (int64_t)row_idx[r] : r;
-            acc += src[mr * ld + c];
-        }
-    part[w][threadIdx.x & 31] = acc;
-    __syncthreads();
-    if (w == 0 && c < cols) {
-        float t = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) t += part[i][threadIdx.x];
-        float* o = out + (int64_t)g * out_gstride + c;
-        *o = accumulate ? *o + t : t;
-    }
-}
-
-// The same sums for a bf16 matrix grouped by expert segment: each CTA owns 64 columns (a lane two) of one segment.
+// Column sums of a bf16 matrix grouped by expert segment, rows in a fixed order: each CTA owns 64 columns (a lane two) of
+// one segment. out[g*out_gstride + c].
 __global__ void __launch_bounds__(256) colsum_bf16_seg_kernel(const __nv_bfloat16* __restrict__ src, int64_t ld,
                                                               const int32_t* __restrict__ offsets, int cols,
                                                               float* __restrict__ out, int64_t out_gstride, int accumulate) {
@@ -309,8 +281,9 @@ int asca_moe_fwd(asca_ctx* ctx, const void* xn, const void* w1, const float* b1,
     p.bias = b1; p.bias_gstride = F;
     p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_M;
     p.epi = gemm::EPI_SILU; p.C2 = hid_p; p.ldc2 = F;
-    if (bf) ASCA_CUDA(ctx, gemm::launch<__nv_bfloat16>(p, ASCA_NN, 1, 1, N, ctx->stream));
-    else ASCA_CUDA(ctx, gemm::launch<float>(p, ASCA_NN, 0, 0, N, ctx->stream));
+    p.mode = ASCA_NN; p.total_rows = N;
+    if (bf) ASCA_CUDA(ctx, gemm::launch<__nv_bfloat16>(ctx, p, 1, 1));
+    else ASCA_CUDA(ctx, gemm::launch<float>(ctx, p, 0, 0));
     ctx->launches++;
     // out[perm[r],:] = hid_p[r,:] W2[eF:(e+1)F,:] + b2
     gemm::Params q{};
@@ -321,7 +294,8 @@ int asca_moe_fwd(asca_ctx* ctx, const void* xn, const void* w1, const float* b1,
     q.bias = b2; q.bias_gstride = 0;
     q.offsets = offsets; q.n_groups = (int)E; q.group_dim = gemm::GROUP_M;
     q.epi = gemm::EPI_NONE;
-    ASCA_CUDA(ctx, gemm::launch<float>(q, ASCA_NN, bf, bf, N, ctx->stream));
+    q.mode = ASCA_NN; q.total_rows = N;
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, q, bf, bf));
     ctx->launches++;
     return ASCA_OK;
 }
@@ -354,57 +328,58 @@ static int moe_bwd_impl(asca_ctx* ctx, const void* xn, const void* w1, const voi
     ASCA_TRY(asca_workspace(ctx, (size_t)N * F * 4 + 256, &ws));
     float* dpre_p = (float*)ws;
 
-    // d_b2[c] = sum over all tokens of dout[t,c]
-    ASCA_TRY(asca_colsum(ctx, dout, d, N, d, d_b2, acc));   // row-sliced, deterministic
-    // d_w2[eF+j, c] = sum_r hid_p[r,j] dout[perm[r],c]      (TN, K = rows of expert e)
-    {
-        gemm::Params p{};
-        p.A = hid_p; p.lda = F;
-        p.B = dout; p.ldb = d; p.b_idx = perm;
-        p.C = d_w2; p.ldc = d; p.c_gstride = F * d; p.accumulate = acc;
-        p.M = (int)F; p.N = (int)d; p.K = 0;
-        p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_K;
-        ASCA_CUDA(ctx, gemm::launch<float>(p, ASCA_TN, bf, 0, N, s));
-        ctx->launches++;
+    // first launch: d_b2, d_w2 and dpre_p, which read dout only
+    gemm::Params db2{};   // d_b2[c] = sum over all tokens of dout[t,c]
+    db2.mode = ASCA_TN; db2.B = dout; db2.ldb = d; db2.N = (int)d; db2.K = (int)N;
+    db2.colsum = d_b2; db2.accumulate = acc;
+    gemm::Params dw2{};   // d_w2[eF+j, c] = sum_r hid_p[r,j] dout[perm[r],c]      (TN, K = rows of expert e)
+    dw2.mode = ASCA_TN;
+    dw2.A = hid_p; dw2.lda = F;
+    dw2.B = dout; dw2.ldb = d; dw2.b_idx = perm;
+    dw2.C = d_w2; dw2.ldc = d; dw2.c_gstride = F * d; dw2.accumulate = acc;
+    dw2.M = (int)F; dw2.N = (int)d;
+    dw2.offsets = offsets; dw2.n_groups = (int)E; dw2.group_dim = gemm::GROUP_K; dw2.total_rows = N;
+    gemm::Params dpre{};  // dpre_p[r,j] = (sum_c dout[perm[r],c] W2[eF+j,c]) * silu'(pre_p[r,j])   (NT)
+    dpre.mode = ASCA_NT;
+    dpre.A = dout; dpre.lda = d; dpre.a_idx = perm;
+    dpre.B = w2; dpre.ldb = d; dpre.b_gstride = F * d;
+    dpre.C = dpre_p; dpre.ldc = F;
+    dpre.N = (int)F; dpre.K = (int)d;
+    dpre.offsets = offsets; dpre.n_groups = (int)E; dpre.group_dim = gemm::GROUP_M; dpre.total_rows = N;
+    dpre.epi = gemm::EPI_SILU_BWD; dpre.aux = pre_p; dpre.ldaux = F;
+    // second launch: d_w1 with d_b1 beside it, and dxn, which read dpre_p
+    gemm::Params dw1{};   // d_w1[c, eF+j] = sum_r xn[perm[r],c] dpre_p[r,j];  d_b1[eF+j] = sum_r dpre_p[r,j]   (TN)
+    dw1.mode = ASCA_TN;
+    dw1.A = xn; dw1.lda = d; dw1.a_idx = perm;
+    dw1.B = dpre_p; dw1.ldb = F;
+    dw1.C = d_w1; dw1.ldc = E * F; dw1.c_gstride = F; dw1.accumulate = acc;
+    dw1.M = (int)d; dw1.N = (int)F;
+    dw1.offsets = offsets; dw1.n_groups = (int)E; dw1.group_dim = gemm::GROUP_K; dw1.total_rows = N;
+    dw1.colsum = d_b1; dw1.colsum_gstride = F;
+    gemm::Params dx{};    // dxn[perm[r], c] = sum_j dpre_p[r,j] W1[c, eF+j]          (NT)
+    dx.mode = ASCA_NT;
+    dx.A = dpre_p; dx.lda = F;
+    dx.B = w1; dx.ldb = E * F; dx.b_gstride = F;
+    dx.C = dxn; dx.ldc = d; dx.c_idx = perm;
+    dx.N = (int)d; dx.K = (int)F;
+    dx.offsets = offsets; dx.n_groups = (int)E; dx.group_dim = gemm::GROUP_M; dx.total_rows = N;
+    if (!bf) {
+        gemm::Multi m{};
+        m.n = 3;
+        m.p[0] = dw2; m.p[1] = dpre; m.p[2] = db2;
+        ASCA_CUDA(ctx, gemm::launch_f32(ctx, m));
+        m.n = 2;
+        m.p[0] = dw1; m.p[1] = dx;
+        ASCA_CUDA(ctx, gemm::launch_f32(ctx, m));
+        ctx->launches += 2;
+        return ASCA_OK;
     }
-    // dpre_p[r,j] = (sum_c dout[perm[r],c] W2[eF+j,c]) * silu'(pre_p[r,j])   (NT)
-    {
-        gemm::Params p{};
-        p.A = dout; p.lda = d; p.a_idx = perm;
-        p.B = w2; p.ldb = d; p.b_gstride = F * d;
-        p.C = dpre_p; p.ldc = F;
-        p.M = 0; p.N = (int)F; p.K = (int)d;
-        p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_M;
-        p.epi = gemm::EPI_SILU_BWD; p.aux = pre_p; p.ldaux = F;
-        ASCA_CUDA(ctx, gemm::launch<float>(p, ASCA_NT, 0, bf, N, s));
-        ctx->launches++;
-    }
-    // d_b1[eF+j] = sum over expert e's rows of dpre_p[r,j]
-    colsum_kernel<<<dim3((unsigned)ceil_div64(F, 32), (unsigned)E), 256, 0, s>>>(dpre_p, F, nullptr, offsets, N, (int)F,
-                                                                               d_b1, F, acc);
-    ASCA_CHECK_LAUNCH(ctx);
-    // d_w1[c, eF+j] = sum_r xn[perm[r],c] dpre_p[r,j]        (TN, K = rows of expert e)
-    {
-        gemm::Params p{};
-        p.A = xn; p.lda = d; p.a_idx = perm;
-        p.B = dpre_p; p.ldb = F;
-        p.C = d_w1; p.ldc = E * F; p.c_gstride = F; p.accumulate = acc;
-        p.M = (int)d; p.N = (int)F; p.K = 0;
-        p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_K;
-        ASCA_CUDA(ctx, gemm::launch<float>(p, ASCA_TN, bf, 0, N, s));
-        ctx->launches++;
-    }
-    // dxn[perm[r], c] = sum_j dpre_p[r,j] W1[c, eF+j]          (NT)
-    {
-        gemm::Params p{};
-        p.A = dpre_p; p.lda = F;
-        p.B = w1; p.ldb = E * F; p.b_gstride = F;
-        p.C = dxn; p.ldc = d; p.c_idx = perm;
-        p.M = 0; p.N = (int)d; p.K = (int)F;
-        p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_M;
-        ASCA_CUDA(ctx, gemm::launch<float>(p, ASCA_NT, 0, bf, N, s));
-        ctx->launches++;
-    }
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, db2, 0, 0));
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, dw2, 1, 0));
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, dpre, 0, 1));
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, dw1, 1, 0));
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, dx, 0, 1));
+    ctx->launches += 5;
     return ASCA_OK;
 }
 
