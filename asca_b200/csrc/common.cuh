@@ -32,6 +32,15 @@ struct asca_ctx {
     void* ws = nullptr;
     size_t ws_bytes = 0;
     int* err_word = nullptr;  // device int the kernels with bounded waits write to
+    // Pinned staging of small host arrays (ids, losses, tokens): copies that neither block the host nor wait for each
+    // other; what goes out is handed to the caller's arrays by the asca_ctx_sync that ends the call.
+    char* pin = nullptr;
+    size_t pin_used = 0;
+    struct PinOut {
+        void* dst;
+        size_t at, bytes;
+    };
+    std::vector<PinOut> pin_out;
     // Dynamic tile claims of the persistent tensor-core products (gemm_tc.cu; ASCA_GEMM_DYNAMIC=0 turns them off).
     // dyn_buf: two counters + the walkers' claim rings.
     void* dyn_buf = nullptr;
@@ -111,6 +120,17 @@ inline cudaError_t asca_launch(asca_ctx* ctx, void (*kern)(KArgs...), dim3 grid,
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 #endif
+// Small host arrays through the context's pinned staging area (a call that uses it ends with asca_ctx_sync, or
+// asca_stage_drop where it fails half way). stage_in: host -> device; stage_out: device -> host, delivered by asca_ctx_sync.
+constexpr size_t ASCA_PIN_BYTES = (size_t)1 << 20;
+int asca_stage_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
+int asca_stage_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
+// Drops what is staged (and waits for the copies that read it) when a call leaves without asca_ctx_sync.
+struct asca_stage_scope {
+    asca_ctx* ctx;
+    explicit asca_stage_scope(asca_ctx* c) : ctx(c) {}
+    ~asca_stage_scope();
+};
 // Returns scratch of at least `bytes` (256-byte aligned); contents are undefined.
 int asca_workspace(asca_ctx* ctx, size_t bytes, void** out);
 

@@ -2,6 +2,8 @@
 // singleton and its DevBuf pool (rust/src/cuda/mod.rs:104-237).
 #include "common.cuh"
 
+#include <cstring>
+
 int asca_fail(asca_ctx* ctx, int code, const char* fmt, ...) {
     char buf[512];
     va_list ap;
@@ -25,6 +27,45 @@ int asca_workspace(asca_ctx* ctx, size_t bytes, void** out) {
     }
     *out = ctx->ws;
     return ASCA_OK;
+}
+
+static int stage_room(asca_ctx* ctx, size_t bytes, char** at) {
+    const size_t want = (bytes + 63) & ~(size_t)63;
+    *at = nullptr;
+    if (want + 64 > ASCA_PIN_BYTES) return ASCA_OK;   // (the last 64 bytes hold the error word's copy)
+    if (!ctx->pin && cudaHostAlloc((void**)&ctx->pin, ASCA_PIN_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return asca_fail(ctx, ASCA_ERR_OOM, "cannot allocate the pinned staging area");
+    }
+    if (ctx->pin_used + want + 64 > ASCA_PIN_BYTES) return ASCA_OK;
+    *at = ctx->pin + ctx->pin_used;
+    ctx->pin_used += want;
+    return ASCA_OK;
+}
+
+int asca_stage_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    char* at;
+    int rc = stage_room(ctx, bytes, &at);
+    if (rc != ASCA_OK) return rc;
+    if (at) memcpy(at, src, bytes);
+    ASCA_CUDA(ctx, cudaMemcpyAsync(dst, at ? at : src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    return ASCA_OK;
+}
+
+int asca_stage_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    char* at;
+    int rc = stage_room(ctx, bytes, &at);
+    if (rc != ASCA_OK) return rc;
+    ASCA_CUDA(ctx, cudaMemcpyAsync(at ? at : dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    if (at) ctx->pin_out.push_back({dst, (size_t)(at - ctx->pin), bytes});
+    return ASCA_OK;
+}
+
+asca_stage_scope::~asca_stage_scope() {
+    if (ctx->pin_used == 0) return;   // asca_ctx_sync has delivered everything
+    cudaStreamSynchronize(ctx->stream);
+    ctx->pin_used = 0;
+    ctx->pin_out.clear();
 }
 
 extern "C" {
@@ -77,6 +118,7 @@ int asca_ctx_destroy(asca_ctx* ctx) {
         cudaFree(kv.second.second);
     }
     if (ctx->err_word) cudaFree(ctx->err_word);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     if (ctx->dyn_buf) cudaFree(ctx->dyn_buf);
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
@@ -104,13 +146,18 @@ int asca_ctx_set_stream(asca_ctx* ctx, void* s) {
 
 int asca_ctx_sync(asca_ctx* ctx) {
     if (!ctx) return ASCA_ERR_ARG;
+    // kernels with bounded waits report a give-up through the error word; its copy rides in front of the one wait
+    char* at;
+    ASCA_TRY(stage_room(ctx, 4, &at));   // (allocates the area)
+    int* word = reinterpret_cast<int*>(ctx->pin + ASCA_PIN_BYTES - 64);
+    ASCA_CUDA(ctx, cudaMemcpyAsync(word, ctx->err_word, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    // kernels with bounded waits report a give-up through this word
-    int word = 0;
-    ASCA_CUDA(ctx, cudaMemcpy(&word, ctx->err_word, sizeof(int), cudaMemcpyDeviceToHost));
-    if (word != 0) {
+    for (const auto& o : ctx->pin_out) memcpy(o.dst, ctx->pin + o.at, o.bytes);
+    ctx->pin_out.clear();
+    ctx->pin_used = 0;
+    if (*word != 0) {
         cudaMemset(ctx->err_word, 0, sizeof(int));
-        return asca_fail(ctx, ASCA_ERR_DEVICE, "a kernel gave up on a bounded wait (code %d)", word);
+        return asca_fail(ctx, ASCA_ERR_DEVICE, "a kernel gave up on a bounded wait (code %d)", *word);
     }
     return ASCA_OK;
 }

@@ -432,7 +432,8 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
     bf16 *x16 = h16(ns * d), *o16 = h16(ns * d), *xn16 = h16(ns * d), *hid16 = h16(ns * F), *hf16 = h16(ns * d);
     ASCA_REQUIRE(ctx, ids && toks && perm && offs && x && qkv && gate && o && y && x_mid && mo && logits && pre_p && x16 && o16 &&
                           xn16 && hid16 && hf16, "model_decode_step: out of memory");
-    ASCA_CUDA(ctx, cudaMemcpyAsync(ids, ids_h, (size_t)ns * 4, cudaMemcpyHostToDevice, ctx->stream));
+    asca_stage_scope staged(ctx);
+    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)ns * 4));
     const bool fused64 = dh == 64;   // one projection for qkv + gate, the warp-per-head state update, casts folded in
     const int64_t ldq = (3 * d + 2 * H + 7) & ~(int64_t)7;
     if (fused64) ASCA_TRY(refresh_dec_w(ctx, m));
@@ -537,7 +538,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
     else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, hf16, d, W + m->head16, V, logits, V, nullptr, 0, BF));
     if (logits_h && step == n_steps - 1) {
         ctx->pdl = false;   // a copy sits between the head product and the argmax
-        ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)ns * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
     }
     if (next_h || tokens_h || step + 1 < n_steps) {
         ASCA_CUDA(ctx, asca_launch(ctx, argmax_kernel, dim3((unsigned)ceil_div64(ns, 8)), dim3(256), 0, (const float*)logits, ns, (int)V, nxt));
@@ -545,8 +546,57 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
     }
     ctx->pdl = false;
     }   // steps
-    if (next_h) ASCA_CUDA(ctx, cudaMemcpyAsync(next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (tokens_h) ASCA_CUDA(ctx, cudaMemcpyAsync(tokens_h, toks, (size_t)ns * n_steps * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4));
+    if (tokens_h) ASCA_TRY(asca_stage_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
+    return asca_ctx_sync(ctx);
+}
+
+// decode_f32.cu: all steps in one launch, where a stream's states fit a cluster's shared memory
+int asca_decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* ids, int64_t ns, int64_t n_steps, uint32_t* tokens,
+                    float* logits);
+
+// f32 decode, n_steps greedy steps from ids_h. Host outputs (each nullable): the last step's logits and choice, every
+// step's choice.
+static int decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* ids_h, int64_t ns, int64_t n_steps, float* logits_h,
+                      uint32_t* next_h, uint32_t* tokens_h) {
+    const int64_t d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab;
+    const float* P = m->params;
+    Bufs bf(ctx);
+    asca_stage_scope staged(ctx);
+    uint32_t* ids = (uint32_t*)bf.f(ns);
+    uint32_t* toks = (uint32_t*)bf.f(ns * n_steps);
+    float* logits = bf.f(ns * V);
+    ASCA_REQUIRE(ctx, ids && toks && logits, "model_decode_step: out of memory");
+    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)ns * 4));
+    int rc = asca_decode_f32(ctx, m, state, ids, ns, n_steps, toks, logits_h ? logits : nullptr);
+    if (rc == ASCA_ERR_UNSUPPORTED) {   // step by step through the single kernels
+        float *x = bf.f(ns * d), *qkv = bf.f(ns * 3 * d), *gate = bf.f(ns * 2 * H), *o = bf.f(ns * d), *y = bf.f(ns * d),
+              *x_mid = bf.f(ns * d), *mo = bf.f(ns * d), *hf = bf.f(ns * d);
+        ASCA_REQUIRE(ctx, x && qkv && gate && o && y && x_mid && mo && hf, "model_decode_step: out of memory");
+        for (int64_t t = 0; t < n_steps; ++t) {
+            const uint32_t* cur = t == 0 ? ids : toks + (t - 1) * ns;
+            ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, cur, ns, d, x));
+            for (int64_t li = 0; li < m->L; ++li) {
+                const Lyr& w = m->lay[li];
+                ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 3 * d, d, x, d, P + w.w_qkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, ASCA_F32));
+                ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 2 * H, d, x, d, P + w.w_gate, 2 * H, gate, 2 * H, P + w.b_gate, 0, ASCA_F32));
+                ASCA_TRY(asca_delta_step(ctx, qkv, nullptr, nullptr, gate, nullptr, state + li * ns * H * dh * dh, ns, H, dh, 1, o));
+                ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, d, d, o, d, P + w.w_o, d, y, d, P + w.b_o, 0, ASCA_F32));
+                ASCA_TRY(asca_residual_rmsnorm(ctx, x, y, x_mid, nullptr, ns, d, 1e-6f));
+                ASCA_TRY(asca_moe_step(ctx, x_mid, cur, P + w.w1, P + w.b1, P + w.w2, P + w.b2, ns, d, F, E, ASCA_F32, mo));
+                ASCA_TRY(asca_residual_rmsnorm(ctx, x_mid, mo, x, nullptr, ns, d, 1e-6f));
+            }
+            ASCA_TRY(asca_rmsnorm_fwd(ctx, x, hf, nullptr, ns, d, 1e-6f));
+            ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, hf, d, P + m->head, V, logits, V, nullptr, 0, ASCA_F32));
+            argmax_kernel<<<(unsigned)ceil_div64(ns, 8), 256, 0, ctx->stream>>>(logits, ns, (int)V, toks + t * ns);
+            ASCA_CHECK_LAUNCH(ctx);
+        }
+    } else {
+        ASCA_TRY(rc);
+    }
+    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
+    if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4));
+    if (tokens_h) ASCA_TRY(asca_stage_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
 
@@ -590,8 +640,9 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
     int32_t* perm = (int32_t*)bf.f(N);
     int32_t* offs = (int32_t*)bf.f(E + 1);
     ASCA_REQUIRE(ctx, ids && tg && perm && offs, "model_forward_backward: out of memory");
-    ASCA_CUDA(ctx, cudaMemcpyAsync(ids, ids_h, (size_t)N * 4, cudaMemcpyHostToDevice, ctx->stream));
-    ASCA_CUDA(ctx, cudaMemcpyAsync(tg, tg_h, (size_t)N * 4, cudaMemcpyHostToDevice, ctx->stream));
+    asca_stage_scope staged(ctx);
+    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
+    ASCA_TRY(asca_stage_in(ctx, tg, tg_h, (size_t)N * 4));
     ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));
 
     struct Act {
@@ -677,12 +728,12 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
         ASCA_TRY(gemm_tc::launch(ctx, th));
         mean_kernel<<<1, 1024, 0, ctx->stream>>>(dlogits, N, 1.0f / (float)N, loss_d);
         ASCA_CHECK_LAUNCH(ctx);
-        ASCA_CUDA(ctx, cudaMemcpyAsync(loss_h, loss_d, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
     } else {
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, V, d, h_final, d, W + m->head16, V, logits, V, nullptr, 0, BF));
         if (logits_h) ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)N * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
         ASCA_TRY(cross_entropy_scaled(ctx, logits, tg, N, V, dlogits, loss_d, m->grad_scale));
-        ASCA_CUDA(ctx, cudaMemcpyAsync(loss_h, loss_d, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
         ASCA_TRY(asca_cast_bf16(ctx, dlogits, dl16, N * V));
     }
     ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, V, N, h_final, d, dl16, V, G + m->head, V, nullptr, acc, BF));
@@ -1039,8 +1090,9 @@ int asca_model_forward_backward_host(asca_ctx* ctx, asca_model* m, const uint32_
     int32_t* perm = (int32_t*)bf.f(N);
     int32_t* offs = (int32_t*)bf.f(E + 1);
     ASCA_REQUIRE(ctx, ids && tg && perm && offs, "model_forward_backward: out of memory");
-    ASCA_CUDA(ctx, cudaMemcpyAsync(ids, ids_h, (size_t)N * 4, cudaMemcpyHostToDevice, ctx->stream));
-    ASCA_CUDA(ctx, cudaMemcpyAsync(tg, tg_h, (size_t)N * 4, cudaMemcpyHostToDevice, ctx->stream));
+    asca_stage_scope staged(ctx);
+    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
+    ASCA_TRY(asca_stage_in(ctx, tg, tg_h, (size_t)N * 4));
     ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));   // same routing for every layer
 
     struct Act {
@@ -1086,7 +1138,7 @@ int asca_model_forward_backward_host(asca_ctx* ctx, asca_model* m, const uint32_
     if (logits_h) ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)N * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
     // ---- backward (rust/src/model.rs:744-794)
     ASCA_TRY(cross_entropy_scaled(ctx, logits, tg, N, V, dlogits, loss_d, m->grad_scale));
-    ASCA_CUDA(ctx, cudaMemcpyAsync(loss_h, loss_d, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
     ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, V, N, h_final, d, dlogits, V, G + m->head, V, nullptr, acc, ASCA_F32));
     float* dh_ = bf.f(N * d);
     float* dx = bf.f(N * d);
@@ -1258,13 +1310,11 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && qkv && gate && y && x_mid && mo && qn && kn && al && be && pre_p &&
                           s_fin && xl && hf && logits && q && k && v && o && xn && hid_p && (!bfm || (x_in && hf_in)),
                  "model_prefill: out of memory");
-    ASCA_CUDA(ctx, cudaMemcpyAsync(ids, ids_h, (size_t)N * 4, cudaMemcpyHostToDevice, ctx->stream));
-    {
-        std::vector<int32_t> lh(ns);
-        for (int64_t s_ = 0; s_ < ns; ++s_) lh[s_] = (int32_t)(s_ * T + T - 1);
-        ASCA_CUDA(ctx, cudaMemcpyAsync(last, lh.data(), (size_t)ns * 4, cudaMemcpyHostToDevice, ctx->stream));
-        ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // lh leaves scope
-    }
+    asca_stage_scope staged(ctx);
+    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
+    std::vector<int32_t> lh(ns);
+    for (int64_t s_ = 0; s_ < ns; ++s_) lh[s_] = (int32_t)(s_ * T + T - 1);
+    ASCA_TRY(asca_stage_in(ctx, last, lh.data(), (size_t)ns * 4));
     ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));
     ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, x));
     const size_t st_layer = (size_t)ns * H * dh * dh;
@@ -1301,11 +1351,11 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
         ASCA_TRY(asca_rmsnorm_fwd(ctx, xl, hf, nullptr, ns, d, 1e-6f));
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, hf, d, P + m->head, V, logits, V, nullptr, 0, DT));
     }
-    if (logits_h) ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)ns * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
     if (next_h) {
         argmax_kernel<<<(unsigned)ceil_div64(ns, 8), 256, 0, ctx->stream>>>(logits, ns, (int)V, nxt);
         ASCA_CHECK_LAUNCH(ctx);
-        ASCA_CUDA(ctx, cudaMemcpyAsync(next_h, nxt, (size_t)ns * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        ASCA_TRY(asca_stage_out(ctx, next_h, nxt, (size_t)ns * 4));
     }
     return asca_ctx_sync(ctx);
 }
@@ -1316,49 +1366,16 @@ int asca_model_decode_greedy_host(asca_ctx* ctx, asca_model* m, float* state, co
     ASCA_REQUIRE(ctx, state && ids_h && tokens_h && ns > 0 && n_steps > 0, "model_decode_greedy: bad arguments");
     for (int64_t i = 0; i < ns; ++i) ASCA_REQUIRE(ctx, ids_h[i] < (uint32_t)m->vocab, "model_decode_greedy: id out of range");
     if (m->compute == ASCA_BF16) return decode_step_bf16(ctx, m, state, ids_h, ns, nullptr, nullptr, n_steps, tokens_h);
-    const uint32_t* cur = ids_h;   // f32 mode: the single-step path, token by token
-    for (int64_t t = 0; t < n_steps; ++t) {
-        ASCA_TRY(asca_model_decode_step_host(ctx, m, state, cur, ns, nullptr, tokens_h + t * ns));
-        cur = tokens_h + t * ns;
-    }
-    return ASCA_OK;
+    return decode_f32(ctx, m, state, ids_h, ns, n_steps, nullptr, nullptr, tokens_h);
 }
 
 int asca_model_decode_step_host(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* ids_h, int64_t ns,
                                 float* logits_h, uint32_t* next_h) {
     if (!ctx || !m) return ASCA_ERR_ARG;
     ASCA_REQUIRE(ctx, state && ids_h && ns > 0, "model_decode_step: bad arguments");
-    const int64_t d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab;
-    for (int64_t i = 0; i < ns; ++i) ASCA_REQUIRE(ctx, ids_h[i] < (uint32_t)V, "model_decode_step: id out of range");
+    for (int64_t i = 0; i < ns; ++i) ASCA_REQUIRE(ctx, ids_h[i] < (uint32_t)m->vocab, "model_decode_step: id out of range");
     if (m->compute == ASCA_BF16) return decode_step_bf16(ctx, m, state, ids_h, ns, logits_h, next_h);
-    float* P = m->params;
-    Bufs bf(ctx);
-    uint32_t* ids = (uint32_t*)bf.f(ns);
-    uint32_t* nxt = (uint32_t*)bf.f(ns);
-    float *x = bf.f(ns * d), *qkv = bf.f(ns * 3 * d), *gate = bf.f(ns * 2 * H), *o = bf.f(ns * d), *y = bf.f(ns * d),
-          *x_mid = bf.f(ns * d), *mo = bf.f(ns * d), *hf = bf.f(ns * d), *logits = bf.f(ns * V);
-    ASCA_REQUIRE(ctx, ids && nxt && x && qkv && gate && o && y && x_mid && mo && hf && logits, "model_decode_step: out of memory");
-    ASCA_CUDA(ctx, cudaMemcpyAsync(ids, ids_h, (size_t)ns * 4, cudaMemcpyHostToDevice, ctx->stream));
-    ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, ns, d, x));
-    for (int64_t li = 0; li < m->L; ++li) {
-        const Lyr& w = m->lay[li];
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 3 * d, d, x, d, P + w.w_qkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, ASCA_F32));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 2 * H, d, x, d, P + w.w_gate, 2 * H, gate, 2 * H, P + w.b_gate, 0, ASCA_F32));
-        ASCA_TRY(asca_delta_step(ctx, qkv, nullptr, nullptr, gate, nullptr, state + li * ns * H * dh * dh, ns, H, dh, 1, o));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, d, d, o, d, P + w.w_o, d, y, d, P + w.b_o, 0, ASCA_F32));
-        ASCA_TRY(asca_residual_rmsnorm(ctx, x, y, x_mid, nullptr, ns, d, 1e-6f));
-        ASCA_TRY(asca_moe_step(ctx, x_mid, ids, P + w.w1, P + w.b1, P + w.w2, P + w.b2, ns, d, F, E, ASCA_F32, mo));
-        ASCA_TRY(asca_residual_rmsnorm(ctx, x_mid, mo, x, nullptr, ns, d, 1e-6f));
-    }
-    ASCA_TRY(asca_rmsnorm_fwd(ctx, x, hf, nullptr, ns, d, 1e-6f));
-    ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, hf, d, P + m->head, V, logits, V, nullptr, 0, ASCA_F32));
-    if (logits_h) ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)ns * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (next_h) {
-        argmax_kernel<<<(unsigned)ceil_div64(ns, 8), 256, 0, ctx->stream>>>(logits, ns, (int)V, nxt);
-        ASCA_CHECK_LAUNCH(ctx);
-        ASCA_CUDA(ctx, cudaMemcpyAsync(next_h, nxt, (size_t)ns * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    return asca_ctx_sync(ctx);
+    return decode_f32(ctx, m, state, ids_h, ns, 1, logits_h, next_h, nullptr);
 }
 
 }  // extern "C"

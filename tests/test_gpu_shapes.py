@@ -46,3 +46,33 @@ def test_f32_expert_products_tile_edges(orc, gpu, n, d, F, E, vocab):
     assert rel_err(out, ref_out) < F32_TOL
     for got, ref in zip((r.d_w1, r.d_b1, r.d_w2, r.d_b2, r.dxn), want):
         assert rel_err(got, ref) < F32_TOL
+
+
+# f32 decode: every cluster width (1 .. 8 CTAs a stream), head dims, more CTAs than heads and the other way round, hidden and
+# vocabulary slices that leave CTAs without work, and the two shapes that fall back to single kernels (an odd number of heads;
+# states too large for shared memory).
+@pytest.mark.parametrize("cfg,ns", [((256, 64, 4, 2, 4, 256), 1), ((256, 64, 4, 2, 4, 256), 70), ((256, 96, 6, 1, 8, 20), 3),
+                                    ((256, 192, 6, 3, 8, 640), 19), ((48, 64, 2, 2, 3, 36), 150), ((256, 128, 1, 2, 2, 64), 2),
+                                    ((256, 256, 4, 1, 2, 128), 40), ((256, 80, 5, 2, 4, 64), 3), ((256, 512, 4, 12, 2, 64), 2)])
+def test_f32_decode_cluster_widths_and_fallbacks(orc, gpu, cfg, ns):
+    import asca_b200
+
+    V = cfg[0]
+    ref = orc.Model(*cfg)
+    ref.params[:] = orc.Rng(sum(cfg)).normal(ref.n, 0.8 * cfg[1] ** -0.5)
+    dev = asca_b200.Model(gpu, *cfg)
+    dev.set_params(ref.params)
+    ids = orc.Rng(ns).below(V, ns)
+    state = dev.new_decode_state(ns)
+    toks = dev.decode_greedy(state, ids.copy(), 3)
+    logits, nxt = dev.decode_step(state, toks[-1].copy())
+    for s in sorted({0, ns // 2, ns - 1}):
+        st, tok = ref.new_decode_state(), ids[s]
+        for t in range(3):
+            lg = ref.step(tok, st)
+            tok = int(lg.argmax())
+            assert tok == toks[t, s]
+        lg = ref.step(tok, st)
+        assert rel_err(logits[s:s + 1], lg) < F32_TOL and nxt[s] == lg.argmax()
+        assert rel_err(state[:, s].cpu().numpy(), st) < F32_TOL
+    dev.free()
