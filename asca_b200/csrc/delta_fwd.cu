@@ -1,12 +1,11 @@
 // Gated delta rule, forward direction, f32-exact kernels:
 //   * delta_fwd_rec_kernel -- the per-step recurrence of rust/src/delta.rs:281-315 with the
-//     dh x dh state split by VALUE column across CTAs. Column i of S evolves independently of
-//     the others (u_i, S[.][i] and o_i only touch column i), so a chain (sequence, head) is
-//     cut into dh/16 CTAs of 128 threads that share nothing; each thread keeps dh/8 state
-//     elements in registers and the whole sequence runs without a block barrier inside a
-//     16-step stage. State is written to HBM only at chunk boundaries (checkpoints for the
-//     backward) and once at the end -- never per step as the reference kernel
-//     (rust/kernels/asca.cu:276-312) does.
+//     dh x dh state split by VALUE column. Column i of S evolves independently of the others
+//     (u_i, S[.][i] and o_i only touch column i), so a chain (sequence, head) is cut into
+//     groups of 4 or 8 lanes (and CTAs) that share nothing; the state lives in registers and the
+//     whole sequence runs without a block barrier inside a 16-step stage. State is written to HBM
+//     only at chunk boundaries (checkpoints for the backward) and once at the end -- never per step
+//     as the reference kernel (rust/kernels/asca.cu:276-312) does.
 //   * delta_step_kernel -- the O(1) decode step (rust/src/delta.rs:356-406): one CTA per
 //     (stream, head) streams S through registers once (read + write = the HBM floor).
 #include "common.cuh"
@@ -24,11 +23,6 @@ int forward(asca_ctx* ctx, const void* q, const void* k, const void* v, const fl
 
 namespace {
 
-constexpr int FW = 16;        // value columns per CTA
-constexpr int FAG = 8;        // key-row groups (lanes that share a column)
-constexpr int FTHREADS = FW * FAG;
-constexpr int FTS = 16;       // timesteps per staged block
-
 template <typename T>
 __device__ __forceinline__ float4 ld4(const T* p);
 template <>
@@ -40,24 +34,60 @@ __device__ __forceinline__ float4 ld4<__nv_bfloat16>(const __nv_bfloat16* p) {
     return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
 }
 
-template <int DH, typename T>
-__global__ void __launch_bounds__(FTHREADS) delta_fwd_rec_kernel(
+// Two f32 in one 64-bit register pair. The pairs stay 64-bit values from the load to the store: built from scalars at each use
+// they cost two moves per FFMA.
+typedef unsigned long long pair_t;
+__device__ __forceinline__ pair_t make_pair(float lo, float hi) {
+    pair_t p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+    return p;
+}
+__device__ __forceinline__ float2 unpair(pair_t p) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void fma2(pair_t& d, pair_t a, pair_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+
+// LANES neighbouring lanes share COLS value columns: a lane holds DH / LANES rows of each. NT: threads per CTA.
+template <int DH, int COLS>
+struct RecCfg {
+    static constexpr int LANES = DH == 128 ? 8 : 4, RPT = DH / LANES;
+    static constexpr int ALL = DH / COLS * LANES;             // threads that hold a whole state
+    static constexpr int NT = ALL < 256 ? ALL : (COLS == 1 ? 128 : 256);
+    static constexpr int FW = NT / LANES * COLS;              // value columns per CTA
+    static constexpr int HT = DH == 128 && COLS < 4 ? 128 : 64;           // helper threads: they stage the inputs and store the outputs
+    static constexpr int FTS = DH == 128 && COLS > 1 ? 8 : 16;   // timesteps per staged block (48 KiB of shared memory)
+    static_assert(RPT % 4 == 0 && NT >= 32, "tile shape");
+};
+
+// One step: sk = S^T k and sq = S^T q from the SAME pass over the old state, u = beta v - alpha beta sk,
+// o = alpha sq + (k.q) u, S = alpha S + k u: the output needs no second reduction, and only sk is on the chain from step to
+// step. Rows are held in pairs (k and q arrive as pairs), so all three passes are packed two-lane FFMAs. With COLS > 1 the
+// 2 COLS sums of a lane group are exchanged by halves: after log2 COLS rounds a lane holds the two sums of one column.
+// What bounds it: with COLS = 1 the reads of k and q (8 bytes per state element and step) once a few chains share an SM, the
+// step's latency before that; COLS = 4 reads a quarter and is bound by FFMA issue.
+template <int DH, int COLS, typename T>
+__global__ void __launch_bounds__(RecCfg<DH, COLS>::NT + RecCfg<DH, COLS>::HT) delta_fwd_rec_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ alpha,
     const float* __restrict__ beta, int B, int Tlen, int H, int chunk, T* __restrict__ o,
     const float* __restrict__ s_init, float* __restrict__ s_final, float* __restrict__ ckpt) {
-    constexpr int RPT = DH / FAG;            // state rows per thread
-    constexpr bool VEC = (RPT % 4) == 0;     // rows held as float4 groups
+    using C = RecCfg<DH, COLS>;
+    constexpr int LANES = C::LANES, RPT = C::RPT, NT = C::NT, HT = C::HT, FW = C::FW, FTS = C::FTS;
     constexpr int KQ4 = FTS * DH / 4;        // float4 units of k (or q) per stage
-    constexpr int KQ_PT = (KQ4 + FTHREADS - 1) / FTHREADS;
+    constexpr int KQ_PT = (KQ4 + HT - 1) / HT, V_PT = (FTS * FW + HT - 1) / HT;
+    static_assert(KQ4 % HT == 0, "whole rows per pass");
     __shared__ __align__(16) float k_s[2][FTS][DH];
     __shared__ __align__(16) float q_s[2][FTS][DH];
-    __shared__ float v_s[2][FTS][FW];
-    __shared__ float a_s[2][FTS], b_s[2][FTS];
-    __shared__ float o_s[FTS][FW];
-    __shared__ float ck_s[DH][FW + 1];
+    __shared__ float v_s[2][FTS][FW];        // beta v
+    // per step: product of the stage's alphas up to and with it, its inverse, -alpha beta times the product before it, k.q
+    __shared__ __align__(16) float4 g_s[2][FTS];
+    __shared__ float2 ab_s[2][FTS];          // alpha, beta
+    __shared__ float decay_s[2];             // product of all the stage's alphas
+    __shared__ float o_s[2][FTS][FW];
 
     const int tid = threadIdx.x;
-    const int ag = tid % FAG, col = tid / FAG;
+    const int ag = tid % LANES, cg = tid / LANES;
     const int chain = blockIdx.y;              // b*H + h
     const int bi = chain / H, h = chain % H;
     const int i0 = blockIdx.x * FW;            // first value column of this CTA
@@ -65,146 +95,228 @@ __global__ void __launch_bounds__(FTHREADS) delta_fwd_rec_kernel(
     const int64_t row0 = (int64_t)bi * Tlen;
     const int n_chunks = (Tlen + chunk - 1) / chunk;
 
-    // row index of register slot r
-    auto row_of = [&](int r) -> int {
-        if (VEC) return ((r >> 2) * FAG + ag) * 4 + (r & 3);
-        return r * FAG + ag;
-    };
-
-    float S[RPT];
-    if (s_init) {
-        const float* si = s_init + (int64_t)chain * DH * DH;
+    const int n_stages = (Tlen + FTS - 1) / FTS;
+    if (tid >= NT) {
+        const int ht = tid - NT;
+        // ---- helpers: while a stage is worked on they store the outputs of the one before it, put the one after it into shared
+        // memory and request the one after that; the working threads see one barrier per stage
+        float4 pk[KQ_PT], pq[KQ_PT];
+        float pv[V_PT], pbv[V_PT], pa = 0.0f, pb = 0.0f;
+        auto fetch = [&](int t0) {
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) S[r] = si[row_of(r) * DH + i0 + col];
-    } else {
+            for (int u = 0; u < KQ_PT; ++u) {
+                const int idx = ht + u * HT;
+                int t = idx / (DH / 4), c4 = idx % (DH / 4);
+                if (idx < KQ4 && t0 + t < Tlen) {
+                    int64_t off = (row0 + t0 + t) * d + h * DH + c4 * 4;
+                    pk[u] = ld4<T>(k + off);
+                    pq[u] = ld4<T>(q + off);
+                } else {
+                    pk[u] = make_float4(0, 0, 0, 0);
+                    pq[u] = make_float4(0, 0, 0, 0);
+                }
+            }
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) S[r] = 0.0f;
+            for (int u = 0; u < V_PT; ++u) {
+                const int idx = ht + u * HT;
+                int t = idx / FW, c = idx % FW;
+                const bool ok = idx < FTS * FW && t0 + t < Tlen;
+                pv[u] = ok ? to_f32<T>(v[(row0 + t0 + t) * d + h * DH + i0 + c]) : 0.0f;
+                pbv[u] = ok ? beta[(row0 + t0 + t) * H + h] : 0.0f;
+            }
+            if (ht < FTS && t0 + ht < Tlen) {
+                pa = alpha[(row0 + t0 + ht) * H + h];
+                pb = beta[(row0 + t0 + ht) * H + h];
+            }
+        };
+        auto stash = [&](int buf) {
+#pragma unroll
+            for (int u = 0; u < KQ_PT; ++u) {
+                const int idx = ht + u * HT;
+                int t = idx / (DH / 4), c4 = idx % (DH / 4);
+                float kq = pk[u].x * pq[u].x + pk[u].y * pq[u].y + pk[u].z * pq[u].z + pk[u].w * pq[u].w;   // the row's lanes: one warp
+#pragma unroll
+                for (int m = (DH / 4 < 32 ? DH / 4 : 32) / 2; m > 0; m >>= 1) kq += __shfl_xor_sync(0xffffffffu, kq, m);
+                if (idx < KQ4) {
+                    *reinterpret_cast<float4*>(&k_s[buf][t][c4 * 4]) = pk[u];
+                    *reinterpret_cast<float4*>(&q_s[buf][t][c4 * 4]) = pq[u];
+                    if (c4 == 0) g_s[buf][t].w = kq;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < V_PT; ++u) {
+                const int idx = ht + u * HT;
+                if (idx < FTS * FW) v_s[buf][idx / FW][idx % FW] = pbv[u] * pv[u];
+            }
+            if (ht < 32) {
+                float dec = ht < FTS ? pa : 1.0f;
+#pragma unroll
+                for (int m = 1; m < FTS; m <<= 1) {
+                    const float x = __shfl_up_sync(0xffffffffu, dec, m);
+                    if (ht >= m) dec *= x;
+                }
+                const float before = __shfl_up_sync(0xffffffffu, dec, 1);
+                if (ht < FTS) {
+                    g_s[buf][ht].x = dec;
+                    g_s[buf][ht].y = 1.0f / dec;
+                    g_s[buf][ht].z = -pa * pb * (ht ? before : 1.0f);
+                    ab_s[buf][ht] = make_float2(pa, pb);
+                }
+                if (ht == FTS - 1) decay_s[buf] = dec;
+            }
+        };
+        auto store = [&](int stage) {
+            const int t0 = stage * FTS, steps = Tlen - t0 < FTS ? Tlen - t0 : FTS;
+            for (int idx = ht; idx < steps * FW; idx += HT) {
+                const int ts = idx / FW, c = idx % FW;
+                o[(row0 + t0 + ts) * d + h * DH + i0 + c] = from_f32<T>(o_s[stage & 1][ts][c]);
+            }
+        };
+        fetch(0);
+        stash(0);
+        if (n_stages > 1) fetch(FTS);
+        __syncthreads();
+        for (int st = 0; st < n_stages; ++st) {
+            if (st > 0) store(st - 1);
+            if (st + 1 < n_stages) stash((st + 1) & 1);
+            if (st + 2 < n_stages) fetch((st + 2) * FTS);
+            __syncthreads();
+        }
+        store(n_stages - 1);
+        return;
     }
 
-    // ---- staging: registers hold the next stage while the current one is consumed
-    float4 pk[KQ_PT], pq[KQ_PT];
-    float pv[(FTS * FW + FTHREADS - 1) / FTHREADS];
-    float pa = 0.0f, pb = 0.0f;
-    auto fetch = [&](int t0) {
+    auto row_of = [&](int p) { return ((p >> 1) * LANES + ag) * 4 + (p & 1) * 2; };   // rows (r, r + 1) of pair p
+    pair_t S[RPT / 2][COLS];
 #pragma unroll
-        for (int u = 0; u < KQ_PT; ++u) {
-            int idx = tid + u * FTHREADS;
-            int t = idx / (DH / 4), c4 = idx % (DH / 4);
-            if (idx < KQ4 && t0 + t < Tlen) {
-                int64_t off = (row0 + t0 + t) * d + h * DH + c4 * 4;
-                pk[u] = ld4<T>(k + off);
-                pq[u] = ld4<T>(q + off);
-            } else {
-                pk[u] = make_float4(0, 0, 0, 0);
-                pq[u] = make_float4(0, 0, 0, 0);
-            }
-        }
+    for (int p = 0; p < RPT / 2; ++p)
 #pragma unroll
-        for (int u = 0; u < (FTS * FW + FTHREADS - 1) / FTHREADS; ++u) {
-            int idx = tid + u * FTHREADS;
-            int t = idx / FW, c = idx % FW;
-            pv[u] = (idx < FTS * FW && t0 + t < Tlen) ? to_f32<T>(v[(row0 + t0 + t) * d + h * DH + i0 + c]) : 0.0f;
+        for (int c = 0; c < COLS; ++c) {
+            const float* si = s_init + (int64_t)chain * DH * DH + i0 + cg * COLS + c;
+            S[p][c] = s_init ? make_pair(si[row_of(p) * DH], si[(row_of(p) + 1) * DH]) : 0;
         }
-        if (tid < FTS && t0 + tid < Tlen) {
-            pa = alpha[(row0 + t0 + tid) * H + h];
-            pb = beta[(row0 + t0 + tid) * H + h];
-        }
+    // The decay is kept out of the registers: inside a stage the state is the product of the alphas so far times S, and a step
+    // adds k (u / product) -- one FFMA per element where alpha S + k u takes a multiply besides. The product is folded in at the
+    // end of the stage; a stage whose product falls below 1e-4 (u / product stays far inside the f32 range above it) folds in
+    // every step's alpha instead.
+    auto fold = [&](float by) {
+#pragma unroll
+        for (int p = 0; p < RPT / 2; ++p)
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) S[p][c] = make_pair(unpair(S[p][c]).x * by, unpair(S[p][c]).y * by);
     };
-    auto stash = [&](int buf) {
+    int mine = 0;   // the column of its group whose sums a lane ends up with
 #pragma unroll
-        for (int u = 0; u < KQ_PT; ++u) {
-            int idx = tid + u * FTHREADS;
-            int t = idx / (DH / 4), c4 = idx % (DH / 4);
-            if (idx < KQ4) {
-                *reinterpret_cast<float4*>(&k_s[buf][t][c4 * 4]) = pk[u];
-                *reinterpret_cast<float4*>(&q_s[buf][t][c4 * 4]) = pq[u];
+    for (int w = COLS / 2, bit = 1; w > 0; w >>= 1, bit <<= 1) mine = mine * 2 + (ag & bit ? 1 : 0);
+    auto write_state = [&](float* dst) {  // dst: dh x dh row-major
+#pragma unroll
+        for (int p = 0; p < RPT / 2; ++p)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float* at = dst + (row_of(p) + e) * DH + i0 + cg * COLS;
+                float x[COLS];
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) x[c] = e ? unpair(S[p][c]).y : unpair(S[p][c]).x;
+                if (COLS == 4) {
+                    *reinterpret_cast<float4*>(at) = make_float4(x[0], x[1 % COLS], x[2 % COLS], x[3 % COLS]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) at[c] = x[c];
+                }
             }
-        }
-#pragma unroll
-        for (int u = 0; u < (FTS * FW + FTHREADS - 1) / FTHREADS; ++u) {
-            int idx = tid + u * FTHREADS;
-            if (idx < FTS * FW) v_s[buf][idx / FW][idx % FW] = pv[u];
-        }
-        if (tid < FTS) {
-            a_s[buf][tid] = pa;
-            b_s[buf][tid] = pb;
-        }
     };
 
-    auto write_state = [&](float* dst) {  // dst: dh x dh row-major, this CTA's column slice
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) ck_s[row_of(r)][col] = S[r];
-        __syncthreads();
-        for (int idx = tid; idx < DH * FW; idx += FTHREADS) {
-            int a = idx / FW, c = idx % FW;
-            dst[a * DH + i0 + c] = ck_s[a][c];
+    int next_ck = ckpt ? 0 : Tlen;
+    __syncthreads();
+    for (int st = 0; st < n_stages; ++st) {
+        const int t0 = st * FTS, buf = st & 1, steps = Tlen - t0 < FTS ? Tlen - t0 : FTS;
+        if (t0 == next_ck) {
+            write_state(ckpt + ((int64_t)chain * n_chunks + t0 / chunk) * DH * DH);
+            next_ck += chunk;
         }
-        __syncthreads();
-    };
-
-    fetch(0);
-    int buf = 0;
-    for (int t0 = 0; t0 < Tlen; t0 += FTS, buf ^= 1) {
-        stash(buf);
-        __syncthreads();
-        if (t0 + FTS < Tlen) fetch(t0 + FTS);
-        const int steps = Tlen - t0 < FTS ? Tlen - t0 : FTS;
-        for (int ts = 0; ts < steps; ++ts) {
-            const int t = t0 + ts;
-            if (ckpt && (t % chunk) == 0)
-                write_state(ckpt + ((int64_t)chain * n_chunks + t / chunk) * DH * DH);
-            const float a = a_s[buf][ts], b = b_s[buf][ts];
-            float kk[RPT];
-            if (VEC) {
+        struct Row {
+            pair_t k[RPT / 2], q[RPT / 2];
+            float4 g;
+            float v;
+        };
+        auto read = [&](int ts, Row& x) {
+            x.g = g_s[buf][ts];
+            x.v = v_s[buf][ts][cg * COLS + mine];
 #pragma unroll
-                for (int g = 0; g < RPT / 4; ++g) {
-                    float4 t4 = *reinterpret_cast<const float4*>(&k_s[buf][ts][(g * FAG + ag) * 4]);
-                    kk[g * 4] = t4.x; kk[g * 4 + 1] = t4.y; kk[g * 4 + 2] = t4.z; kk[g * 4 + 3] = t4.w;
+            for (int r = 0; r < RPT / 4; ++r) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&k_s[buf][ts][(r * LANES + ag) * 4]),
+                                 b = *reinterpret_cast<const ulonglong2*>(&q_s[buf][ts][(r * LANES + ag) * 4]);
+                x.k[2 * r] = a.x; x.k[2 * r + 1] = a.y;
+                x.q[2 * r] = b.x; x.q[2 * r + 1] = b.y;
+            }
+        };
+        // dec: the decay folded in after this step, inv: its inverse, nab: -alpha beta times the decay before it
+        auto step = [&](int ts, const Row& x, float dec, float inv, float nab) {
+            float val[2 * COLS];   // (sk, sq) of each column
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                pair_t sk = 0, sq = 0;
+#pragma unroll
+                for (int p = 0; p < RPT / 2; ++p) {
+                    fma2(sk, S[p][c], x.k[p]);
+                    fma2(sq, S[p][c], x.q[p]);
                 }
-            } else {
-#pragma unroll
-                for (int r = 0; r < RPT; ++r) kk[r] = k_s[buf][ts][r * FAG + ag];
+                val[2 * c] = unpair(sk).x + unpair(sk).y;
+                val[2 * c + 1] = unpair(sq).x + unpair(sq).y;
             }
-            float p0 = 0.0f, p1 = 0.0f;
+            // exchange by halves: round i keeps the columns whose bit i matches the lane's
 #pragma unroll
-            for (int r = 0; r < RPT; r += 2) {
-                p0 = fmaf(S[r], kk[r], p0);
-                if (r + 1 < RPT) p1 = fmaf(S[r + 1], kk[r + 1], p1);
-            }
-            float sk = p0 + p1;
+            for (int w = COLS / 2, bit = 1; w > 0; w >>= 1, bit <<= 1) {
+                const bool up = ag & bit;
 #pragma unroll
-            for (int off = 1; off < FAG; off <<= 1) sk += __shfl_xor_sync(0xffffffffu, sk, off);
-            const float u = b * (v_s[buf][ts][col] - a * sk);
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) S[r] = fmaf(kk[r], u, a * S[r]);
-            if (VEC) {
-#pragma unroll
-                for (int g = 0; g < RPT / 4; ++g) {
-                    float4 t4 = *reinterpret_cast<const float4*>(&q_s[buf][ts][(g * FAG + ag) * 4]);
-                    kk[g * 4] = t4.x; kk[g * 4 + 1] = t4.y; kk[g * 4 + 2] = t4.z; kk[g * 4 + 3] = t4.w;
+                for (int j = 0; j < 2 * w; ++j) {
+                    const float send = up ? val[j] : val[2 * w + j], keep = up ? val[2 * w + j] : val[j];
+                    val[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
                 }
-            } else {
-#pragma unroll
-                for (int r = 0; r < RPT; ++r) kk[r] = q_s[buf][ts][r * FAG + ag];
             }
-            p0 = 0.0f; p1 = 0.0f;
 #pragma unroll
-            for (int r = 0; r < RPT; r += 2) {
-                p0 = fmaf(S[r], kk[r], p0);
-                if (r + 1 < RPT) p1 = fmaf(S[r + 1], kk[r + 1], p1);
+            for (int bit = COLS; bit < LANES; bit <<= 1) {
+                val[0] += __shfl_xor_sync(0xffffffffu, val[0], bit);
+                val[1] += __shfl_xor_sync(0xffffffffu, val[1], bit);
             }
-            float po = p0 + p1;
+            const float u = fmaf(nab, val[0], x.v), us = u * inv;
+            if (ag < COLS) o_s[buf][ts][cg * COLS + mine] = fmaf(dec, val[1], x.g.w * u);
 #pragma unroll
-            for (int off = 1; off < FAG; off <<= 1) po += __shfl_xor_sync(0xffffffffu, po, off);
-            if (ag == 0) o_s[ts][col] = po;
+            for (int c = 0; c < COLS; ++c) {
+                // the lane of the group that holds column c: its bits, most significant column bit first
+                const int src = COLS == 4 ? ((c >> 1) | ((c & 1) << 1)) : c;
+                const float uc = COLS == 1 ? us : __shfl_sync(0xffffffffu, us, ((tid & 31) & ~(LANES - 1)) | src);
+                const pair_t u2 = make_pair(uc, uc);
+#pragma unroll
+                for (int p = 0; p < RPT / 2; ++p) fma2(S[p][c], x.k[p], u2);
+            }
+        };
+        Row ra, rb;
+        read(0, ra);
+        if (steps == FTS && decay_s[buf] > 1e-4f && next_ck >= t0 + FTS) {
+            // a step's rows are read while the one before it is worked on
+#pragma unroll 1
+            for (int ts = 0; ts < FTS; ts += 2) {
+                read(ts + 1, rb);
+                step(ts, ra, ra.g.x, ra.g.y, ra.g.z);
+                read((ts + 2) % FTS, ra);   // (past the last step: a read of no use, but an unconditional one)
+                step(ts + 1, rb, rb.g.x, rb.g.y, rb.g.z);
+            }
+            fold(decay_s[buf]);
+        } else {   // ragged stages, checkpoints inside a stage, strong decay: folded in at every step
+#pragma unroll 1
+            for (int ts = 0; ts < steps; ++ts) {
+                if (t0 + ts == next_ck) {
+                    write_state(ckpt + ((int64_t)chain * n_chunks + (t0 + ts) / chunk) * DH * DH);
+                    next_ck += chunk;
+                }
+                read(ts, ra);
+                const float2 ab = ab_s[buf][ts];
+                fold(ab.x);   // (alpha S)^T k = alpha (S^T k): the decayed state takes the step with decay 1
+                step(ts, ra, 1.0f, 1.0f, -ab.y);
+            }
         }
         __syncthreads();
-        for (int idx = tid; idx < steps * FW; idx += FTHREADS) {
-            int ts = idx / FW, c = idx % FW;
-            o[(row0 + t0 + ts) * d + h * DH + i0 + c] = from_f32<T>(o_s[ts][c]);
-        }
-        // the next iteration's first barrier (after stash) orders these reads of o_s
-        // against the next stage's writes
     }
     if (s_final) write_state(s_final + (int64_t)chain * DH * DH);
 }
@@ -406,14 +518,25 @@ __global__ void __launch_bounds__(SW_WARPS * 32) delta_step_warp64_kernel(
     }
 }
 
-template <int DH, typename T>
-cudaError_t launch_fwd(cudaStream_t st, const void* q, const void* k, const void* v, const float* alpha,
-                       const float* beta, int B, int T_, int H, int chunk, void* o, const float* s_init,
-                       float* s_final, float* ckpt) {
-    dim3 grid(DH / FW, B * H);
-    delta_fwd_rec_kernel<DH, T><<<grid, FTHREADS, 0, st>>>((const T*)q, (const T*)k, (const T*)v, alpha, beta, B, T_, H,
-                                                           chunk, (T*)o, s_init, s_final, ckpt);
+template <int DH, int COLS, typename T>
+cudaError_t launch_fwd_cols(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta, int B,
+                            int T_, int H, int chunk, void* o, const float* s_init, float* s_final, float* ckpt) {
+    using C = RecCfg<DH, COLS>;
+    delta_fwd_rec_kernel<DH, COLS, T><<<dim3(DH / C::FW, B * H), C::NT + C::HT, 0, ctx->stream>>>(
+        (const T*)q, (const T*)k, (const T*)v, alpha, beta, B, T_, H, chunk, (T*)o, s_init, s_final, ckpt);
     return cudaGetLastError();
+}
+// Value columns per lane group: one while the chains leave the SMs idle (a step then takes its latency), more once the reads
+// of k and q fill shared memory. `load`: states of 128 x 128 per SM.
+template <int DH, typename T>
+cudaError_t launch_fwd(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta, int B, int T_,
+                       int H, int chunk, void* o, const float* s_init, float* s_final, float* ckpt) {
+    const double n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148, load = (double)B * H * DH * DH / (128 * 128) / n_sm;
+    if (DH >= 32 && load > 0.5)
+        return launch_fwd_cols<DH, DH >= 32 ? 4 : 1, T>(ctx, q, k, v, alpha, beta, B, T_, H, chunk, o, s_init, s_final, ckpt);
+    if (DH >= 32 && load > 0.25)
+        return launch_fwd_cols<DH, DH >= 32 ? 2 : 1, T>(ctx, q, k, v, alpha, beta, B, T_, H, chunk, o, s_init, s_final, ckpt);
+    return launch_fwd_cols<DH, 1, T>(ctx, q, k, v, alpha, beta, B, T_, H, chunk, o, s_init, s_final, ckpt);
 }
 
 }  // namespace
@@ -456,9 +579,9 @@ int asca_delta_fwd(asca_ctx* ctx, const void* q, const void* k, const void* v, c
     asca_span sp(ctx, "delta_fwd_rec_kernel");
 #define ASCA_FWD(DH_)                                                                                              \
     e = dtype == ASCA_BF16                                                                                         \
-            ? launch_fwd<DH_, __nv_bfloat16>(ctx->stream, q, k, v, alpha, beta, (int)B, (int)T, (int)H, ch, o, s_init, \
+            ? launch_fwd<DH_, __nv_bfloat16>(ctx, q, k, v, alpha, beta, (int)B, (int)T, (int)H, ch, o, s_init, \
                                              s_final, ckpt)                                                        \
-            : launch_fwd<DH_, float>(ctx->stream, q, k, v, alpha, beta, (int)B, (int)T, (int)H, ch, o, s_init,     \
+            : launch_fwd<DH_, float>(ctx, q, k, v, alpha, beta, (int)B, (int)T, (int)H, ch, o, s_init,     \
                                      s_final, ckpt)
     switch (dh) {
         case 16: ASCA_FWD(16); break;
