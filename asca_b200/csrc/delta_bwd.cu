@@ -145,6 +145,7 @@ __device__ __forceinline__ void cta_gemm(const float* __restrict__ A, int lda, c
             epi(KM_VEC ? tm * TM + i : tm + THR_M * i, (ALAY == L_MK && BLAY == L_NK) ? tn + THR_N * j : n0 + j, acc[i][j]);
 }
 
+// dst[t][c] = src[(row0 + t) ld + col0 + c] for t < n, zero for n <= t < C
 template <typename T>
 __device__ __forceinline__ void load_rows(const T* __restrict__ src, int64_t row0, int64_t ld, int col0, int n, int C,
                                           int W, float* __restrict__ dst, int ldd) {
@@ -571,6 +572,649 @@ __global__ void __launch_bounds__(BT, 1) delta_bwd_kernel(
     }
 }
 
+// ------------------------------------------------------------------ checkpoints every 64 tokens: three kernels
+// With one sub-chunk per checkpoint interval (C = chunk = 64) only dS itself runs from chunk to chunk, and by VALUE column
+// that recurrence splits without communication. So:
+//   pre    one CTA per (chain, chunk), all chunks at once:  A, LG = strictlower(Gam K K^T), T = (I + L)^-1 (16-wide diagonal
+//          blocks by substitution, then doubled twice by block products), D = beta T^T A^T dO, Hm = beta T^T diag(eg) K,
+//          Y = (gam Q)^T dO
+//   chain  one CTA per (chain, block of value columns), chunks in reverse:  dZ = D + Hm dS;  dS' = gam_last dS + Y - (gam K)^T dZ
+//   grad   one CTA per (chain, chunk), all chunks at once: everything else, from S0 (the checkpoint), dS and dZ
+// Two products a chunk are left on the serial path where the single kernel above has thirteen and the recomputation of inner
+// states; a launch of few chains (the small models, host calls) fills the GPU with its chunks. Work per token and head is about
+// 13 dh^2 multiply-adds against 21. Every dL and dA appears times beta or L, so nothing is divided by beta:
+//   beta dL = -strictlower(dZ U^T),  beta dbeta_t = dZ_t.Z_t - sum_i (dZ U^T)[t,i] LG[t,i]
+// Bound: shared-memory return bandwidth of the 8 x 4 thread tiles (0.375 loads per FFMA), one CTA per SM at dh 128.
+constexpr int CC = 64;   // tokens per chunk
+constexpr int LX = CC + 4;
+
+// dst[t][c] = src[(row0 + t) ld + col0 + c] for t < n, zero for n <= t < ROWS: asynchronous copies (f32), or every load of the
+// tile in flight before the first store (bf16). tile_wait() makes all tiles asked for so far visible to the CTA.
+template <typename T, int ROWS, int W>
+__device__ __forceinline__ void load_tile(const T* __restrict__ src, int64_t row0, int64_t ld, int col0, int n, float* __restrict__ dst, int ldd) {
+    constexpr int Q = W / 4, IT = (ROWS * Q + BT - 1) / BT;
+    src += row0 * ld + col0;
+    if (sizeof(T) == 4) {
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int idx = threadIdx.x + i * BT, t = idx / Q, c = idx % Q * 4;
+            if (ROWS * Q % BT == 0 || idx < ROWS * Q)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + t * ldd + c)),
+                             "l"(src + (t < n ? t : 0) * ld + c), "r"(t < n ? 16 : 0) : "memory");
+        }
+    } else {
+        uint2 v[IT];
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int idx = threadIdx.x + i * BT, t = idx / Q, c = idx % Q * 4;
+            v[i] = t < n && idx < ROWS * Q ? *reinterpret_cast<const uint2*>(src + t * ld + c) : make_uint2(0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int idx = threadIdx.x + i * BT, t = idx / Q, c = idx % Q * 4;
+            const __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162*>(&v[i].x), b = *reinterpret_cast<__nv_bfloat162*>(&v[i].y);
+            if (idx < ROWS * Q)
+                *reinterpret_cast<float4*>(dst + t * ldd + c) = make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+        }
+    }
+}
+__device__ __forceinline__ void tile_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+}
+// asks for `rows` runs of `bytes` (a multiple of 128 when above it), `pitch` bytes apart, in L2
+__device__ __forceinline__ void prefetch_l2(const void* p, int rows, int bytes, int64_t pitch) {
+    const int lines = (bytes + 127) / 128;
+    for (int i = threadIdx.x; i < rows * lines; i += BT)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p) + i / lines * pitch + i % lines * 128));
+}
+
+// acc += A B for an M x N output in BT threads' registers, K deep, operands in shared memory (row pitches multiples of 4).
+// Thread (tm, tn) owns columns tn + THR_N j and rows in groups of four (tm + THR_M i where it has fewer than four).
+template <int M, int N>
+struct MM {
+    static constexpr int TN = 4, THR_N = N / TN, THR_M = BT / THR_N < M ? BT / THR_N : M, TM = M / THR_M;
+    static constexpr bool R4 = TM % 4 == 0;
+    static_assert(N % 4 == 0 && BT % THR_N == 0 && M % THR_M == 0, "tile shape");
+    float acc[TM][TN];
+    int tn, tm;
+    bool on;
+    __device__ __forceinline__ MM() {
+        tn = threadIdx.x % THR_N;
+        tm = threadIdx.x / THR_N;
+        on = tm < THR_M;
+        clear();
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+    }
+    __device__ __forceinline__ int row(int i) const { return R4 ? (i >> 2) * (4 * THR_M) + tm * 4 + (i & 3) : tm + THR_M * i; }
+    __device__ __forceinline__ int col(int j) const { return tn + THR_N * j; }
+    template <int K, int ALAY, int BLAY>
+    __device__ __forceinline__ void mul(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb) {
+        if (!on) return;
+#pragma unroll (TM > 8 ? 1 : TM > 4 ? 2 : TM > 2 ? 4 : 8)
+        for (int k = 0; k < K; k += 4) {
+            float b[4][TN];   // [k][column]
+            if (BLAY == L_NK) {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    const float4 v = *reinterpret_cast<const float4*>(B + col(j) * ldb + k);
+                    b[0][j] = v.x; b[1][j] = v.y; b[2][j] = v.z; b[3][j] = v.w;
+                }
+            } else {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) b[kk][j] = B[(k + kk) * ldb + col(j)];
+            }
+            if (ALAY == L_MK) {
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const float4 a = *reinterpret_cast<const float4*>(A + row(i) * lda + k);
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        acc[i][j] = fmaf(a.x, b[0][j], acc[i][j]);
+                        acc[i][j] = fmaf(a.y, b[1][j], acc[i][j]);
+                        acc[i][j] = fmaf(a.z, b[2][j], acc[i][j]);
+                        acc[i][j] = fmaf(a.w, b[3][j], acc[i][j]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    float a[TM];
+                    if (R4) {
+#pragma unroll
+                        for (int i = 0; i < TM; i += 4) {
+                            const float4 v = *reinterpret_cast<const float4*>(A + (k + kk) * lda + row(i));
+                            a[i] = v.x; a[(i + 1) % TM] = v.y; a[(i + 2) % TM] = v.z; a[(i + 3) % TM] = v.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < TM; ++i) a[i] = A[(k + kk) * lda + row(i)];
+                    }
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[kk][j], acc[i][j]);
+                }
+            }
+        }
+    }
+    // f(row, column, value) of every element of this thread
+    template <class F>
+    __device__ __forceinline__ void each(F f) {
+        if (!on) return;
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) f(row(i), col(j), acc[i][j]);
+    }
+    // the sum over a row's columns of f(row, column, value), in every lane that shares the row (THR_N neighbouring lanes)
+    template <class F>
+    __device__ __forceinline__ float row_sum(int i, F f) {
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) s += f(row(i), col(j), acc[i][j]);
+#pragma unroll
+        for (int m = THR_N / 2; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+        return s;
+    }
+};
+
+// Gates of a chunk of n live steps (alpha 1, beta 0 behind them): cumulative log alpha g, gam = exp(g), eg = exp(g_last - g).
+struct ChunkGates {
+    float g[CC], gam[CC], eg[CC], be[CC], al[CC];
+};
+__device__ __forceinline__ void load_gates(const float* alpha, const float* beta, int64_t row0, int n, int H, int h, ChunkGates& s) {
+    const int t = threadIdx.x;
+    if (t < CC) {
+        s.al[t] = t < n ? alpha[(row0 + t) * H + h] : 1.0f;
+        s.be[t] = t < n ? beta[(row0 + t) * H + h] : 0.0f;
+    }
+    __syncthreads();
+    if (t < 32) {   // two steps a lane, left to right
+        const float a = logf(s.al[2 * t]), b = logf(s.al[2 * t + 1]);
+        float x = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float y = __shfl_up_sync(0xffffffffu, x, o);
+            if (t >= o) x += y;
+        }
+        const float before = __shfl_up_sync(0xffffffffu, x, 1);
+        s.g[2 * t] = (t ? before : 0.0f) + a;
+        s.g[2 * t + 1] = x;
+    }
+    __syncthreads();
+    if (t < CC) {
+        s.gam[t] = expf(s.g[t]);
+        s.eg[t] = expf(s.g[CC - 1] - s.g[t]);
+    }
+    __syncthreads();
+}
+
+// Per (chain, chunk) scratch, in floats: A, LG, T (CC x CC each), D -> dZ and Hm (CC x DH), Y -> dS at the chunk's end (DH x DH),
+// gam (CC)
+template <int DH>
+struct ChunkScratch {
+    static constexpr int64_t A = 0, LG = CC * CC, T = 2 * CC * CC, D = 3 * CC * CC, HM = D + CC * DH, Y = HM + CC * DH, GAM = Y + DH * DH, SIZE = GAM + CC;
+};
+
+template <int DH, typename T>
+struct PreSmem {
+    static constexpr int LD = DH + 4;
+    static constexpr size_t bytes = (size_t)(4 * CC * LD + 3 * CC * LX) * 4 + sizeof(ChunkGates);
+};
+
+template <int DH, typename T>
+__global__ void __launch_bounds__(BT) delta_bwd_pre_kernel(const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ alpha,
+                                                           const float* __restrict__ beta, const T* __restrict__ d_o,
+                                                           float* __restrict__ scratch, int Tlen, int H, int n_ck) {
+    using SC = ChunkScratch<DH>;
+    constexpr int LD = DH + 4;
+    extern __shared__ __align__(16) float smem[];
+    float *Ks = smem, *Qs = Ks + CC * LD, *Os = Qs + CC * LD, *Xs = Os + CC * LD, *Ls = Xs + CC * LD, *Ts = Ls + CC * LX, *As = Ts + CC * LX;
+    ChunkGates& gt = *reinterpret_cast<ChunkGates*>(As + CC * LX);
+    const int tid = threadIdx.x, ck = blockIdx.x, chain = blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
+    const int n = min(CC, Tlen - ck * CC);
+    const int64_t row0 = (int64_t)bi * Tlen + ck * CC;
+    float* out = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+    load_tile<T, CC, DH>(k, row0, d, h * DH, n, Ks, LD);
+    load_tile<T, CC, DH>(q, row0, d, h * DH, n, Qs, LD);
+    load_tile<T, CC, DH>(d_o, row0, d, h * DH, n, Os, LD);
+    load_gates(alpha, beta, row0, n, H, h, gt);
+    if (tid < CC) out[SC::GAM + tid] = gt.gam[tid];
+    tile_wait();
+    {
+        MM<CC, CC> kk, qk;
+        kk.template mul<DH, L_MK, L_NK>(Ks, LD, Ks, LD);
+        kk.each([&](int t, int i, float v) {
+            const float lg = i < t ? expf(gt.g[t] - gt.g[i]) * v : 0.0f;
+            out[SC::LG + t * CC + i] = lg;
+            Ls[t * LX + i] = gt.be[t] * lg;
+            Ts[t * LX + i] = t == i ? 1.0f : 0.0f;
+        });
+        qk.template mul<DH, L_MK, L_NK>(Qs, LD, Ks, LD);
+        qk.each([&](int t, int i, float v) {
+            const float a = i <= t ? expf(gt.g[t] - gt.g[i]) * v : 0.0f;
+            out[SC::A + t * CC + i] = a;
+            As[t * LX + i] = a;
+        });
+    }
+    __syncthreads();
+    // T: the four 16 x 16 diagonal blocks, a thread per column
+    if (tid < CC) {
+        const int b0 = tid & ~15, c = tid & 15;
+        float x[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            float v[4] = {t == c ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};   // (four partial sums: the chain is the rows', not the terms')
+#pragma unroll
+            for (int i = 0; i < t; i += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(Ls + (b0 + t) * LX + b0 + i);   // zeros from the diagonal on
+                v[0] = fmaf(-l.x, x[i], v[0]);
+                if (i + 1 < t) v[1] = fmaf(-l.y, x[i + 1], v[1]);
+                if (i + 2 < t) v[2] = fmaf(-l.z, x[i + 2], v[2]);
+                if (i + 3 < t) v[3] = fmaf(-l.w, x[i + 3], v[3]);
+            }
+            x[t] = (v[0] + v[1]) + (v[2] + v[3]);
+            Ts[(b0 + t) * LX + b0 + c] = x[t];
+        }
+    }
+    __syncthreads();
+    // ... doubled: T21 = -T2 (L21 T1), the inner product in the not yet needed X area; a thread takes four columns of a row
+#pragma unroll
+    for (int w = 16; w < CC; w *= 2) {
+        const int at = tid * 4, b = at / (w * w) * 2 * w, t = at / w % w, c = at % w;
+        const bool on = at < CC / 2 * w;   // (CC / 2w blocks of w x w)
+        auto product = [&](const float* A, const float* B, int ldb) {   // row of A times w rows of B
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+            for (int i = 0; i < w; ++i) {
+                const float a = A[i];
+                const float4 x = *reinterpret_cast<const float4*>(B + i * ldb);
+                v.x = fmaf(a, x.x, v.x); v.y = fmaf(a, x.y, v.y); v.z = fmaf(a, x.z, v.z); v.w = fmaf(a, x.w, v.w);
+            }
+            return v;
+        };
+        if (on) *reinterpret_cast<float4*>(Xs + at) = product(Ls + (b + w + t) * LX + b, Ts + b * LX + b + c, LX);
+        __syncthreads();
+        if (on) {
+            const float4 v = product(Ts + (b + w + t) * LX + b + w, Xs + at - t * w, w);
+            *reinterpret_cast<float4*>(Ts + (b + w + t) * LX + b + c) = make_float4(-v.x, -v.y, -v.z, -v.w);
+        }
+        __syncthreads();
+    }
+    for (int idx = tid; idx < CC * CC / 4; idx += BT)
+        *reinterpret_cast<float4*>(out + SC::T + idx * 4) = *reinterpret_cast<const float4*>(Ts + idx / (CC / 4) * LX + idx % (CC / 4) * 4);
+    MM<CC, DH> m;
+    m.template mul<CC, L_KM, L_KN>(As, LX, Os, LD);   // A^T dO
+    m.each([&](int t, int c, float v) { Xs[t * LD + c] = v; });
+    __syncthreads();
+    m.clear();
+    m.template mul<CC, L_KM, L_KN>(Ts, LX, Xs, LD);   // D
+    m.each([&](int t, int c, float v) { out[SC::D + t * DH + c] = gt.be[t] * v; });
+    __syncthreads();
+    for (int idx = tid; idx < CC * DH; idx += BT) {
+        const int t = idx / DH, c = idx % DH;
+        Xs[t * LD + c] = gt.eg[t] * Ks[t * LD + c];
+        Qs[t * LD + c] *= gt.gam[t];
+    }
+    __syncthreads();
+    m.clear();
+    m.template mul<CC, L_KM, L_KN>(Ts, LX, Xs, LD);   // Hm
+    m.each([&](int t, int c, float v) { out[SC::HM + t * DH + c] = gt.be[t] * v; });
+    MM<DH, DH> y;
+    y.template mul<CC, L_KM, L_KN>(Qs, LD, Os, LD);
+    y.each([&](int a, int c, float v) { out[SC::Y + a * DH + c] = v; });
+}
+
+// Where the tiles are small the next chunk's are copied while this one is worked on (two buffers, D and Y in registers);
+// elsewhere they are only asked for in L2.
+template <int DH, int W>
+struct ChainSmem {
+    static constexpr bool AHEAD = DH * W <= 64 * 64;
+    static constexpr int LD = DH + 4, LW = W + 4, STAGE = 2 * CC * LD + CC;   // Hm, K, gam
+    static constexpr size_t bytes = (size_t)((AHEAD ? 2 : 1) * STAGE + DH * LW + CC * LW) * 4;
+};
+
+template <int DH, int W, typename T>
+__global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict__ k, float* __restrict__ scratch, int Tlen, int H, int n_ck) {
+    using SC = ChunkScratch<DH>;
+    using SM = ChainSmem<DH, W>;
+    constexpr int LD = SM::LD, LW = SM::LW;
+    constexpr bool AHEAD = SM::AHEAD;
+    extern __shared__ __align__(16) float smem[];
+    float *dS = smem + (AHEAD ? 2 : 1) * SM::STAGE, *dZ = dS + DH * LW;
+    const int tid = threadIdx.x, c0 = blockIdx.x * W, chain = blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
+    for (int i = tid; i < DH * LW; i += BT) dS[i] = 0.0f;
+    MM<DH, W> s_in;   // Y and D of the chunk to come
+    MM<CC, W> z_in;
+    auto request = [&](int ck, float* st) {
+        float* at = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+        load_tile<float, CC, DH>(at + SC::HM, 0, DH, 0, CC, st, LD);
+        load_tile<T, CC, DH>(k, (int64_t)bi * Tlen + ck * CC, d, h * DH, min(CC, Tlen - ck * CC), st + CC * LD, LD);
+        if (tid < CC / 4)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(st + 2 * CC * LD + tid * 4)),
+                         "l"(at + SC::GAM + tid * 4) : "memory");
+        s_in.each([&](int a, int c, float& v) { v = at[SC::Y + a * DH + c0 + c]; });
+        z_in.each([&](int t, int c, float& v) { v = at[SC::D + t * DH + c0 + c]; });
+    };
+    if (AHEAD) request(n_ck - 1, smem + ((n_ck - 1) & 1) * SM::STAGE);
+    for (int ck = n_ck - 1; ck >= 0; --ck) {
+        float* at = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+        float* Hs = smem + (AHEAD ? (ck & 1) * SM::STAGE : 0);
+        const float *Ks = Hs + CC * LD, *gam = Hs + 2 * CC * LD;
+        if (!AHEAD) request(ck, Hs);
+        if (!AHEAD && ck > 0) {
+            prefetch_l2(at - SC::SIZE + SC::HM, 1, CC * DH * 4, 0);
+            prefetch_l2(at - SC::SIZE + SC::D + c0, CC, W * 4, DH * 4);
+            prefetch_l2(at - SC::SIZE + SC::Y + c0, DH, W * 4, DH * 4);
+            prefetch_l2(k + ((int64_t)bi * Tlen + (ck - 1) * CC) * d + h * DH, CC, DH * (int)sizeof(T), (int64_t)d * sizeof(T));
+        }
+        tile_wait();
+        MM<DH, W> s = s_in;
+        MM<CC, W> z = z_in;
+        if (AHEAD && ck > 0) request(ck - 1, smem + ((ck - 1) & 1) * SM::STAGE);
+        s.each([&](int a, int c, float) { at[SC::Y + a * DH + c0 + c] = dS[a * LW + c]; });   // dS at the end of this chunk
+        z.template mul<DH, L_MK, L_KN>(Hs, LD, dS, LW);
+        z.each([&](int t, int c, float v) {
+            at[SC::D + t * DH + c0 + c] = v;
+            dZ[t * LW + c] = -gam[t] * v;
+        });
+        if (ck == 0) break;   // (dS before the first token is nobody's)
+        __syncthreads();
+        const float gl = gam[CC - 1];
+        s.each([&](int a, int c, float& v) { v = fmaf(gl, dS[a * LW + c], v); });
+        s.template mul<CC, L_KM, L_KN>(Ks, LD, dZ, LW);
+        __syncthreads();
+        s.each([&](int a, int c, float v) { dS[a * LW + c] = v; });
+        if (!AHEAD) __syncthreads();   // (with two buffers the next tile_wait is the barrier)
+    }
+}
+
+template <int DH>
+struct GradSmem {
+    static constexpr int LD = DH + 4;
+    static constexpr size_t bytes = (size_t)(4 * CC * LD + DH * LD + CC * LX + 8 * CC + 8 * CC + 64) * 4 + sizeof(ChunkGates);
+};
+
+template <int DH, typename T>
+__global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
+    const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ alpha,
+    const float* __restrict__ beta, const float* __restrict__ qnorm, const float* __restrict__ knorm, const T* __restrict__ d_o,
+    const float* __restrict__ ckpt, const float* __restrict__ scratch, int Tlen, int H, int n_ck, float* __restrict__ d_qkv,
+    float* __restrict__ d_gate) {
+    using SC = ChunkScratch<DH>;
+    constexpr int LD = DH + 4;
+    extern __shared__ __align__(16) float smem[];
+    float *Ks = smem, *Bs = Ks + CC * LD /* V, Z, then dO, then Q */, *Us = Bs + CC * LD, *Zs = Us + CC * LD /* dZ */, *Ss = Zs + CC * LD /* S0, then dS */,
+          *Xs = Ss + DH * LD /* T, then dA Gam, then M + M^T */, *col_part = Xs + CC * LX, *vec = col_part + 8 * CC, *red = vec + 8 * CC;
+    float *row_p = vec, *col_p = vec + CC, *r_qs = vec + 2 * CC, *r_kg = vec + 3 * CC, *r_kw = vec + 4 * CC, *dbe = vec + 5 * CC;
+    ChunkGates& gt = *reinterpret_cast<ChunkGates*>(red + 64);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ck = blockIdx.x, chain = blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
+    const int n = min(CC, Tlen - ck * CC);
+    const int64_t row0 = (int64_t)bi * Tlen + ck * CC;
+    const float* in = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+    const float* S0 = ckpt + ((int64_t)chain * n_ck + ck) * DH * DH;
+    load_tile<T, CC, DH>(k, row0, d, h * DH, n, Ks, LD);
+    load_tile<float, DH, DH>(S0, 0, DH, 0, DH, Ss, LD);
+    load_tile<T, CC, DH>(v, row0, d, h * DH, n, Bs, LD);
+    load_tile<float, CC, DH>(in + SC::D, 0, DH, 0, CC, Zs, LD);
+    load_tile<float, CC, CC>(in + SC::T, 0, CC, 0, CC, Xs, LX);
+    // what comes into these buffers later is on its way to L2
+    prefetch_l2(in + SC::A, 1, 2 * CC * CC * 4, 0);
+    prefetch_l2(in + SC::Y, 1, DH * DH * 4, 0);
+    prefetch_l2(d_o + row0 * d + h * DH, n, DH * (int)sizeof(T), (int64_t)d * sizeof(T));
+    prefetch_l2(q + row0 * d + h * DH, n, DH * (int)sizeof(T), (int64_t)d * sizeof(T));
+    load_gates(alpha, beta, row0, n, H, h, gt);
+    tile_wait();
+    using MD = MM<CC, DH>;
+    {   // Z = V - gam K S0 (beta Z is what U wants), dZ.Z; dV = dZ goes out
+        MD m;
+        m.template mul<DH, L_MK, L_KN>(Ks, LD, Ss, LD);
+#pragma unroll
+        for (int i = 0; i < MD::TM; ++i) {
+            const int t = m.row(i);
+            const float s = m.row_sum(i, [&](int tt, int c, float& x) {
+                const float z = Bs[tt * LD + c] - gt.gam[tt] * x, dz = Zs[tt * LD + c];
+                Bs[tt * LD + c] = gt.be[tt] * z;
+                if (tt < n) d_qkv[(row0 + tt) * 3 * d + 2 * d + h * DH + c] = dz;
+                return z * dz;
+            });
+            if (m.tn == 0) dbe[t] = s;
+        }
+    }
+    __syncthreads();
+    {   // U = T beta Z
+        MD m;
+        m.template mul<CC, L_MK, L_KN>(Xs, LX, Bs, LD);
+        m.each([&](int t, int c, float x) { Us[t * LD + c] = x; });
+    }
+    __syncthreads();
+    load_tile<T, CC, DH>(d_o, row0, d, h * DH, n, Bs, LD);
+    tile_wait();
+    // a C x C matrix of products P = e(acc) o other: row sums and column sums in a fixed order
+    auto sums = [&](auto& m, auto f, bool first) {
+        using MX = MM<CC, CC>;
+        float cp[MX::TN] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < MX::TM; ++i) {
+            float p[MX::TN], s = 0.0f;
+#pragma unroll
+            for (int j = 0; j < MX::TN; ++j) {
+                p[j] = f(m.row(i), m.col(j), m.acc[i][j]);
+                cp[j] += p[j];
+                s += p[j];
+            }
+#pragma unroll
+            for (int o = MX::THR_N / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (m.tn == 0) {
+                if (first) row_p[m.row(i)] = s;
+                else {
+                    row_p[m.row(i)] += s;
+                    dbe[m.row(i)] += s;   // (the second matrix is beta dL o L: it belongs to dbeta as well)
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < MX::TN; ++j) {
+            cp[j] += __shfl_xor_sync(0xffffffffu, cp[j], 16);   // the warp's two row groups
+            if (lane < 16) col_part[warp * CC + m.col(j)] = cp[j];
+        }
+        __syncthreads();
+        if (tid < CC) {
+            float s = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) s += col_part[w * CC + tid];
+            col_p[tid] = first ? s : col_p[tid] + s;
+        }
+    };
+    {   // dA Gam
+        MM<CC, CC> m;
+        m.template mul<DH, L_MK, L_NK>(Bs, LD, Us, LD);
+        sums(m, [&](int t, int i, float x) {
+            Xs[t * LX + i] = i <= t ? expf(gt.g[t] - gt.g[i]) * x : 0.0f;
+            return i <= t ? x * in[SC::A + t * CC + i] : 0.0f;
+        }, true);
+    }
+    {   // dQ = gam dO S0^T + (dA Gam) K, L2-norm backward, out
+        MD m;
+        m.template mul<DH, L_MK, L_NK>(Bs, LD, Ss, LD);
+        float qv[MD::TM][MD::TN];
+#pragma unroll
+        for (int i = 0; i < MD::TM; ++i) {
+            const int t = m.row(i);
+            const float s = m.row_sum(i, [&](int tt, int c, float& x) {
+                x *= gt.gam[tt];
+                return x * (qv[i][(c - m.tn) / MD::THR_N] = tt < n ? to_f32<T>(q[(row0 + tt) * d + h * DH + c]) : 0.0f);
+            });
+            if (m.tn == 0) r_qs[t] = s;
+        }
+        __syncthreads();   // dA Gam is in place
+        m.template mul<CC, L_MK, L_KN>(Xs, LX, Ks, LD);
+#pragma unroll
+        for (int i = 0; i < MD::TM; ++i) {
+            const int t = m.row(i);
+            const float s = m.row_sum(i, [&](int, int c, float x) { return x * qv[i][(c - m.tn) / MD::THR_N]; });
+            if (t < n) {
+                const float nq = qnorm[(row0 + t) * H + h];
+#pragma unroll
+                for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + h * DH + m.col(j)] = (m.acc[i][j] - qv[i][j] * s) / nq;
+            }
+        }
+    }
+    MD dk;   // dK = -gam dZ S0^T + eg U dS^T + (dA Gam)^T Q + (M + M^T) K
+    dk.template mul<DH, L_MK, L_NK>(Zs, LD, Ss, LD);
+#pragma unroll
+    for (int i = 0; i < MD::TM; ++i) {
+        const int t = dk.row(i);
+        const float s = dk.row_sum(i, [&](int tt, int c, float& x) {
+            x *= -gt.gam[tt];
+            return x * Ks[tt * LD + c];
+        });
+        if (dk.tn == 0) r_kg[t] = s;
+    }
+    __syncthreads();   // S0 and dO are done with
+    load_tile<T, CC, DH>(q, row0, d, h * DH, n, Bs, LD);
+    float part = 0.0f;   // <S0, dS>
+    {
+        constexpr int IT = (DH * DH / 4 + BT - 1) / BT, BATCH = IT < 8 ? IT : 8;
+#pragma unroll
+        for (int i0 = 0; i0 < IT; i0 += BATCH) {
+            float4 b[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int idx = tid + (i0 + i) * BT;
+                b[i] = idx < DH * DH / 4 ? *reinterpret_cast<const float4*>(in + SC::Y + idx * 4) : make_float4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int idx = tid + (i0 + i) * BT;
+                if (idx >= DH * DH / 4) continue;
+                float4* at = reinterpret_cast<float4*>(Ss + idx / (DH / 4) * LD + idx % (DH / 4) * 4);
+                const float4 a = *at;
+                part = fmaf(a.x, b[i].x, part); part = fmaf(a.y, b[i].y, part); part = fmaf(a.z, b[i].z, part); part = fmaf(a.w, b[i].w, part);
+                *at = b[i];
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const float sds = block_sum(part, red);   // (holds barriers: dS and Q are in place)
+    {
+        MD m;
+        m.template mul<DH, L_MK, L_NK>(Us, LD, Ss, LD);
+#pragma unroll
+        for (int i = 0; i < MD::TM; ++i) {
+            const int t = m.row(i);
+            const float s = m.row_sum(i, [&](int tt, int c, float& x) {
+                x *= gt.eg[tt];
+                return x * Ks[tt * LD + c];
+            });
+            if (m.tn == 0) r_kw[t] = s;
+#pragma unroll
+            for (int j = 0; j < MD::TN; ++j) dk.acc[i][j] += m.acc[i][j];
+        }
+    }
+    dk.template mul<CC, L_KM, L_KN>(Xs, LX, Bs, LD);
+    {
+        MM<CC, CC> m;   // dZ U^T
+        m.template mul<DH, L_MK, L_NK>(Zs, LD, Us, LD);
+        __syncthreads();   // every reader of dA Gam is done
+        m.each([&](int t, int i, float x) {
+            if (i <= t) Xs[t * LX + i] = i < t ? -expf(gt.g[t] - gt.g[i]) * x : 0.0f;   // M
+        });
+        sums(m, [&](int t, int i, float x) { return i < t ? -x * in[SC::LG + t * CC + i] : 0.0f; }, false);   // (holds a barrier)
+    }
+    for (int idx = tid; idx < CC * CC; idx += BT) {   // M + M^T: the upper triangle is the mirror of the lower
+        const int t = idx / CC, i = idx % CC;
+        if (i > t) Xs[t * LX + i] = Xs[i * LX + t];
+    }
+    __syncthreads();
+    dk.template mul<CC, L_MK, L_KN>(Xs, LX, Ks, LD);
+#pragma unroll
+    for (int i = 0; i < MD::TM; ++i) {
+        const int t = dk.row(i);
+        const float s = dk.row_sum(i, [&](int tt, int c, float x) { return x * Ks[tt * LD + c]; });
+        if (t < n) {
+            const float nk = knorm[(row0 + t) * H + h];
+#pragma unroll
+            for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + d + h * DH + dk.col(j)] = (dk.acc[i][j] - Ks[t * LD + dk.col(j)] * s) / nk;
+        }
+    }
+    // gates: dg, its suffix sums (two steps a lane), sigmoid backward
+    if (warp == 0) {
+        auto dg = [&](int t) { return row_p[t] - col_p[t] + r_qs[t] + r_kg[t] - r_kw[t]; };
+        const float kw = warp_sum(r_kw[2 * lane] + r_kw[2 * lane + 1]);
+        const float a = dg(2 * lane);
+        float b = dg(2 * lane + 1);
+        if (lane == 31) b += gt.gam[CC - 1] * sds + kw;
+        float x = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float y = __shfl_down_sync(0xffffffffu, x, o);
+            if (lane + o < 32) x += y;
+        }
+        const float behind = __shfl_down_sync(0xffffffffu, x, 1);
+        if (lane < 31) b += behind;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = 2 * lane + e;
+            if (t < n) {
+                d_gate[(row0 + t) * 2 * H + h] = (e ? b : x) * (1.0f - gt.al[t]);   // (dlogalpha / alpha) alpha (1 - alpha)
+                d_gate[(row0 + t) * 2 * H + H + h] = dbe[t] * (1.0f - gt.be[t]);
+            }
+        }
+    }
+}
+
+template <int DH, int W, typename T>
+int launch_chain(asca_ctx* ctx, const void* k, float* ws, int B, int Tlen, int H, int n_ck) {
+    auto kern = delta_bwd_chain_kernel<DH, W, T>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChainSmem<DH, W>::bytes));
+    kern<<<dim3(DH / W, B * H), BT, ChainSmem<DH, W>::bytes, ctx->stream>>>((const T*)k, ws, Tlen, H, n_ck);
+    ASCA_CHECK_LAUNCH(ctx);
+    return ASCA_OK;
+}
+
+template <int DH, typename T>
+int launch_bwd64(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta, const float* qnorm,
+                 const float* knorm, const void* d_o, const float* ckpt, int B, int Tlen, int H, float* d_qkv, float* d_gate) {
+    const int n_ck = (Tlen + CC - 1) / CC;
+    void* p;
+    ASCA_TRY(asca_workspace(ctx, (size_t)B * H * n_ck * ChunkScratch<DH>::SIZE * 4 + 256, &p));
+    float* ws = (float*)p;
+    static_assert(PreSmem<DH, T>::bytes <= 227 * 1024 && GradSmem<DH>::bytes <= 227 * 1024, "shared memory budget");
+    auto pre = delta_bwd_pre_kernel<DH, T>;
+    auto grad = delta_bwd_grad_kernel<DH, T>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PreSmem<DH, T>::bytes));
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradSmem<DH>::bytes));
+    {
+        asca_span sp(ctx, "delta_bwd_pre_kernel");
+        pre<<<dim3(n_ck, B * H), BT, PreSmem<DH, T>::bytes, ctx->stream>>>((const T*)q, (const T*)k, alpha, beta, (const T*)d_o, ws, Tlen, H, n_ck);
+        ASCA_CHECK_LAUNCH(ctx);
+    }
+    {   // value columns per CTA: as many as leave every SM a CTA, since wider tiles read less shared memory per FFMA
+        asca_span sp(ctx, "delta_bwd_chain_kernel");
+        const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
+        int w = DH;
+        while (w > 16 && B * H * (DH / w) * 2 <= n_sm) w /= 2;
+        if (w == 128) ASCA_TRY((launch_chain<DH, DH < 128 ? DH : 128, T>(ctx, k, ws, B, Tlen, H, n_ck)));
+        else if (w == 64) ASCA_TRY((launch_chain<DH, DH < 64 ? DH : 64, T>(ctx, k, ws, B, Tlen, H, n_ck)));
+        else if (w == 32) ASCA_TRY((launch_chain<DH, DH < 32 ? DH : 32, T>(ctx, k, ws, B, Tlen, H, n_ck)));
+        else ASCA_TRY((launch_chain<DH, 16, T>(ctx, k, ws, B, Tlen, H, n_ck)));
+    }
+    asca_span sp(ctx, "delta_bwd_grad_kernel");
+    grad<<<dim3(n_ck, B * H), BT, GradSmem<DH>::bytes, ctx->stream>>>((const T*)q, (const T*)k, (const T*)v, alpha, beta, qnorm, knorm, (const T*)d_o,
+                                                                      ckpt, ws, Tlen, H, n_ck, d_qkv, d_gate);
+    ASCA_CHECK_LAUNCH(ctx);
+    return ASCA_OK;
+}
+
 template <int DH, int C, typename T>
 int launch_bwd(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
                const float* qnorm, const float* knorm, const void* d_o, const float* ckpt, int B, int Tlen, int H,
@@ -608,6 +1252,19 @@ extern "C" int asca_delta_bwd(asca_ctx* ctx, const void* q, const void* k, const
     // bf16 mode, dh = 128, checkpoints every 64 tokens: reverse chunked scan on the tensor cores
     if (dtype == ASCA_BF16 && (dh == 128 || dh == 64) && chunk == 64 && asca_tc_enabled() && delta_tc::available())
         return delta_tc::backward(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, B, T, H, dh, d_qkv, d_gate);
+    if (chunk == CC && B * H < 65536) {
+#define ASCA_BWD64(DH_)                                                                                                          \
+    return dtype == ASCA_BF16 ? launch_bwd64<DH_, __nv_bfloat16>(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, (int)B, (int)T, (int)H, \
+                                                                 d_qkv, d_gate)                                                  \
+                              : launch_bwd64<DH_, float>(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, (int)B, (int)T, (int)H, d_qkv, d_gate)
+        switch (dh) {
+            case 16: ASCA_BWD64(16);
+            case 32: ASCA_BWD64(32);
+            case 64: ASCA_BWD64(64);
+            default: ASCA_BWD64(128);
+        }
+#undef ASCA_BWD64
+    }
 #define ASCA_BWD(DH_, C_)                                                                                             \
     return dtype == ASCA_BF16                                                                                         \
                ? launch_bwd<DH_, C_, __nv_bfloat16>(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, (int)B, (int)T, \
