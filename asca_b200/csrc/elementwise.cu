@@ -1,5 +1,5 @@
 // HBM-bound row / element kernels: RMSNorm forward and backward, residual+norm fusion,
-// row gather / scatter, AdamW, and the q/k/v split + L2-normalise + gate prologue.
+// row gather / scatter, AdamW.
 // Every reduction is a fixed tree (no float atomics), so results are run-to-run identical.
 #include "common.cuh"
 
@@ -309,56 +309,17 @@ __global__ void __launch_bounds__(256) adamw_seg_kernel(float* __restrict__ p, c
                                                         float b2, float wd, __nv_bfloat16* __restrict__ p16) {
     adamw_seg_body(p, g, m, v, seg_off, lr_t, eps_t, n_seg, b1, b2, wd, p16);
 }
-// The same with the segment table passed by value (up to 32 tensors): no host-to-device copy in front of the launch. A
+// The same with the segment table passed by value (up to 128 tensors): no host-to-device copy in front of the launch. A
 // copy would queue on a copy engine, behind whatever long peer-to-peer transfers the data-parallel exchange has in flight.
 struct AdamSegTab {
-    int64_t off[33];
-    float lr[32], eps[32];
+    int64_t off[129];
+    float lr[128], eps[128];
 };
 __global__ void __launch_bounds__(256) adamw_seg_tab_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                             float* __restrict__ m, float* __restrict__ v,
                                                             const __grid_constant__ AdamSegTab tab, int n_seg, float b1,
                                                             float b2, float wd, __nv_bfloat16* __restrict__ p16) {
     adamw_seg_body(p, g, m, v, tab.off, tab.lr, tab.eps, n_seg, b1, b2, wd, p16);
-}
-
-// ------------------------------------------------------------------ delta prologue
-// rust/src/delta.rs:134-179: split, per-head L2 normalise (z / max(|z|, 1e-8)), sigmoids.
-// One warp per (row, head).
-__global__ void __launch_bounds__(256) delta_prep_kernel(const float* __restrict__ qkv,
-                                                         const float* __restrict__ gate, int64_t N, int H, int dh,
-                                                         float* __restrict__ q, float* __restrict__ k,
-                                                         float* __restrict__ v, float* __restrict__ qn,
-                                                         float* __restrict__ kn, float* __restrict__ alpha,
-                                                         float* __restrict__ beta) {
-    const int lane = threadIdx.x & 31;
-    const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (unit >= N * H) return;
-    const int64_t r = unit / H;
-    const int h = (int)(unit % H);
-    const int d = H * dh;
-    const float* src = qkv + r * 3 * (int64_t)d + h * dh;
-    float sq = 0.0f, sk = 0.0f;
-    for (int c = lane; c < dh; c += 32) {
-        float a = src[c], b = src[d + c];
-        sq += a * a;
-        sk += b * b;
-    }
-    sq = warp_sum(sq);
-    sk = warp_sum(sk);
-    const float nq = fmaxf(sqrtf(sq), 1e-8f), nk = fmaxf(sqrtf(sk), 1e-8f);
-    const int64_t o = r * (int64_t)d + h * dh;
-    for (int c = lane; c < dh; c += 32) {
-        q[o + c] = src[c] / nq;
-        k[o + c] = src[d + c] / nk;
-        v[o + c] = src[2 * d + c];
-    }
-    if (lane == 0) {
-        qn[r * H + h] = nq;
-        kn[r * H + h] = nk;
-        alpha[r * H + h] = 1.0f / (1.0f + expf(-gate[r * 2 * H + h]));
-        beta[r * H + h] = 1.0f / (1.0f + expf(-gate[r * 2 * H + H + h]));
-    }
 }
 
 inline bool warp_rows_ok(int64_t cols, const void* a, const void* b) {
@@ -508,7 +469,7 @@ int asca_adamw_segmented_cast(asca_ctx* ctx, float* p, const float* g, float* m,
     int64_t blocks = ceil_div64(n, 1024);
     const int64_t cap = (int64_t)ctx->sm_count * 16;
     if (blocks > cap) blocks = cap;
-    if (n_seg <= 32) {   // the table travels with the launch
+    if (n_seg <= 128) {   // the table travels with the launch
         AdamSegTab tab{};
         for (int i = 0; i <= n_seg; ++i) tab.off[i] = seg_off[i];
         for (int i = 0; i < n_seg; ++i) tab.lr[i] = lr_t[i], tab.eps[i] = eps_t[i];
@@ -530,18 +491,6 @@ int asca_adamw_segmented_cast(asca_ctx* ctx, float* p, const float* g, float* m,
     adamw_seg_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(p, g, m, v, (const int64_t*)w, (const float*)(w + off_b),
                                                                  (const float*)(w + off_b + f_b), n_seg, beta1, beta2,
                                                                  wd_eff, (__nv_bfloat16*)p_bf16);
-    ASCA_CHECK_LAUNCH(ctx);
-    return ASCA_OK;
-}
-
-int asca_delta_prep(asca_ctx* ctx, const float* qkv, const float* gate, int64_t N, int64_t H, int64_t dh, float* q,
-                    float* k, float* v, float* qnorm, float* knorm, float* alpha, float* beta) {
-    if (!ctx) return ASCA_ERR_ARG;
-    ASCA_REQUIRE(ctx, qkv && gate && q && k && v && qnorm && knorm && alpha && beta && N >= 0 && H > 0 && dh > 0,
-                 "delta_prep: bad arguments");
-    if (N == 0) return ASCA_OK;
-    delta_prep_kernel<<<(unsigned)ceil_div64(N * H, 8), 256, 0, ctx->stream>>>(qkv, gate, N, (int)H, (int)dh, q, k, v,
-                                                                               qnorm, knorm, alpha, beta);
     ASCA_CHECK_LAUNCH(ctx);
     return ASCA_OK;
 }

@@ -1,5 +1,6 @@
-// bf16-mode companions of the f32 element-wise entry points: the residual stream, the norms and the
-// gates stay f32; what feeds a tensor-core product is written as bf16 by the kernel that produces it.
+// bf16-mode companions of the f32 element-wise entry points -- the residual stream, the norms and the
+// gates stay f32; what feeds a tensor-core product is written as bf16 by the kernel that produces it --
+// and the delta block's prologue in both types.
 #include "common.cuh"
 
 #include <cuda_bf16.h>
@@ -93,56 +94,100 @@ int residual_rmsnorm_bf16_impl(asca_ctx* ctx, const float* x, const float* yadd,
     return ASCA_OK;
 }
 
-// rust/src/delta.rs:134-179 with bf16 q, k, v outputs. One warp per (row, head); norms and gates f32.
-// VEC: head dim 128 -- every lane holds 4 consecutive elements of q, k and v, read once.
-template <bool VEC>
-__global__ void __launch_bounds__(256) delta_prep_bf16_kernel(const float* __restrict__ qkv, const float* __restrict__ gate,
-                                                              int64_t N, int H, int dh, __nv_bfloat16* __restrict__ q,
-                                                              __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v,
-                                                              float* __restrict__ qn, float* __restrict__ kn,
-                                                              float* __restrict__ alpha, float* __restrict__ beta) {
+// Prologue of the delta block, rust/src/delta.rs:134-179: split, per-head L2 normalise (z / max(|z|, 1e-8)), sigmoids. A
+// (row, head) belongs to DH / 4 neighbouring lanes, a float4 of q, k and v each, so that every warp reads and writes whole
+// 512-byte (f32) runs whatever the head width. Bound by HBM; with a warp per (row, head) and scalar accesses a prefill's
+// 14,448 rows of 12 heads of 64 took 104 us, three times this.
+__device__ __forceinline__ void put4(float* p, float a, float b, float c, float d) { *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d); }
+__device__ __forceinline__ void put4(__nv_bfloat16* p, float a, float b, float c, float d) { *reinterpret_cast<uint2*>(p) = pack4_bf16(a, b, c, d); }
+
+template <int DH, typename T>
+__global__ void __launch_bounds__(256) delta_prep_kernel(const float* __restrict__ qkv, const float* __restrict__ gate, int64_t units, int H,
+                                                         T* __restrict__ q, T* __restrict__ k, T* __restrict__ v, float* __restrict__ qn,
+                                                         float* __restrict__ kn, float* __restrict__ alpha, float* __restrict__ beta) {
+    constexpr int G = DH / 4;   // lanes per unit
+    const int64_t u0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) / G;
+    const int64_t unit = u0 < units ? u0 : units - 1;   // (a ragged last warp repeats the last unit: its shuffles stay whole)
+    const int lane = threadIdx.x % G, h = (int)(unit % H), d = H * DH;
+    const int64_t r = unit / H;
+    const float* src = qkv + r * 3 * (int64_t)d + h * DH + lane * 4;
+    const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + d), c = *reinterpret_cast<const float4*>(src + 2 * d);
+    float sq = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w, sk = b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+#pragma unroll
+    for (int m = G / 2; m > 0; m >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, m);
+        sk += __shfl_xor_sync(0xffffffffu, sk, m);
+    }
+    const float nq = fmaxf(sqrtf(sq), 1e-8f), nk = fmaxf(sqrtf(sk), 1e-8f);
+    if (u0 >= units) return;
+    const int64_t o = r * (int64_t)d + h * DH + lane * 4;
+    put4(q + o, a.x / nq, a.y / nq, a.z / nq, a.w / nq);
+    put4(k + o, b.x / nk, b.y / nk, b.z / nk, b.w / nk);
+    put4(v + o, c.x, c.y, c.z, c.w);
+    if (lane == 0) {
+        qn[unit] = nq;
+        kn[unit] = nk;
+        alpha[unit] = 1.0f / (1.0f + expf(-gate[r * 2 * H + h]));
+        beta[unit] = 1.0f / (1.0f + expf(-gate[r * 2 * H + H + h]));
+    }
+}
+// the same for any head width and alignment, one warp per (row, head)
+template <typename T>
+__global__ void __launch_bounds__(256) delta_prep_any_kernel(const float* __restrict__ qkv, const float* __restrict__ gate, int64_t units, int H,
+                                                             int dh, T* __restrict__ q, T* __restrict__ k, T* __restrict__ v,
+                                                             float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ alpha,
+                                                             float* __restrict__ beta) {
     const int lane = threadIdx.x & 31;
     const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (unit >= N * H) return;
+    if (unit >= units) return;
     const int64_t r = unit / H;
     const int h = (int)(unit % H);
     const int d = H * dh;
     const float* src = qkv + r * 3 * (int64_t)d + h * dh;
     const int64_t o = r * (int64_t)d + h * dh;
-    float nq, nk;
-    if (VEC) {
-        const float4 a = reinterpret_cast<const float4*>(src)[lane], b = reinterpret_cast<const float4*>(src + d)[lane],
-                     c = reinterpret_cast<const float4*>(src + 2 * d)[lane];
-        const float sq = warp_sum(a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w);
-        const float sk = warp_sum(b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w);
-        nq = fmaxf(sqrtf(sq), 1e-8f);
-        nk = fmaxf(sqrtf(sk), 1e-8f);
-        reinterpret_cast<uint2*>(q + o)[lane] = pack4_bf16(a.x / nq, a.y / nq, a.z / nq, a.w / nq);
-        reinterpret_cast<uint2*>(k + o)[lane] = pack4_bf16(b.x / nk, b.y / nk, b.z / nk, b.w / nk);
-        reinterpret_cast<uint2*>(v + o)[lane] = pack4_bf16(c.x, c.y, c.z, c.w);
-    } else {
-        float sq = 0.0f, sk = 0.0f;
-        for (int c = lane; c < dh; c += 32) {
-            const float a = src[c], b = src[d + c];
-            sq += a * a;
-            sk += b * b;
-        }
-        sq = warp_sum(sq);
-        sk = warp_sum(sk);
-        nq = fmaxf(sqrtf(sq), 1e-8f);
-        nk = fmaxf(sqrtf(sk), 1e-8f);
-        for (int c = lane; c < dh; c += 32) {
-            q[o + c] = __float2bfloat16(src[c] / nq);
-            k[o + c] = __float2bfloat16(src[d + c] / nk);
-            v[o + c] = __float2bfloat16(src[2 * d + c]);
-        }
+    float sq = 0.0f, sk = 0.0f;
+    for (int c = lane; c < dh; c += 32) {
+        const float a = src[c], b = src[d + c];
+        sq += a * a;
+        sk += b * b;
+    }
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    const float nq = fmaxf(sqrtf(sq), 1e-8f), nk = fmaxf(sqrtf(sk), 1e-8f);
+    for (int c = lane; c < dh; c += 32) {
+        q[o + c] = from_f32<T>(src[c] / nq);
+        k[o + c] = from_f32<T>(src[d + c] / nk);
+        v[o + c] = from_f32<T>(src[2 * d + c]);
     }
     if (lane == 0) {
-        qn[r * H + h] = nq;
-        kn[r * H + h] = nk;
-        alpha[r * H + h] = 1.0f / (1.0f + expf(-gate[r * 2 * H + h]));
-        beta[r * H + h] = 1.0f / (1.0f + expf(-gate[r * 2 * H + H + h]));
+        qn[unit] = nq;
+        kn[unit] = nk;
+        alpha[unit] = 1.0f / (1.0f + expf(-gate[r * 2 * H + h]));
+        beta[unit] = 1.0f / (1.0f + expf(-gate[r * 2 * H + H + h]));
     }
+}
+
+template <typename T>
+int delta_prep(asca_ctx* ctx, const float* qkv, const float* gate, int64_t N, int64_t H, int64_t dh, void* q, void* k, void* v, float* qn,
+               float* kn, float* alpha, float* beta) {
+    ASCA_REQUIRE(ctx, qkv && gate && q && k && v && qn && kn && alpha && beta && N >= 0 && H > 0 && dh > 0, "delta_prep: bad arguments");
+    if (N == 0) return ASCA_OK;
+    const int64_t units = N * H;
+    const uintptr_t out = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v);
+    const bool vec = (reinterpret_cast<uintptr_t>(qkv) & 15) == 0 && (out & (4 * sizeof(T) - 1)) == 0;
+#define ASCA_PREP(DH_)                                                                                                                  \
+    delta_prep_kernel<DH_, T><<<(unsigned)ceil_div64(units * (DH_ / 4), 256), 256, 0, ctx->stream>>>(qkv, gate, units, (int)H, (T*)q, (T*)k, \
+                                                                                                   (T*)v, qn, kn, alpha, beta)
+    if (vec && dh == 128) ASCA_PREP(128);
+    else if (vec && dh == 64) ASCA_PREP(64);
+    else if (vec && dh == 32) ASCA_PREP(32);
+    else if (vec && dh == 16) ASCA_PREP(16);
+    else
+        delta_prep_any_kernel<T><<<(unsigned)ceil_div64(units, 8), 256, 0, ctx->stream>>>(qkv, gate, units, (int)H, (int)dh, (T*)q, (T*)k, (T*)v,
+                                                                                         qn, kn, alpha, beta);
+#undef ASCA_PREP
+    ASCA_CHECK_LAUNCH(ctx);
+    return ASCA_OK;
 }
 
 }  // namespace
@@ -173,22 +218,16 @@ int asca_residual_rmsnorm_bf16(asca_ctx* ctx, const float* x, const float* yadd,
     return residual_rmsnorm_bf16_impl(ctx, x, yadd, x_mid, xn, rows, cols, eps, nullptr);
 }
 
+int asca_delta_prep(asca_ctx* ctx, const float* qkv, const float* gate, int64_t N, int64_t H, int64_t dh, float* q,
+                    float* k, float* v, float* qnorm, float* knorm, float* alpha, float* beta) {
+    if (!ctx) return ASCA_ERR_ARG;
+    return delta_prep<float>(ctx, qkv, gate, N, H, dh, q, k, v, qnorm, knorm, alpha, beta);
+}
+
 int asca_delta_prep_bf16(asca_ctx* ctx, const float* qkv, const float* gate, int64_t N, int64_t H, int64_t dh, void* q,
                          void* k, void* v, float* qnorm, float* knorm, float* alpha, float* beta) {
     if (!ctx) return ASCA_ERR_ARG;
-    ASCA_REQUIRE(ctx, qkv && gate && q && k && v && qnorm && knorm && alpha && beta && N >= 0 && H > 0 && dh > 0,
-                 "delta_prep_bf16: bad arguments");
-    if (N == 0) return ASCA_OK;
-    const bool vec = dh == 128 && (reinterpret_cast<uintptr_t>(qkv) & 15) == 0 &&
-                     ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 7) == 0;
-    if (vec)
-        delta_prep_bf16_kernel<true><<<(unsigned)ceil_div64(N * H, 8), 256, 0, ctx->stream>>>(
-            qkv, gate, N, (int)H, (int)dh, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, qnorm, knorm, alpha, beta);
-    else
-        delta_prep_bf16_kernel<false><<<(unsigned)ceil_div64(N * H, 8), 256, 0, ctx->stream>>>(
-            qkv, gate, N, (int)H, (int)dh, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, qnorm, knorm, alpha, beta);
-    ASCA_CHECK_LAUNCH(ctx);
-    return ASCA_OK;
+    return delta_prep<__nv_bfloat16>(ctx, qkv, gate, N, H, dh, q, k, v, qnorm, knorm, alpha, beta);
 }
 
 }  // extern "C"
