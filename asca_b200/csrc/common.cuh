@@ -31,6 +31,10 @@ struct asca_ctx {
     // lazily grown scratch owned by the context (partials, tile tables, error words)
     void* ws = nullptr;
     size_t ws_bytes = 0;
+    uint64_t ws_epoch = 0;   // changes when the scratch moves
+    // while a launch sequence is being captured into a graph: blocks the sequence gives back belong to the graph
+    std::vector<void*>* hold = nullptr;
+    cudaStream_t cap_stream = nullptr;
     int* err_word = nullptr;  // device int the kernels with bounded waits write to
     // Pinned staging of small host arrays (ids, losses, tokens): copies that neither block the host nor wait for each
     // other; what goes out is handed to the caller's arrays by the asca_ctx_sync that ends the call.

@@ -22,6 +22,7 @@ int asca_workspace(asca_ctx* ctx, size_t bytes, void** out) {
         ctx->ws = nullptr;
         ctx->ws_bytes = 0;
         size_t want = (bytes + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1);
+        ctx->ws_epoch++;
         ASCA_CUDA(ctx, cudaMalloc(&ctx->ws, want));
         ctx->ws_bytes = want;
     }
@@ -120,6 +121,7 @@ int asca_ctx_destroy(asca_ctx* ctx) {
     if (ctx->err_word) cudaFree(ctx->err_word);
     if (ctx->pin) cudaFreeHost(ctx->pin);
     if (ctx->dyn_buf) cudaFree(ctx->dyn_buf);
+    if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return ASCA_OK;
@@ -174,6 +176,7 @@ int asca_ctx_trim(asca_ctx* ctx) {
     if (ctx->ws) cudaFree(ctx->ws);
     ctx->ws = nullptr;
     ctx->ws_bytes = 0;
+    ctx->ws_epoch++;
     return ASCA_OK;
 }
 
@@ -249,6 +252,10 @@ int asca_free(asca_ctx* ctx, void* dptr) {
     if (!dptr) return ASCA_OK;
     auto it = ctx->live.find(dptr);
     if (it == ctx->live.end()) return asca_fail(ctx, ASCA_ERR_ARG, "asca_free: pointer not from asca_malloc");
+    if (ctx->hold) {
+        ctx->hold->push_back(dptr);
+        return ASCA_OK;
+    }
     ctx->pool.insert({it->second, dptr});
     ctx->live.erase(it);
     // tiles kept for a backward of this checkpoint buffer can no longer be claimed: their storage becomes reusable

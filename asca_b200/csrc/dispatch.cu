@@ -2,7 +2,7 @@
 //
 // expert(t) = hash_route(ids[t], E)  (rust/src/model.rs:69-77), and the permutation is the
 // concatenation of the reference's buckets (rust/src/model.rs:190-193): inside an expert,
-// tokens keep ascending token order. Three small kernels, integer only:
+// tokens keep ascending token order. Few tokens: one kernel. Otherwise three, integer only:
 //   1. each warp histograms its contiguous 1024-token segment            -> counts[seg][E]
 //   2. one CTA turns counts into segment start positions (expert-major scan) + offsets[E+1]
 //   3. each warp replays its segment 32 tokens at a time; match_any gives every lane its rank
@@ -124,6 +124,67 @@ __global__ void __launch_bounds__(WARPS * 32) place_kernel(const uint32_t* __res
     }
 }
 
+// The whole sort in one CTA: 32 warps share the tokens in contiguous runs, histogram and ranking as above. For a training
+// step of a small model the three launches cost more than the work (2048 tokens: 17 us in three kernels, 4 here); a warp's
+// run is replayed serially, which is what ends the range.
+constexpr int SMALL_N = 16384, SMALL_E = 256;
+__global__ void __launch_bounds__(1024) dispatch_small_kernel(const uint32_t* __restrict__ ids, int N, int E, int32_t* __restrict__ perm,
+                                                              int32_t* __restrict__ offsets, int32_t* __restrict__ route) {
+    extern __shared__ int32_t sh[];   // counts, then running positions [warp][expert]; expert starts [E + 1]
+    int32_t* start = sh + 32 * E;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int32_t* run = sh + w * E;
+    for (int e = lane; e < E; e += 32) run[e] = 0;
+    __syncwarp();
+    const int per = ((N + 31) / 32 + 31) & ~31, lo = min(N, w * per), hi = min(N, lo + per);
+    for (int t = lo + lane; t < hi; t += 32) {
+        const uint32_t e = hash_route_dev(ids[t], (uint32_t)E);
+        if (route) route[t] = (int32_t)e;
+        atomicAdd(&run[e], 1);   // integer, shared memory: order-independent result
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += 1024) {   // exclusive scan over the warps, totals in start[e + 1]
+        int32_t s = 0;
+        for (int i = 0; i < 32; ++i) {
+            const int32_t c = sh[i * E + e];
+            sh[i * E + e] = s;
+            s += c;
+        }
+        start[e + 1] = s;
+    }
+    if (threadIdx.x == 0) start[0] = 0;
+    __syncthreads();
+    if (w == 0) {   // inclusive scan over the experts, 32 at a time
+        int32_t base = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            int32_t x = e0 + lane < E ? start[e0 + lane + 1] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (e0 + lane < E) start[e0 + lane + 1] = base + x;
+            base += __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e <= E; e += 1024) offsets[e] = start[e];
+    for (int base = lo; base < hi; base += 32) {
+        const int t = base + lane;
+        const bool live = t < hi;
+        const unsigned act = __ballot_sync(0xffffffffu, live);
+        if (live) {
+            const uint32_t e = hash_route_dev(ids[t], (uint32_t)E);
+            const unsigned peers = __match_any_sync(act, e);
+            const int rank = __popc(peers & ((1u << lane) - 1u));
+            perm[start[e] + run[e] + rank] = t;
+            __syncwarp(act);
+            if (rank == 0) run[e] += __popc(peers);
+        }
+        __syncwarp();
+    }
+}
+
 }  // namespace
 
 extern "C" int asca_moe_dispatch(asca_ctx* ctx, const uint32_t* ids, int64_t N, int64_t E, int32_t* perm,
@@ -134,6 +195,11 @@ extern "C" int asca_moe_dispatch(asca_ctx* ctx, const uint32_t* ids, int64_t N, 
     ASCA_REQUIRE(ctx, N < ((int64_t)1 << 31), "moe_dispatch: N must fit int32");
     if (N == 0) {
         ASCA_CUDA(ctx, cudaMemsetAsync(offsets, 0, (size_t)(E + 1) * 4, ctx->stream));
+        return ASCA_OK;
+    }
+    if (N <= SMALL_N && E <= SMALL_E) {
+        dispatch_small_kernel<<<1, 1024, (size_t)(33 * E + 1) * 4, ctx->stream>>>(ids, (int)N, (int)E, perm, offsets, route);
+        ASCA_CHECK_LAUNCH(ctx);
         return ASCA_OK;
     }
     const int64_t n_seg = ceil_div64(N, SEG);

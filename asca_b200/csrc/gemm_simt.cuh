@@ -35,6 +35,7 @@ struct Params {
     int M, N, K;
     const float* bias;      // per output column, nullable
     int accumulate;         // C += result
+    const float* res;       // C = res + result, rows and pitch of C; nullable
     // optional maps from a logical "token" row to a memory row (int32), nullable:
     //   a_idx: rows of A's memory layout; b_idx: rows of B's memory layout (TN only);
     //   c_idx: rows of C.
@@ -209,6 +210,7 @@ __device__ __forceinline__ void emit(const Params& p, float* crow, const float* 
     if (bias) v += bias[n];
     if (p.epi == EPI_SILU_BWD) v *= silu_grad_f(p.aux[lr * p.ldaux + n]);
     if (p.accumulate) v += crow[n];
+    if (p.res) v += p.res[crow - p.C + n];
     crow[n] = v;
     if (p.epi == EPI_SILU) reinterpret_cast<TC2*>(p.C2)[lr * p.ldc2 + n] = from_f32<TC2>(silu_f(v));
 }
@@ -217,7 +219,7 @@ __device__ __forceinline__ void emit(const Params& p, float* crow, const float* 
 template <typename TC2>
 __device__ __forceinline__ bool vec4_ok(const Params& p, const float* C, const float* bias) {
     int64_t pitch = p.ldc;
-    uintptr_t at = reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias);
+    uintptr_t at = reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(p.res);
     if (p.epi == EPI_SILU_BWD) pitch |= p.ldaux, at |= reinterpret_cast<uintptr_t>(p.aux);
     if (p.epi == EPI_SILU) pitch |= p.ldc2, at |= reinterpret_cast<uintptr_t>(p.C2);
     return ((pitch & 3) | (at & 15)) == 0;
@@ -234,6 +236,10 @@ __device__ __forceinline__ void emit4(const Params& p, float* crow, const float*
     }
     if (p.accumulate) {
         const float4 c = *reinterpret_cast<const float4*>(crow + n);
+        v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
+    }
+    if (p.res) {
+        const float4 c = *reinterpret_cast<const float4*>(p.res + (crow - p.C) + n);
         v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
     }
     *reinterpret_cast<float4*>(crow + n) = v;

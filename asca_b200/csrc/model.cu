@@ -5,6 +5,9 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <initializer_list>
+
+#include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 #include "model.cuh"
 
@@ -91,23 +94,19 @@ __global__ void __launch_bounds__(256) embed_fwd_kernel(const float* __restrict_
 // d_table[v, c] += sum over tokens t with ids[t] == v of dx[t, c]. grid (vocab, ceil(d/128)): the fallback for
 // row lengths that are not a multiple of 4.
 __global__ void __launch_bounds__(128) embed_bwd_kernel(const float* __restrict__ dx, const uint32_t* __restrict__ ids,
-                                                        int64_t N, int d, float* __restrict__ d_table) {
+                                                        int64_t N, int d, float* __restrict__ d_table, int accumulate) {
     const uint32_t v = blockIdx.x;
     const int c = blockIdx.y * 128 + threadIdx.x;
     float acc = 0.0f;
-    bool any = false;
     for (int64_t t = 0; t < N; ++t)
-        if (ids[t] == v) {
-            any = true;
-            if (c < d) acc += dx[t * d + c];
-        }
-    if (any && c < d) d_table[(int64_t)v * d + c] += acc;
+        if (ids[t] == v && c < d) acc += dx[t * d + c];
+    if (c < d) d_table[(int64_t)v * d + c] = accumulate ? d_table[(int64_t)v * d + c] + acc : acc;
 }
 // Same sum, deterministic, for d % 4 == 0: CTA (v, y) owns 256 columns of table row v; each of its 8 warps scans
 // a fixed stride of the ids 32 at a time (ballot), adds the matching rows with every lane holding 8 columns,
 // and the 8 partial rows are added in warp order.
 __global__ void __launch_bounds__(256) embed_bwd_ballot_kernel(const float* __restrict__ dx, const uint32_t* __restrict__ ids,
-                                                               int64_t N, int d, float* __restrict__ d_table) {
+                                                               int64_t N, int d, float* __restrict__ d_table, int accumulate) {
     __shared__ float red[8][256];
     const uint32_t v = blockIdx.x;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -139,7 +138,8 @@ __global__ void __launch_bounds__(256) embed_bwd_ballot_kernel(const float* __re
         float t = 0.0f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) t += red[i][threadIdx.x];
-        d_table[(int64_t)v * d + c] += t;
+        float* o = d_table + (int64_t)v * d + c;
+        *o = accumulate ? *o + t : t;
     }
 }
 __global__ void __launch_bounds__(256) add_kernel(const float* __restrict__ a, const float* __restrict__ b,
@@ -605,6 +605,19 @@ static int cross_entropy_scaled(asca_ctx* ctx, const float* logits, const uint32
                                 float* dlogits, float* loss, float grad_scale);
 }
 
+// d_table (+)= the rows of dx summed by token id
+static int embed_bwd(asca_ctx* ctx, const float* dx, const uint32_t* ids, int64_t N, int64_t d, int64_t vocab, float* d_table, int accumulate) {
+    if (!ctx) return ASCA_ERR_ARG;
+    ASCA_REQUIRE(ctx, dx && ids && d_table && N >= 0 && d > 0 && vocab > 0 && vocab < 65536, "embed_bwd: bad arguments");
+    if (N == 0) return ASCA_OK;
+    if ((d & 3) == 0 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0)
+        embed_bwd_ballot_kernel<<<dim3((unsigned)vocab, (unsigned)ceil_div64(d, 256)), 256, 0, ctx->stream>>>(dx, ids, N, (int)d, d_table, accumulate);
+    else
+        embed_bwd_kernel<<<dim3((unsigned)vocab, (unsigned)ceil_div64(d, 128)), 128, 0, ctx->stream>>>(dx, ids, N, (int)d, d_table, accumulate);
+    ASCA_CHECK_LAUNCH(ctx);
+    return ASCA_OK;
+}
+
 static int materialize_zero_grads(asca_ctx* ctx, asca_model* m) {
     if (!m->grads_zero_pending) return ASCA_OK;
     m->grads_zero_pending = false;
@@ -836,10 +849,242 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
         }
         ASCA_TRY(grad_ready(ctx, m, w.w_qkv, w.w1 - w.w_qkv));   // the block's projections
     }
-    if (!acc) ASCA_CUDA(ctx, cudaMemsetAsync(G + m->embed, 0, (size_t)V * d * 4, ctx->stream));
-    ASCA_TRY(asca_embed_bwd(ctx, dx, ids, N, d, V, G + m->embed));
+    ASCA_TRY(embed_bwd(ctx, dx, ids, N, d, V, G + m->embed, acc));
     ASCA_TRY(grad_ready(ctx, m, 0, m->lay[0].w_qkv));   // embedding + head
     ASCA_CUDA(ctx, cudaGetLastError());
+    return asca_ctx_sync(ctx);
+}
+
+// ---------------------------------------------------------------------------------------------
+// f32 mode. Products that do not depend on one another share a launch (gemm_simt.cuh), bias gradients ride with the weight
+// gradients that read the same rows, residual adds with the products that end a branch: 8 launches a block forward and
+// 8 backward, where one call per operation takes 12 and 19.
+int asca_moe_fwd_f32_residual(asca_ctx* ctx, const float* xn, const float* w1, const float* b1, const float* w2, const float* b2,
+                              const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, const float* res,
+                              float* out, float* pre_p, float* hid_p);   // moe.cu
+
+namespace {
+gemm::Params dense(int mode, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
+                   const float* bias = nullptr, int accumulate = 0) {
+    gemm::Params p{};
+    p.mode = mode; p.M = (int)M; p.N = (int)N; p.K = (int)K;
+    p.A = A; p.lda = lda; p.B = B; p.ldb = ldb; p.C = C; p.ldc = ldc;
+    p.bias = bias; p.accumulate = accumulate;
+    return p;
+}
+int run(asca_ctx* ctx, std::initializer_list<gemm::Params> ps) {
+    gemm::Multi m{};
+    for (const auto& p : ps) m.p[m.n++] = p;
+    ASCA_CUDA(ctx, gemm::launch_f32(ctx, m));
+    ctx->launches++;
+    return ASCA_OK;
+}
+}  // namespace
+
+// The device work of one forward + backward: ids, tg (device) -> loss (device), logits (device, N x V), gradients.
+static int forward_backward_f32_device(asca_ctx* ctx, asca_model* m, const uint32_t* ids, const uint32_t* tg, int64_t B, int64_t T, int acc,
+                                       float* loss, float* logits) {
+    const int64_t N = B * T, d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab, L = m->L;
+    const int64_t CH = 64;
+    float* P = m->params;
+    float* G = m->grads;
+    Bufs bf(ctx);
+    int32_t* perm = (int32_t*)bf.f(N);
+    int32_t* offs = (int32_t*)bf.f(E + 1);
+    ASCA_REQUIRE(ctx, perm && offs, "model_forward_backward: out of memory");
+    ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));   // same routing for every layer
+
+    struct Act {
+        float *x_in, *q, *k, *v, *qn, *kn, *al, *be, *o, *ckpt, *x_mid, *xn, *pre_p, *hid_p;
+    };
+    std::vector<Act> acts(L + 1);   // (the last entry: only x_in, the last block's output)
+    const int64_t nck = asca_delta_ckpt_floats(B, T, H, dh, CH);
+    float* qkv = bf.f(N * 3 * d);
+    float* gate = bf.f(N * 2 * H);
+    ASCA_REQUIRE(ctx, qkv && gate, "model_forward_backward: out of memory");
+    for (int64_t li = 0; li <= L; ++li) {
+        Act& a = acts[li];
+        a.x_in = bf.f(N * d);
+        ASCA_REQUIRE(ctx, a.x_in, "model_forward_backward: out of memory");
+        if (li == L) break;
+        a.q = bf.f(N * d); a.k = bf.f(N * d); a.v = bf.f(N * d);
+        a.qn = bf.f(N * H); a.kn = bf.f(N * H); a.al = bf.f(N * H); a.be = bf.f(N * H);
+        a.o = bf.f(N * d); a.ckpt = bf.f(nck); a.x_mid = bf.f(N * d); a.xn = bf.f(N * d);
+        a.pre_p = bf.f(N * F); a.hid_p = bf.f(N * F);
+        ASCA_REQUIRE(ctx, a.q && a.k && a.v && a.qn && a.kn && a.al && a.be && a.o && a.ckpt && a.x_mid && a.xn && a.pre_p && a.hid_p,
+                     "model_forward_backward: out of memory");
+    }
+    ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, acts[0].x_in));
+    // ---- forward (rust/src/model.rs:651-700)
+    for (int64_t li = 0; li < L; ++li) {
+        const Lyr& w = m->lay[li];
+        Act& a = acts[li];
+        ASCA_TRY(run(ctx, {dense(ASCA_NN, N, 3 * d, d, a.x_in, d, P + w.w_qkv, 3 * d, qkv, 3 * d, P + w.b_qkv),
+                           dense(ASCA_NN, N, 2 * H, d, a.x_in, d, P + w.w_gate, 2 * H, gate, 2 * H, P + w.b_gate)}));
+        ASCA_TRY(asca_delta_prep(ctx, qkv, gate, N, H, dh, a.q, a.k, a.v, a.qn, a.kn, a.al, a.be));
+        ASCA_TRY(asca_delta_fwd(ctx, a.q, a.k, a.v, a.al, a.be, B, T, H, dh, CH, ASCA_F32, a.o, nullptr, nullptr, a.ckpt));
+        gemm::Params o = dense(ASCA_NN, N, d, d, a.o, d, P + w.w_o, d, a.x_mid, d, P + w.b_o);
+        o.res = a.x_in;
+        ASCA_TRY(run(ctx, {o}));
+        ASCA_TRY(asca_rmsnorm_fwd(ctx, a.x_mid, a.xn, nullptr, N, d, 1e-6f));
+        ASCA_TRY(asca_moe_fwd_f32_residual(ctx, a.xn, P + w.w1, P + w.b1, P + w.w2, P + w.b2, perm, offs, N, d, F, E, a.x_mid,
+                                           acts[li + 1].x_in, a.pre_p, a.hid_p));
+    }
+    const float* x = acts[L].x_in;
+    float *h_final = bf.f(N * d), *dlogits = bf.f(N * V), *dh_ = bf.f(N * d), *dx = bf.f(N * d), *dxn = bf.f(N * d), *d_o = bf.f(N * d),
+          *d_qkv = bf.f(N * 3 * d), *d_gate = bf.f(N * 2 * H);
+    ASCA_REQUIRE(ctx, h_final && dlogits && dh_ && dx && dxn && d_o && d_qkv && d_gate, "model_forward_backward: out of memory");
+    ASCA_TRY(asca_rmsnorm_fwd(ctx, x, h_final, nullptr, N, d, 1e-6f));
+    ASCA_TRY(run(ctx, {dense(ASCA_NN, N, V, d, h_final, d, P + m->head, V, logits, V)}));
+    // ---- backward (rust/src/model.rs:744-794)
+    ASCA_TRY(cross_entropy_scaled(ctx, logits, tg, N, V, dlogits, loss, m->grad_scale));
+    ASCA_TRY(run(ctx, {dense(ASCA_TN, d, V, N, h_final, d, dlogits, V, G + m->head, V, nullptr, acc),
+                       dense(ASCA_NT, N, d, V, dlogits, V, P + m->head, V, dh_, d)}));
+    ASCA_TRY(asca_rmsnorm_bwd(ctx, x, dh_, dx, N, d, 1e-6f));
+    for (int64_t li = L - 1; li >= 0; --li) {
+        const Lyr& w = m->lay[li];
+        Act& a = acts[li];
+        // HashMoe::backward: gradients accumulate into the flat buffer
+        ASCA_TRY((acc ? asca_moe_bwd_acc : asca_moe_bwd)(ctx, a.xn, P + w.w1, P + w.w2, a.pre_p, a.hid_p, dx, perm, offs, N, d, F, E, ASCA_F32,
+                                  G + w.w1, G + w.b1, G + w.w2, G + w.b2, dxn));
+        ASCA_TRY(grad_ready(ctx, m, w.w1, (li + 1 < L ? m->lay[li + 1].w_qkv : m->n_params) - w.w1));   // the block's experts
+        // d_mid = dx + rmsnorm_bwd(x_mid, dxn)
+        const int rc = asca_rmsnorm_bwd_add_cast(ctx, a.x_mid, dxn, dx, dx, nullptr, N, d, 1e-6f);
+        if (rc == ASCA_ERR_UNSUPPORTED) {
+            ASCA_TRY(asca_rmsnorm_bwd(ctx, a.x_mid, dxn, d_o, N, d, 1e-6f));
+            add_kernel<<<(unsigned)ceil_div64(N * d, 256), 256, 0, ctx->stream>>>(dx, d_o, dx, N * d);
+            ASCA_CHECK_LAUNCH(ctx);
+        } else {
+            ASCA_TRY(rc);
+        }
+        // DeltaBlock::backward (rust/src/delta.rs:615-674)
+        gemm::Params dwo = dense(ASCA_TN, d, d, N, a.o, d, dx, d, G + w.w_o, d, nullptr, acc);
+        dwo.colsum = G + w.b_o;
+        ASCA_TRY(run(ctx, {dense(ASCA_NT, N, d, d, dx, d, P + w.w_o, d, d_o, d), dwo}));
+        ASCA_TRY(asca_delta_bwd(ctx, a.q, a.k, a.v, a.al, a.be, a.qn, a.kn, d_o, a.ckpt, B, T, H, dh, CH, ASCA_F32, d_qkv, d_gate));
+        // dx = d_mid + d_qkv Wqkv^T + d_gate Wg^T   (accumulate onto d_mid in place)
+        gemm::Params dwq = dense(ASCA_TN, d, 3 * d, N, a.x_in, d, d_qkv, 3 * d, G + w.w_qkv, 3 * d, nullptr, acc),
+                     dwg = dense(ASCA_TN, d, 2 * H, N, a.x_in, d, d_gate, 2 * H, G + w.w_gate, 2 * H, nullptr, acc),
+                     dxp = dense(ASCA_NT, N, d, 3 * d, d_qkv, 3 * d, P + w.w_qkv, 3 * d, dx, d, nullptr, 1);
+        dwq.colsum = G + w.b_qkv;
+        dwg.colsum = G + w.b_gate;
+        dxp.A2 = d_gate; dxp.lda2 = 2 * H; dxp.B2 = P + w.w_gate; dxp.ldb2 = 2 * H; dxp.K2 = (int)(2 * H);
+        ASCA_TRY(run(ctx, {dwq, dwg, dxp}));
+        ASCA_TRY(grad_ready(ctx, m, w.w_qkv, w.w1 - w.w_qkv));   // the block's projections
+    }
+    ASCA_TRY(embed_bwd(ctx, dx, ids, N, d, V, G + m->embed, acc));
+    ASCA_TRY(grad_ready(ctx, m, 0, m->lay[0].w_qkv));   // embedding + head
+    ASCA_CUDA(ctx, cudaGetLastError());
+    return ASCA_OK;
+}
+
+static void drop_plan(asca_ctx* ctx, asca_step_plan& p) {
+    if (p.exec) cudaGraphExecDestroy(p.exec);
+    p.exec = nullptr;
+    if (ctx)
+        for (void* b : p.held) asca_free(ctx, b);
+    p.held.clear();
+}
+
+// The plan of this call, or null where a graph is not for it: large batches (their kernels outlast their launches), callers
+// that want to be told of finished gradient ranges, profiling.
+static asca_step_plan* find_plan(asca_ctx* ctx, asca_model* m, int64_t B, int64_t T, int acc) {
+    const int64_t N = B * T;
+    if (m->grad_hook || m->dp || ctx->profiling || N * m->L * (10 * m->d + 2 * m->F) * 4 > ((int64_t)256 << 20)) return nullptr;
+    for (auto& p : m->plans)
+        if (p.B == B && p.T == T && p.acc == acc && p.grad_scale == m->grad_scale) {
+            p.stamp = ++m->plan_clock;
+            return p.broken ? nullptr : &p;
+        }
+    if (m->plans.size() >= MAX_PLANS) {
+        size_t old = 0;
+        for (size_t i = 1; i < m->plans.size(); ++i)
+            if (m->plans[i].stamp < m->plans[old].stamp) old = i;
+        cudaStreamSynchronize(ctx->stream);
+        drop_plan(ctx, m->plans[old]);
+        m->plans.erase(m->plans.begin() + old);
+    }
+    asca_step_plan p;
+    p.B = B; p.T = T; p.acc = acc; p.grad_scale = m->grad_scale; p.stamp = ++m->plan_clock;
+    void* at[4] = {};
+    const size_t bytes[4] = {(size_t)N * 4, (size_t)N * 4, 4, (size_t)N * m->vocab * 4};
+    for (int i = 0; i < 4; ++i) {
+        if (asca_malloc(ctx, bytes[i], &at[i]) != ASCA_OK) {
+            drop_plan(ctx, p);
+            return nullptr;
+        }
+        p.held.push_back(at[i]);
+    }
+    p.ids = (uint32_t*)at[0]; p.tg = (uint32_t*)at[1]; p.loss = (float*)at[2]; p.logits = (float*)at[3];
+    m->plans.push_back(p);
+    return &m->plans.back();
+}
+
+// Captures the step on a stream of its own (the caller's may be one that cannot be captured).
+static int capture_plan(asca_ctx* ctx, asca_model* m, asca_step_plan& p) {
+    if (!ctx->cap_stream) ASCA_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
+    cudaStream_t user = ctx->stream;
+    const int64_t before = ctx->launches;
+    cudaGraph_t graph = nullptr;
+    std::vector<void*> held;
+    ctx->stream = ctx->cap_stream;
+    ctx->hold = &held;
+    int rc = cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeRelaxed) == cudaSuccess ? ASCA_OK : ASCA_ERR_CUDA;
+    if (rc == ASCA_OK) {
+        rc = forward_backward_f32_device(ctx, m, p.ids, p.tg, p.B, p.T, p.acc, p.loss, p.logits);
+        if (cudaStreamEndCapture(ctx->cap_stream, &graph) != cudaSuccess) rc = ASCA_ERR_CUDA;
+    }
+    ctx->hold = nullptr;
+    ctx->stream = user;
+    if (rc == ASCA_OK && cudaGraphInstantiate(&p.exec, graph, 0) != cudaSuccess) rc = ASCA_ERR_CUDA;
+    if (graph) cudaGraphDestroy(graph);
+    p.launches = ctx->launches - before;
+    ctx->launches = before;
+    p.ws_epoch = ctx->ws_epoch;
+    if (rc != ASCA_OK) {
+        cudaGetLastError();
+        p.exec = nullptr;
+        p.broken = true;
+        for (void* b : held) asca_free(ctx, b);
+        return rc;
+    }
+    p.held.insert(p.held.end(), held.begin(), held.end());
+    return ASCA_OK;
+}
+
+static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* ids_h, const uint32_t* tg_h, int64_t B, int64_t T, float* loss_h,
+                                float* logits_h) {
+    const int64_t N = B * T, V = m->vocab;
+    const int acc = m->grads_zero_pending ? 0 : 1;   // first backward after zero_grads: overwrite
+    m->grads_zero_pending = false;
+    asca_stage_scope staged(ctx);
+    Bufs bf(ctx);
+    asca_step_plan* p = find_plan(ctx, m, B, T, acc);
+    uint32_t *ids = p ? p->ids : (uint32_t*)bf.f(N), *tg = p ? p->tg : (uint32_t*)bf.f(N);
+    float *loss = p ? p->loss : bf.f(1), *logits = p ? p->logits : bf.f(N * V);
+    ASCA_REQUIRE(ctx, ids && tg && loss && logits, "model_forward_backward: out of memory");
+    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
+    ASCA_TRY(asca_stage_in(ctx, tg, tg_h, (size_t)N * 4));
+    if (p && p->exec && p->ws_epoch != ctx->ws_epoch) {   // the scratch its kernels name has moved
+        cudaStreamSynchronize(ctx->stream);
+        cudaGraphExecDestroy(p->exec);
+        p->exec = nullptr;
+        while (p->held.size() > 4) {
+            asca_free(ctx, p->held.back());
+            p->held.pop_back();
+        }
+    }
+    // a shape seen a third time is one that repeats
+    if (p && !p->exec && p->runs >= 2) capture_plan(ctx, m, *p);
+    if (p && p->exec) {
+        ASCA_CUDA(ctx, cudaGraphLaunch(p->exec, ctx->stream));
+        ctx->launches += p->launches;
+    } else {
+        if (p) p->runs++;
+        ASCA_TRY(forward_backward_f32_device(ctx, m, ids, tg, B, T, acc, loss, logits));
+    }
+    ASCA_TRY(asca_stage_out(ctx, loss_h, loss, 4));
+    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)N * V * 4));
     return asca_ctx_sync(ctx);
 }
 
@@ -906,15 +1151,7 @@ int asca_embed_fwd(asca_ctx* ctx, const float* table, const uint32_t* ids, int64
 
 int asca_embed_bwd(asca_ctx* ctx, const float* dx, const uint32_t* ids, int64_t N, int64_t d, int64_t vocab,
                    float* d_table) {
-    if (!ctx) return ASCA_ERR_ARG;
-    ASCA_REQUIRE(ctx, dx && ids && d_table && N >= 0 && d > 0 && vocab > 0 && vocab < 65536, "embed_bwd: bad arguments");
-    if (N == 0) return ASCA_OK;
-    if ((d & 3) == 0 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0)
-        embed_bwd_ballot_kernel<<<dim3((unsigned)vocab, (unsigned)ceil_div64(d, 256)), 256, 0, ctx->stream>>>(dx, ids, N, (int)d, d_table);
-    else
-        embed_bwd_kernel<<<dim3((unsigned)vocab, (unsigned)ceil_div64(d, 128)), 128, 0, ctx->stream>>>(dx, ids, N, (int)d, d_table);
-    ASCA_CHECK_LAUNCH(ctx);
-    return ASCA_OK;
+    return embed_bwd(ctx, dx, ids, N, d, vocab, d_table, 1);
 }
 
 int asca_model_create(asca_ctx* ctx, int64_t vocab, int64_t d, int64_t H, int64_t L, int64_t E, int64_t F,
@@ -966,6 +1203,7 @@ int asca_model_create(asca_ctx* ctx, int64_t vocab, int64_t d, int64_t H, int64_
 int asca_model_destroy(asca_ctx* ctx, asca_model* m) {
     if (!m) return ASCA_OK;
     if (ctx) cudaStreamSynchronize(ctx->stream);
+    for (auto& p : m->plans) drop_plan(ctx, p);
     if (m->dp) asca_dp_free(m);   // before the buffers its copies and collectives touch
     for (float* b : {m->params, m->grads, m->m, m->v})
         if (b) cudaFree(b);
@@ -1075,112 +1313,11 @@ int asca_model_forward_backward_host(asca_ctx* ctx, asca_model* m, const uint32_
                                      int64_t B, int64_t T, float* loss_h, float* logits_h) {
     if (!ctx || !m) return ASCA_ERR_ARG;
     ASCA_REQUIRE(ctx, ids_h && tg_h && loss_h && B > 0 && T > 0, "model_forward_backward: bad arguments");
-    const int64_t N = B * T, d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab, L = m->L;
-    const int64_t CH = 64;
+    const int64_t N = B * T, V = m->vocab;
     for (int64_t i = 0; i < N; ++i)
         ASCA_REQUIRE(ctx, ids_h[i] < (uint32_t)V && tg_h[i] < (uint32_t)V, "model_forward_backward: id out of range");
     if (m->compute == ASCA_BF16) return forward_backward_bf16(ctx, m, ids_h, tg_h, B, T, loss_h, logits_h);
-    float* P = m->params;
-    float* G = m->grads;
-    const int acc = m->grads_zero_pending ? 0 : 1;   // first backward after zero_grads: overwrite
-    m->grads_zero_pending = false;
-    Bufs bf(ctx);
-    uint32_t* ids = (uint32_t*)bf.f(N);
-    uint32_t* tg = (uint32_t*)bf.f(N);
-    int32_t* perm = (int32_t*)bf.f(N);
-    int32_t* offs = (int32_t*)bf.f(E + 1);
-    ASCA_REQUIRE(ctx, ids && tg && perm && offs, "model_forward_backward: out of memory");
-    asca_stage_scope staged(ctx);
-    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
-    ASCA_TRY(asca_stage_in(ctx, tg, tg_h, (size_t)N * 4));
-    ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));   // same routing for every layer
-
-    struct Act {
-        float *x_in, *q, *k, *v, *qn, *kn, *al, *be, *o, *ckpt, *x_mid, *xn, *pre_p, *hid_p;
-    };
-    std::vector<Act> acts(L);
-    const int64_t nck = asca_delta_ckpt_floats(B, T, H, dh, CH);
-    float* x = bf.f(N * d);
-    float* qkv = bf.f(N * 3 * d);
-    float* gate = bf.f(N * 2 * H);
-    float* y = bf.f(N * d);
-    float* mo = bf.f(N * d);
-    ASCA_REQUIRE(ctx, x && qkv && gate && y && mo, "model_forward_backward: out of memory");
-    ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, x));
-    // ---- forward (rust/src/model.rs:651-700)
-    for (int64_t li = 0; li < L; ++li) {
-        const Lyr& w = m->lay[li];
-        Act& a = acts[li];
-        a.x_in = bf.f(N * d); a.q = bf.f(N * d); a.k = bf.f(N * d); a.v = bf.f(N * d);
-        a.qn = bf.f(N * H); a.kn = bf.f(N * H); a.al = bf.f(N * H); a.be = bf.f(N * H);
-        a.o = bf.f(N * d); a.ckpt = bf.f(nck); a.x_mid = bf.f(N * d); a.xn = bf.f(N * d);
-        a.pre_p = bf.f(N * F); a.hid_p = bf.f(N * F);
-        ASCA_REQUIRE(ctx, a.x_in && a.q && a.k && a.v && a.qn && a.kn && a.al && a.be && a.o && a.ckpt && a.x_mid && a.xn &&
-                              a.pre_p && a.hid_p, "model_forward_backward: out of memory");
-        ASCA_CUDA(ctx, cudaMemcpyAsync(a.x_in, x, (size_t)N * d * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 3 * d, d, x, d, P + w.w_qkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, ASCA_F32));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 2 * H, d, x, d, P + w.w_gate, 2 * H, gate, 2 * H, P + w.b_gate, 0, ASCA_F32));
-        ASCA_TRY(asca_delta_prep(ctx, qkv, gate, N, H, dh, a.q, a.k, a.v, a.qn, a.kn, a.al, a.be));
-        ASCA_TRY(asca_delta_fwd(ctx, a.q, a.k, a.v, a.al, a.be, B, T, H, dh, CH, ASCA_F32, a.o, nullptr, nullptr, a.ckpt));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, d, d, a.o, d, P + w.w_o, d, y, d, P + w.b_o, 0, ASCA_F32));
-        ASCA_TRY(asca_residual_rmsnorm(ctx, x, y, a.x_mid, a.xn, N, d, 1e-6f));
-        ASCA_TRY(asca_moe_fwd(ctx, a.xn, P + w.w1, P + w.b1, P + w.w2, P + w.b2, perm, offs, N, d, F, E, ASCA_F32, mo,
-                              a.pre_p, a.hid_p));
-        ASCA_TRY(asca_residual_rmsnorm(ctx, a.x_mid, mo, x, nullptr, N, d, 1e-6f));   // x_out
-    }
-    float* h_final = bf.f(N * d);
-    float* logits = bf.f(N * V);
-    float* dlogits = bf.f(N * V);
-    float* loss_d = bf.f(1);
-    ASCA_REQUIRE(ctx, h_final && logits && dlogits && loss_d, "model_forward_backward: out of memory");
-    ASCA_TRY(asca_rmsnorm_fwd(ctx, x, h_final, nullptr, N, d, 1e-6f));
-    ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, V, d, h_final, d, P + m->head, V, logits, V, nullptr, 0, ASCA_F32));
-    if (logits_h) ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)N * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    // ---- backward (rust/src/model.rs:744-794)
-    ASCA_TRY(cross_entropy_scaled(ctx, logits, tg, N, V, dlogits, loss_d, m->grad_scale));
-    ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
-    ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, V, N, h_final, d, dlogits, V, G + m->head, V, nullptr, acc, ASCA_F32));
-    float* dh_ = bf.f(N * d);
-    float* dx = bf.f(N * d);
-    float* dxn = bf.f(N * d);
-    float* d_moe = bf.f(N * d);
-    float* d_o = bf.f(N * d);
-    float* d_qkv = bf.f(N * 3 * d);
-    float* d_gate = bf.f(N * 2 * H);
-    ASCA_REQUIRE(ctx, dh_ && dx && dxn && d_moe && d_o && d_qkv && d_gate, "model_forward_backward: out of memory");
-    ASCA_TRY(asca_gemm(ctx, ASCA_NT, N, d, V, dlogits, V, P + m->head, V, dh_, d, nullptr, 0, ASCA_F32));
-    ASCA_TRY(asca_rmsnorm_bwd(ctx, x, dh_, dx, N, d, 1e-6f));   // x = x_out of the last layer
-    const int64_t blocks_nd = ceil_div64(N * d, 256);
-    for (int64_t li = L - 1; li >= 0; --li) {
-        const Lyr& w = m->lay[li];
-        Act& a = acts[li];
-        // HashMoe::backward: gradients accumulate into the flat buffer
-        ASCA_TRY((acc ? asca_moe_bwd_acc : asca_moe_bwd)(ctx, a.xn, P + w.w1, P + w.w2, a.pre_p, a.hid_p, dx, perm, offs, N, d, F, E, ASCA_F32,
-                                  G + w.w1, G + w.b1, G + w.w2, G + w.b2, dxn));
-        ASCA_TRY(grad_ready(ctx, m, w.w1, (li + 1 < L ? m->lay[li + 1].w_qkv : m->n_params) - w.w1));   // the block's experts
-        ASCA_TRY(asca_rmsnorm_bwd(ctx, a.x_mid, dxn, d_moe, N, d, 1e-6f));
-        add_kernel<<<(unsigned)blocks_nd, 256, 0, ctx->stream>>>(dx, d_moe, dx, N * d);   // d_mid
-        ctx->launches++;
-        // DeltaBlock::backward (rust/src/delta.rs:615-674)
-        ASCA_TRY(asca_gemm(ctx, ASCA_NT, N, d, d, dx, d, P + w.w_o, d, d_o, d, nullptr, 0, ASCA_F32));
-        ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, d, N, a.o, d, dx, d, G + w.w_o, d, nullptr, acc, ASCA_F32));
-        ASCA_TRY(asca_colsum(ctx, dx, d, N, d, G + w.b_o, acc));
-        ASCA_TRY(asca_delta_bwd(ctx, a.q, a.k, a.v, a.al, a.be, a.qn, a.kn, d_o, a.ckpt, B, T, H, dh, CH, ASCA_F32, d_qkv,
-                                d_gate));
-        ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, 3 * d, N, a.x_in, d, d_qkv, 3 * d, G + w.w_qkv, 3 * d, nullptr, acc, ASCA_F32));
-        ASCA_TRY(asca_colsum(ctx, d_qkv, 3 * d, N, 3 * d, G + w.b_qkv, acc));
-        ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, 2 * H, N, a.x_in, d, d_gate, 2 * H, G + w.w_gate, 2 * H, nullptr, acc, ASCA_F32));
-        ASCA_TRY(asca_colsum(ctx, d_gate, 2 * H, N, 2 * H, G + w.b_gate, acc));
-        // dx = d_mid + d_qkv Wqkv^T + d_gate Wg^T   (accumulate onto d_mid in place)
-        ASCA_TRY(asca_gemm(ctx, ASCA_NT, N, d, 3 * d, d_qkv, 3 * d, P + w.w_qkv, 3 * d, dx, d, nullptr, 1, ASCA_F32));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NT, N, d, 2 * H, d_gate, 2 * H, P + w.w_gate, 2 * H, dx, d, nullptr, 1, ASCA_F32));
-        ASCA_TRY(grad_ready(ctx, m, w.w_qkv, w.w1 - w.w_qkv));   // the block's projections
-    }
-    if (!acc) ASCA_CUDA(ctx, cudaMemsetAsync(G + m->embed, 0, (size_t)V * d * 4, ctx->stream));
-    ASCA_TRY(asca_embed_bwd(ctx, dx, ids, N, d, V, G + m->embed));
-    ASCA_TRY(grad_ready(ctx, m, 0, m->lay[0].w_qkv));   // embedding + head
-    ASCA_CUDA(ctx, cudaGetLastError());
-    return asca_ctx_sync(ctx);
+    return forward_backward_f32(ctx, m, ids_h, tg_h, B, T, loss_h, logits_h);
 }
 
 int asca_model_adamw_step(asca_ctx* ctx, asca_model* m, float lr, float beta1, float beta2, float eps, float wd) {

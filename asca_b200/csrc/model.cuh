@@ -12,6 +12,24 @@ struct Lyr {
 
 struct asca_dp;   // dp.cu
 
+// A small model's training step replayed as one graph launch: its dozens of kernels take microseconds each, less than the
+// host needs to launch them one by one. One per (batch shape, first or later backward, gradient scale), least recently used
+// dropped beyond MAX_PLANS; a plan owns the buffers its graph names.
+struct asca_step_plan {
+    int64_t B = 0, T = 0;
+    int acc = 0;
+    float grad_scale = 0.0f;
+    uint32_t *ids = nullptr, *tg = nullptr;
+    float *loss = nullptr, *logits = nullptr;
+    int runs = 0;               // direct runs so far
+    cudaGraphExec_t exec = nullptr;
+    bool broken = false;        // could not be captured
+    uint64_t ws_epoch = 0, stamp = 0;
+    int64_t launches = 0;
+    std::vector<void*> held;
+};
+constexpr size_t MAX_PLANS = 8;
+
 struct asca_model {
     int64_t vocab, d, H, L, E, F, n_params;
     int64_t embed, head;
@@ -48,6 +66,8 @@ struct asca_model {
     // bf16 mode, vocabulary 256: let the head product's epilogue take the cross-entropy (loss and bf16 dlogits) where
     // it runs on CTA pairs and the caller does not ask for the logits (asca_model_set_fused_head)
     bool fused_head = true;
+    std::vector<asca_step_plan> plans;
+    uint64_t plan_clock = 0;
     // data parallelism (dp.cu): the communicator attached to this model and what is in flight on its side stream
     asca_dp* dp = nullptr;
     // set by a sharded optimizer step: the f32 master weights and moments of the other ranks' chunks are not

@@ -217,7 +217,47 @@ int moe_bwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, 
     return gemm_tc::launch(ctx, g4);
 }
 
+// The two FFMA products; res (nullable, (N, d)): added to the output rows.
+int moe_fwd_simt(asca_ctx* ctx, const void* xn, const void* w1, const float* b1, const void* w2, const float* b2, const int32_t* perm,
+                 const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, int bf, const float* res, float* out, float* pre_p,
+                 void* hid_p) {
+    // pre_p[r,:] = xn[perm[r],:] W1[:, eF:(e+1)F] + b1[e];  hid_p = silu(pre_p)
+    gemm::Params p{};
+    p.A = xn; p.lda = d; p.a_idx = perm;
+    p.B = w1; p.ldb = E * F; p.b_gstride = F;
+    p.C = pre_p; p.ldc = F;
+    p.M = 0; p.N = (int)F; p.K = (int)d;
+    p.bias = b1; p.bias_gstride = F;
+    p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_M;
+    p.epi = gemm::EPI_SILU; p.C2 = hid_p; p.ldc2 = F;
+    p.mode = ASCA_NN; p.total_rows = N;
+    if (bf) ASCA_CUDA(ctx, gemm::launch<__nv_bfloat16>(ctx, p, 1, 1));
+    else ASCA_CUDA(ctx, gemm::launch<float>(ctx, p, 0, 0));
+    ctx->launches++;
+    // out[perm[r],:] = hid_p[r,:] W2[eF:(e+1)F,:] + b2
+    gemm::Params q{};
+    q.A = hid_p; q.lda = F;
+    q.B = w2; q.ldb = d; q.b_gstride = F * d;
+    q.C = out; q.ldc = d; q.c_idx = perm;
+    q.res = res;
+    q.M = 0; q.N = (int)d; q.K = (int)F;
+    q.bias = b2; q.bias_gstride = 0;
+    q.offsets = offsets; q.n_groups = (int)E; q.group_dim = gemm::GROUP_M;
+    q.epi = gemm::EPI_NONE;
+    q.mode = ASCA_NN; q.total_rows = N;
+    ASCA_CUDA(ctx, gemm::launch<float>(ctx, q, bf, bf));
+    ctx->launches++;
+    return ASCA_OK;
+}
+
 }  // namespace
+
+// f32 forward with the residual add in the second product's store: out = res + moe(xn)
+int asca_moe_fwd_f32_residual(asca_ctx* ctx, const float* xn, const float* w1, const float* b1, const float* w2, const float* b2,
+                              const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, const float* res,
+                              float* out, float* pre_p, float* hid_p) {
+    return moe_fwd_simt(ctx, xn, w1, b1, w2, b2, perm, offsets, N, d, F, E, 0, res, out, pre_p, hid_p);
+}
 
 // Decode-step form of the layer, on bf16 rows already in expert order: x[perm[r], :] += silu(xp[r] W1_e + b1_e) W2_e + b2
 // in place on the f32 residual rows, with a bf16 copy of the updated rows in x16. Two launches of the few-row
@@ -268,36 +308,11 @@ int asca_moe_fwd(asca_ctx* ctx, const void* xn, const void* w1, const float* b1,
     if (N == 0) return ASCA_OK;
     const int bf = dtype == ASCA_BF16;
     if (bf && tc_shapes_ok(d, F)) {
-        int rc = moe_fwd_tc(ctx, (const __nv_bfloat16*)xn, (const __nv_bfloat16*)w1, b1, (const __nv_bfloat16*)w2, b2,
+        const int rc = moe_fwd_tc(ctx, (const __nv_bfloat16*)xn, (const __nv_bfloat16*)w1, b1, (const __nv_bfloat16*)w2, b2,
                             perm, offsets, N, d, F, E, out, pre_p, (__nv_bfloat16*)hid_p);
         if (rc != ASCA_ERR_UNSUPPORTED) return rc;
     }
-    // pre_p[r,:] = xn[perm[r],:] W1[:, eF:(e+1)F] + b1[e];  hid_p = silu(pre_p)
-    gemm::Params p{};
-    p.A = xn; p.lda = d; p.a_idx = perm;
-    p.B = w1; p.ldb = E * F; p.b_gstride = F;
-    p.C = pre_p; p.ldc = F;
-    p.M = 0; p.N = (int)F; p.K = (int)d;
-    p.bias = b1; p.bias_gstride = F;
-    p.offsets = offsets; p.n_groups = (int)E; p.group_dim = gemm::GROUP_M;
-    p.epi = gemm::EPI_SILU; p.C2 = hid_p; p.ldc2 = F;
-    p.mode = ASCA_NN; p.total_rows = N;
-    if (bf) ASCA_CUDA(ctx, gemm::launch<__nv_bfloat16>(ctx, p, 1, 1));
-    else ASCA_CUDA(ctx, gemm::launch<float>(ctx, p, 0, 0));
-    ctx->launches++;
-    // out[perm[r],:] = hid_p[r,:] W2[eF:(e+1)F,:] + b2
-    gemm::Params q{};
-    q.A = hid_p; q.lda = F;
-    q.B = w2; q.ldb = d; q.b_gstride = F * d;
-    q.C = out; q.ldc = d; q.c_idx = perm;
-    q.M = 0; q.N = (int)d; q.K = (int)F;
-    q.bias = b2; q.bias_gstride = 0;
-    q.offsets = offsets; q.n_groups = (int)E; q.group_dim = gemm::GROUP_M;
-    q.epi = gemm::EPI_NONE;
-    q.mode = ASCA_NN; q.total_rows = N;
-    ASCA_CUDA(ctx, gemm::launch<float>(ctx, q, bf, bf));
-    ctx->launches++;
-    return ASCA_OK;
+    return moe_fwd_simt(ctx, xn, w1, b1, w2, b2, perm, offsets, N, d, F, E, bf, nullptr, out, pre_p, hid_p);
 }
 
 static int moe_bwd_impl(asca_ctx* ctx, const void* xn, const void* w1, const void* w2, const float* pre_p, const void* hid_p,

@@ -76,3 +76,68 @@ def test_f32_decode_cluster_widths_and_fallbacks(orc, gpu, cfg, ns):
         assert rel_err(logits[s:s + 1], lg) < F32_TOL and nxt[s] == lg.argmax()
         assert rel_err(state[:, s].cpu().numpy(), st) < F32_TOL
     dev.free()
+
+
+# The f32 recurrence with one, two and four value columns per lane group (few chains to many), ragged stages, decay strong enough
+# to be folded in step by step, and the three-kernel backward with every width of its chain kernel.
+@pytest.mark.parametrize("B,T,H,dh", [(1, 1, 1, 16), (2, 33, 2, 16), (40, 70, 20, 16), (1, 65, 1, 32), (60, 40, 20, 32), (130, 16, 20, 32),
+                                      (3, 64, 2, 64), (20, 50, 8, 64), (40, 129, 8, 64), (1, 130, 1, 128), (6, 24, 8, 128), (12, 80, 8, 128)])
+@pytest.mark.parametrize("decay", [2.0, -3.0])
+def test_f32_delta_column_splits(orc, gpu, B, T, H, dh, decay):
+    import torch
+    from asca_b200 import ops
+
+    g = np.random.default_rng(B + T + dh)
+    n, d = B * T, H * dh
+    q, k, v, d_o = (g.standard_normal((n, d)).astype(np.float32) for _ in range(4))
+    qn, kn = (np.linalg.norm(x.reshape(n, H, dh), axis=-1).astype(np.float32) for x in (q, k))
+    q, k = ((x.reshape(n, H, dh) / xn[..., None]).reshape(n, d).astype(np.float32) for x, xn in ((q, qn), (k, kn)))
+    alpha = (1 / (1 + np.exp(-(decay + 0.5 * g.standard_normal((n, H)))))).astype(np.float32)
+    beta = (1 / (1 + np.exp(-g.standard_normal((n, H))))).astype(np.float32)
+    tq, tk, tv, ta, tb, tqn, tkn, tdo = (torch.from_numpy(x).cuda() for x in (q, k, v, alpha, beta, qn, kn, d_o))
+    o, s_fin, ckpt = ops.delta_fwd(gpu, tq, tk, tv, ta, tb, B, T, H, dh, want_final=True)
+    d_qkv, d_gate = ops.delta_bwd(gpu, tq, tk, tv, ta, tb, tqn, tkn, tdo, ckpt, B, T, H, dh)
+    gpu.sync()
+    b = B - 1   # the last sequence of the batch stands for all: sequences are independent
+    rows = slice(b * T, B * T)
+    o_ref, s_ref = orc.delta_scan(q[rows], k[rows], v[rows], alpha[rows], beta[rows], 1, T, H, dh)[:2]
+    dq_ref, dg_ref = orc.delta_bptt(q[rows], k[rows], v[rows], alpha[rows], beta[rows], qn[rows], kn[rows], d_o[rows], 1, T, H, dh)
+    assert rel_err(o[rows].cpu().numpy(), o_ref) < F32_TOL
+    assert rel_err(s_fin[b].cpu().numpy(), s_ref.reshape(H, dh, dh)) < F32_TOL
+    assert rel_err(d_qkv[rows].cpu().numpy(), dq_ref) < F32_TOL
+    assert rel_err(d_gate[rows].cpu().numpy(), dg_ref) < F32_TOL
+
+
+# The one-kernel dispatch up to its limits (16,384 tokens, 256 experts) and just past them.
+@pytest.mark.parametrize("n,e", [(1, 1), (32, 4), (33, 256), (1025, 7), (16384, 64), (16384, 256), (16385, 64), (2000, 257)])
+def test_dispatch_small_and_past_it(orc, gpu, n, e):
+    ids = np.random.default_rng(n + e).integers(0, 4096, n).astype(np.uint32)
+    for got, want in zip(gpu.moe_dispatch(ids, e), orc.moe_dispatch(ids, e)):
+        assert np.array_equal(got, want)
+
+
+# A repeated f32 training step is replayed as a graph from its third call on: same losses and gradients, bit for bit, as the
+# direct launches (a gradient hook keeps those), with a second shape and an accumulating backward in between.
+def test_f32_training_step_graph_equals_direct_launches(orc, gpu):
+    import asca_b200
+
+    cfg = (256, 64, 4, 2, 4, 256)
+    params = orc.Rng(5).normal(331408, 0.02)
+    runs = []
+    for hooked in (False, True):
+        m = asca_b200.Model(gpu, *cfg)
+        m.set_params(params)
+        if hooked:
+            m.set_grad_hook(lambda off, cnt: None)
+        out = []
+        for step in range(6):
+            m.zero_grads()
+            for B, T in ((4, 96), (2, 130)):
+                ids, tg = (orc.Rng(100 * step + s).below(256, B * T) for s in (1, 2))
+                out.append(m.forward_backward(ids, tg, B))
+            out.append(m.get()[1])
+            m.adamw_step(1e-3)
+        runs.append(out)
+        m.free()
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
