@@ -74,8 +74,9 @@ constexpr int THREADS = 256;
 
 struct Multi {
     Params p[MAX_PROBLEMS];
-    int tile0[MAX_PROBLEMS + 1];   // first tile of each problem
-    int n, split;
+    int split[MAX_PROBLEMS];      // CTAs that share a tile's k: 1, 2, 4 or 8, at most the launch's cluster size
+    int cta0[MAX_PROBLEMS + 1];   // first CTA of each problem (a multiple of the cluster size: a cluster works on one problem)
+    int n;
 };
 
 template <int BM_, int BN_, int BK_, int TM_, int TN_, int KG_, int STAGES_>
@@ -332,8 +333,12 @@ struct StagerOf<C, T, ROWS, ALONG_K, true> {
     using type = TransposingStager<T, ROWS, C::BK>;
 };
 
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
 template <class C, int MODE, typename TA, typename TB, typename TC2>
-__device__ __forceinline__ void tile_product(const Params& p, int tile, int rank, int split, float* smem, int* sh_group) {
+__device__ __forceinline__ void tile_product(const Params& p, int tile, bool live, int rank, int split, float* smem, int* sh_group) {
     constexpr int BM = C::BM, BN = C::BN, BK = C::BK, TM = C::TM, TN = C::TN, KG = C::KG, STAGES = C::STAGES;
     constexpr bool A_KC = !C::TRANSPOSE && MODE != ASCA_TN, B_KC = !C::TRANSPOSE && MODE == ASCA_NT;   // along k in shared memory
     constexpr int LDA = A_KC ? BK + 4 : BM + (C::TRANSPOSE && MODE != ASCA_TN ? 8 : 4),
@@ -348,7 +353,7 @@ __device__ __forceinline__ void tile_product(const Params& p, int tile, int rank
     const int tiles_n = (N + BN - 1) / BN, tid = threadIdx.x;
     int64_t row_base = 0;   // logical row offset of this group (GROUP_M) or its k offset (GROUP_K)
     int g = 0, t = tile;
-    if (p.group_dim != GROUP_NONE) {
+    if (p.group_dim != GROUP_NONE && live) {
         // locate (group, tile): warp 0 scans the per-group tile counts
         if (tid < 32) {
             const int lane = tid;
@@ -382,8 +387,17 @@ __device__ __forceinline__ void tile_product(const Params& p, int tile, int rank
         }
         __syncthreads();
         g = sh_group[0];
-        if (g < 0) return;   // surplus tile of the upper-bound grid (every CTA of its cluster returns here)
         t = sh_group[1];
+        live = g >= 0;       // else a surplus tile of the upper-bound grid
+    }
+    if (!live) {
+        if (split > 1) {   // (other tiles of the cluster are waiting for it)
+            cluster_sync();
+            cluster_sync();
+        }
+        return;
+    }
+    if (p.group_dim != GROUP_NONE) {
         const int lo = p.offsets[g], n_g = p.offsets[g + 1] - lo;
         row_base = lo;
         if (p.group_dim == GROUP_M) {
@@ -532,14 +546,17 @@ __device__ __forceinline__ void tile_product(const Params& p, int tile, int rank
         for (int j = 0; j < TN; ++j) red_cs[kg * BN + n_of(j)] = cs[j];
     }
     const uint32_t mine = (uint32_t)__cvta_generic_to_shared(smem);
-    if (split > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    uint32_t base;   // first CTA of this tile in its cluster: itself where the tile is not split, whatever the launch's clusters
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(base));
+    base = base / split * split;
+    if (split > 1) cluster_sync();
     else __syncthreads();
     // v + the KG values at off, off + stride, ... (floats) of every CTA, in order
     auto add_all = [&](float4 v, int off, int stride) -> float4 {
         for (int r = 0; r < split; ++r) {
             float4 x[KG];
             uint32_t at;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(r));
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(base + r));
 #pragma unroll
             for (int q = 0; q < KG; ++q)
                 asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -575,7 +592,7 @@ __device__ __forceinline__ void tile_product(const Params& p, int tile, int rank
                 *o = p.accumulate ? *o + x[j] : x[j];
             }
     }
-    if (split > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");   // peers may still read
+    if (split > 1) cluster_sync();   // peers may still read
 }
 
 // MODE: the operand form of every problem of the launch, or ANY_MODE (mixed forms; costs registers).
@@ -584,23 +601,21 @@ template <class C, int MODE, typename TA, typename TB, typename TC2>
 __global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const __grid_constant__ Multi mp) {
     extern __shared__ __align__(16) float smem[];
     __shared__ int sh_group[2];
-    const int split = mp.split, tile = blockIdx.x / split, rank = blockIdx.x % split;
     int i = 0;
 #pragma unroll
     for (int q = 1; q < MAX_PROBLEMS; ++q)
-        if (q < mp.n && tile >= mp.tile0[q]) i = q;
+        if (q < mp.n && (int)blockIdx.x >= mp.cta0[q]) i = q;
     const Params& p = mp.p[i];
-    const int t = tile - mp.tile0[i];
+    const int split = mp.split[i], at = blockIdx.x - mp.cta0[i], t = at / split, rank = at % split;
     const int mode = MODE == ANY_MODE ? p.mode : MODE;
     if (mode == ASCA_TN && p.A == nullptr) {
-        if (rank == 0) colsum_tile(p, t, smem);
-    } else if (mode == ASCA_NN) {
-        tile_product<C, ASCA_NN, TA, TB, TC2>(p, t, rank, split, smem, sh_group);
-    } else if (mode == ASCA_TN) {
-        tile_product<C, ASCA_TN, TA, TB, TC2>(p, t, rank, split, smem, sh_group);
-    } else {
-        tile_product<C, ASCA_NT, TA, TB, TC2>(p, t, rank, split, smem, sh_group);
+        colsum_tile(p, t, smem);   // (split 1; tiles past the last column do nothing)
+        return;
     }
+    const bool live = p.group_dim != GROUP_NONE || t < ((p.M + C::BM - 1) / C::BM) * ((p.N + C::BN - 1) / C::BN);
+    if (mode == ASCA_NN) tile_product<C, ASCA_NN, TA, TB, TC2>(p, t, live, rank, split, smem, sh_group);
+    else if (mode == ASCA_TN) tile_product<C, ASCA_TN, TA, TB, TC2>(p, t, live, rank, split, smem, sh_group);
+    else tile_product<C, ASCA_NT, TA, TB, TC2>(p, t, live, rank, split, smem, sh_group);
 }
 
 // Tiles of one problem (upper bound for GROUP_M: every group can add one ragged tile).
@@ -614,41 +629,42 @@ inline int64_t tiles_of(const Params& p) {
 }
 
 template <class C, int MODE, typename TA, typename TB, typename TC2>
-inline cudaError_t launch_mode(asca_ctx* ctx, Multi& m, int split) {
-    int64_t tiles = 0;
+inline cudaError_t launch_mode(asca_ctx* ctx, Multi& m) {
+    int64_t ctas = 0;
+    int cluster = 1;
+    for (int i = 0; i < m.n; ++i) cluster = std::max(cluster, m.split[i]);
     for (int i = 0; i < m.n; ++i) {
-        m.tile0[i] = (int)tiles;
-        tiles += tiles_of<C>(m.p[i]);
+        m.cta0[i] = (int)ctas;
+        ctas += (tiles_of<C>(m.p[i]) * m.split[i] + cluster - 1) / cluster * cluster;
     }
-    m.tile0[m.n] = (int)tiles;
-    m.split = split;
-    if (tiles == 0) return cudaSuccess;
+    m.cta0[m.n] = (int)ctas;
+    if (ctas == 0) return cudaSuccess;
     auto kern = gemm_kernel<C, MODE, TA, TB, TC2>;
     if (C::SMEM > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * split));
+    cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)split;
+    at[0].val.clusterDim.x = (unsigned)cluster;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = split > 1 ? 1 : 0;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, (const Multi)m);
 }
 
 template <class C, typename TA, typename TB, typename TC2>
-inline cudaError_t launch_cfg(asca_ctx* ctx, Multi& m, int split) {
+inline cudaError_t launch_cfg(asca_ctx* ctx, Multi& m) {
     for (int i = 1; i < m.n; ++i)
-        if (m.p[i].mode != m.p[0].mode) return launch_mode<C, ANY_MODE, TA, TB, TC2>(ctx, m, split);
-    if (m.p[0].mode == ASCA_NN) return launch_mode<C, ASCA_NN, TA, TB, TC2>(ctx, m, split);
-    if (m.p[0].mode == ASCA_TN) return launch_mode<C, ASCA_TN, TA, TB, TC2>(ctx, m, split);
-    return launch_mode<C, ASCA_NT, TA, TB, TC2>(ctx, m, split);
+        if (m.p[i].mode != m.p[0].mode) return launch_mode<C, ANY_MODE, TA, TB, TC2>(ctx, m);
+    if (m.p[0].mode == ASCA_NN) return launch_mode<C, ASCA_NN, TA, TB, TC2>(ctx, m);
+    if (m.p[0].mode == ASCA_TN) return launch_mode<C, ASCA_TN, TA, TB, TC2>(ctx, m);
+    return launch_mode<C, ASCA_NT, TA, TB, TC2>(ctx, m);
 }
 
 // Estimated microseconds of a launch, from the measured time of a slab on an SM (CTAs that share an SM add their slabs: the
@@ -659,49 +675,73 @@ inline cudaError_t launch_cfg(asca_ctx* ctx, Multi& m, int split) {
 struct Shape {
     double slab, cta, cta_split, launch;
 };
+// The best estimate for one tile shape; split: how the problems' k is shared out (the longest problem's chain is halved as
+// long as that helps).
 template <class C>
-inline double estimate(const Multi& m, int split, int n_sm, const Shape& c) {
-    double ctas = 0.0, slabs = 0.0, longest = 0.0;
+inline double estimate(const Multi& m, int n_sm, int max_split, const Shape& c, int (&split)[MAX_PROBLEMS]) {
+    double tiles[MAX_PROBLEMS], slabs[MAX_PROBLEMS];
     for (int i = 0; i < m.n; ++i) {
         const Params& p = m.p[i];
+        split[i] = 1;
+        tiles[i] = slabs[i] = 0.0;
         if (p.mode == ASCA_TN && !p.A) continue;
         const double tn = (p.N + C::BN - 1) / C::BN, groups = p.group_dim == GROUP_NONE ? 1 : p.n_groups;
         const double mean = (double)p.total_rows / groups;   // token rows of a group
         const double tm = std::ceil((p.group_dim == GROUP_M ? mean : (double)p.M) / C::BM);
         const double k = (p.group_dim == GROUP_K ? mean : (double)p.K) + p.K2;
-        const double t = groups * tm * tn, s = std::max(1.0, std::ceil(k / C::BK) / split);
-        ctas += t * split;
-        slabs += t * split * s;
-        longest = std::max(longest, s);
+        tiles[i] = groups * tm * tn;
+        slabs[i] = std::max(1.0, std::ceil(k / C::BK));
     }
-    if (ctas == 0.0) return c.launch;
-    const double rounds = std::ceil(ctas / n_sm);
-    return c.launch + std::max(rounds * slabs / ctas, longest) * c.slab + rounds * (split > 1 ? c.cta_split : c.cta);
+    auto time = [&]() {
+        double ctas = 0.0, work = 0.0, longest = 0.0;
+        for (int i = 0; i < m.n; ++i) {
+            const double one = std::max(1.0, slabs[i] / split[i]) * c.slab + (split[i] > 1 ? c.cta_split : c.cta), n = tiles[i] * split[i];
+            if (n == 0.0) continue;
+            ctas += n;
+            work += n * one;
+            longest = std::max(longest, one);
+        }
+        return ctas == 0.0 ? c.launch : c.launch + std::max(longest, std::ceil(ctas / n_sm) * work / ctas);
+    };
+    double best = time();
+    for (;;) {
+        int at = 0;
+        for (int i = 1; i < m.n; ++i)
+            if (slabs[i] / split[i] > slabs[at] / split[at]) at = i;
+        if (split[at] >= max_split || slabs[at] < 2.0 * split[at]) return best;
+        // (twice may help where once does not: the barriers are paid with the first halving)
+        int keep = split[at], found = 0;
+        for (int s = split[at] * 2; s <= max_split; s *= 2) {
+            split[at] = s;
+            const double t = time();
+            if (t < best) {
+                best = t;
+                keep = s;
+                found = 1;
+            }
+        }
+        split[at] = keep;
+        if (!found) return best;
+    }
 }
 
-inline void plan(const asca_ctx* ctx, const Multi& m, int& shape, int& split) {
+// Tile shape of a launch (0: 128, 1: 64, 2: 32 wide); fills in the k-splits.
+inline int plan(const asca_ctx* ctx, Multi& m) {
     const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
-    double best = 1e300;
-    shape = split = 1;
-    for (int s = 1; s <= 8; s *= 2) {
-        const double e[3] = {s > 1 ? 1e300 : estimate<CfgL>(m, s, n_sm, {1.6, 7.0, 0.0, 3.3}),
-                             estimate<CfgM>(m, s, n_sm, {1.0, 0.8, 3.8, 3.3}), estimate<CfgS>(m, s, n_sm, {0.81, 0.8, 2.3, 2.6})};
-        for (int c = 0; c < 3; ++c)
-            if (e[c] < best) {
-                best = e[c];
-                shape = c;
-                split = s;
-            }
-    }
+    int split[3][MAX_PROBLEMS];
+    const double e[3] = {estimate<CfgL>(m, n_sm, 1, {1.6, 7.0, 0.0, 3.3}, split[0]), estimate<CfgM>(m, n_sm, 8, {1.0, 0.8, 3.8, 3.3}, split[1]),
+                         estimate<CfgS>(m, n_sm, 8, {0.81, 0.8, 2.3, 2.6}, split[2])};
+    const int shape = e[0] < e[1] ? (e[0] < e[2] ? 0 : 2) : (e[1] < e[2] ? 1 : 2);
+    for (int i = 0; i < m.n; ++i) m.split[i] = split[shape][i];
+    return shape;
 }
 
 // One launch of up to MAX_PROBLEMS f32 products.
 inline cudaError_t launch_f32(asca_ctx* ctx, Multi& m) {
-    int shape, split;
-    plan(ctx, m, shape, split);
-    if (shape == 0) return launch_cfg<CfgL, float, float, float>(ctx, m, split);
-    if (shape == 1) return launch_cfg<CfgM, float, float, float>(ctx, m, split);
-    return launch_cfg<CfgS, float, float, float>(ctx, m, split);
+    const int shape = plan(ctx, m);
+    if (shape == 0) return launch_cfg<CfgL, float, float, float>(ctx, m);
+    if (shape == 1) return launch_cfg<CfgM, float, float, float>(ctx, m);
+    return launch_cfg<CfgS, float, float, float>(ctx, m);
 }
 
 // One product with operands of either type. bf16 operands come here only where the tensor-core kernels cannot take the
@@ -711,10 +751,11 @@ inline cudaError_t launch(asca_ctx* ctx, const Params& p, int a_bf16, int b_bf16
     Multi m{};
     m.p[0] = p;
     m.n = 1;
+    m.split[0] = 1;
     if (!a_bf16 && !b_bf16) return launch_f32(ctx, m);
-    if (a_bf16 && b_bf16) return launch_cfg<CfgM, __nv_bfloat16, __nv_bfloat16, TC2>(ctx, m, 1);
-    if (a_bf16) return launch_cfg<CfgM, __nv_bfloat16, float, TC2>(ctx, m, 1);
-    return launch_cfg<CfgM, float, __nv_bfloat16, TC2>(ctx, m, 1);
+    if (a_bf16 && b_bf16) return launch_cfg<CfgM, __nv_bfloat16, __nv_bfloat16, TC2>(ctx, m);
+    if (a_bf16) return launch_cfg<CfgM, __nv_bfloat16, float, TC2>(ctx, m);
+    return launch_cfg<CfgM, float, __nv_bfloat16, TC2>(ctx, m);
 }
 
 }  // namespace gemm

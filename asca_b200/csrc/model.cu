@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) add_cast4_kernel(const float* a, const fl
 __global__ void __launch_bounds__(256) decode_prologue_kernel(const float* __restrict__ table, const uint32_t* __restrict__ ids, int ns,
                                                               int d, int E, float* __restrict__ x, __nv_bfloat16* __restrict__ x16,
                                                               int32_t* __restrict__ perm, int32_t* __restrict__ offs,
-                                                              int32_t* __restrict__ inv_perm) {
+                                                              int32_t* __restrict__ inv_perm, int32_t* __restrict__ counter) {
     __shared__ int32_t cnt[1024 + 1];
     __shared__ uint16_t ex[1024];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(256) decode_prologue_kernel(const float* __res
         }
     }
     if (blockIdx.x != 0) return;
+    if (threadIdx.x == 0) *counter += 1;   // the step's row of the token buffer
     for (int e = threadIdx.x; e <= E; e += 256) cnt[e] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < ns; i += 256) {
@@ -279,9 +280,10 @@ __global__ void __launch_bounds__(256) concat_bias_kernel(const float* __restric
     const int c = blockIdx.x * 256 + threadIdx.x;
     if (c < ld) dst[c] = c < ca ? a[c] : (c < ca + cb ? b[c - ca] : 0.0f);
 }
-// greedy argmax per row, lowest index on ties
+// greedy argmax per row, lowest index on ties; toks (nullable): also written to row *counter (0 without one) of toks
 __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ logits, int64_t N, int V,
-                                                     uint32_t* __restrict__ out) {
+                                                     uint32_t* __restrict__ out, uint32_t* __restrict__ toks = nullptr,
+                                                     const int32_t* __restrict__ counter = nullptr) {
     const int lane = threadIdx.x & 31;
     const int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     pdl_wait();
@@ -305,7 +307,10 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ l
             bi = oi;
         }
     }
-    if (lane == 0) out[t] = (uint32_t)bi;
+    if (lane == 0) {
+        out[t] = (uint32_t)bi;
+        if (toks) toks[(counter ? *counter : 0) * N + t] = (uint32_t)bi;
+    }
 }
 
 // alpha, beta = sigmoid of the gate logits (rust/src/delta.rs:167-179): logits (N, 2H), one thread per (row, head).
@@ -410,63 +415,46 @@ static int refresh_dec_w(asca_ctx* ctx, asca_model* m) {
     return ASCA_OK;
 }
 
-// n_steps steps in bf16 mode. Step 0 consumes ids_h; a later step consumes the previous step's argmax, which never
-// leaves the device (tokens_h, n_steps x ns, receives all of them after the last step). One synchronisation at the end.
-static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* ids_h, int64_t ns, float* logits_h,
-                            uint32_t* next_h, int64_t n_steps = 1, uint32_t* tokens_h = nullptr) {
+// The buffers of a decode step; cur: the step's token ids in, its argmax out.
+namespace {
+struct DecodeBufs {
+    uint32_t *cur, *toks;
+    int32_t *perm, *offs, *inv_perm, *counter;
+    float *x, *qkv, *gate, *o, *y, *x_mid, *mo, *logits, *pre_p, *qg;
+    __nv_bfloat16 *x16, *o16, *xn16, *hid16, *hf16;
+    bool take(Bufs& bf, const asca_model* m, int64_t ns, int64_t n_steps) {
+        const int64_t d = m->d, H = m->H, F = m->F, ldq = (3 * d + 2 * H + 7) & ~(int64_t)7;
+        auto h16 = [&](int64_t n) { return (__nv_bfloat16*)bf.f((n + 1) / 2); };
+        cur = (uint32_t*)bf.f(ns); toks = (uint32_t*)bf.f(ns * n_steps);
+        perm = (int32_t*)bf.f(ns); offs = (int32_t*)bf.f(m->E + 1); inv_perm = (int32_t*)bf.f(ns); counter = (int32_t*)bf.f(1);
+        x = bf.f(ns * d); qkv = bf.f(ns * 3 * d); gate = bf.f(ns * 2 * H); o = bf.f(ns * d); y = bf.f(ns * d); x_mid = bf.f(ns * d);
+        mo = bf.f(ns * d); logits = bf.f(ns * m->vocab); pre_p = bf.f(ns * F); qg = bf.f(ns * ldq);
+        x16 = h16(ns * d); o16 = h16(ns * d); xn16 = h16(ns * d); hid16 = h16(ns * F); hf16 = h16(ns * d);
+        return cur && toks && perm && offs && inv_perm && counter && x && qkv && gate && o && y && x_mid && mo && logits && pre_p && qg && x16 &&
+               o16 && xn16 && hid16 && hf16;
+    }
+};
+// Which form of the step the shapes allow. fused64: head dim 64 (one projection for qkv + gate, the warp-per-head state update,
+// casts folded in). sorted_moe: with a handful of tokens per expert the MoE runs on rows in expert order end to end -- the norm
+// writes its bf16 rows at their expert-order position (the gather), and the second expert product adds into the residual rows
+// through the permutation and writes the next block's bf16 input (the combine, the residual add and the cast). packed: every
+// product of the step is then a few-row product whose weights are read once, from a copy in the order that kernel streams them
+// (per layer: qkv+gate, out, experts' W1, experts' W2; then the head). one_prologue: dispatch, embedding and its cast in one
+// launch, which also advances the token buffer's row.
+struct DecodeForm {
+    bool fused64, sorted_moe, packed, one_prologue;
+    int64_t ldq, r_qg, r_o, r_w1, r_w2, r_layer, r_head;
+};
+}  // namespace
+
+// One decode step from b.cur; the choice lands in b.cur and in the token buffer (toks_row where the prologue does not count).
+static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeForm& f, const DecodeBufs& b, float* state, int64_t ns,
+                                   bool pdl_first, uint32_t* toks_row) {
     typedef __nv_bfloat16 bf16;
-    const int64_t d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab;
+    const int64_t d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab, ldq = f.ldq;
     const int BF = ASCA_BF16;
-    ASCA_TRY(refresh_params16(ctx, m));
-    ASCA_TRY(asca_dp_wait_all(ctx, m));
     const float* P = m->params;
     const bf16* W = m->params16;
-    Bufs bf(ctx);
-    auto h16 = [&](int64_t n) { return (bf16*)bf.f((n + 1) / 2); };
-    uint32_t* ids = (uint32_t*)bf.f(ns);
-    uint32_t* toks = (uint32_t*)bf.f(ns * n_steps);   // every step's chosen ids
-    int32_t* perm = (int32_t*)bf.f(ns);
-    int32_t* offs = (int32_t*)bf.f(E + 1);
-    float *x = bf.f(ns * d), *qkv = bf.f(ns * 3 * d), *gate = bf.f(ns * 2 * H), *o = bf.f(ns * d), *y = bf.f(ns * d),
-          *x_mid = bf.f(ns * d), *mo = bf.f(ns * d), *logits = bf.f(ns * V), *pre_p = bf.f(ns * F);
-    bf16 *x16 = h16(ns * d), *o16 = h16(ns * d), *xn16 = h16(ns * d), *hid16 = h16(ns * F), *hf16 = h16(ns * d);
-    ASCA_REQUIRE(ctx, ids && toks && perm && offs && x && qkv && gate && o && y && x_mid && mo && logits && pre_p && x16 && o16 &&
-                          xn16 && hid16 && hf16, "model_decode_step: out of memory");
-    asca_stage_scope staged(ctx);
-    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)ns * 4));
-    const bool fused64 = dh == 64;   // one projection for qkv + gate, the warp-per-head state update, casts folded in
-    const int64_t ldq = (3 * d + 2 * H + 7) & ~(int64_t)7;
-    if (fused64) ASCA_TRY(refresh_dec_w(ctx, m));
-    float* qg = fused64 ? bf.f(ns * ldq) : nullptr;
-    ASCA_REQUIRE(ctx, !fused64 || qg, "model_decode_step: out of memory");
-    // With a handful of tokens per expert the MoE runs on rows in expert order end to end: the norm writes its bf16
-    // rows at their expert-order position (the gather), and the second expert product adds into the residual rows
-    // through the permutation and writes the next block's bf16 input (the combine, the residual add and the cast).
-    const bool sorted_moe = asca_moe_fwd_sorted_residual(ctx, xn16, W + m->lay16[0].w1, P + m->lay[0].b1, W + m->lay16[0].w2,
-                                                         P + m->lay[0].b2, perm, offs, ns, d, F, E, x, x16, hid16, 1, 0) == ASCA_OK;
-    // ... and then every product of the step is a few-row product whose weights are read once: they are kept a second
-    // time in the order that kernel streams them (per layer: qkv+gate, out, experts' W1, experts' W2; then the head)
-    const bool packed = fused64 && sorted_moe && ns <= 256;
-    const int64_t r_qg = gemm_tc::skinny_packed_rows(1, d, ldq), r_o = gemm_tc::skinny_packed_rows(1, d, d),
-                  r_w1 = gemm_tc::skinny_packed_rows(E, d, F), r_w2 = gemm_tc::skinny_packed_rows(E, F, d),
-                  r_layer = r_qg + r_o + r_w1 + r_w2, r_head = gemm_tc::skinny_packed_rows(1, d, V);
-    if (packed && !m->dec_pk) {
-        if (cudaMalloc((void**)&m->dec_pk, (size_t)(m->L * r_layer + r_head) * 128) != cudaSuccess)
-            return asca_fail(ctx, ASCA_ERR_OOM, "model: cannot allocate the decode weight copy");
-        m->dec_pk_stale = true;
-    }
-    if (packed && m->dec_pk_stale) {
-        for (int64_t li = 0; li < m->L; ++li) {
-            const Lyr& w16 = m->lay16[li];
-            bf16* pk = m->dec_pk + li * r_layer * 64;
-            ASCA_TRY(gemm_tc::skinny_pack(ctx, m->dec_w + li * d * ldq, ldq, 1, 0, 0, d, ldq, pk));
-            ASCA_TRY(gemm_tc::skinny_pack(ctx, W + w16.w_o, d, 1, 0, 0, d, d, pk + r_qg * 64));
-            ASCA_TRY(gemm_tc::skinny_pack(ctx, W + w16.w1, E * F, E, F, 0, d, F, pk + (r_qg + r_o) * 64));
-            ASCA_TRY(gemm_tc::skinny_pack(ctx, W + w16.w2, d, E, 0, F, F, d, pk + (r_qg + r_o + r_w1) * 64));
-        }
-        ASCA_TRY(gemm_tc::skinny_pack(ctx, W + m->head16, V, 1, 0, 0, d, V, m->dec_pk + m->L * r_layer * 64));
-        m->dec_pk_stale = false;
-    }
     auto few_rows = [&](const bf16* X, int64_t K, const bf16* Wpk, int64_t N, float* C, int64_t ldc, const float* bias) -> int {
         gemm_tc::Args t{};
         t.mode = ASCA_NN;
@@ -478,75 +466,203 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         if (!gemm_tc::supported(t)) return asca_fail(ctx, ASCA_ERR_UNSUPPORTED, "model_decode_step: product not supported");
         return gemm_tc::launch_skinny(ctx, t);
     };
-    int32_t* inv_perm = sorted_moe ? (int32_t*)bf.f(ns) : nullptr;
-    ASCA_REQUIRE(ctx, !sorted_moe || inv_perm, "model_decode_step: out of memory");
     struct PdlScope {
         asca_ctx* c;
         explicit PdlScope(asca_ctx* c_) : c(c_) {}
         ~PdlScope() { c->pdl = false; }
     } pdl_scope(ctx);
-    for (int64_t step = 0; step < n_steps; ++step) {
-    const uint32_t* cur = step == 0 ? ids : toks + (step - 1) * ns;
-    uint32_t* nxt = toks + step * ns;
     ctx->pdl = false;
-    if (sorted_moe && ns <= 1024 && E <= 1024 && (d & 3) == 0) {   // dispatch, embedding and its bf16 copy: one launch
-        ctx->pdl = step > 0;   // after the previous step's argmax
-        ASCA_CUDA(ctx, asca_launch(ctx, decode_prologue_kernel, dim3((unsigned)ceil_div64(ns, 8)), dim3(256), 0, P + m->embed, cur, (int)ns,
-                                   (int)d, (int)E, x, x16, perm, offs, inv_perm));
+    if (f.one_prologue) {
+        ctx->pdl = pdl_first;   // after the previous step's argmax
+        ASCA_CUDA(ctx, asca_launch(ctx, decode_prologue_kernel, dim3((unsigned)ceil_div64(ns, 8)), dim3(256), 0, P + m->embed, b.cur, (int)ns,
+                                   (int)d, (int)E, b.x, b.x16, b.perm, b.offs, b.inv_perm, b.counter));
         ctx->launches++;
     } else {
-        ASCA_TRY(asca_moe_dispatch(ctx, cur, ns, E, perm, offs, nullptr));
-        ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, cur, ns, d, x));
-        if (sorted_moe) {
-            invert_perm_kernel<<<(unsigned)ceil_div64(ns, 256), 256, 0, ctx->stream>>>(perm, inv_perm, ns);
+        ASCA_TRY(asca_moe_dispatch(ctx, b.cur, ns, E, b.perm, b.offs, nullptr));
+        ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, b.cur, ns, d, b.x));
+        if (f.sorted_moe) {
+            invert_perm_kernel<<<(unsigned)ceil_div64(ns, 256), 256, 0, ctx->stream>>>(b.perm, b.inv_perm, ns);
             ASCA_CHECK_LAUNCH(ctx);
         }
-        ASCA_TRY(asca_cast_bf16(ctx, x, x16, ns * d));
+        ASCA_TRY(asca_cast_bf16(ctx, b.x, b.x16, ns * d));
     }
     // the block chain is short kernels back to back: each may become resident while its predecessor drains
     ctx->pdl = true;
     for (int64_t li = 0; li < m->L; ++li) {
         const Lyr& w = m->lay[li];
         const Lyr& w16 = m->lay16[li];
-        if (fused64) {
-            if (packed) ASCA_TRY(few_rows(x16, d, m->dec_pk + li * r_layer * 64, ldq, qg, ldq, m->dec_b + li * ldq));
-            else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, ldq, d, x16, d, m->dec_w + li * d * ldq, ldq, qg, ldq, m->dec_b + li * ldq, 0, BF));
-            ASCA_TRY(asca_delta_step_strided(ctx, qg, ldq, qg + 3 * d, ldq, state + li * ns * H * dh * dh, ns, H, o, o16));
+        if (f.fused64) {
+            if (f.packed) ASCA_TRY(few_rows(b.x16, d, m->dec_pk + li * f.r_layer * 64, ldq, b.qg, ldq, m->dec_b + li * ldq));
+            else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, ldq, d, b.x16, d, m->dec_w + li * d * ldq, ldq, b.qg, ldq, m->dec_b + li * ldq, 0, BF));
+            ASCA_TRY(asca_delta_step_strided(ctx, b.qg, ldq, b.qg + 3 * d, ldq, state + li * ns * H * dh * dh, ns, H, b.o, b.o16));
         } else {
-            ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 3 * d, d, x16, d, W + w16.w_qkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, BF));
-            ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 2 * H, d, x16, d, W + w16.w_gate, 2 * H, gate, 2 * H, P + w.b_gate, 0, BF));
-            ASCA_TRY(asca_delta_step(ctx, qkv, nullptr, nullptr, gate, nullptr, state + li * ns * H * dh * dh, ns, H, dh, 1, o));
-            ASCA_TRY(asca_cast_bf16(ctx, o, o16, ns * d));
+            ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 3 * d, d, b.x16, d, W + w16.w_qkv, 3 * d, b.qkv, 3 * d, P + w.b_qkv, 0, BF));
+            ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 2 * H, d, b.x16, d, W + w16.w_gate, 2 * H, b.gate, 2 * H, P + w.b_gate, 0, BF));
+            ASCA_TRY(asca_delta_step(ctx, b.qkv, nullptr, nullptr, b.gate, nullptr, state + li * ns * H * dh * dh, ns, H, dh, 1, b.o));
+            ASCA_TRY(asca_cast_bf16(ctx, b.o, b.o16, ns * d));
         }
-        if (packed) ASCA_TRY(few_rows(o16, d, m->dec_pk + (li * r_layer + r_qg) * 64, d, y, d, P + w.b_o));
-        else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, d, d, o16, d, W + w16.w_o, d, y, d, P + w.b_o, 0, BF));
-        if (sorted_moe) {
-            ASCA_TRY(asca_residual_rmsnorm_bf16_rows(ctx, x, y, x, xn16, ns, d, 1e-6f, inv_perm));   // x += y in place
-            const bf16* pk = m->dec_pk + (li * r_layer + r_qg + r_o) * 64;
-            ASCA_TRY(asca_moe_fwd_sorted_residual(ctx, xn16, packed ? pk : W + w16.w1, P + w.b1, packed ? pk + r_w1 * 64 : W + w16.w2,
-                                                  P + w.b2, perm, offs, ns, d, F, E, x, x16, hid16, 0, packed ? 1 : 0));
+        if (f.packed) ASCA_TRY(few_rows(b.o16, d, m->dec_pk + (li * f.r_layer + f.r_qg) * 64, d, b.y, d, P + w.b_o));
+        else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, d, d, b.o16, d, W + w16.w_o, d, b.y, d, P + w.b_o, 0, BF));
+        if (f.sorted_moe) {
+            ASCA_TRY(asca_residual_rmsnorm_bf16_rows(ctx, b.x, b.y, b.x, b.xn16, ns, d, 1e-6f, b.inv_perm));   // x += y in place
+            const bf16* pk = f.packed ? m->dec_pk + (li * f.r_layer + f.r_qg + f.r_o) * 64 : nullptr;
+            ASCA_TRY(asca_moe_fwd_sorted_residual(ctx, b.xn16, f.packed ? pk : W + w16.w1, P + w.b1, f.packed ? pk + f.r_w1 * 64 : W + w16.w2,
+                                                  P + w.b2, b.perm, b.offs, ns, d, F, E, b.x, b.x16, b.hid16, 0, f.packed ? 1 : 0));
             continue;
         }
-        ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, y, x_mid, xn16, ns, d, 1e-6f));
-        ASCA_TRY(asca_moe_fwd(ctx, xn16, W + w16.w1, P + w.b1, W + w16.w2, P + w.b2, perm, offs, ns, d, F, E, BF, mo, pre_p, hid16));
-        ASCA_CUDA(ctx, asca_launch(ctx, add_cast_kernel, dim3((unsigned)ceil_div64(ns * d, 256)), dim3(256), 0, x_mid, mo, x, x16,
+        ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, b.x, b.y, b.x_mid, b.xn16, ns, d, 1e-6f));
+        ASCA_TRY(asca_moe_fwd(ctx, b.xn16, W + w16.w1, P + w.b1, W + w16.w2, P + w.b2, b.perm, b.offs, ns, d, F, E, BF, b.mo, b.pre_p, b.hid16));
+        ASCA_CUDA(ctx, asca_launch(ctx, add_cast_kernel, dim3((unsigned)ceil_div64(ns * d, 256)), dim3(256), 0, b.x_mid, b.mo, b.x, b.x16,
                                    ns * d));   // x_out (+ bf16)
         ctx->launches++;
     }
-    ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, nullptr, nullptr, hf16, ns, d, 1e-6f));
-    if (packed) ASCA_TRY(few_rows(hf16, d, m->dec_pk + m->L * r_layer * 64, V, logits, V, nullptr));
-    else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, hf16, d, W + m->head16, V, logits, V, nullptr, 0, BF));
-    if (logits_h && step == n_steps - 1) {
-        ctx->pdl = false;   // a copy sits between the head product and the argmax
-        ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
+    ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, b.x, nullptr, nullptr, b.hf16, ns, d, 1e-6f));
+    if (f.packed) ASCA_TRY(few_rows(b.hf16, d, m->dec_pk + m->L * f.r_layer * 64, V, b.logits, V, nullptr));
+    else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, b.hf16, d, W + m->head16, V, b.logits, V, nullptr, 0, BF));
+    ASCA_CUDA(ctx, asca_launch(ctx, argmax_kernel, dim3((unsigned)ceil_div64(ns, 8)), dim3(256), 0, (const float*)b.logits, ns, (int)V, b.cur,
+                               f.one_prologue ? b.toks : toks_row, (const int32_t*)(f.one_prologue ? b.counter : nullptr)));
+    ctx->launches++;
+    return ASCA_OK;
+}
+
+static void drop_decode_plan(asca_ctx* ctx, asca_decode_plan& p) {
+    if (p.exec) cudaGraphExecDestroy(p.exec);
+    p.exec = nullptr;
+    if (ctx)
+        for (void* x : p.held) asca_free(ctx, x);
+    p.held.clear();
+}
+
+// Captures `body` (launches on ctx->stream) into an executable graph, on a stream of the context's own: the caller's may be
+// one that cannot be captured. Blocks the sequence gives back meanwhile go to `held`.
+template <class Body>
+static int capture(asca_ctx* ctx, cudaGraphExec_t* exec, int64_t* launches, std::vector<void*>* held, Body body) {
+    if (!ctx->cap_stream) ASCA_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
+    cudaStream_t user = ctx->stream;
+    const int64_t before = ctx->launches;
+    cudaGraph_t graph = nullptr;
+    std::vector<void*> got;
+    ctx->stream = ctx->cap_stream;
+    ctx->hold = &got;
+    int rc = cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeRelaxed) == cudaSuccess ? ASCA_OK : ASCA_ERR_CUDA;
+    if (rc == ASCA_OK) {
+        rc = body();
+        if (cudaStreamEndCapture(ctx->cap_stream, &graph) != cudaSuccess) rc = ASCA_ERR_CUDA;
     }
-    if (next_h || tokens_h || step + 1 < n_steps) {
-        ASCA_CUDA(ctx, asca_launch(ctx, argmax_kernel, dim3((unsigned)ceil_div64(ns, 8)), dim3(256), 0, (const float*)logits, ns, (int)V, nxt));
-        ctx->launches++;
+    ctx->hold = nullptr;
+    ctx->stream = user;
+    if (rc == ASCA_OK && cudaGraphInstantiate(exec, graph, 0) != cudaSuccess) rc = ASCA_ERR_CUDA;
+    if (graph) cudaGraphDestroy(graph);
+    *launches = ctx->launches - before;
+    ctx->launches = before;
+    if (rc != ASCA_OK) {
+        cudaGetLastError();
+        *exec = nullptr;
+        for (void* b : got) asca_free(ctx, b);
+        return rc;
     }
-    ctx->pdl = false;
-    }   // steps
-    if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4));
+    held->insert(held->end(), got.begin(), got.end());
+    return ASCA_OK;
+}
+
+// n_steps steps in bf16 mode. Step 0 consumes ids_h; a later step consumes the previous step's argmax, which never
+// leaves the device (tokens_h, n_steps x ns, receives all of them after the last step). One synchronisation at the end.
+static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* ids_h, int64_t ns, float* logits_h,
+                            uint32_t* next_h, int64_t n_steps = 1, uint32_t* tokens_h = nullptr) {
+    typedef __nv_bfloat16 bf16;
+    const int64_t d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab;
+    ASCA_TRY(refresh_params16(ctx, m));
+    ASCA_TRY(asca_dp_wait_all(ctx, m));
+    const float* P = m->params;
+    const bf16* W = m->params16;
+    asca_stage_scope staged(ctx);
+    Bufs bf(ctx);
+    DecodeForm f{};
+    f.ldq = (3 * d + 2 * H + 7) & ~(int64_t)7;
+    f.fused64 = dh == 64;
+    if (f.fused64) ASCA_TRY(refresh_dec_w(ctx, m));
+    f.sorted_moe = asca_moe_fwd_sorted_residual(ctx, W, W + m->lay16[0].w1, P + m->lay[0].b1, W + m->lay16[0].w2, P + m->lay[0].b2, nullptr, nullptr,
+                                                ns, d, F, E, nullptr, nullptr, nullptr, 1, 0) == ASCA_OK;
+    f.packed = f.fused64 && f.sorted_moe && ns <= 256;
+    f.one_prologue = f.sorted_moe && ns <= 1024 && E <= 1024 && (d & 3) == 0;
+    f.r_qg = gemm_tc::skinny_packed_rows(1, d, f.ldq); f.r_o = gemm_tc::skinny_packed_rows(1, d, d);
+    f.r_w1 = gemm_tc::skinny_packed_rows(E, d, F); f.r_w2 = gemm_tc::skinny_packed_rows(E, F, d);
+    f.r_layer = f.r_qg + f.r_o + f.r_w1 + f.r_w2; f.r_head = gemm_tc::skinny_packed_rows(1, d, V);
+    if (f.packed && !m->dec_pk) {
+        if (cudaMalloc((void**)&m->dec_pk, (size_t)(m->L * f.r_layer + f.r_head) * 128) != cudaSuccess)
+            return asca_fail(ctx, ASCA_ERR_OOM, "model: cannot allocate the decode weight copy");
+        m->dec_pk_stale = true;
+    }
+    if (f.packed && m->dec_pk_stale) {
+        for (int64_t li = 0; li < m->L; ++li) {
+            const Lyr& w16 = m->lay16[li];
+            bf16* pk = m->dec_pk + li * f.r_layer * 64;
+            ASCA_TRY(gemm_tc::skinny_pack(ctx, m->dec_w + li * d * f.ldq, f.ldq, 1, 0, 0, d, f.ldq, pk));
+            ASCA_TRY(gemm_tc::skinny_pack(ctx, W + w16.w_o, d, 1, 0, 0, d, d, pk + f.r_qg * 64));
+            ASCA_TRY(gemm_tc::skinny_pack(ctx, W + w16.w1, E * F, E, F, 0, d, F, pk + (f.r_qg + f.r_o) * 64));
+            ASCA_TRY(gemm_tc::skinny_pack(ctx, W + w16.w2, d, E, 0, F, F, d, pk + (f.r_qg + f.r_o + f.r_w1) * 64));
+        }
+        ASCA_TRY(gemm_tc::skinny_pack(ctx, W + m->head16, V, 1, 0, 0, d, V, m->dec_pk + m->L * f.r_layer * 64));
+        m->dec_pk_stale = false;
+    }
+    // A step is some eighty launches, each with its tensor maps: half a millisecond of host time, which is what a small batch's
+    // step takes. A (state, streams) pair that comes a third time is replayed as a graph, one launch a step.
+    asca_decode_plan* p = nullptr;
+    if (f.packed && f.one_prologue && !ctx->profiling) {
+        for (auto& q : m->dec_plans)
+            if (q.ns == ns && q.state == state && q.cap >= n_steps && q.w16 == W && q.dec_w == m->dec_w && q.dec_pk == m->dec_pk) p = &q;
+        if (!p) {
+            if (m->dec_plans.size() >= MAX_PLANS) {
+                size_t old = 0;
+                for (size_t i = 1; i < m->dec_plans.size(); ++i)
+                    if (m->dec_plans[i].stamp < m->dec_plans[old].stamp) old = i;
+                cudaStreamSynchronize(ctx->stream);
+                drop_decode_plan(ctx, m->dec_plans[old]);
+                m->dec_plans.erase(m->dec_plans.begin() + old);
+            }
+            asca_decode_plan q;
+            q.ns = ns; q.state = state; q.w16 = W; q.dec_w = m->dec_w; q.dec_pk = m->dec_pk;
+            q.cap = 1;
+            while (q.cap < n_steps) q.cap *= 2;
+            m->dec_plans.push_back(q);
+            p = &m->dec_plans.back();
+        }
+        p->stamp = ++m->plan_clock;
+        if (!p->exec && !p->broken && p->runs >= 2) {
+            DecodeBufs pb;
+            Bufs own(ctx);
+            int rc = pb.take(own, m, ns, p->cap) ? ASCA_OK : ASCA_ERR_OOM;
+            if (rc == ASCA_OK)
+                rc = capture(ctx, &p->exec, &p->launches, &p->held, [&] { return decode_step_bf16_device(ctx, m, f, pb, state, ns, false, nullptr); });
+            if (rc == ASCA_OK) {
+                p->held.insert(p->held.end(), own.p.begin(), own.p.end());   // the graph's buffers stay with it
+                own.p.clear();
+                p->cur = pb.cur; p->toks = pb.toks; p->counter = pb.counter; p->logits = pb.logits;
+            } else {
+                p->broken = true;
+            }
+        }
+        p->runs++;
+    }
+    uint32_t *cur, *toks;
+    float* logits;
+    if (p && p->exec) {
+        cur = p->cur; toks = p->toks; logits = p->logits;
+        ASCA_TRY(asca_stage_in(ctx, cur, ids_h, (size_t)ns * 4));
+        ASCA_CUDA(ctx, cudaMemsetAsync(p->counter, 0xff, 4, ctx->stream));
+        for (int64_t step = 0; step < n_steps; ++step) ASCA_CUDA(ctx, cudaGraphLaunch(p->exec, ctx->stream));
+        ctx->launches += p->launches * n_steps;
+    } else {
+        DecodeBufs b;
+        ASCA_REQUIRE(ctx, b.take(bf, m, ns, n_steps), "model_decode_step: out of memory");
+        cur = b.cur; toks = b.toks; logits = b.logits;
+        ASCA_TRY(asca_stage_in(ctx, cur, ids_h, (size_t)ns * 4));
+        ASCA_CUDA(ctx, cudaMemsetAsync(b.counter, 0xff, 4, ctx->stream));
+        for (int64_t step = 0; step < n_steps; ++step)
+            ASCA_TRY(decode_step_bf16_device(ctx, m, f, b, state, ns, step > 0, toks + step * ns));
+    }
+    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
+    if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, cur, (size_t)ns * 4));
     if (tokens_h) ASCA_TRY(asca_stage_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
@@ -1020,36 +1136,12 @@ static asca_step_plan* find_plan(asca_ctx* ctx, asca_model* m, int64_t B, int64_
     return &m->plans.back();
 }
 
-// Captures the step on a stream of its own (the caller's may be one that cannot be captured).
 static int capture_plan(asca_ctx* ctx, asca_model* m, asca_step_plan& p) {
-    if (!ctx->cap_stream) ASCA_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
-    cudaStream_t user = ctx->stream;
-    const int64_t before = ctx->launches;
-    cudaGraph_t graph = nullptr;
-    std::vector<void*> held;
-    ctx->stream = ctx->cap_stream;
-    ctx->hold = &held;
-    int rc = cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeRelaxed) == cudaSuccess ? ASCA_OK : ASCA_ERR_CUDA;
-    if (rc == ASCA_OK) {
-        rc = forward_backward_f32_device(ctx, m, p.ids, p.tg, p.B, p.T, p.acc, p.loss, p.logits);
-        if (cudaStreamEndCapture(ctx->cap_stream, &graph) != cudaSuccess) rc = ASCA_ERR_CUDA;
-    }
-    ctx->hold = nullptr;
-    ctx->stream = user;
-    if (rc == ASCA_OK && cudaGraphInstantiate(&p.exec, graph, 0) != cudaSuccess) rc = ASCA_ERR_CUDA;
-    if (graph) cudaGraphDestroy(graph);
-    p.launches = ctx->launches - before;
-    ctx->launches = before;
+    const int rc = capture(ctx, &p.exec, &p.launches, &p.held,
+                           [&] { return forward_backward_f32_device(ctx, m, p.ids, p.tg, p.B, p.T, p.acc, p.loss, p.logits); });
     p.ws_epoch = ctx->ws_epoch;
-    if (rc != ASCA_OK) {
-        cudaGetLastError();
-        p.exec = nullptr;
-        p.broken = true;
-        for (void* b : held) asca_free(ctx, b);
-        return rc;
-    }
-    p.held.insert(p.held.end(), held.begin(), held.end());
-    return ASCA_OK;
+    p.broken = rc != ASCA_OK;
+    return rc;
 }
 
 static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* ids_h, const uint32_t* tg_h, int64_t B, int64_t T, float* loss_h,
@@ -1204,6 +1296,7 @@ int asca_model_destroy(asca_ctx* ctx, asca_model* m) {
     if (!m) return ASCA_OK;
     if (ctx) cudaStreamSynchronize(ctx->stream);
     for (auto& p : m->plans) drop_plan(ctx, p);
+    for (auto& p : m->dec_plans) drop_decode_plan(ctx, p);
     if (m->dp) asca_dp_free(m);   // before the buffers its copies and collectives touch
     for (float* b : {m->params, m->grads, m->m, m->v})
         if (b) cudaFree(b);

@@ -30,6 +30,22 @@ struct asca_step_plan {
 };
 constexpr size_t MAX_PLANS = 8;
 
+// The same for a bf16 decode step on the packed weights: one graph is one step, its tokens in and out through `cur`.
+struct asca_decode_plan {
+    int64_t ns = 0, cap = 0;    // streams; tokens of how many steps `toks` holds
+    const void* state = nullptr;
+    const void *w16 = nullptr, *dec_w = nullptr, *dec_pk = nullptr;   // the weight copies the graph reads
+    uint32_t *cur = nullptr, *toks = nullptr;
+    int32_t* counter = nullptr;
+    float* logits = nullptr;
+    int runs = 0;
+    cudaGraphExec_t exec = nullptr;
+    bool broken = false;
+    uint64_t stamp = 0;
+    int64_t launches = 0;
+    std::vector<void*> held;
+};
+
 struct asca_model {
     int64_t vocab, d, H, L, E, F, n_params;
     int64_t embed, head;
@@ -67,6 +83,7 @@ struct asca_model {
     // it runs on CTA pairs and the caller does not ask for the logits (asca_model_set_fused_head)
     bool fused_head = true;
     std::vector<asca_step_plan> plans;
+    std::vector<asca_decode_plan> dec_plans;
     uint64_t plan_clock = 0;
     // data parallelism (dp.cu): the communicator attached to this model and what is in flight on its side stream
     asca_dp* dp = nullptr;
