@@ -675,8 +675,7 @@ inline cudaError_t launch_cfg(asca_ctx* ctx, Multi& m) {
 struct Shape {
     double slab, cta, cta_split, launch;
 };
-// The best estimate for one tile shape; split: how the problems' k is shared out (the longest problem's chain is halved as
-// long as that helps).
+// The best estimate for one tile shape; split: how the problems' k is shared out.
 template <class C>
 inline double estimate(const Multi& m, int n_sm, int max_split, const Shape& c, int (&split)[MAX_PROBLEMS]) {
     double tiles[MAX_PROBLEMS], slabs[MAX_PROBLEMS];
@@ -687,7 +686,7 @@ inline double estimate(const Multi& m, int n_sm, int max_split, const Shape& c, 
         if (p.mode == ASCA_TN && !p.A) continue;
         const double tn = (p.N + C::BN - 1) / C::BN, groups = p.group_dim == GROUP_NONE ? 1 : p.n_groups;
         const double mean = (double)p.total_rows / groups;   // token rows of a group
-        const double tm = std::ceil((p.group_dim == GROUP_M ? mean : (double)p.M) / C::BM);
+        const double tm = p.group_dim == GROUP_M ? mean / C::BM + 0.5 : std::ceil((double)p.M / C::BM);   // (ragged last tiles)
         const double k = (p.group_dim == GROUP_K ? mean : (double)p.K) + p.K2;
         tiles[i] = groups * tm * tn;
         slabs[i] = std::max(1.0, std::ceil(k / C::BK));
@@ -703,26 +702,23 @@ inline double estimate(const Multi& m, int n_sm, int max_split, const Shape& c, 
         }
         return ctas == 0.0 ? c.launch : c.launch + std::max(longest, std::ceil(ctas / n_sm) * work / ctas);
     };
-    double best = time();
-    for (;;) {
-        int at = 0;
-        for (int i = 1; i < m.n; ++i)
-            if (slabs[i] / split[i] > slabs[at] / split[at]) at = i;
-        if (split[at] >= max_split || slabs[at] < 2.0 * split[at]) return best;
-        // (twice may help where once does not: the barriers are paid with the first halving)
-        int keep = split[at], found = 0;
-        for (int s = split[at] * 2; s <= max_split; s *= 2) {
-            split[at] = s;
+    // every chain length a split can reach is tried as the bound for all problems (halving the longest one while that helps
+    // stops early where two problems are equally long: a 576 x 64 x 2048 gradient beside a short product took 34 us, 16 so)
+    double best = 1e300;
+    int found[MAX_PROBLEMS] = {};
+    for (int i = 0; i < m.n; ++i)
+        for (int s = 1; s <= max_split; s *= 2) {
+            const double bound = slabs[i] / s;
+            for (int j = 0; j < m.n; ++j)
+                for (split[j] = 1; split[j] < max_split && slabs[j] / split[j] > bound && slabs[j] >= 2.0 * split[j];) split[j] *= 2;
             const double t = time();
             if (t < best) {
                 best = t;
-                keep = s;
-                found = 1;
+                for (int j = 0; j < m.n; ++j) found[j] = split[j];
             }
         }
-        split[at] = keep;
-        if (!found) return best;
-    }
+    for (int j = 0; j < m.n; ++j) split[j] = found[j];
+    return best;
 }
 
 // Tile shape of a launch (0: 128, 1: 64, 2: 32 wide); fills in the k-splits.
