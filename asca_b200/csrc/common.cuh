@@ -45,6 +45,7 @@ struct asca_ctx {
         size_t at, bytes;
     };
     std::vector<PinOut> pin_out;
+    struct asca_hostcopy* hostcopy = nullptr;   // threads and pinned ring for large pageable arrays (hostcopy.cu)
     // Dynamic tile claims of the persistent tensor-core products (gemm_tc.cu; ASCA_GEMM_DYNAMIC=0 turns them off).
     // dyn_buf: two counters + the walkers' claim rings.
     void* dyn_buf = nullptr;
@@ -129,6 +130,11 @@ inline cudaError_t asca_launch(asca_ctx* ctx, void (*kern)(KArgs...), dim3 grid,
 constexpr size_t ASCA_PIN_BYTES = (size_t)1 << 20;
 int asca_stage_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
 int asca_stage_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
+// Any host array: small ones staged as above, large ones through the context's copy threads (hostcopy.cu). asca_copy_out
+// delivers large arrays before it returns.
+int asca_copy_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
+int asca_copy_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
+void asca_hostcopy_free(asca_ctx* ctx);
 // Drops what is staged (and waits for the copies that read it) when a call leaves without asca_ctx_sync.
 struct asca_stage_scope {
     asca_ctx* ctx;

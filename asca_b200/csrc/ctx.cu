@@ -62,6 +62,15 @@ int asca_stage_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
     return ASCA_OK;
 }
 
+// Waits for the stream and hands out what was staged.
+static int asca_stage_deliver(asca_ctx* ctx) {
+    ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    for (const auto& o : ctx->pin_out) memcpy(o.dst, ctx->pin + o.at, o.bytes);
+    ctx->pin_out.clear();
+    ctx->pin_used = 0;
+    return ASCA_OK;
+}
+
 asca_stage_scope::~asca_stage_scope() {
     if (ctx->pin_used == 0) return;   // asca_ctx_sync has delivered everything
     cudaStreamSynchronize(ctx->stream);
@@ -120,6 +129,7 @@ int asca_ctx_destroy(asca_ctx* ctx) {
     }
     if (ctx->err_word) cudaFree(ctx->err_word);
     if (ctx->pin) cudaFreeHost(ctx->pin);
+    asca_hostcopy_free(ctx);
     if (ctx->dyn_buf) cudaFree(ctx->dyn_buf);
     if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
     cudaStreamDestroy(ctx->own_stream);
@@ -153,10 +163,7 @@ int asca_ctx_sync(asca_ctx* ctx) {
     ASCA_TRY(stage_room(ctx, 4, &at));   // (allocates the area)
     int* word = reinterpret_cast<int*>(ctx->pin + ASCA_PIN_BYTES - 64);
     ASCA_CUDA(ctx, cudaMemcpyAsync(word, ctx->err_word, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    for (const auto& o : ctx->pin_out) memcpy(o.dst, ctx->pin + o.at, o.bytes);
-    ctx->pin_out.clear();
-    ctx->pin_used = 0;
+    ASCA_TRY(asca_stage_deliver(ctx));
     if (*word != 0) {
         cudaMemset(ctx->err_word, 0, sizeof(int));
         return asca_fail(ctx, ASCA_ERR_DEVICE, "a kernel gave up on a bounded wait (code %d)", *word);
@@ -173,6 +180,7 @@ int asca_ctx_trim(asca_ctx* ctx) {
     ctx->dtiles.clear();
     for (auto& kv : ctx->pool) cudaFree(kv.second);
     ctx->pool.clear();
+    asca_hostcopy_free(ctx);
     if (ctx->ws) cudaFree(ctx->ws);
     ctx->ws = nullptr;
     ctx->ws_bytes = 0;
@@ -266,15 +274,16 @@ int asca_free(asca_ctx* ctx, void* dptr) {
 
 int asca_memcpy_h2d(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!ctx) return ASCA_ERR_ARG;
-    ASCA_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    asca_stage_scope staged(ctx);   // (waits for what is staged)
+    ASCA_TRY(asca_copy_in(ctx, dst, src, bytes));
     ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return ASCA_OK;
 }
 int asca_memcpy_d2h(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!ctx) return ASCA_ERR_ARG;
-    ASCA_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return ASCA_OK;
+    asca_stage_scope staged(ctx);
+    ASCA_TRY(asca_copy_out(ctx, dst, src, bytes));
+    return asca_stage_deliver(ctx);
 }
 int asca_memset(asca_ctx* ctx, void* dst, int byte, size_t bytes) {
     if (!ctx) return ASCA_ERR_ARG;

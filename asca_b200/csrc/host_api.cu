@@ -10,7 +10,8 @@ namespace {
 struct Scope {
     asca_ctx* ctx;
     std::vector<void*> bufs;
-    explicit Scope(asca_ctx* c) : ctx(c) {}
+    asca_stage_scope staged;
+    explicit Scope(asca_ctx* c) : ctx(c), staged(c) {}
     ~Scope() {
         for (void* b : bufs) asca_free(ctx, b);
     }
@@ -22,8 +23,7 @@ struct Scope {
     int upload(const void* host, size_t bytes, void** out) {
         int rc = alloc(bytes, out);
         if (rc != ASCA_OK) return rc;
-        cudaError_t e = cudaMemcpyAsync(*out, host, bytes, cudaMemcpyHostToDevice, ctx->stream);
-        return e == cudaSuccess ? ASCA_OK : asca_fail(ctx, ASCA_ERR_CUDA, "H2D copy failed: %s", cudaGetErrorString(e));
+        return asca_copy_in(ctx, *out, host, bytes);
     }
     void keep(void* p) {  // ownership moves to a handle
         for (auto& b : bufs)
@@ -36,8 +36,7 @@ struct Scope {
 };
 
 int download(asca_ctx* ctx, void* host, const void* dev, size_t bytes) {
-    ASCA_CUDA(ctx, cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    return ASCA_OK;
+    return asca_copy_out(ctx, host, dev, bytes);
 }
 
 constexpr int64_t HOST_CHUNK = 64;  // checkpoint interval used by the host-form delta scan

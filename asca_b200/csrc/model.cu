@@ -661,9 +661,9 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         for (int64_t step = 0; step < n_steps; ++step)
             ASCA_TRY(decode_step_bf16_device(ctx, m, f, b, state, ns, step > 0, toks + step * ns));
     }
-    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
+    if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)ns * V * 4));
     if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, cur, (size_t)ns * 4));
-    if (tokens_h) ASCA_TRY(asca_stage_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
+    if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
 
@@ -683,7 +683,7 @@ static int decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t
     uint32_t* toks = (uint32_t*)bf.f(ns * n_steps);
     float* logits = bf.f(ns * V);
     ASCA_REQUIRE(ctx, ids && toks && logits, "model_decode_step: out of memory");
-    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)ns * 4));
+    ASCA_TRY(asca_copy_in(ctx, ids, ids_h, (size_t)ns * 4));
     int rc = asca_decode_f32(ctx, m, state, ids, ns, n_steps, toks, logits_h ? logits : nullptr);
     if (rc == ASCA_ERR_UNSUPPORTED) {   // step by step through the single kernels
         float *x = bf.f(ns * d), *qkv = bf.f(ns * 3 * d), *gate = bf.f(ns * 2 * H), *o = bf.f(ns * d), *y = bf.f(ns * d),
@@ -710,9 +710,9 @@ static int decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t
     } else {
         ASCA_TRY(rc);
     }
-    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
+    if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)ns * V * 4));
     if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4));
-    if (tokens_h) ASCA_TRY(asca_stage_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
+    if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
 
@@ -770,8 +770,8 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
     int32_t* offs = (int32_t*)bf.f(E + 1);
     ASCA_REQUIRE(ctx, ids && tg && perm && offs, "model_forward_backward: out of memory");
     asca_stage_scope staged(ctx);
-    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
-    ASCA_TRY(asca_stage_in(ctx, tg, tg_h, (size_t)N * 4));
+    ASCA_TRY(asca_copy_in(ctx, ids, ids_h, (size_t)N * 4));
+    ASCA_TRY(asca_copy_in(ctx, tg, tg_h, (size_t)N * 4));
     ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));
 
     struct Act {
@@ -860,7 +860,7 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
         ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
     } else {
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, V, d, h_final, d, W + m->head16, V, logits, V, nullptr, 0, BF));
-        if (logits_h) ASCA_CUDA(ctx, cudaMemcpyAsync(logits_h, logits, (size_t)N * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)N * V * 4));
         ASCA_TRY(cross_entropy_scaled(ctx, logits, tg, N, V, dlogits, loss_d, m->grad_scale));
         ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
         ASCA_TRY(asca_cast_bf16(ctx, dlogits, dl16, N * V));
@@ -1155,8 +1155,8 @@ static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* id
     uint32_t *ids = p ? p->ids : (uint32_t*)bf.f(N), *tg = p ? p->tg : (uint32_t*)bf.f(N);
     float *loss = p ? p->loss : bf.f(1), *logits = p ? p->logits : bf.f(N * V);
     ASCA_REQUIRE(ctx, ids && tg && loss && logits, "model_forward_backward: out of memory");
-    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
-    ASCA_TRY(asca_stage_in(ctx, tg, tg_h, (size_t)N * 4));
+    ASCA_TRY(asca_copy_in(ctx, ids, ids_h, (size_t)N * 4));
+    ASCA_TRY(asca_copy_in(ctx, tg, tg_h, (size_t)N * 4));
     if (p && p->exec && p->ws_epoch != ctx->ws_epoch) {   // the scratch its kernels name has moved
         cudaStreamSynchronize(ctx->stream);
         cudaGraphExecDestroy(p->exec);
@@ -1176,7 +1176,7 @@ static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* id
         ASCA_TRY(forward_backward_f32_device(ctx, m, ids, tg, B, T, acc, loss, logits));
     }
     ASCA_TRY(asca_stage_out(ctx, loss_h, loss, 4));
-    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)N * V * 4));
+    if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)N * V * 4));
     return asca_ctx_sync(ctx);
 }
 
@@ -1541,7 +1541,7 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
                           s_fin && xl && hf && logits && q && k && v && o && xn && hid_p && (!bfm || (x_in && hf_in)),
                  "model_prefill: out of memory");
     asca_stage_scope staged(ctx);
-    ASCA_TRY(asca_stage_in(ctx, ids, ids_h, (size_t)N * 4));
+    ASCA_TRY(asca_copy_in(ctx, ids, ids_h, (size_t)N * 4));
     std::vector<int32_t> lh(ns);
     for (int64_t s_ = 0; s_ < ns; ++s_) lh[s_] = (int32_t)(s_ * T + T - 1);
     ASCA_TRY(asca_stage_in(ctx, last, lh.data(), (size_t)ns * 4));
@@ -1581,7 +1581,7 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
         ASCA_TRY(asca_rmsnorm_fwd(ctx, xl, hf, nullptr, ns, d, 1e-6f));
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, V, d, hf, d, P + m->head, V, logits, V, nullptr, 0, DT));
     }
-    if (logits_h) ASCA_TRY(asca_stage_out(ctx, logits_h, logits, (size_t)ns * V * 4));
+    if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)ns * V * 4));
     if (next_h) {
         argmax_kernel<<<(unsigned)ceil_div64(ns, 8), 256, 0, ctx->stream>>>(logits, ns, (int)V, nxt);
         ASCA_CHECK_LAUNCH(ctx);

@@ -141,3 +141,46 @@ def test_f32_training_step_graph_equals_direct_launches(orc, gpu):
         m.free()
     for a, b in zip(*runs):
         assert np.array_equal(a, b)
+
+
+# Pageable host arrays around the sizes where the copies change form: staged, one piece more, one slot of the ring and one
+# byte more, more than the whole ring.
+@pytest.mark.parametrize("n", [1, 65536, 65537, 1 << 20, (1 << 20) + 1, (8 << 20) + 3, (19 << 20) + 70001])
+def test_host_copies(gpu, n):
+    import ctypes as C
+    import torch
+
+    src, back = np.random.default_rng(n).integers(0, 256, n).astype(np.uint8), np.zeros(n + 2, np.uint8)
+    buf = torch.zeros(n + 64, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        gpu._call("asca_memcpy_h2d", gpu._ctx, C.c_void_p(buf.data_ptr()), C.c_void_p(src.ctypes.data), C.c_size_t(n))
+        gpu._call("asca_memcpy_d2h", gpu._ctx, C.c_void_p(back.ctypes.data + 1), C.c_void_p(buf.data_ptr()), C.c_size_t(n))
+        assert np.array_equal(back[1:-1], src) and back[0] == back[-1] == 0
+        src = src[::-1].copy()
+    assert not buf[n:].any()
+
+
+# A repeated bf16 decode step is replayed as a graph; profiled calls launch directly. Same tokens and logits either way, for
+# two batch sizes in turn.
+def test_bf16_decode_graph_equals_direct_launches(orc, gpu):
+    import asca_b200
+
+    m = asca_b200.Model(gpu, 256, 128, 2, 2, 4, 256)
+    m.set_params(orc.Rng(9).normal(m.n, 0.05))
+    m.set_compute(asca_b200.BF16)
+    runs = []
+    for direct in (False, True):
+        gpu.profile(direct)
+        states = {ns: m.new_decode_state(ns) for ns in (5, 16)}
+        out = []
+        for step in range(6):
+            for ns, st in states.items():
+                out += list(m.decode_step(st, orc.Rng(step + ns).below(256, ns)))
+                if step % 2:
+                    out.append(m.decode_greedy(st, orc.Rng(step).below(256, ns), 3 + step))
+        gpu.profile(False)
+        runs.append(out)
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+    m.free()
