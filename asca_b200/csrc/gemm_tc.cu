@@ -8,12 +8,10 @@
 //   warp 1      allocates 256 TMEM columns = two accumulator buffers, and one thread issues
 //               tcgen05.mma (M128 N128 K16, 4 per k-tile) into the buffer of the current tile;
 //               tcgen05.commit releases ring slots and hands the finished buffer to the epilogue;
-//   warps 2-5   epilogue: tcgen05.ld the accumulator (each warp its 32-lane quarter), 32 columns at a
-//               time, through the warp's shared-memory staging rows so that global memory sees
-//               whole 64-byte row segments; bias / SiLU / SiLU' / accumulate are applied there;
-//               f32 output (and an optional bf16 second output), optionally through a row map (the
-//               un-permute scatter of the MoE combine). The buffer is released after the last
-//               tcgen05.ld, and the main loop of the next tile runs meanwhile in the other buffer.
+//   warps 2-5   epilogue (2-9 in the pair shape's eight-warp form): tcgen05.ld the accumulator (each warp its 32-lane quarter), 32
+//               columns of a row per lane; bias / SiLU / SiLU' / accumulate are applied in registers; f32 output (and an
+//               optional bf16 second output), optionally through a row map (the un-permute scatter of the MoE combine). The
+//               buffer is released after the last tcgen05.ld, and the main loop of the next tile runs meanwhile in the other.
 //
 // Operand majorness covers the three modes without any transposed copy: NN = A K-major, B
 // MN-major; TN = A MN-major, B MN-major; NT = A K-major, B K-major. Expert grouping: GROUP_M
@@ -43,9 +41,12 @@ constexpr int A_BYTES = BM * BK * 2;
 // PAIR: a cluster of two CTAs computes 256 x 256 tiles with cta_group::2 instructions (M = 256, N = 256). Each CTA
 // loads its own 128 rows of A and its own 128 of the tile's 256 B columns (32 KiB per k-tile for 4.2 MFLOP on this SM
 // against 48 KiB for the 128 x 256 tile and 32 KiB per 2.1 MFLOP for the 128 x 128 one): shared-memory traffic per
-// FLOP, which is what bounds the single-CTA shapes, halves. 6-stage ring, all 512 TMEM columns, one CTA per SM.
+// FLOP, which is what bounds the single-CTA shapes, halves. 7-stage ring, all 512 TMEM columns, one CTA per SM. What bounds its
+// main loop is the round trip of a stage (slot free -> load -> barrier -> instruction) against the ring's depth: the odd CTA's loads
+// complete on the even CTA's barrier (they used to be reported by a thread of the odd CTA) and the ring is as deep as shared
+// memory allows; 65,536 x 4096 x 1024 went from 433 to 400 us (1270 -> 1375 TFLOP/s).
 template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct Shape {
-    static constexpr int STAGES = PAIR ? 6 : BN == 128 ? (DEEP ? 6 : 3) : 4;
+    static constexpr int STAGES = PAIR ? 7 : BN == 128 ? (DEEP ? 7 : 3) : 4;   // (one fewer where the tile table needs the room)
     static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;      // two accumulator buffers
@@ -56,10 +57,9 @@ template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct
     // 128 columns are one head). Plain dense and k-grouped products are faster with four (1181 / 878 against 1056 / 781).
     static constexpr int EPI_WARPS = (PAIR && EW8) ? 8 : 4;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-    static constexpr size_t SMEM_FIXED = (size_t)STAGES * STAGE_BYTES + EPI_WARPS * 2048 /*epilogue staging*/ + 1024 /*alignment slack*/ +
-                                         256 /*barriers*/;   // + (groups + 2) * 4 for the tile table
+    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 256 /*barriers*/;   // + stages + tile table
 };
-constexpr int MAX_GROUPS = 2048;
+constexpr int MAX_GROUPS = 2048, MAX_STAGES = 8;
 
 struct KP {
     float* C;
@@ -96,12 +96,8 @@ struct KP {
     uint32_t dyn_seq;                  // launch number
     int dyn_batch;                     // consecutive tiles per claim (short tiles: one claim's latency per several tiles)
     int* err_word;
+    uint32_t stages;                   // ring depth: what the shared memory holds beside the tile table, at most MAX_STAGES
 };
-// 32-column accumulator loads issued per wait in the epilogue. 4 (128 registers) was measured on the four-warp shapes:
-// no gain (expert weight-gradient products at 512 rows per expert 1.09 against 1.05 ms, train step 335.6 against 334.4 ms).
-#ifndef ASCA_EPI_LG
-#define ASCA_EPI_LG 1
-#endif
 constexpr int DYN_Q = 16;              // claims a walker's producer can be ahead of its slowest role, with room to spare
 
 // bf16 mode only (2e-2 tolerance; the results are rounded to bf16 or multiply bf16 products): fast exp and divide.
@@ -112,26 +108,95 @@ __device__ __forceinline__ float silu_grad_f(float p) {
     return sg * (1.0f + p * (1.0f - sg));
 }
 
+// Up to 32 columns of a row between global memory and a lane's registers, `n` of them inside the matrix: 32 bytes at once where
+// every row starts on a 32-byte boundary (w = 8), else 16 (w = 4), else one element.
+__device__ __forceinline__ void load_row(float (&v)[32], const float* p, int n, int w) {
+    if (w == 8 && n >= 32) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+            asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=f"(v[j]), "=f"(v[j + 1]), "=f"(v[j + 2]), "=f"(v[j + 3]), "=f"(v[j + 4]), "=f"(v[j + 5]), "=f"(v[j + 6]), "=f"(v[j + 7])
+                         : "l"(p + j));
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        if (w >= 4 && j + 4 <= n) {
+            const float4 t = *reinterpret_cast<const float4*>(p + j);
+            v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
+        } else {
+#pragma unroll
+            for (int i = j; i < j + 4; ++i) v[i] = i < n ? p[i] : 0.0f;
+        }
+    }
+}
+__device__ __forceinline__ void store_row(float* p, const float (&v)[32], int n, int w) {
+    if (w == 8 && n >= 32) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+            asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                         ::"f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]), "f"(v[j + 4]), "f"(v[j + 5]), "f"(v[j + 6]), "f"(v[j + 7]),
+                         "l"(p + j)
+                         : "memory");
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        if (w >= 4 && j + 4 <= n) {
+            *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        } else {
+#pragma unroll
+            for (int i = j; i < j + 4; ++i)
+                if (i < n) p[i] = v[i];
+        }
+    }
+}
+__device__ __forceinline__ void store_row(__nv_bfloat16* p, const float (&v)[32], int n, int w) {
+    if (w >= 4 && n >= 32) {
+        uint32_t h[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            h[j] = *reinterpret_cast<const uint32_t*>(&t);
+        }
+        if (w == 8) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 8)
+                asm volatile("st.global.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                             ::"r"(h[j]), "r"(h[j + 1]), "r"(h[j + 2]), "r"(h[j + 3]), "r"(h[j + 4]), "r"(h[j + 5]), "r"(h[j + 6]), "r"(h[j + 7]),
+                             "l"(p + 2 * j)
+                             : "memory");
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(p + 2 * j) = make_uint4(h[j], h[j + 1], h[j + 2], h[j + 3]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+        if (j < n) p[j] = __float2bfloat16(v[j]);
+}
+
 template <int MODE, int BN, bool DEEP, bool PAIR, bool EW8>
 __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN, DEEP, PAIR, EW8>::CTAS_PER_SM) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                                                              const __grid_constant__ CUtensorMap mapB, const KP p) {
     constexpr bool A_MN = (MODE == ASCA_TN);   // A operand MN-major
     constexpr bool B_MN = (MODE != ASCA_NT);   // B operand MN-major
     using SH = Shape<BN, DEEP, PAIR, EW8>;
-    constexpr int STAGES = SH::STAGES, STAGE_BYTES = SH::STAGE_BYTES, TMEM_COLS = SH::TMEM_COLS;
+    constexpr int STAGE_BYTES = SH::STAGE_BYTES, TMEM_COLS = SH::TMEM_COLS;
+    const uint32_t STAGES = p.stages;
     constexpr int TM = PAIR ? 2 * BM : BM;       // rows of an output tile (both CTAs of a pair)
     constexpr int BNL = PAIR ? BN / 2 : BN;      // B columns this CTA loads per tile
     const int rank = PAIR ? (int)tc::cluster_ctarank() : 0;   // 0 = the CTA that issues the pair's instructions
     const int n_walkers = PAIR ? (int)gridDim.x / 2 : (int)gridDim.x, walker = PAIR ? (int)blockIdx.x / 2 : (int)blockIdx.x;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* staging = tiles + STAGES * STAGE_BYTES;                 // 4 epilogue warps x 2 KiB
-    uint64_t* full = reinterpret_cast<uint64_t*>(staging + SH::EPI_WARPS * 2048);
-    uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;     // [2] accumulator buffer written (MMA -> epilogue)
+    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES);
+    uint64_t* empty = full + MAX_STAGES;
+    uint64_t* acc_full = empty + MAX_STAGES; // [2] accumulator buffer written (MMA -> epilogue)
     uint64_t* acc_empty = acc_full + 2;      // [2] accumulator buffer read out (epilogue -> MMA)
-    uint64_t* peer_full = acc_empty + 2;     // [STAGES] PAIR, even CTA: the odd CTA's stage has landed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_full + STAGES);
+    uint64_t* peer_full = acc_empty + 2;     // [stage] PAIR, even CTA: the odd CTA has zeroed the ragged end of its k-tile
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_full + MAX_STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* prefix = const_cast<int*>(abort_flag) + 1;                  // [n_groups + 1] first tile of every group
 
@@ -168,7 +233,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         if (lane == 0) {
             prefix[n_groups] = base;
             *abort_flag = 0;
-            for (int s = 0; s < STAGES; ++s) {
+            for (uint32_t s = 0; s < STAGES; ++s) {
                 tc::mbar_init(&full[s], 1);
                 tc::mbar_init(&empty[s], 1);
                 tc::mbar_init(&peer_full[s], 1);
@@ -256,7 +321,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (one thread)
         if (lane == 0) {
-            uint32_t it = 0;   // k-tiles issued so far, across tiles: ring slot it % STAGES
+            uint32_t s = 0, round = 0;   // ring slot of the next k-tile and how often the ring has been around
             bool ok = true;
             // The claiming thread asks for claim ci + 1 before it loads claim ci's tiles and publishes it after them: the
             // atomic's round trip hides behind the loads, and no other role needs the next claim before this one is used up.
@@ -274,30 +339,39 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
               for (int t = t0; t < t0 + batch && t < total_tiles && ok; ++t) {
                 const Tile x = locate(t);
                 const int nl0 = x.n0 + rank * BNL;   // first B column this CTA loads
-                for (int kt = 0; kt < x.num_k; ++kt, ++it) {
-                    const int s = it % STAGES;
-                    if (it >= STAGES && !tc::mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag, p.err_word, 101)) {
+                for (int kt = 0; kt < x.num_k; ++kt) {
+                    if (round > 0 && !tc::mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.err_word, 101)) {
                         ok = false;
                         break;
                     }
                     uint8_t* a_s = tiles + s * STAGE_BYTES;
                     uint8_t* b_s = a_s + A_BYTES;
-                    tc::mbar_expect_tx(&full[s], STAGE_BYTES);
+                    // A pair's stage completes on the even CTA's barrier, for both CTAs' bytes at once. A ragged k-tile is zeroed
+                    // in part by each CTA first, so each waits for its own bytes.
+                    const bool joint = PAIR && !(p.group_dim == GROUP_K && kt + 1 == x.num_k && (x.K % BK) != 0);
+                    const uint32_t bar = tc::smem_u32(&full[s]), bar0 = joint && rank ? tc::mapa_u32(bar, 0) : bar;
+                    if (!joint) tc::mbar_expect_tx(&full[s], STAGE_BYTES);
+                    else if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                    auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1) {
+                        if (PAIR) tc::tma_load_2d_pair(dst, map, c0, c1, bar0);
+                        else tc::tma_load_2d(dst, map, c0, c1, &full[s]);
+                    };
                     const int k0 = kt * BK;
                     if (A_MN) {   // memory (k rows x M): two boxes of 64 columns
-                        tc::tma_load_2d(a_s, &mapA, x.m0, x.row_base_k + k0, &full[s]);
-                        tc::tma_load_2d(a_s + 8192, &mapA, x.m0 + 64, x.row_base_k + k0, &full[s]);
+                        load(a_s, &mapA, x.m0, x.row_base_k + k0);
+                        load(a_s + 8192, &mapA, x.m0 + 64, x.row_base_k + k0);
                     } else {      // memory (rows x K): one box 64 k x 128 rows
-                        tc::tma_load_2d(a_s, &mapA, k0, x.row_base_m + x.m0, &full[s]);
+                        load(a_s, &mapA, k0, x.row_base_m + x.m0);
                     }
                     if (B_MN) {   // memory (k rows x N)
                         const int kr = (MODE == ASCA_TN ? x.row_base_k : 0) + k0 + x.b_out;
 #pragma unroll
                         for (int nb = 0; nb < BNL / 64; ++nb)   // boxes of 64 columns
-                            tc::tma_load_2d(b_s + nb * 8192, &mapB, nl0 + nb * 64 + x.b_in, kr, &full[s]);
+                            load(b_s + nb * 8192, &mapB, nl0 + nb * 64 + x.b_in, kr);
                     } else {      // memory (N rows x K)
-                        tc::tma_load_2d(b_s, &mapB, k0 + x.b_in, nl0 + x.b_out, &full[s]);
+                        load(b_s, &mapB, k0 + x.b_in, nl0 + x.b_out);
                     }
+                    if (++s == STAGES) s = 0, ++round;
                 }
               }
                 if (claimer) {   // (after a wait that gave up: "none left", so that the walker's other roles stop too)
@@ -318,7 +392,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         const uint32_t a_lo0 = ((tc::smem_u32(tiles) >> 4) & 0x3FFF) | (A_LBO << 16);
         const uint32_t b_lo0 = (((tc::smem_u32(tiles) + A_BYTES) >> 4) & 0x3FFF) | (B_LBO << 16);
         bool ok = true;
-        uint32_t it = 0;
+        uint32_t s = 0, par = 0;         // ring slot and parity of the next k-tile (kept by every lane)
+        uint32_t rag_own = 0, rag_peer = 0;   // PAIR: parity of every slot's next ragged k-tile (odd CTA: full; even CTA: peer_full)
         int tl = 0;   // tiles done by this CTA: accumulator buffer tl & 1
         for (int ci = 0;; ++ci) {
             int t0 = lane == 0 && ok ? read_tile(ci) : -1;
@@ -330,58 +405,60 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             const uint32_t tmem_acc = tmem_base + buf * BN;
             const bool ragged = p.group_dim == GROUP_K && (x.K % BK) != 0;   // warp-uniform
             const int n_plain = ragged ? x.num_k - 1 : x.num_k;
-            if (PAIR && rank == 1) {
-                // the odd CTA issues nothing: it tells the even CTA when each of its stages has landed
-                if (lane == 0) {
-                    for (int kt = 0; kt < n_plain && ok; ++kt, ++it) {
-                        const uint32_t s = it % STAGES;
-                        ok = tc::mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, p.err_word, 105);
-                        if (ok) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&peer_full[s]), 0));
-                    }
+            auto next = [&] {
+                if (++s == STAGES) s = 0, par ^= 1;
+            };
+            auto issue = [&](int kt) {   // the even CTA's (or the only) lane 0: one k-tile's instructions, slot release, tile hand-over
+                const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = b_lo0 + s * (STAGE_BYTES >> 4);
+#pragma unroll
+                for (int k16 = 0; k16 < BK / 16; ++k16) {
+                    const uint64_t da = ((uint64_t)DESC_HI << 32) | (a_lo + k16 * A_K16), db = ((uint64_t)DESC_HI << 32) | (b_lo + k16 * B_K16);
+                    if (PAIR) tc::umma_bf16_pair(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
+                    else tc::umma_bf16(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
                 }
-            } else if (lane == 0) {
+                if (PAIR) {
+                    tc::umma_commit_pair(&empty[s]);              // the slot is free in both CTAs once these MMAs retire
+                    if (kt == x.num_k - 1) tc::umma_commit_pair(&acc_full[buf]);
+                } else {
+                    tc::umma_commit(&empty[s]);                   // slot free once these MMAs retire
+                    if (kt == x.num_k - 1) tc::umma_commit(&acc_full[buf]);
+                }
+            };
+            if (lane == 0 && rank == 0) {
                 if (tl >= 2) {   // the epilogue (of both CTAs) has read this buffer's previous tile out
                     ok = PAIR ? tc::mbar_wait_cluster(&acc_empty[buf], ((tl >> 1) - 1) & 1, abort_flag, p.err_word, 104)
                               : tc::mbar_wait(&acc_empty[buf], ((tl >> 1) - 1) & 1, abort_flag, p.err_word, 104);
                 }
                 tc::tcgen05_fence_after();
-                for (int kt = 0; kt < n_plain && ok; ++kt, ++it) {
-                    const uint32_t s = it % STAGES;
-                    ok = tc::mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, p.err_word, 102);
-                    if (ok && PAIR) ok = tc::mbar_wait_cluster(&peer_full[s], (it / STAGES) & 1, abort_flag, p.err_word, 106);
+                for (int kt = 0; kt < n_plain && ok; ++kt) {
+                    ok = tc::mbar_wait(&full[s], par, abort_flag, p.err_word, 102);
                     if (!ok) break;
                     tc::tcgen05_fence_after();
-                    const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = b_lo0 + s * (STAGE_BYTES >> 4);
-#pragma unroll
-                    for (int k16 = 0; k16 < BK / 16; ++k16) {
-                        const uint64_t da = ((uint64_t)DESC_HI << 32) | (a_lo + k16 * A_K16), db = ((uint64_t)DESC_HI << 32) | (b_lo + k16 * B_K16);
-                        if (PAIR) tc::umma_bf16_pair(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
-                        else tc::umma_bf16(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
-                    }
-                    if (PAIR) {
-                        tc::umma_commit_pair(&empty[s]);              // the slot is free in both CTAs once these MMAs retire
-                        if (kt == x.num_k - 1) tc::umma_commit_pair(&acc_full[buf]);
-                    } else {
-                        tc::umma_commit(&empty[s]);                   // slot free once these MMAs retire
-                        if (kt == x.num_k - 1) tc::umma_commit(&acc_full[buf]);
-                    }
+                    issue(kt);
+                    next();
+                }
+            }
+            if (p.group_dim == GROUP_K) {   // (the other lanes and the odd CTA need the slot for ragged k-tiles only)
+                if (rank == 1) {
+                    const uint32_t at = s + (uint32_t)n_plain;
+                    par ^= (at / STAGES) & 1;
+                    s = at % STAGES;
+                } else {
+                    s = __shfl_sync(0xffffffffu, s, 0);
+                    par = __shfl_sync(0xffffffffu, par, 0);
                 }
             }
             if (ragged) {
-                // last k-tile of this expert: rows >= K - kt*BK belong to the next expert and are zeroed by the whole warp
+                // last k-tile of this expert: rows >= K - kt*BK belong to the next expert and are zeroed by the whole warp,
+                // in each CTA's own half; the odd CTA then reports to the issuer
                 const int kt = x.num_k - 1;
                 int got = 0;
-                if (lane == 0) {
-                    got = ok && tc::mbar_wait(&full[(it) % STAGES], ((it) / STAGES) & 1, abort_flag, p.err_word, 102) ? 1 : 0;
-                    if (got && PAIR && rank == 0)   // the odd CTA zeroes its own tile before it reports the stage
-                        got = tc::mbar_wait_cluster(&peer_full[(it) % STAGES], ((it) / STAGES) & 1, abort_flag, p.err_word, 106) ? 1 : 0;
-                }
+                if (lane == 0) got = ok && tc::mbar_wait(&full[s], rank == 1 ? (rag_own >> s) & 1 : par, abort_flag, p.err_word, 105) ? 1 : 0;
+                rag_own ^= 1u << s;
                 got = __shfl_sync(0xffffffffu, got, 0);
-                const uint32_t it_r = __shfl_sync(0xffffffffu, it, 0);
                 ok = got != 0;
                 if (ok) {
                     tc::tcgen05_fence_after();
-                    const uint32_t s = it_r % STAGES;
                     uint8_t* a_s = tiles + s * STAGE_BYTES;
                     const int valid = x.K - kt * BK;
                     const int lines = (BK - valid) * 2;  // 128-byte lines in the two A boxes
@@ -396,24 +473,16 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                         if (PAIR && rank == 1) {
                             tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&peer_full[s]), 0));
                         } else {
-                            const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = b_lo0 + s * (STAGE_BYTES >> 4);
-#pragma unroll
-                            for (int k16 = 0; k16 < BK / 16; ++k16) {
-                                const uint64_t da = ((uint64_t)DESC_HI << 32) | (a_lo + k16 * A_K16), db = ((uint64_t)DESC_HI << 32) | (b_lo + k16 * B_K16);
-                                if (PAIR) tc::umma_bf16_pair(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
-                                else tc::umma_bf16(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
-                            }
-                            if (PAIR) {
-                                tc::umma_commit_pair(&empty[s]);
-                                tc::umma_commit_pair(&acc_full[buf]);
-                            } else {
-                                tc::umma_commit(&empty[s]);
-                                tc::umma_commit(&acc_full[buf]);
+                            if (PAIR) ok = tc::mbar_wait_cluster(&peer_full[s], (rag_peer >> s) & 1, abort_flag, p.err_word, 106);
+                            if (ok) {
+                                tc::tcgen05_fence_after();
+                                issue(kt);
                             }
                         }
-                        ++it;
                     }
+                    rag_peer ^= 1u << s;
                 }
+                next();
             }
             if (lane == 0 && ok && x.num_k == 0 && rank == 0) {   // empty expert: the epilogue stores zeros
                 tc::mbar_arrive(&acc_full[buf]);
@@ -423,20 +492,30 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
           }
         }
     } else {
-        // ------------------------------------------------------------ epilogue (warps 2..5)
-        // Each warp owns the 32 accumulator rows of its TMEM lane quarter and moves them 32 columns at a time:
-        // tcgen05.ld (one row per lane) -> the warp's 2 KiB of shared memory, 16 columns per pass -> global
-        // memory with 4 lanes on each row's 64 bytes, where bias, activation and accumulation are applied. The TMEM buffer is
-        // released after the last tcgen05.ld; the next tile's main loop runs meanwhile in the other buffer.
+        // ------------------------------------------------------------ epilogue (warps 2..5, EW8: 2..9)
+        // A lane holds a row: tcgen05.ld hands it 32 columns of its row, bias / activation / accumulation are applied to those
+        // 32 independent values, and they leave as 32-byte stores -- whole sectors, so neither a transpose through shared memory nor
+        // row maps and ragged rows (a lane's own address, a lane's own predicate) cost anything. What bounds an epilogue of one
+        // or two warps per scheduler is the latency of its instructions, not the bytes: hence the 32-wide straight-line code and
+        // the loads of `aux` / of the old C two column groups ahead, the first of them before the accumulator is awaited. Measured on the
+        // expert products of 65,536 tokens, 1024 -> 4096 (two outputs, SiLU; SiLU' with its f32 read), whose tiles have 6 us of main
+        // loop: 1076 -> 691 us and 1166 -> 725 us. The TMEM buffer is released after the last tcgen05.ld; the next tile's main loop runs
+        // meanwhile in the other buffer.
         const int q = warp & 3;                 // TMEM lane quarter this warp may read
         const int ew = warp - 2;                // epilogue warp index; warps ew and ew + 4 share lane quarter q
-        constexpr int C_PER_WARP = (BN / 32) / (SH::EPI_WARPS / 4);   // 32-column passes of a row per warp
+        constexpr int C_PER_WARP = (BN / 32) / (SH::EPI_WARPS / 4);   // 32-column groups of a row per warp
         const int c_lo = (ew >> 2) * C_PER_WARP;
-        float4* stg = reinterpret_cast<float4*>(staging + ew * 2048);   // [32 rows][4 float4], index XOR ((row >> 1) & 3)
-        const bool c_vec = ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) && ((p.c_gstride & 3) == 0);
-        const bool c2_vec = p.C2 && ((p.ldc2 & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C2) & 7) == 0);
-        const bool aux_vec = p.aux && ((p.ldaux & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.aux) & 15) == 0);
-        const int l4 = lane & 3, rsub = lane >> 2;   // store phase: 4 lanes per row (64 bytes), 8 rows per instruction
+        // elements a lane may move at once: 8 (32 bytes), 4 or 1
+        auto width = [](const void* base, int64_t ld, int64_t gstride, int unit) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(base) | (uintptr_t)(ld * unit) | (uintptr_t)(gstride * unit);
+            return (a & 31) == 0 ? 8 : (a & 15) == 0 ? 4 : 1;
+        };
+        const int c_w = width(p.C, p.ldc, p.group_dim == GROUP_K ? p.c_gstride : 0, 4);
+        const int aux_w = width(p.aux, p.ldaux, 0, 4);
+        const int bias_w = width(p.bias, 0, p.bias_gstride, 4);
+        const int c2_w = width(p.C2, p.ldc2, 0, 2);
+        const int qkv_w = min(width(p.qkv_q, p.qkv_d, 0, 2), min(width(p.qkv_k, 0, 0, 2), width(p.qkv_v, 0, 0, 2)));
+        const bool with_aux = p.epi == EPI_SILU_BWD;
         bool ok = true;
         int tl = 0;
         for (int ci = 0; ok; ++ci) {
@@ -446,7 +525,22 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
           for (int t = t0; t < t0 + batch && t < total_tiles; ++t, ++tl) {
             const Tile x = locate(t);
             const int buf = tl & 1;
-            const uint32_t tmem_acc = tmem_base + buf * BN;
+            const uint32_t tmem_acc = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
+            const bool live = x.M - (x.m0 + q * 32) > lane;   // rows past the matrix's or the expert's end are computed, not stored
+            const int64_t lr = (int64_t)x.row_base_m + x.m0 + (live ? q * 32 + lane : 0);
+            const int64_t cr = p.c_idx && live ? (int64_t)p.c_idx[lr] : lr;
+            float* crow = p.C + (p.group_dim == GROUP_K ? (int64_t)x.g * p.c_gstride : 0) + cr * p.ldc + x.n0;
+            const float* arow = p.aux + lr * p.ldaux + x.n0;
+            const float* brow = p.bias ? p.bias + (int64_t)x.g * p.bias_gstride + x.n0 : nullptr;
+            // aux, or where there is none the old C, two column groups ahead
+            const float* prow = with_aux ? arow : crow;
+            const bool ahead = live && (with_aux || p.accumulate);
+            const int p_w = with_aux ? aux_w : c_w;
+            float pre[2][32];
+            if (ahead) {
+#pragma unroll
+                for (int g = 0; g < 2; ++g) load_row(pre[g], prow + (c_lo + g) * 32, p.N - x.n0 - (c_lo + g) * 32, p_w);
+            }
             int got = 0;
             if (lane == 0)
                 got = (PAIR ? tc::mbar_wait_cluster(&acc_full[buf], (tl >> 1) & 1, abort_flag, p.err_word, 103)
@@ -454,25 +548,20 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             ok = __shfl_sync(0xffffffffu, got, 0) != 0;  // uniform: tcgen05.ld below is warp-aligned
             if (!ok) break;
             tc::tcgen05_fence_after();
-            float* cbase = p.C + (p.group_dim == GROUP_K ? (int64_t)x.g * p.c_gstride : 0);
-            const int rows_here = x.M - (x.m0 + q * 32);   // live rows of this warp's quarter (may be <= 0 or > 32)
-            // the common case gets straight-line code: full tile, plain f32 output (bias and accumulate allowed)
             // fused qkv epilogue (pair shape, whole tiles: the launcher checks): this warp's 128 columns are one head of q, k or v
             const bool qkv = PAIR && EW8 && p.epi == EPI_QKV;
             float qkv_scale = 1.0f;                 // 1 / max(|z|, 1e-8) of this lane's row (q, k), 1 for v
-            __nv_bfloat16* c2p = p.C2;
-            int64_t ldc2 = p.ldc2;
+            __nv_bfloat16* hrow = p.C2 + lr * p.ldc2 + x.n0;
             if (qkv) {
                 const int hc0 = x.n0 + c_lo * 32;   // first column of the head
                 const int sec = hc0 / p.qkv_d;      // 0 q, 1 k, 2 v
-                c2p = (sec == 0 ? p.qkv_q : sec == 1 ? p.qkv_k : p.qkv_v) - sec * p.qkv_d;   // column = global column - sec d
-                ldc2 = p.qkv_d;
+                hrow = (sec == 0 ? p.qkv_q : sec == 1 ? p.qkv_k : p.qkv_v) + lr * p.qkv_d + (x.n0 - sec * p.qkv_d);
                 if (sec < 2) {
                     float ss = 0.0f;
 #pragma unroll 1
                     for (int c = c_lo; c < c_lo + C_PER_WARP; ++c) {
                         uint32_t r[32];
-                        tc::tmem_ld_32x32(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), r);
+                        tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), r);
                         tc::tmem_ld_wait();
                         const float4* bb = reinterpret_cast<const float4*>(p.bias + x.n0 + c * 32);
 #pragma unroll
@@ -486,7 +575,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     const float nrm = fmaxf(sqrtf(ss), 1e-8f);
                     qkv_scale = 1.0f / nrm;
                     const int heads = p.qkv_d / 128, head = (hc0 - sec * p.qkv_d) / 128;
-                    (sec == 0 ? p.qkv_qn : p.qkv_kn)[((int64_t)x.m0 + q * 32 + lane) * heads + head] = nrm;
+                    (sec == 0 ? p.qkv_qn : p.qkv_kn)[lr * heads + head] = nrm;
                 }
             }
             // fused cross-entropy (pair shape, four epilogue warps: a warp's lanes hold whole rows of 256 logits)
@@ -494,13 +583,12 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             float ce_max = 0.0f, ce_inv = 0.0f;
             int ce_t = 0;
             if (ce) {
-                const int64_t row = (int64_t)x.m0 + q * 32 + lane;
-                ce_t = (int)p.ce_targets[row];
+                ce_t = (int)p.ce_targets[lr];
                 float mx = -INFINITY, sum = 0.0f, zt = 0.0f;
 #pragma unroll 1
                 for (int c = 0; c < BN / 32; ++c) {   // online max / sum of exponentials over the row
                     uint32_t r[32];
-                    tc::tmem_ld_32x32(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), r);
+                    tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), r);
                     tc::tmem_ld_wait();
                     float cm = mx;
 #pragma unroll
@@ -515,41 +603,26 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     sum = sum * expf(mx - cm) + part;
                     mx = cm;
                 }
-                p.ce_loss[row] = (mx + logf(sum)) - zt;
+                p.ce_loss[lr] = (mx + logf(sum)) - zt;
                 ce_max = mx;
                 ce_inv = 1.0f / sum;
             }
-            const bool fast = qkv || ce || (c_vec && !p.c_idx && (!p.C2 || (p.c2_only && c2_vec)) && p.epi == EPI_NONE && rows_here >= 32 && x.n0 + BN <= p.N &&
-                              (!p.bias || (((reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) && (p.bias_gstride & 3) == 0)));
-            float* frow = cbase + ((int64_t)x.row_base_m + x.m0 + q * 32 + rsub) * p.ldc + x.n0 + 4 * l4;   // row rsub, this lane's columns
-            const float* fbias = (p.bias && !qkv) ? p.bias + (int64_t)x.g * p.bias_gstride + x.n0 + 4 * l4 : nullptr;
-            // row bookkeeping of the 4 store iterations: row = 8 * i + rsub
-            int64_t lrs[4], crs[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int rr = 8 * i + rsub;
-                lrs[i] = (int64_t)x.row_base_m + x.m0 + (rr < rows_here ? q * 32 + rr : 0);
-                crs[i] = p.c_idx && rr < rows_here ? (int64_t)p.c_idx[lrs[i]] : lrs[i];
-            }
-            // LG 32-column loads are issued together and waited for once: a tcgen05.ld queues behind the MMAs the issuer
-            // has in flight for the next tile, and one wait per load pays that queue once per 32 columns.
-            constexpr int LG = (SH::CTAS_PER_SM == 2 || EW8) ? 1 : ASCA_EPI_LG;   // (two CTAs per SM, or 320 threads: no room for 128 more registers)
-            static_assert(C_PER_WARP % LG == 0, "epilogue load groups");
-#pragma unroll 1
-            for (int cg = c_lo; cg < c_lo + C_PER_WARP; cg += LG) {
-                uint32_t rr[LG][32];
+            const bool c_out = !(p.c2_only || qkv || ce), h_out = qkv || ce || p.C2;
+            const int h_w = qkv ? qkv_w : c2_w;
+#pragma unroll 2
+            for (int c = c_lo; c < c_lo + C_PER_WARP; ++c) {
+                float v[32];
                 if (x.num_k > 0) {
-#pragma unroll
-                    for (int g = 0; g < LG; ++g)
-                        tc::tmem_ld_32x32(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)((cg + g) * 32), rr[g]);
+                    uint32_t r[32];
+                    tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), r);
                     tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
                 } else {
 #pragma unroll
-                    for (int g = 0; g < LG; ++g)
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) rr[g][j] = 0u;
+                    for (int j = 0; j < 32; ++j) v[j] = 0.0f;
                 }
-                if (cg + LG == c_lo + C_PER_WARP) {   // this warp's share of the buffer is free for the tile after next
+                if (c + 1 == c_lo + C_PER_WARP) {   // this warp's share of the buffer is free for the tile after next
                     tc::tcgen05_fence_before();
                     __syncwarp();
                     if (lane == 0) {
@@ -557,147 +630,49 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                         else tc::mbar_arrive(&acc_empty[buf]);
                     }
                 }
-#pragma unroll
-              for (int g = 0; g < LG; ++g) {
-                const int c = cg + g;
-                uint32_t(&r)[32] = rr[g];
+                const int n_left = p.N - x.n0 - c * 32;   // columns of the matrix from here on
+                if (n_left <= 0) continue;
                 if (ce) {    // dlogits = (softmax - onehot) * scale
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        float pr = expf(__uint_as_float(r[j]) - ce_max) * ce_inv;
+                        float pr = expf(v[j] - ce_max) * ce_inv;
                         if (c * 32 + j == ce_t) pr -= 1.0f;
-                        r[j] = __float_as_uint(pr * p.ce_scale);
+                        v[j] = pr * p.ce_scale;
                     }
                 }
-                if (qkv) {   // bias, then the row's scale, on the f32 accumulators (lane = row)
-                    const float4* bb = reinterpret_cast<const float4*>(p.bias + x.n0 + c * 32);
+                if (brow) {
+                    float b[32];
+                    load_row(b, brow + c * 32, n_left, bias_w);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float4 b4 = bb[j];
-                        r[4 * j] = __float_as_uint((__uint_as_float(r[4 * j]) + b4.x) * qkv_scale);
-                        r[4 * j + 1] = __float_as_uint((__uint_as_float(r[4 * j + 1]) + b4.y) * qkv_scale);
-                        r[4 * j + 2] = __float_as_uint((__uint_as_float(r[4 * j + 2]) + b4.z) * qkv_scale);
-                        r[4 * j + 3] = __float_as_uint((__uint_as_float(r[4 * j + 3]) + b4.w) * qkv_scale);
-                    }
+                    for (int j = 0; j < 32; ++j) v[j] += b[j];
                 }
+                if (qkv) {
 #pragma unroll
-                for (int hlf = 0; hlf < 2; ++hlf) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        stg[lane * 4 + (j ^ ((lane >> 1) & 3))] =
-                            make_float4(__uint_as_float(r[16 * hlf + 4 * j]), __uint_as_float(r[16 * hlf + 4 * j + 1]),
-                                        __uint_as_float(r[16 * hlf + 4 * j + 2]), __uint_as_float(r[16 * hlf + 4 * j + 3]));
-                    __syncwarp();
-                    if (fast) {
-                        const int co = c * 32 + hlf * 16;
-                        float4 b4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), acc4[4], old4[4];
-                        if (fbias) b4 = *reinterpret_cast<const float4*>(fbias + co);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            acc4[i] = stg[(8 * i + rsub) * 4 + (l4 ^ (((8 * i + rsub) >> 1) & 3))];
-                            old4[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            if (p.accumulate) old4[i] = *reinterpret_cast<const float4*>(frow + (int64_t)(8 * i) * p.ldc + co);
-                        }
-                        if (p.c2_only || qkv || ce) {   // bf16 is all the consumer reads
-                            __nv_bfloat16* hrow = c2p + ((int64_t)x.row_base_m + x.m0 + q * 32 + rsub) * ldc2 + x.n0 + 4 * l4 + co;
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const __nv_bfloat162 lo2 = __floats2bfloat162_rn(acc4[i].x + b4.x, acc4[i].y + b4.y),
-                                                     hi2 = __floats2bfloat162_rn(acc4[i].z + b4.z, acc4[i].w + b4.w);
-                                *reinterpret_cast<uint2*>(hrow + (int64_t)(8 * i) * ldc2) =
-                                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo2), *reinterpret_cast<const uint32_t*>(&hi2));
-                            }
-                            __syncwarp();
-                            continue;
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            *reinterpret_cast<float4*>(frow + (int64_t)(8 * i) * p.ldc + co) =
-                                make_float4(acc4[i].x + b4.x + old4[i].x, acc4[i].y + b4.y + old4[i].y,
-                                            acc4[i].z + b4.z + old4[i].z, acc4[i].w + b4.w + old4[i].w);
-                        __syncwarp();
-                        continue;
-                    }
-                    const int nb = x.n0 + c * 32 + hlf * 16 + 4 * l4;   // this lane's 4 columns in the store phase
-                    if (nb < p.N) {
-                        const bool full4 = nb + 4 <= p.N;
-                        float bias4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                        if (p.bias) {
-                            const float* bias = p.bias + (int64_t)x.g * p.bias_gstride;
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                if (nb + j < p.N) bias4[j] = bias[nb + j];
-                        }
-                        float4 aux4[4], old4[4];   // every global load of the pass is issued before any is used
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            aux4[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            old4[i] = aux4[i];
-                            if (8 * i + rsub >= rows_here) continue;
-                            if (p.epi == EPI_SILU_BWD) {
-                                const float* ax = p.aux + lrs[i] * p.ldaux + nb;
-                                if (full4 && aux_vec) aux4[i] = *reinterpret_cast<const float4*>(ax);
-                                else {
-                                    aux4[i].x = ax[0];
-                                    if (nb + 1 < p.N) aux4[i].y = ax[1];
-                                    if (nb + 2 < p.N) aux4[i].z = ax[2];
-                                    if (nb + 3 < p.N) aux4[i].w = ax[3];
-                                }
-                            }
-                            if (p.accumulate) {
-                                const float* crow = cbase + crs[i] * p.ldc + nb;
-                                if (full4 && c_vec) old4[i] = *reinterpret_cast<const float4*>(crow);
-                                else {
-                                    old4[i].x = crow[0];
-                                    if (nb + 1 < p.N) old4[i].y = crow[1];
-                                    if (nb + 2 < p.N) old4[i].z = crow[2];
-                                    if (nb + 3 < p.N) old4[i].w = crow[3];
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int rr = 8 * i + rsub;
-                            if (rr >= rows_here) continue;
-                            const float4 acc4 = stg[rr * 4 + (l4 ^ ((rr >> 1) & 3))];
-                            float v[4] = {acc4.x + bias4[0], acc4.y + bias4[1], acc4.z + bias4[2], acc4.w + bias4[3]};
-                            if (p.epi == EPI_SILU_BWD) {
-                                v[0] *= silu_grad_f(aux4[i].x); v[1] *= silu_grad_f(aux4[i].y);
-                                v[2] *= silu_grad_f(aux4[i].z); v[3] *= silu_grad_f(aux4[i].w);
-                            }
-                            v[0] += old4[i].x; v[1] += old4[i].y; v[2] += old4[i].z; v[3] += old4[i].w;
-                            float* crow = cbase + crs[i] * p.ldc + nb;
-                            if (p.c2_only) {
-                                // bf16 output only
-                            } else if (full4 && c_vec) {
-                                *reinterpret_cast<float4*>(crow) = make_float4(v[0], v[1], v[2], v[3]);
-                            } else {
-#pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    if (nb + j < p.N) crow[j] = v[j];
-                            }
-                            if (p.C2) {
-                                __nv_bfloat16* c2 = p.C2 + lrs[i] * p.ldc2 + nb;
-                                float y[4] = {v[0], v[1], v[2], v[3]};
-                                if (p.epi == EPI_SILU) {
-#pragma unroll
-                                    for (int j = 0; j < 4; ++j) y[j] = silu_f(y[j]);
-                                }
-                                if (full4 && c2_vec) {
-                                    const __nv_bfloat162 lo2 = __floats2bfloat162_rn(y[0], y[1]), hi2 = __floats2bfloat162_rn(y[2], y[3]);
-                                    *reinterpret_cast<uint2*>(c2) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo2),
-                                                                               *reinterpret_cast<const uint32_t*>(&hi2));
-                                } else {
-#pragma unroll
-                                    for (int j = 0; j < 4; ++j)
-                                        if (nb + j < p.N) c2[j] = __float2bfloat16(y[j]);
-                                }
-                            }
-                        }
-                    }
-                    __syncwarp();   // every lane is done with the staging rows before the next pass overwrites them
+                    for (int j = 0; j < 32; ++j) v[j] *= qkv_scale;
                 }
-              }
+                if (with_aux) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] *= silu_grad_f(pre[(c - c_lo) & 1][j]);
+                    if (p.accumulate && live) {
+                        float old[32];
+                        load_row(old, crow + c * 32, n_left, c_w);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] += old[j];
+                    }
+                } else if (p.accumulate) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] += pre[(c - c_lo) & 1][j];
+                }
+                if (ahead && c + 2 < c_lo + C_PER_WARP) load_row(pre[(c - c_lo) & 1], prow + (c + 2) * 32, n_left - 64, p_w);
+                if (!live) continue;
+                if (c_out) store_row(crow + c * 32, v, n_left, c_w);
+                if (h_out) {
+                    if (p.epi == EPI_SILU) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = silu_f(v[j]);
+                    }
+                    store_row(hrow + c * 32, v, n_left, h_w);
+                }
             }
           }
         }
@@ -806,9 +781,11 @@ static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid, int64_t tile
         }
     }
     using SH = Shape<BN, DEEP, PAIR, EW8>;
-    const size_t smem = SH::SMEM_FIXED + (size_t)(2 * (a.group_dim == GROUP_NONE ? 1 : a.n_groups) + 4) * 4;   // tile table + group offsets
+    const size_t table = (size_t)(2 * (a.group_dim == GROUP_NONE ? 1 : a.n_groups) + 4) * 4;   // tile table + group offsets
+    p.stages = (uint32_t)std::min<size_t>(SH::STAGES, (ctx->smem_optin - SH::SMEM_FIXED - table) / SH::STAGE_BYTES);
+    const size_t smem = SH::SMEM_FIXED + p.stages * SH::STAGE_BYTES + table;
     auto go = [&](auto kern) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SH::SMEM_FIXED + (2 * MAX_GROUPS + 4) * 4));
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         if (!PAIR) return asca_launch(ctx, kern, dim3((unsigned)grid), dim3(SH::THREADS), smem, mapA, mapB, p);
         // pairs of CTAs: a cluster of two per walker (grid = 2 x walkers)
@@ -901,12 +878,15 @@ int launch(asca_ctx* ctx, const Args& a) {
     return launch_shape<128, false>(ctx, a, std::min<int64_t>(grid, 2 * n_sm), grid);
 }
 
+// A pair runs a 256 x 256 tile 1.6 times as fast as two SMs run its four quarters in the 128 x 128 shape (two CTAs an SM), so pairs win
+// from half of them busy on; below that, each quarter has an SM of its own in the deep 128 x 128 form. With 64 tiles (1024 x 65,536 x
+// 4096, A^T B): 906 -> 402 us. Rows grouped by expert need 512 rows an expert, or padding to 256 rows costs more than that.
 static bool pair_wanted(asca_ctx* ctx, const Args& a) {
     const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
     const int64_t pairs = tile_bound(a, 256, 256);
     static const bool pair_rows = [] { const char* e = getenv("ASCA_GEMM_PAIR"); return !(e && e[0] == '1'); }();
     const bool pair_shape = a.group_dim == GROUP_M ? (pair_rows && a.total_rows >= 512 * (int64_t)a.n_groups) : a.M >= 256;
-    return pair_enabled() && pair_shape && a.N >= 256 && pairs >= n_sm / 2;
+    return pair_enabled() && pair_shape && a.N >= 256 && (a.group_dim == GROUP_M ? pairs >= n_sm / 2 : pairs > n_sm / 4);
 }
 
 }  // namespace gemm_tc

@@ -165,6 +165,14 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
                                                   int code) {
     return mbar_wait(bar, parity, abort_flag, err_word, code);
 }
+// Tile load into this CTA's shared memory that completes on a barrier of either CTA of the pair (a shared::cluster address):
+// the even CTA's issuer then waits once for both CTAs' bytes. Not a multicast: one destination.
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int c_inner, int c_outer, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(c_inner), "r"(c_outer), "r"(cluster_bar)
+        : "memory");
+}
 // D[tmem of both CTAs] (+)= A * B over the CTA pair; issued by ONE thread of the even CTA.
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                uint32_t accumulate) {
