@@ -47,7 +47,7 @@ struct asca_ctx {
     std::vector<PinOut> pin_out;
     struct asca_hostcopy* hostcopy = nullptr;   // threads and pinned ring for large pageable arrays (hostcopy.cu)
     // Dynamic tile claims of the persistent tensor-core products (gemm_tc.cu; ASCA_GEMM_DYNAMIC=0 turns them off).
-    // dyn_buf: two counters + the walkers' claim rings.
+    // dyn_buf: two counters, used in turn.
     void* dyn_buf = nullptr;
     uint32_t dyn_seq = 0;
     // tiles of the tensor-core delta forwards that wrote checkpoints, kept for their backwards: one entry per

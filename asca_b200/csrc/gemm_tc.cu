@@ -5,7 +5,7 @@
 //   warp 0      TMA producer: one thread streams 128x64 A and 64x128 B bf16 tiles (128-byte
 //               swizzle, plain non-multicast cp.async.bulk.tensor) through a 3-stage ring of
 //               mbarriers, running ahead across tile boundaries;
-//   warp 1      allocates 256 TMEM columns = two accumulator buffers, and one thread issues
+//   warp 1      allocates two accumulator buffers in TMEM, and one thread issues
 //               tcgen05.mma (M128 N128 K16, 4 per k-tile) into the buffer of the current tile;
 //               tcgen05.commit releases ring slots and hands the finished buffer to the epilogue;
 //   warps 2-5   epilogue (2-9 in the pair shape's eight-warp form): tcgen05.ld the accumulator (each warp its 32-lane quarter), 32
@@ -33,9 +33,7 @@ namespace {
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
 // Two tile shapes. 128 x 128: 3-stage ring, 256 TMEM columns, two CTAs per SM (two independent MMA streams keep the
-// tensor pipe fed). 128 x 256: one M128 N256 K16 instruction does twice the work of an N128 one for the same issue
-// latency, so a single stream per SM suffices: 4-stage ring of 48 KiB, all 512 TMEM columns, one CTA per SM. It is
-// used when the problem has at least two waves of such tiles.
+// tensor pipe fed).
 // DEEP: a problem of at most one 128 x 128 tile per SM (a decode step's products) runs one CTA per SM with a
 // 6-stage ring: its k-loop streams weights that are cold in L2, and three stages do not cover the HBM latency.
 // PAIR: a cluster of two CTAs computes 256 x 256 tiles with cta_group::2 instructions (M = 256, N = 256). Each CTA
@@ -46,18 +44,18 @@ constexpr int A_BYTES = BM * BK * 2;
 // complete on the even CTA's barrier (they used to be reported by a thread of the odd CTA) and the ring is as deep as shared
 // memory allows; 65,536 x 4096 x 1024 went from 433 to 400 us (1270 -> 1375 TFLOP/s).
 template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct Shape {
-    static constexpr int STAGES = PAIR ? 7 : BN == 128 ? (DEEP ? 7 : 3) : 4;   // (one fewer where the tile table needs the room)
+    static constexpr int STAGES = PAIR || DEEP ? 7 : 3;   // (one fewer where the tile table needs the room)
     static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;      // two accumulator buffers
-    static constexpr int CTAS_PER_SM = (BN == 128 && !DEEP) ? 2 : 1;
+    static constexpr int CTAS_PER_SM = PAIR || DEEP ? 1 : 2;
     // epilogue warps: one per TMEM lane quarter. EW8 (pair shape): two warps share each quarter and split the 256 columns
     // -- for the row-grouped expert products, whose epilogues (activation, two outputs, row scatter) would otherwise
     // outlast the main loop (837 against 603 TFLOP/s inside the training step), and for the fused qkv epilogue (a warp's
     // 128 columns are one head). Plain dense and k-grouped products are faster with four (1181 / 878 against 1056 / 781).
     static constexpr int EPI_WARPS = (PAIR && EW8) ? 8 : 4;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 256 /*barriers*/;   // + stages + tile table
+    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 384 /*barriers, claims*/;   // + stages + tile table
 };
 constexpr int MAX_GROUPS = 2048, MAX_STAGES = 8;
 
@@ -88,24 +86,27 @@ struct KP {
     // or a CTA pair -- takes the next unclaimed tile whenever it starts one, so CTAs that find their SM occupied by
     // another stream's kernels (a collective running beside the step) simply claim fewer tiles instead of holding the
     // launch up with a fixed share. The producer thread of the walker's first CTA claims (atomicAdd) and publishes the
-    // claim in a small ring in global memory, tagged with launch and claim number; every other role of the walker, and
-    // the pair's second CTA, read it from there.
+    // claim in a small ring in the shared memory of both CTAs, tagged with its number; every other role reads it from
+    // there (through global memory the read took 2,000 of an epilogue's 22,000 cycles a tile).
     int* dyn_ctr;                      // this launch's counter (zero at launch)
     int* dyn_reset;                    // the next launch's counter, zeroed by this launch
-    unsigned long long* dyn_ring;      // [walkers][DYN_Q] (tag << 32 | tile)
-    uint32_t dyn_seq;                  // launch number
-    int dyn_batch;                     // consecutive tiles per claim (short tiles: one claim's latency per several tiles)
     int* err_word;
     uint32_t stages;                   // ring depth: what the shared memory holds beside the tile table, at most MAX_STAGES
 };
 constexpr int DYN_Q = 16;              // claims a walker's producer can be ahead of its slowest role, with room to spare
 
-// bf16 mode only (2e-2 tolerance; the results are rounded to bf16 or multiply bf16 products): fast exp and divide.
-// A 128 x 128 tile applies these 16 k times, which with the accurate forms costs more than the tile's main loop.
-__device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+// bf16 mode only (2e-2 tolerance; the results are rounded to bf16 or multiply bf16 products): the hardware's base-2 exponential
+// and reciprocal without the denormal handling around them, 5 and 7 instructions. An epilogue is bound by its instructions.
+__device__ __forceinline__ float sigmoid_f(float x) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return r;
+}
+__device__ __forceinline__ float silu_f(float x) { return x * sigmoid_f(x); }
 __device__ __forceinline__ float silu_grad_f(float p) {
-    const float sg = __fdividef(1.0f, 1.0f + __expf(-p));
-    return sg * (1.0f + p * (1.0f - sg));
+    const float sg = sigmoid_f(p);
+    return sg * fmaf(p, 1.0f - sg, 1.0f);
 }
 
 // Up to 32 columns of a row between global memory and a lane's registers, `n` of them inside the matrix: 32 bytes at once where
@@ -198,7 +199,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
     uint64_t* peer_full = acc_empty + 2;     // [stage] PAIR, even CTA: the odd CTA has zeroed the ragged end of its k-tile
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_full + MAX_STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* prefix = const_cast<int*>(abort_flag) + 1;                  // [n_groups + 1] first tile of every group
+    volatile unsigned long long* claims = reinterpret_cast<volatile unsigned long long*>(tmem_slot + 2);   // [DYN_Q] (number + 1) << 32 | tile
+    int* prefix = reinterpret_cast<int*>(const_cast<unsigned long long*>(claims) + DYN_Q);             // [n_groups + 1] first tile of every group
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_n = (p.N + BN - 1) / BN;
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         if (lane == 0) {
             prefix[n_groups] = base;
             *abort_flag = 0;
+            for (int i = 0; i < DYN_Q; ++i) claims[i] = 0;
             for (uint32_t s = 0; s < STAGES; ++s) {
                 tc::mbar_init(&full[s], 1);
                 tc::mbar_init(&empty[s], 1);
@@ -288,26 +291,24 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
 
     // The i-th tile of this walker (-1: none left). claim_tile is for the walker's claiming thread only.
     const bool dyn = p.dyn_ctr != nullptr;
-    unsigned long long* dyn_slot0 = dyn ? p.dyn_ring + (size_t)walker * DYN_Q : nullptr;
-    auto dyn_tag = [&](int i) { return p.dyn_seq * 4096u + (uint32_t)(i & 4095); };
-    const int batch = dyn ? p.dyn_batch : 1;
-    auto publish_claim = [&](int i, int t) {   // claim i = tiles [t, t + batch) (-1: none left)
+    auto publish_claim = [&](int i, int t) {   // claim i = tile t (-1: none left)
         if (t >= total_tiles) t = -1;
-        const unsigned long long v = ((unsigned long long)dyn_tag(i) << 32) | (uint32_t)t;
-        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(dyn_slot0 + (i % DYN_Q)), "l"(v) : "memory");
+        const unsigned long long v = ((unsigned long long)(uint32_t)(i + 1) << 32) | (uint32_t)t;
+        claims[i % DYN_Q] = v;
+        if (PAIR)
+            asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;"
+                         ::"r"(tc::mapa_u32(tc::smem_u32(const_cast<unsigned long long*>(claims + i % DYN_Q)), 1)), "l"(v)
+                         : "memory");
     };
     auto read_tile = [&](int i) -> int {   // one thread polls; bounded like every other wait of the kernel
         if (!dyn) {
             const int t = walker + i * n_walkers;
             return t < total_tiles ? t : -1;
         }
-        const unsigned long long* e = dyn_slot0 + (i % DYN_Q);
-        const uint32_t want = dyn_tag(i);
         const long long t0 = clock64();
         while (true) {
-            unsigned long long v;
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(e) : "memory");
-            if ((uint32_t)(v >> 32) == want) return (int)(uint32_t)v;
+            const unsigned long long v = claims[i % DYN_Q];
+            if ((uint32_t)(v >> 32) == (uint32_t)(i + 1)) return (int)(uint32_t)v;
             if (*abort_flag) return -1;
             if (clock64() - t0 > tc::WAIT_LIMIT_CYCLES) {
                 *abort_flag = 1;
@@ -323,23 +324,27 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         if (lane == 0) {
             uint32_t s = 0, round = 0;   // ring slot of the next k-tile and how often the ring has been around
             bool ok = true;
-            // The claiming thread asks for claim ci + 1 before it loads claim ci's tiles and publishes it after them: the
+            // The claiming thread asks for claim ci + 1 half way through claim ci's loads and publishes it after them: the
             // atomic's round trip hides behind the loads, and no other role needs the next claim before this one is used up.
+            // (Not earlier: with about as many tiles as walkers the first to start would take two each, 190 us against 110 for
+            // 64 tiles.)
             const bool claimer = dyn && rank == 0;
             int cur = 0;
             if (claimer) {
-                cur = atomicAdd(p.dyn_ctr, batch);
+                cur = atomicAdd(p.dyn_ctr, 1);
                 publish_claim(0, cur);
             }
             for (int ci = 0; ok; ++ci) {
-                const int t0 = claimer ? (cur < total_tiles ? cur : -1) : read_tile(ci);
-                if (t0 < 0) break;
+                const int t = claimer ? (cur < total_tiles ? cur : -1) : read_tile(ci);
+                if (t < 0) break;
                 int nxt = 0;
-                if (claimer) nxt = atomicAdd(p.dyn_ctr, batch);
-              for (int t = t0; t < t0 + batch && t < total_tiles && ok; ++t) {
                 const Tile x = locate(t);
                 const int nl0 = x.n0 + rank * BNL;   // first B column this CTA loads
+                // (a tile without k-tiles takes no ring slot: the claims of a run of them wait for the epilogue instead)
+                if (claimer && x.num_k == 0 && ci >= 2) ok = tc::mbar_wait(&acc_empty[ci & 1], ((ci >> 1) - 1) & 1, abort_flag, p.err_word, 108);
+                if (claimer && x.num_k == 0) nxt = atomicAdd(p.dyn_ctr, 1);
                 for (int kt = 0; kt < x.num_k; ++kt) {
+                    if (claimer && kt == x.num_k / 2) nxt = atomicAdd(p.dyn_ctr, 1);
                     if (round > 0 && !tc::mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.err_word, 101)) {
                         ok = false;
                         break;
@@ -373,7 +378,6 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     }
                     if (++s == STAGES) s = 0, ++round;
                 }
-              }
                 if (claimer) {   // (after a wait that gave up: "none left", so that the walker's other roles stop too)
                     cur = ok ? nxt : total_tiles;
                     publish_claim(ci + 1, cur);
@@ -394,12 +398,10 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         bool ok = true;
         uint32_t s = 0, par = 0;         // ring slot and parity of the next k-tile (kept by every lane)
         uint32_t rag_own = 0, rag_peer = 0;   // PAIR: parity of every slot's next ragged k-tile (odd CTA: full; even CTA: peer_full)
-        int tl = 0;   // tiles done by this CTA: accumulator buffer tl & 1
-        for (int ci = 0;; ++ci) {
-            int t0 = lane == 0 && ok ? read_tile(ci) : -1;
-            t0 = __shfl_sync(0xffffffffu, t0, 0);
-            if (t0 < 0) break;
-          for (int t = t0; t < t0 + batch && t < total_tiles && ok; ++t, ++tl) {
+        for (int tl = 0;; ++tl) {   // tiles done by this CTA: accumulator buffer tl & 1
+            int t = lane == 0 && ok ? read_tile(tl) : -1;
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t < 0) break;
             const Tile x = locate(t);
             const int buf = tl & 1;
             const uint32_t tmem_acc = tmem_base + buf * BN;
@@ -489,7 +491,6 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                 if (PAIR) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&acc_full[buf]), 1));
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;   // lane 0's verdict; keeps the warp's tile loops in step
-          }
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5, EW8: 2..9)
@@ -497,9 +498,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         // 32 independent values, and they leave as 32-byte stores -- whole sectors, so neither a transpose through shared memory nor
         // row maps and ragged rows (a lane's own address, a lane's own predicate) cost anything. What bounds an epilogue of one
         // or two warps per scheduler is the latency of its instructions, not the bytes: hence the 32-wide straight-line code and
-        // the loads of `aux` / of the old C two column groups ahead, the first of them before the accumulator is awaited. Measured on the
+        // the loads of `aux` / of the old C a column group or two ahead, the first before the accumulator is awaited. Measured on the
         // expert products of 65,536 tokens, 1024 -> 4096 (two outputs, SiLU; SiLU' with its f32 read), whose tiles have 6 us of main
-        // loop: 1076 -> 691 us and 1166 -> 725 us. The TMEM buffer is released after the last tcgen05.ld; the next tile's main loop runs
+        // loop: 1076 -> 670 us and 1166 -> 730 us. The TMEM buffer is released after the last tcgen05.ld; the next tile's main loop runs
         // meanwhile in the other buffer.
         const int q = warp & 3;                 // TMEM lane quarter this warp may read
         const int ew = warp - 2;                // epilogue warp index; warps ew and ew + 4 share lane quarter q
@@ -517,12 +518,10 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         const int qkv_w = min(width(p.qkv_q, p.qkv_d, 0, 2), min(width(p.qkv_k, 0, 0, 2), width(p.qkv_v, 0, 0, 2)));
         const bool with_aux = p.epi == EPI_SILU_BWD;
         bool ok = true;
-        int tl = 0;
-        for (int ci = 0; ok; ++ci) {
-            int t0 = lane == 0 ? read_tile(ci) : -1;
-            t0 = __shfl_sync(0xffffffffu, t0, 0);
-            if (t0 < 0) break;
-          for (int t = t0; t < t0 + batch && t < total_tiles; ++t, ++tl) {
+        for (int tl = 0; ok; ++tl) {
+            int t = lane == 0 ? read_tile(tl) : -1;
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t < 0) break;
             const Tile x = locate(t);
             const int buf = tl & 1;
             const uint32_t tmem_acc = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
@@ -532,15 +531,18 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             float* crow = p.C + (p.group_dim == GROUP_K ? (int64_t)x.g * p.c_gstride : 0) + cr * p.ldc + x.n0;
             const float* arow = p.aux + lr * p.ldaux + x.n0;
             const float* brow = p.bias ? p.bias + (int64_t)x.g * p.bias_gstride + x.n0 : nullptr;
-            // aux, or where there is none the old C, two column groups ahead
+            // aux, or where there is none the old C, ahead of their use
             const float* prow = with_aux ? arow : crow;
             const bool ahead = live && (with_aux || p.accumulate);
             const int p_w = with_aux ? aux_w : c_w;
-            float pre[2][32];
+            constexpr int AHEAD = PAIR && !EW8 ? 2 : 1;   // (registers: 255 with four epilogue warps, 168 with eight)
+            float pre[AHEAD][32];
             if (ahead) {
 #pragma unroll
-                for (int g = 0; g < 2; ++g) load_row(pre[g], prow + (c_lo + g) * 32, p.N - x.n0 - (c_lo + g) * 32, p_w);
+                for (int g = 0; g < AHEAD; ++g) load_row(pre[g], prow + (c_lo + g) * 32, p.N - x.n0 - (c_lo + g) * 32, p_w);
             }
+            if (brow && lane < C_PER_WARP && x.n0 + (c_lo + lane) * 32 < p.N)   // this warp's bias on its way into L1
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(brow + (c_lo + lane) * 32));
             int got = 0;
             if (lane == 0)
                 got = (PAIR ? tc::mbar_wait_cluster(&acc_full[buf], (tl >> 1) & 1, abort_flag, p.err_word, 103)
@@ -609,19 +611,22 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             }
             const bool c_out = !(p.c2_only || qkv || ce), h_out = qkv || ce || p.C2;
             const int h_w = qkv ? qkv_w : c2_w;
-#pragma unroll 2
-            for (int c = c_lo; c < c_lo + C_PER_WARP; ++c) {
+            // A tcgen05.ld takes about 1,000 cycles beside the next tile's instructions, so the next group's is under way while one is
+            // processed. (Unrolled to the end: what it loads may not pass through a loop's register moves before the wait. The four-warp
+            // form, which takes the cross-entropy alone, loads in turn.)
+            constexpr bool TWO = C_PER_WARP <= 4;
+            uint32_t acc[TWO ? 2 : 1][32];
+            if (TWO) tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c_lo * 32), acc[0]);
+#pragma unroll(TWO ? C_PER_WARP : 2)
+            for (int i = 0; i < C_PER_WARP; ++i) {
+                const int c = c_lo + i;
+                const int n_left = p.N - x.n0 - c * 32;   // columns of the matrix from here on
                 float v[32];
-                if (x.num_k > 0) {
-                    uint32_t r[32];
-                    tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), r);
-                    tc::tmem_ld_wait();
+                if (!TWO) tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), acc[0]);
+                tc::tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = 0.0f;
-                }
+                for (int j = 0; j < 32; ++j) v[j] = x.num_k > 0 ? __uint_as_float(acc[TWO ? i & 1 : 0][j]) : 0.0f;
+                if (TWO && i + 1 < C_PER_WARP) tc::tmem_ld_32x32(tmem_acc + (uint32_t)((c + 1) * 32), acc[(i + 1) & 1]);
                 if (c + 1 == c_lo + C_PER_WARP) {   // this warp's share of the buffer is free for the tile after next
                     tc::tcgen05_fence_before();
                     __syncwarp();
@@ -630,7 +635,6 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                         else tc::mbar_arrive(&acc_empty[buf]);
                     }
                 }
-                const int n_left = p.N - x.n0 - c * 32;   // columns of the matrix from here on
                 if (n_left <= 0) continue;
                 if (ce) {    // dlogits = (softmax - onehot) * scale
 #pragma unroll
@@ -652,7 +656,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                 }
                 if (with_aux) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] *= silu_grad_f(pre[(c - c_lo) & 1][j]);
+                    for (int j = 0; j < 32; ++j) v[j] *= silu_grad_f(pre[i % AHEAD][j]);
                     if (p.accumulate && live) {
                         float old[32];
                         load_row(old, crow + c * 32, n_left, c_w);
@@ -661,9 +665,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     }
                 } else if (p.accumulate) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] += pre[(c - c_lo) & 1][j];
+                    for (int j = 0; j < 32; ++j) v[j] += pre[i % AHEAD][j];
                 }
-                if (ahead && c + 2 < c_lo + C_PER_WARP) load_row(pre[(c - c_lo) & 1], prow + (c + 2) * 32, n_left - 64, p_w);
+                if (ahead && i + AHEAD < C_PER_WARP) load_row(pre[i % AHEAD], prow + (c + AHEAD) * 32, n_left - 32 * AHEAD, p_w);
                 if (!live) continue;
                 if (c_out) store_row(crow + c * 32, v, n_left, c_w);
                 if (h_out) {
@@ -674,7 +678,6 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     store_row(hrow + c * 32, v, n_left, h_w);
                 }
             }
-          }
         }
     }
     // ---- teardown: everyone meets, then the allocating warp frees TMEM
@@ -737,7 +740,7 @@ bool supported(const Args& a) {
 }
 
 template <int BN, bool DEEP, bool PAIR = false, bool EW8 = false>
-static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid, int64_t tiles_est) {
+static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid) {
     CUtensorMap mapA, mapB;
     bool ok;
     if (a.mode == ASCA_TN) ok = make_map(&mapA, a.A, a.a_rows, a.a_cols, a.lda, 64, 64);
@@ -759,25 +762,18 @@ static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid, int64_t tile
         static const int dyn_env = [] { const char* e = getenv("ASCA_GEMM_DYNAMIC"); return e ? atoi(e) : 1; }();
         const bool want = dyn_env != 0;   // on unless ASCA_GEMM_DYNAMIC=0
         if (want && !ctx->pdl) {
-            constexpr size_t RING_OFF = 256, BYTES = RING_OFF + 1024 * DYN_Q * 8;   // up to 1024 walkers
             if (!ctx->dyn_buf) {
-                if (cudaMalloc(&ctx->dyn_buf, BYTES) != cudaSuccess) return asca_fail(ctx, ASCA_ERR_OOM, "gemm_tc: cannot allocate the tile-claim buffer");
-                ASCA_CUDA(ctx, cudaMemsetAsync(ctx->dyn_buf, 0, BYTES, ctx->stream));
+                if (cudaMalloc(&ctx->dyn_buf, 256) != cudaSuccess) return asca_fail(ctx, ASCA_ERR_OOM, "gemm_tc: cannot allocate the tile counters");
+                ASCA_CUDA(ctx, cudaMemsetAsync(ctx->dyn_buf, 0, 256, ctx->stream));
                 ctx->dyn_seq = 0;
             }
-            if (grid <= 1024) {
-                const uint32_t seq = ++ctx->dyn_seq;
-                int* ctrs = static_cast<int*>(ctx->dyn_buf);
-                p.dyn_ctr = ctrs + (seq & 1) * 32;          // the two counters sit in different 128-byte lines
-                p.dyn_reset = ctrs + ((seq + 1) & 1) * 32;
-                p.dyn_ring = reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->dyn_buf) + RING_OFF);
-                p.dyn_seq = seq;
-                // One tile per claim. Several consecutive tiles per claim were measured (8 where a walker has > 128 tiles):
-                // the train step went from 335.9 to 355.4 ms -- neighbouring walkers no longer work on neighbouring tiles
-                // at the same time, which is what lets them share operand tiles in L2.
-                (void)tiles_est;
-                p.dyn_batch = 1;
-            }
+            // One tile per claim. Several consecutive tiles per claim were measured (8 where a walker has > 128 tiles):
+            // the train step went from 335.9 to 355.4 ms -- neighbouring walkers no longer work on neighbouring tiles
+            // at the same time, which is what lets them share operand tiles in L2.
+            const uint32_t seq = ++ctx->dyn_seq;
+            int* ctrs = static_cast<int*>(ctx->dyn_buf);
+            p.dyn_ctr = ctrs + (seq & 1) * 32;          // the two counters sit in different 128-byte lines
+            p.dyn_reset = ctrs + ((seq + 1) & 1) * 32;
         }
     }
     using SH = Shape<BN, DEEP, PAIR, EW8>;
@@ -856,26 +852,16 @@ int launch(asca_ctx* ctx, const Args& a) {
                                                 : "gemm_tc_kernel (expert-grouped k)",
                  2.0 * rows_m * (double)a.N * rows_k);
     const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
-    // persistent: the CTAs claim tile after tile. Wide tiles for dense problems with a long k-loop and at least
-    // two waves of tiles (measured: +10-15 % there; with k <= 2048 or expert-grouped rows the 128 KiB epilogue per
-    // tile and the single stream per SM cost more than the wider instruction gains).
-    // CTA pairs on 256 x 256 tiles: dense and expert-grouped products with at least one tile per pair of SMs
-    const int64_t pairs = tile_bound(a, 256, 256);
-    const int64_t wide = tile_bound(a, 256);
-    const bool wide_ok = a.group_dim == GROUP_NONE && a.K >= 4096 && a.N >= 256 && wide >= 2 * n_sm;
-    // measured at 32768 x 2048 x 6144: A B^T with a long k runs 1389 TFLOP/s on 128 x 256 single-CTA tiles against 1320 on
-    // pairs (both operands K-major: the widest TMA boxes); every other dense form is faster on pairs
-    if (pair_wanted(ctx, a) && !(wide_ok && a.mode == ASCA_NT && a.epi != EPI_QKV)) {
-        const int64_t g2 = 2 * std::min<int64_t>(pairs, n_sm / 2);
-        if (a.group_dim == GROUP_M || a.epi == EPI_QKV) return launch_shape<256, false, true, true>(ctx, a, g2, pairs);
-        return launch_shape<256, false, true, false>(ctx, a, g2, pairs);
+    // persistent: the CTAs (or pairs, on 256 x 256 tiles) claim tile after tile
+    if (pair_wanted(ctx, a)) {
+        const int64_t g2 = 2 * std::min<int64_t>(tile_bound(a, 256, 256), n_sm / 2);
+        if (a.group_dim == GROUP_M || a.epi == EPI_QKV) return launch_shape<256, false, true, true>(ctx, a, g2);
+        return launch_shape<256, false, true, false>(ctx, a, g2);
     }
-    if (wide_ok)
-        return launch_shape<256, false>(ctx, a, std::min<int64_t>(wide, n_sm), wide);
     const int64_t grid = tile_bound(a, 128);
     if (grid <= 0) return ASCA_OK;
-    if (grid <= n_sm) return launch_shape<128, true>(ctx, a, grid, grid);
-    return launch_shape<128, false>(ctx, a, std::min<int64_t>(grid, 2 * n_sm), grid);
+    if (grid <= n_sm) return launch_shape<128, true>(ctx, a, grid);
+    return launch_shape<128, false>(ctx, a, std::min<int64_t>(grid, 2 * n_sm));
 }
 
 // A pair runs a 256 x 256 tile 1.6 times as fast as two SMs run its four quarters in the 128 x 128 shape (two CTAs an SM), so pairs win
