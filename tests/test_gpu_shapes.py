@@ -184,3 +184,55 @@ def test_bf16_decode_graph_equals_direct_launches(orc, gpu):
     for a, b in zip(*runs):
         assert np.array_equal(a, b)
     m.free()
+
+
+# The tensor-core products around their tile shapes: pairs from half the chip on (37 tiles), one 128 x 128 tile an SM, two CTAs
+# an SM; ragged last rows and columns, rows off the 32-byte grid, k below and between k-tiles, bias and accumulation.
+@pytest.mark.parametrize("m,k,n", [(1536, 64, 1600), (1537, 72, 1604), (2560, 1032, 2050), (1100, 200, 1030), (130, 520, 40), (2100, 136, 2100)])
+@pytest.mark.parametrize("mode", ["NN", "TN", "NT"])
+def test_bf16_product_tile_edges(gpu, m, k, n, mode):
+    import torch
+    import asca_b200
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(m + 7 * k + 13 * n)
+    a, b = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((m, k), (k, n)))
+    bias, c0 = torch.randn(n, generator=g, device="cuda"), torch.randn(m, n, generator=g, device="cuda")
+    out = c0.clone()
+    ops.gemm(gpu, a.t().contiguous() if mode == "TN" else a, b.t().contiguous() if mode == "NT" else b, getattr(asca_b200, mode), bias=bias,
+             out=out, accumulate=True)
+    gpu.sync()
+    ref = a.double() @ b.double() + bias.double() + c0.double()
+    assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) < F32_TOL
+
+
+# The bf16 expert layer with a skewed load, experts of no token in long runs, and segments around the tile and cluster sizes.
+@pytest.mark.parametrize("n,d,F,E,vocab", [(1025, 512, 1024, 256, 1), (4096, 256, 320, 4, 256), (6000, 256, 512, 8, 3), (640, 128, 1088, 2, 256)])
+def test_bf16_expert_layer_edges(gpu, n, d, F, E, vocab):
+    import torch
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = torch.randint(0, vocab, (n,), generator=g, device="cuda", dtype=torch.int32)
+    perm, offs = ops.moe_dispatch(gpu, ids, E)
+    xn = torch.randn(n, d, generator=g, device="cuda").bfloat16()
+    w1, w2 = (torch.randn(*s, generator=g, device="cuda").mul_(s[0] ** -0.5 if s[0] == d else F ** -0.5).bfloat16() for s in ((d, E * F), (E * F, d)))
+    b1, b2 = torch.randn(E * F, generator=g, device="cuda"), torch.randn(d, generator=g, device="cuda")
+    dout = torch.randn(n, d, generator=g, device="cuda")
+    out, pre, hid = ops.moe_fwd(gpu, xn, w1, b1, w2, b2, perm, offs, F, E)
+    d_w1, d_b1, d_w2, d_b2, dxn = ops.moe_bwd(gpu, xn, w1, w2, pre, hid, dout, perm, offs, F, E)
+    gpu.sync()
+    o = offs.cpu().tolist()
+    close = lambda got, want: rel_err(got.float().cpu().numpy(), want.float().cpu().numpy()) < 2e-2
+    assert close(d_b2, dout.sum(0))
+    for e in range(E):
+        rows, f = perm[o[e]:o[e + 1]].long(), slice(e * F, (e + 1) * F)
+        if o[e] == o[e + 1]:
+            assert not (d_w1[:, f].any() or d_w2[f].any() or d_b1[f].any())
+            continue
+        x, dy = xn[rows].float(), dout[rows]
+        p = x @ w1[:, f].float() + b1[f]
+        s = torch.sigmoid(p)
+        h, dp = p * s, (dy @ w2[f].float().t()) * (s * (1 + p * (1 - s)))
+        assert close(out[rows], h @ w2[f].float() + b2) and close(dxn[rows], dp @ w1[:, f].float().t())
+        assert close(d_w1[:, f], x.t() @ dp) and close(d_w2[f], h.t() @ dy) and close(d_b1[f], dp.sum(0))
