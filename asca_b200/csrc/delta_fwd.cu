@@ -71,7 +71,7 @@ template <int DH, int COLS, typename T>
 __global__ void __launch_bounds__(RecCfg<DH, COLS>::NT + RecCfg<DH, COLS>::HT) delta_fwd_rec_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ alpha,
     const float* __restrict__ beta, int B, int Tlen, int H, int chunk, T* __restrict__ o,
-    const float* __restrict__ s_init, float* __restrict__ s_final, float* __restrict__ ckpt) {
+    const float* s_init, float* s_final /* may be s_init */, float* __restrict__ ckpt) {
     using C = RecCfg<DH, COLS>;
     constexpr int LANES = C::LANES, RPT = C::RPT, NT = C::NT, HT = C::HT, FW = C::FW, FTS = C::FTS;
     constexpr int KQ4 = FTS * DH / 4;        // float4 units of k (or q) per stage

@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) delta_fwd_tc_kernel(
     const __grid_constant__ CUtensorMap mapWQ, const __grid_constant__ CUtensorMap mapUV,
     const __grid_constant__ CUtensorMap mapKW, const __grid_constant__ CUtensorMap mapAA,
     const __grid_constant__ CUtensorMap mapS0, const float* __restrict__ GC,
-    int T, int H, int dhi, int n_chunks, TO* __restrict__ o, const float* __restrict__ s_init, float* __restrict__ s_final,
+    int T, int H, int dhi, int n_chunks, TO* __restrict__ o, const float* s_init, float* s_final /* may be s_init */,
     float* __restrict__ ckpt, __nv_bfloat16* __restrict__ s0b, int* err_word) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);

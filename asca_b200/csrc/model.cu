@@ -380,6 +380,10 @@ bool asca_tc_enabled();  // gemm.cu
 // elementwise.cu
 int asca_rmsnorm_bwd_add_cast(asca_ctx* ctx, const float* x, const float* dy, const float* add, float* dx, void* dx16, int64_t rows,
                               int64_t cols, float eps);
+// moe.cu
+int asca_moe_fwd_bf16_nopre(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1, const __nv_bfloat16* w2, const float* b2,
+                            const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, float* out,
+                            __nv_bfloat16* hid_p);
 // moe.cu / mixed.cu: the decode-step forms on rows in expert order
 int asca_moe_fwd_sorted_residual(asca_ctx* ctx, const __nv_bfloat16* xp, const __nv_bfloat16* w1, const float* b1,
                                  const __nv_bfloat16* w2, const float* b2, const int32_t* perm, const int32_t* offsets, int64_t N,
@@ -1530,15 +1534,14 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     int32_t* last = (int32_t*)bf.f(ns);
     uint32_t* nxt = (uint32_t*)bf.f(ns);
     float *x = bf.f(N * d), *qkv = bf.f(N * 3 * d), *gate = bf.f(N * 2 * H), *y = bf.f(N * d), *x_mid = bf.f(N * d), *mo = bf.f(N * d);
-    float *qn = bf.f(N * H), *kn = bf.f(N * H), *al = bf.f(N * H), *be = bf.f(N * H), *pre_p = bf.f(N * F);
-    float* s_fin = bf.f(ns * H * dh * dh);
+    float *qn = bf.f(N * H), *kn = bf.f(N * H), *al = bf.f(N * H), *be = bf.f(N * H), *pre_p = nullptr;
     float *xl = bf.f(ns * d), *hf = bf.f(ns * d), *logits = bf.f(ns * V);
     // activations a product reads: bf16 in bf16 mode, f32 otherwise (same element counts)
     auto act = [&](int64_t n) { return bfm ? (void*)h16(n) : (void*)bf.f(n); };
     void *x_in = bfm ? act(N * d) : nullptr, *q = act(N * d), *k = act(N * d), *v = act(N * d), *o = act(N * d), *xn = act(N * d),
          *hid_p = act(N * F), *hf_in = bfm ? act(ns * d) : nullptr;
-    ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && qkv && gate && y && x_mid && mo && qn && kn && al && be && pre_p &&
-                          s_fin && xl && hf && logits && q && k && v && o && xn && hid_p && (!bfm || (x_in && hf_in)),
+    ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && qkv && gate && y && x_mid && mo && qn && kn && al && be &&
+                          xl && hf && logits && q && k && v && o && xn && hid_p && (!bfm || (x_in && hf_in)),
                  "model_prefill: out of memory");
     asca_stage_scope staged(ctx);
     ASCA_TRY(asca_copy_in(ctx, ids, ids_h, (size_t)N * 4));
@@ -1548,14 +1551,12 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));
     ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, x));
     const size_t st_layer = (size_t)ns * H * dh * dh;
+    const bool join = bfm && N * d % 4 == 0;   // the residual add also writes the next block's bf16 input
     for (int64_t li = 0; li < L; ++li) {
         const Lyr& w = m->lay[li];
         const Lyr& w16 = m->lay16[li];
-        const void* xi = x;
-        if (bfm) {
-            ASCA_TRY(asca_cast_bf16(ctx, x, x_in, N * d));
-            xi = x_in;
-        }
+        const void* xi = bfm ? x_in : (const void*)x;
+        if (bfm && (li == 0 || !join)) ASCA_TRY(asca_cast_bf16(ctx, x, x_in, N * d));
         const void *Wqkv = bfm ? (const void*)(W + w16.w_qkv) : (const void*)(P + w.w_qkv), *Wg = bfm ? (const void*)(W + w16.w_gate) : (const void*)(P + w.w_gate),
                    *Wo = bfm ? (const void*)(W + w16.w_o) : (const void*)(P + w.w_o), *W1 = bfm ? (const void*)(W + w16.w1) : (const void*)(P + w.w1),
                    *W2 = bfm ? (const void*)(W + w16.w2) : (const void*)(P + w.w2);
@@ -1564,13 +1565,25 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
         if (bfm) ASCA_TRY(asca_delta_prep_bf16(ctx, qkv, gate, N, H, dh, q, k, v, qn, kn, al, be));
         else ASCA_TRY(asca_delta_prep(ctx, qkv, gate, N, H, dh, (float*)q, (float*)k, (float*)v, qn, kn, al, be));
         float* st = state + (size_t)li * st_layer;
-        ASCA_TRY(asca_delta_fwd(ctx, q, k, v, al, be, ns, T, H, dh, 64, DT, o, st, s_fin, nullptr));
-        ASCA_CUDA(ctx, cudaMemcpyAsync(st, s_fin, st_layer * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+        ASCA_TRY(asca_delta_fwd(ctx, q, k, v, al, be, ns, T, H, dh, 64, DT, o, st, st, nullptr));   // (in place: a CTA's own part)
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, d, d, o, d, Wo, d, y, d, P + w.b_o, 0, DT));
         if (bfm) ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, y, x_mid, xn, N, d, 1e-6f));
         else ASCA_TRY(asca_residual_rmsnorm(ctx, x, y, x_mid, (float*)xn, N, d, 1e-6f));
-        ASCA_TRY(asca_moe_fwd(ctx, xn, W1, P + w.b1, W2, P + w.b2, perm, offs, N, d, F, E, DT, mo, pre_p, hid_p));
-        ASCA_TRY(asca_residual_rmsnorm(ctx, x_mid, mo, x, nullptr, N, d, 1e-6f));
+        int rc = bfm ? asca_moe_fwd_bf16_nopre(ctx, (const bf16*)xn, (const bf16*)W1, P + w.b1, (const bf16*)W2, P + w.b2, perm, offs, N, d, F, E, mo,
+                                               (bf16*)hid_p)
+                     : ASCA_ERR_UNSUPPORTED;
+        if (rc == ASCA_ERR_UNSUPPORTED) {
+            if (!pre_p) pre_p = bf.f(N * F);
+            ASCA_REQUIRE(ctx, pre_p, "model_prefill: out of memory");
+            rc = asca_moe_fwd(ctx, xn, W1, P + w.b1, W2, P + w.b2, perm, offs, N, d, F, E, DT, mo, pre_p, hid_p);
+        }
+        ASCA_TRY(rc);
+        if (join) {
+            add_cast4_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(N * d / 4, 256), 148 * 8), 256, 0, ctx->stream>>>(x_mid, mo, x, (bf16*)x_in, N * d / 4);
+            ASCA_CHECK_LAUNCH(ctx);
+        } else {
+            ASCA_TRY(asca_residual_rmsnorm(ctx, x_mid, mo, x, nullptr, N, d, 1e-6f));
+        }
     }
     // the head on each stream's last token only
     ASCA_TRY(asca_gather_rows(ctx, x, last, ns, d, xl));

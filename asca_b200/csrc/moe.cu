@@ -146,7 +146,7 @@ inline bool tc_shapes_ok(int64_t d, int64_t F) { return asca_tc_enabled() && d %
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Tensor-core forward: permute xn once, then two grouped tcgen05 GEMMs.
+// Tensor-core forward: permute xn once, then two grouped tcgen05 GEMMs. pre_p null: the pre-activations are not kept.
 int moe_fwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1,
                const __nv_bfloat16* w2, const float* b2, const int32_t* perm, const int32_t* offsets, int64_t N,
                int64_t d, int64_t F, int64_t E, float* out, float* pre_p, __nv_bfloat16* hid_p) {
@@ -160,7 +160,7 @@ int moe_fwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, 
     a.C = pre_p; a.ldc = F; a.N = (int)F; a.K = (int)d;
     a.bias = b1; a.bias_gstride = F;
     a.offsets = offsets; a.n_groups = (int)E; a.group_dim = gemm_tc::GROUP_M; a.total_rows = N;
-    a.epi = gemm_tc::EPI_SILU; a.C2 = hid_p; a.ldc2 = F;
+    a.epi = gemm_tc::EPI_SILU; a.C2 = hid_p; a.ldc2 = F; a.c2_only = pre_p == nullptr;
     gemm_tc::Args b{};
     b.mode = ASCA_NN;
     b.A = hid_p; b.lda = F; b.a_rows = N; b.a_cols = F;
@@ -279,6 +279,14 @@ int moe_fwd_simt(asca_ctx* ctx, const void* xn, const void* w1, const float* b1,
 }
 
 }  // namespace
+
+// bf16 forward that keeps no pre-activations (no backward follows: a third of the first product's epilogue and two thirds of its
+// bytes). ASCA_ERR_UNSUPPORTED where the tensor-core products cannot run; the caller then uses asca_moe_fwd.
+int asca_moe_fwd_bf16_nopre(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1, const __nv_bfloat16* w2, const float* b2,
+                            const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, float* out, __nv_bfloat16* hid_p) {
+    if (!tc_shapes_ok(d, F)) return ASCA_ERR_UNSUPPORTED;
+    return moe_fwd_tc(ctx, xn, w1, b1, w2, b2, perm, offsets, N, d, F, E, out, nullptr, hid_p);
+}
 
 // f32 forward with the residual add in the second product's store: out = res + moe(xn)
 int asca_moe_fwd_f32_residual(asca_ctx* ctx, const float* xn, const float* w1, const float* b1, const float* w2, const float* b2,
