@@ -78,7 +78,7 @@ struct KP {
     int c2_only;
     __nv_bfloat16 *qkv_q, *qkv_k, *qkv_v;
     float *qkv_qn, *qkv_kn;
-    int qkv_d;
+    int qkv_d, qkv_dh;
     const uint32_t* ce_targets;
     float* ce_loss;
     float ce_scale;
@@ -550,34 +550,42 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             ok = __shfl_sync(0xffffffffu, got, 0) != 0;  // uniform: tcgen05.ld below is warp-aligned
             if (!ok) break;
             tc::tcgen05_fence_after();
-            // fused qkv epilogue (pair shape, whole tiles: the launcher checks): this warp's 128 columns are one head of q, k or v
+            // fused qkv epilogue (pair shape): this warp's 128 columns are one head of q, k or v, or two of 64
             const bool qkv = PAIR && EW8 && p.epi == EPI_QKV;
-            float qkv_scale = 1.0f;                 // 1 / max(|z|, 1e-8) of this lane's row (q, k), 1 for v
+            float qkv_scale[2] = {1.0f, 1.0f};      // 1 / max(|z|, 1e-8) of this lane's row (q, k), 1 for v; per 64 columns
             __nv_bfloat16* hrow = p.C2 + lr * p.ldc2 + x.n0;
             if (qkv) {
                 const int hc0 = x.n0 + c_lo * 32;   // first column of the head
                 const int sec = hc0 / p.qkv_d;      // 0 q, 1 k, 2 v
                 hrow = (sec == 0 ? p.qkv_q : sec == 1 ? p.qkv_k : p.qkv_v) + lr * p.qkv_d + (x.n0 - sec * p.qkv_d);
                 if (sec < 2) {
-                    float ss = 0.0f;
+                    float ss[2] = {0.0f, 0.0f};
 #pragma unroll 1
-                    for (int c = c_lo; c < c_lo + C_PER_WARP; ++c) {
+                    for (int c = 0; c < C_PER_WARP; ++c) {
                         uint32_t r[32];
-                        tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), r);
+                        tc::tmem_ld_32x32(tmem_acc + (uint32_t)((c_lo + c) * 32), r);
                         tc::tmem_ld_wait();
-                        const float4* bb = reinterpret_cast<const float4*>(p.bias + x.n0 + c * 32);
+                        const float4* bb = reinterpret_cast<const float4*>(p.bias + hc0 + c * 32);
+                        float sq = 0.0f;
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
                             const float4 b4 = bb[j];
                             const float v0 = __uint_as_float(r[4 * j]) + b4.x, v1 = __uint_as_float(r[4 * j + 1]) + b4.y,
                                         v2 = __uint_as_float(r[4 * j + 2]) + b4.z, v3 = __uint_as_float(r[4 * j + 3]) + b4.w;
-                            ss += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
+                            sq += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
                         }
+                        if (c < C_PER_WARP / 2) ss[0] += sq;
+                        else ss[1] += sq;
                     }
-                    const float nrm = fmaxf(sqrtf(ss), 1e-8f);
-                    qkv_scale = 1.0f / nrm;
-                    const int heads = p.qkv_d / 128, head = (hc0 - sec * p.qkv_d) / 128;
-                    (sec == 0 ? p.qkv_qn : p.qkv_kn)[lr * heads + head] = nrm;
+                    const bool two = p.qkv_dh == 64;
+                    if (!two) ss[0] += ss[1];
+                    const int heads = p.qkv_d / p.qkv_dh, head = (hc0 - sec * p.qkv_d) / p.qkv_dh;
+                    float* norms = (sec == 0 ? p.qkv_qn : p.qkv_kn) + lr * heads + head;
+                    const float n0 = fmaxf(sqrtf(ss[0]), 1e-8f), n1 = two ? fmaxf(sqrtf(ss[1]), 1e-8f) : n0;
+                    qkv_scale[0] = 1.0f / n0;
+                    qkv_scale[1] = 1.0f / n1;
+                    if (live) norms[0] = n0;
+                    if (live && two) norms[1] = n1;
                 }
             }
             // fused cross-entropy (pair shape, four epilogue warps: a warp's lanes hold whole rows of 256 logits)
@@ -652,7 +660,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                 }
                 if (qkv) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] *= qkv_scale;
+                    for (int j = 0; j < 32; ++j) v[j] *= qkv_scale[2 * i / C_PER_WARP];
                 }
                 if (with_aux) {
 #pragma unroll
@@ -756,7 +764,7 @@ static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid) {
     p.c_gstride = a.c_gstride; p.bias_gstride = a.bias_gstride;
     p.epi = a.epi; p.aux = a.aux; p.ldaux = a.ldaux; p.C2 = a.C2; p.ldc2 = a.ldc2; p.c2_only = a.c2_only;
     p.ce_targets = a.ce_targets; p.ce_loss = a.ce_loss; p.ce_scale = a.ce_scale;
-    p.qkv_q = a.qkv_q; p.qkv_k = a.qkv_k; p.qkv_v = a.qkv_v; p.qkv_qn = a.qkv_qn; p.qkv_kn = a.qkv_kn; p.qkv_d = a.qkv_d;
+    p.qkv_q = a.qkv_q; p.qkv_k = a.qkv_k; p.qkv_v = a.qkv_v; p.qkv_qn = a.qkv_qn; p.qkv_kn = a.qkv_kn; p.qkv_d = a.qkv_d; p.qkv_dh = a.qkv_dh;
     p.err_word = ctx->err_word;
     {   // dynamic tile claims: not under programmatic dependent launch (the counter hand-over relies on stream order)
         static const int dyn_env = [] { const char* e = getenv("ASCA_GEMM_DYNAMIC"); return e ? atoi(e) : 1; }();
@@ -829,7 +837,7 @@ static bool pair_wanted(asca_ctx* ctx, const Args& a);
 
 bool qkv_fusable(asca_ctx* ctx, const Args& a) {
     return supported(a) && !skinny_wanted(a) && a.group_dim == GROUP_NONE && a.mode == ASCA_NN && pair_wanted(ctx, a) && a.qkv_d > 0 &&
-           a.qkv_d % 256 == 0 && a.N == 3 * a.qkv_d && a.M % 256 == 0 && a.bias && (reinterpret_cast<uintptr_t>(a.bias) & 15) == 0 &&
+           a.qkv_d % 256 == 0 && (a.qkv_dh == 128 || a.qkv_dh == 64) && a.N == 3 * a.qkv_d && a.bias && (reinterpret_cast<uintptr_t>(a.bias) & 15) == 0 &&
            a.qkv_q && a.qkv_k && a.qkv_v && a.qkv_qn && a.qkv_kn && !a.accumulate && !a.c_idx &&
            ((reinterpret_cast<uintptr_t>(a.qkv_q) | reinterpret_cast<uintptr_t>(a.qkv_k) | reinterpret_cast<uintptr_t>(a.qkv_v)) & 7) == 0;
 }

@@ -5,7 +5,7 @@
 
 namespace gemm_tc {
 
-// EPI_QKV: the product is the qkv projection of a Delta block (N = 3 d, head dim 128): instead of C, the epilogue writes
+// EPI_QKV: the product is the qkv projection of a Delta block (N = 3 d, head dim 128 or 64): instead of C, the epilogue writes
 // q and k L2-normalised per head (z / max(|z|, 1e-8), rust/src/delta.rs:146-165) and v, all as bf16 (rows x d each), and
 // the norms of q and k (rows x H, f32). Bias is added first. CTA-pair shape only; see qkv_fusable().
 // EPI_CE: the product is the output head (N = 256 = the byte vocabulary, one tile wide): the epilogue holds a row's 256
@@ -46,8 +46,8 @@ struct Args {
     int c2_mapped;            // few-row kernel only: C2's rows go through c_idx like C's
     int b_packed;             // few-row kernel only: B is a buffer made by skinny_pack (b_rows = its rows of 64)
     __nv_bfloat16 *qkv_q, *qkv_k, *qkv_v;   // EPI_QKV outputs (rows x qkv_d, bf16)
-    float *qkv_qn, *qkv_kn;                 // EPI_QKV: norms (rows x qkv_d / 128)
-    int qkv_d;
+    float *qkv_qn, *qkv_kn;                 // EPI_QKV: norms (rows x qkv_d / qkv_dh)
+    int qkv_d, qkv_dh;                      // EPI_QKV: width of q, k, v and of a head
     const uint32_t* ce_targets;             // EPI_CE: target id per row
     float* ce_loss;                         // EPI_CE: per-row loss
     float ce_scale;                         // EPI_CE: multiplies (softmax - onehot): grad scale / rows
@@ -64,7 +64,7 @@ bool supported(const Args& a);
 // Enqueues the kernel on ctx->stream. Returns ASCA_OK or an error code.
 int launch(asca_ctx* ctx, const Args& a);
 // True when launch() would run this dense product on CTA pairs AND its shape suits the fused qkv epilogue (EPI_QKV):
-// whole 256-row tiles, N = 3 d with d a multiple of 256, bias present and 16-byte aligned.
+// N = 3 d with d a multiple of 256, bias present and 16-byte aligned.
 bool qkv_fusable(asca_ctx* ctx, const Args& a);
 // Likewise for the fused cross-entropy epilogue (EPI_CE): N = 256, whole 256-row tiles, no bias, bf16 dlogits in C2.
 bool ce_fusable(asca_ctx* ctx, const Args& a);

@@ -812,9 +812,9 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
         tq.B = W + w16.w_qkv; tq.ldb = 3 * d; tq.b_rows = d; tq.b_cols = 3 * d;
         tq.C = qkv; tq.ldc = 3 * d; tq.M = (int)N; tq.N = (int)(3 * d); tq.K = (int)d;
         tq.bias = P + w.b_qkv; tq.group_dim = gemm_tc::GROUP_NONE; tq.epi = gemm_tc::EPI_QKV;
-        tq.qkv_q = a.q; tq.qkv_k = a.k; tq.qkv_v = a.v; tq.qkv_qn = a.qn; tq.qkv_kn = a.kn; tq.qkv_d = (int)d;
+        tq.qkv_q = a.q; tq.qkv_k = a.k; tq.qkv_v = a.v; tq.qkv_qn = a.qn; tq.qkv_kn = a.kn; tq.qkv_d = (int)d; tq.qkv_dh = (int)dh;
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 2 * H, d, a.x_in, d, W + w16.w_gate, 2 * H, gate, 2 * H, P + w.b_gate, 0, BF));
-        if (m->fused_qkv && dh == 128 && asca_tc_enabled() && gemm_tc::qkv_fusable(ctx, tq)) {
+        if (m->fused_qkv && asca_tc_enabled() && gemm_tc::qkv_fusable(ctx, tq)) {
             ASCA_TRY(gemm_tc::launch(ctx, tq));
             gate_sigmoid_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(N * H, 256), 148 * 8), 256, 0, ctx->stream>>>(gate, N * H, (int)H, a.al, a.be);
             ASCA_CHECK_LAUNCH(ctx);
@@ -1560,9 +1560,22 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
         const void *Wqkv = bfm ? (const void*)(W + w16.w_qkv) : (const void*)(P + w.w_qkv), *Wg = bfm ? (const void*)(W + w16.w_gate) : (const void*)(P + w.w_gate),
                    *Wo = bfm ? (const void*)(W + w16.w_o) : (const void*)(P + w.w_o), *W1 = bfm ? (const void*)(W + w16.w1) : (const void*)(P + w.w1),
                    *W2 = bfm ? (const void*)(W + w16.w2) : (const void*)(P + w.w2);
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 3 * d, d, xi, d, Wqkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, DT));
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 2 * H, d, xi, d, Wg, 2 * H, gate, 2 * H, P + w.b_gate, 0, DT));
-        if (bfm) ASCA_TRY(asca_delta_prep_bf16(ctx, qkv, gate, N, H, dh, q, k, v, qn, kn, al, be));
+        gemm_tc::Args tq{};   // q, k, v from the product's epilogue where it can (as in the training step)
+        if (bfm) {
+            tq.mode = ASCA_NN; tq.A = xi; tq.lda = d; tq.a_rows = N; tq.a_cols = d;
+            tq.B = Wqkv; tq.ldb = 3 * d; tq.b_rows = d; tq.b_cols = 3 * d;
+            tq.ldc = 3 * d; tq.M = (int)N; tq.N = (int)(3 * d); tq.K = (int)d;
+            tq.bias = P + w.b_qkv; tq.group_dim = gemm_tc::GROUP_NONE; tq.epi = gemm_tc::EPI_QKV;
+            tq.qkv_q = (bf16*)q; tq.qkv_k = (bf16*)k; tq.qkv_v = (bf16*)v; tq.qkv_qn = qn; tq.qkv_kn = kn; tq.qkv_d = (int)d; tq.qkv_dh = (int)dh;
+        }
+        const bool fused = bfm && m->fused_qkv && asca_tc_enabled() && gemm_tc::qkv_fusable(ctx, tq);
+        if (!fused) ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 3 * d, d, xi, d, Wqkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, DT));
+        if (fused) {
+            ASCA_TRY(gemm_tc::launch(ctx, tq));
+            gate_sigmoid_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(N * H, 256), 148 * 8), 256, 0, ctx->stream>>>(gate, N * H, (int)H, al, be);
+            ASCA_CHECK_LAUNCH(ctx);
+        } else if (bfm) ASCA_TRY(asca_delta_prep_bf16(ctx, qkv, gate, N, H, dh, q, k, v, qn, kn, al, be));
         else ASCA_TRY(asca_delta_prep(ctx, qkv, gate, N, H, dh, (float*)q, (float*)k, (float*)v, qn, kn, al, be));
         float* st = state + (size_t)li * st_layer;
         ASCA_TRY(asca_delta_fwd(ctx, q, k, v, al, be, ns, T, H, dh, 64, DT, o, st, st, nullptr));   // (in place: a CTA's own part)

@@ -236,3 +236,24 @@ def test_bf16_expert_layer_edges(gpu, n, d, F, E, vocab):
         h, dp = p * s, (dy @ w2[f].float().t()) * (s * (1 + p * (1 - s)))
         assert close(out[rows], h @ w2[f].float() + b2) and close(dxn[rows], dp @ w1[:, f].float().t())
         assert close(d_w1[:, f], x.t() @ dp) and close(d_w2[f], h.t() @ dy) and close(d_b1[f], dp.sum(0))
+
+
+# q, k and v from the projection's epilogue (one head of 128 or two of 64 a warp, ragged last rows) against the separate pass:
+# a prefill's states and logits.
+@pytest.mark.parametrize("d,H,ns,T", [(256, 4, 33, 97), (256, 2, 16, 192), (768, 12, 9, 301)])
+def test_prefill_with_the_fused_qkv_epilogue(orc, gpu, d, H, ns, T):
+    import asca_b200
+
+    m = asca_b200.Model(gpu, 256, d, H, 2, 4, 256)
+    m.set_params(orc.Rng(d + H).normal(m.n, 0.05))
+    m.set_compute(asca_b200.BF16)
+    ids = orc.Rng(T).below(256, ns * T).reshape(ns, T)
+    got = []
+    for fused in (False, True):
+        m.set_fused_qkv(fused)
+        st = m.new_decode_state(ns)
+        logits, _ = m.prefill(st, ids)
+        got.append((np.asarray(logits), st.cpu().numpy()))
+    m.free()
+    for a, b in zip(*got):
+        assert rel_err(b, a) < 5e-3
