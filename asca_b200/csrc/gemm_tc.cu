@@ -35,7 +35,7 @@ constexpr int A_BYTES = BM * BK * 2;
 // Two tile shapes. 128 x 128: 3-stage ring, 256 TMEM columns, two CTAs per SM (two independent MMA streams keep the
 // tensor pipe fed).
 // DEEP: a problem of at most one 128 x 128 tile per SM (a decode step's products) runs one CTA per SM with a
-// 6-stage ring: its k-loop streams weights that are cold in L2, and three stages do not cover the HBM latency.
+// 7-stage ring: its k-loop streams weights that are cold in L2, and three stages do not cover the HBM latency.
 // PAIR: a cluster of two CTAs computes 256 x 256 tiles with cta_group::2 instructions (M = 256, N = 256). Each CTA
 // loads its own 128 rows of A and its own 128 of the tile's 256 B columns (32 KiB per k-tile for 4.2 MFLOP on this SM
 // against 48 KiB for the 128 x 256 tile and 32 KiB per 2.1 MFLOP for the 128 x 128 one): shared-memory traffic per
@@ -49,10 +49,10 @@ template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;      // two accumulator buffers
     static constexpr int CTAS_PER_SM = PAIR || DEEP ? 1 : 2;
-    // epilogue warps: one per TMEM lane quarter. EW8 (pair shape): two warps share each quarter and split the 256 columns
-    // -- for the row-grouped expert products, whose epilogues (activation, two outputs, row scatter) would otherwise
-    // outlast the main loop (837 against 603 TFLOP/s inside the training step), and for the fused qkv epilogue (a warp's
-    // 128 columns are one head). Plain dense and k-grouped products are faster with four (1181 / 878 against 1056 / 781).
+    // epilogue warps: one per TMEM lane quarter. EW8 (pair shape): two warps share each quarter and split the 256 columns -- for
+    // the row-grouped expert products, whose epilogues (activation, two outputs, row scatter) would otherwise outlast the
+    // main loop, and for the fused qkv epilogue (a warp's 128 columns are one head, or two of 64). Plain dense and k-grouped
+    // products are faster with four (14,448 x 768 -> 2304: 56 against 68 us).
     static constexpr int EPI_WARPS = (PAIR && EW8) ? 8 : 4;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
     static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 384 /*barriers, claims*/;   // + stages + tile table
