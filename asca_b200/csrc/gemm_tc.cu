@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             // atomic's round trip hides behind the loads, and no other role needs the next claim before this one is used up.
             // (Not earlier: with about as many tiles as walkers the first to start would take two each, 190 us against 110 for
             // 64 tiles.)
-            const bool claimer = dyn && rank == 0;
+            const bool claimer = dyn && rank == 0, may_be_empty = p.group_dim == GROUP_K || p.K == 0;
             int cur = 0;
             if (claimer) {
                 cur = atomicAdd(p.dyn_ctr, 1);
@@ -340,8 +340,6 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                 int nxt = 0;
                 const Tile x = locate(t);
                 const int nl0 = x.n0 + rank * BNL;   // first B column this CTA loads
-                // (a tile without k-tiles takes no ring slot: the claims of a run of them wait for the epilogue instead)
-                if (claimer && x.num_k == 0 && ci >= 2) ok = tc::mbar_wait(&acc_empty[ci & 1], ((ci >> 1) - 1) & 1, abort_flag, p.err_word, 108);
                 if (claimer && x.num_k == 0) nxt = atomicAdd(p.dyn_ctr, 1);
                 for (int kt = 0; kt < x.num_k; ++kt) {
                     if (claimer && kt == x.num_k / 2) nxt = atomicAdd(p.dyn_ctr, 1);
@@ -378,9 +376,17 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     }
                     if (++s == STAGES) s = 0, ++round;
                 }
-                if (claimer) {   // (after a wait that gave up: "none left", so that the walker's other roles stop too)
-                    cur = ok ? nxt : total_tiles;
-                    publish_claim(ci + 1, cur);
+                if (claimer) {
+                    // A tile without k-tiles takes no ring slot, so nothing above holds the claims of a run of them back: each waits
+                    // for the epilogue to release its accumulator buffer once more (of the tile two before it, or of one before that
+                    // where ring slots have let the claims run further ahead; the distance then stays). The wait stands in front of
+                    // the publication: behind it, the epilogues could be through the new tile already, and the parity would
+                    // mean a tile that is yet to be claimed.
+                    const int c = ci + 1;
+                    if (ok && may_be_empty && c >= 2 && nxt < total_tiles && locate(nxt).num_k == 0)
+                        ok = tc::mbar_wait(&acc_empty[c & 1], ((c >> 1) - 1) & 1, abort_flag, p.err_word, 108);
+                    cur = ok ? nxt : total_tiles;   // (after a wait that gave up: "none left", so that the other roles stop too)
+                    publish_claim(c, cur);
                 }
             }
         }

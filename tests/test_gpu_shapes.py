@@ -206,8 +206,10 @@ def test_bf16_product_tile_edges(gpu, m, k, n, mode):
     assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) < F32_TOL
 
 
-# The bf16 expert layer with a skewed load, experts of no token in long runs, and segments around the tile and cluster sizes.
-@pytest.mark.parametrize("n,d,F,E,vocab", [(1025, 512, 1024, 256, 1), (4096, 256, 320, 4, 256), (6000, 256, 512, 8, 3), (640, 128, 1088, 2, 256)])
+# The bf16 expert layer with a skewed load, experts of no token in long runs and in turn with experts of one k-tile (whose claims are
+# held back by the epilogue and by the ring), and segments around the tile and cluster sizes.
+@pytest.mark.parametrize("n,d,F,E,vocab", [(1025, 512, 1024, 256, 1), (4096, 256, 320, 4, 256), (6000, 256, 512, 8, 3), (640, 128, 1088, 2, 256),
+                                           (700, 256, 512, 512, 256), (700, 128, 128, 1024, 200), (130, 256, 256, 1500, 4096)])
 def test_bf16_expert_layer_edges(gpu, n, d, F, E, vocab):
     import torch
     from asca_b200 import ops
