@@ -126,12 +126,13 @@ inline cudaError_t asca_launch(asca_ctx* ctx, void (*kern)(KArgs...), dim3 grid,
 }
 #endif
 // Small host arrays through the context's pinned staging area (a call that uses it ends with asca_ctx_sync, or
-// asca_stage_drop where it fails half way). stage_in: host -> device; stage_out: device -> host, delivered by asca_ctx_sync.
+// asca_stage_scope's destructor where it fails half way). stage_in: host -> device; stage_out: device -> host, delivered by
+// asca_ctx_sync. The host touches the array: a pointer that a caller gave goes through asca_copy_in / asca_copy_out, which check it.
 constexpr size_t ASCA_PIN_BYTES = (size_t)1 << 20;
 int asca_stage_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
 int asca_stage_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
-// Any host array: small ones staged as above, large ones through the context's copy threads (hostcopy.cu). asca_copy_out
-// delivers large arrays before it returns.
+// Any host array: small ones staged as above, large ones through the context's copy threads (hostcopy.cu); a device address is
+// refused with ASCA_ERR_ARG. asca_copy_out delivers large arrays before it returns.
 int asca_copy_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
 int asca_copy_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes);
 void asca_hostcopy_free(asca_ctx* ctx);

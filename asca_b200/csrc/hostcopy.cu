@@ -97,11 +97,20 @@ struct asca_hostcopy {
     }
 };
 
-static bool pinned(const void* p) {   // the copy engine reads and writes it at full speed by itself
+// What a caller's array is. The copies below touch a pageable array from the host, so anything else is told apart first: pinned
+// memory goes to the copy engine as it is (at full speed), managed memory too, and a device address is refused.
+enum class Mem { pageable, pinned, managed };
+static int host_array(asca_ctx* ctx, const void* p, Mem* kind) {
     cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeHost;
-    cudaGetLastError();
-    return false;
+    *kind = Mem::pageable;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return ASCA_OK;
+    }
+    ASCA_REQUIRE(ctx, at.type != cudaMemoryTypeDevice, "a host array is expected here, got a device address");
+    if (at.type == cudaMemoryTypeHost) *kind = Mem::pinned;
+    else if (at.type == cudaMemoryTypeManaged) *kind = Mem::managed;
+    return ASCA_OK;
 }
 
 static asca_hostcopy* hostcopy(asca_ctx* ctx) {
@@ -146,8 +155,10 @@ void asca_hostcopy_free(asca_ctx* ctx) {
 }
 
 int asca_copy_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
-    if (bytes <= PIECE) return asca_stage_in(ctx, dst, src, bytes);
-    asca_hostcopy* h = pinned(src) ? nullptr : hostcopy(ctx);
+    Mem kind;
+    ASCA_TRY(host_array(ctx, src, &kind));
+    if (bytes <= PIECE && kind != Mem::managed) return asca_stage_in(ctx, dst, src, bytes);
+    asca_hostcopy* h = kind != Mem::pageable ? nullptr : hostcopy(ctx);
     if (!h) {
         ASCA_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
         return ASCA_OK;
@@ -166,8 +177,10 @@ int asca_copy_in(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
 
 // Small arrays arrive with the asca_ctx_sync that ends the call, large ones before this returns.
 int asca_copy_out(asca_ctx* ctx, void* dst, const void* src, size_t bytes) {
-    if (bytes <= PIECE) return asca_stage_out(ctx, dst, src, bytes);
-    asca_hostcopy* h = pinned(dst) ? nullptr : hostcopy(ctx);
+    Mem kind;
+    ASCA_TRY(host_array(ctx, dst, &kind));
+    if (bytes <= PIECE && kind != Mem::managed) return asca_stage_out(ctx, dst, src, bytes);
+    asca_hostcopy* h = kind != Mem::pageable ? nullptr : hostcopy(ctx);
     if (!h) {
         ASCA_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         return ASCA_OK;

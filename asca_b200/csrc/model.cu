@@ -666,7 +666,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
             ASCA_TRY(decode_step_bf16_device(ctx, m, f, b, state, ns, step > 0, toks + step * ns));
     }
     if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)ns * V * 4));
-    if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, cur, (size_t)ns * 4));
+    if (next_h) ASCA_TRY(asca_copy_out(ctx, next_h, cur, (size_t)ns * 4));
     if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
@@ -715,7 +715,7 @@ static int decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t
         ASCA_TRY(rc);
     }
     if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)ns * V * 4));
-    if (next_h) ASCA_TRY(asca_stage_out(ctx, next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4));
+    if (next_h) ASCA_TRY(asca_copy_out(ctx, next_h, toks + (n_steps - 1) * ns, (size_t)ns * 4));
     if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
@@ -861,12 +861,12 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
         ASCA_TRY(gemm_tc::launch(ctx, th));
         mean_kernel<<<1, 1024, 0, ctx->stream>>>(dlogits, N, 1.0f / (float)N, loss_d);
         ASCA_CHECK_LAUNCH(ctx);
-        ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
+        ASCA_TRY(asca_copy_out(ctx, loss_h, loss_d, 4));
     } else {
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, V, d, h_final, d, W + m->head16, V, logits, V, nullptr, 0, BF));
         if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)N * V * 4));
         ASCA_TRY(cross_entropy_scaled(ctx, logits, tg, N, V, dlogits, loss_d, m->grad_scale));
-        ASCA_TRY(asca_stage_out(ctx, loss_h, loss_d, 4));
+        ASCA_TRY(asca_copy_out(ctx, loss_h, loss_d, 4));
         ASCA_TRY(asca_cast_bf16(ctx, dlogits, dl16, N * V));
     }
     ASCA_TRY(asca_gemm(ctx, ASCA_TN, d, V, N, h_final, d, dl16, V, G + m->head, V, nullptr, acc, BF));
@@ -1179,7 +1179,7 @@ static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* id
         if (p) p->runs++;
         ASCA_TRY(forward_backward_f32_device(ctx, m, ids, tg, B, T, acc, loss, logits));
     }
-    ASCA_TRY(asca_stage_out(ctx, loss_h, loss, 4));
+    ASCA_TRY(asca_copy_out(ctx, loss_h, loss, 4));
     if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)N * V * 4));
     return asca_ctx_sync(ctx);
 }
@@ -1611,7 +1611,7 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     if (next_h) {
         argmax_kernel<<<(unsigned)ceil_div64(ns, 8), 256, 0, ctx->stream>>>(logits, ns, (int)V, nxt);
         ASCA_CHECK_LAUNCH(ctx);
-        ASCA_TRY(asca_stage_out(ctx, next_h, nxt, (size_t)ns * 4));
+        ASCA_TRY(asca_copy_out(ctx, next_h, nxt, (size_t)ns * 4));
     }
     return asca_ctx_sync(ctx);
 }

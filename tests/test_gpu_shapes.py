@@ -161,6 +161,32 @@ def test_host_copies(gpu, n):
     assert not buf[n:].any()
 
 
+# A device address where a host array belongs is an error code, in both directions and at both copy forms, and the context goes
+# on working; pinned arrays are taken.
+def test_device_address_as_host_array_is_refused(gpu):
+    import ctypes as C
+    import torch
+    import asca_b200
+
+    n = 1 << 20
+    dev, back = torch.arange(2 * n, dtype=torch.uint8, device="cuda"), torch.zeros(n, dtype=torch.uint8).pin_memory()
+    torch.cuda.synchronize()
+    at = dev.data_ptr()
+    for size in (64, n):
+        for call in ("asca_memcpy_h2d", "asca_memcpy_d2h"):
+            with pytest.raises(asca_b200.AscaError, match="device address"):
+                gpu._call(call, gpu._ctx, C.c_void_p(at), C.c_void_p(at + n), C.c_size_t(size))
+        gpu._call("asca_memcpy_d2h", gpu._ctx, C.c_void_p(back.data_ptr()), C.c_void_p(at), C.c_size_t(size))
+        assert torch.equal(back[:size], dev[:size].cpu())
+    m = asca_b200.Model(gpu, 256, 64, 4, 1, 2, 64)
+    ids = np.zeros(4, np.uint32)
+    with pytest.raises(asca_b200.AscaError, match="device address"):
+        gpu._call("asca_model_forward_backward_host", gpu._ctx, m._h, C.c_void_p(ids.ctypes.data), C.c_void_p(ids.ctypes.data), C.c_int64(1),
+                  C.c_int64(4), C.c_void_p(at), None)
+    assert np.isfinite(m.forward_backward(ids, ids, 1))
+    m.free()
+
+
 # A repeated bf16 decode step is replayed as a graph; profiled calls launch directly. Same tokens and logits either way, for
 # two batch sizes in turn.
 def test_bf16_decode_graph_equals_direct_launches(orc, gpu):
