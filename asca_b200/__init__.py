@@ -49,6 +49,7 @@ def load() -> C.CDLL:
         _lib.asca_describe.restype = C.c_char_p
         _lib.asca_version.restype = C.c_char_p
         _lib.asca_launch_count.restype = C.c_int64
+        _lib.asca_graph_launch_count.restype = C.c_int64
         _lib.asca_delta_ckpt_floats.restype = C.c_int64
         _lib.asca_delta_ckpt_floats.argtypes = [C.c_int64] * 5
     return _lib
@@ -166,6 +167,10 @@ class Gpu:
 
     def launch_count(self) -> int:
         return int(self.lib.asca_launch_count(self._ctx))
+
+    def graph_launch_count(self) -> int:
+        """Replays of a recorded launch sequence as one CUDA graph (repeated small training steps, bf16 decode steps)."""
+        return int(self.lib.asca_graph_launch_count(self._ctx))
 
     def set_stream(self, cuda_stream: int | None):
         self._call("asca_ctx_set_stream", self._ctx, C.c_void_p(cuda_stream or 0))

@@ -20,7 +20,7 @@ struct asca_ctx {
     size_t smem_optin = 0;
     std::string err;
     std::string desc;
-    int64_t launches = 0;
+    int64_t launches = 0, graph_launches = 0;
     // Programmatic dependent launch: while set, launches made through asca_launch may start their prologue before the
     // previous kernel on the stream has finished (only kernels that execute pdl_wait() first are launched that way).
     bool pdl = false;

@@ -16,6 +16,8 @@ int asca_fail(asca_ctx* ctx, int code, const char* fmt, ...) {
 
 int asca_workspace(asca_ctx* ctx, size_t bytes, void** out) {
     if (bytes > ctx->ws_bytes) {
+        // (a captured sequence has run directly with the scratch it needs; waiting on a capturing stream would spoil the capture)
+        if (ctx->hold) return asca_fail(ctx, ASCA_ERR_CUDA, "the scratch cannot grow while a launch sequence is being captured");
         // growing the scratch must not race with kernels still reading the old one
         ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (ctx->ws) cudaFree(ctx->ws);
@@ -224,6 +226,7 @@ int asca_ctx_profile_work(asca_ctx* ctx, int index, double* work) {
 const char* asca_last_error(const asca_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 const char* asca_describe(asca_ctx* ctx) { return ctx ? ctx->desc.c_str() : "null context"; }
 int64_t asca_launch_count(const asca_ctx* ctx) { return ctx ? ctx->launches : 0; }
+int64_t asca_graph_launch_count(const asca_ctx* ctx) { return ctx ? ctx->graph_launches : 0; }
 
 static size_t size_class(size_t bytes) {
     size_t c = 256;
@@ -242,6 +245,10 @@ int asca_malloc(asca_ctx* ctx, size_t bytes, void** dptr) {
         ctx->pool.erase(it);
     } else {
         cudaError_t e = cudaMalloc(dptr, c);
+        if (e != cudaSuccess && ctx->hold) {   // inside a capture: neither wait nor free
+            cudaGetLastError();
+            return asca_fail(ctx, ASCA_ERR_OOM, "out of device memory while a launch sequence is being captured");
+        }
         if (e != cudaSuccess) {
             // give cached blocks back and retry once
             ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -656,6 +656,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         ASCA_CUDA(ctx, cudaMemsetAsync(p->counter, 0xff, 4, ctx->stream));
         for (int64_t step = 0; step < n_steps; ++step) ASCA_CUDA(ctx, cudaGraphLaunch(p->exec, ctx->stream));
         ctx->launches += p->launches * n_steps;
+        ctx->graph_launches += n_steps;
     } else {
         DecodeBufs b;
         ASCA_REQUIRE(ctx, b.take(bf, m, ns, n_steps), "model_decode_step: out of memory");
@@ -1143,7 +1144,6 @@ static asca_step_plan* find_plan(asca_ctx* ctx, asca_model* m, int64_t B, int64_
 static int capture_plan(asca_ctx* ctx, asca_model* m, asca_step_plan& p) {
     const int rc = capture(ctx, &p.exec, &p.launches, &p.held,
                            [&] { return forward_backward_f32_device(ctx, m, p.ids, p.tg, p.B, p.T, p.acc, p.loss, p.logits); });
-    p.ws_epoch = ctx->ws_epoch;
     p.broken = rc != ASCA_OK;
     return rc;
 }
@@ -1161,7 +1161,10 @@ static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* id
     ASCA_REQUIRE(ctx, ids && tg && loss && logits, "model_forward_backward: out of memory");
     ASCA_TRY(asca_copy_in(ctx, ids, ids_h, (size_t)N * 4));
     ASCA_TRY(asca_copy_in(ctx, tg, tg_h, (size_t)N * 4));
-    if (p && p->exec && p->ws_epoch != ctx->ws_epoch) {   // the scratch its kernels name has moved
+    // The scratch has moved since this shape's last run: a graph made before names the old one, and what is there now may be
+    // too small (or nothing, after a trim) -- a capture cannot make it grow, a direct run can.
+    const bool moved = p && p->ws_epoch != ctx->ws_epoch;
+    if (moved && p->exec) {
         cudaStreamSynchronize(ctx->stream);
         cudaGraphExecDestroy(p->exec);
         p->exec = nullptr;
@@ -1171,13 +1174,17 @@ static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* id
         }
     }
     // a shape seen a third time is one that repeats
-    if (p && !p->exec && p->runs >= 2) capture_plan(ctx, m, *p);
+    if (p && !p->exec && p->runs >= 2 && !moved) capture_plan(ctx, m, *p);
     if (p && p->exec) {
         ASCA_CUDA(ctx, cudaGraphLaunch(p->exec, ctx->stream));
         ctx->launches += p->launches;
+        ctx->graph_launches++;
     } else {
-        if (p) p->runs++;
         ASCA_TRY(forward_backward_f32_device(ctx, m, ids, tg, B, T, acc, loss, logits));
+        if (p) {
+            p->runs++;
+            p->ws_epoch = ctx->ws_epoch;
+        }
     }
     ASCA_TRY(asca_copy_out(ctx, loss_h, loss, 4));
     if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)N * V * 4));

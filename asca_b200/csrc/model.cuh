@@ -24,7 +24,8 @@ struct asca_step_plan {
     int runs = 0;               // direct runs so far
     cudaGraphExec_t exec = nullptr;
     bool broken = false;        // could not be captured
-    uint64_t ws_epoch = 0, stamp = 0;
+    uint64_t ws_epoch = 0;      // of the scratch that its last direct run, or its graph, worked with
+    uint64_t stamp = 0;
     int64_t launches = 0;
     std::vector<void*> held;
 };

@@ -58,6 +58,9 @@ const char* asca_last_error(const asca_ctx* ctx);
 const char* asca_describe(asca_ctx* ctx);
 /* Kernel launches issued through this context since creation (rust/src/cuda/mod.rs:25-33). */
 int64_t asca_launch_count(const asca_ctx* ctx);
+/* How many times a recorded sequence of them was replayed as a CUDA graph instead (a repeated small f32 training step, a
+ * repeated bf16 decode step); the kernels of a replay are counted above as well. */
+int64_t asca_graph_launch_count(const asca_ctx* ctx);
 /* Per-kernel timing for measurement harnesses (the role of the reference's ASCA_PROF scopes,
  * rust/src/prof.rs): while on, the delta-rule kernels and the tensor-core products are bracketed by CUDA events on the
  * context's stream. asca_ctx_profile(ctx, on) clears the record and switches it;

@@ -143,6 +143,40 @@ def test_f32_training_step_graph_equals_direct_launches(orc, gpu):
         assert np.array_equal(a, b)
 
 
+# The replay survives a scratch that moves: given back by a trim (between any two steps), or grown by another call.
+@pytest.mark.parametrize("before", [1, 2, 4])
+@pytest.mark.parametrize("how", ["trim", "grow"])
+def test_f32_training_step_graph_after_the_scratch_moved(orc, gpu, before, how):
+    import asca_b200
+
+    m = asca_b200.Model(gpu, 256, 64, 4, 2, 4, 256)
+    m.set_params(orc.Rng(5).normal(m.n, 0.02))
+    ids, tg = (orc.Rng(s).below(256, 384) for s in (1, 2))
+    gpu._call("asca_ctx_trim", gpu._ctx)
+
+    def step():
+        n = gpu.graph_launch_count()
+        m.zero_grads()
+        loss = m.forward_backward(ids, tg, 4)
+        return gpu.graph_launch_count() - n, loss, m.get()[1]
+
+    first = [step() for _ in range(before)]
+    assert [n for n, _, _ in first] == [0, 0, 1, 1][:before]
+    if how == "trim":
+        gpu._call("asca_ctx_trim", gpu._ctx)
+    else:   # a far larger expert layer takes a far larger scratch
+        x = np.zeros((20000, 256), np.float32)
+        _, dev = gpu.moe_forward_dev(x, np.zeros((256, 1024), np.float32), np.zeros(1024, np.float32), np.zeros((1024, 256), np.float32),
+                                     np.zeros(256, np.float32), np.zeros(20000, np.uint32), 512)
+        gpu.moe_bwd_dev(dev, x)
+        dev.free()
+    after = [step() for _ in range(4)]
+    assert after[0][0] == 0 and after[-1][0] == 1
+    for _, loss, g in after:
+        assert loss == first[0][1] and np.array_equal(g, first[0][2])
+    m.free()
+
+
 # Pageable host arrays around the sizes where the copies change form: staged, one piece more, one slot of the ring and one
 # byte more, more than the whole ring.
 @pytest.mark.parametrize("n", [1, 65536, 65537, 1 << 20, (1 << 20) + 1, (8 << 20) + 3, (19 << 20) + 70001])
