@@ -35,6 +35,7 @@ struct asca_ctx {
     // while a launch sequence is being captured into a graph: blocks the sequence gives back belong to the graph
     std::vector<void*>* hold = nullptr;
     cudaStream_t cap_stream = nullptr;
+    std::vector<struct asca_model*> planned;   // the models with plans whose buffers are this context's (model.cu)
     int* err_word = nullptr;  // device int the kernels with bounded waits write to
     // Pinned staging of small host arrays (ids, losses, tokens): copies that neither block the host nor wait for each
     // other; what goes out is handed to the caller's arrays by the asca_ctx_sync that ends the call.
@@ -142,6 +143,9 @@ struct asca_stage_scope {
     explicit asca_stage_scope(asca_ctx* c) : ctx(c) {}
     ~asca_stage_scope();
 };
+// Drops the plans made in this context, those a call is working with excepted; the caller has waited for the stream (model.cu).
+void asca_release_plans(asca_ctx* ctx);
+void asca_forget_planned(asca_ctx* ctx);   // the context is going: its models no longer know it
 // Returns scratch of at least `bytes` (256-byte aligned); contents are undefined.
 int asca_workspace(asca_ctx* ctx, size_t bytes, void** out);
 

@@ -14,6 +14,16 @@ int asca_fail(asca_ctx* ctx, int code, const char* fmt, ...) {
     return code;
 }
 
+// After a cudaMalloc that failed: gives back what is held for later use (idle plans, cached blocks).
+static int reclaim(asca_ctx* ctx) {
+    cudaGetLastError();
+    ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    asca_release_plans(ctx);
+    for (auto& kv : ctx->pool) cudaFree(kv.second);
+    ctx->pool.clear();
+    return ASCA_OK;
+}
+
 int asca_workspace(asca_ctx* ctx, size_t bytes, void** out) {
     if (bytes > ctx->ws_bytes) {
         // (a captured sequence has run directly with the scratch it needs; waiting on a capturing stream would spoil the capture)
@@ -25,7 +35,15 @@ int asca_workspace(asca_ctx* ctx, size_t bytes, void** out) {
         ctx->ws_bytes = 0;
         size_t want = (bytes + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1);
         ctx->ws_epoch++;
-        ASCA_CUDA(ctx, cudaMalloc(&ctx->ws, want));
+        if (cudaMalloc(&ctx->ws, want) != cudaSuccess) {
+            ctx->ws = nullptr;
+            ASCA_TRY(reclaim(ctx));
+            if (cudaMalloc(&ctx->ws, want) != cudaSuccess) {
+                ctx->ws = nullptr;
+                cudaGetLastError();   // (or the next launch would be taken for the one that failed)
+                return asca_fail(ctx, ASCA_ERR_OOM, "cannot allocate %zu bytes of scratch", want);
+            }
+        }
         ctx->ws_bytes = want;
     }
     *out = ctx->ws;
@@ -120,6 +138,8 @@ int asca_ctx_destroy(asca_ctx* ctx) {
     if (!ctx) return ASCA_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    asca_release_plans(ctx);
+    asca_forget_planned(ctx);
     for (auto& kv : ctx->pool) cudaFree(kv.second);
     for (auto& kv : ctx->live) cudaFree(kv.first);
     if (ctx->ws) cudaFree(ctx->ws);
@@ -180,9 +200,14 @@ int asca_ctx_trim(asca_ctx* ctx) {
     for (auto& e : ctx->dtiles)
         if (e.buf) cudaFree(e.buf);
     ctx->dtiles.clear();
+    asca_release_plans(ctx);   // (their buffers go to the pool)
     for (auto& kv : ctx->pool) cudaFree(kv.second);
     ctx->pool.clear();
     asca_hostcopy_free(ctx);
+    if (ctx->pin && ctx->pin_used == 0) {
+        cudaFreeHost(ctx->pin);
+        ctx->pin = nullptr;
+    }
     if (ctx->ws) cudaFree(ctx->ws);
     ctx->ws = nullptr;
     ctx->ws_bytes = 0;
@@ -245,17 +270,16 @@ int asca_malloc(asca_ctx* ctx, size_t bytes, void** dptr) {
         ctx->pool.erase(it);
     } else {
         cudaError_t e = cudaMalloc(dptr, c);
-        if (e != cudaSuccess && ctx->hold) {   // inside a capture: neither wait nor free
-            cudaGetLastError();
-            return asca_fail(ctx, ASCA_ERR_OOM, "out of device memory while a launch sequence is being captured");
-        }
         if (e != cudaSuccess) {
-            // give cached blocks back and retry once
-            ASCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            for (auto& kv : ctx->pool) cudaFree(kv.second);
-            ctx->pool.clear();
             cudaGetLastError();
-            ASCA_CUDA(ctx, cudaMalloc(dptr, c));
+            // (inside a capture there is neither waiting nor freeing)
+            if (ctx->hold) return asca_fail(ctx, ASCA_ERR_OOM, "out of device memory while a launch sequence is being captured");
+            ASCA_TRY(reclaim(ctx));
+            e = cudaMalloc(dptr, c);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                return asca_fail(ctx, ASCA_ERR_OOM, "cannot allocate %zu bytes of device memory", c);
+            }
         }
     }
     ctx->live[*dptr] = c;

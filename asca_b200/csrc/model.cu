@@ -529,13 +529,61 @@ static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeFor
     return ASCA_OK;
 }
 
-static void drop_decode_plan(asca_ctx* ctx, asca_decode_plan& p) {
+// A plan's graph and buffers go; the stream has been waited for.
+static void drop_plan(asca_plan& p) {
     if (p.exec) cudaGraphExecDestroy(p.exec);
     p.exec = nullptr;
-    if (ctx)
-        for (void* x : p.held) asca_free(ctx, x);
+    for (void* x : p.held) asca_free(p.ctx, x);
     p.held.clear();
 }
+template <class Plan>
+static void drop_idle_plans(std::list<Plan>& plans, asca_ctx* ctx) {
+    for (auto p = plans.begin(); p != plans.end();) {
+        if (p->ctx == ctx && !p->busy) {
+            drop_plan(*p);
+            p = plans.erase(p);
+        } else {
+            ++p;
+        }
+    }
+}
+void asca_release_plans(asca_ctx* ctx) {
+    for (asca_model* m : ctx->planned) {
+        drop_idle_plans(m->plans, ctx);
+        drop_idle_plans(m->dec_plans, ctx);
+    }
+}
+// A new plan of this model and context, in place of the least recently used beyond MAX_PLANS.
+template <class Plan>
+static Plan* new_plan(asca_ctx* ctx, asca_model* m, std::list<Plan>& plans, const Plan& from) {
+    if (plans.size() >= MAX_PLANS) {
+        auto old = std::min_element(plans.begin(), plans.end(), [](const Plan& a, const Plan& b) { return a.stamp < b.stamp; });
+        cudaStreamSynchronize(old->ctx->stream);
+        drop_plan(*old);
+        plans.erase(old);
+    }
+    plans.push_back(from);
+    plans.back().ctx = ctx;
+    if (std::find(ctx->planned.begin(), ctx->planned.end(), m) == ctx->planned.end()) {   // either outlives the other
+        ctx->planned.push_back(m);
+        m->planned_in.push_back(ctx);
+    }
+    return &plans.back();
+}
+void asca_forget_planned(asca_ctx* ctx) {
+    for (asca_model* m : ctx->planned) m->planned_in.erase(std::find(m->planned_in.begin(), m->planned_in.end(), ctx));
+    ctx->planned.clear();
+}
+struct PlanUse {   // keeps a plan while a call works with it
+    asca_plan* p = nullptr;
+    void take(asca_plan* p_) {
+        p = p_;
+        if (p) p->busy = true;
+    }
+    ~PlanUse() {
+        if (p) p->busy = false;
+    }
+};
 
 // Captures `body` (launches on ctx->stream) into an executable graph, on a stream of the context's own: the caller's may be
 // one that cannot be captured. Blocks the sequence gives back meanwhile go to `held`.
@@ -612,26 +660,19 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
     // A step is some eighty launches, each with its tensor maps: half a millisecond of host time, which is what a small batch's
     // step takes. A (state, streams) pair that comes a third time is replayed as a graph, one launch a step.
     asca_decode_plan* p = nullptr;
+    PlanUse use;
     if (f.packed && f.one_prologue && !ctx->profiling) {
         for (auto& q : m->dec_plans)
-            if (q.ns == ns && q.state == state && q.cap >= n_steps && q.w16 == W && q.dec_w == m->dec_w && q.dec_pk == m->dec_pk) p = &q;
+            if (q.ctx == ctx && q.ns == ns && q.state == state && q.cap >= n_steps && q.w16 == W && q.dec_w == m->dec_w && q.dec_pk == m->dec_pk) p = &q;
         if (!p) {
-            if (m->dec_plans.size() >= MAX_PLANS) {
-                size_t old = 0;
-                for (size_t i = 1; i < m->dec_plans.size(); ++i)
-                    if (m->dec_plans[i].stamp < m->dec_plans[old].stamp) old = i;
-                cudaStreamSynchronize(ctx->stream);
-                drop_decode_plan(ctx, m->dec_plans[old]);
-                m->dec_plans.erase(m->dec_plans.begin() + old);
-            }
             asca_decode_plan q;
             q.ns = ns; q.state = state; q.w16 = W; q.dec_w = m->dec_w; q.dec_pk = m->dec_pk;
             q.cap = 1;
             while (q.cap < n_steps) q.cap *= 2;
-            m->dec_plans.push_back(q);
-            p = &m->dec_plans.back();
+            p = new_plan(ctx, m, m->dec_plans, q);
         }
         p->stamp = ++m->plan_clock;
+        use.take(p);
         if (!p->exec && !p->broken && p->runs >= 2) {
             DecodeBufs pb;
             Bufs own(ctx);
@@ -1099,46 +1140,31 @@ static int forward_backward_f32_device(asca_ctx* ctx, asca_model* m, const uint3
     return ASCA_OK;
 }
 
-static void drop_plan(asca_ctx* ctx, asca_step_plan& p) {
-    if (p.exec) cudaGraphExecDestroy(p.exec);
-    p.exec = nullptr;
-    if (ctx)
-        for (void* b : p.held) asca_free(ctx, b);
-    p.held.clear();
-}
-
-// The plan of this call, or null where a graph is not for it: large batches (their kernels outlast their launches), callers
-// that want to be told of finished gradient ranges, profiling.
+// The plan of this call, or null where a graph is not for it: large batches (their kernels outlast their launches; also what
+// bounds a plan's memory: 256 MiB of activations, 64 MiB of logits and their gradients), callers that want to be told of finished
+// gradient ranges, profiling.
 static asca_step_plan* find_plan(asca_ctx* ctx, asca_model* m, int64_t B, int64_t T, int acc) {
     const int64_t N = B * T;
-    if (m->grad_hook || m->dp || ctx->profiling || N * m->L * (10 * m->d + 2 * m->F) * 4 > ((int64_t)256 << 20)) return nullptr;
+    if (m->grad_hook || m->dp || ctx->profiling) return nullptr;
+    if (N * m->L * (10 * m->d + 2 * m->F) * 4 > ((int64_t)256 << 20) || N * m->vocab * 8 > ((int64_t)64 << 20)) return nullptr;
     for (auto& p : m->plans)
-        if (p.B == B && p.T == T && p.acc == acc && p.grad_scale == m->grad_scale) {
+        if (p.ctx == ctx && p.B == B && p.T == T && p.acc == acc && p.grad_scale == m->grad_scale) {
             p.stamp = ++m->plan_clock;
             return p.broken ? nullptr : &p;
         }
-    if (m->plans.size() >= MAX_PLANS) {
-        size_t old = 0;
-        for (size_t i = 1; i < m->plans.size(); ++i)
-            if (m->plans[i].stamp < m->plans[old].stamp) old = i;
-        cudaStreamSynchronize(ctx->stream);
-        drop_plan(ctx, m->plans[old]);
-        m->plans.erase(m->plans.begin() + old);
-    }
     asca_step_plan p;
-    p.B = B; p.T = T; p.acc = acc; p.grad_scale = m->grad_scale; p.stamp = ++m->plan_clock;
+    p.ctx = ctx; p.B = B; p.T = T; p.acc = acc; p.grad_scale = m->grad_scale; p.stamp = ++m->plan_clock;
     void* at[4] = {};
     const size_t bytes[4] = {(size_t)N * 4, (size_t)N * 4, 4, (size_t)N * m->vocab * 4};
     for (int i = 0; i < 4; ++i) {
         if (asca_malloc(ctx, bytes[i], &at[i]) != ASCA_OK) {
-            drop_plan(ctx, p);
+            drop_plan(p);
             return nullptr;
         }
         p.held.push_back(at[i]);
     }
     p.ids = (uint32_t*)at[0]; p.tg = (uint32_t*)at[1]; p.loss = (float*)at[2]; p.logits = (float*)at[3];
-    m->plans.push_back(p);
-    return &m->plans.back();
+    return new_plan(ctx, m, m->plans, p);
 }
 
 static int capture_plan(asca_ctx* ctx, asca_model* m, asca_step_plan& p) {
@@ -1156,6 +1182,8 @@ static int forward_backward_f32(asca_ctx* ctx, asca_model* m, const uint32_t* id
     asca_stage_scope staged(ctx);
     Bufs bf(ctx);
     asca_step_plan* p = find_plan(ctx, m, B, T, acc);
+    PlanUse use;
+    use.take(p);
     uint32_t *ids = p ? p->ids : (uint32_t*)bf.f(N), *tg = p ? p->tg : (uint32_t*)bf.f(N);
     float *loss = p ? p->loss : bf.f(1), *logits = p ? p->logits : bf.f(N * V);
     ASCA_REQUIRE(ctx, ids && tg && loss && logits, "model_forward_backward: out of memory");
@@ -1306,8 +1334,12 @@ int asca_model_create(asca_ctx* ctx, int64_t vocab, int64_t d, int64_t H, int64_
 int asca_model_destroy(asca_ctx* ctx, asca_model* m) {
     if (!m) return ASCA_OK;
     if (ctx) cudaStreamSynchronize(ctx->stream);
-    for (auto& p : m->plans) drop_plan(ctx, p);
-    for (auto& p : m->dec_plans) drop_decode_plan(ctx, p);
+    for (asca_ctx* c : m->planned_in) {
+        cudaStreamSynchronize(c->stream);
+        c->planned.erase(std::find(c->planned.begin(), c->planned.end(), m));
+    }
+    for (auto& p : m->plans) drop_plan(p);
+    for (auto& p : m->dec_plans) drop_plan(p);
     if (m->dp) asca_dp_free(m);   // before the buffers its copies and collectives touch
     for (float* b : {m->params, m->grads, m->m, m->v})
         if (b) cudaFree(b);

@@ -4,6 +4,7 @@
 #pragma once
 #include "common.cuh"
 
+#include <list>
 #include <vector>
 
 struct Lyr {
@@ -12,39 +13,40 @@ struct Lyr {
 
 struct asca_dp;   // dp.cu
 
-// A small model's training step replayed as one graph launch: its dozens of kernels take microseconds each, less than the
-// host needs to launch them one by one. One per (batch shape, first or later backward, gradient scale), least recently used
-// dropped beyond MAX_PLANS; a plan owns the buffers its graph names.
-struct asca_step_plan {
-    int64_t B = 0, T = 0;
-    int acc = 0;
-    float grad_scale = 0.0f;
-    uint32_t *ids = nullptr, *tg = nullptr;
-    float *loss = nullptr, *logits = nullptr;
+// A launch sequence replayed as one graph. A plan owns the buffers its graph names; they come from the context that made it, and
+// go back to it with the plan: when it is the least recently used of more than MAX_PLANS, with asca_ctx_trim, where the
+// device runs out of memory (while no call works with it), with its model or with its context.
+struct asca_plan {
+    asca_ctx* ctx = nullptr;
     int runs = 0;               // direct runs so far
     cudaGraphExec_t exec = nullptr;
     bool broken = false;        // could not be captured
-    uint64_t ws_epoch = 0;      // of the scratch that its last direct run, or its graph, worked with
+    bool busy = false;          // a call is working with it
     uint64_t stamp = 0;
     int64_t launches = 0;
     std::vector<void*> held;
 };
 constexpr size_t MAX_PLANS = 8;
 
+// A small model's training step: its dozens of kernels take microseconds each, less than the host needs to launch them one by
+// one. One per (batch shape, first or later backward, gradient scale).
+struct asca_step_plan : asca_plan {
+    int64_t B = 0, T = 0;
+    int acc = 0;
+    float grad_scale = 0.0f;
+    uint32_t *ids = nullptr, *tg = nullptr;
+    float *loss = nullptr, *logits = nullptr;
+    uint64_t ws_epoch = 0;      // of the scratch that its last direct run, or its graph, worked with
+};
+
 // The same for a bf16 decode step on the packed weights: one graph is one step, its tokens in and out through `cur`.
-struct asca_decode_plan {
+struct asca_decode_plan : asca_plan {
     int64_t ns = 0, cap = 0;    // streams; tokens of how many steps `toks` holds
     const void* state = nullptr;
     const void *w16 = nullptr, *dec_w = nullptr, *dec_pk = nullptr;   // the weight copies the graph reads
     uint32_t *cur = nullptr, *toks = nullptr;
     int32_t* counter = nullptr;
     float* logits = nullptr;
-    int runs = 0;
-    cudaGraphExec_t exec = nullptr;
-    bool broken = false;
-    uint64_t stamp = 0;
-    int64_t launches = 0;
-    std::vector<void*> held;
 };
 
 struct asca_model {
@@ -83,8 +85,9 @@ struct asca_model {
     // bf16 mode, vocabulary 256: let the head product's epilogue take the cross-entropy (loss and bf16 dlogits) where
     // it runs on CTA pairs and the caller does not ask for the logits (asca_model_set_fused_head)
     bool fused_head = true;
-    std::vector<asca_step_plan> plans;
-    std::vector<asca_decode_plan> dec_plans;
+    std::list<asca_step_plan> plans;
+    std::list<asca_decode_plan> dec_plans;
+    std::vector<asca_ctx*> planned_in;   // the contexts whose `planned` names this model
     uint64_t plan_clock = 0;
     // data parallelism (dp.cu): the communicator attached to this model and what is in flight on its side stream
     asca_dp* dp = nullptr;

@@ -78,10 +78,13 @@ int asca_selftest_wait_timeout(asca_ctx* ctx, int64_t limit_cycles, int* gave_up
 /* Library version string and the arch it was compiled for ("sm_100a"). */
 const char* asca_version(void);
 
-/* Memory the context holds beyond what the caller sees: freed asca_malloc blocks (cached per size class),
- * the grow-only scratch of the kernels, and the tiles the tensor-core delta forward keeps for its backward
- * (at most `bytes` of them, default 32 GiB, least recently used set reused beyond that).
- * asca_ctx_trim synchronises the stream and gives all three back to the driver. */
+/* Memory the context holds beyond what the caller sees: freed asca_malloc blocks (cached per size class), the grow-only
+ * scratch of the kernels, the tiles the tensor-core delta forward keeps for its backward (at most `bytes` of them, default
+ * 32 GiB, least recently used set reused beyond that), what models keep to replay a repeated step as a CUDA graph (at most eight
+ * training shapes of 320 MiB and eight decode shapes a model, least recently used first), and for host arrays a pinned staging
+ * area of 1 MiB and an 8 MiB ring with its copy threads. asca_ctx_trim synchronises the stream and gives all of it back; what a
+ * later call needs is made again (a repeated step is recorded anew). Idle graphs and cached blocks also go when the device
+ * runs out of memory. */
 int asca_ctx_trim(asca_ctx* ctx);
 int asca_ctx_set_tile_cache_bytes(asca_ctx* ctx, size_t bytes);
 

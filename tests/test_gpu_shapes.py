@@ -177,6 +177,53 @@ def test_f32_training_step_graph_after_the_scratch_moved(orc, gpu, before, how):
     m.free()
 
 
+# A trim gives back what the replayed steps hold (a training plan of 80 MB, a decode plan), and both go on afterwards with the
+# results they had; a model may go before or after the context that its plans came from.
+def test_trim_gives_back_the_replayed_steps(orc, gpu):
+    import torch
+    import asca_b200
+
+    ids, tg = (orc.Rng(s).below(256, 8192) for s in (1, 2))
+
+    def work(m, st):
+        st.zero_()
+        m.set_compute(asca_b200.F32)
+        m.zero_grads()
+        out = [m.forward_backward(ids, tg, 16), m.get()[1]]
+        m.set_compute(asca_b200.BF16)
+        return out + [m.decode_greedy(st, ids[:64].copy(), 40)]
+
+    def free():
+        gpu._call("asca_ctx_trim", gpu._ctx)
+        return torch.cuda.mem_get_info()[0]
+
+    for rest in range(2):   # (the first round loads the kernels)
+        m = asca_b200.Model(gpu, 256, 128, 2, 2, 4, 256)
+        m.set_params(orc.Rng(5).normal(m.n, 0.05))
+        st = m.new_decode_state(64)
+        first = work(m, st)
+        before = free()
+        n = gpu.graph_launch_count()
+        for _ in range(3):
+            work(m, st)
+        assert gpu.graph_launch_count() > n + 40
+        if rest:
+            assert before - free() < 16 << 20
+        for a, b in zip(first, work(m, st)):
+            assert np.array_equal(a, b)
+        m.free()
+
+    for model_first in (True, False):
+        g2 = asca_b200.Gpu(0)
+        m = asca_b200.Model(g2, 256, 64, 4, 1, 2, 64)
+        m.set_params(orc.Rng(5).normal(m.n, 0.05))
+        for _ in range(4):
+            loss = m.forward_backward(ids[:64], tg[:64], 1)
+        assert g2.graph_launch_count() > 0 and np.isfinite(loss)
+        (m.free if model_first else g2.close)()
+        (g2.close if model_first else m.free)()
+
+
 # Pageable host arrays around the sizes where the copies change form: staged, one piece more, one slot of the ring and one
 # byte more, more than the whole ring.
 @pytest.mark.parametrize("n", [1, 65536, 65537, 1 << 20, (1 << 20) + 1, (8 << 20) + 3, (19 << 20) + 70001])
