@@ -419,25 +419,7 @@ static int refresh_dec_w(asca_ctx* ctx, asca_model* m) {
     return ASCA_OK;
 }
 
-// The buffers of a decode step; cur: the step's token ids in, its argmax out.
 namespace {
-struct DecodeBufs {
-    uint32_t *cur, *toks;
-    int32_t *perm, *offs, *inv_perm, *counter;
-    float *x, *qkv, *gate, *o, *y, *x_mid, *mo, *logits, *pre_p, *qg;
-    __nv_bfloat16 *x16, *o16, *xn16, *hid16, *hf16;
-    bool take(Bufs& bf, const asca_model* m, int64_t ns, int64_t n_steps) {
-        const int64_t d = m->d, H = m->H, F = m->F, ldq = (3 * d + 2 * H + 7) & ~(int64_t)7;
-        auto h16 = [&](int64_t n) { return (__nv_bfloat16*)bf.f((n + 1) / 2); };
-        cur = (uint32_t*)bf.f(ns); toks = (uint32_t*)bf.f(ns * n_steps);
-        perm = (int32_t*)bf.f(ns); offs = (int32_t*)bf.f(m->E + 1); inv_perm = (int32_t*)bf.f(ns); counter = (int32_t*)bf.f(1);
-        x = bf.f(ns * d); qkv = bf.f(ns * 3 * d); gate = bf.f(ns * 2 * H); o = bf.f(ns * d); y = bf.f(ns * d); x_mid = bf.f(ns * d);
-        mo = bf.f(ns * d); logits = bf.f(ns * m->vocab); pre_p = bf.f(ns * F); qg = bf.f(ns * ldq);
-        x16 = h16(ns * d); o16 = h16(ns * d); xn16 = h16(ns * d); hid16 = h16(ns * F); hf16 = h16(ns * d);
-        return cur && toks && perm && offs && inv_perm && counter && x && qkv && gate && o && y && x_mid && mo && logits && pre_p && qg && x16 &&
-               o16 && xn16 && hid16 && hf16;
-    }
-};
 // Which form of the step the shapes allow. fused64: head dim 64 (one projection for qkv + gate, the warp-per-head state update,
 // casts folded in). sorted_moe: with a handful of tokens per expert the MoE runs on rows in expert order end to end -- the norm
 // writes its bf16 rows at their expert-order position (the gather), and the second expert product adds into the residual rows
@@ -448,6 +430,32 @@ struct DecodeBufs {
 struct DecodeForm {
     bool fused64, sorted_moe, packed, one_prologue;
     int64_t ldq, r_qg, r_o, r_w1, r_w2, r_layer, r_head;
+};
+// The buffers of a decode step; cur: the step's token ids in, its argmax out.
+struct DecodeBufs {
+    uint32_t *cur, *toks;
+    int32_t *perm, *offs, *inv_perm, *counter;
+    float *x, *qkv, *gate, *o, *y, *x_mid, *mo, *logits, *pre_p, *qg;
+    __nv_bfloat16 *x16, *o16, *xn16, *hid16, *hf16;
+    // (a buffer that the form of the step has no use for stays null)
+    bool take(Bufs& bf, const asca_model* m, const DecodeForm& f, int64_t ns, int64_t n_steps) {
+        const int64_t d = m->d, H = m->H, F = m->F;
+        bool ok = true;
+        auto f32 = [&](int64_t n, bool wanted = true) -> float* {
+            float* p = wanted ? bf.f(n) : nullptr;
+            ok = ok && (p || !wanted);
+            return p;
+        };
+        auto i32 = [&](int64_t n, bool wanted = true) { return (int32_t*)f32(n, wanted); };
+        auto h16 = [&](int64_t n) { return (__nv_bfloat16*)f32((n + 1) / 2); };
+        cur = (uint32_t*)f32(ns); toks = (uint32_t*)f32(ns * n_steps);
+        perm = i32(ns); offs = i32(m->E + 1); inv_perm = i32(ns, f.sorted_moe); counter = i32(1);
+        x = f32(ns * d); o = f32(ns * d); y = f32(ns * d); logits = f32(ns * m->vocab);
+        qg = f32(ns * f.ldq, f.fused64); qkv = f32(ns * 3 * d, !f.fused64); gate = f32(ns * 2 * H, !f.fused64);
+        x_mid = f32(ns * d, !f.sorted_moe); mo = f32(ns * d, !f.sorted_moe); pre_p = f32(ns * F, !f.sorted_moe);
+        x16 = h16(ns * d); o16 = h16(ns * d); xn16 = h16(ns * d); hid16 = h16(ns * F); hf16 = h16(ns * d);
+        return ok;
+    }
 };
 }  // namespace
 
@@ -676,7 +684,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         if (!p->exec && !p->broken && p->runs >= 2) {
             DecodeBufs pb;
             Bufs own(ctx);
-            int rc = pb.take(own, m, ns, p->cap) ? ASCA_OK : ASCA_ERR_OOM;
+            int rc = pb.take(own, m, f, ns, p->cap) ? ASCA_OK : ASCA_ERR_OOM;
             if (rc == ASCA_OK)
                 rc = capture(ctx, &p->exec, &p->launches, &p->held, [&] { return decode_step_bf16_device(ctx, m, f, pb, state, ns, false, nullptr); });
             if (rc == ASCA_OK) {
@@ -700,7 +708,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         ctx->graph_launches += n_steps;
     } else {
         DecodeBufs b;
-        ASCA_REQUIRE(ctx, b.take(bf, m, ns, n_steps), "model_decode_step: out of memory");
+        ASCA_REQUIRE(ctx, b.take(bf, m, f, ns, n_steps), "model_decode_step: out of memory");
         cur = b.cur; toks = b.toks; logits = b.logits;
         ASCA_TRY(asca_stage_in(ctx, cur, ids_h, (size_t)ns * 4));
         ASCA_CUDA(ctx, cudaMemsetAsync(b.counter, 0xff, 4, ctx->stream));

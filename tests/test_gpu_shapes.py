@@ -224,6 +224,23 @@ def test_trim_gives_back_the_replayed_steps(orc, gpu):
         (g2.close if model_first else m.free)()
 
 
+# A bf16 decode step takes the buffers of its own form only: no f32 pre-activations (16 MB here) beside the packed products.
+def test_bf16_decode_takes_the_buffers_of_its_form(orc, gpu):
+    import torch
+    import asca_b200
+
+    m = asca_b200.Model(gpu, 256, 128, 2, 1, 4, 16384)
+    m.set_params(orc.Rng(9).normal(m.n, 0.02))
+    m.set_compute(asca_b200.BF16)
+    st, ids = m.new_decode_state(256), orc.Rng(3).below(256, 256)
+    m.decode_step(st, ids)   # loads the kernels, makes the weight copies
+    gpu._call("asca_ctx_trim", gpu._ctx)
+    before = torch.cuda.mem_get_info()[0]
+    m.decode_step(st, ids)
+    assert before - torch.cuda.mem_get_info()[0] < 16 << 20
+    m.free()
+
+
 # Pageable host arrays around the sizes where the copies change form: staged, one piece more, one slot of the ring and one
 # byte more, more than the whole ring.
 @pytest.mark.parametrize("n", [1, 65536, 65537, 1 << 20, (1 << 20) + 1, (8 << 20) + 3, (19 << 20) + 70001])
