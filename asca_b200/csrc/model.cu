@@ -835,11 +835,11 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
     std::vector<Act> acts(L);
     const int64_t nck = asca_delta_ckpt_floats(B, T, H, dh, CH);
     float* x = bf.f(N * d);
-    float* qkv = bf.f(N * 3 * d);
+    float* qkv = nullptr;   // only where the projection's epilogue does not write q, k and v itself
     float* gate = bf.f(N * 2 * H);
     float* y = bf.f(N * d);
     float* mo = bf.f(N * d);
-    ASCA_REQUIRE(ctx, x && qkv && gate && y && mo, "model_forward_backward: out of memory");
+    ASCA_REQUIRE(ctx, x && gate && y && mo, "model_forward_backward: out of memory");
     ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, x));
     const bool vec4 = (d & 3) == 0;
     const unsigned add_grid = (unsigned)std::min<int64_t>(ceil_div64(N * d / 4, 256), 148 * 16);
@@ -860,7 +860,7 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
         gemm_tc::Args tq{};
         tq.mode = ASCA_NN; tq.A = a.x_in; tq.lda = d; tq.a_rows = N; tq.a_cols = d;
         tq.B = W + w16.w_qkv; tq.ldb = 3 * d; tq.b_rows = d; tq.b_cols = 3 * d;
-        tq.C = qkv; tq.ldc = 3 * d; tq.M = (int)N; tq.N = (int)(3 * d); tq.K = (int)d;
+        tq.ldc = 3 * d; tq.M = (int)N; tq.N = (int)(3 * d); tq.K = (int)d;
         tq.bias = P + w.b_qkv; tq.group_dim = gemm_tc::GROUP_NONE; tq.epi = gemm_tc::EPI_QKV;
         tq.qkv_q = a.q; tq.qkv_k = a.k; tq.qkv_v = a.v; tq.qkv_qn = a.qn; tq.qkv_kn = a.kn; tq.qkv_d = (int)d; tq.qkv_dh = (int)dh;
         ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 2 * H, d, a.x_in, d, W + w16.w_gate, 2 * H, gate, 2 * H, P + w.b_gate, 0, BF));
@@ -869,6 +869,8 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
             gate_sigmoid_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(N * H, 256), 148 * 8), 256, 0, ctx->stream>>>(gate, N * H, (int)H, a.al, a.be);
             ASCA_CHECK_LAUNCH(ctx);
         } else {
+            if (!qkv) qkv = bf.f(N * 3 * d);
+            ASCA_REQUIRE(ctx, qkv, "model_forward_backward: out of memory");
             ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 3 * d, d, a.x_in, d, W + w16.w_qkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, BF));
             ASCA_TRY(asca_delta_prep_bf16(ctx, qkv, gate, N, H, dh, a.q, a.k, a.v, a.qn, a.kn, a.al, a.be));
         }
@@ -1580,14 +1582,14 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     int32_t* offs = (int32_t*)bf.f(E + 1);
     int32_t* last = (int32_t*)bf.f(ns);
     uint32_t* nxt = (uint32_t*)bf.f(ns);
-    float *x = bf.f(N * d), *qkv = bf.f(N * 3 * d), *gate = bf.f(N * 2 * H), *y = bf.f(N * d), *x_mid = bf.f(N * d), *mo = bf.f(N * d);
-    float *qn = bf.f(N * H), *kn = bf.f(N * H), *al = bf.f(N * H), *be = bf.f(N * H), *pre_p = nullptr;
+    float *x = bf.f(N * d), *gate = bf.f(N * 2 * H), *y = bf.f(N * d), *x_mid = bf.f(N * d), *mo = bf.f(N * d);
+    float *qn = bf.f(N * H), *kn = bf.f(N * H), *al = bf.f(N * H), *be = bf.f(N * H), *qkv = nullptr, *pre_p = nullptr;   // (two where they are needed)
     float *xl = bf.f(ns * d), *hf = bf.f(ns * d), *logits = bf.f(ns * V);
     // activations a product reads: bf16 in bf16 mode, f32 otherwise (same element counts)
     auto act = [&](int64_t n) { return bfm ? (void*)h16(n) : (void*)bf.f(n); };
     void *x_in = bfm ? act(N * d) : nullptr, *q = act(N * d), *k = act(N * d), *v = act(N * d), *o = act(N * d), *xn = act(N * d),
          *hid_p = act(N * F), *hf_in = bfm ? act(ns * d) : nullptr;
-    ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && qkv && gate && y && x_mid && mo && qn && kn && al && be &&
+    ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && gate && y && x_mid && mo && qn && kn && al && be &&
                           xl && hf && logits && q && k && v && o && xn && hid_p && (!bfm || (x_in && hf_in)),
                  "model_prefill: out of memory");
     asca_stage_scope staged(ctx);
@@ -1617,7 +1619,11 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
             tq.qkv_q = (bf16*)q; tq.qkv_k = (bf16*)k; tq.qkv_v = (bf16*)v; tq.qkv_qn = qn; tq.qkv_kn = kn; tq.qkv_d = (int)d; tq.qkv_dh = (int)dh;
         }
         const bool fused = bfm && m->fused_qkv && asca_tc_enabled() && gemm_tc::qkv_fusable(ctx, tq);
-        if (!fused) ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 3 * d, d, xi, d, Wqkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, DT));
+        if (!fused) {
+            if (!qkv) qkv = bf.f(N * 3 * d);
+            ASCA_REQUIRE(ctx, qkv, "model_prefill: out of memory");
+            ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, 3 * d, d, xi, d, Wqkv, 3 * d, qkv, 3 * d, P + w.b_qkv, 0, DT));
+        }
         if (fused) {
             ASCA_TRY(gemm_tc::launch(ctx, tq));
             gate_sigmoid_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(N * H, 256), 148 * 8), 256, 0, ctx->stream>>>(gate, N * H, (int)H, al, be);

@@ -241,6 +241,31 @@ def test_bf16_decode_takes_the_buffers_of_its_form(orc, gpu):
     m.free()
 
 
+# Where the projection's epilogue writes q, k and v, the f32 qkv matrix (50 MB here) is not allocated.
+@pytest.mark.parametrize("what", ["train", "prefill"])
+def test_fused_qkv_allocates_no_f32_matrix(orc, gpu, what):
+    import torch
+    import asca_b200
+
+    m = asca_b200.Model(gpu, 256, 256, 2, 1, 4, 256)
+    m.set_params(orc.Rng(9).normal(m.n, 0.05))
+    m.set_compute(asca_b200.BF16)
+    ids = orc.Rng(3).below(256, 16384)
+    used = {}
+    for fused in (False, True, False, True):   # (the first two load the kernels)
+        m.set_fused_qkv(fused)
+        gpu._call("asca_ctx_trim", gpu._ctx)
+        before = torch.cuda.mem_get_info()[0]
+        if what == "train":
+            m.zero_grads()
+            m.forward_backward(ids, ids, 4)
+        else:
+            m.prefill(m.new_decode_state(4), ids.reshape(4, -1))
+        used[fused] = before - torch.cuda.mem_get_info()[0]
+    assert used[False] - used[True] > 40 << 20
+    m.free()
+
+
 # Pageable host arrays around the sizes where the copies change form: staged, one piece more, one slot of the ring and one
 # byte more, more than the whole ring.
 @pytest.mark.parametrize("n", [1, 65536, 65537, 1 << 20, (1 << 20) + 1, (8 << 20) + 3, (19 << 20) + 70001])
