@@ -5,6 +5,8 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cstddef>
+#include <cstring>
 #include <initializer_list>
 
 #include "gemm_simt.cuh"
@@ -431,9 +433,16 @@ struct DecodeForm {
     bool fused64, sorted_moe, packed, one_prologue;
     int64_t ldq, r_qg, r_o, r_w1, r_w2, r_layer, r_head;
 };
+// What a decode call uploads in one copy, the first tokens behind it.
+struct DecodeIn {
+    int64_t state;     // where the states are, in floats behind this record
+    int32_t counter;   // row of the token buffer, advanced by the prologue of each step
+    int32_t unused;
+};
 // The buffers of a decode step; cur: the step's token ids in, its argmax out.
 struct DecodeBufs {
-    uint32_t *cur, *toks;
+    uint32_t *in, *cur, *toks;
+    const int64_t* state_off;
     int32_t *perm, *offs, *inv_perm, *counter;
     float *x, *qkv, *gate, *o, *y, *x_mid, *mo, *logits, *pre_p, *qg;
     __nv_bfloat16 *x16, *o16, *xn16, *hid16, *hf16;
@@ -448,8 +457,10 @@ struct DecodeBufs {
         };
         auto i32 = [&](int64_t n, bool wanted = true) { return (int32_t*)f32(n, wanted); };
         auto h16 = [&](int64_t n) { return (__nv_bfloat16*)f32((n + 1) / 2); };
-        cur = (uint32_t*)f32(ns); toks = (uint32_t*)f32(ns * n_steps);
-        perm = i32(ns); offs = i32(m->E + 1); inv_perm = i32(ns, f.sorted_moe); counter = i32(1);
+        constexpr int64_t HEAD = sizeof(DecodeIn) / 4;
+        in = (uint32_t*)f32(HEAD + ns); cur = in + HEAD; toks = (uint32_t*)f32(ns * n_steps);
+        state_off = reinterpret_cast<const int64_t*>(in); counter = reinterpret_cast<int32_t*>(in) + offsetof(DecodeIn, counter) / 4;
+        perm = i32(ns); offs = i32(m->E + 1); inv_perm = i32(ns, f.sorted_moe);
         x = f32(ns * d); o = f32(ns * d); y = f32(ns * d); logits = f32(ns * m->vocab);
         qg = f32(ns * f.ldq, f.fused64); qkv = f32(ns * 3 * d, !f.fused64); gate = f32(ns * 2 * H, !f.fused64);
         x_mid = f32(ns * d, !f.sorted_moe); mo = f32(ns * d, !f.sorted_moe); pre_p = f32(ns * F, !f.sorted_moe);
@@ -459,7 +470,11 @@ struct DecodeBufs {
 };
 }  // namespace
 
+int asca_delta_step_at(asca_ctx* ctx, const float* qkv, int64_t ld_qkv, const float* gate, int64_t ld_gate, float* S, const int64_t* S_off,
+                       int64_t n_streams, int64_t H, float* o, void* o16);   // delta_fwd.cu
+
 // One decode step from b.cur; the choice lands in b.cur and in the token buffer (toks_row where the prologue does not count).
+// state null (the fused64 form only): the states are where b.state_off says.
 static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeForm& f, const DecodeBufs& b, float* state, int64_t ns,
                                    bool pdl_first, uint32_t* toks_row) {
     typedef __nv_bfloat16 bf16;
@@ -506,7 +521,9 @@ static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeFor
         if (f.fused64) {
             if (f.packed) ASCA_TRY(few_rows(b.x16, d, m->dec_pk + li * f.r_layer * 64, ldq, b.qg, ldq, m->dec_b + li * ldq));
             else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, ldq, d, b.x16, d, m->dec_w + li * d * ldq, ldq, b.qg, ldq, m->dec_b + li * ldq, 0, BF));
-            ASCA_TRY(asca_delta_step_strided(ctx, b.qg, ldq, b.qg + 3 * d, ldq, state + li * ns * H * dh * dh, ns, H, b.o, b.o16));
+            const int64_t at = li * ns * H * dh * dh;
+            ASCA_TRY(asca_delta_step_at(ctx, b.qg, ldq, b.qg + 3 * d, ldq, (state ? state : (float*)b.in) + at, state ? nullptr : b.state_off, ns, H,
+                                        b.o, b.o16));
         } else {
             ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 3 * d, d, b.x16, d, W + w16.w_qkv, 3 * d, b.qkv, 3 * d, P + w.b_qkv, 0, BF));
             ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 2 * H, d, b.x16, d, W + w16.w_gate, 2 * H, b.gate, 2 * H, P + w.b_gate, 0, BF));
@@ -665,18 +682,24 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         ASCA_TRY(gemm_tc::skinny_pack(ctx, W + m->head16, V, 1, 0, 0, d, V, m->dec_pk + m->L * f.r_layer * 64));
         m->dec_pk_stale = false;
     }
+    std::vector<uint32_t> in(sizeof(DecodeIn) / 4 + ns);
+    auto upload = [&](uint32_t* to) {
+        const DecodeIn head = {(int64_t)(reinterpret_cast<intptr_t>(state) - reinterpret_cast<intptr_t>(to)) / 4, -1, 0};
+        memcpy(in.data(), &head, sizeof head);
+        memcpy(in.data() + sizeof head / 4, ids_h, (size_t)ns * 4);
+        return asca_stage_in(ctx, to, in.data(), in.size() * 4);
+    };
     // A step is some eighty launches, each with its tensor maps: half a millisecond of host time, which is what a small batch's
-    // step takes. A (state, streams) pair that comes a third time is replayed as a graph, one launch a step.
+    // step takes. A number of streams that comes a third time is replayed as a graph, one launch a step.
     asca_decode_plan* p = nullptr;
     PlanUse use;
-    if (f.packed && f.one_prologue && !ctx->profiling) {
+    const int64_t cap = std::max<int64_t>(1, ((int64_t)1 << 18) / ns);   // a plan's token buffer: the steps that 1 MiB holds
+    if (f.packed && f.one_prologue && !ctx->profiling && (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
         for (auto& q : m->dec_plans)
-            if (q.ctx == ctx && q.ns == ns && q.state == state && q.cap >= n_steps && q.w16 == W && q.dec_w == m->dec_w && q.dec_pk == m->dec_pk) p = &q;
+            if (q.ctx == ctx && q.ns == ns && q.w16 == W && q.dec_w == m->dec_w && q.dec_pk == m->dec_pk) p = &q;
         if (!p) {
             asca_decode_plan q;
-            q.ns = ns; q.state = state; q.w16 = W; q.dec_w = m->dec_w; q.dec_pk = m->dec_pk;
-            q.cap = 1;
-            while (q.cap < n_steps) q.cap *= 2;
+            q.ns = ns; q.w16 = W; q.dec_w = m->dec_w; q.dec_pk = m->dec_pk;
             p = new_plan(ctx, m, m->dec_plans, q);
         }
         p->stamp = ++m->plan_clock;
@@ -684,40 +707,44 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
         if (!p->exec && !p->broken && p->runs >= 2) {
             DecodeBufs pb;
             Bufs own(ctx);
-            int rc = pb.take(own, m, f, ns, p->cap) ? ASCA_OK : ASCA_ERR_OOM;
+            int rc = pb.take(own, m, f, ns, cap) ? ASCA_OK : ASCA_ERR_OOM;
             if (rc == ASCA_OK)
-                rc = capture(ctx, &p->exec, &p->launches, &p->held, [&] { return decode_step_bf16_device(ctx, m, f, pb, state, ns, false, nullptr); });
+                rc = capture(ctx, &p->exec, &p->launches, &p->held, [&] { return decode_step_bf16_device(ctx, m, f, pb, nullptr, ns, false, nullptr); });
             if (rc == ASCA_OK) {
                 p->held.insert(p->held.end(), own.p.begin(), own.p.end());   // the graph's buffers stay with it
                 own.p.clear();
-                p->cur = pb.cur; p->toks = pb.toks; p->counter = pb.counter; p->logits = pb.logits;
+                p->in = pb.in; p->cur = pb.cur; p->toks = pb.toks; p->counter = pb.counter; p->logits = pb.logits;
             } else {
                 p->broken = true;
             }
         }
         p->runs++;
     }
-    uint32_t *cur, *toks;
+    uint32_t* cur;
     float* logits;
     if (p && p->exec) {
-        cur = p->cur; toks = p->toks; logits = p->logits;
-        ASCA_TRY(asca_stage_in(ctx, cur, ids_h, (size_t)ns * 4));
-        ASCA_CUDA(ctx, cudaMemsetAsync(p->counter, 0xff, 4, ctx->stream));
-        for (int64_t step = 0; step < n_steps; ++step) ASCA_CUDA(ctx, cudaGraphLaunch(p->exec, ctx->stream));
+        cur = p->cur; logits = p->logits;
+        ASCA_TRY(upload(p->in));
+        for (int64_t done = 0; done < n_steps;) {
+            const int64_t k = std::min(cap, n_steps - done);
+            if (done > 0) ASCA_CUDA(ctx, cudaMemsetAsync(p->counter, 0xff, 4, ctx->stream));
+            for (int64_t step = 0; step < k; ++step) ASCA_CUDA(ctx, cudaGraphLaunch(p->exec, ctx->stream));
+            if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h + done * ns, p->toks, (size_t)ns * k * 4));
+            done += k;
+        }
         ctx->launches += p->launches * n_steps;
         ctx->graph_launches += n_steps;
     } else {
         DecodeBufs b;
         ASCA_REQUIRE(ctx, b.take(bf, m, f, ns, n_steps), "model_decode_step: out of memory");
-        cur = b.cur; toks = b.toks; logits = b.logits;
-        ASCA_TRY(asca_stage_in(ctx, cur, ids_h, (size_t)ns * 4));
-        ASCA_CUDA(ctx, cudaMemsetAsync(b.counter, 0xff, 4, ctx->stream));
+        cur = b.cur; logits = b.logits;
+        ASCA_TRY(upload(b.in));
         for (int64_t step = 0; step < n_steps; ++step)
-            ASCA_TRY(decode_step_bf16_device(ctx, m, f, b, state, ns, step > 0, toks + step * ns));
+            ASCA_TRY(decode_step_bf16_device(ctx, m, f, b, state, ns, step > 0, b.toks + step * ns));
+        if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h, b.toks, (size_t)ns * n_steps * 4));
     }
     if (logits_h) ASCA_TRY(asca_copy_out(ctx, logits_h, logits, (size_t)ns * V * 4));
     if (next_h) ASCA_TRY(asca_copy_out(ctx, next_h, cur, (size_t)ns * 4));
-    if (tokens_h) ASCA_TRY(asca_copy_out(ctx, tokens_h, toks, (size_t)ns * n_steps * 4));
     return asca_ctx_sync(ctx);
 }
 

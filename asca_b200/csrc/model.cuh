@@ -39,12 +39,12 @@ struct asca_step_plan : asca_plan {
     uint64_t ws_epoch = 0;      // of the scratch that its last direct run, or its graph, worked with
 };
 
-// The same for a bf16 decode step on the packed weights: one graph is one step, its tokens in and out through `cur`.
+// The same for a bf16 decode step on the packed weights: one graph is one step of `ns` streams, its tokens in and out through
+// `cur`. Where the states are is part of the input (`in`), so any state buffer of that many streams is served.
 struct asca_decode_plan : asca_plan {
-    int64_t ns = 0, cap = 0;    // streams; tokens of how many steps `toks` holds
-    const void* state = nullptr;
+    int64_t ns = 0;
     const void *w16 = nullptr, *dec_w = nullptr, *dec_pk = nullptr;   // the weight copies the graph reads
-    uint32_t *cur = nullptr, *toks = nullptr;
+    uint32_t *in = nullptr, *cur = nullptr, *toks = nullptr;
     int32_t* counter = nullptr;
     float* logits = nullptr;
 };

@@ -335,6 +335,40 @@ def test_bf16_decode_graph_equals_direct_launches(orc, gpu):
     m.free()
 
 
+# The decode graph belongs to a number of streams, not to a state buffer: requests that come with states of their own are replayed
+# from the third on, eleven states in turn go on being replayed, and a call longer than the token buffer (1024 steps of 256
+# streams) is replayed in parts.
+def test_bf16_decode_graph_serves_any_state(orc, gpu):
+    import asca_b200
+
+    m = asca_b200.Model(gpu, 256, 128, 2, 1, 4, 256)
+    m.set_params(orc.Rng(9).normal(m.n, 0.05))
+    m.set_compute(asca_b200.BF16)
+    states = [m.new_decode_state(5) for _ in range(11)]
+    for rest in range(3):
+        for i, st in enumerate(states):
+            n = gpu.graph_launch_count()
+            got = m.decode_step(st, orc.Rng(i + 20 * rest).below(256, 5))
+            assert gpu.graph_launch_count() - n == (0 if rest == 0 and i < 2 else 1)
+            if i == 7:
+                first = (got[0], st.clone())
+    gpu.profile(True)
+    other = m.new_decode_state(5)
+    for rest in range(3):
+        want = m.decode_step(other, orc.Rng(7 + 20 * rest).below(256, 5))
+    gpu.profile(False)
+    assert np.array_equal(first[0], want[0]) and bool((first[1] == other).all())
+
+    ids, toks = orc.Rng(1).below(256, 256), []
+    for replayed in (False, False, True):
+        n = gpu.graph_launch_count()
+        st = m.new_decode_state(256)
+        toks.append((m.decode_greedy(st, ids, 1030), st))
+        assert gpu.graph_launch_count() - n == (1030 if replayed else 0)
+    assert np.array_equal(toks[0][0], toks[2][0]) and bool((toks[0][1] == toks[2][1]).all())
+    m.free()
+
+
 # The tensor-core products around their tile shapes: pairs from half the chip on (37 tiles), one 128 x 128 tile an SM, two CTAs
 # an SM; ragged last rows and columns, rows off the 32-byte grid, k below and between k-tiles, bias and accumulation.
 @pytest.mark.parametrize("m,k,n", [(1536, 64, 1600), (1537, 72, 1604), (2560, 1032, 2050), (1100, 200, 1030), (130, 520, 40), (2100, 136, 2100)])
