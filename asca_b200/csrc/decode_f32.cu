@@ -12,7 +12,7 @@
 //   * a product's weights are requested before the barrier in front of it: they do not depend on it.
 //   * the RMSNorm factor multiplies the finished sums (a row's norm is needed only there).
 // Weights come through L1: a 331k model's share of a CTA stays there over the steps.
-// Before: 21 launches and a host round trip per token and two-block model, 120 us a token.
+// Launch by launch a token of the 331k model takes 106 us, here 17.6 (one stream).
 #include "model.cuh"
 
 #include <algorithm>
@@ -328,6 +328,29 @@ __global__ void __launch_bounds__(DT, 1) decode_f32_kernel(const __grid_constant
         }
 }
 
+// Whether a call of n_steps steps is better off in this launch (`cs` CTAs a stream, so many streams at a time) than step by step
+// through the single kernels. Each stream of a launch reads all its weights by itself: once every SM has one, the launch takes
+// wave after wave, while a batched step shares the weights' way through L2 and is bound by its kernels' latencies. In microseconds:
+//   a wave, per step   5 a block (its exchanges) + the stream's weight bytes at 37.8 kB/us an SM;  once  its states at 1 kB/us
+//   a batched step     45 a block + 0.065 (a model of up to 32 MB, measured at 1 - 11) or 0.165 (measured at 51) for each dependent load of
+//                      the expert kernel's two matrix-vector products, which is most of it
+// Measured, us a step in one launch / batched, 32 steps a call: d 64, 2 blocks (331k) 512 streams 88 / 126, 740: 112 / 134, 1024:
+// 155 / 146, 2048: 307 / 197; d 192, 6 blocks (12.7m) 296: 566 / 1315, 592: 1129 / 1459, 740: 1412 / 1513, 1024: 1952 / 1600; d 256, 4 heads,
+// 2 blocks, expert width 512: 148: 127 / 226, 149: 233 / 227, 297: 349 / 235, 1024: 872 / 494. One step a call: 12.7m 296: 1233 / 1321,
+// 384: 1702 / 1359; 331k 592: 135 / 148, 740: 161 / 160, 1024: 212 / 174. Of 102 points the rule takes the slower side at three: by 4 % at a
+// d 96 model, by 25 and 32 % for one step a call of 384 and 444 streams of the 12.7m model, whose states then cost more than the
+// estimate. Up to one wave the launch was ahead by 1.8 and more everywhere.
+bool one_launch_pays(const asca_model* m, int64_t ns, int64_t n_steps, int cs, int n_sm) {
+    const int64_t at_once = std::max<int64_t>(1, n_sm / cs), waves = ceil_div64(ns, at_once);
+    if (waves <= 1) return true;
+    const double d = (double)m->d, dh = d / (double)m->H, F = (double)m->F, L = (double)m->L, n = (double)n_steps;
+    const double weights = 4.0 * (L * (4.0 * d * d + 2.0 * d * (double)m->H + 2.0 * d * F) + d * (double)m->vocab) / cs;
+    const double states = 4.0 * L * (double)m->H * dh * dh / cs;
+    const double loads = (double)ceil_div64(m->F, 256) * d + (double)ceil_div64(m->d, 256) * F;
+    const double batched = L * (45.0 + (m->n_params * 4 <= ((int64_t)32 << 20) ? 0.065 : 0.165) * loads);
+    return (double)waves * (n * (5.0 * L + weights / 37.8e3) + states / 1e3) <= n * batched;
+}
+
 size_t smem_bytes(const asca_model* m, int cs, int fl, int vl) {
     const int64_t d = m->d, dh = d / m->H, nh = (m->H + cs - 1) / cs;
     return (size_t)(d + 2 * cs * d + 4 * DT + nh * 3 * dh + 2 * nh + nh * dh + 2 + std::max(fl, vl) + 2 * cs + m->L * nh * dh * dh) * 4;
@@ -336,8 +359,8 @@ size_t smem_bytes(const asca_model* m, int cs, int fl, int vl) {
 }  // namespace
 
 // n_steps greedy steps of ns streams from ids (device); tokens (device, n_steps x ns), logits (device, nullable) of the last
-// step. ASCA_ERR_UNSUPPORTED, nothing launched: a stream's states do not fit its cluster's shared memory, or the shapes rule
-// out 16-byte weight loads (the caller steps through the single kernels then).
+// step. ASCA_ERR_UNSUPPORTED, nothing launched: a stream's states do not fit its cluster's shared memory, the shapes rule
+// out 16-byte weight loads, or there are more streams than this form is good for (the caller steps through the single kernels then).
 int asca_decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* ids, int64_t ns, int64_t n_steps, uint32_t* tokens,
                     float* logits) {
     const int64_t d = m->d, H = m->H, dh = d / H, F = m->F, V = m->vocab;
@@ -359,6 +382,7 @@ int asca_decode_f32(asca_ctx* ctx, asca_model* m, float* state, const uint32_t* 
         if (smem <= ctx->smem_optin && ceil_div64(H, cs) * 3 * dh <= 4 * DT && std::max(g.fl, g.vl) <= 4 * DT) break;
         if (cs == 8) return ASCA_ERR_UNSUPPORTED;
     }
+    if (!one_launch_pays(m, ns, n_steps, cs, n_sm)) return ASCA_ERR_UNSUPPORTED;
     g.P = m->params; g.embed = m->embed; g.head = m->head; g.layer_stride = stride; g.l0 = a;
     g.d = (int)d; g.H = (int)H; g.L = (int)m->L; g.E = (int)m->E; g.F = (int)F; g.V = (int)V; g.ns = (int)ns;
     g.n_steps = n_steps; g.state = state; g.ids = ids; g.tokens = tokens; g.logits = logits;

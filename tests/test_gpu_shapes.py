@@ -78,6 +78,37 @@ def test_f32_decode_cluster_widths_and_fallbacks(orc, gpu, cfg, ns):
     dev.free()
 
 
+# f32 decode past one wave of streams: where a launch of its own for every stream costs more than the batched step, the call takes
+# the batched step (two steps a call: from the fifth wave of 148 streams on at d 64, from the second at d 256); the same tokens, logits
+# and states on both sides of the line.
+@pytest.mark.parametrize("cfg,ns,steps,one", [((256, 64, 4, 2, 4, 256), 148, 2, True), ((256, 64, 4, 2, 4, 256), 592, 2, True),
+                                              ((256, 64, 4, 2, 4, 256), 593, 2, False), ((256, 256, 4, 2, 4, 512), 148, 2, True),
+                                              ((256, 256, 4, 2, 4, 512), 149, 2, False)])
+def test_f32_decode_more_streams_than_fit_at_once(orc, gpu, cfg, ns, steps, one):
+    import asca_b200
+
+    V = cfg[0]
+    ref = orc.Model(*cfg)
+    ref.params[:] = orc.Rng(sum(cfg)).normal(ref.n, 0.8 * cfg[1] ** -0.5)
+    dev = asca_b200.Model(gpu, *cfg)
+    dev.set_params(ref.params)
+    ids = orc.Rng(ns).below(V, ns)
+    state = dev.new_decode_state(ns)
+    before = gpu.launch_count()
+    toks = dev.decode_greedy(state, ids.copy(), steps)
+    assert (gpu.launch_count() - before == 1) == one
+    logits, nxt = dev.decode_step(state, toks[-1].copy())
+    for s in sorted({0, ns // 2, ns - 1}):
+        st, tok = ref.new_decode_state(), ids[s]
+        for t in range(steps):
+            tok = int(ref.step(tok, st).argmax())
+            assert tok == toks[t, s]
+        lg = ref.step(tok, st)
+        assert rel_err(logits[s:s + 1], lg) < F32_TOL and nxt[s] == lg.argmax()
+        assert rel_err(state[:, s].cpu().numpy(), st) < F32_TOL
+    dev.free()
+
+
 # The f32 recurrence with one, two and four value columns per lane group (few chains to many), ragged stages, decay strong enough
 # to be folded in step by step, and the three-kernel backward with every width of its chain kernel.
 @pytest.mark.parametrize("B,T,H,dh", [(1, 1, 1, 16), (2, 33, 2, 16), (40, 70, 20, 16), (1, 65, 1, 32), (60, 40, 20, 32), (130, 16, 20, 32),
