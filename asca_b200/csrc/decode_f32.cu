@@ -317,9 +317,8 @@ __global__ void __launch_bounds__(DT, 1) decode_f32_kernel(const __grid_constant
                 bi = i;
             }
         }
-        id = (uint32_t)bi;
+        id = bi == 0x7fffffff ? 0u : (uint32_t)bi;   // (a row of NaNs or of -inf: token 0)
         if (rank == 0 && tid == 0) g.tokens[step * g.ns + s] = id;
-        if (id >= (uint32_t)g.V) id = 0;   // (a row of NaNs has no argmax: keep the next step inside the table)
     }
     for (int li = 0; li < g.L; ++li)
         for (int i = tid; i < nh * DH * DH; i += DT) {

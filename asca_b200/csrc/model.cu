@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256) concat_bias_kernel(const float* __restric
     const int c = blockIdx.x * 256 + threadIdx.x;
     if (c < ld) dst[c] = c < ca ? a[c] : (c < ca + cb ? b[c - ca] : 0.0f);
 }
-// greedy argmax per row, lowest index on ties; toks (nullable): also written to row *counter (0 without one) of toks
+// greedy argmax per row, lowest index on ties (index 0 where nothing compares, so that the choice is a token); toks (nullable): also written to row *counter (0 without one) of toks
 __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ logits, int64_t N, int V,
                                                      uint32_t* __restrict__ out, uint32_t* __restrict__ toks = nullptr,
                                                      const int32_t* __restrict__ counter = nullptr) {
@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ l
         }
     }
     if (lane == 0) {
+        if (bi == 0x7fffffff) bi = 0;   // a row of NaNs or of -inf
         out[t] = (uint32_t)bi;
         if (toks) toks[(counter ? *counter : 0) * N + t] = (uint32_t)bi;
     }

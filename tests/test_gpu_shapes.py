@@ -109,6 +109,29 @@ def test_f32_decode_more_streams_than_fit_at_once(orc, gpu, cfg, ns, steps, one)
     dev.free()
 
 
+# Logits that do not compare (a head of NaNs, or all of them -inf): the choice is token 0, in every form of the step, and the next step
+# reads that row of the embedding and no other.
+@pytest.mark.parametrize("cfg,ns,mode", [((256, 64, 4, 1, 4, 64), 3, "F32"), ((256, 80, 5, 1, 4, 64), 3, "F32"), ((256, 128, 2, 1, 4, 64), 5, "BF16"),
+                                         ((256, 128, 2, 1, 4, 64), 300, "BF16"), ((256, 128, 1, 1, 4, 64), 5, "BF16")])
+@pytest.mark.parametrize("bad", [float("nan"), float("-inf")])
+def test_greedy_choice_without_a_largest_logit(orc, gpu, cfg, ns, mode, bad):
+    import asca_b200
+
+    m = asca_b200.Model(gpu, *cfg)
+    params = np.abs(orc.Rng(5).normal(m.n, 0.1)) + 0.01   # positive throughout: -inf weights give -inf logits
+    V, d = cfg[:2]
+    params[V * d:2 * V * d] = bad
+    m.set_params(params)
+    m.set_compute(getattr(asca_b200, mode))
+    ids = orc.Rng(6).below(V, ns)
+    for _ in range(3):
+        st = m.new_decode_state(ns)
+        assert not m.decode_greedy(st, ids.copy(), 3).any()
+        assert not m.decode_step(st, ids.copy())[1].any() and bool(st.isfinite().all())
+    assert not m.prefill(m.new_decode_state(ns), np.tile(ids[:, None], (1, 5)))[1].any()
+    m.free()
+
+
 # The f32 recurrence with one, two and four value columns per lane group (few chains to many), ragged stages, decay strong enough
 # to be folded in step by step, and the three-kernel backward with every width of its chain kernel.
 @pytest.mark.parametrize("B,T,H,dh", [(1, 1, 1, 16), (2, 33, 2, 16), (40, 70, 20, 16), (1, 65, 1, 32), (60, 40, 20, 32), (130, 16, 20, 32),
