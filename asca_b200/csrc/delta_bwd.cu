@@ -28,6 +28,8 @@
 // floats so float4 reads along a row are aligned and rows fall in different banks.
 #include "common.cuh"
 
+#include <algorithm>
+
 bool asca_tc_enabled();  // gemm.cu
 namespace delta_tc {
 bool available();
@@ -584,6 +586,8 @@ __global__ void __launch_bounds__(BT, 1) delta_bwd_kernel(
 // states; a launch of few chains (the small models, host calls) fills the GPU with its chunks. Work per token and head is about
 // 13 dh^2 multiply-adds against 21. Every dL and dA appears times beta or L, so nothing is divided by beta:
 //   beta dL = -strictlower(dZ U^T),  beta dbeta_t = dZ_t.Z_t - sum_i (dZ U^T)[t,i] LG[t,i]
+// A launch takes a group of chains and a segment of their chunks (`Range`), last segment first, so that the scratch between the
+// kernels stays bounded; the chain kernel hands dS from segment to segment through `carry`.
 // Bound: shared-memory return bandwidth of the 8 x 4 thread tiles (0.375 loads per FFMA), one CTA per SM at dh 128.
 constexpr int CC = 64;   // tokens per chunk
 constexpr int LX = CC + 4;
@@ -764,6 +768,12 @@ struct ChunkScratch {
     static constexpr int64_t A = 0, LG = CC * CC, T = 2 * CC * CC, D = 3 * CC * CC, HM = D + CC * DH, Y = HM + CC * DH, GAM = Y + DH * DH, SIZE = GAM + CC;
 };
 
+// The chains [chain0, chain0 + gridDim.y) and chunks [ck0, ck0 + n) of a launch; scratch tiles are numbered inside it.
+struct Range {
+    int chain0, ck0, n;
+    __device__ __forceinline__ int64_t tile(int chain, int ck) const { return (int64_t)(chain - chain0) * n + (ck - ck0); }
+};
+
 template <int DH, typename T>
 struct PreSmem {
     static constexpr int LD = DH + 4;
@@ -773,16 +783,16 @@ struct PreSmem {
 template <int DH, typename T>
 __global__ void __launch_bounds__(BT) delta_bwd_pre_kernel(const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ alpha,
                                                            const float* __restrict__ beta, const T* __restrict__ d_o,
-                                                           float* __restrict__ scratch, int Tlen, int H, int n_ck) {
+                                                           float* __restrict__ scratch, int Tlen, int H, const Range range) {
     using SC = ChunkScratch<DH>;
     constexpr int LD = DH + 4;
     extern __shared__ __align__(16) float smem[];
     float *Ks = smem, *Qs = Ks + CC * LD, *Os = Qs + CC * LD, *Xs = Os + CC * LD, *Ls = Xs + CC * LD, *Ts = Ls + CC * LX, *As = Ts + CC * LX;
     ChunkGates& gt = *reinterpret_cast<ChunkGates*>(As + CC * LX);
-    const int tid = threadIdx.x, ck = blockIdx.x, chain = blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
+    const int tid = threadIdx.x, ck = range.ck0 + blockIdx.x, chain = range.chain0 + blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
     const int n = min(CC, Tlen - ck * CC);
     const int64_t row0 = (int64_t)bi * Tlen + ck * CC;
-    float* out = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+    float* out = scratch + range.tile(chain, ck) * SC::SIZE;
     load_tile<T, CC, DH>(k, row0, d, h * DH, n, Ks, LD);
     load_tile<T, CC, DH>(q, row0, d, h * DH, n, Qs, LD);
     load_tile<T, CC, DH>(d_o, row0, d, h * DH, n, Os, LD);
@@ -883,19 +893,22 @@ struct ChainSmem {
 };
 
 template <int DH, int W, typename T>
-__global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict__ k, float* __restrict__ scratch, int Tlen, int H, int n_ck) {
+__global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict__ k, float* __restrict__ scratch, float* __restrict__ carry,
+                                                             int Tlen, int H, const Range range, int last) {
     using SC = ChunkScratch<DH>;
     using SM = ChainSmem<DH, W>;
     constexpr int LD = SM::LD, LW = SM::LW;
     constexpr bool AHEAD = SM::AHEAD;
     extern __shared__ __align__(16) float smem[];
     float *dS = smem + (AHEAD ? 2 : 1) * SM::STAGE, *dZ = dS + DH * LW;
-    const int tid = threadIdx.x, c0 = blockIdx.x * W, chain = blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
-    for (int i = tid; i < DH * LW; i += BT) dS[i] = 0.0f;
+    const int tid = threadIdx.x, c0 = blockIdx.x * W, chain = range.chain0 + blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
+    const int ck_end = range.ck0 + range.n;
+    carry += (int64_t)blockIdx.y * DH * DH + c0;   // dS between segments: `last` starts from zero, the first leaves none behind
+    for (int i = tid; i < DH * W; i += BT) dS[i / W * LW + i % W] = last ? 0.0f : carry[i / W * DH + i % W];
     MM<DH, W> s_in;   // Y and D of the chunk to come
     MM<CC, W> z_in;
     auto request = [&](int ck, float* st) {
-        float* at = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+        float* at = scratch + range.tile(chain, ck) * SC::SIZE;
         load_tile<float, CC, DH>(at + SC::HM, 0, DH, 0, CC, st, LD);
         load_tile<T, CC, DH>(k, (int64_t)bi * Tlen + ck * CC, d, h * DH, min(CC, Tlen - ck * CC), st + CC * LD, LD);
         if (tid < CC / 4)
@@ -904,13 +917,13 @@ __global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict
         s_in.each([&](int a, int c, float& v) { v = at[SC::Y + a * DH + c0 + c]; });
         z_in.each([&](int t, int c, float& v) { v = at[SC::D + t * DH + c0 + c]; });
     };
-    if (AHEAD) request(n_ck - 1, smem + ((n_ck - 1) & 1) * SM::STAGE);
-    for (int ck = n_ck - 1; ck >= 0; --ck) {
-        float* at = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+    if (AHEAD) request(ck_end - 1, smem + ((ck_end - 1) & 1) * SM::STAGE);
+    for (int ck = ck_end - 1; ck >= range.ck0; --ck) {
+        float* at = scratch + range.tile(chain, ck) * SC::SIZE;
         float* Hs = smem + (AHEAD ? (ck & 1) * SM::STAGE : 0);
         const float *Ks = Hs + CC * LD, *gam = Hs + 2 * CC * LD;
         if (!AHEAD) request(ck, Hs);
-        if (!AHEAD && ck > 0) {
+        if (!AHEAD && ck > range.ck0) {
             prefetch_l2(at - SC::SIZE + SC::HM, 1, CC * DH * 4, 0);
             prefetch_l2(at - SC::SIZE + SC::D + c0, CC, W * 4, DH * 4);
             prefetch_l2(at - SC::SIZE + SC::Y + c0, DH, W * 4, DH * 4);
@@ -919,7 +932,7 @@ __global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict
         tile_wait();
         MM<DH, W> s = s_in;
         MM<CC, W> z = z_in;
-        if (AHEAD && ck > 0) request(ck - 1, smem + ((ck - 1) & 1) * SM::STAGE);
+        if (AHEAD && ck > range.ck0) request(ck - 1, smem + ((ck - 1) & 1) * SM::STAGE);
         s.each([&](int a, int c, float) { at[SC::Y + a * DH + c0 + c] = dS[a * LW + c]; });   // dS at the end of this chunk
         z.template mul<DH, L_MK, L_KN>(Hs, LD, dS, LW);
         z.each([&](int t, int c, float v) {
@@ -932,6 +945,10 @@ __global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict
         s.each([&](int a, int c, float& v) { v = fmaf(gl, dS[a * LW + c], v); });
         s.template mul<CC, L_KM, L_KN>(Ks, LD, dZ, LW);
         __syncthreads();
+        if (ck == range.ck0) {
+            s.each([&](int a, int c, float v) { carry[a * DH + c] = v; });
+            break;
+        }
         s.each([&](int a, int c, float v) { dS[a * LW + c] = v; });
         if (!AHEAD) __syncthreads();   // (with two buffers the next tile_wait is the barrier)
     }
@@ -947,8 +964,8 @@ template <int DH, typename T>
 __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ alpha,
     const float* __restrict__ beta, const float* __restrict__ qnorm, const float* __restrict__ knorm, const T* __restrict__ d_o,
-    const float* __restrict__ ckpt, const float* __restrict__ scratch, int Tlen, int H, int n_ck, float* __restrict__ d_qkv,
-    float* __restrict__ d_gate) {
+    const float* __restrict__ ckpt, const float* __restrict__ scratch, int Tlen, int H, int n_ck, const Range range,
+    float* __restrict__ d_qkv, float* __restrict__ d_gate) {
     using SC = ChunkScratch<DH>;
     constexpr int LD = DH + 4;
     extern __shared__ __align__(16) float smem[];
@@ -956,10 +973,11 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
           *Xs = Ss + DH * LD /* T, then dA Gam, then M + M^T */, *col_part = Xs + CC * LX, *vec = col_part + 8 * CC, *red = vec + 8 * CC;
     float *row_p = vec, *col_p = vec + CC, *r_qs = vec + 2 * CC, *r_kg = vec + 3 * CC, *r_kw = vec + 4 * CC, *dbe = vec + 5 * CC;
     ChunkGates& gt = *reinterpret_cast<ChunkGates*>(red + 64);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ck = blockIdx.x, chain = blockIdx.y, bi = chain / H, h = chain % H, d = H * DH;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ck = range.ck0 + blockIdx.x, chain = range.chain0 + blockIdx.y, bi = chain / H,
+              h = chain % H, d = H * DH;
     const int n = min(CC, Tlen - ck * CC);
     const int64_t row0 = (int64_t)bi * Tlen + ck * CC;
-    const float* in = scratch + ((int64_t)chain * n_ck + ck) * SC::SIZE;
+    const float* in = scratch + range.tile(chain, ck) * SC::SIZE;
     const float* S0 = ckpt + ((int64_t)chain * n_ck + ck) * DH * DH;
     load_tile<T, CC, DH>(k, row0, d, h * DH, n, Ks, LD);
     load_tile<float, DH, DH>(S0, 0, DH, 0, DH, Ss, LD);
@@ -1172,49 +1190,6 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
     }
 }
 
-template <int DH, int W, typename T>
-int launch_chain(asca_ctx* ctx, const void* k, float* ws, int B, int Tlen, int H, int n_ck) {
-    auto kern = delta_bwd_chain_kernel<DH, W, T>;
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChainSmem<DH, W>::bytes));
-    kern<<<dim3(DH / W, B * H), BT, ChainSmem<DH, W>::bytes, ctx->stream>>>((const T*)k, ws, Tlen, H, n_ck);
-    ASCA_CHECK_LAUNCH(ctx);
-    return ASCA_OK;
-}
-
-template <int DH, typename T>
-int launch_bwd64(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta, const float* qnorm,
-                 const float* knorm, const void* d_o, const float* ckpt, int B, int Tlen, int H, float* d_qkv, float* d_gate) {
-    const int n_ck = (Tlen + CC - 1) / CC;
-    void* p;
-    ASCA_TRY(asca_workspace(ctx, (size_t)B * H * n_ck * ChunkScratch<DH>::SIZE * 4 + 256, &p));
-    float* ws = (float*)p;
-    static_assert(PreSmem<DH, T>::bytes <= 227 * 1024 && GradSmem<DH>::bytes <= 227 * 1024, "shared memory budget");
-    auto pre = delta_bwd_pre_kernel<DH, T>;
-    auto grad = delta_bwd_grad_kernel<DH, T>;
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PreSmem<DH, T>::bytes));
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradSmem<DH>::bytes));
-    {
-        asca_span sp(ctx, "delta_bwd_pre_kernel");
-        pre<<<dim3(n_ck, B * H), BT, PreSmem<DH, T>::bytes, ctx->stream>>>((const T*)q, (const T*)k, alpha, beta, (const T*)d_o, ws, Tlen, H, n_ck);
-        ASCA_CHECK_LAUNCH(ctx);
-    }
-    {   // value columns per CTA: as many as leave every SM a CTA, since wider tiles read less shared memory per FFMA
-        asca_span sp(ctx, "delta_bwd_chain_kernel");
-        const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
-        int w = DH;
-        while (w > 16 && B * H * (DH / w) * 2 <= n_sm) w /= 2;
-        if (w == 128) ASCA_TRY((launch_chain<DH, DH < 128 ? DH : 128, T>(ctx, k, ws, B, Tlen, H, n_ck)));
-        else if (w == 64) ASCA_TRY((launch_chain<DH, DH < 64 ? DH : 64, T>(ctx, k, ws, B, Tlen, H, n_ck)));
-        else if (w == 32) ASCA_TRY((launch_chain<DH, DH < 32 ? DH : 32, T>(ctx, k, ws, B, Tlen, H, n_ck)));
-        else ASCA_TRY((launch_chain<DH, 16, T>(ctx, k, ws, B, Tlen, H, n_ck)));
-    }
-    asca_span sp(ctx, "delta_bwd_grad_kernel");
-    grad<<<dim3(n_ck, B * H), BT, GradSmem<DH>::bytes, ctx->stream>>>((const T*)q, (const T*)k, (const T*)v, alpha, beta, qnorm, knorm, (const T*)d_o,
-                                                                      ckpt, ws, Tlen, H, n_ck, d_qkv, d_gate);
-    ASCA_CHECK_LAUNCH(ctx);
-    return ASCA_OK;
-}
-
 template <int DH, int C, typename T>
 int launch_bwd(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
                const float* qnorm, const float* knorm, const void* d_o, const float* ckpt, int B, int Tlen, int H,
@@ -1230,6 +1205,78 @@ int launch_bwd(asca_ctx* ctx, const void* q, const void* k, const void* v, const
     kern<<<B * H, BT, SM::bytes, ctx->stream>>>((const T*)q, (const T*)k, (const T*)v, alpha, beta, qnorm, knorm,
                                                 (const T*)d_o, ckpt, (float*)ws, B, Tlen, H, chunk, d_qkv, d_gate);
     ASCA_CHECK_LAUNCH(ctx);
+    return ASCA_OK;
+}
+
+template <int DH, int W, typename T>
+int launch_chain(asca_ctx* ctx, const void* k, float* ws, float* carry, int chains, int Tlen, int H, const Range& range, bool last) {
+    auto kern = delta_bwd_chain_kernel<DH, W, T>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChainSmem<DH, W>::bytes));
+    kern<<<dim3(DH / W, chains), BT, ChainSmem<DH, W>::bytes, ctx->stream>>>((const T*)k, ws, carry, Tlen, H, range, last ? 1 : 0);
+    ASCA_CHECK_LAUNCH(ctx);
+    return ASCA_OK;
+}
+
+// Scratch of a launch of the three kernels at most. 8,192 tiles at dh 128 (8 x 4096 tokens of 16 heads) are 1.48 GB and stay one launch;
+// a launch this size is 60 waves of the chunk kernels, whose ends then cost nothing that shows. Where the device has no room
+// for it, a fourth, and a sixteenth, and then the single kernel, which needs a few states per chain.
+constexpr int64_t BWD64_SCRATCH = (int64_t)3 << 29;
+constexpr int MIN_SEGMENT = 16;   // chunks a launch takes of a chain before it takes fewer chains (the chain kernel's start-up)
+
+template <int DH, typename T>
+int launch_bwd64(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta, const float* qnorm,
+                 const float* knorm, const void* d_o, const float* ckpt, int B, int Tlen, int H, float* d_qkv, float* d_gate) {
+    const int n_ck = (Tlen + CC - 1) / CC, n_chains = B * H;
+    static_assert(PreSmem<DH, T>::bytes <= 227 * 1024 && GradSmem<DH>::bytes <= 227 * 1024, "shared memory budget");
+    int chains = n_chains, seg = n_ck;   // of a launch
+    void* p = nullptr;
+    for (int64_t room = BWD64_SCRATCH;; room /= 4) {
+        if (room < BWD64_SCRATCH / 16)
+            return launch_bwd<DH, DH == 128 ? 16 : 32, T>(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, B, Tlen, H, CC, d_qkv, d_gate);
+        const int64_t tiles = room / (ChunkScratch<DH>::SIZE * 4);
+        if ((int64_t)n_chains * n_ck > tiles) {   // even groups of chains, even segments
+            const int64_t groups = ceil_div64(n_chains, std::max<int64_t>(1, tiles / std::min(MIN_SEGMENT, n_ck)));
+            chains = (int)ceil_div64(n_chains, groups);
+            const int64_t segs = ceil_div64(n_ck, std::max<int64_t>(1, tiles / chains));
+            seg = (int)ceil_div64(n_ck, segs);
+        }
+        const int rc = asca_workspace(ctx, ((size_t)chains * seg * ChunkScratch<DH>::SIZE + (seg < n_ck ? (size_t)chains * DH * DH : 0)) * 4 + 256, &p);
+        if (rc == ASCA_OK) break;
+        if (rc != ASCA_ERR_OOM) return rc;
+    }
+    float *ws = (float*)p, *carry = ws + (int64_t)chains * seg * ChunkScratch<DH>::SIZE;
+    auto pre = delta_bwd_pre_kernel<DH, T>;
+    auto grad = delta_bwd_grad_kernel<DH, T>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PreSmem<DH, T>::bytes));
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradSmem<DH>::bytes));
+    const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    for (int chain0 = 0; chain0 < n_chains; chain0 += chains) {
+        const int nc = std::min(chains, n_chains - chain0);
+        for (int end = n_ck; end > 0;) {
+            const int ck0 = std::max(0, end - seg), n = end - ck0;
+            const Range range = {chain0, ck0, n};
+            {
+                asca_span sp(ctx, "delta_bwd_pre_kernel");
+                pre<<<dim3(n, nc), BT, PreSmem<DH, T>::bytes, ctx->stream>>>((const T*)q, (const T*)k, alpha, beta, (const T*)d_o, ws, Tlen, H, range);
+                ASCA_CHECK_LAUNCH(ctx);
+            }
+            {   // value columns per CTA: as many as leave every SM a CTA, since wider tiles read less shared memory per FFMA
+                asca_span sp(ctx, "delta_bwd_chain_kernel");
+                const bool last = end == n_ck;
+                int w = DH;
+                while (w > 16 && nc * (DH / w) * 2 <= n_sm) w /= 2;
+                if (w == 128) ASCA_TRY((launch_chain<DH, DH < 128 ? DH : 128, T>(ctx, k, ws, carry, nc, Tlen, H, range, last)));
+                else if (w == 64) ASCA_TRY((launch_chain<DH, DH < 64 ? DH : 64, T>(ctx, k, ws, carry, nc, Tlen, H, range, last)));
+                else if (w == 32) ASCA_TRY((launch_chain<DH, DH < 32 ? DH : 32, T>(ctx, k, ws, carry, nc, Tlen, H, range, last)));
+                else ASCA_TRY((launch_chain<DH, 16, T>(ctx, k, ws, carry, nc, Tlen, H, range, last)));
+            }
+            asca_span sp(ctx, "delta_bwd_grad_kernel");
+            grad<<<dim3(n, nc), BT, GradSmem<DH>::bytes, ctx->stream>>>((const T*)q, (const T*)k, (const T*)v, alpha, beta, qnorm, knorm,
+                                                                        (const T*)d_o, ckpt, ws, Tlen, H, n_ck, range, d_qkv, d_gate);
+            ASCA_CHECK_LAUNCH(ctx);
+            end = ck0;
+        }
+    }
     return ASCA_OK;
 }
 

@@ -162,6 +162,50 @@ def test_f32_delta_column_splits(orc, gpu, B, T, H, dh, decay):
     assert rel_err(d_gate[rows].cpu().numpy(), dg_ref) < F32_TOL
 
 
+# The f32 backward where its chunks do not fit the scratch of one launch (27,473 tiles at dh 16, 8,923 at dh 128): segments of one
+# long chain, segments of many chains, groups of chains, both, and a device without room for any of it (the single kernel). The
+# scratch stays below 1.6 GB; the reference is the single kernel on checkpoints every 32 tokens (both are held to F32_TOL of the
+# oracle, so twice that between them).
+@pytest.mark.parametrize("B,T,H,dh,left", [(1, 27483 * 64 - 5, 1, 16, None), (60, 32 * 64 - 1, 16, 16, None), (150, 19 * 64, 16, 16, None),
+                                           (150, 33 * 64 + 7, 16, 16, None), (2, 4500 * 64 + 1, 1, 128, None), (60, 32 * 64 - 1, 16, 16, 64 << 20),
+                                           (60, 32 * 64 - 1, 16, 16, 600 << 20)])
+def test_f32_delta_backward_in_bounded_scratch(gpu, B, T, H, dh, left):
+    import ctypes as C
+    import torch
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    n, d = B * T, H * dh
+    norm = lambda *shape: torch.randn(*shape, generator=g, device="cuda")  # noqa: E731
+    q, k = norm(n, H, dh), norm(n, H, dh)
+    qn, kn = q.norm(dim=-1), k.norm(dim=-1)
+    q, k = ((x / xn[..., None]).reshape(n, d) for x, xn in ((q, qn), (k, kn)))
+    v, d_o = norm(n, d), norm(n, d)
+    alpha, beta = torch.sigmoid(4 + norm(n, H)), torch.sigmoid(norm(n, H))   # decay slow enough to cross segments
+    ckpt = ops.delta_fwd(gpu, q, k, v, alpha, beta, B, T, H, dh, chunk=32)[2]
+    want = ops.delta_bwd(gpu, q, k, v, alpha, beta, qn, kn, d_o, ckpt, B, T, H, dh, chunk=32)
+    ckpt = ops.delta_fwd(gpu, q, k, v, alpha, beta, B, T, H, dh)[2]
+    got = [torch.empty_like(x) for x in want]
+    torch.cuda.empty_cache()
+    gpu._call("asca_ctx_trim", gpu._ctx)
+    before, hog = torch.cuda.mem_get_info()[0], C.c_void_p()
+    if left:
+        gpu._call("asca_malloc", gpu._ctx, C.c_size_t(before - left), C.byref(hog))
+    gpu.profile(True)
+    ops.delta_bwd(gpu, q, k, v, alpha, beta, qn, kn, d_o, ckpt, B, T, H, dh, d_qkv=got[0], d_gate=got[1])
+    kernels = [name for name, _ in gpu.profile_read()]
+    gpu.profile(False)
+    used = before - torch.cuda.mem_get_info()[0]
+    if left:
+        gpu._call("asca_free", gpu._ctx, hog)
+        gpu._call("asca_ctx_trim", gpu._ctx)
+        assert kernels == ["delta_bwd_kernel"] if left == 64 << 20 else kernels.count("delta_bwd_chain_kernel") > 4
+    else:
+        assert used < 1600 << 20 and kernels.count("delta_bwd_chain_kernel") > 1
+    for a, b in zip(got, want):
+        assert float((a - b).abs().max() / b.abs().max()) < 2 * F32_TOL
+
+
 # The one-kernel dispatch up to its limits (16,384 tokens, 256 experts) and just past them.
 @pytest.mark.parametrize("n,e", [(1, 1), (32, 4), (33, 256), (1025, 7), (16384, 64), (16384, 256), (16385, 64), (2000, 257)])
 def test_dispatch_small_and_past_it(orc, gpu, n, e):
