@@ -12,7 +12,7 @@
 //   * a product's weights are requested before the barrier in front of it: they do not depend on it.
 //   * the RMSNorm factor multiplies the finished sums (a row's norm is needed only there).
 // Weights come through L1: a 331k model's share of a CTA stays there over the steps.
-// Launch by launch a token of the 331k model takes 106 us, here 17.6 (one stream).
+// One stream of the 331k model: 17.6 us a token (128 a call); step by step through the single kernels 106.
 #include "model.cuh"
 
 #include <algorithm>

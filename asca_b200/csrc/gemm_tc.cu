@@ -37,12 +37,12 @@ constexpr int A_BYTES = BM * BK * 2;
 // DEEP: a problem of at most one 128 x 128 tile per SM (a decode step's products) runs one CTA per SM with a
 // 7-stage ring: its k-loop streams weights that are cold in L2, and three stages do not cover the HBM latency.
 // PAIR: a cluster of two CTAs computes 256 x 256 tiles with cta_group::2 instructions (M = 256, N = 256). Each CTA
-// loads its own 128 rows of A and its own 128 of the tile's 256 B columns (32 KiB per k-tile for 4.2 MFLOP on this SM
-// against 48 KiB for the 128 x 256 tile and 32 KiB per 2.1 MFLOP for the 128 x 128 one): shared-memory traffic per
-// FLOP, which is what bounds the single-CTA shapes, halves. 7-stage ring, all 512 TMEM columns, one CTA per SM. What bounds its
-// main loop is the round trip of a stage (slot free -> load -> barrier -> instruction) against the ring's depth: the odd CTA's loads
-// complete on the even CTA's barrier (they used to be reported by a thread of the odd CTA) and the ring is as deep as shared
-// memory allows; 65,536 x 4096 x 1024 went from 433 to 400 us (1270 -> 1375 TFLOP/s).
+// loads its own 128 rows of A and its own 128 of the tile's 256 B columns: 32 KiB per k-tile for 4.2 MFLOP on this SM where the
+// 128 x 128 tile has 32 KiB per 2.1, so the shared-memory traffic per FLOP, which is what bounds the single-CTA shape, is half of
+// its. 7-stage ring, all 512 TMEM columns, one CTA per SM. What bounds its main loop is the round trip of a stage (slot free ->
+// load -> barrier -> instruction) against the ring's depth: the odd CTA's loads complete on the even CTA's barrier and the
+// ring is as deep as shared memory allows. 65,536 x 4096 x 1024: 400 us, 1375 TFLOP/s (433 us with six stages and the odd CTA's
+// loads reported by one of its threads); 32,768 x 6144 x 2048: tensor pipe 76 % busy.
 template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct Shape {
     static constexpr int STAGES = PAIR || DEEP ? 7 : 3;   // (one fewer where the tile table needs the room)
     static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
@@ -96,7 +96,7 @@ struct KP {
 constexpr int DYN_Q = 16;              // claims a walker's producer can be ahead of its slowest role, with room to spare
 
 // bf16 mode only (2e-2 tolerance; the results are rounded to bf16 or multiply bf16 products): the hardware's base-2 exponential
-// and reciprocal without the denormal handling around them, 5 and 7 instructions. An epilogue is bound by its instructions.
+// and reciprocal without the denormal handling around them. An epilogue is bound by its instructions.
 __device__ __forceinline__ float sigmoid_f(float x) {
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
@@ -506,8 +506,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         // or two warps per scheduler is the latency of its instructions, not the bytes: hence the 32-wide straight-line code and
         // the loads of `aux` / of the old C a column group or two ahead, the first before the accumulator is awaited. Measured on the
         // expert products of 65,536 tokens, 1024 -> 4096 (two outputs, SiLU; SiLU' with its f32 read), whose tiles have 6 us of main
-        // loop: 1076 -> 670 us and 1166 -> 730 us. The TMEM buffer is released after the last tcgen05.ld; the next tile's main loop runs
-        // meanwhile in the other buffer.
+        // loop: 670 and 730 us, against 1076 and 1166 with results staged through shared memory. The TMEM buffer is released after
+        // the last tcgen05.ld; the next tile's main loop runs meanwhile in the other buffer.
         const int q = warp & 3;                 // TMEM lane quarter this warp may read
         const int ew = warp - 2;                // epilogue warp index; warps ew and ew + 4 share lane quarter q
         constexpr int C_PER_WARP = (BN / 32) / (SH::EPI_WARPS / 4);   // 32-column groups of a row per warp
@@ -781,9 +781,9 @@ static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid) {
                 ASCA_CUDA(ctx, cudaMemsetAsync(ctx->dyn_buf, 0, 256, ctx->stream));
                 ctx->dyn_seq = 0;
             }
-            // One tile per claim. Several consecutive tiles per claim were measured (8 where a walker has > 128 tiles):
-            // the train step went from 335.9 to 355.4 ms -- neighbouring walkers no longer work on neighbouring tiles
-            // at the same time, which is what lets them share operand tiles in L2.
+            // One tile per claim: with several consecutive ones (8 where a walker has > 128 tiles) a train step took 355.4 ms
+            // against 335.9 -- neighbouring walkers then do not work on neighbouring tiles at the same time, which is what
+            // lets them share operand tiles in L2.
             const uint32_t seq = ++ctx->dyn_seq;
             int* ctrs = static_cast<int*>(ctx->dyn_buf);
             p.dyn_ctr = ctrs + (seq & 1) * 32;          // the two counters sit in different 128-byte lines
@@ -880,7 +880,7 @@ int launch(asca_ctx* ctx, const Args& a) {
 
 // A pair runs a 256 x 256 tile 1.6 times as fast as two SMs run its four quarters in the 128 x 128 shape (two CTAs an SM), so pairs win
 // from half of them busy on; below that, each quarter has an SM of its own in the deep 128 x 128 form. With 64 tiles (1024 x 65,536 x
-// 4096, A^T B): 906 -> 402 us. Rows grouped by expert need 512 rows an expert, or padding to 256 rows costs more than that.
+// 4096, A^T B): 402 us in pairs, 906 in quarters. Rows grouped by expert need 512 rows an expert, or padding to 256 rows costs more than that.
 static bool pair_wanted(asca_ctx* ctx, const Args& a) {
     const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
     const int64_t pairs = tile_bound(a, 256, 256);
