@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(RecCfg<DH, COLS>::NT + RecCfg<DH, COLS>::HT) d
     int mine = 0;   // the column of its group whose sums a lane ends up with
 #pragma unroll
     for (int w = COLS / 2, bit = 1; w > 0; w >>= 1, bit <<= 1) mine = mine * 2 + (ag & bit ? 1 : 0);
-    auto write_state = [&](float* dst) {  // dst: dh x dh row-major
+    auto write_state = [&](float* dst) {  // dst: dh x dh row-major, the caller's buffer: of any alignment
+        const bool vec = COLS == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
 #pragma unroll
         for (int p = 0; p < RPT / 2; ++p)
 #pragma unroll
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(RecCfg<DH, COLS>::NT + RecCfg<DH, COLS>::HT) d
                 float x[COLS];
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) x[c] = e ? unpair(S[p][c]).y : unpair(S[p][c]).x;
-                if (COLS == 4) {
+                if (vec) {
                     *reinterpret_cast<float4*>(at) = make_float4(x[0], x[1 % COLS], x[2 % COLS], x[3 % COLS]);
                 } else {
 #pragma unroll

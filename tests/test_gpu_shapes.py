@@ -162,6 +162,33 @@ def test_f32_delta_column_splits(orc, gpu, B, T, H, dh, decay):
     assert rel_err(d_gate[rows].cpu().numpy(), dg_ref) < F32_TOL
 
 
+# The state buffers of the f32 forward may start at any float, in every split of the value columns.
+@pytest.mark.parametrize("B,H,dh", [(2, 2, 32), (30, 20, 32), (80, 20, 32), (20, 8, 64), (40, 8, 64), (2, 8, 128), (6, 8, 128), (12, 8, 128)])
+def test_f32_delta_forward_unaligned_states(gpu, B, H, dh):
+    import ctypes as C
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(B + dh)
+    T, n, size = 70, B * 70, B * H * dh * dh
+    q, k, v = (torch.randn(n, H * dh, generator=g, device="cuda") * dh ** -0.5 for _ in range(3))
+    alpha, beta = (torch.sigmoid(torch.randn(n, H, generator=g, device="cuda")) for _ in range(2))
+    s0 = torch.randn(size, generator=g, device="cuda")
+    got = []
+    for off in (0, 1):
+        init, fin, ck = (torch.zeros(m + 8, device="cuda") for m in (size, size, 2 * size))
+        init[off:off + size] = s0
+        o = torch.empty_like(q)
+        torch.cuda.synchronize()
+        ptr = lambda t: t.data_ptr() + 4 * off  # noqa: E731
+        i64 = C.c_int64
+        gpu._call("asca_delta_fwd", gpu._ctx, *(C.c_void_p(t.data_ptr()) for t in (q, k, v, alpha, beta)), i64(B), i64(T), i64(H), i64(dh), i64(64),
+                  C.c_int(0), C.c_void_p(o.data_ptr()), C.c_void_p(ptr(init)), C.c_void_p(ptr(fin)), C.c_void_p(ptr(ck)))
+        gpu.sync()
+        got.append((o, fin[off:off + size].clone(), ck[off:off + 2 * size].clone()))
+        assert not fin[off + size:].any() and not ck[off + 2 * size:].any()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 # The f32 backward where its chunks do not fit the scratch of one launch (27,473 tiles at dh 16, 8,923 at dh 128): segments of one
 # long chain, segments of many chains, groups of chains, both, and a device without room for any of it (the single kernel). The
 # scratch stays below 1.6 GB; the reference is the single kernel on checkpoints every 32 tokens (both are held to F32_TOL of the
