@@ -650,7 +650,10 @@ __global__ void __launch_bounds__(CH_THREADS, 1) delta_fwd_tc_kernel(
                 float f[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]);
-                if (dst && tid < dhi && cc * 32 < dhi) {
+                if (dst && tid < dhi && cc * 32 < dhi && (reinterpret_cast<uintptr_t>(dst) & 15)) {   // (the caller's s_final)
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) dst[(int64_t)tid * dhi + cc * 32 + j] = f[j];
+                } else if (dst && tid < dhi && cc * 32 < dhi) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         reinterpret_cast<float4*>(dst + (int64_t)tid * dhi + cc * 32)[j] =
@@ -1429,6 +1432,7 @@ int backward(asca_ctx* ctx, const void* q, const void* k, const void* v, const f
              const float* qnorm, const float* knorm, const void* d_o, const float* ckpt, int64_t B, int64_t T, int64_t H,
              int64_t dh, float* d_qkv, float* d_gate) {
     const int64_t n_chunks = (T + C - 1) / C, chains = B * H, n_tiles = chains * n_chunks;
+    ASCA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(d_qkv) & 15) == 0, "delta_bwd: d_qkv must be 16-byte aligned in tensor-core mode");
     Tiles t{};
     int slot = -1;
     for (size_t i = 0; i < ctx->dtiles.size(); ++i) {

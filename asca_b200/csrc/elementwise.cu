@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256) move_rows_kernel(const float* __restrict_
     const int64_t j = idx[r];
     const float* s = src + (SCATTER ? r : j) * (int64_t)cols;
     float* d = dst + (SCATTER ? j : r) * (int64_t)cols;
-    if ((cols & 3) == 0) {
+    if ((((uintptr_t)cols * 4) | reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % 16 == 0) {
         for (int c = lane * 4; c < cols; c += 128)
             *reinterpret_cast<float4*>(d + c) = *reinterpret_cast<const float4*>(s + c);
     } else {
@@ -233,8 +233,10 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, const
                                                     float* __restrict__ m, float* __restrict__ v, int64_t n,
                                                     float lr_t, float b1, float b2, float eps_t, float wd) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * 4;
+    const bool vec_ok = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
+                          reinterpret_cast<uintptr_t>(v)) & 15) == 0;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += stride) {
-        if (i + 3 < n) {
+        if (i + 3 < n && vec_ok) {
             float4 P = *reinterpret_cast<float4*>(p + i), M = *reinterpret_cast<float4*>(m + i),
                    V = *reinterpret_cast<float4*>(v + i);
             const float4 G = *reinterpret_cast<const float4*>(g + i);
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, const
             *reinterpret_cast<float4*>(m + i) = M;
             *reinterpret_cast<float4*>(v + i) = V;
         } else {
-            for (int64_t j = i; j < n; ++j) adamw_one(p[j], g[j], m[j], v[j], lr_t, b1, b2, eps_t, wd);
+            for (int64_t j = i; j < n && j < i + 4; ++j) adamw_one(p[j], g[j], m[j], v[j], lr_t, b1, b2, eps_t, wd);
         }
     }
 }

@@ -196,8 +196,8 @@ int moe_fwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, 
     b.C = out; b.ldc = d; b.N = (int)d; b.K = (int)F; b.c_idx = perm;
     b.bias = b2; b.bias_gstride = 0;
     b.offsets = offsets; b.n_groups = (int)E; b.group_dim = gemm_tc::GROUP_M; b.total_rows = N;
-    // nothing is launched unless every product can run here: the caller falls back as a whole
-    if (!gemm_tc::supported(a) || !gemm_tc::supported(b)) return ASCA_ERR_UNSUPPORTED;
+    // nothing is launched unless the gather (16-byte copies) and every product can run here: the caller falls back as a whole
+    if ((reinterpret_cast<uintptr_t>(xn) & 15) || !gemm_tc::supported(a) || !gemm_tc::supported(b)) return ASCA_ERR_UNSUPPORTED;
     ASCA_CUDA(ctx, asca_launch(ctx, gather_rows_bf16_kernel, dim3((unsigned)ceil_div64(N, 8)), dim3(256), 0, xn, perm, xp, N, (int)d));
     ctx->launches++;
     ASCA_TRY(gemm_tc::launch(ctx, a));
@@ -251,8 +251,9 @@ int moe_bwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, 
     g4.B = w1; g4.ldb = E * F; g4.b_rows = d; g4.b_cols = E * F; g4.b_goff_inner = (int)F;
     g4.C = dxn; g4.ldc = d; g4.N = (int)d; g4.K = (int)F; g4.c_idx = perm;
     g4.offsets = offsets; g4.n_groups = (int)E; g4.group_dim = gemm_tc::GROUP_M; g4.total_rows = N;
-    // nothing is launched unless every product can run here: the caller falls back as a whole, and with
-    // `acc` a partial run followed by the fallback would add some gradients twice
+    // nothing is launched unless the gathers (16-byte loads) and every product can run here: the caller falls back as a whole,
+    // and with `acc` a partial run followed by the fallback would add some gradients twice
+    if (((reinterpret_cast<uintptr_t>(xn) | reinterpret_cast<uintptr_t>(dout)) & 15) != 0) return ASCA_ERR_UNSUPPORTED;
     if (!gemm_tc::supported(g1) || !gemm_tc::supported(g2) || !gemm_tc::supported(g3) || !gemm_tc::supported(g4))
         return ASCA_ERR_UNSUPPORTED;
     gather_rows_bf16_kernel<<<(unsigned)ceil_div64(N, 8), 256, 0, s>>>(xn, perm, xp, N, (int)d);

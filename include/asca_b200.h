@@ -188,7 +188,7 @@ int asca_delta_fwd(asca_ctx* ctx, const void* q, const void* k, const void* v, c
  * rust/src/delta.rs:485-611. Outputs d_qkv (B*T, 3*H*dh) = [dq|dk|dv] after the per-head
  * L2-norm backward and d_gate (B*T, 2H) after the sigmoid backward, both f32. qnorm, knorm
  * (B*T, H) are the pre-normalisation norms from the forward. ckpt comes from asca_delta_fwd
- * with the same `chunk`. */
+ * with the same `chunk`. q, k, v, d_o, ckpt, and d_qkv in the tensor-core mode, must be 16-byte aligned. */
 int asca_delta_bwd(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha,
                    const float* beta, const float* qnorm, const float* knorm, const void* d_o,
                    const float* ckpt, int64_t B, int64_t T, int64_t H, int64_t dh, int64_t chunk,

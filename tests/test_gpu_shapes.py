@@ -233,6 +233,71 @@ def test_f32_delta_backward_in_bounded_scratch(gpu, B, T, H, dh, left):
         assert float((a - b).abs().max() / b.abs().max()) < 2 * F32_TOL
 
 
+# Buffers off the 16-byte grid where the aligned ones move 16 bytes at a time: same results from rows moved, AdamW, the bf16 expert layer
+# (which leaves the tensor cores for it) and the bf16 recurrence's final state; its d_qkv is refused.
+def test_unaligned_device_buffers(gpu):
+    import ctypes as C
+    import torch
+    import asca_b200
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    norm = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    i64, vp = C.c_int64, lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+
+    def off(t):   # the same values one element further on
+        buf = torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")
+        buf[1:1 + t.numel()] = t.reshape(-1)
+        return buf[1:1 + t.numel()].reshape(t.shape)
+
+    src, idx = norm(50, 64), torch.randperm(50, generator=g, device="cuda").int()
+    for call in ("asca_gather_rows", "asca_scatter_rows"):
+        dst = [torch.zeros(50, 64, device="cuda"), off(torch.zeros(50, 64, device="cuda"))]
+        torch.cuda.synchronize()
+        for s, d in zip((src, off(src)), dst):
+            gpu._call(call, gpu._ctx, vp(s), vp(idx), i64(50), i64(64), vp(d))
+        gpu.sync()
+        assert torch.equal(*dst) and dst[0].any()
+
+    p, m, v, gr = norm(1003), norm(1003), norm(1003).abs(), norm(1003)
+    both = [[t.clone() for t in (p, gr, m, v)], [off(t) for t in (p, gr, m, v)]]
+    torch.cuda.synchronize()
+    for a in both:
+        gpu._call("asca_adamw", gpu._ctx, *(vp(t) for t in a), i64(1003), *(C.c_float(x) for x in (1e-2, 0.9, 0.95, 1e-8, 1e-3)))
+    gpu.sync()
+    # (the two loops may contract other multiply-add pairs: a few units of 2^-24 on values of order one)
+    assert all(rel_err(b.cpu().numpy(), a.cpu().numpy()) < 1e-6 for a, b in zip(*both)) and not torch.equal(both[0][0], p)
+
+    n, d, F, E = 300, 128, 192, 4
+    xn, w1, w2 = norm(n, d).bfloat16(), norm(d, E * F).mul(0.1).bfloat16(), norm(E * F, d).mul(0.1).bfloat16()
+    b1, b2, dout = norm(E * F), norm(d), norm(n, d)
+    perm, offs = ops.moe_dispatch(gpu, torch.randint(0, 99, (n,), generator=g, device="cuda", dtype=torch.int32), E)
+    got = []
+    for x, do in ((xn, dout), (off(xn), dout), (xn, off(dout))):
+        out, pre, hid = ops.moe_fwd(gpu, x, w1, b1, w2, b2, perm, offs, F, E)
+        got.append((out, *ops.moe_bwd(gpu, x, w1, w2, pre, hid, do, perm, offs, F, E)))
+    gpu.sync()
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert rel_err(b.cpu().numpy(), a.cpu().numpy()) < 2e-2
+
+    B, T, H, dh = 2, 130, 2, 64
+    q, k, v, d_o = (torch.nn.functional.normalize(norm(B * T, H, dh), dim=-1).reshape(B * T, H * dh).bfloat16() for _ in range(4))
+    alpha, beta, qn = torch.sigmoid(2 + norm(B * T, H)), torch.sigmoid(norm(B * T, H)), torch.ones(B * T, H, device="cuda")
+    fins = [torch.zeros(B, H, dh, dh, device="cuda"), off(torch.zeros(B, H, dh, dh, device="cuda"))]
+    o, ckpt = torch.empty_like(q), torch.empty(ops.delta_ckpt_floats(gpu, B, T, H, dh, 64), device="cuda")
+    torch.cuda.synchronize()
+    for fin in fins:
+        gpu._call("asca_delta_fwd", gpu._ctx, *(vp(t) for t in (q, k, v, alpha, beta)), i64(B), i64(T), i64(H), i64(dh), i64(64),
+                  C.c_int(asca_b200.BF16), vp(o), None, vp(fin), vp(ckpt))
+    gpu.sync()
+    assert torch.equal(*fins) and fins[0].any()
+    d_gate = torch.empty(B * T, 2 * H, device="cuda")
+    with pytest.raises(asca_b200.AscaError, match="d_qkv must be 16-byte aligned"):
+        gpu._call("asca_delta_bwd", gpu._ctx, *(vp(t) for t in (q, k, v, alpha, beta, qn, qn, d_o, ckpt)), i64(B), i64(T), i64(H), i64(dh), i64(64),
+                  C.c_int(asca_b200.BF16), vp(off(torch.empty(B * T, 3 * H * dh, device="cuda"))), vp(d_gate))
+
+
 # The one-kernel dispatch up to its limits (16,384 tokens, 256 experts) and just past them.
 @pytest.mark.parametrize("n,e", [(1, 1), (32, 4), (33, 256), (1025, 7), (16384, 64), (16384, 256), (16385, 64), (2000, 257)])
 def test_dispatch_small_and_past_it(orc, gpu, n, e):
