@@ -330,6 +330,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             // 64 tiles.)
             const bool claimer = dyn && rank == 0, may_be_empty = p.group_dim == GROUP_K || p.K == 0;
             int cur = 0;
+            Tile ahead{};            // the claimer's next tile, where it has been located already
+            bool located = false;
             if (claimer) {
                 cur = atomicAdd(p.dyn_ctr, 1);
                 publish_claim(0, cur);
@@ -338,7 +340,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                 const int t = claimer ? (cur < total_tiles ? cur : -1) : read_tile(ci);
                 if (t < 0) break;
                 int nxt = 0;
-                const Tile x = locate(t);
+                const Tile x = located ? ahead : locate(t);
+                located = false;
                 const int nl0 = x.n0 + rank * BNL;   // first B column this CTA loads
                 if (claimer && x.num_k == 0) nxt = atomicAdd(p.dyn_ctr, 1);
                 for (int kt = 0; kt < x.num_k; ++kt) {
@@ -383,8 +386,11 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     // the publication: behind it, the epilogues could be through the new tile already, and the parity would
                     // mean a tile that is yet to be claimed.
                     const int c = ci + 1;
-                    if (ok && may_be_empty && c >= 2 && nxt < total_tiles && locate(nxt).num_k == 0)
-                        ok = tc::mbar_wait(&acc_empty[c & 1], ((c >> 1) - 1) & 1, abort_flag, p.err_word, 108);
+                    if (ok && may_be_empty && nxt < total_tiles) {
+                        ahead = locate(nxt);
+                        located = true;
+                        if (ahead.num_k == 0 && c >= 2) ok = tc::mbar_wait(&acc_empty[c & 1], ((c >> 1) - 1) & 1, abort_flag, p.err_word, 108);
+                    }
                     cur = ok ? nxt : total_tiles;   // (after a wait that gave up: "none left", so that the other roles stop too)
                     publish_claim(c, cur);
                 }
