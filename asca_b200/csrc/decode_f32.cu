@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(DT, 1) decode_f32_kernel(const __grid_constant
         __syncthreads();
         if (warp == 0) {
             float bv = -INFINITY;
-            int bi = 0x7fffffff;
+            int bi = lane < nv ? v0 + lane : 0x7fffffff;   // (a row of NaNs or of -inf: the lowest index)
             for (int j = lane; j < nv; j += 32)
                 if (hid[j] > bv) {
                     bv = hid[j];
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(DT, 1) decode_f32_kernel(const __grid_constant
                 bi = i;
             }
         }
-        id = bi == 0x7fffffff ? 0u : (uint32_t)bi;   // (a row of NaNs or of -inf: token 0)
+        id = (uint32_t)bi;
         if (rank == 0 && tid == 0) g.tokens[step * g.ns + s] = id;
     }
     for (int li = 0; li < g.L; ++li)

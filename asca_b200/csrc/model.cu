@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ l
     pdl_launch_dependents();
     if (t >= N) return;
     float best = -INFINITY;
-    int bi = 0x7fffffff;
+    int bi = lane < V ? lane : 0x7fffffff;   // (a row of NaNs or of -inf: the lowest index)
     for (int c = lane; c < V; c += 32) {
         const float x = logits[t * V + c];
         if (x > best) {
@@ -310,7 +310,6 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ l
         }
     }
     if (lane == 0) {
-        if (bi == 0x7fffffff) bi = 0;   // a row of NaNs or of -inf
         out[t] = (uint32_t)bi;
         if (toks) toks[(counter ? *counter : 0) * N + t] = (uint32_t)bi;
     }
