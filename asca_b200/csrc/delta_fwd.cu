@@ -10,6 +10,8 @@
 //     (stream, head) streams S through registers once (read + write = the HBM floor).
 #include "common.cuh"
 
+#include <type_traits>
+
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -431,17 +433,14 @@ __global__ void __launch_bounds__(StepCfg<DH>::THREADS) delta_step_kernel(
 // per-column quantity (S^T k, u, the update, S^T q) is local to the lane, so the step needs no block barrier and
 // no cross-lane reduction except the two norms of the fused prologue; k and q are broadcast from the warp's slice
 // of shared memory. qkv / gate may be the two parts of one wider row (row pitches ld_qkv, ld_gate); o16, when
-// given, receives a bf16 copy of the output for a following tensor-core product. S_off, when given, is a device word
-// that holds how many floats behind S the states are (a captured launch then serves any state buffer; an offset and not an
-// address, so that the compiler still knows the memory space); like the state itself it was final before the previous kernel began.
+// given, receives a bf16 copy of the output for a following tensor-core product.
 constexpr int SW_WARPS = 8;
 __global__ void __launch_bounds__(SW_WARPS * 32) delta_step_warp64_kernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, const float* __restrict__ alpha,
-    const float* __restrict__ beta, float* __restrict__ S, const int64_t* __restrict__ S_off, int64_t n_units, int H, int fused,
-    int64_t ld_qkv, int64_t ld_gate, float* __restrict__ o, __nv_bfloat16* __restrict__ o16) {
+    const float* __restrict__ beta, float* __restrict__ S, int64_t n_units, int H, int fused, int64_t ld_qkv,
+    int64_t ld_gate, float* __restrict__ o, __nv_bfloat16* __restrict__ o16) {
     constexpr int DH = 64;
     __shared__ __align__(16) float kq_s[SW_WARPS][2][DH];
-    if (S_off) S += *S_off;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     bool waited = false;   // the state is this kernel's own (last written a step ago): the first unit's loads are issued
                            // before the wait for the previous kernel, whose output is only q, k, v and the gates
@@ -545,8 +544,20 @@ cudaError_t launch_fwd(asca_ctx* ctx, const void* q, const void* k, const void* 
 
 }  // namespace
 
-int asca_delta_step_at(asca_ctx* ctx, const float* qkv, int64_t ld_qkv, const float* gate, int64_t ld_gate, float* S, const int64_t* S_off,
-                       int64_t n_streams, int64_t H, float* o, void* o16);
+template <typename... A>
+std::integral_constant<int, sizeof...(A)> n_args(void (*)(A...));
+// A recorded launch of delta_step_warp64_kernel goes to the states at S from now on (launches under way keep theirs).
+int asca_delta_step_repoint(asca_ctx* ctx, cudaGraphExec_t exec, cudaGraphNode_t node, float* S) {
+    constexpr int N_ARGS = decltype(n_args(delta_step_warp64_kernel))::value, S_ARG = 5;   // (q, k, v, alpha, beta, S, ...)
+    cudaKernelNodeParams kp;
+    ASCA_CUDA(ctx, cudaGraphKernelNodeGetParams(node, &kp));
+    void* args[N_ARGS];
+    for (int i = 0; i < N_ARGS; ++i) args[i] = kp.kernelParams[i];
+    args[S_ARG] = &S;
+    kp.kernelParams = args;
+    ASCA_CUDA(ctx, cudaGraphExecKernelNodeSetParams(exec, node, &kp));
+    return ASCA_OK;
+}
 
 extern "C" {
 
@@ -606,13 +617,6 @@ int asca_delta_fwd(asca_ctx* ctx, const void* q, const void* k, const void* v, c
 // o16 (nullable) gets a bf16 copy of o. dh = 64.
 int asca_delta_step_strided(asca_ctx* ctx, const float* qkv, int64_t ld_qkv, const float* gate, int64_t ld_gate, float* S,
                             int64_t n_streams, int64_t H, float* o, void* o16) {
-    return asca_delta_step_at(ctx, qkv, ld_qkv, gate, ld_gate, S, nullptr, n_streams, H, o, o16);
-}
-}  // extern "C"
-
-// The same with the states S_off floats behind S (a device word; null: at S).
-int asca_delta_step_at(asca_ctx* ctx, const float* qkv, int64_t ld_qkv, const float* gate, int64_t ld_gate, float* S, const int64_t* S_off,
-                       int64_t n_streams, int64_t H, float* o, void* o16) {
     if (!ctx) return ASCA_ERR_ARG;
     ASCA_REQUIRE(ctx, qkv && gate && S && o && n_streams >= 0 && H > 0, "delta_step_strided: bad arguments");
     ASCA_REQUIRE(ctx, ld_qkv >= 3 * H * 64 && ld_gate >= 2 * H && (ld_qkv & 1) == 0, "delta_step_strided: bad row pitch");
@@ -623,12 +627,10 @@ int asca_delta_step_at(asca_ctx* ctx, const float* qkv, int64_t ld_qkv, const fl
     const int64_t n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
     asca_span sp(ctx, "delta_step_warp64_kernel", (double)units * 2.0 * 64 * 64 * 4);   // state bytes read + written
     ASCA_CUDA(ctx, asca_launch(ctx, delta_step_warp64_kernel, dim3((unsigned)std::min(n_sm, ceil_div64(units, SW_WARPS))), dim3(SW_WARPS * 32), 0,
-                               qkv, nullptr, nullptr, gate, nullptr, S, S_off, units, (int)H, 1, ld_qkv, ld_gate, o, (__nv_bfloat16*)o16));
+                               qkv, nullptr, nullptr, gate, nullptr, S, units, (int)H, 1, ld_qkv, ld_gate, o, (__nv_bfloat16*)o16));
     ctx->launches++;
     return ASCA_OK;
 }
-
-extern "C" {
 
 int asca_delta_step(asca_ctx* ctx, const float* q, const float* k, const float* v, const float* alpha,
                     const float* beta, float* S, int64_t n_streams, int64_t H, int64_t dh, int fused, float* o) {
@@ -645,7 +647,7 @@ int asca_delta_step(asca_ctx* ctx, const float* q, const float* k, const float* 
         const int64_t units = n_streams * H;
         const int64_t n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
         delta_step_warp64_kernel<<<(unsigned)std::min(n_sm, ceil_div64(units, SW_WARPS)), SW_WARPS * 32, 0, ctx->stream>>>(
-            q, k, v, alpha, beta, S, nullptr, units, (int)H, fused, 3 * H * dh, 2 * H, o, nullptr);
+            q, k, v, alpha, beta, S, units, (int)H, fused, 3 * H * dh, 2 * H, o, nullptr);
         ASCA_CHECK_LAUNCH(ctx);
         return ASCA_OK;
     }

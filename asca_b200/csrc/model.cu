@@ -435,14 +435,12 @@ struct DecodeForm {
 };
 // What a decode call uploads in one copy, the first tokens behind it.
 struct DecodeIn {
-    int64_t state;     // where the states are, in floats behind this record
     int32_t counter;   // row of the token buffer, advanced by the prologue of each step
-    int32_t unused;
+    int32_t unused[3];
 };
 // The buffers of a decode step; cur: the step's token ids in, its argmax out.
 struct DecodeBufs {
     uint32_t *in, *cur, *toks;
-    const int64_t* state_off;
     int32_t *perm, *offs, *inv_perm, *counter;
     float *x, *qkv, *gate, *o, *y, *x_mid, *mo, *logits, *pre_p, *qg;
     __nv_bfloat16 *x16, *o16, *xn16, *hid16, *hf16;
@@ -459,7 +457,7 @@ struct DecodeBufs {
         auto h16 = [&](int64_t n) { return (__nv_bfloat16*)f32((n + 1) / 2); };
         constexpr int64_t HEAD = sizeof(DecodeIn) / 4;
         in = (uint32_t*)f32(HEAD + ns); cur = in + HEAD; toks = (uint32_t*)f32(ns * n_steps);
-        state_off = reinterpret_cast<const int64_t*>(in); counter = reinterpret_cast<int32_t*>(in) + offsetof(DecodeIn, counter) / 4;
+        counter = reinterpret_cast<int32_t*>(in) + offsetof(DecodeIn, counter) / 4;
         perm = i32(ns); offs = i32(m->E + 1); inv_perm = i32(ns, f.sorted_moe);
         x = f32(ns * d); o = f32(ns * d); y = f32(ns * d); logits = f32(ns * m->vocab);
         qg = f32(ns * f.ldq, f.fused64); qkv = f32(ns * 3 * d, !f.fused64); gate = f32(ns * 2 * H, !f.fused64);
@@ -470,13 +468,12 @@ struct DecodeBufs {
 };
 }  // namespace
 
-int asca_delta_step_at(asca_ctx* ctx, const float* qkv, int64_t ld_qkv, const float* gate, int64_t ld_gate, float* S, const int64_t* S_off,
-                       int64_t n_streams, int64_t H, float* o, void* o16);   // delta_fwd.cu
+int asca_delta_step_repoint(asca_ctx* ctx, cudaGraphExec_t exec, cudaGraphNode_t node, float* S);   // delta_fwd.cu
 
 // One decode step from b.cur; the choice lands in b.cur and in the token buffer (toks_row where the prologue does not count).
-// state null (the fused64 form only): the states are where b.state_off says.
+// updates (nullable; the fused64 form under capture): gets the graph nodes of the state updates, block by block.
 static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeForm& f, const DecodeBufs& b, float* state, int64_t ns,
-                                   bool pdl_first, uint32_t* toks_row) {
+                                   bool pdl_first, uint32_t* toks_row, std::vector<cudaGraphNode_t>* updates = nullptr) {
     typedef __nv_bfloat16 bf16;
     const int64_t d = m->d, H = m->H, dh = d / H, E = m->E, F = m->F, V = m->vocab, ldq = f.ldq;
     const int BF = ASCA_BF16;
@@ -521,9 +518,16 @@ static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeFor
         if (f.fused64) {
             if (f.packed) ASCA_TRY(few_rows(b.x16, d, m->dec_pk + li * f.r_layer * 64, ldq, b.qg, ldq, m->dec_b + li * ldq));
             else ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, ldq, d, b.x16, d, m->dec_w + li * d * ldq, ldq, b.qg, ldq, m->dec_b + li * ldq, 0, BF));
-            const int64_t at = li * ns * H * dh * dh;
-            ASCA_TRY(asca_delta_step_at(ctx, b.qg, ldq, b.qg + 3 * d, ldq, (state ? state : (float*)b.in) + at, state ? nullptr : b.state_off, ns, H,
-                                        b.o, b.o16));
+            ASCA_TRY(asca_delta_step_strided(ctx, b.qg, ldq, b.qg + 3 * d, ldq, state + li * ns * H * dh * dh, ns, H, b.o, b.o16));
+            if (updates) {
+                cudaStreamCaptureStatus st;
+                const cudaGraphNode_t* last;
+                const cudaGraphEdgeData* edges;
+                size_t n = 0;
+                ASCA_CUDA(ctx, cudaStreamGetCaptureInfo_v3(ctx->stream, &st, nullptr, nullptr, &last, &edges, &n));
+                ASCA_REQUIRE(ctx, st == cudaStreamCaptureStatusActive && n == 1, "model_decode_step: not the only launch under capture");
+                updates->push_back(last[0]);
+            }
         } else {
             ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 3 * d, d, b.x16, d, W + w16.w_qkv, 3 * d, b.qkv, 3 * d, P + w.b_qkv, 0, BF));
             ASCA_TRY(asca_gemm(ctx, ASCA_NN, ns, 2 * H, d, b.x16, d, W + w16.w_gate, 2 * H, b.gate, 2 * H, P + w.b_gate, 0, BF));
@@ -557,7 +561,9 @@ static int decode_step_bf16_device(asca_ctx* ctx, asca_model* m, const DecodeFor
 // A plan's graph and buffers go; the stream has been waited for.
 static void drop_plan(asca_plan& p) {
     if (p.exec) cudaGraphExecDestroy(p.exec);
+    if (p.graph) cudaGraphDestroy(p.graph);
     p.exec = nullptr;
+    p.graph = nullptr;
     for (void* x : p.held) asca_free(p.ctx, x);
     p.held.clear();
 }
@@ -611,9 +617,9 @@ struct PlanUse {   // keeps a plan while a call works with it
 };
 
 // Captures `body` (launches on ctx->stream) into an executable graph, on a stream of the context's own: the caller's may be
-// one that cannot be captured. Blocks the sequence gives back meanwhile go to `held`.
+// one that cannot be captured. Blocks the sequence gives back meanwhile go to `held`; kept (nullable): the graph itself.
 template <class Body>
-static int capture(asca_ctx* ctx, cudaGraphExec_t* exec, int64_t* launches, std::vector<void*>* held, Body body) {
+static int capture(asca_ctx* ctx, cudaGraphExec_t* exec, int64_t* launches, std::vector<void*>* held, Body body, cudaGraph_t* kept = nullptr) {
     if (!ctx->cap_stream) ASCA_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
     cudaStream_t user = ctx->stream;
     const int64_t before = ctx->launches;
@@ -629,7 +635,8 @@ static int capture(asca_ctx* ctx, cudaGraphExec_t* exec, int64_t* launches, std:
     ctx->hold = nullptr;
     ctx->stream = user;
     if (rc == ASCA_OK && cudaGraphInstantiate(exec, graph, 0) != cudaSuccess) rc = ASCA_ERR_CUDA;
-    if (graph) cudaGraphDestroy(graph);
+    if (kept && rc == ASCA_OK) *kept = graph;
+    else if (graph) cudaGraphDestroy(graph);
     *launches = ctx->launches - before;
     ctx->launches = before;
     if (rc != ASCA_OK) {
@@ -684,7 +691,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
     }
     std::vector<uint32_t> in(sizeof(DecodeIn) / 4 + ns);
     auto upload = [&](uint32_t* to) {
-        const DecodeIn head = {(int64_t)(reinterpret_cast<intptr_t>(state) - reinterpret_cast<intptr_t>(to)) / 4, -1, 0};
+        const DecodeIn head = {-1, {}};
         memcpy(in.data(), &head, sizeof head);
         memcpy(in.data() + sizeof head / 4, ids_h, (size_t)ns * 4);
         return asca_stage_in(ctx, to, in.data(), in.size() * 4);
@@ -694,7 +701,7 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
     asca_decode_plan* p = nullptr;
     PlanUse use;
     const int64_t cap = std::max<int64_t>(1, ((int64_t)1 << 18) / ns);   // a plan's token buffer: the steps that 1 MiB holds
-    if (f.packed && f.one_prologue && !ctx->profiling && (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
+    if (f.packed && f.one_prologue && !ctx->profiling && (reinterpret_cast<uintptr_t>(state) & 7) == 0) {
         for (auto& q : m->dec_plans)
             if (q.ctx == ctx && q.ns == ns && q.w16 == W && q.dec_w == m->dec_w && q.dec_pk == m->dec_pk) p = &q;
         if (!p) {
@@ -709,12 +716,27 @@ static int decode_step_bf16(asca_ctx* ctx, asca_model* m, float* state, const ui
             Bufs own(ctx);
             int rc = pb.take(own, m, f, ns, cap) ? ASCA_OK : ASCA_ERR_OOM;
             if (rc == ASCA_OK)
-                rc = capture(ctx, &p->exec, &p->launches, &p->held, [&] { return decode_step_bf16_device(ctx, m, f, pb, nullptr, ns, false, nullptr); });
+                rc = capture(ctx, &p->exec, &p->launches, &p->held,
+                             [&] { return decode_step_bf16_device(ctx, m, f, pb, state, ns, false, nullptr, &p->updates); }, &p->graph);
             if (rc == ASCA_OK) {
+                p->state = state;
                 p->held.insert(p->held.end(), own.p.begin(), own.p.end());   // the graph's buffers stay with it
                 own.p.clear();
                 p->in = pb.in; p->cur = pb.cur; p->toks = pb.toks; p->counter = pb.counter; p->logits = pb.logits;
             } else {
+                p->broken = true;
+            }
+        }
+        if (p->exec && p->state != state) {   // another state buffer than last time
+            int rc = ASCA_OK;
+            for (size_t li = 0; li < p->updates.size() && rc == ASCA_OK; ++li)
+                rc = asca_delta_step_repoint(ctx, p->exec, p->updates[li], state + (int64_t)li * ns * H * dh * dh);
+            p->state = state;
+            if (rc != ASCA_OK) {   // this many streams are launched directly from now on
+                cudaGetLastError();
+                cudaStreamSynchronize(ctx->stream);
+                cudaGraphExecDestroy(p->exec);
+                p->exec = nullptr;
                 p->broken = true;
             }
         }

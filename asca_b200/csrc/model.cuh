@@ -20,6 +20,7 @@ struct asca_plan {
     asca_ctx* ctx = nullptr;
     int runs = 0;               // direct runs so far
     cudaGraphExec_t exec = nullptr;
+    cudaGraph_t graph = nullptr;   // kept where its nodes are asked for later
     bool broken = false;        // could not be captured
     bool busy = false;          // a call is working with it
     uint64_t stamp = 0;
@@ -40,10 +41,13 @@ struct asca_step_plan : asca_plan {
 };
 
 // The same for a bf16 decode step on the packed weights: one graph is one step of `ns` streams, its tokens in and out through
-// `cur`. Where the states are is part of the input (`in`), so any state buffer of that many streams is served.
+// `cur`. The state updates of the blocks are pointed at another state buffer when a call comes with one (about a
+// microsecond a block; a word on the device that they would all read first takes 0.4 us a block and step).
 struct asca_decode_plan : asca_plan {
     int64_t ns = 0;
     const void *w16 = nullptr, *dec_w = nullptr, *dec_pk = nullptr;   // the weight copies the graph reads
+    const float* state = nullptr;                                     // where its state updates go at present
+    std::vector<cudaGraphNode_t> updates;                             // one per block
     uint32_t *in = nullptr, *cur = nullptr, *toks = nullptr;
     int32_t* counter = nullptr;
     float* logits = nullptr;
