@@ -650,10 +650,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) delta_fwd_tc_kernel(
                 float f[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]);
-                if (dst && tid < dhi && cc * 32 < dhi && (reinterpret_cast<uintptr_t>(dst) & 15)) {   // (the caller's s_final)
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) dst[(int64_t)tid * dhi + cc * 32 + j] = f[j];
-                } else if (dst && tid < dhi && cc * 32 < dhi) {
+                if (dst && tid < dhi && cc * 32 < dhi) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         reinterpret_cast<float4*>(dst + (int64_t)tid * dhi + cc * 32)[j] =
@@ -1356,6 +1353,16 @@ static int run_prepass(asca_ctx* ctx, const void* q, const void* k, const void* 
 // in its first half: the backward loads them by TMA as tensor-core operands.
 int forward(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
             int64_t B, int64_t T, int64_t H, int64_t dh, void* o, const float* s_init, float* s_final, float* ckpt) {
+    if (s_final && (reinterpret_cast<uintptr_t>(s_final) & 15)) {   // the kernel writes the final state 16 bytes at a time
+        const size_t bytes = (size_t)(B * H * dh * dh) * 4;
+        void* fin;
+        ASCA_TRY(asca_malloc(ctx, bytes, &fin));
+        int rc = forward(ctx, q, k, v, alpha, beta, B, T, H, dh, o, s_init, (float*)fin, ckpt);
+        if (rc == ASCA_OK && cudaMemcpyAsync(s_final, fin, bytes, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
+            rc = asca_fail(ctx, ASCA_ERR_CUDA, "delta_fwd: cannot copy the final state");
+        asca_free(ctx, fin);   // (reused by later work on the stream only)
+        return rc;
+    }
     const int64_t n_chunks = (T + C - 1) / C, chains = B * H, n_tiles = chains * n_chunks;
     Tiles t{};
     const bool keep = ckpt != nullptr;
