@@ -586,7 +586,7 @@ int asca_delta_fwd(asca_ctx* ctx, const void* q, const void* k, const void* v, c
         }
         return ASCA_OK;
     }
-    // bf16 mode, dh = 128 (or 64, zero-padded inside): chunk-parallel WY/UT form on the tensor cores (checkpoints every 64)
+    // bf16 mode, dh = 128 or 64: chunk-parallel WY/UT form on the tensor cores (checkpoints every 64)
     if (dtype == ASCA_BF16 && (dh == 128 || dh == 64) && (!ckpt || chunk == 64) && asca_tc_enabled() && delta_tc::available())
         return delta_tc::forward(ctx, q, k, v, alpha, beta, B, T, H, dh, o, s_init, s_final, ckpt);
     if (ckpt)

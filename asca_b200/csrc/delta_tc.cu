@@ -1,90 +1,117 @@
-// Gated delta rule, bf16 mode, chunk-parallel WY/UT forward on the 5th-generation tensor cores.
+// Gated delta rule, bf16 mode: chunk-parallel WY/UT form on the 5th-generation tensor cores, head dim 128 or 64.
 //
-// Chunk of C = 64 tokens, head dim 128, state S (128 x 128) kept in f32 in TMEM for the whole
-// sequence. With g = cumsum(log alpha), gam = exp(g), Gam[t,i] = exp(g_t - g_i), eg = exp(g_C - g):
+// Chunk of C = 64 tokens, state S (DH x DH, key x value) in f32 in TMEM for the whole sequence. With g = cumsum(log alpha) inside
+// a chunk, gam = exp(g), Gam[t,i] = exp(g_t - g_i), eg = exp(g_C - g), everything that depends on neither S nor dS is taken off the
+// two serial chains:
 //
-//   pre-pass (one CTA per (sequence, head, chunk) -- fully parallel, nothing depends on S):
-//     KK = K K^T, QK = Q K^T                                   tcgen05, M128 N64 K128 ([K;Q] stacked)
-//     L  = strictlower(beta_t Gam KK)   A = lower(Gam QK)      f32 registers
-//     X  = (I + L)^-1  (T' = X - I)                            f32, 16 x 16 blocks: substitution on the
-//                                                              diagonal, block products below it
-//     W^ = X (beta gam K),  Uv = X (beta V)                    tcgen05, two M64 N128 K64 products sharing
-//                                                              TMEM columns in the two lane halves
-//     Qg = gam Q,  Kw = eg K                                   bf16 tiles for the chain kernel
-//   chain (one CTA per (sequence, head), 64 dependent chunks):
-//     [W^ S0 ; Qg S0]                                          tcgen05, M128 N128 K128
-//     U  = Uv - W^ S0                                          TMEM -> registers -> bf16 smem operand
-//     O  = Qg S0 + A U                                         tcgen05 accumulate, M128(padded) N128 K64
-//     S  = gam_C S0 + Kw^T U                                   tcgen05 accumulate onto the f32 state in
-//                                                              TMEM, pre-scaled by gam_C with ld/st
-// The chain kernel's tiles arrive by TMA (plain 2-D tile loads, 128-byte swizzle, two stages);
-// U and the bf16 copy of S are written into the same swizzled operand layouts by the compute
-// threads. S reaches HBM only as chunk-boundary checkpoints (f32) and the final state.
+//   delta_prep_tc_kernel   one CTA per (chunk, chain)
+//     L = strictlower(beta_t Gam K K^T), A = lower(Gam Q K^T), X = (I + L)^-1 (f32), W^ = X diag(beta gam) K, Uv = X diag(beta) V
+//   delta_fwd_tc_kernel    one CTA per chain, two dependent products a chunk
+//     U = Uv - W^ S          S <- gam_C S + K^T (eg U)          o = gam (Q S) + A U      (o off the serial path)
+//   delta_bwd_tc_kernel    one CTA per chain in reverse, three dependent products a chunk
+//     dU = A^T dO + eg (K dS)    dR = X^T dU    dS <- gam_C dS + Q^T (gam dO) - K^T (beta gam dR)    dv = beta dR
+//   delta_grad_tc_kernel   one CTA per (chunk, chain): dq, dk and the gate gradients from S, dS, U and dR, see its header
+//
+// Row factors (gam, eg, beta) are applied in f32 to results or to the rows of a 64-row operand just before it is rounded, never
+// to copies of q, k, v: the kernels read those straight from the caller's tensors, and what travels between them per (chunk, chain) is
+// W^, Uv, A, X - I (56 KB at DH 128) and, for a backward, S, U (in the checkpoint buffer) and dS, dR. A travels as two bf16
+// tiles, value and remainder: the rounding of an entry of A meets a whole row of U or dO, an error common to 128 columns that was most of
+// what the gate gradients and o's sums over heads had.
+//
+// Tiles arrive by TMA (plain loads, 128-byte swizzle); a box that runs past a sequence's end is filled with zeros. Many products have
+// 64 rows: they either run as M = 128 with whatever lies behind the operand as rows 64 - 127 (the results of those rows land
+// in TMEM lanes that nobody reads; an M = 64 instruction takes as long), or as two M = 64 products in the two 16-lane halves of
+// each TMEM lane quarter.
 //
 // Every mbarrier wait is bounded (tc::mbar_wait): a wait that runs out sets the context's error
 // word, and the CTA still frees its TMEM and exits.
-//
-// Head dim 64 runs on the same kernels with every head zero-padded to 128 (`dhi` = the head dim in the caller's
-// tensors): the pre-pass reads 64 columns and fills the other 64 of its operand tiles with zeros, the chain kernels'
-// tiles, TMEM state and products keep the 128 shapes (the padded rows and columns of S, dS and of every product are
-// exact zeros), and only the accesses to the caller's tensors (q, k, v, o, dO, d_qkv, initial / final state, and the
-// chunk-start states kept for the backward: the live 64 x 64 block as bf16) use the 64-wide layout.
 #include "common.cuh"
 #include "tc_common.cuh"
 
 namespace delta_tc {
 
 constexpr int C = 64;     // chunk length
-constexpr int DH = 128;   // head dim handled by this file
-constexpr int NB = DH / 64;
 
-struct Tiles {            // intermediate buffers, one tile per (chain, chunk)
-    __nv_bfloat16* WQ;    // [tile][128][DH]: rows 0-63 W^, rows 64-127 Qg
-    __nv_bfloat16* UV;    // [tile][64][DH]
-    __nv_bfloat16* KW;    // [tile][64][DH]
-    __nv_bfloat16* AA;    // [tile][64][64]
-    float* GC;            // [tile] gam_C (total decay of the chunk)
-    // backward-only outputs (null in the forward)
-    __nv_bfloat16* BK;    // [tile][64][DH]  beta gam K
-    __nv_bfloat16* BV;    // [tile] beta V, 64 x DH, lane-major (see lm_off128)
-    __nv_bfloat16* UVT;   // [tile] Uv, 64 x DH, lane-major copy for the backward
-    __nv_bfloat16* TP;    // [tile][64][64]  T' = (I+L)^-1 - I, row-major
-    __nv_bfloat16* KKo;   // [tile] K K^T, 64 x 64, lane-major (see lm_off64)
-    __nv_bfloat16* QKo;   // [tile] Q K^T, 64 x 64, lane-major
-    float* GV;            // [tile][64] cumulative log alpha
-    float* BE;            // [tile][64] beta (0 on padded steps)
+// Intermediate buffers, one tile per (chain, chunk), DH wide; and per-token vectors.
+struct Tiles {
+    __nv_bfloat16* WH;    // [tile][64][DH]  W^
+    __nv_bfloat16* UV;    // [tile][64][DH]  Uv
+    __nv_bfloat16* AA;    // [tile][64][64]  A
+    __nv_bfloat16* AL;    // [tile][64][64]  what A loses in bf16, itself bf16
+    __nv_bfloat16* TP;    // [tile][64][64]  X - I (null without a backward)
+    float* GB;            // [tile][64], [64] cumulative log alpha (constant past the sequence's end), beta (0 there)
 };
 
-// Lane-major tile layouts for rows that the backward's threads read straight from global memory.
-// There, thread (warp quarter wq = row / 16, lane = row % 16, column half) reads its 16-byte chunks
-// j = 0.. one per instruction; storing chunk j of 16 consecutive rows side by side makes each such
-// instruction touch 256 contiguous bytes. Offsets are in bf16 elements within one tile.
-__device__ __forceinline__ int lm_off128(int row, int chunk16) {   // 64 x 128 tile, column halves of 8 chunks
-    return ((((row >> 4) * 2 + (chunk16 >> 3)) * 8 + (chunk16 & 7)) * 16 + (row & 15)) * 8;
+// 512 bytes (a tile's row of GB) into shared memory
+__device__ __forceinline__ void load_vec(void* dst, const float* src, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 512, [%2];"
+                 ::"r"(tc::smem_u32(dst)), "l"(src), "r"(tc::smem_u32(bar))
+                 : "memory");
 }
-__device__ __forceinline__ int lm_off64(int row, int chunk16) {    // 64 x 64 tile, column halves of 4 chunks
-    return ((((row >> 4) * 2 + (chunk16 >> 2)) * 4 + (chunk16 & 3)) * 16 + (row & 15)) * 8;
+// 32 columns of a row, 32 bytes at a time where the rows lie on that grid
+__device__ __forceinline__ void store32(float* p, const float (&v)[32], bool w32) {
+    if (w32) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+            asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                         ::"f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]), "f"(v[j + 4]), "f"(v[j + 5]), "f"(v[j + 6]), "f"(v[j + 7]), "l"(p + j)
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    }
+}
+__device__ __forceinline__ void store16(float* p, const float (&v)[16], bool w32) {
+    if (w32) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 8)
+            asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                         ::"f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]), "f"(v[j + 4]), "f"(v[j + 5]), "f"(v[j + 6]), "f"(v[j + 7]), "l"(p + j)
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    }
+}
+__device__ __forceinline__ void store32_bf16(__nv_bfloat16* p, const float (&v)[32], bool w32) {
+    uint4 h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = tc::pack8_bf16(v + 8 * j);
+    if (w32) {
+#pragma unroll
+        for (int j = 0; j < 4; j += 2)
+            asm volatile("st.global.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                         ::"r"(h[j].x), "r"(h[j].y), "r"(h[j].z), "r"(h[j].w), "r"(h[j + 1].x), "r"(h[j + 1].y), "r"(h[j + 1].z), "r"(h[j + 1].w), "l"(p + 8 * j)
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(p)[j] = h[j];
+    }
 }
 
 // ------------------------------------------------------------------ pre-pass
-constexpr int PRE_THREADS = 128;
-constexpr int LF_LD = 68;     // row stride (floats) of the f32 L and X matrices: float4 rows, conflict-free
-constexpr int YF_LD = 16;
-// Shared memory is sized for three CTAs per SM: the K/Q operand tiles are dead once KK and QK exist, so the
-// f32 L and X matrices, and later the bf16 operand tile of X, live in the same region.
-constexpr int PRE_R1 = 2 * 64 * LF_LD * 4;        // >= NB * 16384
-constexpr size_t PRE_SMEM = 1024 + PRE_R1 + 2 * NB * 8192 /*Bop, later W^/Uv staging*/ + 3 * 16 * YF_LD * 4 + 4 * 64 * 4 + 64;
-static_assert(PRE_R1 >= NB * 16384 && PRE_R1 % 1024 == 0 && (64 * LF_LD * 4) % 1024 == 0, "pre-pass shared-memory layout");
+constexpr int PRE_THREADS = 256;
+// The f32 matrices L and X are lower triangular: their ten 16 x 16 blocks are kept side by side, rows 20 floats apart (float4
+// reads of eight rows at a time fall in different banks).
+constexpr int BLD = 20, BSZ = 16 * BLD;
+constexpr int TRI_BYTES = 10 * BSZ * 4;           // 12,800
+constexpr int L_BYTES = 13312;                    // TRI_BYTES and two 64-float vectors; later an 8 KiB operand tile in L's place
+static_assert(L_BYTES == TRI_BYTES + 512 && L_BYTES % 1024 == 0, "pre-pass shared-memory layout");
+__host__ __device__ constexpr int tri(int I, int J) { return (I * (I + 1) / 2 + J) * BSZ; }
+template <int DH>
+constexpr size_t pre_smem() {
+    return 1024 + (size_t)(DH / 64) * 24576 /*K, Q, V*/ + L_BYTES + TRI_BYTES + 64 * 4 + 64;
+}
 
 // One 1 x 4 strip of a 16 x 16 block product  acc += Lrow[0..16) * X[0..16)[c4..c4+4)  (f32, shared memory).
-__device__ __forceinline__ void strip16(const float* __restrict__ lrow, const float* __restrict__ x, int ldx, float acc[4]) {
+__device__ __forceinline__ void strip16(const float* __restrict__ lrow, const float* __restrict__ x, float acc[4]) {
 #pragma unroll
     for (int k4 = 0; k4 < 4; ++k4) {
         const float4 l4 = *reinterpret_cast<const float4*>(lrow + 4 * k4);
         const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const float4 x4 = *reinterpret_cast<const float4*>(x + (4 * k4 + e) * ldx);
+            const float4 x4 = *reinterpret_cast<const float4*>(x + (4 * k4 + e) * BLD);
             acc[0] = fmaf(lv[e], x4.x, acc[0]);
             acc[1] = fmaf(lv[e], x4.y, acc[1]);
             acc[2] = fmaf(lv[e], x4.z, acc[2]);
@@ -92,64 +119,70 @@ __device__ __forceinline__ void strip16(const float* __restrict__ lrow, const fl
         }
     }
 }
+__device__ __forceinline__ void put4(float* p, const float acc[4], float f) {
+    *reinterpret_cast<float4*>(p) = make_float4(f * acc[0], f * acc[1], f * acc[2], f * acc[3]);
+}
 
+// Three CTAs of eight warps per SM. K, Q and V come by TMA and are never copied: the factors beta gam and beta go into the
+// columns of X - I, once per product, and the rows that the identity contributes are added in f32 (a rounded diagonal would be an error
+// common to a whole row of W^ and Uv: 15 % of the error of o, dq and dk).
+template <int DH>
 __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
-    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-    const float* __restrict__ alpha, const float* __restrict__ beta, int T, int H, int dhi, int n_chunks, Tiles out,
-    int* err_word) {
+    const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapV,
+    const __grid_constant__ CUtensorMap mapWH, const __grid_constant__ CUtensorMap mapUV, const float* __restrict__ alpha,
+    const float* __restrict__ beta, int T, int H, int n_chunks, Tiles out, int* err_word) {
+    constexpr int NB = DH / 64;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* KQ_s = base;                         // NB k-boxes x (128 rows x 128 B): rows 0-63 K, 64-127 Q
-    uint8_t* Bop_s = KQ_s + PRE_R1;               // 2*NB n-boxes x (64 k-rows x 128 B): [beta gam K | beta V]
-    float* Xf = reinterpret_cast<float*>(KQ_s);   // (I + L)^-1 in f32, once K and Q have been consumed
-    float* Lf = Xf + 64 * LF_LD;                  // L in f32
-    uint8_t* Tp_s = reinterpret_cast<uint8_t*>(Lf);   // 64 rows x 128 B: (I + L)^-1 as the K-major operand, once L is dead
-    float* Yf = reinterpret_cast<float*>(Bop_s + 2 * NB * 8192);   // [3][16][YF_LD] block products in flight
-    float* g_s = Yf + 3 * 16 * YF_LD;
-    float* gam_s = g_s + 64;
-    float* eg_s = gam_s + 64;
-    float* be_s = eg_s + 64;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(be_s + 64);   // [0] MMA-A done, [1] MMA-B done
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 2);
+    uint8_t* KQ_s = base;                         // NB boxes of 128 rows x 128 B: rows 0-63 K, 64-127 Q
+    uint8_t* V_s = KQ_s + NB * 16384;             // NB boxes of 64 rows
+    float* Lf = reinterpret_cast<float*>(V_s + NB * 8192);
+    float* Xf = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(Lf) + L_BYTES);
+    float* g_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(Xf) + TRI_BYTES);
+    float* bg_s = Lf + TRI_BYTES / 4;             // beta gam
+    float* be_s = bg_s + 64;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(g_s + 64);   // [0] K, Q; [1] MMA-A done; [2] MMA-B done; [3] V
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* wtot = reinterpret_cast<float*>(tmem_slot + 2);
+    uint8_t* X1_s = KQ_s + 8192;                  // (X - I) diag(beta gam) as an operand: where Q's first box was
+    uint8_t* X2_s = reinterpret_cast<uint8_t*>(Lf);   // (X - I) diag(beta): where L was
+    float* Yf = reinterpret_cast<float*>(X1_s);   // [4] blocks in flight
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int wq = warp & 3, cg = warp >> 2;      // TMEM lane quarter, column group
     const int chunk = blockIdx.x, chain = blockIdx.y;
     const int b = chain / H, h = chain % H;
-    const int d = H * dhi;
     const int t0 = chunk * C;
     const int n = T - t0 < C ? T - t0 : C;
     const int64_t row0 = (int64_t)b * T + t0;
     const int64_t tix = (int64_t)chain * n_chunks + chunk;
 
-    // K, Q, V rows of the chunk: every load is issued before anything waits on one
-    const int sj = tid & 15;                      // 16-byte chunk of the row handled by this thread
-    uint4 k8[8], q8[8], v8[8];
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-        const int t = (tid >> 4) + it * 8;
-        k8[it] = q8[it] = v8[it] = make_uint4(0, 0, 0, 0);
-        if (t < n && sj * 8 < dhi) {
-            const int64_t off = (row0 + t) * d + h * dhi + sj * 8;
-            k8[it] = *reinterpret_cast<const uint4*>(k + off);
-            q8[it] = *reinterpret_cast<const uint4*>(q + off);
-            v8[it] = *reinterpret_cast<const uint4*>(v + off);
-        }
+    float al = 1.0f, be = 0.0f;
+    if (tid < n) {
+        al = alpha[(row0 + tid) * H + h];
+        be = beta[(row0 + tid) * H + h];
     }
     if (tid == 0) {
         *abort_flag = 0;
-        tc::mbar_init(&bar[0], 1);
-        tc::mbar_init(&bar[1], 1);
+        for (int i = 0; i < 4; ++i) tc::mbar_init(&bar[i], 1);
         tc::mbar_fence_init();
+        tc::mbar_expect_tx(&bar[0], NB * 16384);
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) {
+            tc::tma_load_3d(KQ_s + kb * 16384, &mapK, h * DH + kb * 64, t0, b, &bar[0]);
+            tc::tma_load_3d(KQ_s + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, t0, b, &bar[0]);
+        }
+        tc::mbar_expect_tx(&bar[3], NB * 8192);
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) tc::tma_load_3d(V_s + kb * 8192, &mapV, h * DH + kb * 64, t0, b, &bar[3]);
     }
-    if (warp == 0) tc::tmem_alloc(tmem_slot, 128);
+    if (warp == 7) tc::tmem_alloc(tmem_slot, DH);
     // g = cumsum(log alpha): warp scans over the 64 tokens
     float gx = 0.0f;
     if (tid < C) {
-        const bool live = tid < n;
-        be_s[tid] = live ? beta[(row0 + tid) * H + h] : 0.0f;
-        gx = live ? logf(alpha[(row0 + tid) * H + h]) : 0.0f;
+        be_s[tid] = be;
+        gx = tid < n ? logf(al) : 0.0f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float y = __shfl_up_sync(0xffffffffu, gx, o);
@@ -161,1117 +194,1117 @@ __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
     __syncthreads();
     tc::tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
-    if (tid < C) {
-        if (tid >= 32) gx += *wtot;
-        g_s[tid] = gx;
-        gam_s[tid] = expf(gx);
-    }
-    __syncthreads();
-    if (tid < C) eg_s[tid] = expf(g_s[C - 1] - g_s[tid]);
-    __syncthreads();
-
-    // ---- stage K, Q (K-major, swizzled), build [beta gam K | beta V], emit Qg, Kw and the backward's copies
-    {
-        const int box = sj >> 3, jc = sj & 7;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const int t = (tid >> 4) + it * 8;
-            *reinterpret_cast<uint4*>(KQ_s + box * 16384 + tc::sw128_off(t, jc)) = k8[it];
-            *reinterpret_cast<uint4*>(KQ_s + box * 16384 + tc::sw128_off(64 + t, jc)) = q8[it];
-            float kf[8], qf[8], vf[8], tmp[8];
-            tc::unpack8_bf16(k8[it], kf);
-            tc::unpack8_bf16(q8[it], qf);
-            tc::unpack8_bf16(v8[it], vf);
-            const float be = be_s[t], gm = gam_s[t], eg = eg_s[t];
-            const int64_t o64 = (tix * 64 + t) * DH + sj * 8;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) tmp[e] = be * gm * kf[e];
-            const uint4 bk = tc::pack8_bf16(tmp);
-            *reinterpret_cast<uint4*>(Bop_s + box * 8192 + tc::sw128_off(t, jc)) = bk;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) tmp[e] = be * vf[e];
-            *reinterpret_cast<uint4*>(Bop_s + (NB + box) * 8192 + tc::sw128_off(t, jc)) = tc::pack8_bf16(tmp);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) tmp[e] = gm * qf[e];
-            *reinterpret_cast<uint4*>(out.WQ + (tix * 128 + 64 + t) * DH + sj * 8) = tc::pack8_bf16(tmp);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) tmp[e] = eg * kf[e];
-            *reinterpret_cast<uint4*>(out.KW + o64) = tc::pack8_bf16(tmp);
-            if (out.BK) {
-                *reinterpret_cast<uint4*>(out.BK + o64) = bk;
-            }
-        }
-    }
-    if (out.GV && tid < C) {
-        out.GV[tix * 64 + tid] = g_s[tid];
-        out.BE[tix * 64 + tid] = be_s[tid];
-    }
-    tc::fence_proxy_async_smem();
-    __syncthreads();
-
-    // ---- MMA-A: [KK ; QK] = [K ; Q] K^T   (M128 N64 K128)
-    if (tid == 0) {
+    auto warp_wait = [&](int i) -> bool {
+        int got = 1;
+        if (lane == 0) got = tc::mbar_wait(&bar[i], 0, abort_flag, err_word, 200 + i) ? 1 : 0;
+        return __shfl_sync(0xffffffffu, got, 0) != 0;
+    };
+    // ---- MMA-A: [KK ; QK] = [K ; Q] K^T   (M128 N64 K = DH)
+    if (tid == 128 && tc::mbar_wait(&bar[0], 0, abort_flag, err_word, 200)) {
         constexpr uint32_t IDESC = tc::idesc_bf16_f32(128, 64, 0, 0);
         const uint32_t kq = tc::smem_u32(KQ_s);
 #pragma unroll
         for (int k16 = 0; k16 < DH / 16; ++k16) {
             const uint32_t off = (k16 >> 2) * 16384 + (k16 & 3) * 32;
-            tc::umma_bf16(tmem, tc::smem_desc_sw128(kq + off, 16, 1024), tc::smem_desc_sw128(kq + off, 16, 1024), IDESC,
-                          k16 > 0 ? 1u : 0u);
+            tc::umma_bf16(tmem, tc::smem_desc_sw128(kq + off, 16, 1024), tc::smem_desc_sw128(kq + off, 16, 1024), IDESC, k16 > 0 ? 1u : 0u);
         }
-        tc::umma_commit(&bar[0]);
+        tc::umma_commit(&bar[1]);
     }
-    // beta V in the lane-major layout, from the operand tile (consecutive threads, consecutive 16 bytes)
-    if (out.BV) {
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const int L = tid + it * PRE_THREADS;
-            const int row = (L >> 8) * 16 + (L & 15), c16 = ((L >> 7) & 1) * 8 + ((L >> 4) & 7);
-            *reinterpret_cast<uint4*>(out.BV + tix * (64 * DH) + L * 8) =
-                *reinterpret_cast<const uint4*>(Bop_s + (NB + (c16 >> 3)) * 8192 + tc::sw128_off(row, c16 & 7));
-        }
+    if (tid < C) {
+        if (tid >= 32) gx += *wtot;
+        g_s[tid] = gx;
+        bg_s[tid] = be * expf(gx);
+        out.GB[tix * 128 + tid] = gx;
+        out.GB[tix * 128 + 64 + tid] = be;
     }
-    int got = 1;
-    if (lane == 0) got = tc::mbar_wait(&bar[0], 0, abort_flag, err_word, 201) ? 1 : 0;
-    bool ok = __shfl_sync(0xffffffffu, got, 0) != 0;
+    __syncthreads();   // the per-token vectors
+    bool ok = warp_wait(1);
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
     tc::tcgen05_fence_after();
-    // ---- L = strictlower(beta_t Gam KK) (f32, threads 0-63); A = lower(Gam QK) (bf16, threads 64-127)
+    // ---- 32 columns per thread: L = strictlower(beta_t Gam KK) (f32, lanes 0-63); A = lower(Gam QK) (bf16, lanes 64-127)
     if (ok) {
+        const int t = 32 * (wq & 1) + lane;
+        const bool empty = cg > (wq & 1);         // columns 32-63 of rows 0-31
         uint32_t r[32];
-        const int t = tid & 63;
-        const float gt = g_s[t], bt = be_s[t];
+        float e[32];
+        if (!empty) {
+            tc::tmem_ld_32x32(tmem + ((uint32_t)(wq * 32) << 16) + cg * 32, r);
+            const float gt = g_s[t];
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            tc::tmem_ld_32x32(tmem + ((uint32_t)(warp * 32) << 16) + cc * 32, r);
+            for (int j4 = 0; j4 < 8; ++j4) {
+                const float4 g4 = *reinterpret_cast<const float4*>(g_s + cg * 32 + 4 * j4);
+                e[4 * j4] = __expf(gt - g4.x);
+                e[4 * j4 + 1] = __expf(gt - g4.y);
+                e[4 * j4 + 2] = __expf(gt - g4.z);
+                e[4 * j4 + 3] = __expf(gt - g4.w);
+            }
             tc::tmem_ld_wait();
-            if (tid < 64) {
+        }
+        if (wq < 2) {
+            const float bt = be_s[t];
+            if (!empty) {
 #pragma unroll
                 for (int j4 = 0; j4 < 8; ++j4) {
-                    float l[4];
+                    const int J = cg * 2 + (j4 >> 2);
+                    if (J <= (t >> 4)) {
+                        float l[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int i = cc * 32 + 4 * j4 + e;
-                        l[e] = i < t ? bt * __expf(gt - g_s[i]) * __uint_as_float(r[4 * j4 + e]) : 0.0f;
+                        for (int i = 0; i < 4; ++i) l[i] = cg * 32 + 4 * j4 + i < t ? bt * e[4 * j4 + i] * __uint_as_float(r[4 * j4 + i]) : 0.0f;
+                        *reinterpret_cast<float4*>(&Lf[tri(t >> 4, J) + (t & 15) * BLD + 4 * (j4 & 3)]) = make_float4(l[0], l[1], l[2], l[3]);
                     }
-                    *reinterpret_cast<float4*>(&Lf[t * LF_LD + cc * 32 + 4 * j4]) = make_float4(l[0], l[1], l[2], l[3]);
                 }
-                if (out.KKo) {
-                    float a[32];
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) a[j] = __uint_as_float(r[j]);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        *reinterpret_cast<uint4*>(out.KKo + tix * 4096 + lm_off64(t, cc * 4 + j)) = tc::pack8_bf16(a + 8 * j);
-                }
-            } else {
-                float a[32];
-                if (out.QKo) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) a[j] = __uint_as_float(r[j]);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        *reinterpret_cast<uint4*>(out.QKo + tix * 4096 + lm_off64(t, cc * 4 + j)) = tc::pack8_bf16(a + 8 * j);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int i = cc * 32 + j;
-                    a[j] = i <= t ? __expf(gt - g_s[i]) * __uint_as_float(r[j]) : 0.0f;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    *reinterpret_cast<uint4*>(out.AA + (tix * 64 + t) * 64 + cc * 32 + j * 8) = tc::pack8_bf16(a + 8 * j);
             }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) e[j] = !empty && cg * 32 + j <= t ? e[j] * __uint_as_float(r[j]) : 0.0f;
+            store32_bf16(out.AA + (tix * 64 + t) * 64 + cg * 32, e, true);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) e[j] -= __bfloat162float(__float2bfloat16(e[j]));
+            store32_bf16(out.AL + (tix * 64 + t) * 64 + cg * 32, e, true);
         }
     }
     tc::tcgen05_fence_before();
     __syncthreads();
 
-    // ---- X = (I + L)^-1 in f32, by 16 x 16 blocks: the four diagonal blocks by forward substitution (one
-    //      column per thread), then the blocks 1, 2 and 3 below the diagonal as X_IJ = -X_II (sum_K L_IK X_KJ)
+    // ---- X = (I + L)^-1 in f32. The four 16 x 16 diagonal blocks, one column per thread; then the block below the diagonal in each
+    //      half (1,0), (3,2); then the lower left quarter as two products over pairs of blocks
     if (tid < 64) {
         const int I = tid >> 4, jj = tid & 15;
-        const float* Lb = Lf + (I * 16) * LF_LD + I * 16;
+        const float* Lb = Lf + tri(I, I);
         float x[16];
 #pragma unroll
-        for (int t = 0; t < 16; ++t) x[t] = 0.0f;
+        for (int t = 0; t < 16; ++t) x[t] = t == jj ? 1.0f : 0.0f;
 #pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            float s = 0.0f;
+        for (int kb = 0; kb < 4; ++kb) {
+            float4 l[16];
 #pragma unroll
-            for (int g4 = 0; g4 < (t + 3) / 4; ++g4) {      // entries at and right of the diagonal are zero in L
-                const float4 l4 = *reinterpret_cast<const float4*>(Lb + t * LF_LD + 4 * g4);
-                s = fmaf(l4.x, x[4 * g4], s);
-                s = fmaf(l4.y, x[4 * g4 + 1], s);
-                s = fmaf(l4.z, x[4 * g4 + 2], s);
-                s = fmaf(l4.w, x[4 * g4 + 3], s);
-            }
-            x[t] = (t == jj ? 1.0f : 0.0f) - s;
+            for (int t = 4 * kb + 1; t < 16; ++t) l[t] = *reinterpret_cast<const float4*>(Lb + t * BLD + 4 * kb);
+#pragma unroll
+            for (int t = 4 * kb + 1; t < 16; ++t) x[t] = fmaf(-l[t].x, x[4 * kb], x[t]);
+#pragma unroll
+            for (int t = 4 * kb + 2; t < 16; ++t) x[t] = fmaf(-l[t].y, x[4 * kb + 1], x[t]);
+#pragma unroll
+            for (int t = 4 * kb + 3; t < 16; ++t) x[t] = fmaf(-l[t].z, x[4 * kb + 2], x[t]);
+#pragma unroll
+            for (int t = 4 * kb + 4; t < 16; ++t) x[t] = fmaf(-l[t].w, x[4 * kb + 3], x[t]);
         }
 #pragma unroll
-        for (int t = 0; t < 16; ++t) Xf[(I * 16 + t) * LF_LD + I * 16 + jj] = x[t];
+        for (int t = 0; t < 16; ++t) Xf[tri(I, I) + t * BLD + jj] = x[t];
     }
     __syncthreads();
-#pragma unroll
-    for (int dd = 1; dd < 4; ++dd) {
-        const int pieces = (4 - dd) * 64;           // 1 x 4 strips of the (4 - dd) blocks at distance dd
-        for (int p = tid; p < pieces; p += PRE_THREADS) {
-            const int bI = (p >> 6) + dd, bJ = p >> 6, r = (p >> 2) & 15, c4 = (p & 3) * 4;
+    {
+        const int r = (tid >> 2) & 15, c4 = (tid & 3) * 4;
+        if (tid < 128) {
+            const int I = 2 * (tid >> 6) + 1, J = I - 1;
             float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int kk = 0; kk < dd; ++kk)
-                strip16(Lf + (bI * 16 + r) * LF_LD + (bJ + kk) * 16, Xf + ((bJ + kk) * 16) * LF_LD + bJ * 16 + c4, LF_LD, acc);
-            *reinterpret_cast<float4*>(&Yf[((p >> 6) * 16 + r) * YF_LD + c4]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            strip16(Lf + tri(I, J) + r * BLD, Xf + tri(J, J) + c4, acc);
+            put4(&Yf[(tid >> 6) * BSZ + r * BLD + c4], acc, 1.0f);
         }
         __syncthreads();
-        for (int p = tid; p < pieces; p += PRE_THREADS) {
-            const int bI = (p >> 6) + dd, bJ = p >> 6, r = (p >> 2) & 15, c4 = (p & 3) * 4;
+        if (tid < 128) {
+            const int I = 2 * (tid >> 6) + 1, J = I - 1;
             float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            strip16(Xf + (bI * 16 + r) * LF_LD + bI * 16, Yf + ((p >> 6) * 16) * YF_LD + c4, YF_LD, acc);
-            *reinterpret_cast<float4*>(&Xf[(bI * 16 + r) * LF_LD + bJ * 16 + c4]) = make_float4(-acc[0], -acc[1], -acc[2], -acc[3]);
+            strip16(Xf + tri(I, I) + r * BLD, Yf + (tid >> 6) * BSZ + c4, acc);
+            put4(&Xf[tri(I, J) + r * BLD + c4], acc, -1.0f);
+        }
+        __syncthreads();
+        const int I = tid >> 7, J = (tid >> 6) & 1;   // block (2 + I, J) of the lower left quarter
+        {
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (J == 0) strip16(Lf + tri(2 + I, 0) + r * BLD, Xf + tri(0, 0) + c4, acc);
+            strip16(Lf + tri(2 + I, 1) + r * BLD, Xf + tri(1, J) + c4, acc);
+            put4(&Yf[(2 * I + J) * BSZ + r * BLD + c4], acc, 1.0f);
+        }
+        __syncthreads();
+        {
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            strip16(Xf + tri(2 + I, 2) + r * BLD, Yf + J * BSZ + c4, acc);
+            if (I == 1) strip16(Xf + tri(3, 3) + r * BLD, Yf + (2 + J) * BSZ + c4, acc);
+            put4(&Xf[tri(2 + I, J) + r * BLD + c4], acc, -1.0f);
         }
         __syncthreads();
     }
-    // ---- X -> bf16 operand tile (K-major) and, for the backward, T' = X - I row-major
+    // ---- (X - I) diag(beta gam), (X - I) diag(beta) -> bf16 operand tiles (K-major) and, for the backward, X - I row-major
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
+    for (int it = 0; it < 512 / PRE_THREADS; ++it) {
         const int idx = tid + it * PRE_THREADS, t = idx >> 3, jc = idx & 7;
-        float x8[8];
+        float x8[8], y8[8];
         if ((jc >> 1) <= (t >> 4)) {
-            const float4 a = *reinterpret_cast<const float4*>(&Xf[t * LF_LD + jc * 8]);
-            const float4 c = *reinterpret_cast<const float4*>(&Xf[t * LF_LD + jc * 8 + 4]);
+            const float* src = &Xf[tri(t >> 4, jc >> 1) + (t & 15) * BLD + (jc & 1) * 8];
+            const float4 a = *reinterpret_cast<const float4*>(src);
+            const float4 c = *reinterpret_cast<const float4*>(src + 4);
             x8[0] = a.x, x8[1] = a.y, x8[2] = a.z, x8[3] = a.w, x8[4] = c.x, x8[5] = c.y, x8[6] = c.z, x8[7] = c.w;
         } else {
 #pragma unroll
             for (int e = 0; e < 8; ++e) x8[e] = 0.0f;
         }
-        *reinterpret_cast<uint4*>(Tp_s + tc::sw128_off(t, jc)) = tc::pack8_bf16(x8);
-        if (out.TP) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (jc * 8 + e == t) x8[e] = 0.0f;
-            *reinterpret_cast<uint4*>(out.TP + (tix * 64 + t) * 64 + jc * 8) = tc::pack8_bf16(x8);
-        }
+        for (int e = 0; e < 8; ++e)
+            if (jc * 8 + e == t) x8[e] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y8[e] = x8[e] * bg_s[jc * 8 + e];
+        *reinterpret_cast<uint4*>(X1_s + tc::sw128_off(t, jc)) = tc::pack8_bf16(y8);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y8[e] = x8[e] * be_s[jc * 8 + e];
+        *reinterpret_cast<uint4*>(X2_s + tc::sw128_off(t, jc)) = tc::pack8_bf16(y8);
+        if (out.TP) *reinterpret_cast<uint4*>(out.TP + (tix * 64 + t) * 64 + jc * 8) = tc::pack8_bf16(x8);
     }
     tc::fence_proxy_async_smem();
     __syncthreads();
 
-    // ---- MMA-B: W^ = X (beta gam K) in lane half 0, Uv = X (beta V) in lane half 1   (2 x M64 N128 K64)
-    if (tid == 0 && ok) {
+    // ---- MMA-B: X1 K in lane half 0, X2 V in lane half 1   (2 x M64 N = DH K64)
+    if (tid == 0 && ok && tc::mbar_wait(&bar[3], 0, abort_flag, err_word, 203)) {
         constexpr uint32_t IDESC = tc::idesc_bf16_f32(64, DH, 0, 1);
-        const uint32_t ta = tc::smem_u32(Tp_s), bo = tc::smem_u32(Bop_s);
+        const uint32_t x1 = tc::smem_u32(X1_s), x2 = tc::smem_u32(X2_s), kb = tc::smem_u32(KQ_s), vb = tc::smem_u32(V_s);
         tc::tcgen05_fence_after();
 #pragma unroll
         for (int k16 = 0; k16 < C / 16; ++k16)
-            tc::umma_bf16(tmem, tc::smem_desc_sw128(ta + k16 * 32, 16, 1024), tc::smem_desc_sw128(bo + k16 * 2048, 8192, 1024),
-                          IDESC, k16 > 0 ? 1u : 0u);
+            tc::umma_bf16(tmem, tc::smem_desc_sw128(x1 + k16 * 32, 16, 1024), tc::smem_desc_sw128(kb + k16 * 2048, 16384, 1024), IDESC, k16 > 0 ? 1u : 0u);
 #pragma unroll
         for (int k16 = 0; k16 < C / 16; ++k16)
-            tc::umma_bf16(tmem + (16u << 16), tc::smem_desc_sw128(ta + k16 * 32, 16, 1024),
-                          tc::smem_desc_sw128(bo + NB * 8192 + k16 * 2048, 8192, 1024), IDESC, k16 > 0 ? 1u : 0u);
-        tc::umma_commit(&bar[1]);
+            tc::umma_bf16(tmem + (16u << 16), tc::smem_desc_sw128(x2 + k16 * 32, 16, 1024), tc::smem_desc_sw128(vb + k16 * 2048, 8192, 1024), IDESC,
+                          k16 > 0 ? 1u : 0u);
+        tc::umma_commit(&bar[2]);
     }
-    if (ok) {
-        got = 1;
-        if (lane == 0) got = tc::mbar_wait(&bar[1], 0, abort_flag, err_word, 202) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, got, 0) != 0;
-    }
+    if (ok) ok = warp_wait(2);
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
     tc::tcgen05_fence_after();
-    // rows to the staging area (the operand tiles are consumed): [W^ | Uv] 64 x 256 B each, chunks XOR-swizzled
+    // + the identity's rows; into the (consumed) operand tiles of K and V, and out by TMA
     if (ok) {
-        const int half = lane >> 4, row = 16 * warp + (lane & 15);
-        uint8_t* stg = Bop_s + half * 16384 + row * 256;
+        const int half = lane >> 4, row = 16 * wq + (lane & 15);
+        const float f = half == 0 ? bg_s[row] : be_s[row];
 #pragma unroll
-        for (int cc = 0; cc < DH / 32; ++cc) {
+        for (int cc = 0; cc < DH / 64; ++cc) {
             uint32_t r[32];
-            tc::tmem_ld_32x32(tmem + ((uint32_t)(warp * 32) << 16) + cc * 32, r);
+            tc::tmem_ld_32x32(tmem + ((uint32_t)(wq * 32) << 16) + cg * (DH / 2) + cc * 32, r);
             tc::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
+                const int c16 = cg * (DH / 16) + cc * 4 + j;
+                uint4* at = reinterpret_cast<uint4*>((half == 0 ? KQ_s + (c16 >> 3) * 16384 : V_s + (c16 >> 3) * 8192) + tc::sw128_off(row, c16 & 7));
                 float o8[8];
+                tc::unpack8_bf16(*at, o8);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) o8[e] = __uint_as_float(r[8 * j + e]);
-                *reinterpret_cast<uint4*>(stg + (((cc * 4 + j) ^ (row & 15)) << 4)) = tc::pack8_bf16(o8);
+                for (int e = 0; e < 8; ++e) o8[e] = fmaf(f, o8[e], __uint_as_float(r[8 * j + e]));
+                *at = tc::pack8_bf16(o8);
             }
         }
+        tc::fence_proxy_async_smem();
     }
-    __syncthreads();
-    if (ok) {
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const int idx = tid + it * PRE_THREADS, t = idx >> 4, c16 = idx & 15;
-            const uint32_t so = t * 256 + ((c16 ^ (t & 15)) << 4);
-            *reinterpret_cast<uint4*>(out.WQ + (tix * 128 + t) * DH + c16 * 8) = *reinterpret_cast<const uint4*>(Bop_s + so);
-            *reinterpret_cast<uint4*>(out.UV + (tix * 64 + t) * DH + c16 * 8) = *reinterpret_cast<const uint4*>(Bop_s + 16384 + so);
-        }
-        if (out.UVT) {
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int L = tid + it * PRE_THREADS;
-                const int row = (L >> 8) * 16 + (L & 15), c16 = ((L >> 7) & 1) * 8 + ((L >> 4) & 7);
-                *reinterpret_cast<uint4*>(out.UVT + tix * (64 * DH) + L * 8) =
-                    *reinterpret_cast<const uint4*>(Bop_s + 16384 + row * 256 + ((c16 ^ (row & 15)) << 4));
-            }
-        }
-    }
-    if (tid == 0) out.GC[tix] = gam_s[C - 1];
     tc::tcgen05_fence_before();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, 128);
+    if (tid == 0 && ok) {
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) {
+            tc::tma_store_2d(&mapWH, KQ_s + kb * 16384, kb * 64, (int)(tix * 64));
+            tc::tma_store_2d(&mapUV, V_s + kb * 8192, kb * 64, (int)(tix * 64));
+        }
+        tc::bulk_commit_group();
+        tc::bulk_wait_read();
+    }
+    if (warp == 7) tc::tmem_dealloc(tmem, DH);
+    if (*abort_flag) __nanosleep(20000);   // (a load that never arrived must not land in another CTA's shared memory)
 }
 
-// ------------------------------------------------------------------ chain kernel
-constexpr int CH_THREADS = 160;
-constexpr int STAGE_BYTES = NB * 16384 /*WQ*/ + NB * 8192 /*UV*/ + NB * 8192 /*KW*/ + 16384 /*[0;A]*/;
-constexpr int TX_BYTES = NB * 16384 + NB * 8192 + NB * 8192 + 8192;
-constexpr size_t CH_SMEM = 1024 + 2 * STAGE_BYTES + NB * DH * 128 /*S bf16*/ + NB * 8192 /*U bf16*/ + 128;
+// ------------------------------------------------------------------ forward chain
+// Threads: 4 warps per 32 columns of the state (warp w: TMEM lane quarter w & 3, columns 32 (w >> 2) ..), one that loads and issues the
+// products, one that stores operand tiles (its waits for their reading are off the serial path).
+// Quarters 0 and 1 hold the 64 rows of U, quarters 2 and 3 those of o; the state's DH rows are all four quarters (DH 128) or 0 and 1.
+template <int DH>
+struct ChainCfg {
+    static constexpr int NB = DH / 64, NG = DH / 32, COMPUTE = 128 * NG, THREADS = COMPUTE + 64;
+    static constexpr int S_WARPS = (DH == 128 ? 4 : 2) * NG, ROW_WARPS = 2 * NG;
+    static constexpr int S_BYTES = NB * DH * 128;
+    static constexpr int F_STAGE = NB * 32768 + 16384, F_K = NB * 16384, F_UV = NB * 24576, F_A = NB * 32768, F_AL = F_A + 8192;   // (W^, Q from 0)
+    static constexpr size_t F_SMEM = 1024 + 2 * F_STAGE + S_BYTES + 4 * 512 + 128;
+        static constexpr int B_STAGE = NB * 24576 + 24576, B_KQ = 0, B_DO = NB * 16384, B_A = NB * 24576, B_AL = B_A + 8192, B_TP = B_AL + 8192;
+    static constexpr int B_RS = DH == 128 ? B_AL : B_TP;   // beta gam dR, where X - I (and AL) were
+    static constexpr size_t B_SMEM = 1024 + 2 * B_STAGE + S_BYTES + (DH == 128 ? 16384 : 0) /*dU then dR; at 64 where A was*/ + 2 * 512 + 128;
+};
 
-template <typename TO>
-__global__ void __launch_bounds__(CH_THREADS, 1) delta_fwd_tc_kernel(
-    const __grid_constant__ CUtensorMap mapWQ, const __grid_constant__ CUtensorMap mapUV,
-    const __grid_constant__ CUtensorMap mapKW, const __grid_constant__ CUtensorMap mapAA,
-    const __grid_constant__ CUtensorMap mapS0, const float* __restrict__ GC,
-    int T, int H, int dhi, int n_chunks, TO* __restrict__ o, const float* s_init, float* s_final /* may be s_init */,
-    float* __restrict__ ckpt, __nv_bfloat16* __restrict__ s0b, int* err_word) {
+// What bounds it: at 128 chains the tiles of HBM (136 KB per chunk with a backward to follow, 88 without), at few chains the two
+// products and three register passes of a chunk.
+template <int DH>
+__global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delta_fwd_tc_kernel(
+    const __grid_constant__ CUtensorMap mapWH, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
+    const __grid_constant__ CUtensorMap mapUV, const __grid_constant__ CUtensorMap mapAA, const __grid_constant__ CUtensorMap mapAL,
+    const __grid_constant__ CUtensorMap mapS0, const __grid_constant__ CUtensorMap mapU, const float* __restrict__ GB, int T, int H, int n_chunks, __nv_bfloat16* __restrict__ o,
+    const float* s_init, float* s_final /* may be s_init */, int keep /* states and U go out */, int* err_word) {
+    using Cfg = ChainCfg<DH>;
+    constexpr int NB = Cfg::NB;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* stage0 = base;
-    uint8_t* S_s = base + 2 * STAGE_BYTES;       // NB n-boxes x (DH k-rows x 128 B)
-    uint8_t* U_s = S_s + NB * DH * 128;          // NB n-boxes x (64 k-rows x 128 B)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(U_s + NB * 8192);
-    uint64_t* full = bars;            // [2]
-    uint64_t* mma1_done = bars + 2;
-    uint64_t* u_ready = bars + 3;
-    uint64_t* mma2_done = bars + 4;
-    uint64_t* s_ready = bars + 5;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int chain = blockIdx.x;
-    const int b = chain / H, h = chain % H;
-    const int d = H * dhi;
-    const int64_t row0 = (int64_t)b * T;
-    const int64_t tile0 = (int64_t)chain * n_chunks;
-
-    if (tid == 0) {
-        *abort_flag = 0;
-        tc::mbar_init(&full[0], 1);
-        tc::mbar_init(&full[1], 1);
-        tc::mbar_init(mma1_done, 1);
-        tc::mbar_init(u_ready, 64);
-        tc::mbar_init(mma2_done, 1);
-        tc::mbar_init(s_ready, 128);
-        tc::mbar_fence_init();
-    }
-    if (warp == 4) tc::tmem_alloc(tmem_slot, 2 * DH);
-    // the zero halves of the two [0;A] operands
-    for (int i = tid; i < 2 * 8192 / 16; i += CH_THREADS) {
-        const int st = i / (8192 / 16), w = i % (8192 / 16);
-        *reinterpret_cast<uint4*>(stage0 + st * STAGE_BYTES + NB * 32768 + w * 16) = make_uint4(0, 0, 0, 0);
-    }
-    tc::fence_proxy_async_smem();
-    tc::tcgen05_fence_before();
-    __syncthreads();
-    tc::tcgen05_fence_after();
-    const uint32_t tmem_S = *tmem_slot, tmem_D = tmem_S + DH;
-
-    auto warp_wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
-        int got = 1;
-        if (lane == 0) got = tc::mbar_wait(bar, parity, abort_flag, err_word, code) ? 1 : 0;
-        return __shfl_sync(0xffffffffu, got, 0) != 0;
-    };
-
-    if (warp == 4) {
-        // ------------------------------------------------------------ TMA + MMA issuer (one thread)
-        if (lane == 0) {
-            auto load = [&](int c, int s) {
-                uint8_t* st = stage0 + s * STAGE_BYTES;
-                const int t = (int)(tile0 + c);
-                tc::mbar_expect_tx(&full[s], TX_BYTES);
-#pragma unroll
-                for (int kb = 0; kb < NB; ++kb) tc::tma_load_2d(st + kb * 16384, &mapWQ, kb * 64, t * 128, &full[s]);
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb) {
-                    tc::tma_load_2d(st + NB * 16384 + nb * 8192, &mapUV, nb * 64, t * 64, &full[s]);
-                    tc::tma_load_2d(st + NB * 24576 + nb * 8192, &mapKW, nb * 64, t * 64, &full[s]);
-                }
-                tc::tma_load_2d(st + NB * 32768 + 8192, &mapAA, 0, t * 64, &full[s]);
-            };
-            load(0, 0);
-            if (n_chunks > 1) load(1, 1);
-            constexpr uint32_t ID1 = tc::idesc_bf16_f32(128, DH, 0, 1);   // A K-major, B MN-major
-            constexpr uint32_t ID3 = tc::idesc_bf16_f32(128, DH, 1, 1);   // A MN-major, B MN-major
-            const uint32_t s_addr = tc::smem_u32(S_s), u_addr = tc::smem_u32(U_s);
-            for (int c = 0; c < n_chunks; ++c) {
-                const int s = c & 1;
-                const uint32_t st = tc::smem_u32(stage0 + s * STAGE_BYTES);
-                if (!tc::mbar_wait(&full[s], (c >> 1) & 1, abort_flag, err_word, 211)) break;
-                if (!tc::mbar_wait(s_ready, c & 1, abort_flag, err_word, 212)) break;
-                tc::tcgen05_fence_after();
-                if (s0b) {   // the state at the start of chunk c, bf16, straight from the operand tile: two 128 x 64 boxes
-                             // (head dim 64: the live 64 x 64 block, the first 8 KiB of the first box)
-                    tc::tma_store_2d(&mapS0, S_s, 0, (int)(tile0 + c) * dhi);
-                    if (dhi == DH) tc::tma_store_2d(&mapS0, S_s + DH * 128, 64, (int)(tile0 + c) * DH);
-                    tc::bulk_commit_group();
-                }
-                // D1 = [W^ ; Qg] S0
-#pragma unroll
-                for (int k16 = 0; k16 < DH / 16; ++k16)
-                    tc::umma_bf16(tmem_D, tc::smem_desc_sw128(st + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                                  tc::smem_desc_sw128(s_addr + k16 * 2048, DH * 128, 1024), ID1, k16 > 0 ? 1u : 0u);
-                tc::umma_commit(mma1_done);
-                if (!tc::mbar_wait(u_ready, c & 1, abort_flag, err_word, 213)) break;
-                tc::tcgen05_fence_after();
-                // D1 += [0 ; A] U      S += Kw^T U
-#pragma unroll
-                for (int k16 = 0; k16 < C / 16; ++k16)
-                    tc::umma_bf16(tmem_D, tc::smem_desc_sw128(st + NB * 32768 + k16 * 32, 16, 1024),
-                                  tc::smem_desc_sw128(u_addr + k16 * 2048, 8192, 1024), ID1, 1u);
-#pragma unroll
-                for (int k16 = 0; k16 < C / 16; ++k16)
-                    tc::umma_bf16(tmem_S, tc::smem_desc_sw128(st + NB * 24576 + k16 * 2048, 8192, 1024),
-                                  tc::smem_desc_sw128(u_addr + k16 * 2048, 8192, 1024), ID3, 1u);
-                if (s0b) tc::bulk_wait_read();   // the state store has read the operand tile: it may be rewritten after this commit
-                tc::umma_commit(mma2_done);
-                if (c + 2 < n_chunks) {
-                    if (!tc::mbar_wait(mma2_done, c & 1, abort_flag, err_word, 214)) break;
-                    load(c + 2, s);
-                }
-            }
-            if (s0b) tc::bulk_wait_all();   // stores have landed before the CTA exits
-        }
-    } else {
-        // ------------------------------------------------------------ compute threads: TMEM lane = tid
-        const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
-        float* ck = ckpt ? ckpt + tile0 * DH * DH : nullptr;
-        // initial state: checkpoint 0, bf16 operand copy, f32 state scaled by the first chunk's decay
-        {
-            const float g0 = GC[tile0];
-            const float* si = s_init && tid < dhi ? s_init + (int64_t)chain * dhi * dhi + (int64_t)tid * dhi : nullptr;
-#pragma unroll 1
-            for (int cc = 0; cc < DH / 32; ++cc) {
-                uint32_t r[32];
-                float f[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) f[j] = si && cc * 32 < dhi ? si[cc * 32 + j] : 0.0f;
-                if (ck) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        reinterpret_cast<float4*>(ck + (int64_t)tid * DH + cc * 32)[j] =
-                            make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int chunk16 = cc * 4 + j;   // 16-byte chunk index along the row (8 bf16 each)
-                    const uint4 pk = tc::pack8_bf16(f + 8 * j);
-                    *reinterpret_cast<uint4*>(S_s + (chunk16 >> 3) * (DH * 128) + tc::sw128_off(tid, chunk16 & 7)) = pk;
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(g0 * f[j]);
-                tc::tmem_st_32x32(tmem_S + lane_addr + cc * 32, r);
-            }
-            tc::tmem_st_wait();
-            tc::fence_proxy_async_smem();
-            tc::tcgen05_fence_before();
-            tc::mbar_arrive(s_ready);
-        }
-        for (int c = 0; c < n_chunks; ++c) {
-            const int s = c & 1;
-            uint8_t* st = stage0 + s * STAGE_BYTES;
-            if (!warp_wait(mma1_done, c & 1, 221)) break;
-            tc::tcgen05_fence_after();
-            if (warp < 2) {
-                // U = Uv - W^ S0  ->  bf16 operand (k rows = t, n cols = value index)
-                if (!warp_wait(&full[s], (c >> 1) & 1, 222)) break;   // TMA-written Uv visible to this thread
-                const int t = tid;
-#pragma unroll 1
-                for (int cc = 0; cc < DH / 32; ++cc) {
-                    uint32_t r[32];
-                    tc::tmem_ld_32x32(tmem_D + lane_addr + cc * 32, r);
-                    tc::tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int chunk16 = cc * 4 + j;
-                        const uint32_t off = (chunk16 >> 3) * 8192 + tc::sw128_off(t, chunk16 & 7);
-                        float uv[8], u8[8];
-                        tc::unpack8_bf16(*reinterpret_cast<const uint4*>(st + NB * 16384 + off), uv);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) u8[e] = uv[e] - __uint_as_float(r[8 * j + e]);
-                        *reinterpret_cast<uint4*>(U_s + off) = tc::pack8_bf16(u8);
-                    }
-                }
-                tc::fence_proxy_async_smem();
-                tc::tcgen05_fence_before();
-                tc::mbar_arrive(u_ready);
-            }
-            if (!warp_wait(mma2_done, c & 1, 223)) break;
-            tc::tcgen05_fence_after();
-            if (warp >= 2) {
-                // O rows (TMEM lanes 64-127 of D1)
-                const int t = tid - 64;
-                const bool live = c * C + t < T;
-                TO* orow = o + (row0 + c * C + (live ? t : 0)) * d + h * dhi;
-#pragma unroll 1
-                for (int cc = 0; cc < DH / 32; ++cc) {
-                    uint32_t r[32];
-                    tc::tmem_ld_32x32(tmem_D + lane_addr + cc * 32, r);
-                    tc::tmem_ld_wait();
-                    if (live && cc * 32 < dhi) {
-                        if (sizeof(TO) == 2) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                float f8[8];
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) f8[e] = __uint_as_float(r[8 * j + e]);
-                                reinterpret_cast<uint4*>(orow + cc * 32)[j] = tc::pack8_bf16(f8);
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                reinterpret_cast<float4*>(orow + cc * 32)[j] =
-                                    make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                                __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-                        }
-                    }
-                }
-            }
-            // new state: checkpoint / final state (f32), bf16 operand copy, pre-scale for the next chunk
-            const bool last = c + 1 == n_chunks;
-            const float gnext = last ? 1.0f : GC[tile0 + c + 1];
-            float* dst = last ? (s_final ? s_final + (int64_t)chain * dhi * dhi : nullptr)
-                              : (ck ? ck + (int64_t)(c + 1) * DH * DH : nullptr);   // (f32 checkpoints: head dim 128 only)
-#pragma unroll 1
-            for (int cc = 0; cc < DH / 32; ++cc) {
-                uint32_t r[32];
-                tc::tmem_ld_32x32(tmem_S + lane_addr + cc * 32, r);
-                tc::tmem_ld_wait();
-                float f[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]);
-                if (dst && tid < dhi && cc * 32 < dhi) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        reinterpret_cast<float4*>(dst + (int64_t)tid * dhi + cc * 32)[j] =
-                            make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-                }
-                if (!last) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int chunk16 = cc * 4 + j;
-                        const uint4 pk = tc::pack8_bf16(f + 8 * j);
-                        *reinterpret_cast<uint4*>(S_s + (chunk16 >> 3) * (DH * 128) + tc::sw128_off(tid, chunk16 & 7)) = pk;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gnext * f[j]);
-                    tc::tmem_st_32x32(tmem_S + lane_addr + cc * 32, r);
-                }
-            }
-            if (!last) {
-                tc::tmem_st_wait();
-                tc::fence_proxy_async_smem();
-                tc::tcgen05_fence_before();
-                tc::mbar_arrive(s_ready);
-            }
-        }
-    }
-    tc::tcgen05_fence_before();
-    __syncthreads();
-    if (*abort_flag) __nanosleep(20000);
-    if (warp == 4) tc::tmem_dealloc(tmem_S, 2 * DH);
-}
-
-// ------------------------------------------------------------------ backward chain kernel
-// One CTA (128 threads) per (sequence, head) walks the chunks in reverse with dS (f32) resident
-// in TMEM columns [0,128). Products with 64 token rows use M = 64 MMAs; two of them share a
-// column range by living in the two 16-lane halves of every 32-lane TMEM quarter (lane offset 0
-// and 16), so thread (warp w, lane l) sees row 16w + (l & 15) of the product in half (l >> 4).
-//
-//   G1  ACC_A.h0 = W^ S0               ACC_A.h1 = (beta gam K) S0  (= P2)
-//   G2  ACC_B.h1 = A^T dO + Kw dS      (= dU)
-//   G3  ACC_B.h1 += T'^T dU            (= dR)         G8  ACC_C.h1 = U dS^T (= dW)
-//   G4  ACC_C.h0 = [dR U^T | dO U^T]   (-> dL, dA)    G5  ACC_A.h0 = dO S0^T,  ACC_A.h1 = dR S0^T
-//   G6  ACC_B.h0 = (dA.Gam) K          ACC_B.h1 = M K + M^T K + (dA.Gam)^T Q
-//   G9  dS = gam_C dS + Qg^T dO - (beta gam K)^T dR
-// with U = Uv - W^ S0, R = beta V - P2, dV = beta dR, M = dL.Gam.beta, and
-//   dq = gam X + G6.h0,  dk = G6.h1 + eg dW - beta gam Y  (X, Y = the two halves of G5),
-// followed by the L2-norm backward, the gate gradients and the [dq|dk|dv] concat as in the f32
-// kernel (delta_bwd.cu).
-constexpr int NCQ = 4;                   // column groups per row: warp w and w + 4 k share TMEM lane quarter (w & 3)
-constexpr int BW_THREADS = 128 * NCQ;
-constexpr int CW = DH / NCQ;             // columns of a row handled by one thread
-constexpr int NCI = CW / 32;             // 32-column TMEM loads per thread and product
-constexpr int DW = C / NCQ;              // columns of the 64 x 64 dL / dA products per thread
-constexpr int NWARPS = BW_THREADS / 32;
-constexpr int R_WH = 0, R_BK = 16384, R_QG = 32768, R_KW = 49152, R_K = 65536, R_Q = 81920, R_DO = 98304,
-              R_A = 114688, R_TP = 122880, R_S0 = 131072, R_DS = 163840, R_DR = 196608, R_END = 212992;
-constexpr int R_U = R_WH, R_P = R_KW, R_DAG = R_A, R_M = R_TP, R_STG = R_S0;   // staging: S0 + dS regions (64 KiB)
-constexpr int BW_NVEC = 128 + 6 * NCQ * 64 + BW_THREADS + 128 + 64 + (BW_THREADS / 64) * 64;
-constexpr size_t BW_SMEM = 1024 + R_END + BW_NVEC * 4 + 256;
-constexpr int BW_TX_A = 32768 + 16384 * 2;        // S0, W^, beta gam K
-constexpr int BW_TX_B = 16384 * 2 + 8192;         // Kw, dO, A
-constexpr int BW_TX_C = 16384 * 3 + 8192;         // Qg, K, Q, T'
-
-// 128 * NCQ threads: warps w, w + 4, ... share TMEM lane quarter (w & 3) and split every row's 128
-// columns in NCQ groups (colhalf = w >> 2), so each thread handles CW columns of one row.
-__global__ void __launch_bounds__(BW_THREADS, 1) delta_bwd_tc_kernel(
-    const __grid_constant__ CUtensorMap mapWQ, const __grid_constant__ CUtensorMap map64x128,  // BK tiles
-    const __grid_constant__ CUtensorMap mapKW, const __grid_constant__ CUtensorMap mapKR,
-    const __grid_constant__ CUtensorMap mapQR, const __grid_constant__ CUtensorMap mapDO,
-    const __grid_constant__ CUtensorMap mapAA, const __grid_constant__ CUtensorMap mapTP,
-    const __grid_constant__ CUtensorMap mapS0, Tiles tl,
-    const float* __restrict__ alpha, const float* __restrict__ qnorm, const float* __restrict__ knorm, int T, int H, int dhi, int n_chunks,
-    float* __restrict__ d_qkv, float* __restrict__ d_gate, int* err_word) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    float* vec = reinterpret_cast<float*>(sm + R_END);
-    float* g_s = vec;              // cumulative log alpha
-    float* be_s = vec + 64;        // beta
-    float* v_rowp = vec + 128;                 // [NCQ][64] row sums of P per column group
-    float* v_rqs = v_rowp + NCQ * 64;          // [NCQ][64]
-    float* v_rkg = v_rqs + NCQ * 64;           // [NCQ][64]
-    float* v_rkw = v_rkg + NCQ * 64;           // [NCQ][64]
-    float* v_rdr = v_rkw + NCQ * 64;           // [NCQ][64]
-    float* v_dls = v_rdr + NCQ * 64;           // [NCQ][64]
-    float* v_red = v_dls + NCQ * 64;           // [BW_THREADS] partials of <S0, dS>
-    float* v_nrm = v_red + BW_THREADS;         // [128] |q| rows then |k| rows of the chunk
-    float* v_al = v_nrm + 128;                 // [64] alpha
-    float* v_colp4 = v_al + 64;                // [BW_THREADS / 64][64] partial column sums of P
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + R_END + BW_NVEC * 4);   // [0],[7],[8] TMA groups, [1..6] MMA groups
+    uint8_t* S_s = base + 2 * Cfg::F_STAGE;      // NB n-boxes x (DH k-rows x 128 B)
+    auto U_s = [&](int s) { return base + s * Cfg::F_STAGE + Cfg::F_UV; };   // U takes Uv's place: NB n-boxes x (64 k-rows x 128 B)
+    auto Ue_s = [&](int s) { return base + s * Cfg::F_STAGE; };              // eg U takes W^'s place: n-boxes 16 KiB apart
+    float* gb_s = reinterpret_cast<float*>(S_s + Cfg::S_BYTES);   // [4][128]: loaded with the stages, read two chunks longer
+    uint64_t* bars = reinterpret_cast<uint64_t*>(gb_s + 512);
+    uint64_t *full = bars, *mma1_done = bars + 2, *u_ready = bars + 3, *mma2_done = bars + 4, *s_ready = bars + 5, *mma3_done = bars + 6,
+             *o_done = bars + 7, *s_stored = bars + 8, *u_stored = bars + 9;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wq = warp & 3, colhalf = warp >> 2;
-    const int half = (lane >> 4) & 1, row = 16 * wq + (lane & 15);   // M=64 accumulator mapping
-    const int arow = 32 * wq + lane;                                 // M=128 accumulator (dS) mapping
     const int chain = blockIdx.x;
     const int b = chain / H, h = chain % H;
-    const int d = H * dhi;
-    const int64_t seq_row0 = (int64_t)b * T;
+    const int d = H * DH;
     const int64_t tile0 = (int64_t)chain * n_chunks;
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 9; ++i) tc::mbar_init(&bars[i], 1);
+        for (int i = 0; i < 10; ++i) {
+            const uint64_t* w = bars + i;
+            tc::mbar_init(&bars[i], w == u_ready || w == o_done ? Cfg::ROW_WARPS : w == s_ready ? Cfg::S_WARPS : 1);
+        }
         tc::mbar_fence_init();
     }
-    if (warp == 0) tc::tmem_alloc(tmem_slot, 512);
+    if (warp == Cfg::COMPUTE / 32) tc::tmem_alloc(tmem_slot, 4 * DH);
     tc::tcgen05_fence_before();
     __syncthreads();
     tc::tcgen05_fence_after();
-    const uint32_t tm = *tmem_slot;
-    const uint32_t ACC_S = tm, ACC_A = tm + 128, ACC_B = tm + 256, ACC_C = tm + 384;
-    const uint32_t H1 = 16u << 16;                         // lane offset of the second M=64 half
-    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
-    const int c0 = colhalf * NCI;                          // first 32-column chunk of this thread
+    const uint32_t tmem_S = *tmem_slot, tmem_D1 = tmem_S + DH /* two, in turn */, tmem_D2 = tmem_S + 3 * DH;
 
-    // dS = 0 (TMEM f32 and the bf16 operand copy)
-    {
-        uint32_t z[32];
+    if (warp == Cfg::COMPUTE / 32) {
+        // ------------------------------------------------------------ TMA loads + MMA issuer (one thread)
+        if (lane == 0) {
+            auto load = [&](int c, int s) {
+                uint8_t* st = base + s * Cfg::F_STAGE;
+                const int t = (int)(tile0 + c);
+                tc::mbar_expect_tx(&full[s], Cfg::F_STAGE + 512);
+                load_vec(gb_s + (c & 3) * 128, GB + (int64_t)t * 128, &full[s]);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) z[j] = 0u;
+                for (int kb = 0; kb < NB; ++kb) {
+                    tc::tma_load_2d(st + kb * 16384, &mapWH, kb * 64, t * 64, &full[s]);
+                    tc::tma_load_3d(st + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, c * C, b, &full[s]);
+                    tc::tma_load_2d(st + Cfg::F_UV + kb * 8192, &mapUV, kb * 64, t * 64, &full[s]);
+                    tc::tma_load_3d(st + Cfg::F_K + kb * 8192, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
+                }
+                tc::tma_load_2d(st + Cfg::F_A, &mapAA, 0, t * 64, &full[s]);
+                tc::tma_load_2d(st + Cfg::F_AL, &mapAL, 0, t * 64, &full[s]);
+            };
+            load(0, 0);
+            if (n_chunks > 1) load(1, 1);
+            constexpr uint32_t ID_KM = tc::idesc_bf16_f32(128, DH, 0, 1);   // A K-major, B MN-major
+            constexpr uint32_t ID_MM = tc::idesc_bf16_f32(128, DH, 1, 1);   // A MN-major, B MN-major
+            const uint32_t s_addr = tc::smem_u32(S_s);
+            for (int c = 0; c < n_chunks; ++c) {
+                const int s = c & 1;
+                const uint32_t st = tc::smem_u32(base + s * Cfg::F_STAGE);
+                if (!tc::mbar_wait(&full[s], (c >> 1) & 1, abort_flag, err_word, 211)) break;
+                if (!tc::mbar_wait(s_ready, c & 1, abort_flag, err_word, 212)) break;
+                tc::tcgen05_fence_after();
+                // D1 = [W^ ; Q] S
+                const uint32_t d1 = tmem_D1 + s * DH;
 #pragma unroll
-        for (int ci = 0; ci < NCI; ++ci) tc::tmem_st_32x32(ACC_S + lane_addr + (c0 + ci) * 32, z);
-        tc::tmem_st_wait();
-        for (int i = tid; i < 32768 / 16; i += BW_THREADS) *reinterpret_cast<uint4*>(sm + R_DS + i * 16) = make_uint4(0, 0, 0, 0);
-    }
-    // Head dim 64: a chunk-start state arrives as its live 64 x 64 block (rows 0-63 of the first column box); the rest of
-    // the S0 operand must read as zeros. The region doubles as staging, so it is cleared again after every chunk.
-    auto clear_s0_pad = [&] {
-        for (int i = tid; i < (32768 - 8192) / 16; i += BW_THREADS) *reinterpret_cast<uint4*>(sm + R_S0 + 8192 + i * 16) = make_uint4(0, 0, 0, 0);
-    };
-    if (dhi != DH) clear_s0_pad();
-
-    // Three groups in the order the chunk needs them: [0] S0, W^, beta gam K; [7] Kw, dO, A; [8] the rest.
-    auto issue_tma = [&](int c) {
-        const int t = (int)(tile0 + c);
-        const int grow = (int)(seq_row0 + (int64_t)c * C);
-        tc::mbar_expect_tx(&bars[0], dhi == DH ? BW_TX_A : BW_TX_A - 32768 + 8192);
-        // caller's tensors, head dim 64: the second column box starts past the last column and arrives as TMA's zero fill
-        const int xc[2] = {h * dhi, dhi == DH ? h * DH + 64 : H * dhi};
+                for (int k16 = 0; k16 < DH / 16; ++k16)
+                    tc::umma_bf16(d1, tc::smem_desc_sw128(st + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
+                                  tc::smem_desc_sw128(s_addr + k16 * 2048, DH * 128, 1024), ID_KM, k16 > 0 ? 1u : 0u);
+                tc::umma_commit(mma1_done);
+                if (!tc::mbar_wait(u_ready, c & 1, abort_flag, err_word, 213)) break;
+                tc::tcgen05_fence_after();
+                // S += K^T (eg U)   (head dim 64: rows 64-127 multiply what lies behind K and are not read)
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-            if (dhi == DH) tc::tma_load_2d(sm + R_S0 + kb * 16384, &mapS0, kb * 64, t * 128, &bars[0]);
-            else if (kb == 0) tc::tma_load_2d(sm + R_S0, &mapS0, 0, t * 64, &bars[0]);
-            tc::tma_load_2d(sm + R_WH + kb * 8192, &mapWQ, kb * 64, t * 128, &bars[0]);
-            tc::tma_load_2d(sm + R_BK + kb * 8192, &map64x128, kb * 64, t * 64, &bars[0]);
-        }
-        tc::mbar_expect_tx(&bars[7], BW_TX_B);
-        tc::tma_load_2d(sm + R_A, &mapAA, 0, t * 64, &bars[7]);
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_S, tc::smem_desc_sw128(st + Cfg::F_K + k16 * 2048, 8192, 1024),
+                                  tc::smem_desc_sw128(st + k16 * 2048, 16384, 1024), ID_MM, 1u);
+                tc::umma_commit(mma2_done);
+                // D2 = [.. ; A] U + [.. ; AL] U   (rows 0-63 multiply what lies in front and are not read)
+                if (c > 0 && !tc::mbar_wait(o_done, (c - 1) & 1, abort_flag, err_word, 214)) break;
+                tc::tcgen05_fence_after();
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-            tc::tma_load_2d(sm + R_DO + kb * 8192, &mapDO, xc[kb], grow, &bars[7]);
-            tc::tma_load_2d(sm + R_KW + kb * 8192, &mapKW, kb * 64, t * 64, &bars[7]);
-        }
-        tc::mbar_expect_tx(&bars[8], BW_TX_C);
-        tc::tma_load_2d(sm + R_TP, &mapTP, 0, t * 64, &bars[8]);
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_D2, tc::smem_desc_sw128(st + Cfg::F_A - 8192 + k16 * 32, 16, 1024),
+                                  tc::smem_desc_sw128(st + Cfg::F_UV + k16 * 2048, 8192, 1024), ID_KM, k16 > 0 ? 1u : 0u);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-            tc::tma_load_2d(sm + R_QG + kb * 8192, &mapWQ, kb * 64, t * 128 + 64, &bars[8]);
-            // K and Q straight from the caller's tensors (like dO): rows past the sequence end hold the next
-            // sequence's tokens (or TMA's zero fill past the tensor); every product that reads them multiplies by an
-            // exact zero there (beta = 0, U rows = 0, and dA rows masked below)
-            tc::tma_load_2d(sm + R_K + kb * 8192, &mapKR, xc[kb], grow, &bars[8]);
-            tc::tma_load_2d(sm + R_Q + kb * 8192, &mapQR, xc[kb], grow, &bars[8]);
-        }
-    };
-    auto wait_bar = [&](int i, uint32_t parity) {
-        if (lane == 0) tc::mbar_wait(&bars[i], parity, abort_flag, err_word, 300 + i);
-        __syncwarp();
-    };
-    // Shared-memory matrix descriptors (128-byte swizzle, version 1). The address field is (base + offset) >> 4
-    // with every offset a compile-time constant, so one add per descriptor remains at run time.
-    const uint32_t sb4 = tc::smem_u32(sm) >> 4;
-    auto desc = [&](uint32_t off, uint32_t lbo, uint32_t sbo) -> uint64_t {
-        const uint32_t lo = sb4 + ((off >> 4) + ((lbo >> 4) << 16));
-        const uint32_t hi = (sbo >> 4) | (1u << 14) | (2u << 29);
-        return ((uint64_t)hi << 32) | lo;
-    };
-    auto kmaj = [&](int reg, int k16) {       // K-major, 64-row tile, 8 KiB per 64-wide k box
-        return desc(reg + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024);
-    };
-    auto kmaj128 = [&](int reg, int k16) {    // K-major, 128-row tile (S0 / dS), 16 KiB per k box
-        return desc(reg + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024);
-    };
-    auto mnmaj = [&](int reg, int k16, int lbo) {   // MN-major: k rows, 64-wide mn boxes `lbo` bytes apart
-        return desc(reg + k16 * 2048, lbo, 1024);
-    };
-    // 64-row operand tile written by the threads: 16-byte chunk `chunk16` (0..15) of row r
-    auto tile64 = [&](int reg, int r, int chunk16) -> uint4* {
-        return reinterpret_cast<uint4*>(sm + reg + (chunk16 >> 3) * 8192 + tc::sw128_off(r, chunk16 & 7));
-    };
-    auto tile128 = [&](int reg, int r, int chunk16) -> uint4* {
-        return reinterpret_cast<uint4*>(sm + reg + (chunk16 >> 3) * 16384 + tc::sw128_off(r, chunk16 & 7));
-    };
-    constexpr uint32_t I64_KM = tc::idesc_bf16_f32(64, 128, 0, 1);
-    constexpr uint32_t I64_MM = tc::idesc_bf16_f32(64, 128, 1, 1);
-    constexpr uint32_t I64_KK = tc::idesc_bf16_f32(64, 128, 0, 0);
-    constexpr uint32_t I64_KK64 = tc::idesc_bf16_f32(64, 64, 0, 0);
-    constexpr uint32_t I128_MM = tc::idesc_bf16_f32(128, 128, 1, 1);
-    constexpr uint32_t I128_MM_NEG = I128_MM | (1u << 13);
-
-    // Small per-chunk inputs are fetched one chunk ahead, before that chunk's TMA traffic is queued:
-    // rows of Uv (half 0) / beta V (half 1), 64 columns each, and the per-token scalars.
-    uint4 pre[CW / 8];
-    float nx0 = 0.0f, nx1 = 0.0f;
-    auto fetch_small = [&](int c) {
-        const int64_t tix = tile0 + c;
-        const int t0 = c * C;
-        const int n = T - t0 < C ? T - t0 : C;
-        const int64_t grow = seq_row0 + t0;
-        const __nv_bfloat16* src = (half == 0 ? tl.UVT : tl.BV) + tix * (64 * DH) + lm_off128(row, colhalf * (CW / 8));
-#pragma unroll
-        for (int j = 0; j < CW / 8; ++j) pre[j] = *reinterpret_cast<const uint4*>(src + j * 128);
-        if (tid < 64) {
-            nx0 = tl.GV[tix * 64 + tid];
-            nx1 = tl.BE[tix * 64 + tid];
-        } else if (tid < 128) {
-            const int t = min(tid - 64, n - 1);          // unconditional loads: nothing waits on them here
-            nx0 = alpha[(grow + t) * H + h];
-        } else if (tid < 256) {
-            const int t = min(tid & 63, n - 1);
-            nx0 = (tid < 192 ? qnorm : knorm)[(grow + t) * H + h];
-        }
-    };
-    fetch_small(n_chunks - 1);
-    if (tid == 0) issue_tma(n_chunks - 1);
-    // A wait that gives up raises *abort_flag; later waits then return at once, the iteration runs to its
-    // end on whatever data it has (every block barrier is still reached by every thread) and the loop
-    // exits at the block-uniform check below. The host sees the error word.
-    for (int c = n_chunks - 1, it = 0; c >= 0; --c, ++it) {
-        const uint32_t par = it & 1;
-        const int t0 = c * C;
-        const int n = T - t0 < C ? T - t0 : C;
-        const int64_t tix = tile0 + c;
-        const int64_t grow = seq_row0 + t0;
-        // ---- A. per-token scalars of the chunk (fetched during the previous chunk)
-        if (tid < 64) {
-            g_s[tid] = nx0;
-            be_s[tid] = nx1;
-        } else if (tid < 128) {
-            v_al[tid - 64] = nx0;
-        } else if (tid < 256) {
-            v_nrm[tid - 128] = nx0;
-        }
-        tc::fence_proxy_async_smem();   // the dS operand copy written at the end of the previous chunk
-        tc::tcgen05_fence_before();
-        __syncthreads();
-        wait_bar(0, par);
-        if (tid == 0) {
-            tc::tcgen05_fence_after();
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_A, kmaj(R_WH, k16), mnmaj(R_S0, k16, 16384), I64_KM, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_A + H1, kmaj(R_BK, k16), mnmaj(R_S0, k16, 16384), I64_KM, k16 > 0);
-            tc::umma_commit(&bars[1]);
-        }
-        wait_bar(7, par);
-        if (tid == 0) {
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16) tc::umma_bf16(ACC_B + H1, mnmaj(R_A, k16, 8192), mnmaj(R_DO, k16, 8192), I64_MM, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_B + H1, kmaj(R_KW, k16), mnmaj(R_DS, k16, 16384), I64_KM, 1u);
-            tc::umma_commit(&bars[2]);
-        }
-        const float g_row = g_s[row], g_last = g_s[C - 1];
-        const float gam_row = __expf(g_row), eg_row = __expf(g_last - g_row), be_row = be_s[row];
-        const bool live = row < n;
-        // ---- B. U = Uv - W^ S0 (half 0);  dU -> bf16 (half 1)
-        wait_bar(1, par);
-        tc::tcgen05_fence_after();
-#pragma unroll
-        for (int ci = 0; ci < NCI; ++ci) {
-            uint32_t r[32];
-            tc::tmem_ld_32x32(ACC_A + lane_addr + (c0 + ci) * 32, r);
-            tc::tmem_ld_wait();
-            if (half == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float x8[8], u8[8];
-                    tc::unpack8_bf16(pre[ci * 4 + j], x8);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) u8[e] = x8[e] - __uint_as_float(r[8 * j + e]);
-                    *tile64(R_U, row, (c0 + ci) * 4 + j) = tc::pack8_bf16(u8);
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_D2, tc::smem_desc_sw128(st + Cfg::F_A + k16 * 32, 16, 1024),
+                                  tc::smem_desc_sw128(st + Cfg::F_UV + k16 * 2048, 8192, 1024), ID_KM, 1u);
+                tc::umma_commit(mma3_done);
+                if (c + 2 < n_chunks) {
+                    if (!tc::mbar_wait(mma3_done, c & 1, abort_flag, err_word, 215)) break;
+                    if (keep && !tc::mbar_wait(u_stored, c & 1, abort_flag, err_word, 216)) break;   // (U lies in the stage)
+                    load(c + 2, s);
                 }
             }
         }
-        wait_bar(2, par);
-        tc::tcgen05_fence_after();
+    } else if (warp > Cfg::COMPUTE / 32) {
+        // ------------------------------------------------------------ state and U out, straight from the operand tiles (one thread)
+        if (lane == 0 && keep) {
+            for (int c = 0; c < n_chunks; ++c) {
+                if (!tc::mbar_wait(s_ready, c & 1, abort_flag, err_word, 217)) break;
 #pragma unroll
-        for (int ci = 0; ci < NCI; ++ci) {
-            uint32_t r[32];
-            tc::tmem_ld_32x32(ACC_B + lane_addr + (c0 + ci) * 32, r);
-            tc::tmem_ld_wait();
-            if (half == 1) {
+                for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapS0, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
+                tc::bulk_commit_group();
+                if (!tc::mbar_wait(u_ready, c & 1, abort_flag, err_word, 218)) break;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float f8[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) f8[e] = __uint_as_float(r[8 * j + e]);
-                    *tile64(R_DR, row, (c0 + ci) * 4 + j) = tc::pack8_bf16(f8);
-                }
+                for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapU, U_s(c & 1) + nb * 8192, nb * 64, (int)(tile0 + c) * 64);
+                tc::bulk_commit_group();
+                tc::bulk_wait_read_but_one();
+                tc::mbar_arrive(s_stored);
+                tc::bulk_wait_read();
+                tc::mbar_arrive(u_stored);
             }
+            tc::bulk_wait_read();   // before the CTA's shared memory goes
         }
-        tc::fence_proxy_async_smem();
-        tc::tcgen05_fence_before();
-        wait_bar(8, par);
-        __syncthreads();
-        if (tid == 0) {
+    } else {
+        const int wq = warp & 3, cg = warp >> 2, arow = 32 * wq + lane, row = arow & 63;
+        const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+        const int col = cg * 32;
+        const bool s_warp = DH == 128 || wq < 2;
+        const bool w32 = (reinterpret_cast<uintptr_t>(o) & 31) == 0;
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+            int got = 1;
+            if (lane == 0) got = tc::mbar_wait(bar, parity, abort_flag, err_word, code) ? 1 : 0;
+            got = __shfl_sync(0xffffffffu, got, 0);
             tc::tcgen05_fence_after();
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16) tc::umma_bf16(ACC_B + H1, mnmaj(R_TP, k16, 8192), mnmaj(R_DR, k16, 8192), I64_MM, 1u);
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_C + H1, kmaj(R_U, k16), kmaj128(R_DS, k16), I64_KK, k16 > 0);
-            tc::umma_commit(&bars[3]);
-        }
-        // rows of K K^T and Q K^T (32 columns each) for the dL / dA phase, fetched ahead
-        uint4 pkk[DW / 8], pqk[DW / 8];
-        if (half == 0) {
-            const __nv_bfloat16* kk = tl.KKo + tix * 4096 + lm_off64(row, colhalf * (DW / 8));
-            const __nv_bfloat16* qk = tl.QKo + tix * 4096 + lm_off64(row, colhalf * (DW / 8));
+            return got != 0;
+        };
+        auto arrive = [&](uint64_t* bar) {   // one arrival per warp, after every lane's accesses
+            tc::fence_proxy_async_smem();
+            tc::tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bar);
+        };
+        bool ok = warp_wait(&full[0], 0, 220);
+        if (s_warp && ok) {   // initial state: bf16 operand copy, and f32 scaled by the first chunk's decay
+            const float g0 = expf(gb_s[C - 1]);
+            const float* si = s_init ? s_init + ((int64_t)chain * DH + arow) * DH + col : nullptr;
+            uint32_t r[32];
+            float f[32];
 #pragma unroll
-            for (int j = 0; j < DW / 8; ++j) {
-                pkk[j] = *reinterpret_cast<const uint4*>(kk + j * 128);
-                pqk[j] = *reinterpret_cast<const uint4*>(qk + j * 128);
+            for (int j = 0; j < 32; ++j) f[j] = si ? si[j] : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int c16 = cg * 4 + j;
+                *reinterpret_cast<uint4*>(S_s + (c16 >> 3) * (DH * 128) + tc::sw128_off(arow, c16 & 7)) = tc::pack8_bf16(f + 8 * j);
             }
-        }
-        // ---- C. dR: dV out, R = beta V - P2, r_dr, r_kg, bf16 dR tile (half 1)
-        wait_bar(3, par);
-        tc::tcgen05_fence_after();
-        {
-            float r_dr = 0.0f, r_kg = 0.0f;
 #pragma unroll
-            for (int ci = 0; ci < NCI; ++ci) {
-                uint32_t r[32], p2[32];
-                tc::tmem_ld_32x32(ACC_B + lane_addr + (c0 + ci) * 32, r);
-                tc::tmem_ld_32x32(ACC_A + lane_addr + (c0 + ci) * 32, p2);
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(g0 * f[j]);
+            tc::tmem_st_32x32(tmem_S + lane_addr + col, r);
+            tc::tmem_st_wait();
+            arrive(s_ready);
+        }
+        for (int c = 0; ok && c < n_chunks; ++c) {   // (entered with the chunk's tiles in their stage)
+            const int s = c & 1;
+            const bool last = c + 1 == n_chunks;
+            const float g_row = gb_s[(c & 3) * 128 + row], g_last = gb_s[(c & 3) * 128 + C - 1];
+            uint32_t r[32];
+            if (wq < 2) {
+                // U = Uv - W^ S  ->  bf16 operands U and eg U (k rows = tokens, n = value columns)
+                const float eg = expf(g_last - g_row);
+                if (!warp_wait(mma1_done, c & 1, 222)) break;
+                tc::tmem_ld_32x32(tmem_D1 + s * DH + lane_addr + col, r);
                 tc::tmem_ld_wait();
-                if (half == 1) {
-                    float4* dvs = reinterpret_cast<float4*>(sm + R_DS) + row * 32;   // dV rows staged in the free dS region
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int c16 = cg * 4 + j;
+                    const uint32_t off = tc::sw128_off(row, c16 & 7);
+                    uint4* at = reinterpret_cast<uint4*>(U_s(s) + (c16 >> 3) * 8192 + off);
+                    float uv[8], u8[8];
+                    tc::unpack8_bf16(*at, uv);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) u8[e] = uv[e] - __uint_as_float(r[8 * j + e]);
+                    *at = tc::pack8_bf16(u8);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) u8[e] *= eg;
+                    *reinterpret_cast<uint4*>(Ue_s(s) + (c16 >> 3) * 16384 + off) = tc::pack8_bf16(u8);
+                }
+                arrive(u_ready);
+            }
+            const float gam = expf(g_row);
+            if (!last && !warp_wait(&full[s ^ 1], ((c + 1) >> 1) & 1, 223)) break;
+            if (s_warp) {
+                // new state: final state (f32), or bf16 operand copy and pre-scale for the next chunk
+                const float gnext = expf(gb_s[((c + 1) & 3) * 128 + C - 1]);
+                if (keep && !warp_wait(s_stored, c & 1, 224)) break;
+                if (!warp_wait(mma2_done, c & 1, 225)) break;
+                tc::tmem_ld_32x32(tmem_S + lane_addr + col, r);
+                tc::tmem_ld_wait();
+                float f[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]);
+                if (last) {
+                    if (s_final) store32(s_final + ((int64_t)chain * DH + arow) * DH + col, f, false);
+                } else {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        float x8[8], f8[8];
-                        tc::unpack8_bf16(pre[ci * 4 + j], x8);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const float dr = __uint_as_float(r[8 * j + e]), pp = __uint_as_float(p2[8 * j + e]);
-                            f8[e] = dr;
-                            r_dr = fmaf(dr, x8[e] - pp, r_dr);
-                            r_kg = fmaf(-dr, pp, r_kg);
-                        }
-                        {
-                            const int f4 = ((c0 + ci) * 4 + j) * 2, swz = row & 31;
-                            dvs[f4 ^ swz] = make_float4(be_row * f8[0], be_row * f8[1], be_row * f8[2], be_row * f8[3]);
-                            dvs[(f4 + 1) ^ swz] = make_float4(be_row * f8[4], be_row * f8[5], be_row * f8[6], be_row * f8[7]);
-                        }
-                        *tile64(R_DR, row, (c0 + ci) * 4 + j) = tc::pack8_bf16(f8);
+                        const int c16 = cg * 4 + j;
+                        *reinterpret_cast<uint4*>(S_s + (c16 >> 3) * (DH * 128) + tc::sw128_off(arow, c16 & 7)) = tc::pack8_bf16(f + 8 * j);
                     }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gnext * f[j]);
+                    tc::tmem_st_32x32(tmem_S + lane_addr + col, r);
+                    tc::tmem_st_wait();
+                    arrive(s_ready);
                 }
             }
-            if (half == 1) {
-                v_rdr[colhalf * 64 + row] = r_dr;
-                v_rkg[colhalf * 64 + row] = r_kg;
-            }
-        }
-        tc::fence_proxy_async_smem();
-        tc::tcgen05_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc::tcgen05_fence_after();
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_C, kmaj(R_DR, k16), kmaj(R_U, k16), I64_KK64, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_C + 64, kmaj(R_DO, k16), kmaj(R_U, k16), I64_KK64, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_A, kmaj(R_DO, k16), kmaj128(R_S0, k16), I64_KK, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 8; ++k16) tc::umma_bf16(ACC_A + H1, kmaj(R_DR, k16), kmaj128(R_S0, k16), I64_KK, k16 > 0);
-            tc::umma_commit(&bars[4]);
-        }
-        // ---- D. while G4/G5 run: dV rows out (8 lanes per row, coalesced), scale dS by gam_C, <S0, dS>
-#pragma unroll
-        for (int itv = 0; itv < 64 / (BW_THREADS / 8); ++itv) {
-            const int r_ = itv * (BW_THREADS / 8) + (tid >> 3), l8 = tid & 7;
-            if (r_ < n) {
-                float* dv = d_qkv + (grow + r_) * 3 * d + 2 * d + h * dhi;
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if ((l8 + 8 * i) * 4 < dhi)
-                        reinterpret_cast<float4*>(dv)[l8 + 8 * i] = reinterpret_cast<const float4*>(sm + R_DS)[r_ * 32 + ((l8 + 8 * i) ^ (r_ & 31))];
-            }
-        }
-        {
-            const float gC = __expf(g_last);
-            float part = 0.0f;
-#pragma unroll
-            for (int ci = 0; ci < NCI; ++ci) {
-                uint32_t r[32];
-                tc::tmem_ld_32x32(ACC_S + lane_addr + (c0 + ci) * 32, r);
+            if (wq >= 2) {
+                // o = gam (Q S) + A U: TMEM lanes 64-127
+                if (!warp_wait(mma3_done, c & 1, 226)) break;
+                uint32_t q[32];
+                tc::tmem_ld_32x32(tmem_D1 + s * DH + lane_addr + col, q);
+                tc::tmem_ld_32x32(tmem_D2 + lane_addr + col, r);
                 tc::tmem_ld_wait();
+                tc::tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(o_done);
+                if (c * C + row < T) {
+                    float f[32];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float s8[8];
-                    tc::unpack8_bf16(*tile128(R_S0, arow, (c0 + ci) * 4 + j), s8);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) part = fmaf(s8[e], __uint_as_float(r[8 * j + e]), part);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gC * __uint_as_float(r[j]));
-                tc::tmem_st_32x32(ACC_S + lane_addr + (c0 + ci) * 32, r);
-            }
-            tc::tmem_st_wait();
-            v_red[tid] = part;
-        }
-        wait_bar(4, par);
-        tc::tcgen05_fence_after();
-        // dL / dA rows (half 0; this thread's DW columns): M tile, dA.Gam tile, P row, dbeta
-        {
-            float rowp = 0.0f, dls = 0.0f;
-            uint32_t rl[DW], ra[DW];
-            tc::tmem_ld_cols<DW>(ACC_C + lane_addr + colhalf * DW, rl);
-            tc::tmem_ld_cols<DW>(ACC_C + lane_addr + 64 + colhalf * DW, ra);
-            tc::tmem_ld_wait();
-            if (half == 0) {
-#pragma unroll
-                for (int j = 0; j < DW / 8; ++j) {
-                    float kk8[8], qk8[8], m8[8], a8[8];
-                    tc::unpack8_bf16(pkk[j], kk8);
-                    tc::unpack8_bf16(pqk[j], qk8);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int i = colhalf * DW + 8 * j + e;
-                        const float gm = i <= row ? __expf(g_row - g_s[i]) : 0.0f;
-                        const float dlg = i < row ? -__uint_as_float(rl[8 * j + e]) * gm : 0.0f;   // dL.Gam
-                        const float dag = live ? __uint_as_float(ra[8 * j + e]) * gm : 0.0f;       // dA.Gam (dO rows past the end are not ours)
-                        dls = fmaf(dlg, kk8[e], dls);
-                        m8[e] = dlg * be_row;
-                        a8[e] = dag;
-                        const float pv = dag * qk8[e] + m8[e] * kk8[e];
-                        rowp += pv;
-                        reinterpret_cast<float*>(sm + R_P)[row * 64 + ((i + row) & 63)] = pv;
-                    }
-                    const int chunk16 = colhalf * (DW / 8) + j;
-                    *reinterpret_cast<uint4*>(sm + R_M + tc::sw128_off(row, chunk16)) = tc::pack8_bf16(m8);
-                    *reinterpret_cast<uint4*>(sm + R_DAG + tc::sw128_off(row, chunk16)) = tc::pack8_bf16(a8);
-                }
-                v_rowp[colhalf * 64 + row] = rowp;
-                v_dls[colhalf * 64 + row] = dls;
-            }
-        }
-        tc::fence_proxy_async_smem();
-        tc::tcgen05_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc::tcgen05_fence_after();
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16)
-                tc::umma_bf16(ACC_B, desc(R_DAG + k16 * 32, 16, 1024), mnmaj(R_K, k16, 8192), I64_KM, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16)
-                tc::umma_bf16(ACC_B + H1, desc(R_M + k16 * 32, 16, 1024), mnmaj(R_K, k16, 8192), I64_KM, k16 > 0);
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16) tc::umma_bf16(ACC_B + H1, mnmaj(R_M, k16, 8192), mnmaj(R_K, k16, 8192), I64_MM, 1u);
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16) tc::umma_bf16(ACC_B + H1, mnmaj(R_DAG, k16, 8192), mnmaj(R_Q, k16, 8192), I64_MM, 1u);
-            tc::umma_commit(&bars[5]);
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16) tc::umma_bf16(ACC_S, mnmaj(R_QG, k16, 8192), mnmaj(R_DO, k16, 8192), I128_MM, 1u);
-            _Pragma("unroll") for (int k16 = 0; k16 < 4; ++k16) tc::umma_bf16(ACC_S, mnmaj(R_BK, k16, 8192), mnmaj(R_DR, k16, 8192), I128_MM_NEG, 1u);
-            tc::umma_commit(&bars[6]);
-        }
-        // column sums of P while G6 runs: BW_THREADS / 64 threads per column
-        {
-            constexpr int RPP = 64 / (BW_THREADS / 64);   // rows per partial sum
-            const int col = tid & 63, part = tid >> 6;
-            float cs = 0.0f;
-            const float* P = reinterpret_cast<const float*>(sm + R_P);
-#pragma unroll
-            for (int t = part * RPP; t < part * RPP + RPP; ++t) cs += P[t * 64 + ((col + t) & 63)];
-            v_colp4[part * 64 + col] = cs;
-        }
-        // ---- E. dq rows (half 0) and dk rows (half 1) into the f32 staging area (S0 + dS regions are free)
-        wait_bar(5, par);
-        tc::tcgen05_fence_after();
-        {
-            const int srow = half * 64 + row;
-            float4* stg = reinterpret_cast<float4*>(sm + R_STG) + srow * 32;
-            const int swz = (row + 16 * half) & 31;
-            float rr = 0.0f;
-#pragma unroll
-            for (int pc = 0; pc < CW / 16; ++pc) {   // 16 columns at a time keeps the three accumulators in 48 registers
-                uint32_t xa[16], xb[16], xc[16];
-                const uint32_t col = (uint32_t)(colhalf * CW + pc * 16);
-                tc::tmem_ld_cols<16>(ACC_A + lane_addr + col, xa);    // X (h0) | Y (h1)
-                tc::tmem_ld_cols<16>(ACC_B + lane_addr + col, xb);    // G6
-                tc::tmem_ld_cols<16>(ACC_C + lane_addr + col, xc);    // (h0: dL|dA) | dW (h1)
-                tc::tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int chunk16 = colhalf * (CW / 8) + pc * 2 + j;
-                    float z8[8], g8[8];
-                    tc::unpack8_bf16(*tile64(half == 0 ? R_QG : R_K, row, chunk16), z8);   // Qg_t | k_t
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float A_ = __uint_as_float(xa[8 * j + e]), B_ = __uint_as_float(xb[8 * j + e]),
-                                    C_ = __uint_as_float(xc[8 * j + e]);
-                        if (half == 0) {
-                            g8[e] = fmaf(gam_row, A_, B_);
-                            rr = fmaf(z8[e], A_, rr);                    // Qg_t . X_t
-                        } else {
-                            g8[e] = B_ + eg_row * C_ - be_row * gam_row * A_;
-                            rr = fmaf(eg_row * z8[e], C_, rr);           // eg k_t . dW_t
-                        }
-                    }
-                    stg[(2 * chunk16) ^ swz] = make_float4(g8[0], g8[1], g8[2], g8[3]);
-                    stg[(2 * chunk16 + 1) ^ swz] = make_float4(g8[4], g8[5], g8[6], g8[7]);
-                }
-            }
-            (half == 0 ? v_rqs : v_rkw)[colhalf * 64 + row] = rr;
-        }
-        __syncthreads();
-        if (c > 0) fetch_small(c - 1);
-        // L2-norm backward and store: 8 lanes per staged row (4 float4 each), 4 rows per warp at a time
-        {
-            constexpr int RPW = 128 / NWARPS;            // staged rows per warp (64 dq rows, then 64 dk rows)
-            const int l8 = lane & 7, hh = (warp * RPW) >> 6;
-            const int ytile = hh == 0 ? R_Q : R_K;
-#pragma unroll
-            for (int itn = 0; itn < RPW / 4; ++itn) {
-                const int srow = warp * RPW + itn * 4 + (lane >> 3), r_ = srow & 63;
-                const int swz = (r_ + 16 * hh) & 31;
-                float4 g4[4];
-                float y[4][4];
-                float dot = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int f4 = l8 + 8 * i;
-                    g4[i] = reinterpret_cast<const float4*>(sm + R_STG)[srow * 32 + (f4 ^ swz)];
-                    const uint2 yraw = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(tile64(ytile, r_, f4 >> 1)) + (f4 & 1) * 8);
-                    const __nv_bfloat162 y01 = *reinterpret_cast<const __nv_bfloat162*>(&yraw.x), y23 = *reinterpret_cast<const __nv_bfloat162*>(&yraw.y);
-                    y[i][0] = __low2float(y01), y[i][1] = __high2float(y01), y[i][2] = __low2float(y23), y[i][3] = __high2float(y23);
-                    dot += y[i][0] * g4[i].x + y[i][1] * g4[i].y + y[i][2] * g4[i].z + y[i][3] * g4[i].w;
-                }
-                dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-                dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-                dot += __shfl_xor_sync(0xffffffffu, dot, 4);
-                if (r_ < n) {
-                    const float inv = 1.0f / v_nrm[srow];
-                    float* dst = d_qkv + (grow + r_) * 3 * d + (hh == 0 ? 0 : d) + h * dhi;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if ((l8 + 8 * i) * 4 < dhi)
-                            reinterpret_cast<float4*>(dst)[l8 + 8 * i] = make_float4((g4[i].x - y[i][0] * dot) * inv, (g4[i].y - y[i][1] * dot) * inv,
-                                                                                  (g4[i].z - y[i][2] * dot) * inv, (g4[i].w - y[i][3] * dot) * inv);
+                    for (int j = 0; j < 32; ++j) f[j] = fmaf(gam, __uint_as_float(q[j]), __uint_as_float(r[j]));
+                    store32_bf16(o + ((int64_t)b * T + c * C + row) * d + h * DH + col, f, w32);
                 }
             }
         }
-        // gates (warp 0): dg, reverse cumulative sum, sigmoid backward
-        if (warp == 0) {
-            float sds = 0.0f;
-            for (int i = lane; i < BW_THREADS; i += 32) sds += v_red[i];
-            sds = warp_sum(sds);
-            auto sumq = [&](const float* v, int t) {   // the NCQ column-group partials of one token
-                float a = 0.0f;
-#pragma unroll
-                for (int qd = 0; qd < NCQ; ++qd) a += v[qd * 64 + t];
-                return a;
-            };
-            auto colp = [&](int t) {
-                float a = 0.0f;
-#pragma unroll
-                for (int qd = 0; qd < BW_THREADS / 64; ++qd) a += v_colp4[qd * 64 + t];
-                return a;
-            };
-            const int tA = lane, tB = lane + 32;
-            const float kwA = sumq(v_rkw, tA), kwB = sumq(v_rkw, tB);
-            const float extra = __expf(g_last) * sds + warp_sum(kwA + kwB);
-            float dgA = sumq(v_rowp, tA) - colp(tA) + sumq(v_rqs, tA) + sumq(v_rkg, tA) - kwA;
-            float dgB = sumq(v_rowp, tB) - colp(tB) + sumq(v_rqs, tB) + sumq(v_rkg, tB) - kwB;
-            if (lane == 31) dgB += extra;
-            // suffix sums over t = 0..63 (A holds 0..31, B holds 32..63)
-            float sB = dgB, sA = dgA;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float nb = __shfl_down_sync(0xffffffffu, sB, o), na = __shfl_down_sync(0xffffffffu, sA, o);
-                if (lane + o < 32) {
-                    sB += nb;
-                    sA += na;
-                }
-            }
-            const float totB = __shfl_sync(0xffffffffu, sB, 0);
-            sA += totB;
-            if (tA < n) {
-                const int64_t r = grow + tA;
-                const float be = be_s[tA];
-                d_gate[r * 2 * H + h] = sA * (1.0f - v_al[tA]);
-                d_gate[r * 2 * H + H + h] = (sumq(v_rdr, tA) + be * sumq(v_dls, tA)) * (1.0f - be);
-            }
-            if (tB < n) {
-                const int64_t r = grow + tB;
-                const float be = be_s[tB];
-                d_gate[r * 2 * H + h] = sB * (1.0f - v_al[tB]);
-                d_gate[r * 2 * H + H + h] = (sumq(v_rdr, tB) + be * sumq(v_dls, tB)) * (1.0f - be);
-            }
-        }
-        // ---- F. new dS -> bf16 operand copy for the next chunk; next chunk's tiles
-        wait_bar(6, par);
-        tc::tcgen05_fence_after();
-        __syncthreads();   // staging reads are finished before the dS region is rewritten
-        if (c > 0) {
-            if (dhi != DH) clear_s0_pad();
-            if (tid == 0) {
-                tc::fence_proxy_async_smem();
-                issue_tma(c - 1);
-            }
-#pragma unroll
-            for (int ci = 0; ci < NCI; ++ci) {
-                uint32_t r[32];
-                tc::tmem_ld_32x32(ACC_S + lane_addr + (c0 + ci) * 32, r);
-                tc::tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float f8[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) f8[e] = __uint_as_float(r[8 * j + e]);
-                    *tile128(R_DS, arow, (c0 + ci) * 4 + j) = tc::pack8_bf16(f8);
-                }
-            }
-        }
-        if (__syncthreads_or(*abort_flag ? 1 : 0)) break;
     }
     tc::tcgen05_fence_before();
     __syncthreads();
     if (*abort_flag) __nanosleep(20000);
-    if (warp == 0) tc::tmem_dealloc(tm, 512);
+    if (warp == Cfg::COMPUTE / 32) tc::tmem_dealloc(tmem_S, 4 * DH);
 }
 
+// ------------------------------------------------------------------ backward chain
+// Same threads as the forward: quarters 0 and 1 hold the 64 rows of dU and dR, quarters 2 and 3 scale the rows of dO by gam in place
+// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO.
+template <int DH>
+__global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delta_bwd_tc_kernel(
+    const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapDO,
+    const __grid_constant__ CUtensorMap mapAA, const __grid_constant__ CUtensorMap mapAL, const __grid_constant__ CUtensorMap mapTP,
+    const __grid_constant__ CUtensorMap mapDS,
+    const __grid_constant__ CUtensorMap mapDR, const float* __restrict__ GB, const __nv_bfloat16* __restrict__ v,
+    int T, int H, int n_chunks, float* __restrict__ d_qkv, float* __restrict__ VD /* [tile][NG][64]: v . dv over 32 columns */, int* err_word) {
+    using Cfg = ChainCfg<DH>;
+    constexpr int NB = Cfg::NB, NG = Cfg::NG;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* S_s = base + 2 * Cfg::B_STAGE;      // dS: NB n-boxes x (DH k-rows x 128 B)
+    auto R_s = [&](int s) {                      // dU, then dR: NB n-boxes x (64 k-rows x 128 B)
+        return DH == 128 ? S_s + Cfg::S_BYTES : base + s * Cfg::B_STAGE + Cfg::B_A;
+    };
+    auto Rs_s = [&](int s) { return base + s * Cfg::B_STAGE + Cfg::B_RS; };
+    float* gb_s = reinterpret_cast<float*>(S_s + Cfg::S_BYTES + (DH == 128 ? 16384 : 0));   // [2][128], with the stages
+    uint64_t* bars = reinterpret_cast<uint64_t*>(gb_s + 256);
+    uint64_t *full = bars, *mma0_done = bars + 2, *mma1_done = bars + 3, *mma2_done = bars + 4, *mma3_done = bars + 5, *s_ready = bars + 6,
+             *do_ready = bars + 7, *du_ready = bars + 8, *dr_ready = bars + 9, *s_stored = bars + 10, *r_stored = bars + 11;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int chain = blockIdx.x;
+    const int b = chain / H, h = chain % H;
+    const int d = H * DH;
+    const int64_t tile0 = (int64_t)chain * n_chunks;
+
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < 12; ++i) {
+            const uint64_t* w = bars + i;
+            tc::mbar_init(&bars[i], w == s_ready ? Cfg::S_WARPS : w == do_ready || w == du_ready || w == dr_ready ? Cfg::ROW_WARPS : 1);
+        }
+        tc::mbar_fence_init();
+    }
+    constexpr int TMEM_COLS = 4 * DH;   // 3 DH, and a power of two
+    if (warp == Cfg::COMPUTE / 32) tc::tmem_alloc(tmem_slot, TMEM_COLS);
+    tc::tcgen05_fence_before();
+    __syncthreads();
+    tc::tcgen05_fence_after();
+    const uint32_t tmem_S = *tmem_slot, tmem_D1 = tmem_S + DH, tmem_D2 = tmem_S + 2 * DH;
+
+    if (warp == Cfg::COMPUTE / 32) {
+        // ------------------------------------------------------------ TMA loads + MMA issuer (one thread)
+        if (lane == 0) {
+            auto load = [&](int it) {
+                const int c = n_chunks - 1 - it, s = it & 1;
+                uint8_t* st = base + s * Cfg::B_STAGE;
+                const int t = (int)(tile0 + c);
+                tc::mbar_expect_tx(&full[s], Cfg::B_STAGE + 512);
+                load_vec(gb_s + s * 128, GB + (int64_t)t * 128, &full[s]);
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) tc::tma_load_3d(st + Cfg::B_DO + kb * 8192, &mapDO, h * DH + kb * 64, c * C, b, &full[s]);
+                tc::tma_load_2d(st + Cfg::B_A, &mapAA, 0, t * 64, &full[s]);
+                tc::tma_load_2d(st + Cfg::B_AL, &mapAL, 0, t * 64, &full[s]);
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) {
+                    tc::tma_load_3d(st + kb * 16384, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
+                    tc::tma_load_3d(st + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, c * C, b, &full[s]);
+                }
+                tc::tma_load_2d(st + Cfg::B_TP, &mapTP, 0, t * 64, &full[s]);
+            };
+            constexpr uint32_t ID_KM = tc::idesc_bf16_f32(128, DH, 0, 1), ID_MM = tc::idesc_bf16_f32(128, DH, 1, 1), ID_MM_NEG = ID_MM | (1u << 13);
+            const uint32_t s_addr = tc::smem_u32(S_s);
+            // D2 = (A + AL)^T dO of step `it`   (rows 64-127 multiply what lies behind and are not read)
+            auto mma0 = [&](int it) -> bool {
+                const int s = it & 1;
+                if (!tc::mbar_wait(&full[s], (it >> 1) & 1, abort_flag, err_word, 301)) return false;
+                const uint32_t st = tc::smem_u32(base + s * Cfg::B_STAGE);
+                tc::tcgen05_fence_after();
+#pragma unroll
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_D2, tc::smem_desc_sw128(st + Cfg::B_A + k16 * 2048, 8192, 1024),
+                                  tc::smem_desc_sw128(st + Cfg::B_DO + k16 * 2048, 8192, 1024), ID_MM, k16 > 0 ? 1u : 0u);
+#pragma unroll
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_D2, tc::smem_desc_sw128(st + Cfg::B_AL + k16 * 2048, 8192, 1024),
+                                  tc::smem_desc_sw128(st + Cfg::B_DO + k16 * 2048, 8192, 1024), ID_MM, 1u);
+                tc::umma_commit(mma0_done);
+                return true;
+            };
+            load(0);
+            if (n_chunks > 1) load(1);
+            bool ok = mma0(0);
+            for (int it = 0; ok && it < n_chunks; ++it) {
+                const int c = n_chunks - 1 - it, par = it & 1;
+                const uint32_t st = tc::smem_u32(base + par * Cfg::B_STAGE), r_addr = tc::smem_u32(R_s(par)), rs_addr = tc::smem_u32(Rs_s(par));
+                if (!tc::mbar_wait(s_ready, par, abort_flag, err_word, 302)) break;
+                tc::tcgen05_fence_after();
+                // D1 = K dS   (rows 64-127 multiply Q and are not read)
+#pragma unroll
+                for (int k16 = 0; k16 < DH / 16; ++k16)
+                    tc::umma_bf16(tmem_D1, tc::smem_desc_sw128(st + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
+                                  tc::smem_desc_sw128(s_addr + k16 * 2048, DH * 128, 1024), ID_KM, k16 > 0 ? 1u : 0u);
+                tc::umma_commit(mma1_done);
+                if (!tc::mbar_wait(du_ready, par, abort_flag, err_word, 303)) break;
+                tc::tcgen05_fence_after();
+                // D1 = (X - I)^T dU
+#pragma unroll
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_D1, tc::smem_desc_sw128(st + Cfg::B_TP + k16 * 2048, 8192, 1024),
+                                  tc::smem_desc_sw128(r_addr + k16 * 2048, 8192, 1024), ID_MM, k16 > 0 ? 1u : 0u);
+                tc::umma_commit(mma2_done);
+                if (c == 0) break;
+                // dS += Q^T (gam dO), while dR is formed
+                if (!tc::mbar_wait(do_ready, par, abort_flag, err_word, 304)) break;
+                tc::tcgen05_fence_after();
+#pragma unroll
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_S, tc::smem_desc_sw128(st + 8192 + k16 * 2048, 16384, 1024),
+                                  tc::smem_desc_sw128(st + Cfg::B_DO + k16 * 2048, 8192, 1024), ID_MM, 1u);
+                if (!tc::mbar_wait(dr_ready, par, abort_flag, err_word, 305)) break;
+                tc::tcgen05_fence_after();
+                // dS -= K^T (beta gam dR)
+#pragma unroll
+                for (int k16 = 0; k16 < C / 16; ++k16)
+                    tc::umma_bf16(tmem_S, tc::smem_desc_sw128(st + k16 * 2048, 16384, 1024),
+                                  tc::smem_desc_sw128(rs_addr + k16 * 2048, 8192, 1024), ID_MM_NEG, 1u);
+                tc::umma_commit(mma3_done);
+                if (!mma0(it + 1)) break;
+                if (it + 2 < n_chunks) {
+                    if (!tc::mbar_wait(mma3_done, par, abort_flag, err_word, 306)) break;
+                    if (DH != 128 && !tc::mbar_wait(r_stored, par, abort_flag, err_word, 309)) break;   // (dR lies in the stage)
+                    load(it + 2);
+                }
+            }
+        }
+    } else if (warp > Cfg::COMPUTE / 32) {
+        // ------------------------------------------------------------ dS at the end of each chunk and dR out (one thread)
+        if (lane == 0) {
+            for (int it = 0; it < n_chunks; ++it) {
+                const int c = n_chunks - 1 - it, par = it & 1;
+                if (!tc::mbar_wait(s_ready, par, abort_flag, err_word, 307)) break;
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapDS, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
+                tc::bulk_commit_group();
+                if (!tc::mbar_wait(dr_ready, par, abort_flag, err_word, 308)) break;
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapDR, R_s(par) + nb * 8192, nb * 64, (int)(tile0 + c) * 64);
+                tc::bulk_commit_group();
+                tc::bulk_wait_read_but_one();
+                tc::mbar_arrive(s_stored);
+                tc::bulk_wait_read();
+                tc::mbar_arrive(r_stored);
+            }
+            tc::bulk_wait_read();   // before the CTA's shared memory goes
+        }
+    } else {
+        const int wq = warp & 3, cg = warp >> 2, arow = 32 * wq + lane, row = arow & 63;
+        const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+        const int col = cg * 32;
+        const bool s_warp = DH == 128 || wq < 2;
+        const bool w32 = (reinterpret_cast<uintptr_t>(d_qkv) & 31) == 0;
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+            int got = 1;
+            if (lane == 0) got = tc::mbar_wait(bar, parity, abort_flag, err_word, code) ? 1 : 0;
+            got = __shfl_sync(0xffffffffu, got, 0);
+            tc::tcgen05_fence_after();
+            return got != 0;
+        };
+        auto arrive = [&](uint64_t* bar) {   // one arrival per warp, after every lane's accesses
+            tc::fence_proxy_async_smem();
+            tc::tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bar);
+        };
+        if (s_warp) {   // dS = 0
+            uint32_t z[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) z[j] = 0u;
+            tc::tmem_st_32x32(tmem_S + lane_addr + col, z);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int c16 = cg * 4 + j;
+                *reinterpret_cast<uint4*>(S_s + (c16 >> 3) * (DH * 128) + tc::sw128_off(arow, c16 & 7)) = make_uint4(0, 0, 0, 0);
+            }
+            tc::tmem_st_wait();
+            arrive(s_ready);
+        }
+        bool ok = warp_wait(&full[0], 0, 310);
+        for (int it = 0; ok && it < n_chunks; ++it) {   // (entered with the chunk's tiles in their stage)
+            const int c = n_chunks - 1 - it, par = it & 1;
+            uint8_t* st = base + par * Cfg::B_STAGE;
+            const float g_row = gb_s[par * 128 + row], be_row = gb_s[par * 128 + 64 + row], gam = expf(g_row);
+            float du[32];
+            uint4 v4[4];
+            if (wq >= 2) {
+                if (c > 0) {   // gam dO in place, once A^T dO is done
+                    if (!warp_wait(mma0_done, par, 311)) break;
+                    uint8_t* dot = st + Cfg::B_DO;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int c16 = cg * 4 + j;
+                        uint4* at = reinterpret_cast<uint4*>(dot + (c16 >> 3) * 8192 + tc::sw128_off(row, c16 & 7));
+                        float x8[8];
+                        tc::unpack8_bf16(*at, x8);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) x8[e] *= gam;
+                        *at = tc::pack8_bf16(x8);
+                    }
+                    arrive(do_ready);
+                }
+            } else {
+                // dU = A^T dO + eg (K dS)
+                const float eg = expf(gb_s[par * 128 + C - 1] - g_row);
+                if (it > 0 && !warp_wait(r_stored, (it - 1) & 1, 312)) break;
+                if (!warp_wait(mma1_done, par, 313)) break;   // (and A^T dO before it)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t a[16], r[16];
+                    tc::tmem_ld_32x16(tmem_D2 + lane_addr + col + 16 * i, a);
+                    tc::tmem_ld_32x16(tmem_D1 + lane_addr + col + 16 * i, r);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) du[16 * i + j] = fmaf(eg, __uint_as_float(r[j]), __uint_as_float(a[j]));
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int c16 = cg * 4 + 2 * i + j;
+                        *reinterpret_cast<uint4*>(R_s(par) + (c16 >> 3) * 8192 + tc::sw128_off(row, c16 & 7)) = tc::pack8_bf16(du + 16 * i + 8 * j);
+                    }
+                }
+                arrive(du_ready);
+                // dR = dU + (X - I)^T dU
+                if (!warp_wait(mma2_done, par, 314)) break;
+                const float bg = be_row * gam;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t r[16];
+                    tc::tmem_ld_32x16(tmem_D1 + lane_addr + col + 16 * i, r);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) du[16 * i + j] += __uint_as_float(r[j]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int c16 = cg * 4 + 2 * i + j;
+                        const uint32_t off = (c16 >> 3) * 8192 + tc::sw128_off(row, c16 & 7);
+                        *reinterpret_cast<uint4*>(R_s(par) + off) = tc::pack8_bf16(du + 16 * i + 8 * j);
+                        float x8[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) x8[e] = bg * du[16 * i + 8 * j + e];
+                        *reinterpret_cast<uint4*>(Rs_s(par) + off) = tc::pack8_bf16(x8);
+                    }
+                }
+                arrive(dr_ready);
+                // the row of v is asked for here and used behind the state's update
+                const __nv_bfloat16* vr = v + ((int64_t)b * T + c * C + row) * d + h * DH + col;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v4[j] = c * C + row < T ? reinterpret_cast<const uint4*>(vr)[j] : make_uint4(0, 0, 0, 0);
+            }
+            if (c > 0) {
+                if (!warp_wait(&full[par ^ 1], ((it + 1) >> 1) & 1, 315)) break;
+                if (s_warp) {   // dS at the start of the chunk: bf16 operand copy, and f32 scaled by the chunk before's decay
+                    const float gC = expf(gb_s[(par ^ 1) * 128 + C - 1]);
+                    if (!warp_wait(s_stored, par, 316)) break;
+                    if (!warp_wait(mma3_done, par, 317)) break;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        uint32_t r[16];
+                        float f[16];
+                        tc::tmem_ld_32x16(tmem_S + lane_addr + col + 16 * i, r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(r[j]);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            const int c16 = cg * 4 + 2 * i + j;
+                            *reinterpret_cast<uint4*>(S_s + (c16 >> 3) * (DH * 128) + tc::sw128_off(arow, c16 & 7)) = tc::pack8_bf16(f + 8 * j);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gC * f[j]);
+                        tc::tmem_st_32x16(tmem_S + lane_addr + col + 16 * i, r);
+                    }
+                    tc::tmem_st_wait();
+                    arrive(s_ready);
+                }
+            }
+            if (wq < 2) {   // dv = beta dR, and this thread's part of v . dv
+                float vd = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float x8[8];
+                    tc::unpack8_bf16(v4[j], x8);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        du[8 * j + e] *= be_row;
+                        vd = fmaf(x8[e], du[8 * j + e], vd);
+                    }
+                }
+                VD[((tile0 + c) * NG + cg) * 64 + row] = vd;
+                if (c * C + row < T) store32(d_qkv + ((int64_t)b * T + c * C + row) * 3 * d + 2 * d + h * DH + col, du, w32);
+            }
+        }
+    }
+    tc::tcgen05_fence_before();
+    __syncthreads();
+    if (*abort_flag) __nanosleep(20000);
+    if (warp == Cfg::COMPUTE / 32) tc::tmem_dealloc(tmem_S, TMEM_COLS);
+}
+
+// ------------------------------------------------------------------ gradients per chunk
+// One CTA per (chunk, chain), two per SM; nothing here depends on another chunk. With S and dS the (bf16) state at the chunk's start
+// and gradient at its end:
+//   dL = dR U^T,  dA = dO U^T,  X = dO S^T,  Y = dR S^T,  dW = U dS^T              one group of products, value columns 64 at a time
+//   M = -beta Gam dL (strictly lower),  P = Gam dA (lower);  X *= gam,  Y *= -beta gam   (in TMEM)
+//   dq = X + P K,   dk = Y + M^T K + P^T Q + M K + eg dW                           second group
+// and the gate gradients from row sums of these alone: with qdq_t = q_t . dq_t, kdk_t = k_t . dk_t and w_t = k_t . (M K + Y)_t
+//   d log alpha_t = sum over t' >= t of (qdq - kdk + 2 w)_t' + gam_C <S, dS> + sum over t' of eg k . dW
+//   d beta_t = (v_t . dv_t + w_t) / beta_t
+// (Row t of dA's and dL's products with Q K^T and K K^T, which these sums otherwise need, are q_t . (P K)_t and k_t . (M K)_t; their column
+// sums are what k . dk holds beyond them. The bf16 tiles P and M enter row and column sums alike, so that what should cancel does.)
+// TMEM halves: thread (warp, lane) sees row 16 (warp & 3) + (lane & 15) of the product in half lane >> 4.
+constexpr int GR_THREADS = 256;
+template <int DH>
+struct GradCfg {
+    static constexpr int NB = DH / 64, HB = 3 * 8192 + 2 * DH * 128 /*dO, dR, U, S, dS: one 64-wide box each*/;
+    static constexpr int R_K = 0, R_Q = NB * 8192, R_DO = NB * 16384, R_DR = R_DO + 8192, R_U = R_DR + 8192, R_S = R_U + 8192, R_DS = R_S + DH * 128,
+                         R_END = R_DS + DH * 128, R_M = R_DO, R_P = R_DR;
+    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 /*dots*/ + 2 * 64 * 3 /*k.MK, k.Y, k.dW*/ + 64 /*v.dv*/ + 8;
+    static constexpr size_t SMEM = 1024 + R_END + NVEC * 4 + 64;
+};
+
+template <int DH>
+__global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
+    const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapDO,
+    const __grid_constant__ CUtensorMap mapDR, const __grid_constant__ CUtensorMap mapU, const __grid_constant__ CUtensorMap mapS0,
+    const __grid_constant__ CUtensorMap mapDS, const float* __restrict__ GB, const float* __restrict__ VD, const float* __restrict__ alpha,
+    const float* __restrict__ qnorm, const float* __restrict__ knorm, int T, int H, int n_chunks,
+    float* __restrict__ d_qkv, float* __restrict__ d_gate, int* err_word) {
+    using Cfg = GradCfg<DH>;
+    constexpr int NB = Cfg::NB, CW = DH / 2 /*columns of a row per thread*/;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    float* g_s = reinterpret_cast<float*>(sm + Cfg::R_END);
+    float *be_s = g_s + 64, *al_s = be_s + 64, *nrm_s = al_s + 64 /*q rows, k rows*/, *dot_s = nrm_s + 128 /*[2][128]*/, *mk_s = dot_s + 256 /*[2][64]*/,
+          *ky_s = mk_s + 128, *kw_s = ky_s + 128, *vd_s = kw_s + 128, *red_s = vd_s + 64;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(red_s + 8);   // [0] K, Q; [1] a set of value columns; [2] its products; [3] second group
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int wq = warp & 3, cg = warp >> 2, half = lane >> 4, row = 16 * wq + (lane & 15);
+    const int chunk = blockIdx.x, chain = blockIdx.y;
+    const int b = chain / H, h = chain % H;
+    const int d = H * DH;
+    const int t0 = chunk * C;
+    const int n = T - t0 < C ? T - t0 : C;
+    const int64_t grow = (int64_t)b * T + t0;
+    const int64_t tix = (int64_t)chain * n_chunks + chunk;
+    const bool w32 = (reinterpret_cast<uintptr_t>(d_qkv) & 31) == 0;
+
+    auto load_half = [&](int hv) {
+        const int t = (int)tix;
+        tc::mbar_expect_tx(&bars[1], Cfg::HB);
+        tc::tma_load_2d(sm + Cfg::R_DR, &mapDR, hv * 64, t * 64, &bars[1]);
+        tc::tma_load_2d(sm + Cfg::R_U, &mapU, hv * 64, t * 64, &bars[1]);
+        tc::tma_load_3d(sm + Cfg::R_DO, &mapDO, h * DH + hv * 64, t0, b, &bars[1]);
+        tc::tma_load_2d(sm + Cfg::R_S, &mapS0, hv * 64, t * DH, &bars[1]);
+        tc::tma_load_2d(sm + Cfg::R_DS, &mapDS, hv * 64, t * DH, &bars[1]);
+    };
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < 4; ++i) tc::mbar_init(&bars[i], 1);
+        tc::mbar_fence_init();
+        load_half(0);
+        tc::mbar_expect_tx(&bars[0], NB * 16384);
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) {
+            tc::tma_load_3d(sm + Cfg::R_K + kb * 8192, &mapK, h * DH + kb * 64, t0, b, &bars[0]);
+            tc::tma_load_3d(sm + Cfg::R_Q + kb * 8192, &mapQ, h * DH + kb * 64, t0, b, &bars[0]);
+        }
+    }
+    if (warp == 0) tc::tmem_alloc(tmem_slot, 256);
+    {
+        const int t = tid & 63;
+        const bool live = t < n;
+        const int64_t r = (grow + (live ? t : 0)) * H + h;
+        if (tid < 64) {
+            g_s[t] = GB[tix * 128 + t];
+            be_s[t] = GB[tix * 128 + 64 + t];
+        } else if (tid < 128) {
+            al_s[t] = alpha[r];
+            float s = 0.0f;
+#pragma unroll
+            for (int i = 0; i < DH / 32; ++i) s += VD[(tix * (DH / 32) + i) * 64 + t];
+            vd_s[t] = s;
+        } else if (tid < 192) {
+            nrm_s[t] = qnorm[r];
+        } else {
+            nrm_s[64 + t] = knorm[r];
+        }
+    }
+    tc::tcgen05_fence_before();
+    __syncthreads();
+    tc::tcgen05_fence_after();
+    const uint32_t tm = *tmem_slot;
+    const uint32_t ACC_A = tm /* X | Y, then dq | dk */, ACC_D = tm + DH /* dL | dA, then M K */, ACC_W = tm + DH + 64 /* dW */;
+    constexpr uint32_t H1 = 16u << 16;                    // lane offset of the second half
+    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+    const uint32_t sb = tc::smem_u32(sm);
+    auto kmaj = [&](uint32_t off, int k16) { return tc::smem_desc_sw128(sb + off + k16 * 32, 16, 1024); };          // one 64-wide k box
+    auto mnmaj = [&](uint32_t off, int k16) { return tc::smem_desc_sw128(sb + off + k16 * 2048, 8192, 1024); };     // 64 k rows, boxes 8 KiB apart
+    auto tile = [&](uint32_t off, int r, int c16) -> uint4* {
+        return reinterpret_cast<uint4*>(sm + off + (c16 >> 3) * 8192 + tc::sw128_off(r, c16 & 7));
+    };
+    // A wait that gives up raises *abort_flag; the CTA then runs to its end on whatever it has (every block barrier is reached by
+    // every thread). The host sees the error word.
+    auto wait_bar = [&](int i, uint32_t parity) {
+        if (lane == 0) tc::mbar_wait(&bars[i], parity, abort_flag, err_word, 320 + i);
+        __syncwarp();
+        tc::tcgen05_fence_after();
+    };
+
+    // ---- first group, 64 value columns at a time; <S, dS> beside it
+    float sds = 0.0f;
+#pragma unroll 1
+    for (int hv = 0; hv < NB; ++hv) {
+        wait_bar(1, hv & 1);
+        if (tid == 0) {
+            constexpr uint32_t I64 = tc::idesc_bf16_f32(64, 64, 0, 0), IDH = tc::idesc_bf16_f32(64, DH, 0, 0);
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16) {
+                const uint32_t acc = hv > 0 || k16 > 0;
+                const uint64_t dr = kmaj(Cfg::R_DR, k16), dO = kmaj(Cfg::R_DO, k16), u = kmaj(Cfg::R_U, k16), s0 = kmaj(Cfg::R_S, k16);
+                tc::umma_bf16(ACC_D, dr, u, I64, acc);
+                tc::umma_bf16(ACC_D + H1, dO, u, I64, acc);
+                tc::umma_bf16(ACC_A, dO, s0, IDH, acc);
+                tc::umma_bf16(ACC_A + H1, dr, s0, IDH, acc);
+                if constexpr (DH == 128) {   // keys 0-63 in half 0, 64-127 in half 1
+                    tc::umma_bf16(ACC_W, u, kmaj(Cfg::R_DS, k16), I64, acc);
+                    tc::umma_bf16(ACC_W + H1, u, kmaj(Cfg::R_DS + 8192, k16), I64, acc);
+                } else {
+                    tc::umma_bf16(ACC_W + H1, u, kmaj(Cfg::R_DS, k16), I64, acc);
+                }
+            }
+            tc::umma_commit(&bars[2]);
+        }
+#pragma unroll
+        for (int i = 0; i < DH * 8 / GR_THREADS; ++i) {   // (the tiles have one layout: element by element)
+            float s8[8], d8[8];
+            tc::unpack8_bf16(*reinterpret_cast<const uint4*>(sm + Cfg::R_S + (tid + i * GR_THREADS) * 16), s8);
+            tc::unpack8_bf16(*reinterpret_cast<const uint4*>(sm + Cfg::R_DS + (tid + i * GR_THREADS) * 16), d8);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sds = fmaf(s8[e], d8[e], sds);
+        }
+        if (hv + 1 < NB) {
+            wait_bar(2, hv & 1);
+            __syncthreads();
+            if (tid == 0) {
+                tc::fence_proxy_async_smem();
+                load_half(hv + 1);
+            }
+        }
+    }
+    const float g_row = g_s[row], be_row = be_s[row], gam = __expf(g_row), eg = __expf(g_s[C - 1] - g_row);
+    sds = warp_sum(sds);
+    if (lane == 0) red_s[warp] = sds;
+    wait_bar(2, (NB - 1) & 1);
+    wait_bar(0, 0);
+    // ---- M (half 0) and P (half 1): 32 columns of a row per thread
+    {
+        uint32_t r[32];
+        tc::tmem_ld_32x32(ACC_D + lane_addr + cg * 32, r);
+        tc::tmem_ld_wait();
+        const float f = half == 0 ? -be_row : 1.0f;
+        const int lim = row + half;   // M: i < row; P: i <= row
+        // (the operand tiles lie where dO and dR were: the first group, and every thread's reading of S and dS, are over for this warp;
+        // nobody reads dO or dR outside the products)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float x8[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int i = cg * 32 + 8 * j + e;
+                x8[e] = i < lim ? f * __expf(g_row - g_s[i]) * __uint_as_float(r[8 * j + e]) : 0.0f;
+            }
+            *reinterpret_cast<uint4*>(sm + (half == 0 ? Cfg::R_M : Cfg::R_P) + tc::sw128_off(row, cg * 4 + j)) = tc::pack8_bf16(x8);
+        }
+    }
+    // ---- X *= gam, Y *= -beta gam, k . Y
+    {
+        const float f = half == 0 ? gam : -be_row * gam;
+        float ky = 0.0f;
+#pragma unroll
+        for (int pc = 0; pc < CW / 16; ++pc) {
+            const int col = cg * CW + pc * 16;
+            uint32_t r[16];
+            tc::tmem_ld_32x16(ACC_A + lane_addr + col, r);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float k8[8];
+                tc::unpack8_bf16(*tile(Cfg::R_K, row, (col >> 3) + j), k8);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float x = f * __uint_as_float(r[8 * j + e]);
+                    ky = fmaf(k8[e], x, ky);
+                    r[8 * j + e] = __float_as_uint(x);
+                }
+            }
+            tc::tmem_st_32x16(ACC_A + lane_addr + col, r);
+        }
+        if (half == 1) ky_s[cg * 64 + row] = ky;
+        tc::tmem_st_wait();
+    }
+    tc::fence_proxy_async_smem();
+    tc::tcgen05_fence_before();
+    __syncthreads();
+    // ---- second group
+    if (tid == 0) {
+        constexpr uint32_t IKM = tc::idesc_bf16_f32(64, DH, 0, 1), IMM = tc::idesc_bf16_f32(64, DH, 1, 1), IKM64 = tc::idesc_bf16_f32(64, 64, 0, 1);
+        tc::tcgen05_fence_after();
+#pragma unroll
+        for (int k16 = 0; k16 < 4; ++k16) {
+            const uint64_t kk = mnmaj(Cfg::R_K, k16), mk = kmaj(Cfg::R_M, k16);
+            tc::umma_bf16(ACC_A, kmaj(Cfg::R_P, k16), kk, IKM, 1u);                                  // P K
+            tc::umma_bf16(ACC_A + H1, mnmaj(Cfg::R_M, k16), kk, IMM, 1u);                            // M^T K
+            tc::umma_bf16(ACC_A + H1, mnmaj(Cfg::R_P, k16), mnmaj(Cfg::R_Q, k16), IMM, 1u);          // P^T Q
+            if constexpr (DH == 128) {
+                tc::umma_bf16(ACC_D, mk, kk, IKM64, k16 > 0);                                        // M K, keys 0-63 | 64-127
+                tc::umma_bf16(ACC_D + H1, mk, mnmaj(Cfg::R_K + 8192, k16), IKM64, k16 > 0);
+            } else {
+                tc::umma_bf16(ACC_D + H1, mk, kk, IKM64, k16 > 0);
+            }
+        }
+        tc::umma_commit(&bars[3]);
+    }
+    wait_bar(3, 0);
+    // ---- dq (half 0) and dk (half 1) before the norm's backward: back to TMEM; row sums
+    const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
+    {
+        float dot = 0.0f, mks = 0.0f, kws = 0.0f;
+#pragma unroll
+        for (int pc = 0; pc < CW / 16; ++pc) {
+            const int col = cg * CW + pc * 16;
+            uint32_t x[16], mk[16], w[16];
+            const uint32_t acol = DH == 128 ? pc * 16 : col;
+            tc::tmem_ld_32x16(ACC_A + lane_addr + col, x);
+            tc::tmem_ld_32x16(ACC_D + lane_addr + acol, mk);
+            tc::tmem_ld_32x16(ACC_W + lane_addr + acol, w);
+            tc::tmem_ld_wait();
+            if constexpr (DH == 128) {   // keys 64 cg .. of a row sit in half cg
+                const int src = (lane & 15) | (cg << 4);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    mk[j] = __shfl_sync(0xffffffffu, mk[j], src);
+                    w[j] = __shfl_sync(0xffffffffu, w[j], src);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float y8[8];
+                tc::unpack8_bf16(*tile(ytile, row, (col >> 3) + j), y8);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    float g = __uint_as_float(x[8 * j + e]);
+                    if (half == 1) {
+                        const float m_ = __uint_as_float(mk[8 * j + e]), w_ = eg * __uint_as_float(w[8 * j + e]);
+                        g += m_ + w_;
+                        mks = fmaf(y8[e], m_, mks);
+                        kws = fmaf(y8[e], w_, kws);
+                    }
+                    dot = fmaf(y8[e], g, dot);
+                    x[8 * j + e] = __float_as_uint(g);
+                }
+            }
+            tc::tmem_st_32x16(ACC_A + lane_addr + col, x);
+        }
+        dot_s[cg * 128 + half * 64 + row] = dot;
+        if (half == 1) {
+            mk_s[cg * 64 + row] = mks;
+            kw_s[cg * 64 + row] = kws;
+        }
+        tc::tmem_st_wait();
+    }
+    __syncthreads();
+    // ---- L2-norm backward and store
+    {
+        const float dot = dot_s[half * 64 + row] + dot_s[128 + half * 64 + row], inv = 1.0f / nrm_s[half * 64 + row];
+        float* dst = d_qkv + (grow + row) * 3 * d + half * d + h * DH;
+#pragma unroll
+        for (int pc = 0; pc < CW / 16; ++pc) {
+            const int col = cg * CW + pc * 16;
+            uint32_t x[16];
+            tc::tmem_ld_32x16(ACC_A + lane_addr + col, x);
+            tc::tmem_ld_wait();
+            float f[16];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float y8[8];
+                tc::unpack8_bf16(*tile(ytile, row, (col >> 3) + j), y8);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[8 * j + e] = (__uint_as_float(x[8 * j + e]) - y8[e] * dot) * inv;
+            }
+            if (row < n) store16(dst + col, f, w32);
+        }
+    }
+    // ---- gates (warp 0): reverse cumulative sum, sigmoid backward
+    if (warp == 0) {
+        float s[2], w[2], kw = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int t = lane + 32 * i;
+            w[i] = mk_s[t] + mk_s[64 + t] + ky_s[t] + ky_s[64 + t];
+            s[i] = dot_s[t] + dot_s[128 + t] - (dot_s[64 + t] + dot_s[192 + t]) + 2.0f * w[i];
+            kw += kw_s[t] + kw_s[64 + t];
+        }
+        float all = 0.0f;
+#pragma unroll
+        for (int i = 0; i < GR_THREADS / 32; ++i) all += red_s[i];
+        const float extra = __expf(g_s[C - 1]) * all + warp_sum(kw);
+        if (lane == 31) s[1] += extra;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {   // suffix sums over t = 0..63
+            const float nb = __shfl_down_sync(0xffffffffu, s[1], o), na = __shfl_down_sync(0xffffffffu, s[0], o);
+            if (lane + o < 32) {
+                s[1] += nb;
+                s[0] += na;
+            }
+        }
+        s[0] += __shfl_sync(0xffffffffu, s[1], 0);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int t = lane + 32 * i;
+            if (t < n) {
+                float* dst = d_gate + (grow + t) * 2 * H + h;
+                dst[0] = s[i] * (1.0f - al_s[t]);
+                dst[H] = (vd_s[t] + w[i]) * (1.0f - be_s[t]);
+            }
+        }
+    }
+    tc::tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tm, 256);
+    if (*abort_flag) __nanosleep(20000);
+}
+
+// ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1298,78 +1331,80 @@ static bool make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t col
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+static bool make_map3(CUtensorMap* m, const void* base, int64_t B, int64_t T, int64_t cols) {   // (columns, tokens, sequences), 64 x 64 boxes
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)T, (cuuint64_t)B};
+    cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)(T * cols) * 2};
+    cuuint32_t box[3] = {64, C, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 static inline size_t al(size_t x) { return (x + 1023) & ~(size_t)1023; }
+static inline char* al_ptr(void* p) { return reinterpret_cast<char*>(al(reinterpret_cast<size_t>(p))); }
 
 bool available() { return encode_fn() != nullptr; }
 
-// Carves the per-(chain, chunk) tile buffers out of `w` (1024-byte aligned). With `full` the
-// backward-only tiles are included.
-static size_t carve_tiles(char* w, int64_t n_tiles, bool full, Tiles* t) {
-    const size_t b128 = al((size_t)n_tiles * 128 * DH * 2), b64 = al((size_t)n_tiles * 64 * DH * 2),
-                 bcc = al((size_t)n_tiles * 64 * 64 * 2), bv = al((size_t)n_tiles * 64 * 4), bg = al((size_t)n_tiles * 4);
-    char* p = w;
-    auto take = [&](size_t n) {
-        char* r = p;
-        p += n;
+// Carves the per-(chain, chunk) buffers out of memory that starts on a 1024-byte boundary (null: counts).
+struct Carver {
+    char* base;
+    size_t at = 0;
+    template <typename P>
+    P* take(int64_t n) {
+        P* r = base ? reinterpret_cast<P*>(base + at) : nullptr;
+        at += al((size_t)n * sizeof(P));
         return r;
-    };
-    Tiles z{};
-    z.WQ = (__nv_bfloat16*)take(b128);
-    z.UV = (__nv_bfloat16*)take(b64);
-    z.KW = (__nv_bfloat16*)take(b64);
-    z.AA = (__nv_bfloat16*)take(bcc);
-    z.GC = (float*)take(bg);
-    if (full) {
-        z.BK = (__nv_bfloat16*)take(b64);
-        z.BV = (__nv_bfloat16*)take(b64);
-        z.UVT = (__nv_bfloat16*)take(b64);
-        z.TP = (__nv_bfloat16*)take(bcc);
-        z.KKo = (__nv_bfloat16*)take(bcc);
-        z.QKo = (__nv_bfloat16*)take(bcc);
-        z.GV = (float*)take(bv);
-        z.BE = (float*)take(bv);
     }
-    if (t) *t = z;
-    return (size_t)(p - w);
+};
+static void carve_kept(Carver& w, int64_t n_tiles, bool full, Tiles* t) {   // what a backward reads again
+    t->AA = w.take<__nv_bfloat16>(n_tiles * C * C);
+    t->AL = w.take<__nv_bfloat16>(n_tiles * C * C);
+    t->TP = full ? w.take<__nv_bfloat16>(n_tiles * C * C) : nullptr;
+    t->GB = w.take<float>(n_tiles * 2 * C);
+}
+static void carve_rows(Carver& w, int64_t n_tiles, int64_t dh, Tiles* t) {
+    t->WH = w.take<__nv_bfloat16>(n_tiles * C * dh);
+    t->UV = w.take<__nv_bfloat16>(n_tiles * C * dh);
 }
 
-static int run_prepass(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha,
-                       const float* beta, int64_t T, int64_t H, int64_t dh, int64_t n_chunks, int64_t chains, const Tiles& t) {
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(delta_prep_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PRE_SMEM));
+template <int DH>
+static int run_prepass(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta, int64_t B, int64_t T,
+                       int64_t H, int64_t n_chunks, const Tiles& t) {
+    CUtensorMap mK, mQ, mV, mWH, mUV;
+    const int64_t n_tiles = B * H * n_chunks;
+    if (!make_map3(&mK, k, B, T, H * DH) || !make_map3(&mQ, q, B, T, H * DH) || !make_map3(&mV, v, B, T, H * DH) ||
+        !make_map(&mWH, t.WH, n_tiles * C, DH, 64, C) || !make_map(&mUV, t.UV, n_tiles * C, DH, 64, C))
+        return asca_fail(ctx, ASCA_ERR_CUDA, "delta_tc: cuTensorMapEncodeTiled failed");
+    auto kern = delta_prep_tc_kernel<DH>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pre_smem<DH>()));
     {
         asca_span sp(ctx, "delta_prep_tc_kernel");
-        delta_prep_tc_kernel<<<dim3((unsigned)n_chunks, (unsigned)chains), PRE_THREADS, PRE_SMEM, ctx->stream>>>(
-            (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, alpha, beta, (int)T, (int)H, (int)dh,
-            (int)n_chunks, t, ctx->err_word);
+        kern<<<dim3((unsigned)n_chunks, (unsigned)(B * H)), PRE_THREADS, pre_smem<DH>(), ctx->stream>>>(
+            mK, mQ, mV, mWH, mUV, alpha, beta, (int)T, (int)H, (int)n_chunks, t, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     return ASCA_OK;
 }
 
-// Forward for bf16 q,k,v (dh = 128, or 64 zero-padded to 128 inside). o is bf16. When checkpoints are requested (a
-// backward will follow) the pre-pass also writes the backward-only tiles into a context-owned buffer keyed by
-// the checkpoint pointer, so that the backward does not repeat the pre-pass. In this mode the
-// checkpoint buffer holds the chunk-start states rounded to bf16, (B, H, n_chunks, dh, dh) row-major
-// in its first half: the backward loads them by TMA as tensor-core operands.
-int forward(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
-            int64_t B, int64_t T, int64_t H, int64_t dh, void* o, const float* s_init, float* s_final, float* ckpt) {
-    if (s_final && (reinterpret_cast<uintptr_t>(s_final) & 15)) {   // the kernel writes the final state 16 bytes at a time
-        const size_t bytes = (size_t)(B * H * dh * dh) * 4;
-        void* fin;
-        ASCA_TRY(asca_malloc(ctx, bytes, &fin));
-        int rc = forward(ctx, q, k, v, alpha, beta, B, T, H, dh, o, s_init, (float*)fin, ckpt);
-        if (rc == ASCA_OK && cudaMemcpyAsync(s_final, fin, bytes, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-            rc = asca_fail(ctx, ASCA_ERR_CUDA, "delta_fwd: cannot copy the final state");
-        asca_free(ctx, fin);   // (reused by later work on the stream only)
-        return rc;
-    }
+// Forward for bf16 q, k, v. o is bf16. When checkpoints are requested (a backward will follow) the buffer receives, as bf16, the
+// chunk-start states (B, H, n_chunks, dh, dh) in its first half and the rows U (B, H, n_chunks, 64, dh) behind them; A, X - I and the
+// decays stay in a context-owned buffer keyed by the checkpoint pointer, so that the backward does not repeat the pre-pass.
+template <int DH>
+static int forward_dh(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+                      int64_t B, int64_t T, int64_t H, void* o, const float* s_init, float* s_final, float* ckpt) {
     const int64_t n_chunks = (T + C - 1) / C, chains = B * H, n_tiles = chains * n_chunks;
     Tiles t{};
     const bool keep = ckpt != nullptr;
-    const size_t need = carve_tiles(nullptr, n_tiles, keep, nullptr) + 1024;
-    char* w;
     int slot = -1;
+    void* ws;
     if (keep) {
+        Carver kept{nullptr}, rows{nullptr};
+        carve_kept(kept, n_tiles, true, &t);
+        carve_rows(rows, n_tiles, DH, &t);
+        const size_t need = kept.at + 1024;
         auto& dt = ctx->dtiles;
         for (size_t i = 0; i < dt.size(); ++i)
             if (dt[i].buf && dt[i].ckpt == (const void*)ckpt) slot = (int)i;
@@ -1398,28 +1433,36 @@ int forward(asca_ctx* ctx, const void* q, const void* k, const void* v, const fl
             ASCA_CUDA(ctx, cudaMalloc(&e.buf, need));
             e.bytes = need;
         }
-        w = (char*)e.buf;
+        kept = Carver{al_ptr(e.buf)};
+        carve_kept(kept, n_tiles, true, &t);
+        ASCA_TRY(asca_workspace(ctx, rows.at + 1024, &ws));
+        rows = Carver{al_ptr(ws)};
+        carve_rows(rows, n_tiles, DH, &t);
     } else {
-        void* ws;
-        ASCA_TRY(asca_workspace(ctx, need, &ws));
-        w = (char*)ws;
+        Carver w{nullptr};
+        carve_kept(w, n_tiles, false, &t);
+        carve_rows(w, n_tiles, DH, &t);
+        ASCA_TRY(asca_workspace(ctx, w.at + 1024, &ws));
+        w = Carver{al_ptr(ws)};
+        carve_kept(w, n_tiles, false, &t);
+        carve_rows(w, n_tiles, DH, &t);
     }
-    w = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(w) + 1023) & ~(uintptr_t)1023);
-    carve_tiles(w, n_tiles, keep, &t);
-    ASCA_TRY(run_prepass(ctx, q, k, v, alpha, beta, T, H, dh, n_chunks, chains, t));
-    CUtensorMap mWQ, mUV, mKW, mAA, mS0;
-    if (!make_map(&mWQ, t.WQ, n_tiles * 128, DH, 64, 128) || !make_map(&mUV, t.UV, n_tiles * 64, DH, 64, 64) ||
-        !make_map(&mKW, t.KW, n_tiles * 64, DH, 64, 64) || !make_map(&mAA, t.AA, n_tiles * 64, 64, 64, 64) ||
-        !(keep ? make_map(&mS0, ckpt, n_tiles * dh, dh, 64, (int)dh)   // bf16 states in the checkpoint buffer
-               : make_map(&mS0, t.WQ, n_tiles * DH, DH, 64, 128)))    // (unused)
+    ASCA_TRY((run_prepass<DH>(ctx, q, k, v, alpha, beta, B, T, H, n_chunks, t)));
+    CUtensorMap mWH, mQ, mK, mUV, mAA, mAL, mS0, mU;
+    const char* u_rows = reinterpret_cast<const char*>(ckpt) + (size_t)n_tiles * DH * DH * 2;
+    if (!make_map(&mWH, t.WH, n_tiles * C, DH, 64, C) || !make_map3(&mQ, q, B, T, H * DH) || !make_map3(&mK, k, B, T, H * DH) ||
+        !make_map(&mUV, t.UV, n_tiles * C, DH, 64, C) || !make_map(&mAA, t.AA, n_tiles * C, C, 64, C) ||
+        !make_map(&mAL, t.AL, n_tiles * C, C, 64, C) ||
+        !(keep ? make_map(&mS0, ckpt, n_tiles * DH, DH, 64, DH) && make_map(&mU, u_rows, n_tiles * C, DH, 64, C)
+               : make_map(&mS0, t.WH, n_tiles * C, DH, 64, C) && make_map(&mU, t.WH, n_tiles * C, DH, 64, C)))   // (unused)
         return asca_fail(ctx, ASCA_ERR_CUDA, "delta_tc: cuTensorMapEncodeTiled failed");
-    auto kern = delta_fwd_tc_kernel<__nv_bfloat16>;
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM));
+    using Cfg = ChainCfg<DH>;
+    auto kern = delta_fwd_tc_kernel<DH>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::F_SMEM));
     {
         asca_span sp(ctx, "delta_fwd_tc_kernel");
-        kern<<<(unsigned)chains, CH_THREADS, CH_SMEM, ctx->stream>>>(mWQ, mUV, mKW, mAA, mS0, t.GC, (int)T, (int)H, (int)dh,
-                                                                    (int)n_chunks, (__nv_bfloat16*)o, s_init, s_final,
-                                                                    nullptr, reinterpret_cast<__nv_bfloat16*>(ckpt), ctx->err_word);
+        kern<<<(unsigned)chains, Cfg::THREADS, Cfg::F_SMEM, ctx->stream>>>(mWH, mQ, mK, mUV, mAA, mAL, mS0, mU, t.GB, (int)T, (int)H, (int)n_chunks,
+                                                                           (__nv_bfloat16*)o, s_init, s_final, keep ? 1 : 0, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     if (keep) {
@@ -1428,18 +1471,34 @@ int forward(asca_ctx* ctx, const void* q, const void* k, const void* v, const fl
         e.q = q; e.k = k; e.v = v; e.alpha = alpha; e.beta = beta;
         e.B = B;
         e.T = T;
-        e.H = H * 1024 + dh;   // heads and head dim in one key field
+        e.H = H * 1024 + DH;   // heads and head dim in one key field
         e.stamp = ++ctx->dtiles_clock;
     }
     return ASCA_OK;
 }
 
-// Backward for bf16 q,k,v,d_o (dh = 128 or 64, checkpoints every 64 tokens from the forward).
-int backward(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
-             const float* qnorm, const float* knorm, const void* d_o, const float* ckpt, int64_t B, int64_t T, int64_t H,
-             int64_t dh, float* d_qkv, float* d_gate) {
+int forward(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+            int64_t B, int64_t T, int64_t H, int64_t dh, void* o, const float* s_init, float* s_final, float* ckpt) {
+    if (s_final && (reinterpret_cast<uintptr_t>(s_final) & 15)) {   // the kernel writes the final state 16 bytes at a time
+        const size_t bytes = (size_t)(B * H * dh * dh) * 4;
+        void* fin;
+        ASCA_TRY(asca_malloc(ctx, bytes, &fin));
+        int rc = forward(ctx, q, k, v, alpha, beta, B, T, H, dh, o, s_init, (float*)fin, ckpt);
+        if (rc == ASCA_OK && cudaMemcpyAsync(s_final, fin, bytes, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
+            rc = asca_fail(ctx, ASCA_ERR_CUDA, "delta_fwd: cannot copy the final state");
+        asca_free(ctx, fin);   // (reused by later work on the stream only)
+        return rc;
+    }
+    return dh == 128 ? forward_dh<128>(ctx, q, k, v, alpha, beta, B, T, H, o, s_init, s_final, ckpt)
+                     : forward_dh<64>(ctx, q, k, v, alpha, beta, B, T, H, o, s_init, s_final, ckpt);
+}
+
+// Backward for bf16 q, k, v, d_o (checkpoints every 64 tokens from the forward).
+template <int DH>
+static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+                       const float* qnorm, const float* knorm, const void* d_o, const float* ckpt, int64_t B, int64_t T, int64_t H,
+                       float* d_qkv, float* d_gate) {
     const int64_t n_chunks = (T + C - 1) / C, chains = B * H, n_tiles = chains * n_chunks;
-    ASCA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(d_qkv) & 15) == 0, "delta_bwd: d_qkv must be 16-byte aligned in tensor-core mode");
     Tiles t{};
     int slot = -1;
     for (size_t i = 0; i < ctx->dtiles.size(); ++i) {
@@ -1447,37 +1506,64 @@ int backward(asca_ctx* ctx, const void* q, const void* k, const void* v, const f
         // the tiles are functions of q, k, v, alpha, beta: the same buffers must come back (their contents are the
         // caller's contract, see the header); anything else rebuilds the tiles
         if (e.buf && e.ckpt == (const void*)ckpt && e.q == q && e.k == k && e.v == v && e.alpha == (const void*)alpha &&
-            e.beta == (const void*)beta && e.B == B && e.T == T && e.H == H * 1024 + dh)
+            e.beta == (const void*)beta && e.B == B && e.T == T && e.H == H * 1024 + DH)
             slot = (int)i;
     }
-    if (slot >= 0) {
-        // the forward that wrote `ckpt` left its tiles (functions of the same q,k,v,alpha,beta) here
-        ctx->dtiles[slot].stamp = ++ctx->dtiles_clock;
-        char* w = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ctx->dtiles[slot].buf) + 1023) & ~(uintptr_t)1023);
-        carve_tiles(w, n_tiles, true, &t);
-    } else {
-        void* ws;
-        ASCA_TRY(asca_workspace(ctx, carve_tiles(nullptr, n_tiles, true, nullptr) + 1024, &ws));
-        char* w = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~(uintptr_t)1023);
-        carve_tiles(w, n_tiles, true, &t);
-        ASCA_TRY(run_prepass(ctx, q, k, v, alpha, beta, T, H, dh, n_chunks, chains, t));
+    __nv_bfloat16 *dS, *dR;
+    float* VD;
+    void* ws;
+    for (int pass = 0; pass < 2; ++pass) {   // count, then carve
+        Carver w{pass ? al_ptr(ws) : nullptr};
+        dS = w.take<__nv_bfloat16>(n_tiles * DH * DH);
+        dR = w.take<__nv_bfloat16>(n_tiles * C * DH);
+        VD = w.take<float>(n_tiles * C * (DH / 32));
+        if (slot < 0) {
+            carve_kept(w, n_tiles, true, &t);
+            carve_rows(w, n_tiles, DH, &t);
+        }
+        if (!pass) ASCA_TRY(asca_workspace(ctx, w.at + 1024, &ws));
     }
-    CUtensorMap mWQ, mBK, mKW, mKR, mQR, mDO, mAA, mTP, mS0;
-    bool ok = make_map(&mWQ, t.WQ, n_tiles * 128, DH, 64, 64) && make_map(&mBK, t.BK, n_tiles * 64, DH, 64, 64) &&
-              make_map(&mKW, t.KW, n_tiles * 64, DH, 64, 64) && make_map(&mKR, k, B * T, H * dh, 64, 64) &&
-              make_map(&mQR, q, B * T, H * dh, 64, 64) && make_map(&mDO, d_o, B * T, H * dh, 64, 64) &&
-              make_map(&mAA, t.AA, n_tiles * 64, 64, 64, 64) && make_map(&mTP, t.TP, n_tiles * 64, 64, 64, 64) &&
-              make_map(&mS0, ckpt, n_tiles * dh, dh, 64, (int)dh);
-    if (!ok) return asca_fail(ctx, ASCA_ERR_CUDA, "delta_tc: cuTensorMapEncodeTiled failed");
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(delta_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BW_SMEM));
+    if (slot >= 0) {   // the forward that wrote `ckpt` left its tiles here
+        ctx->dtiles[slot].stamp = ++ctx->dtiles_clock;
+        Carver kept{al_ptr(ctx->dtiles[slot].buf)};
+        carve_kept(kept, n_tiles, true, &t);
+    } else {
+        ASCA_TRY((run_prepass<DH>(ctx, q, k, v, alpha, beta, B, T, H, n_chunks, t)));
+    }
+    CUtensorMap mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, mS0, mU;
+    const char* u_rows = reinterpret_cast<const char*>(ckpt) + (size_t)n_tiles * DH * DH * 2;
+    if (!make_map3(&mK, k, B, T, H * DH) || !make_map3(&mQ, q, B, T, H * DH) || !make_map3(&mDO, d_o, B, T, H * DH) ||
+        !make_map(&mAA, t.AA, n_tiles * C, C, 64, C) || !make_map(&mAL, t.AL, n_tiles * C, C, 64, C) ||
+        !make_map(&mTP, t.TP, n_tiles * C, C, 64, C) ||
+        !make_map(&mDS, dS, n_tiles * DH, DH, 64, DH) || !make_map(&mDR, dR, n_tiles * C, DH, 64, C) ||
+        !make_map(&mS0, ckpt, n_tiles * DH, DH, 64, DH) || !make_map(&mU, u_rows, n_tiles * C, DH, 64, C))
+        return asca_fail(ctx, ASCA_ERR_CUDA, "delta_tc: cuTensorMapEncodeTiled failed");
+    using Cfg = ChainCfg<DH>;
+    auto chain = delta_bwd_tc_kernel<DH>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::B_SMEM));
     {
         asca_span sp(ctx, "delta_bwd_tc_kernel");
-        delta_bwd_tc_kernel<<<(unsigned)chains, BW_THREADS, BW_SMEM, ctx->stream>>>(
-            mWQ, mBK, mKW, mKR, mQR, mDO, mAA, mTP, mS0, t, alpha, qnorm, knorm, (int)T, (int)H, (int)dh, (int)n_chunks, d_qkv,
-            d_gate, ctx->err_word);
+        chain<<<(unsigned)chains, Cfg::THREADS, Cfg::B_SMEM, ctx->stream>>>(mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, t.GB, (const __nv_bfloat16*)v, (int)T,
+                                                                            (int)H, (int)n_chunks, d_qkv, VD, ctx->err_word);
+    }
+    ASCA_CHECK_LAUNCH(ctx);
+    auto grad = delta_grad_tc_kernel<DH>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradCfg<DH>::SMEM));
+    {
+        asca_span sp(ctx, "delta_grad_tc_kernel");
+        grad<<<dim3((unsigned)n_chunks, (unsigned)chains), GR_THREADS, GradCfg<DH>::SMEM, ctx->stream>>>(
+            mK, mQ, mDO, mDR, mU, mS0, mDS, t.GB, VD, alpha, qnorm, knorm, (int)T, (int)H, (int)n_chunks, d_qkv, d_gate, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     return ASCA_OK;
+}
+
+int backward(asca_ctx* ctx, const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+             const float* qnorm, const float* knorm, const void* d_o, const float* ckpt, int64_t B, int64_t T, int64_t H,
+             int64_t dh, float* d_qkv, float* d_gate) {
+    ASCA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(d_qkv) & 15) == 0, "delta_bwd: d_qkv must be 16-byte aligned in tensor-core mode");
+    return dh == 128 ? backward_dh<128>(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, B, T, H, d_qkv, d_gate)
+                     : backward_dh<64>(ctx, q, k, v, alpha, beta, qnorm, knorm, d_o, ckpt, B, T, H, d_qkv, d_gate);
 }
 
 }  // namespace delta_tc

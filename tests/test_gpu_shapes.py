@@ -632,3 +632,66 @@ def test_prefill_with_the_fused_qkv_epilogue(orc, gpu, d, H, ns, T):
     m.free()
     for a, b in zip(*got):
         assert rel_err(b, a) < 5e-3
+
+
+# bf16 delta on the tensor cores: a sequence's last, ragged chunk must not read the next sequence's rows (zero times NaN is NaN),
+# and what comes out is as close to 64-bit arithmetic as bf16 operands allow.
+@pytest.mark.parametrize("dh", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(2, 1, 1), (2, 63, 2), (3, 65, 1), (2, 129, 3)])
+def test_delta_tc_sequences_do_not_mix(gpu, B, T, H, dh):
+    import torch
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(7 * T + dh)
+    n = B * T
+
+    def norm(*s):
+        return torch.randn(*s, generator=g, device="cuda")
+
+    q, k = (torch.nn.functional.normalize(norm(n, H, dh), dim=-1).reshape(n, H * dh).bfloat16() for _ in range(2))
+    v, d_o = norm(n, H * dh).bfloat16(), norm(n, H * dh).bfloat16()
+    al, be, qn = torch.sigmoid(2 + norm(n, H)), torch.sigmoid(norm(n, H)), 1 + torch.rand(n, H, generator=g, device="cuda")
+
+    def run(q, k, v, d_o):
+        o, fin, ck = ops.delta_fwd(gpu, q, k, v, al, be, B, T, H, dh, want_final=True)
+        d_qkv, d_gate = ops.delta_bwd(gpu, q, k, v, al, be, qn, qn, d_o, ck, B, T, H, dh)
+        gpu.sync()
+        return o, fin, d_qkv, d_gate
+
+    want = run(q, k, v, d_o)
+    bad = [x.clone() for x in (q, k, v, d_o)]
+    for x in bad:
+        x[T:2 * T] = float("nan")   # the second sequence
+    got = run(*bad)
+    keep = torch.ones(n, dtype=torch.bool, device="cuda")
+    keep[T:2 * T] = False
+    seqs = torch.arange(B, device="cuda") != 1
+    for a, b, m in zip(got, want, (keep, seqs, keep, keep)):
+        assert torch.equal(a[m], b[m]) and not torch.isnan(b).any()
+    assert torch.isnan(got[0][~keep]).any()
+
+    # the recurrence in 64 bits on the same bf16 inputs, gradients by autograd
+    q64, k64, v64, do64 = (x.double().view(B, T, H, dh).transpose(1, 2).clone().requires_grad_() for x in (q, k, v, d_o))
+    la = al.double().log().view(B, T, H).transpose(1, 2).clone().requires_grad_()
+    b64 = be.double().view(B, T, H).transpose(1, 2).clone().requires_grad_()
+    S, outs = torch.zeros(B, H, dh, dh, dtype=torch.float64, device="cuda"), []
+    for t in range(T):
+        S = la[:, :, t].exp()[..., None, None] * S
+        u = b64[:, :, t, None] * (v64[:, :, t] - torch.einsum("bhai,bha->bhi", S, k64[:, :, t]))
+        S = S + k64[:, :, t, :, None] * u[:, :, None, :]
+        outs.append(torch.einsum("bhai,bha->bhi", S, q64[:, :, t]))
+    o64 = torch.stack(outs, 2)
+    (o64 * do64).sum().backward()
+
+    def back(x, y):   # the L2 norm's backward
+        return (x.grad - y * (y * x.grad).sum(-1, keepdim=True)) / qn.double().view(B, T, H).transpose(1, 2)[..., None]
+
+    def flat(x):
+        return x.transpose(1, 2).reshape(n, -1)
+
+    d64 = torch.cat([flat(back(q64, q64.detach())), flat(back(k64, k64.detach())), flat(v64.grad)], 1)
+    g64 = torch.cat([flat(la.grad * (1 - la.exp())), flat(b64.grad * b64 * (1 - b64))], 1)
+    # a handful of bf16 roundings (2^-9 each) on the way to every value
+    for got_, ref in zip(want, (flat(o64), S, d64, g64)):
+        ref = ref.detach()
+        assert (got_.double() - ref).norm() < 8e-3 * ref.norm()
