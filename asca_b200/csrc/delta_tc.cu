@@ -48,6 +48,23 @@ __device__ __forceinline__ void load_vec(void* dst, const float* src, uint64_t* 
                  ::"r"(tc::smem_u32(dst)), "l"(src), "r"(tc::smem_u32(bar))
                  : "memory");
 }
+// acc += the products of eight pairs of bf16, exact each, added one by one in f32
+__device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc) {
+    const uint32_t a4[4] = {a.x, a.y, a.z, a.w}, b4[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
+            "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
+            : "+f"(acc)
+            : "r"(a4[i]), "r"(b4[i]));
+    return acc;
+}
+// exp(x) like __expf, in an instruction the compiler does not move under a condition
+__device__ __forceinline__ float exp_neg(float x) {
+    float y;
+    asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504f));
+    return y;
+}
 // 32 columns of a row, 32 bytes at a time where the rows lie on that grid
 __device__ __forceinline__ void store32(float* p, const float (&v)[32], bool w32) {
     if (w32) {
@@ -103,31 +120,49 @@ constexpr size_t pre_smem() {
     return 1024 + (size_t)(DH / 64) * 24576 /*K, Q, V*/ + L_BYTES + TRI_BYTES + 64 * 4 + 64;
 }
 
-// One 1 x 4 strip of a 16 x 16 block product  acc += Lrow[0..16) * X[0..16)[c4..c4+4)  (f32, shared memory).
-__device__ __forceinline__ void strip16(const float* __restrict__ lrow, const float* __restrict__ x, float acc[4]) {
+// An R x 4 tile of a 16 x 16 block product  acc += L[r..r+R)[0..16) * X[0..16)[c..c+4)  (f32, shared memory): R + 4 reads of 16 bytes
+// per 16 R multiply-adds. What counts here is the shared-memory read path, so tiles of four rows on a few lanes beat strips of one
+// row on all of them.
+template <int R>
+__device__ __forceinline__ void tile16(const float* __restrict__ l, const float* __restrict__ x, float (&acc)[R][4]) {
 #pragma unroll
     for (int k4 = 0; k4 < 4; ++k4) {
-        const float4 l4 = *reinterpret_cast<const float4*>(lrow + 4 * k4);
-        const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
+        float4 lr[R], xr[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float4 x4 = *reinterpret_cast<const float4*>(x + (4 * k4 + e) * BLD);
-            acc[0] = fmaf(lv[e], x4.x, acc[0]);
-            acc[1] = fmaf(lv[e], x4.y, acc[1]);
-            acc[2] = fmaf(lv[e], x4.z, acc[2]);
-            acc[3] = fmaf(lv[e], x4.w, acc[3]);
+        for (int i = 0; i < R; ++i) lr[i] = *reinterpret_cast<const float4*>(l + i * BLD + 4 * k4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) xr[e] = *reinterpret_cast<const float4*>(x + (4 * k4 + e) * BLD);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float lv[4] = {lr[i].x, lr[i].y, lr[i].z, lr[i].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[i][0] = fmaf(lv[e], xr[e].x, acc[i][0]);
+                acc[i][1] = fmaf(lv[e], xr[e].y, acc[i][1]);
+                acc[i][2] = fmaf(lv[e], xr[e].z, acc[i][2]);
+                acc[i][3] = fmaf(lv[e], xr[e].w, acc[i][3]);
+            }
         }
     }
 }
-__device__ __forceinline__ void put4(float* p, const float acc[4], float f) {
-    *reinterpret_cast<float4*>(p) = make_float4(f * acc[0], f * acc[1], f * acc[2], f * acc[3]);
+template <int R>
+__device__ __forceinline__ void put_tile(float* p, float (&acc)[R][4], float f) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        *reinterpret_cast<float4*>(p + i * BLD) = make_float4(f * acc[i][0], f * acc[i][1], f * acc[i][2], f * acc[i][3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
+    }
 }
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-// Three CTAs of eight warps per SM. K, Q and V come by TMA and are never copied: the factors beta gam and beta go into the
+// Three CTAs of eight warps per SM (four at head dim 64): bound by the latency of a CTA's chain -- tiles, [K;Q]K^T, the solve on four
+// warps, the second products -- of which the stores are a sixth. 8192 chunks of 64 x 128: 235 us (440 with scaled copies of K, Q and V
+// kept for the chains and the solve on all warps, strip by strip); 64 x 64: 193. K, Q and V come by TMA and are never copied: the factors beta gam and beta go into the
 // columns of X - I, once per product, and the rows that the identity contributes are added in f32 (a rounded diagonal would be an error
 // common to a whole row of W^ and Uv: 15 % of the error of o, dq and dk).
 template <int DH>
-__global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
+__global__ void __launch_bounds__(PRE_THREADS, DH == 64 ? 4 : 3) delta_prep_tc_kernel(
     const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapV,
     const __grid_constant__ CUtensorMap mapWH, const __grid_constant__ CUtensorMap mapUV, const float* __restrict__ alpha,
     const float* __restrict__ beta, int T, int H, int n_chunks, Tiles out, int* err_word) {
@@ -231,12 +266,12 @@ __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
             tc::tmem_ld_32x32(tmem + ((uint32_t)(wq * 32) << 16) + cg * 32, r);
             const float gt = g_s[t];
 #pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4) {
+            for (int j4 = 0; j4 < 8; ++j4) {   // (every one, also above the diagonal: branches around them cost more)
                 const float4 g4 = *reinterpret_cast<const float4*>(g_s + cg * 32 + 4 * j4);
-                e[4 * j4] = __expf(gt - g4.x);
-                e[4 * j4 + 1] = __expf(gt - g4.y);
-                e[4 * j4 + 2] = __expf(gt - g4.z);
-                e[4 * j4 + 3] = __expf(gt - g4.w);
+                e[4 * j4] = exp_neg(gt - g4.x);
+                e[4 * j4 + 1] = exp_neg(gt - g4.y);
+                e[4 * j4 + 2] = exp_neg(gt - g4.z);
+                e[4 * j4 + 3] = exp_neg(gt - g4.w);
             }
             tc::tmem_ld_wait();
         }
@@ -262,72 +297,71 @@ __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
             for (int j = 0; j < 32; ++j) e[j] -= __bfloat162float(__float2bfloat16(e[j]));
             store32_bf16(out.AL + (tix * 64 + t) * 64 + cg * 32, e, true);
         }
+        if (wq < 2) bar_sync(2, 128);   // the four warps that hold L
+    }
+
+    // ---- X = (I + L)^-1 in f32 on warps 0 - 3, while the others finish. Warps 0 and 1: two diagonal blocks each, one column per lane, and
+    //      the block below them; then warp 2I + J the block (2 + I, J) of the lower left quarter
+    if (warp < 2 && ok) {
+        {
+            const int I = tid >> 4, jj = tid & 15;
+            const float* Lb = Lf + tri(I, I);
+            float x[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) x[t] = t == jj ? 1.0f : 0.0f;
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                float4 l[16];
+#pragma unroll
+                for (int t = 4 * kb + 1; t < 16; ++t) l[t] = *reinterpret_cast<const float4*>(Lb + t * BLD + 4 * kb);
+#pragma unroll
+                for (int t = 4 * kb + 1; t < 16; ++t) x[t] = fmaf(-l[t].x, x[4 * kb], x[t]);
+#pragma unroll
+                for (int t = 4 * kb + 2; t < 16; ++t) x[t] = fmaf(-l[t].y, x[4 * kb + 1], x[t]);
+#pragma unroll
+                for (int t = 4 * kb + 3; t < 16; ++t) x[t] = fmaf(-l[t].z, x[4 * kb + 2], x[t]);
+#pragma unroll
+                for (int t = 4 * kb + 4; t < 16; ++t) x[t] = fmaf(-l[t].w, x[4 * kb + 3], x[t]);
+            }
+#pragma unroll
+            for (int t = 0; t < 16; ++t) Xf[tri(I, I) + t * BLD + jj] = x[t];
+        }
+        __syncwarp();
+        const int tr = lane >> 2, c4 = (lane & 3) * 4;
+        {
+            const int I = 2 * warp + 1, J = 2 * warp;
+            float acc[2][4] = {};
+            tile16(Lf + tri(I, J) + 2 * tr * BLD, Xf + tri(J, J) + c4, acc);
+            put_tile(&Yf[warp * BSZ + 2 * tr * BLD + c4], acc, 1.0f);
+            __syncwarp();
+            tile16(Xf + tri(I, I) + 2 * tr * BLD, Yf + warp * BSZ + c4, acc);
+            put_tile(&Xf[tri(I, J) + 2 * tr * BLD + c4], acc, -1.0f);
+        }
+    }
+    if (warp < 4 && ok) {
+        const int tr = lane >> 2, c4 = (lane & 3) * 4, I = warp >> 1, J = warp & 1;
+        float acc[2][4] = {};
+        bar_sync(1, 128);
+        if (J == 0) tile16(Lf + tri(2 + I, 0) + 2 * tr * BLD, Xf + tri(0, 0) + c4, acc);
+        tile16(Lf + tri(2 + I, 1) + 2 * tr * BLD, Xf + tri(1, J) + c4, acc);
+        put_tile(&Yf[(2 * J + I) * BSZ + 2 * tr * BLD + c4], acc, 1.0f);
+        bar_sync(1, 128);
+        tile16(Xf + tri(2 + I, 2) + 2 * tr * BLD, Yf + 2 * J * BSZ + c4, acc);
+        if (I == 1) tile16(Xf + tri(3, 3) + 2 * tr * BLD, Yf + (2 * J + 1) * BSZ + c4, acc);
+        put_tile(&Xf[tri(2 + I, J) + 2 * tr * BLD + c4], acc, -1.0f);
     }
     tc::tcgen05_fence_before();
     __syncthreads();
-
-    // ---- X = (I + L)^-1 in f32. The four 16 x 16 diagonal blocks, one column per thread; then the block below the diagonal in each
-    //      half (1,0), (3,2); then the lower left quarter as two products over pairs of blocks
-    if (tid < 64) {
-        const int I = tid >> 4, jj = tid & 15;
-        const float* Lb = Lf + tri(I, I);
-        float x[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) x[t] = t == jj ? 1.0f : 0.0f;
-#pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
-            float4 l[16];
-#pragma unroll
-            for (int t = 4 * kb + 1; t < 16; ++t) l[t] = *reinterpret_cast<const float4*>(Lb + t * BLD + 4 * kb);
-#pragma unroll
-            for (int t = 4 * kb + 1; t < 16; ++t) x[t] = fmaf(-l[t].x, x[4 * kb], x[t]);
-#pragma unroll
-            for (int t = 4 * kb + 2; t < 16; ++t) x[t] = fmaf(-l[t].y, x[4 * kb + 1], x[t]);
-#pragma unroll
-            for (int t = 4 * kb + 3; t < 16; ++t) x[t] = fmaf(-l[t].z, x[4 * kb + 2], x[t]);
-#pragma unroll
-            for (int t = 4 * kb + 4; t < 16; ++t) x[t] = fmaf(-l[t].w, x[4 * kb + 3], x[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < 16; ++t) Xf[tri(I, I) + t * BLD + jj] = x[t];
-    }
-    __syncthreads();
-    {
-        const int r = (tid >> 2) & 15, c4 = (tid & 3) * 4;
-        if (tid < 128) {
-            const int I = 2 * (tid >> 6) + 1, J = I - 1;
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            strip16(Lf + tri(I, J) + r * BLD, Xf + tri(J, J) + c4, acc);
-            put4(&Yf[(tid >> 6) * BSZ + r * BLD + c4], acc, 1.0f);
-        }
-        __syncthreads();
-        if (tid < 128) {
-            const int I = 2 * (tid >> 6) + 1, J = I - 1;
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            strip16(Xf + tri(I, I) + r * BLD, Yf + (tid >> 6) * BSZ + c4, acc);
-            put4(&Xf[tri(I, J) + r * BLD + c4], acc, -1.0f);
-        }
-        __syncthreads();
-        const int I = tid >> 7, J = (tid >> 6) & 1;   // block (2 + I, J) of the lower left quarter
-        {
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (J == 0) strip16(Lf + tri(2 + I, 0) + r * BLD, Xf + tri(0, 0) + c4, acc);
-            strip16(Lf + tri(2 + I, 1) + r * BLD, Xf + tri(1, J) + c4, acc);
-            put4(&Yf[(2 * I + J) * BSZ + r * BLD + c4], acc, 1.0f);
-        }
-        __syncthreads();
-        {
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            strip16(Xf + tri(2 + I, 2) + r * BLD, Yf + J * BSZ + c4, acc);
-            if (I == 1) strip16(Xf + tri(3, 3) + r * BLD, Yf + (2 + J) * BSZ + c4, acc);
-            put4(&Xf[tri(2 + I, J) + r * BLD + c4], acc, -1.0f);
-        }
-        __syncthreads();
-    }
     // ---- (X - I) diag(beta gam), (X - I) diag(beta) -> bf16 operand tiles (K-major) and, for the backward, X - I row-major
+    float bg8[8], be8[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        bg8[e] = bg_s[(tid & 7) * 8 + e];
+        be8[e] = be_s[(tid & 7) * 8 + e];
+    }
 #pragma unroll
     for (int it = 0; it < 512 / PRE_THREADS; ++it) {
-        const int idx = tid + it * PRE_THREADS, t = idx >> 3, jc = idx & 7;
+        const int idx = tid + it * PRE_THREADS, t = idx >> 3, jc = tid & 7;
         float x8[8], y8[8];
         if ((jc >> 1) <= (t >> 4)) {
             const float* src = &Xf[tri(t >> 4, jc >> 1) + (t & 15) * BLD + (jc & 1) * 8];
@@ -342,10 +376,10 @@ __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
         for (int e = 0; e < 8; ++e)
             if (jc * 8 + e == t) x8[e] = 0.0f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) y8[e] = x8[e] * bg_s[jc * 8 + e];
+        for (int e = 0; e < 8; ++e) y8[e] = x8[e] * bg8[e];
         *reinterpret_cast<uint4*>(X1_s + tc::sw128_off(t, jc)) = tc::pack8_bf16(y8);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) y8[e] = x8[e] * be_s[jc * 8 + e];
+        for (int e = 0; e < 8; ++e) y8[e] = x8[e] * be8[e];
         *reinterpret_cast<uint4*>(X2_s + tc::sw128_off(t, jc)) = tc::pack8_bf16(y8);
         if (out.TP) *reinterpret_cast<uint4*>(out.TP + (tix * 64 + t) * 64 + jc * 8) = tc::pack8_bf16(x8);
     }
@@ -375,12 +409,13 @@ __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
         const float f = half == 0 ? bg_s[row] : be_s[row];
 #pragma unroll
         for (int cc = 0; cc < DH / 64; ++cc) {
+            const int col = cg * (DH / 2) + cc * 32;
             uint32_t r[32];
-            tc::tmem_ld_32x32(tmem + ((uint32_t)(wq * 32) << 16) + cg * (DH / 2) + cc * 32, r);
+            tc::tmem_ld_32x32(tmem + ((uint32_t)(wq * 32) << 16) + col, r);
             tc::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int c16 = cg * (DH / 16) + cc * 4 + j;
+                const int c16 = (col >> 3) + j;
                 uint4* at = reinterpret_cast<uint4*>((half == 0 ? KQ_s + (c16 >> 3) * 16384 : V_s + (c16 >> 3) * 8192) + tc::sw128_off(row, c16 & 7));
                 float o8[8];
                 tc::unpack8_bf16(*at, o8);
@@ -407,8 +442,9 @@ __global__ void __launch_bounds__(PRE_THREADS, 3) delta_prep_tc_kernel(
 }
 
 // ------------------------------------------------------------------ forward chain
-// Threads: 4 warps per 32 columns of the state (warp w: TMEM lane quarter w & 3, columns 32 (w >> 2) ..), one that loads and issues the
-// products, one that stores operand tiles (its waits for their reading are off the serial path).
+// Threads: 4 warps per 32 columns of the state (warp w: TMEM lane quarter w & 3, columns 32 (w >> 2) ..), one that issues the products
+// and one that moves tiles in and out (a TMA instruction waits for its turn at a busy memory: in the issuing thread's loop twelve of
+// them were a thousand cycles of every chunk).
 // Quarters 0 and 1 hold the 64 rows of U, quarters 2 and 3 those of o; the state's DH rows are all four quarters (DH 128) or 0 and 1.
 template <int DH>
 struct ChainCfg {
@@ -422,14 +458,14 @@ struct ChainCfg {
     static constexpr size_t B_SMEM = 1024 + 2 * B_STAGE + S_BYTES + (DH == 128 ? 16384 : 0) /*dU then dR; at 64 where A was*/ + 2 * 512 + 128;
 };
 
-// What bounds it: at 128 chains the tiles of HBM (136 KB per chunk with a backward to follow, 88 without), at few chains the two
-// products and three register passes of a chunk.
+// What bounds it: at 128 chains HBM (145 KB per chunk with a backward to follow: 5.8 TB/s at 203 us for 64 chunks, 281 before), at few
+// chains the two products and two register passes of a chunk (2.9 us).
 template <int DH>
 __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delta_fwd_tc_kernel(
     const __grid_constant__ CUtensorMap mapWH, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
     const __grid_constant__ CUtensorMap mapUV, const __grid_constant__ CUtensorMap mapAA, const __grid_constant__ CUtensorMap mapAL,
     const __grid_constant__ CUtensorMap mapS0, const __grid_constant__ CUtensorMap mapU, const float* __restrict__ GB, int T, int H, int n_chunks, __nv_bfloat16* __restrict__ o,
-    const float* s_init, float* s_final /* may be s_init */, int keep /* states and U go out */, int* err_word) {
+    const float* s_init, float* s_final /* may be s_init */, int keep /* states and U go out */, int ahead /* L2 prefetch */, int* err_word) {
     using Cfg = ChainCfg<DH>;
     constexpr int NB = Cfg::NB;
     extern __shared__ uint8_t smem_raw[];
@@ -439,8 +475,10 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     auto Ue_s = [&](int s) { return base + s * Cfg::F_STAGE; };              // eg U takes W^'s place: n-boxes 16 KiB apart
     float* gb_s = reinterpret_cast<float*>(S_s + Cfg::S_BYTES);   // [4][128]: loaded with the stages, read two chunks longer
     uint64_t* bars = reinterpret_cast<uint64_t*>(gb_s + 512);
-    uint64_t *full = bars, *mma1_done = bars + 2, *u_ready = bars + 3, *mma2_done = bars + 4, *s_ready = bars + 5, *mma3_done = bars + 6,
-             *o_done = bars + 7, *s_stored = bars + 8, *u_stored = bars + 9;
+    // mma3_done per stage: the moving thread may see it late, and its next phase needs tiles only that thread loads. Every other barrier's
+    // next phase needs an arrival or a product of who waits for it.
+    uint64_t *full = bars, *mma1_done = bars + 2, *u_ready = bars + 3, *mma2_done = bars + 4, *s_ready = bars + 5, *mma3_done = bars + 6 /*[2]*/,
+             *o_done = bars + 8, *s_stored = bars + 9;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -465,25 +503,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     const uint32_t tmem_S = *tmem_slot, tmem_D1 = tmem_S + DH /* two, in turn */, tmem_D2 = tmem_S + 3 * DH;
 
     if (warp == Cfg::COMPUTE / 32) {
-        // ------------------------------------------------------------ TMA loads + MMA issuer (one thread)
+        // ------------------------------------------------------------ MMA issuer (one thread)
         if (lane == 0) {
-            auto load = [&](int c, int s) {
-                uint8_t* st = base + s * Cfg::F_STAGE;
-                const int t = (int)(tile0 + c);
-                tc::mbar_expect_tx(&full[s], Cfg::F_STAGE + 512);
-                load_vec(gb_s + (c & 3) * 128, GB + (int64_t)t * 128, &full[s]);
-#pragma unroll
-                for (int kb = 0; kb < NB; ++kb) {
-                    tc::tma_load_2d(st + kb * 16384, &mapWH, kb * 64, t * 64, &full[s]);
-                    tc::tma_load_3d(st + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, c * C, b, &full[s]);
-                    tc::tma_load_2d(st + Cfg::F_UV + kb * 8192, &mapUV, kb * 64, t * 64, &full[s]);
-                    tc::tma_load_3d(st + Cfg::F_K + kb * 8192, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
-                }
-                tc::tma_load_2d(st + Cfg::F_A, &mapAA, 0, t * 64, &full[s]);
-                tc::tma_load_2d(st + Cfg::F_AL, &mapAL, 0, t * 64, &full[s]);
-            };
-            load(0, 0);
-            if (n_chunks > 1) load(1, 1);
             constexpr uint32_t ID_KM = tc::idesc_bf16_f32(128, DH, 0, 1);   // A K-major, B MN-major
             constexpr uint32_t ID_MM = tc::idesc_bf16_f32(128, DH, 1, 1);   // A MN-major, B MN-major
             const uint32_t s_addr = tc::smem_u32(S_s);
@@ -509,7 +530,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                                   tc::smem_desc_sw128(st + k16 * 2048, 16384, 1024), ID_MM, 1u);
                 tc::umma_commit(mma2_done);
                 // D2 = [.. ; A] U + [.. ; AL] U   (rows 0-63 multiply what lies in front and are not read)
-                if (c > 0 && !tc::mbar_wait(o_done, (c - 1) & 1, abort_flag, err_word, 214)) break;
+                if (!tc::mbar_wait(o_done, c & 1, abort_flag, err_word, 214)) break;
                 tc::tcgen05_fence_after();
 #pragma unroll
                 for (int k16 = 0; k16 < C / 16; ++k16)
@@ -519,32 +540,64 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 for (int k16 = 0; k16 < C / 16; ++k16)
                     tc::umma_bf16(tmem_D2, tc::smem_desc_sw128(st + Cfg::F_A + k16 * 32, 16, 1024),
                                   tc::smem_desc_sw128(st + Cfg::F_UV + k16 * 2048, 8192, 1024), ID_KM, 1u);
-                tc::umma_commit(mma3_done);
-                if (c + 2 < n_chunks) {
-                    if (!tc::mbar_wait(mma3_done, c & 1, abort_flag, err_word, 215)) break;
-                    if (keep && !tc::mbar_wait(u_stored, c & 1, abort_flag, err_word, 216)) break;   // (U lies in the stage)
-                    load(c + 2, s);
-                }
+                tc::umma_commit(&mma3_done[s]);
             }
         }
     } else if (warp > Cfg::COMPUTE / 32) {
-        // ------------------------------------------------------------ state and U out, straight from the operand tiles (one thread)
-        if (lane == 0 && keep) {
+        // ------------------------------------------------------------ everything that moves (one thread): tiles in, state and U out
+        if (lane == 0) {
+            auto load = [&](int c, int s) {
+                uint8_t* st = base + s * Cfg::F_STAGE;
+                const int t = (int)(tile0 + c);
+                tc::mbar_expect_tx(&full[s], Cfg::F_STAGE + 512);
+                load_vec(gb_s + (c & 3) * 128, GB + (int64_t)t * 128, &full[s]);
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) {
+                    tc::tma_load_2d(st + kb * 16384, &mapWH, kb * 64, t * 64, &full[s]);
+                    tc::tma_load_3d(st + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, c * C, b, &full[s]);
+                    tc::tma_load_2d(st + Cfg::F_UV + kb * 8192, &mapUV, kb * 64, t * 64, &full[s]);
+                    tc::tma_load_3d(st + Cfg::F_K + kb * 8192, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
+                }
+                tc::tma_load_2d(st + Cfg::F_A, &mapAA, 0, t * 64, &full[s]);
+                tc::tma_load_2d(st + Cfg::F_AL, &mapAL, 0, t * 64, &full[s]);
+            };
+            // With one chain per SM two stages in flight do not cover the memory's latency: the next chunk's tiles are asked into L2
+            auto prefetch = [&](int c) {
+                if (c >= n_chunks) return;
+                const int t = (int)(tile0 + c);
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) {
+                    tc::tma_prefetch_2d(&mapWH, kb * 64, t * 64);
+                    tc::tma_prefetch_3d(&mapQ, h * DH + kb * 64, c * C, b);
+                    tc::tma_prefetch_2d(&mapUV, kb * 64, t * 64);
+                    tc::tma_prefetch_3d(&mapK, h * DH + kb * 64, c * C, b);
+                }
+                tc::tma_prefetch_2d(&mapAA, 0, t * 64);
+                tc::tma_prefetch_2d(&mapAL, 0, t * 64);
+            };
+            load(0, 0);
+            if (n_chunks > 1) load(1, 1);
+            if (ahead) prefetch(2);
             for (int c = 0; c < n_chunks; ++c) {
-                if (!tc::mbar_wait(s_ready, c & 1, abort_flag, err_word, 217)) break;
+                if (keep) {   // straight from the operand tiles
+                    if (!tc::mbar_wait(s_ready, c & 1, abort_flag, err_word, 215)) break;
 #pragma unroll
-                for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapS0, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
-                tc::bulk_commit_group();
-                if (!tc::mbar_wait(u_ready, c & 1, abort_flag, err_word, 218)) break;
+                    for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapS0, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
+                    tc::bulk_commit_group();
+                    tc::bulk_wait_read();
+                    if (!tc::mbar_wait(u_ready, c & 1, abort_flag, err_word, 216)) break;
+                    tc::mbar_arrive(s_stored);   // (the new state, whose update needs U as well, may take the old one's place)
 #pragma unroll
-                for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapU, U_s(c & 1) + nb * 8192, nb * 64, (int)(tile0 + c) * 64);
-                tc::bulk_commit_group();
-                tc::bulk_wait_read_but_one();
-                tc::mbar_arrive(s_stored);
-                tc::bulk_wait_read();
-                tc::mbar_arrive(u_stored);
+                    for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapU, U_s(c & 1) + nb * 8192, nb * 64, (int)(tile0 + c) * 64);
+                    tc::bulk_commit_group();
+                    tc::bulk_wait_read();
+                }
+                if (c + 2 < n_chunks) {
+                    if (!tc::mbar_wait(&mma3_done[c & 1], (c >> 1) & 1, abort_flag, err_word, 217)) break;
+                    load(c + 2, c & 1);
+                    if (ahead) prefetch(c + 3);
+                }
             }
-            tc::bulk_wait_read();   // before the CTA's shared memory goes
         }
     } else {
         const int wq = warp & 3, cg = warp >> 2, arow = 32 * wq + lane, row = arow & 63;
@@ -566,6 +619,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
             if (lane == 0) tc::mbar_arrive(bar);
         };
         bool ok = warp_wait(&full[0], 0, 220);
+        if (wq >= 2 && lane == 0) tc::mbar_arrive(o_done);   // phase c: D2 and the other D1 are free for chunk c
         if (s_warp && ok) {   // initial state: bf16 operand copy, and f32 scaled by the first chunk's decay
             const float g0 = expf(gb_s[C - 1]);
             const float* si = s_init ? s_init + ((int64_t)chain * DH + arow) * DH + col : nullptr;
@@ -640,7 +694,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
             }
             if (wq >= 2) {
                 // o = gam (Q S) + A U: TMEM lanes 64-127
-                if (!warp_wait(mma3_done, c & 1, 226)) break;
+                if (!warp_wait(&mma3_done[s], (c >> 1) & 1, 226)) break;
                 uint32_t q[32];
                 tc::tmem_ld_32x32(tmem_D1 + s * DH + lane_addr + col, q);
                 tc::tmem_ld_32x32(tmem_D2 + lane_addr + col, r);
@@ -665,14 +719,16 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 
 // ------------------------------------------------------------------ backward chain
 // Same threads as the forward: quarters 0 and 1 hold the 64 rows of dU and dR, quarters 2 and 3 scale the rows of dO by gam in place
-// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO.
+// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO. 170 KB of HBM per chunk
+// (dv in f32 among them) at 3.8 TB/s: 367 us for 64 chunks of 128 chains, three products and their register passes one after another.
+// With the gradients on the same chain a chunk was nine groups of products: 914 us.
 template <int DH>
 __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delta_bwd_tc_kernel(
     const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapDO,
     const __grid_constant__ CUtensorMap mapAA, const __grid_constant__ CUtensorMap mapAL, const __grid_constant__ CUtensorMap mapTP,
     const __grid_constant__ CUtensorMap mapDS,
-    const __grid_constant__ CUtensorMap mapDR, const float* __restrict__ GB, const __nv_bfloat16* __restrict__ v,
-    int T, int H, int n_chunks, float* __restrict__ d_qkv, float* __restrict__ VD /* [tile][NG][64]: v . dv over 32 columns */, int* err_word) {
+    const __grid_constant__ CUtensorMap mapDR, const __grid_constant__ CUtensorMap mapV, const float* __restrict__ GB, const __nv_bfloat16* __restrict__ v,
+    int T, int H, int n_chunks, float* __restrict__ d_qkv, float* __restrict__ VD /* [tile][NG][64]: v . dv over 32 columns */, int ahead, int* err_word) {
     using Cfg = ChainCfg<DH>;
     constexpr int NB = Cfg::NB, NG = Cfg::NG;
     extern __shared__ uint8_t smem_raw[];
@@ -684,9 +740,9 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     auto Rs_s = [&](int s) { return base + s * Cfg::B_STAGE + Cfg::B_RS; };
     float* gb_s = reinterpret_cast<float*>(S_s + Cfg::S_BYTES + (DH == 128 ? 16384 : 0));   // [2][128], with the stages
     uint64_t* bars = reinterpret_cast<uint64_t*>(gb_s + 256);
-    uint64_t *full = bars, *mma0_done = bars + 2, *mma1_done = bars + 3, *mma2_done = bars + 4, *mma3_done = bars + 5, *s_ready = bars + 6,
-             *do_ready = bars + 7, *du_ready = bars + 8, *dr_ready = bars + 9, *s_stored = bars + 10, *r_stored = bars + 11;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+    uint64_t *full = bars, *mma0_done = bars + 2, *mma1_done = bars + 3, *mma2_done = bars + 4, *mma3_done = bars + 5 /*[2], per stage as in the forward*/,
+             *s_ready = bars + 7, *do_ready = bars + 8, *du_ready = bars + 9, *dr_ready = bars + 10, *s_stored = bars + 11, *r_stored = bars + 12;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -697,7 +753,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 12; ++i) {
+        for (int i = 0; i < 13; ++i) {
             const uint64_t* w = bars + i;
             tc::mbar_init(&bars[i], w == s_ready ? Cfg::S_WARPS : w == do_ready || w == du_ready || w == dr_ready ? Cfg::ROW_WARPS : 1);
         }
@@ -711,25 +767,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     const uint32_t tmem_S = *tmem_slot, tmem_D1 = tmem_S + DH, tmem_D2 = tmem_S + 2 * DH;
 
     if (warp == Cfg::COMPUTE / 32) {
-        // ------------------------------------------------------------ TMA loads + MMA issuer (one thread)
+        // ------------------------------------------------------------ MMA issuer (one thread)
         if (lane == 0) {
-            auto load = [&](int it) {
-                const int c = n_chunks - 1 - it, s = it & 1;
-                uint8_t* st = base + s * Cfg::B_STAGE;
-                const int t = (int)(tile0 + c);
-                tc::mbar_expect_tx(&full[s], Cfg::B_STAGE + 512);
-                load_vec(gb_s + s * 128, GB + (int64_t)t * 128, &full[s]);
-#pragma unroll
-                for (int kb = 0; kb < NB; ++kb) tc::tma_load_3d(st + Cfg::B_DO + kb * 8192, &mapDO, h * DH + kb * 64, c * C, b, &full[s]);
-                tc::tma_load_2d(st + Cfg::B_A, &mapAA, 0, t * 64, &full[s]);
-                tc::tma_load_2d(st + Cfg::B_AL, &mapAL, 0, t * 64, &full[s]);
-#pragma unroll
-                for (int kb = 0; kb < NB; ++kb) {
-                    tc::tma_load_3d(st + kb * 16384, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
-                    tc::tma_load_3d(st + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, c * C, b, &full[s]);
-                }
-                tc::tma_load_2d(st + Cfg::B_TP, &mapTP, 0, t * 64, &full[s]);
-            };
             constexpr uint32_t ID_KM = tc::idesc_bf16_f32(128, DH, 0, 1), ID_MM = tc::idesc_bf16_f32(128, DH, 1, 1), ID_MM_NEG = ID_MM | (1u << 13);
             const uint32_t s_addr = tc::smem_u32(S_s);
             // D2 = (A + AL)^T dO of step `it`   (rows 64-127 multiply what lies behind and are not read)
@@ -749,8 +788,6 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 tc::umma_commit(mma0_done);
                 return true;
             };
-            load(0);
-            if (n_chunks > 1) load(1);
             bool ok = mma0(0);
             for (int it = 0; ok && it < n_chunks; ++it) {
                 const int c = n_chunks - 1 - it, par = it & 1;
@@ -786,34 +823,67 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 for (int k16 = 0; k16 < C / 16; ++k16)
                     tc::umma_bf16(tmem_S, tc::smem_desc_sw128(st + k16 * 2048, 16384, 1024),
                                   tc::smem_desc_sw128(rs_addr + k16 * 2048, 8192, 1024), ID_MM_NEG, 1u);
-                tc::umma_commit(mma3_done);
+                tc::umma_commit(&mma3_done[par]);
                 if (!mma0(it + 1)) break;
-                if (it + 2 < n_chunks) {
-                    if (!tc::mbar_wait(mma3_done, par, abort_flag, err_word, 306)) break;
-                    if (DH != 128 && !tc::mbar_wait(r_stored, par, abort_flag, err_word, 309)) break;   // (dR lies in the stage)
-                    load(it + 2);
-                }
             }
         }
     } else if (warp > Cfg::COMPUTE / 32) {
-        // ------------------------------------------------------------ dS at the end of each chunk and dR out (one thread)
+        // ------------------------------------------------------------ everything that moves (one thread): tiles in, dS and dR out
         if (lane == 0) {
+            auto load = [&](int it) {
+                const int c = n_chunks - 1 - it, s = it & 1;
+                uint8_t* st = base + s * Cfg::B_STAGE;
+                const int t = (int)(tile0 + c);
+                tc::mbar_expect_tx(&full[s], Cfg::B_STAGE + 512);
+                load_vec(gb_s + s * 128, GB + (int64_t)t * 128, &full[s]);
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) tc::tma_load_3d(st + Cfg::B_DO + kb * 8192, &mapDO, h * DH + kb * 64, c * C, b, &full[s]);
+                tc::tma_load_2d(st + Cfg::B_A, &mapAA, 0, t * 64, &full[s]);
+                tc::tma_load_2d(st + Cfg::B_AL, &mapAL, 0, t * 64, &full[s]);
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) {
+                    tc::tma_load_3d(st + kb * 16384, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
+                    tc::tma_load_3d(st + kb * 16384 + 8192, &mapQ, h * DH + kb * 64, c * C, b, &full[s]);
+                }
+                tc::tma_load_2d(st + Cfg::B_TP, &mapTP, 0, t * 64, &full[s]);
+            };
+            auto prefetch = [&](int it) {   // into L2, as in the forward; v is read from there by the threads
+                const int c = n_chunks - 1 - it, t = (int)(tile0 + c);
+                if (c < 0) return;
+#pragma unroll
+                for (int kb = 0; kb < NB; ++kb) {
+                    tc::tma_prefetch_3d(&mapDO, h * DH + kb * 64, c * C, b);
+                    tc::tma_prefetch_3d(&mapK, h * DH + kb * 64, c * C, b);
+                    tc::tma_prefetch_3d(&mapQ, h * DH + kb * 64, c * C, b);
+                    tc::tma_prefetch_3d(&mapV, h * DH + kb * 64, c * C, b);
+                }
+                tc::tma_prefetch_2d(&mapAA, 0, t * 64);
+                tc::tma_prefetch_2d(&mapAL, 0, t * 64);
+                tc::tma_prefetch_2d(&mapTP, 0, t * 64);
+            };
+            load(0);
+            if (n_chunks > 1) load(1);
+            if (ahead) prefetch(2);
             for (int it = 0; it < n_chunks; ++it) {
                 const int c = n_chunks - 1 - it, par = it & 1;
-                if (!tc::mbar_wait(s_ready, par, abort_flag, err_word, 307)) break;
+                if (!tc::mbar_wait(s_ready, par, abort_flag, err_word, 306)) break;
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapDS, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
                 tc::bulk_commit_group();
-                if (!tc::mbar_wait(dr_ready, par, abort_flag, err_word, 308)) break;
+                tc::bulk_wait_read();
+                tc::mbar_arrive(s_stored);
+                if (!tc::mbar_wait(dr_ready, par, abort_flag, err_word, 307)) break;
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapDR, R_s(par) + nb * 8192, nb * 64, (int)(tile0 + c) * 64);
                 tc::bulk_commit_group();
-                tc::bulk_wait_read_but_one();
-                tc::mbar_arrive(s_stored);
                 tc::bulk_wait_read();
                 tc::mbar_arrive(r_stored);
+                if (it + 2 < n_chunks) {
+                    if (!tc::mbar_wait(&mma3_done[par], (it >> 1) & 1, abort_flag, err_word, 308)) break;
+                    load(it + 2);
+                    if (ahead) prefetch(it + 3);
+                }
             }
-            tc::bulk_wait_read();   // before the CTA's shared memory goes
         }
     } else {
         const int wq = warp & 3, cg = warp >> 2, arow = 32 * wq + lane, row = arow & 63;
@@ -922,7 +992,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 if (s_warp) {   // dS at the start of the chunk: bf16 operand copy, and f32 scaled by the chunk before's decay
                     const float gC = expf(gb_s[(par ^ 1) * 128 + C - 1]);
                     if (!warp_wait(s_stored, par, 316)) break;
-                    if (!warp_wait(mma3_done, par, 317)) break;
+                    if (!warp_wait(&mma3_done[par], (it >> 1) & 1, 317)) break;
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         uint32_t r[16];
@@ -968,7 +1038,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 }
 
 // ------------------------------------------------------------------ gradients per chunk
-// One CTA per (chunk, chain), two per SM; nothing here depends on another chunk. With S and dS the (bf16) state at the chunk's start
+// One CTA per (chunk, chain), two per SM; nothing here depends on another chunk. 209 KB of HBM a chunk: 395 us for 8192 of 64 x 128
+// (4.3 TB/s; two CTAs per SM are what 103 KB of tiles allow, and one's loads and stores hide the other's register passes). With S and dS the (bf16) state at the chunk's start
 // and gradient at its end:
 //   dL = dR U^T,  dA = dO U^T,  X = dO S^T,  Y = dR S^T,  dW = U dS^T              one group of products, value columns 64 at a time
 //   M = -beta Gam dL (strictly lower),  P = Gam dA (lower);  X *= gam,  Y *= -beta gam   (in TMEM)
@@ -982,9 +1053,12 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 constexpr int GR_THREADS = 256;
 template <int DH>
 struct GradCfg {
-    static constexpr int NB = DH / 64, HB = 3 * 8192 + 2 * DH * 128 /*dO, dR, U, S, dS: one 64-wide box each*/;
-    static constexpr int R_K = 0, R_Q = NB * 8192, R_DO = NB * 16384, R_DR = R_DO + 8192, R_U = R_DR + 8192, R_S = R_U + 8192, R_DS = R_S + DH * 128,
-                         R_END = R_DS + DH * 128, R_M = R_DO, R_P = R_DR;
+    // Value columns are taken 64 at a time. Head dim 128: rows (dR, U, dO) of both halves, S and the first half of dS come at once; what
+    // the first half's products have consumed makes room for the second half of dS, K and Q. Head dim 64: everything at once.
+    static constexpr int NB = DH / 64, SB = DH * 128 /*64 columns of S*/, R_DR = 0, R_U = 8192, R_DO = 16384, R_ROWS = 24576 /*per half*/,
+                         R_S = NB * R_ROWS, R_DS = R_S + SB, R_S1 = R_DS + SB, R_DS1 = R_S,
+                         R_K = DH == 128 ? R_DS : R_DS + SB, R_Q = DH == 128 ? R_DR : R_K + 8192, R_END = DH == 128 ? R_S1 + SB : R_Q + 8192,
+                         R_M = (NB - 1) * R_ROWS + R_DR, R_P = (NB - 1) * R_ROWS + R_DO;
     static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 /*dots*/ + 2 * 64 * 3 /*k.MK, k.Y, k.dW*/ + 64 /*v.dv*/ + 8;
     static constexpr size_t SMEM = 1024 + R_END + NVEC * 4 + 64;
 };
@@ -1003,8 +1077,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     float* g_s = reinterpret_cast<float*>(sm + Cfg::R_END);
     float *be_s = g_s + 64, *al_s = be_s + 64, *nrm_s = al_s + 64 /*q rows, k rows*/, *dot_s = nrm_s + 128 /*[2][128]*/, *mk_s = dot_s + 256 /*[2][64]*/,
           *ky_s = mk_s + 128, *kw_s = ky_s + 128, *vd_s = kw_s + 128, *red_s = vd_s + 64;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(red_s + 8);   // [0] K, Q; [1] a set of value columns; [2] its products; [3] second group
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(red_s + 8);   // tiles: [0], [1] by half, [2] dS's second, [3] K, Q; products: [4], [5] by half, [6] second group
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1018,25 +1092,33 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     const int64_t tix = (int64_t)chain * n_chunks + chunk;
     const bool w32 = (reinterpret_cast<uintptr_t>(d_qkv) & 31) == 0;
 
-    auto load_half = [&](int hv) {
-        const int t = (int)tix;
-        tc::mbar_expect_tx(&bars[1], Cfg::HB);
-        tc::tma_load_2d(sm + Cfg::R_DR, &mapDR, hv * 64, t * 64, &bars[1]);
-        tc::tma_load_2d(sm + Cfg::R_U, &mapU, hv * 64, t * 64, &bars[1]);
-        tc::tma_load_3d(sm + Cfg::R_DO, &mapDO, h * DH + hv * 64, t0, b, &bars[1]);
-        tc::tma_load_2d(sm + Cfg::R_S, &mapS0, hv * 64, t * DH, &bars[1]);
-        tc::tma_load_2d(sm + Cfg::R_DS, &mapDS, hv * 64, t * DH, &bars[1]);
+    auto load_rows = [&](int hv, uint64_t* bar) {
+        tc::tma_load_2d(sm + hv * Cfg::R_ROWS + Cfg::R_DR, &mapDR, hv * 64, (int)tix * 64, bar);
+        tc::tma_load_2d(sm + hv * Cfg::R_ROWS + Cfg::R_U, &mapU, hv * 64, (int)tix * 64, bar);
+        tc::tma_load_3d(sm + hv * Cfg::R_ROWS + Cfg::R_DO, &mapDO, h * DH + hv * 64, t0, b, bar);
+    };
+    auto load_kq = [&] {
+        tc::mbar_expect_tx(&bars[3], NB * 16384);
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) {
+            tc::tma_load_3d(sm + Cfg::R_K + kb * 8192, &mapK, h * DH + kb * 64, t0, b, &bars[3]);
+            tc::tma_load_3d(sm + Cfg::R_Q + kb * 8192, &mapQ, h * DH + kb * 64, t0, b, &bars[3]);
+        }
     };
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 4; ++i) tc::mbar_init(&bars[i], 1);
+        for (int i = 0; i < 7; ++i) tc::mbar_init(&bars[i], 1);
         tc::mbar_fence_init();
-        load_half(0);
-        tc::mbar_expect_tx(&bars[0], NB * 16384);
-#pragma unroll
-        for (int kb = 0; kb < NB; ++kb) {
-            tc::tma_load_3d(sm + Cfg::R_K + kb * 8192, &mapK, h * DH + kb * 64, t0, b, &bars[0]);
-            tc::tma_load_3d(sm + Cfg::R_Q + kb * 8192, &mapQ, h * DH + kb * 64, t0, b, &bars[0]);
+        tc::mbar_expect_tx(&bars[0], Cfg::R_ROWS + 2 * Cfg::SB);
+        load_rows(0, &bars[0]);
+        tc::tma_load_2d(sm + Cfg::R_S, &mapS0, 0, (int)tix * DH, &bars[0]);
+        tc::tma_load_2d(sm + Cfg::R_DS, &mapDS, 0, (int)tix * DH, &bars[0]);
+        if constexpr (DH == 128) {
+            tc::mbar_expect_tx(&bars[1], Cfg::R_ROWS + Cfg::SB);
+            load_rows(1, &bars[1]);
+            tc::tma_load_2d(sm + Cfg::R_S1, &mapS0, 64, (int)tix * DH, &bars[1]);
+        } else {
+            load_kq();
         }
     }
     if (warp == 0) tc::tmem_alloc(tmem_slot, 256);
@@ -1080,72 +1162,90 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
         tc::tcgen05_fence_after();
     };
 
-    // ---- first group, 64 value columns at a time; <S, dS> beside it
-    float sds = 0.0f;
-#pragma unroll 1
-    for (int hv = 0; hv < NB; ++hv) {
-        wait_bar(1, hv & 1);
-        if (tid == 0) {
-            constexpr uint32_t I64 = tc::idesc_bf16_f32(64, 64, 0, 0), IDH = tc::idesc_bf16_f32(64, DH, 0, 0);
+    // ---- first group; <S, dS> beside it
+    constexpr uint32_t I64 = tc::idesc_bf16_f32(64, 64, 0, 0), IDH = tc::idesc_bf16_f32(64, DH, 0, 0);
+    auto group1 = [&](int hv) {
+        const uint32_t rows = hv * Cfg::R_ROWS, s0 = hv == 0 ? Cfg::R_S : Cfg::R_S1;
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) {
-                const uint32_t acc = hv > 0 || k16 > 0;
-                const uint64_t dr = kmaj(Cfg::R_DR, k16), dO = kmaj(Cfg::R_DO, k16), u = kmaj(Cfg::R_U, k16), s0 = kmaj(Cfg::R_S, k16);
-                tc::umma_bf16(ACC_D, dr, u, I64, acc);
-                tc::umma_bf16(ACC_D + H1, dO, u, I64, acc);
-                tc::umma_bf16(ACC_A, dO, s0, IDH, acc);
-                tc::umma_bf16(ACC_A + H1, dr, s0, IDH, acc);
-                if constexpr (DH == 128) {   // keys 0-63 in half 0, 64-127 in half 1
-                    tc::umma_bf16(ACC_W, u, kmaj(Cfg::R_DS, k16), I64, acc);
-                    tc::umma_bf16(ACC_W + H1, u, kmaj(Cfg::R_DS + 8192, k16), I64, acc);
-                } else {
-                    tc::umma_bf16(ACC_W + H1, u, kmaj(Cfg::R_DS, k16), I64, acc);
-                }
+        for (int k16 = 0; k16 < 4; ++k16) {
+            const uint32_t acc = hv > 0 || k16 > 0;
+            const uint64_t dr = kmaj(rows + Cfg::R_DR, k16), dO = kmaj(rows + Cfg::R_DO, k16), u = kmaj(rows + Cfg::R_U, k16);
+            tc::umma_bf16(ACC_D, dr, u, I64, acc);
+            tc::umma_bf16(ACC_D + H1, dO, u, I64, acc);
+            tc::umma_bf16(ACC_A, dO, kmaj(s0, k16), IDH, acc);
+            tc::umma_bf16(ACC_A + H1, dr, kmaj(s0, k16), IDH, acc);
+        }
+    };
+    auto products_dw = [&](int hv) {
+        const uint32_t rows = hv * Cfg::R_ROWS, ds = hv == 0 ? Cfg::R_DS : Cfg::R_DS1;
+#pragma unroll
+        for (int k16 = 0; k16 < 4; ++k16) {
+            const uint32_t acc = hv > 0 || k16 > 0;
+            const uint64_t u = kmaj(rows + Cfg::R_U, k16);
+            if constexpr (DH == 128) {   // keys 0-63 in half 0, 64-127 in half 1
+                tc::umma_bf16(ACC_W, u, kmaj(ds, k16), I64, acc);
+                tc::umma_bf16(ACC_W + H1, u, kmaj(ds + 8192, k16), I64, acc);
+            } else {
+                tc::umma_bf16(ACC_W + H1, u, kmaj(ds, k16), I64, acc);
             }
-            tc::umma_commit(&bars[2]);
         }
+    };
+    float sds = 0.0f;
+    auto dot_sds = [&](uint32_t a, uint32_t d_) {   // (the tiles have one layout: element by element)
 #pragma unroll
-        for (int i = 0; i < DH * 8 / GR_THREADS; ++i) {   // (the tiles have one layout: element by element)
-            float s8[8], d8[8];
-            tc::unpack8_bf16(*reinterpret_cast<const uint4*>(sm + Cfg::R_S + (tid + i * GR_THREADS) * 16), s8);
-            tc::unpack8_bf16(*reinterpret_cast<const uint4*>(sm + Cfg::R_DS + (tid + i * GR_THREADS) * 16), d8);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sds = fmaf(s8[e], d8[e], sds);
-        }
-        if (hv + 1 < NB) {
-            wait_bar(2, hv & 1);
-            __syncthreads();
-            if (tid == 0) {
+        for (int i = 0; i < DH * 8 / GR_THREADS; ++i)
+            sds = dot8(*reinterpret_cast<const uint4*>(sm + a + (tid + i * GR_THREADS) * 16),
+                       *reinterpret_cast<const uint4*>(sm + d_ + (tid + i * GR_THREADS) * 16), sds);
+    };
+    wait_bar(0, 0);
+    if (tid == 0) {
+        group1(0);
+        products_dw(0);
+        tc::umma_commit(&bars[4]);
+    }
+    dot_sds(Cfg::R_S, Cfg::R_DS);
+    if constexpr (DH == 128) {
+        __syncthreads();   // everybody has read the first half of S and dS
+        if (tid == 0) {
+            tc::mbar_wait(&bars[1], 0, abort_flag, err_word, 321);
+            group1(1);
+            tc::umma_commit(&bars[5]);
+            if (tc::mbar_wait(&bars[4], 0, abort_flag, err_word, 324)) {
                 tc::fence_proxy_async_smem();
-                load_half(hv + 1);
+                tc::mbar_expect_tx(&bars[2], Cfg::SB);
+                tc::tma_load_2d(sm + Cfg::R_DS1, &mapDS, 64, (int)tix * DH, &bars[2]);
+                load_kq();
             }
         }
     }
     const float g_row = g_s[row], be_row = be_s[row], gam = __expf(g_row), eg = __expf(g_s[C - 1] - g_row);
-    sds = warp_sum(sds);
-    if (lane == 0) red_s[warp] = sds;
-    wait_bar(2, (NB - 1) & 1);
-    wait_bar(0, 0);
-    // ---- M (half 0) and P (half 1): 32 columns of a row per thread
+    wait_bar(3 + NB, 0);
+    // ---- M (half 0) and P (half 1): 32 columns of a row per thread, where the last dR and dO were
     {
         uint32_t r[32];
         tc::tmem_ld_32x32(ACC_D + lane_addr + cg * 32, r);
         tc::tmem_ld_wait();
         const float f = half == 0 ? -be_row : 1.0f;
-        const int lim = row + half;   // M: i < row; P: i <= row
-        // (the operand tiles lie where dO and dR were: the first group, and every thread's reading of S and dS, are over for this warp;
-        // nobody reads dO or dR outside the products)
+        const int lim = row + half - cg * 32;   // M: i < row; P: i <= row
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float x8[8];
+            const float4 ga = *reinterpret_cast<const float4*>(g_s + cg * 32 + 8 * j), gb = *reinterpret_cast<const float4*>(g_s + cg * 32 + 8 * j + 4);
+            const float g8[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+            // Masked exponentials are skipped one by one at head dim 128 and all taken at 64, where the branches cost more than the
+            // exponentials (64: 264 -> 228 us at 8192 chunks; 128 the other way about: 449 and 411).
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int i = cg * 32 + 8 * j + e;
-                x8[e] = i < lim ? f * __expf(g_row - g_s[i]) * __uint_as_float(r[8 * j + e]) : 0.0f;
-            }
+            for (int e = 0; e < 8; ++e) x8[e] = DH == 64 ? exp_neg(g_row - g8[e]) : 8 * j + e < lim ? __expf(g_row - g8[e]) : 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x8[e] = 8 * j + e < lim ? f * x8[e] * __uint_as_float(r[8 * j + e]) : 0.0f;
             *reinterpret_cast<uint4*>(sm + (half == 0 ? Cfg::R_M : Cfg::R_P) + tc::sw128_off(row, cg * 4 + j)) = tc::pack8_bf16(x8);
         }
     }
+    if constexpr (DH == 128) {
+        wait_bar(2, 0);
+        if (tid == 0) products_dw(1);   // (finished when the second group is)
+    }
+    wait_bar(3, 0);
     // ---- X *= gam, Y *= -beta gam, k . Y
     {
         const float f = half == 0 ? gam : -be_row * gam;
@@ -1192,9 +1292,12 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
                 tc::umma_bf16(ACC_D + H1, mk, kk, IKM64, k16 > 0);
             }
         }
-        tc::umma_commit(&bars[3]);
+        tc::umma_commit(&bars[6]);
     }
-    wait_bar(3, 0);
+    if constexpr (DH == 128) dot_sds(Cfg::R_S1, Cfg::R_DS1);   // (while the products run)
+    sds = warp_sum(sds);
+    if (lane == 0) red_s[warp] = sds;
+    wait_bar(6, 0);
     // ---- dq (half 0) and dk (half 1) before the norm's backward: back to TMEM; row sums
     const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
     {
@@ -1462,7 +1565,7 @@ static int forward_dh(asca_ctx* ctx, const void* q, const void* k, const void* v
     {
         asca_span sp(ctx, "delta_fwd_tc_kernel");
         kern<<<(unsigned)chains, Cfg::THREADS, Cfg::F_SMEM, ctx->stream>>>(mWH, mQ, mK, mUV, mAA, mAL, mS0, mU, t.GB, (int)T, (int)H, (int)n_chunks,
-                                                                           (__nv_bfloat16*)o, s_init, s_final, keep ? 1 : 0, ctx->err_word);
+                                                                           (__nv_bfloat16*)o, s_init, s_final, keep ? 1 : 0, chains <= ctx->sm_count, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     if (keep) {
@@ -1530,9 +1633,9 @@ static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* 
     } else {
         ASCA_TRY((run_prepass<DH>(ctx, q, k, v, alpha, beta, B, T, H, n_chunks, t)));
     }
-    CUtensorMap mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, mS0, mU;
+    CUtensorMap mK, mQ, mV, mDO, mAA, mAL, mTP, mDS, mDR, mS0, mU;
     const char* u_rows = reinterpret_cast<const char*>(ckpt) + (size_t)n_tiles * DH * DH * 2;
-    if (!make_map3(&mK, k, B, T, H * DH) || !make_map3(&mQ, q, B, T, H * DH) || !make_map3(&mDO, d_o, B, T, H * DH) ||
+    if (!make_map3(&mK, k, B, T, H * DH) || !make_map3(&mQ, q, B, T, H * DH) || !make_map3(&mV, v, B, T, H * DH) || !make_map3(&mDO, d_o, B, T, H * DH) ||
         !make_map(&mAA, t.AA, n_tiles * C, C, 64, C) || !make_map(&mAL, t.AL, n_tiles * C, C, 64, C) ||
         !make_map(&mTP, t.TP, n_tiles * C, C, 64, C) ||
         !make_map(&mDS, dS, n_tiles * DH, DH, 64, DH) || !make_map(&mDR, dR, n_tiles * C, DH, 64, C) ||
@@ -1543,8 +1646,8 @@ static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* 
     ASCA_CUDA(ctx, cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::B_SMEM));
     {
         asca_span sp(ctx, "delta_bwd_tc_kernel");
-        chain<<<(unsigned)chains, Cfg::THREADS, Cfg::B_SMEM, ctx->stream>>>(mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, t.GB, (const __nv_bfloat16*)v, (int)T,
-                                                                            (int)H, (int)n_chunks, d_qkv, VD, ctx->err_word);
+        chain<<<(unsigned)chains, Cfg::THREADS, Cfg::B_SMEM, ctx->stream>>>(mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, mV, t.GB, (const __nv_bfloat16*)v, (int)T,
+                                                                            (int)H, (int)n_chunks, d_qkv, VD, chains <= ctx->sm_count, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     auto grad = delta_grad_tc_kernel<DH>;
