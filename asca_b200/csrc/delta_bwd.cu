@@ -635,6 +635,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int rows, int bytes, 
 
 // acc += A B for an M x N output in BT threads' registers, K deep, operands in shared memory (row pitches multiples of 4).
 // Thread (tm, tn) owns columns tn + THR_N j and rows in groups of four (tm + THR_M i where it has fewer than four).
+// 8 x 4 tiles run at two thirds of the FFMA rate (64 x 128 x 128 on one CTA per SM: 12.2 thousand cycles of 8.2); 8 x 8 tiles over lanes that
+// share k, which read a third less shared memory, were no faster (13 - 15), nor were operands read a step ahead or packed pairs of k.
 template <int M, int N>
 struct MM {
     static constexpr int TN = 4, THR_N = N / TN, THR_M = BT / THR_N < M ? BT / THR_N : M, TM = M / THR_M;
@@ -642,11 +644,12 @@ struct MM {
     static_assert(N % 4 == 0 && BT % THR_N == 0 && M % THR_M == 0, "tile shape");
     float acc[TM][TN];
     int tn, tm;
-    bool on;
+    bool on, first;   // first: the one lane of a row that speaks for it
     __device__ __forceinline__ MM() {
         tn = threadIdx.x % THR_N;
         tm = threadIdx.x / THR_N;
         on = tm < THR_M;
+        first = tn == 0;
         clear();
     }
     __device__ __forceinline__ void clear() {
@@ -718,12 +721,23 @@ struct MM {
 #pragma unroll
             for (int j = 0; j < TN; ++j) f(row(i), col(j), acc[i][j]);
     }
-    // the sum over a row's columns of f(row, column, value), in every lane that shares the row (THR_N neighbouring lanes)
+    template <class F>
+    __device__ __forceinline__ void each_index(F f) {   // f(row, column, index of the row, of the column)
+        if (!on) return;
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) f(row(i), col(j), i, j);
+    }
+    // the sum over a row's columns of f(row, column, value, index of the column), in every lane that shares the row (THR_N neighbouring lanes)
     template <class F>
     __device__ __forceinline__ float row_sum(int i, F f) {
         float s = 0.0f;
 #pragma unroll
-        for (int j = 0; j < TN; ++j) s += f(row(i), col(j), acc[i][j]);
+        for (int j = 0; j < TN; ++j) s += f(row(i), col(j), acc[i][j], j);
+        return lanes_sum(s);
+    }
+    __device__ __forceinline__ float lanes_sum(float s) const {
 #pragma unroll
         for (int m = THR_N / 2; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
         return s;
@@ -781,7 +795,7 @@ struct PreSmem {
 };
 
 template <int DH, typename T>
-__global__ void __launch_bounds__(BT) delta_bwd_pre_kernel(const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ alpha,
+__global__ void __launch_bounds__(BT, DH == 128 ? 1 : DH == 64 ? 2 : 3) delta_bwd_pre_kernel(const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ alpha,
                                                            const float* __restrict__ beta, const T* __restrict__ d_o,
                                                            float* __restrict__ scratch, int Tlen, int H, const Range range) {
     using SC = ChunkScratch<DH>;
@@ -893,7 +907,7 @@ struct ChainSmem {
 };
 
 template <int DH, int W, typename T>
-__global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict__ k, float* __restrict__ scratch, float* __restrict__ carry,
+__global__ void __launch_bounds__(BT, DH >= 64 ? 1 : 2) delta_bwd_chain_kernel(const T* __restrict__ k, float* __restrict__ scratch, float* __restrict__ carry,
                                                              int Tlen, int H, const Range range, int last) {
     using SC = ChunkScratch<DH>;
     using SM = ChainSmem<DH, W>;
@@ -954,14 +968,25 @@ __global__ void __launch_bounds__(BT) delta_bwd_chain_kernel(const T* __restrict
     }
 }
 
+// x / n for a row's common n and its reciprocal: one Newton step on the quotient, as close as a division; the plain quotient where the step
+// is not finite (n zero or infinite, or an overflow)
+__device__ __forceinline__ float div_row(float x, float n, float inv) {
+    const float q = x * inv, e = fmaf(-n, q, x);
+    return fabsf(e) < INFINITY ? fmaf(e, inv, q) : q;
+}
+
 template <int DH>
 struct GradSmem {
     static constexpr int LD = DH + 4;
     static constexpr size_t bytes = (size_t)(4 * CC * LD + DH * LD + CC * LX + 8 * CC + 8 * CC + 64) * 4 + sizeof(ChunkGates);
 };
 
+// 7.35 M multiply-adds per chunk at head dim 128, where one CTA fills an SM and may use every register. Of its 127 thousand cycles 93 are
+// products at two thirds of the FFMA rate; what it reads beside them (A, LG, dS, norms) is asked for ahead of a product, since eight warps
+// wait for each such load (171 thousand cycles, 4.78 -> 3.69 ms for 8192 chunks; launched together with L2 requests for the CTA
+// that follows on the SM: 4.6).
 template <int DH, typename T>
-__global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
+__global__ void __launch_bounds__(BT, DH == 128 ? 1 : DH == 64 ? 2 : 3) delta_bwd_grad_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ alpha,
     const float* __restrict__ beta, const float* __restrict__ qnorm, const float* __restrict__ knorm, const T* __restrict__ d_o,
     const float* __restrict__ ckpt, const float* __restrict__ scratch, int Tlen, int H, int n_ck, const Range range,
@@ -971,7 +996,8 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
     extern __shared__ __align__(16) float smem[];
     float *Ks = smem, *Bs = Ks + CC * LD /* V, Z, then dO, then Q */, *Us = Bs + CC * LD, *Zs = Us + CC * LD /* dZ */, *Ss = Zs + CC * LD /* S0, then dS */,
           *Xs = Ss + DH * LD /* T, then dA Gam, then M + M^T */, *col_part = Xs + CC * LX, *vec = col_part + 8 * CC, *red = vec + 8 * CC;
-    float *row_p = vec, *col_p = vec + CC, *r_qs = vec + 2 * CC, *r_kg = vec + 3 * CC, *r_kw = vec + 4 * CC, *dbe = vec + 5 * CC;
+    float *row_p = vec, *col_p = vec + CC, *r_qs = vec + 2 * CC, *r_kg = vec + 3 * CC, *r_kw = vec + 4 * CC, *dbe = vec + 5 * CC,
+          *nq_s = vec + 6 * CC, *nk_s = vec + 7 * CC;
     ChunkGates& gt = *reinterpret_cast<ChunkGates*>(red + 64);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ck = range.ck0 + blockIdx.x, chain = range.chain0 + blockIdx.y, bi = chain / H,
               h = chain % H, d = H * DH;
@@ -984,27 +1010,32 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
     load_tile<T, CC, DH>(v, row0, d, h * DH, n, Bs, LD);
     load_tile<float, CC, DH>(in + SC::D, 0, DH, 0, CC, Zs, LD);
     load_tile<float, CC, CC>(in + SC::T, 0, CC, 0, CC, Xs, LX);
+    if (tid < 2 * CC) {
+        const int t = tid & (CC - 1);
+        (tid < CC ? nq_s : nk_s)[t] = t < n ? (tid < CC ? qnorm : knorm)[(row0 + t) * H + h] : 1.0f;
+    }
+    load_gates(alpha, beta, row0, n, H, h, gt);
+    tile_wait();
     // what comes into these buffers later is on its way to L2
     prefetch_l2(in + SC::A, 1, 2 * CC * CC * 4, 0);
     prefetch_l2(in + SC::Y, 1, DH * DH * 4, 0);
     prefetch_l2(d_o + row0 * d + h * DH, n, DH * (int)sizeof(T), (int64_t)d * sizeof(T));
     prefetch_l2(q + row0 * d + h * DH, n, DH * (int)sizeof(T), (int64_t)d * sizeof(T));
-    load_gates(alpha, beta, row0, n, H, h, gt);
-    tile_wait();
     using MD = MM<CC, DH>;
+    using MX = MM<CC, CC>;
     {   // Z = V - gam K S0 (beta Z is what U wants), dZ.Z; dV = dZ goes out
         MD m;
         m.template mul<DH, L_MK, L_KN>(Ks, LD, Ss, LD);
 #pragma unroll
         for (int i = 0; i < MD::TM; ++i) {
             const int t = m.row(i);
-            const float s = m.row_sum(i, [&](int tt, int c, float& x) {
+            const float s = m.row_sum(i, [&](int tt, int c, float& x, int j) {
                 const float z = Bs[tt * LD + c] - gt.gam[tt] * x, dz = Zs[tt * LD + c];
                 Bs[tt * LD + c] = gt.be[tt] * z;
                 if (tt < n) d_qkv[(row0 + tt) * 3 * d + 2 * d + h * DH + c] = dz;
                 return z * dz;
             });
-            if (m.tn == 0) dbe[t] = s;
+            if (m.first) dbe[t] = s;
         }
     }
     __syncthreads();
@@ -1018,20 +1049,18 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
     tile_wait();
     // a C x C matrix of products P = e(acc) o other: row sums and column sums in a fixed order
     auto sums = [&](auto& m, auto f, bool first) {
-        using MX = MM<CC, CC>;
-        float cp[MX::TN] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float cp[MX::TN] = {};
 #pragma unroll
         for (int i = 0; i < MX::TM; ++i) {
             float p[MX::TN], s = 0.0f;
 #pragma unroll
             for (int j = 0; j < MX::TN; ++j) {
-                p[j] = f(m.row(i), m.col(j), m.acc[i][j]);
+                p[j] = f(m.row(i), m.col(j), m.acc[i][j], i, j);
                 cp[j] += p[j];
                 s += p[j];
             }
-#pragma unroll
-            for (int o = MX::THR_N / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (m.tn == 0) {
+            s = m.lanes_sum(s);
+            if (m.first) {
                 if (first) row_p[m.row(i)] = s;
                 else {
                     row_p[m.row(i)] += s;
@@ -1053,11 +1082,13 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
         }
     };
     {   // dA Gam
-        MM<CC, CC> m;
+        MX m;
+        float a[MX::TM][MX::TN];   // A, asked for ahead of the product
+        m.each_index([&](int t, int i, int ti, int tj) { a[ti][tj] = in[SC::A + t * CC + i]; });
         m.template mul<DH, L_MK, L_NK>(Bs, LD, Us, LD);
-        sums(m, [&](int t, int i, float x) {
+        sums(m, [&](int t, int i, float x, int ti, int tj) {
             Xs[t * LX + i] = i <= t ? expf(gt.g[t] - gt.g[i]) * x : 0.0f;
-            return i <= t ? x * in[SC::A + t * CC + i] : 0.0f;
+            return i <= t ? x * a[ti][tj] : 0.0f;
         }, true);
     }
     {   // dQ = gam dO S0^T + (dA Gam) K, L2-norm backward, out
@@ -1067,58 +1098,60 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
 #pragma unroll
         for (int i = 0; i < MD::TM; ++i) {
             const int t = m.row(i);
-            const float s = m.row_sum(i, [&](int tt, int c, float& x) {
+            const float s = m.row_sum(i, [&](int tt, int c, float& x, int j) {
                 x *= gt.gam[tt];
-                return x * (qv[i][(c - m.tn) / MD::THR_N] = tt < n ? to_f32<T>(q[(row0 + tt) * d + h * DH + c]) : 0.0f);
+                return x * (qv[i][j] = tt < n ? to_f32<T>(q[(row0 + tt) * d + h * DH + c]) : 0.0f);
             });
-            if (m.tn == 0) r_qs[t] = s;
+            if (m.first) r_qs[t] = s;
         }
         __syncthreads();   // dA Gam is in place
         m.template mul<CC, L_MK, L_KN>(Xs, LX, Ks, LD);
 #pragma unroll
         for (int i = 0; i < MD::TM; ++i) {
             const int t = m.row(i);
-            const float s = m.row_sum(i, [&](int, int c, float x) { return x * qv[i][(c - m.tn) / MD::THR_N]; });
+            const float s = m.row_sum(i, [&](int, int, float x, int j) { return x * qv[i][j]; });
             if (t < n) {
-                const float nq = qnorm[(row0 + t) * H + h];
+                const float nq = nq_s[t], inv = 1.0f / nq;
 #pragma unroll
-                for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + h * DH + m.col(j)] = (m.acc[i][j] - qv[i][j] * s) / nq;
+                for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + h * DH + m.col(j)] = div_row(m.acc[i][j] - qv[i][j] * s, nq, inv);
             }
         }
     }
+    constexpr int IT = (DH * DH / 4 + BT - 1) / BT, BATCH = IT < 8 ? IT : 8;
+    float4 ds[BATCH];   // dS; the first batch is asked for ahead of the product
+    auto ask = [&](int i0) {
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int idx = tid + (i0 + i) * BT;
+            ds[i] = idx < DH * DH / 4 ? *reinterpret_cast<const float4*>(in + SC::Y + idx * 4) : make_float4(0, 0, 0, 0);
+        }
+    };
+    ask(0);
     MD dk;   // dK = -gam dZ S0^T + eg U dS^T + (dA Gam)^T Q + (M + M^T) K
     dk.template mul<DH, L_MK, L_NK>(Zs, LD, Ss, LD);
 #pragma unroll
     for (int i = 0; i < MD::TM; ++i) {
         const int t = dk.row(i);
-        const float s = dk.row_sum(i, [&](int tt, int c, float& x) {
+        const float s = dk.row_sum(i, [&](int tt, int c, float& x, int j) {
             x *= -gt.gam[tt];
             return x * Ks[tt * LD + c];
         });
-        if (dk.tn == 0) r_kg[t] = s;
+        if (dk.first) r_kg[t] = s;
     }
     __syncthreads();   // S0 and dO are done with
     load_tile<T, CC, DH>(q, row0, d, h * DH, n, Bs, LD);
     float part = 0.0f;   // <S0, dS>
-    {
-        constexpr int IT = (DH * DH / 4 + BT - 1) / BT, BATCH = IT < 8 ? IT : 8;
 #pragma unroll
-        for (int i0 = 0; i0 < IT; i0 += BATCH) {
-            float4 b[BATCH];
+    for (int i0 = 0; i0 < IT; i0 += BATCH) {
+        if (i0) ask(i0);
 #pragma unroll
-            for (int i = 0; i < BATCH; ++i) {
-                const int idx = tid + (i0 + i) * BT;
-                b[i] = idx < DH * DH / 4 ? *reinterpret_cast<const float4*>(in + SC::Y + idx * 4) : make_float4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int i = 0; i < BATCH; ++i) {
-                const int idx = tid + (i0 + i) * BT;
-                if (idx >= DH * DH / 4) continue;
-                float4* at = reinterpret_cast<float4*>(Ss + idx / (DH / 4) * LD + idx % (DH / 4) * 4);
-                const float4 a = *at;
-                part = fmaf(a.x, b[i].x, part); part = fmaf(a.y, b[i].y, part); part = fmaf(a.z, b[i].z, part); part = fmaf(a.w, b[i].w, part);
-                *at = b[i];
-            }
+        for (int i = 0; i < BATCH; ++i) {
+            const int idx = tid + (i0 + i) * BT;
+            if (idx >= DH * DH / 4) continue;
+            float4* at = reinterpret_cast<float4*>(Ss + idx / (DH / 4) * LD + idx % (DH / 4) * 4);
+            const float4 a = *at;
+            part = fmaf(a.x, ds[i].x, part); part = fmaf(a.y, ds[i].y, part); part = fmaf(a.z, ds[i].z, part); part = fmaf(a.w, ds[i].w, part);
+            *at = ds[i];
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -1129,24 +1162,26 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
 #pragma unroll
         for (int i = 0; i < MD::TM; ++i) {
             const int t = m.row(i);
-            const float s = m.row_sum(i, [&](int tt, int c, float& x) {
+            const float s = m.row_sum(i, [&](int tt, int c, float& x, int j) {
                 x *= gt.eg[tt];
                 return x * Ks[tt * LD + c];
             });
-            if (m.tn == 0) r_kw[t] = s;
+            if (m.first) r_kw[t] = s;
 #pragma unroll
             for (int j = 0; j < MD::TN; ++j) dk.acc[i][j] += m.acc[i][j];
         }
     }
     dk.template mul<CC, L_KM, L_KN>(Xs, LX, Bs, LD);
     {
-        MM<CC, CC> m;   // dZ U^T
+        MX m;   // dZ U^T
+        float lg[MX::TM][MX::TN];
+        m.each_index([&](int t, int i, int ti, int tj) { lg[ti][tj] = in[SC::LG + t * CC + i]; });
         m.template mul<DH, L_MK, L_NK>(Zs, LD, Us, LD);
         __syncthreads();   // every reader of dA Gam is done
         m.each([&](int t, int i, float x) {
             if (i <= t) Xs[t * LX + i] = i < t ? -expf(gt.g[t] - gt.g[i]) * x : 0.0f;   // M
         });
-        sums(m, [&](int t, int i, float x) { return i < t ? -x * in[SC::LG + t * CC + i] : 0.0f; }, false);   // (holds a barrier)
+        sums(m, [&](int t, int i, float x, int ti, int tj) { return i < t ? -x * lg[ti][tj] : 0.0f; }, false);   // (holds a barrier)
     }
     for (int idx = tid; idx < CC * CC; idx += BT) {   // M + M^T: the upper triangle is the mirror of the lower
         const int t = idx / CC, i = idx % CC;
@@ -1157,11 +1192,11 @@ __global__ void __launch_bounds__(BT) delta_bwd_grad_kernel(
 #pragma unroll
     for (int i = 0; i < MD::TM; ++i) {
         const int t = dk.row(i);
-        const float s = dk.row_sum(i, [&](int tt, int c, float x) { return x * Ks[tt * LD + c]; });
+        const float s = dk.row_sum(i, [&](int tt, int c, float x, int) { return x * Ks[tt * LD + c]; });
         if (t < n) {
-            const float nk = knorm[(row0 + t) * H + h];
+            const float nk = nk_s[t], inv = 1.0f / nk;
 #pragma unroll
-            for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + d + h * DH + dk.col(j)] = (dk.acc[i][j] - Ks[t * LD + dk.col(j)] * s) / nk;
+            for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + d + h * DH + dk.col(j)] = div_row(dk.acc[i][j] - Ks[t * LD + dk.col(j)] * s, nk, inv);
         }
     }
     // gates: dg, its suffix sums (two steps a lane), sigmoid backward

@@ -695,3 +695,31 @@ def test_delta_tc_sequences_do_not_mix(gpu, B, T, H, dh):
     for got_, ref in zip(want, (flat(o64), S, d64, g64)):
         ref = ref.detach()
         assert (got_.double() - ref).norm() < 8e-3 * ref.norm()
+
+
+# f32 delta backward: a row's gradients are divided by its norm through the reciprocal; zero, infinite and tiny norms behave as a division.
+@pytest.mark.parametrize("dh", [32, 64, 128])
+def test_delta_f32_norm_division_at_its_edges(gpu, dh):
+    import torch
+    from asca_b200 import ops
+
+    B, T, H = 1, 70, 2
+    g = torch.Generator(device="cuda").manual_seed(dh)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, H, dh, generator=g, device="cuda"), dim=-1).reshape(T, H * dh) for _ in range(2))
+    v, d_o = (torch.randn(T, H * dh, generator=g, device="cuda") for _ in range(2))
+    al, be = (torch.sigmoid(torch.randn(T, H, generator=g, device="cuda")) for _ in range(2))
+    one = torch.ones(T, H, device="cuda")
+    _, _, ck = ops.delta_fwd(gpu, q, k, v, al, be, B, T, H, dh)
+    want, want_g = ops.delta_bwd(gpu, q, k, v, al, be, one, one, d_o, ck, B, T, H, dh)
+    norm = 10.0 ** torch.empty(T, H, device="cuda").uniform_(-30, 30, generator=g)
+    norm[3], norm[5], norm[66] = 0.0, float("inf"), 3.0
+    got, got_g = ops.delta_bwd(gpu, q, k, v, al, be, norm, norm, d_o, ck, B, T, H, dh)
+    gpu.sync()
+    assert torch.equal(got_g, want_g)
+    for part in range(2):
+        a, w = (x.view(T, 3, H, dh)[:, part] for x in (got, want))
+        w = w / norm[..., None]
+        fin = torch.isfinite(w)
+        assert torch.equal(fin, torch.isfinite(a)) and torch.equal(torch.isnan(a), torch.isnan(w))
+        # one rounding of the quotient on each side; denormal results on the spacing of denormals
+        assert ((a - w)[fin].abs() <= 2 ** -22 * w[fin].abs() + 2 ** -148).all()
