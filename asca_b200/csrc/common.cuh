@@ -112,18 +112,31 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Launches `kern` on the context's stream; with ctx->pdl set, as a programmatic dependent of the previous kernel.
 // Only for kernels whose every thread calls pdl_wait() before its first global memory access.
 template <typename... KArgs, typename... Args>
-inline cudaError_t asca_launch(asca_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+inline cudaError_t asca_launch_cluster(asca_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (ctx->pdl) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = ctx->pdl ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t asca_launch(asca_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+    return asca_launch_cluster(ctx, kern, grid, block, smem, 1, args...);
 }
 #endif
 // Small host arrays through the context's pinned staging area (a call that uses it ends with asca_ctx_sync, or

@@ -14,6 +14,10 @@
 // at a time through shared memory, so that global memory sees 16-byte accesses with 8 lanes on each token's
 // 128 bytes. Bias, SiLU (bf16 second output), accumulation and the row map of the MoE combine are applied there.
 //
+// With few tiles a tile's k range is shared by the S CTAs of a cluster (S = 2 or 4), since one SM draws
+// at most about its share of the memory rate. Each epilogue warp's quarter of a tile (32 features) has one CTA that finishes it; the
+// others write their sums into a slot of its shared memory and arrive on its barrier, and it adds them in rank order.
+//
 // Every mbarrier wait is bounded; a wait that runs out raises the error word and the CTA frees its TMEM and exits.
 #include "gemm_tc.cuh"
 
@@ -27,14 +31,17 @@ constexpr int BF = 128, BK = 64, THREADS = 192;
 constexpr int W_BYTES = BF * BK * 2;
 constexpr int SK_MAX_GROUPS = 512;
 
-template <int NT, int ST> struct SkShape {
-    static constexpr int STAGES = ST;                          // 10 x 20 KiB (NT 32) or 8 x 24 KiB (NT 64): one CTA per SM
+template <int NT, int ST, int S> struct SkShape {
+    static constexpr int STAGES = ST;                          // 10 (9 with a k split) x 20 KiB (NT 32) or 8 x 24 KiB (NT 64): one CTA per SM
+    static constexpr int SLOT = 32 * NT * 4;                   // a quarter of a tile from another CTA, [token][32 features]
+    static constexpr int PEERS = S - 1, QUARTERS = S == 2 ? 2 : 1;   // others that add to a tile; quarters finished here at most
+    static constexpr int SLOT_BYTES = S > 1 ? PEERS * QUARTERS * SLOT : 0;
     static constexpr int X_BYTES = NT * BK * 2;
     static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;      // 20 / 24 KiB: every stage starts 1024-byte aligned
     static constexpr int TMEM_COLS = 2 * NT;                   // two accumulator buffers
     static constexpr int CTAS_PER_SM = ST * STAGE_BYTES <= 102 * 1024 ? 2 : 1;
-    static constexpr size_t SMEM_FIXED = (size_t)STAGES * STAGE_BYTES + 4 * 2048 /*epilogue staging*/ + 1024 /*alignment slack*/ +
-                                         256 /*barriers*/;
+    static constexpr size_t SMEM_FIXED = (size_t)STAGES * STAGE_BYTES + SLOT_BYTES + 4 * 2048 /*epilogue staging*/ + 1024 /*alignment slack*/ +
+                                         384 /*barriers*/;
 };
 
 struct SkP {
@@ -59,19 +66,46 @@ struct SkP {
 
 __device__ __forceinline__ float sk_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
-template <int NT, int ST>
-__global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_skinny_kernel(const __grid_constant__ CUtensorMap mapW,
+// Waits whose arrivals come with data from another CTA of the cluster
+__device__ __forceinline__ bool wait_peers(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err_word, int code) {
+    const long long t0 = clock64();
+    while (true) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(tc::smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > tc::WAIT_LIMIT_CYCLES) {
+            *abort_flag = 1;
+            if (err_word) atomicExch(err_word, code);
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ void arrive_peer(uint64_t* bar, uint32_t rank) {   // releases what this thread has seen, to the cluster
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tc::mapa_u32(tc::smem_u32(bar), rank)) : "memory");
+}
+
+template <int NT, int ST, int S>
+__global__ void __launch_bounds__(THREADS, SkShape<NT, ST, S>::CTAS_PER_SM) gemm_skinny_kernel(const __grid_constant__ CUtensorMap mapW,
                                                                                        const __grid_constant__ CUtensorMap mapX,
                                                                                        const SkP p) {
-    constexpr int STAGES = ST, STAGE_BYTES = SkShape<NT, ST>::STAGE_BYTES, TMEM_COLS = SkShape<NT, ST>::TMEM_COLS;
+    using Shape = SkShape<NT, ST, S>;
+    constexpr int STAGES = ST, STAGE_BYTES = Shape::STAGE_BYTES, TMEM_COLS = Shape::TMEM_COLS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* staging = tiles + STAGES * STAGE_BYTES;                 // 4 epilogue warps x 2 KiB
-    uint64_t* full = reinterpret_cast<uint64_t*>(staging + 4 * 2048);
+    uint8_t* slots = staging + 4 * 2048;
+    uint64_t* full = reinterpret_cast<uint64_t*>(slots + Shape::SLOT_BYTES);
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* peer_full = acc_empty + 2;    // [4] by quarter: the others' sums are in the slots
+    uint64_t* peer_empty = peer_full + 4;   // [4]: the slot this CTA's quarter goes to has been read
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_empty + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* prefix = const_cast<int*>(abort_flag) + 1;   // [n_groups + 1] first tile of every group
 
@@ -90,6 +124,12 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(&acc_full[b], 1);
             tc::mbar_init(&acc_empty[b], 4);
+        }
+        if (S > 1) {
+            for (int q = 0; q < 4; ++q) {
+                tc::mbar_init(&peer_full[q], Shape::PEERS);
+                tc::mbar_init(&peer_empty[q], 1);
+            }
         }
         tc::mbar_fence_init();
         tc::prefetch_tensormap(&mapW);
@@ -121,9 +161,14 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
     tc::tcgen05_fence_before();
     __syncthreads();
     tc::tcgen05_fence_after();
+    if (S > 1) tc::cluster_sync_all();   // every CTA's barriers exist
     pdl_launch_dependents();   // after this CTA holds its TMEM: a dependent that becomes resident early cannot take it
     const uint32_t tmem_base = *tmem_slot;
     const int total_tiles = prefix[n_groups];
+
+    // this CTA's tiles, and its k-tiles of each
+    const int rank = S > 1 ? (int)tc::cluster_ctarank() : 0, t0 = blockIdx.x / S, t_step = gridDim.x / S;
+    const int k_lo = num_k * rank / S, k_hi = num_k * (rank + 1) / S;
 
     struct Tile {
         int g, f0, row0, rows, w_in, w_out;   // row0: first memory row of the token tile; rows: live tokens in it
@@ -170,17 +215,17 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
             // running (this CTA is resident early under programmatic dependent launch); the tokens follow after the wait.
             uint32_t n_pre = 0;
             if (p.early) {
-                for (int t = blockIdx.x; t < total_tiles && n_pre < STAGES; t += gridDim.x) {
+                for (int t = t0; t < total_tiles && n_pre < STAGES; t += t_step) {
                     const Tile x = locate(t);
-                    for (int kt = 0; kt < num_k && n_pre < STAGES; ++kt, ++n_pre) load_w(x, kt, n_pre);
+                    for (int kt = k_lo; kt < k_hi && n_pre < STAGES; ++kt, ++n_pre) load_w(x, kt, n_pre);
                 }
                 pdl_wait();
             }
             uint32_t it = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+            for (int t = t0; t < total_tiles && ok; t += t_step) {
                 const Tile x = locate(t);
-                for (int kt = 0; kt < num_k; ++kt, ++it) {
+                for (int kt = k_lo; kt < k_hi; ++kt, ++it) {
                     const int s = it % STAGES;
                     if (it >= n_pre) {
                         if (it >= STAGES && !tc::mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag, p.err_word, 111)) {
@@ -205,12 +250,12 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
             bool ok = true;
             uint32_t it = 0;
             int tl = 0;
-            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tl) {
+            for (int t = t0; t < total_tiles && ok; t += t_step, ++tl) {
                 const int buf = tl & 1;
                 const uint32_t tmem_acc = tmem_base + buf * NT;
                 if (tl >= 2) ok = tc::mbar_wait(&acc_empty[buf], ((tl >> 1) - 1) & 1, abort_flag, p.err_word, 114);
                 tc::tcgen05_fence_after();
-                for (int kt = 0; kt < num_k && ok; ++kt, ++it) {
+                for (int kt = k_lo; kt < k_hi && ok; ++kt, ++it) {
                     const uint32_t s = it % STAGES;
                     ok = tc::mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, p.err_word, 112);
                     if (!ok) break;
@@ -219,9 +264,9 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
 #pragma unroll
                     for (int k16 = 0; k16 < BK / 16; ++k16)
                         tc::umma_bf16(tmem_acc, ((uint64_t)DESC_HI << 32) | (w_lo + k16 * W_K16),
-                                      ((uint64_t)DESC_HI << 32) | (x_lo + k16 * X_K16), IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
+                                      ((uint64_t)DESC_HI << 32) | (x_lo + k16 * X_K16), IDESC, (kt > k_lo || k16 > 0) ? 1u : 0u);
                     tc::umma_commit(&empty[s]);
-                    if (kt == num_k - 1) tc::umma_commit(&acc_full[buf]);
+                    if (kt == k_hi - 1) tc::umma_commit(&acc_full[buf]);
                 }
             }
         }
@@ -237,11 +282,40 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
         const bool vec_c = p.C && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
         const bool vec_c2 = p.C2 && (p.ldc2 & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C2) & 7) == 0;
         bool ok = true;
+        const int owner = S == 4 ? q : S == 2 ? q >> 1 : 0;   // who finishes this quarter
         int tl = 0;
-        for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tl) {
+        for (int t = t0; t < total_tiles && ok; t += t_step, ++tl) {
             const Tile x = locate(t);
-            const int buf = tl & 1;
+            const int buf = tl & 1, phase = (tl >> 1) & 1;
             const uint32_t tmem_acc = tmem_base + buf * NT;
+            if (S > 1 && owner != rank) {   // this quarter is finished elsewhere: the sums go to its slot there
+                int got = 0;
+                if (lane == 0)
+                    got = tc::mbar_wait(&acc_full[buf], phase, abort_flag, p.err_word, 113) &&
+                          (tl == 0 || wait_peers(&peer_empty[q], (tl - 1) & 1, abort_flag, p.err_word, 115)) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, got, 0) != 0;
+                if (!ok) break;
+                tc::tcgen05_fence_after();
+                const int slot = S == 2 ? q & 1 : rank - (rank > owner);
+                const uint32_t at = tc::mapa_u32(tc::smem_u32(slots + slot * Shape::SLOT), owner) + lane * 4;
+#pragma unroll 1
+                for (int c = 0; c < NT / 16; ++c) {
+                    uint32_t r[16];
+                    tc::tmem_ld_32x16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), r);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e)
+                        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(at + (c * 16 + e) * 128), "r"(r[e]) : "memory");
+                }
+                tc::tcgen05_fence_before();
+                asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    tc::mbar_arrive(&acc_empty[buf]);
+                    arrive_peer(&peer_full[q], owner);
+                }
+                continue;
+            }
             const int fb = x.f0 + q * 32 + col4 * 4;   // this lane's first feature in the store phase
             const bool full4 = fb + 4 <= p.N;
             float b4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -252,9 +326,11 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
                     if (fb + e < p.N) b4[e] = bias[fb + e];
             }
             int got = 0;
-            if (lane == 0) got = tc::mbar_wait(&acc_full[buf], (tl >> 1) & 1, abort_flag, p.err_word, 113) ? 1 : 0;
+            if (lane == 0) got = tc::mbar_wait(&acc_full[buf], phase, abort_flag, p.err_word, 113) ? 1 : 0;
+            if (S > 1 && got) got = wait_peers(&peer_full[q], tl & 1, abort_flag, p.err_word, 116) ? 1 : 0;   // (lane 0 alone)
             ok = __shfl_sync(0xffffffffu, got, 0) != 0;
             if (!ok) break;
+            if (S > 1) asm volatile("fence.acq_rel.cluster;" ::: "memory");
             tc::tcgen05_fence_after();
 #pragma unroll 1
             for (int c = 0; c < NT / 16; ++c) {
@@ -280,6 +356,14 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
                     const int rr = 4 * i + rsub;
                     rows_m[i] = __shfl_sync(0xffffffffu, my_row, rr);
                     acc4[i] = *reinterpret_cast<const float4*>(stg + rr * 32 + col4 * 4);
+                    if (S > 1) {
+#pragma unroll
+                        for (int o = 0; o < Shape::PEERS; ++o) {
+                            const int slot = S == 2 ? q & 1 : o;
+                            const float4 v = *reinterpret_cast<const float4*>(slots + slot * Shape::SLOT + (c * 16 + rr) * 128 + col4 * 16);
+                            acc4[i].x += v.x; acc4[i].y += v.y; acc4[i].z += v.z; acc4[i].w += v.w;
+                        }
+                    }
                     old4[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     if (p.accumulate && p.C && rows_m[i] >= 0 && fb < p.N) {
                         const float* crow = p.C + (int64_t)rows_m[i] * p.ldc + fb;
@@ -326,12 +410,17 @@ __global__ void __launch_bounds__(THREADS, SkShape<NT, ST>::CTAS_PER_SM) gemm_sk
                 }
                 __syncwarp();   // every lane is done with the staging rows before the next pass overwrites them
             }
+            if (S > 1 && lane == 0) {   // the slots may be written for the next tile
+                for (int o = 0; o < S; ++o)
+                    if (o != rank) arrive_peer(&peer_empty[q], o);
+            }
         }
     }
     // ---- teardown
     tc::tcgen05_fence_before();
     __syncthreads();
     if (*abort_flag) __nanosleep(20000);   // let copies already in flight land before the CTA exits
+    if (S > 1) tc::cluster_sync_all();     // nobody writes to this CTA's shared memory any more
     if (warp == 1) tc::tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
@@ -390,7 +479,7 @@ bool sk_make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, i
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int NT, int ST>
+template <int NT, int ST, int S = 1>
 int sk_launch_shape(asca_ctx* ctx, const Args& a, int64_t tiles) {
     CUtensorMap mapW, mapX;
     const bool w_ok = a.b_packed ? sk_make_map(&mapW, a.B, a.b_rows, 64, 64, 64, 128) : sk_make_map(&mapW, a.B, a.b_rows, a.b_cols, a.ldb, 64, 64);
@@ -405,15 +494,28 @@ int sk_launch_shape(asca_ctx* ctx, const Args& a, int64_t tiles) {
     p.w_packed = a.b_packed;
     p.early = a.b_early;
     p.err_word = ctx->err_word;
+    using Shape = SkShape<NT, ST, S>;
     const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
-    const int64_t grid = std::min<int64_t>(tiles, (int64_t)n_sm * SkShape<NT, ST>::CTAS_PER_SM);
-    const size_t smem = SkShape<NT, ST>::SMEM_FIXED + (size_t)((p.grouped ? a.n_groups : 1) + 2) * 4;
-    auto kern = gemm_skinny_kernel<NT, ST>;
-    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(SkShape<NT, ST>::SMEM_FIXED + (SK_MAX_GROUPS + 2) * 4)));
-    ASCA_CUDA(ctx, asca_launch(ctx, kern, dim3((unsigned)grid), dim3(THREADS), smem, mapW, mapX, p));
+    const size_t smem = Shape::SMEM_FIXED + (size_t)((p.grouped ? a.n_groups : 1) + 2) * 4;
+    auto kern = gemm_skinny_kernel<NT, ST, S>;
+    ASCA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(Shape::SMEM_FIXED + (SK_MAX_GROUPS + 2) * 4)));
+    const int64_t grid = std::min<int64_t>(tiles, (int64_t)n_sm * Shape::CTAS_PER_SM / S) * S;
+    ASCA_CUDA(ctx, asca_launch_cluster(ctx, kern, dim3((unsigned)grid), dim3(THREADS), smem, S, mapW, mapX, p));
     ctx->launches++;
     return ASCA_OK;
+}
+
+// CTAs that share a tile's k range in an expert product: as many as the SMs that would have no tile allow, each with three k-tiles at least.
+// The tiles are taken as one token tile for every group that can have a row (their number is known on the device only). 768 -> 3072 -> 768 with 16
+// experts, us a decode step of 12 blocks without and with it: 1 stream 536 / 447, 5 573 / 493, 12 672 / 641; from 24 streams on
+// the second product has its 96 tiles and nothing is shared. Measured and not taken: eight CTAs (1 stream 454, 3 streams 597 / 508
+// with four), three CTAs for two tiles (256 streams 941 / 1150: three SMs of one GPC are rarely free at once), and the dense
+// products of the same step (12 streams 641 / 646, 40 706 / 721: their time is not the stream of weights).
+int sk_split(asca_ctx* ctx, const Args& a, int64_t tiles_f) {
+    const int64_t n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148, tiles = std::min<int64_t>(a.n_groups, a.total_rows) * tiles_f, num_k = (a.K + BK - 1) / BK;
+    if (tiles * 4 <= n_sm && num_k >= 12) return 4;
+    if (tiles * 2 <= n_sm && num_k >= 6) return 2;
+    return 1;
 }
 
 }  // namespace
@@ -439,13 +541,18 @@ int launch_skinny(asca_ctx* ctx, const Args& a) {
                  2.0 * (double)a.K * (double)a.N * (a.group_dim == GROUP_NONE ? 1.0 : (double)a.n_groups));
     // One CTA per SM with the whole shared memory as its ring: a CTA's k-loop is one latency-bound stream, and what
     // keeps HBM busy is the bytes in flight per SM (10 stages of 20 KiB, or 8 of 24 KiB).
+    const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
     if (a.group_dim == GROUP_NONE) {
-        const int n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148;
         // token tiles of 32 while they still fit one wave: more CTAs streaming, and 10 of a tile's k-tiles in its ring
         if (a.M <= 32 || ((a.M + 31) / 32) * tiles_f <= n_sm) return sk_launch_shape<32, 10>(ctx, a, ((a.M + 31) / 32) * tiles_f);
         return sk_launch_shape<64, 8>(ctx, a, ((a.M + 63) / 64) * tiles_f);
     }
-    return sk_launch_shape<32, 10>(ctx, a, (a.total_rows / 32 + a.n_groups) * tiles_f);
+    const int64_t most = (a.total_rows / 32 + a.n_groups) * tiles_f;
+    switch (sk_split(ctx, a, tiles_f)) {
+        case 4: return sk_launch_shape<32, 9, 4>(ctx, a, most);
+        case 2: return sk_launch_shape<32, 9, 2>(ctx, a, most);
+        default: return sk_launch_shape<32, 10>(ctx, a, most);
+    }
 }
 
 // Rows of a packed weight buffer (64 bf16 each) for `groups` matrices of K x N.

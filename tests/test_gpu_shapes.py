@@ -723,3 +723,32 @@ def test_delta_f32_norm_division_at_its_edges(gpu, dh):
         assert torch.equal(fin, torch.isfinite(a)) and torch.equal(torch.isnan(a), torch.isnan(w))
         # one rounding of the quotient on each side; denormal results on the spacing of denormals
         assert ((a - w)[fin].abs() <= 2 ** -22 * w[fin].abs() + 2 ** -148).all()
+
+
+# Expert products of a few tokens, whose k range two or four CTAs share: odd numbers of k-tiles, experts without tokens and with more than
+# one token tile (several tiles a cluster), and just past the rule; against f64 sums over the hidden rows as they were stored.
+@pytest.mark.parametrize("tokens,experts,d,F", [(1, 16, 768, 3072), (3, 16, 768, 3072), (12, 16, 768, 3072), (13, 16, 768, 3072), (70, 2, 128, 1664), (300, 6, 64, 832), (200, 40, 64, 448)])
+def test_few_tokens_per_expert_with_a_shared_k_range(gpu, tokens, experts, d, F):
+    import torch
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+
+    def norm(*s, scale=1.0):
+        return torch.randn(*s, generator=g, device="cuda") * scale
+
+    xn, w1, w2 = norm(tokens, d).bfloat16(), norm(d, experts * F, scale=d ** -0.5).bfloat16(), norm(experts * F, d, scale=F ** -0.5).bfloat16()
+    b1, b2 = norm(experts * F), norm(d)
+    ids = torch.randint(0, 256, (tokens,), generator=g, device="cuda", dtype=torch.int32)
+    perm, offs = ops.moe_dispatch(gpu, ids, experts)
+    out, _, hid = ops.moe_fwd(gpu, xn, w1, b1, w2, b2, perm, offs, F, experts)
+    out2, _, _ = ops.moe_fwd(gpu, xn, w1, b1, w2, b2, perm, offs, F, experts)
+    gpu.sync()
+    assert torch.equal(out, out2)
+    route = torch.repeat_interleave(torch.arange(experts, device="cuda"), (offs[1:] - offs[:-1]).long())
+    want = torch.empty(tokens, d, dtype=torch.float64, device="cuda")
+    for e in range(experts):
+        rows = (route == e).nonzero().flatten()
+        if len(rows):   # from the hidden rows as they were stored (bf16)
+            want[perm[rows].long()] = hid[rows].double() @ w2[e * F:(e + 1) * F].double() + b2.double()
+    assert (out - want).abs().max() < 4e-6 * F ** 0.5
