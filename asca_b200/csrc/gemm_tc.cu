@@ -64,7 +64,7 @@ struct KP {
     int64_t ldc;
     int M, N, K;
     const float* bias;
-    int accumulate;
+    const float* old;                  // added to the product, rows and pitch like C's (C itself where it accumulates); null: nothing
     const int32_t* c_idx;
     const int32_t* offsets;
     int n_groups, group_dim;
@@ -75,7 +75,7 @@ struct KP {
     int64_t ldaux;
     __nv_bfloat16* C2;
     int64_t ldc2;
-    int c2_only;
+    int c2_only, c2_mapped;
     __nv_bfloat16 *qkv_q, *qkv_k, *qkv_v;
     float *qkv_qn, *qkv_kn;
     int qkv_d, qkv_dh;
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             const uintptr_t a = reinterpret_cast<uintptr_t>(base) | (uintptr_t)(ld * unit) | (uintptr_t)(gstride * unit);
             return (a & 31) == 0 ? 8 : (a & 15) == 0 ? 4 : 1;
         };
-        const int c_w = width(p.C, p.ldc, p.group_dim == GROUP_K ? p.c_gstride : 0, 4);
+        const int c_w = min(width(p.C, p.ldc, p.group_dim == GROUP_K ? p.c_gstride : 0, 4), width(p.old, 0, 0, 4));
         const int aux_w = width(p.aux, p.ldaux, 0, 4);
         const int bias_w = width(p.bias, 0, p.bias_gstride, 4);
         const int c2_w = width(p.C2, p.ldc2, 0, 2);
@@ -540,12 +540,16 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             const bool live = x.M - (x.m0 + q * 32) > lane;   // rows past the matrix's or the expert's end are computed, not stored
             const int64_t lr = (int64_t)x.row_base_m + x.m0 + (live ? q * 32 + lane : 0);
             const int64_t cr = p.c_idx && live ? (int64_t)p.c_idx[lr] : lr;
-            float* crow = p.C + (p.group_dim == GROUP_K ? (int64_t)x.g * p.c_gstride : 0) + cr * p.ldc + x.n0;
+            const int64_t c_off = (p.group_dim == GROUP_K ? (int64_t)x.g * p.c_gstride : 0) + cr * p.ldc + x.n0;
+            float* crow = p.C + c_off;
+            const float* orow = p.old + c_off;
             const float* arow = p.aux + lr * p.ldaux + x.n0;
             const float* brow = p.bias ? p.bias + (int64_t)x.g * p.bias_gstride + x.n0 : nullptr;
-            // aux, or where there is none the old C, ahead of their use
-            const float* prow = with_aux ? arow : crow;
-            const bool ahead = live && (with_aux || p.accumulate);
+            // aux, or where there is none the rows to add, ahead of their use (an add of the residual here, with the bf16 copy the
+            // next block reads, hides behind the next tile's instructions: a prefill of 14,448 tokens x 12 blocks took 6.06 ms with
+            // the adds in passes of their own, 5.92 with them here; a training step of 8,192 x 2048 15.95 and 15.82 ms)
+            const float* prow = with_aux ? arow : orow;
+            const bool ahead = live && (with_aux || p.old);
             const int p_w = with_aux ? aux_w : c_w;
             constexpr int AHEAD = PAIR && !EW8 ? 2 : 1;   // (registers: 255 with four epilogue warps, 168 with eight)
             float pre[AHEAD][32];
@@ -565,7 +569,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             // fused qkv epilogue (pair shape): this warp's 128 columns are one head of q, k or v, or two of 64
             const bool qkv = PAIR && EW8 && p.epi == EPI_QKV;
             float qkv_scale[2] = {1.0f, 1.0f};      // 1 / max(|z|, 1e-8) of this lane's row (q, k), 1 for v; per 64 columns
-            __nv_bfloat16* hrow = p.C2 + lr * p.ldc2 + x.n0;
+            __nv_bfloat16* hrow = p.C2 + (p.c2_mapped ? cr : lr) * p.ldc2 + x.n0;
             if (qkv) {
                 const int hc0 = x.n0 + c_lo * 32;   // first column of the head
                 const int sec = hc0 / p.qkv_d;      // 0 q, 1 k, 2 v
@@ -677,13 +681,13 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                 if (with_aux) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] *= silu_grad_f(pre[i % AHEAD][j]);
-                    if (p.accumulate && live) {
+                    if (p.old && live) {
                         float old[32];
-                        load_row(old, crow + c * 32, n_left, c_w);
+                        load_row(old, orow + c * 32, n_left, c_w);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] += old[j];
                     }
-                } else if (p.accumulate) {
+                } else if (p.old) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] += pre[i % AHEAD][j];
                 }
@@ -755,7 +759,8 @@ bool supported(const Args& a) {
     if (a.group_dim == GROUP_K && a.mode != ASCA_TN) return false;
     if (a.group_dim == GROUP_M && a.mode == ASCA_TN) return false;
     if (a.c2_only && (!a.C2 || a.accumulate || (a.epi != EPI_NONE && a.epi != EPI_SILU && a.epi != EPI_SILU_BWD) || a.c_idx || skinny_wanted(a))) return false;
-    if ((a.c2_mapped || a.b_packed) && !skinny_wanted(a)) return false;
+    if (a.b_packed && !skinny_wanted(a)) return false;
+    if (a.res && (!a.accumulate || a.group_dim == GROUP_K || skinny_wanted(a))) return false;
     return true;
 }
 
@@ -770,11 +775,11 @@ static int launch_shape(asca_ctx* ctx, const Args& a, int64_t grid) {
     if (!ok) return asca_fail(ctx, ASCA_ERR_CUDA, "gemm_tc: cuTensorMapEncodeTiled failed");
     KP p{};
     p.C = a.C; p.ldc = a.ldc; p.M = a.M; p.N = a.N; p.K = a.K;
-    p.bias = a.bias; p.accumulate = a.accumulate; p.c_idx = a.c_idx;
+    p.bias = a.bias; p.old = a.accumulate ? (a.res ? a.res : a.C) : nullptr; p.c_idx = a.c_idx;
     p.offsets = a.offsets; p.n_groups = a.n_groups; p.group_dim = a.group_dim;
     p.b_goff_inner = a.b_goff_inner; p.b_goff_outer = a.b_goff_outer;
     p.c_gstride = a.c_gstride; p.bias_gstride = a.bias_gstride;
-    p.epi = a.epi; p.aux = a.aux; p.ldaux = a.ldaux; p.C2 = a.C2; p.ldc2 = a.ldc2; p.c2_only = a.c2_only;
+    p.epi = a.epi; p.aux = a.aux; p.ldaux = a.ldaux; p.C2 = a.C2; p.ldc2 = a.ldc2; p.c2_only = a.c2_only; p.c2_mapped = a.c2_mapped;
     p.ce_targets = a.ce_targets; p.ce_loss = a.ce_loss; p.ce_scale = a.ce_scale;
     p.qkv_q = a.qkv_q; p.qkv_k = a.qkv_k; p.qkv_v = a.qkv_v; p.qkv_qn = a.qkv_qn; p.qkv_kn = a.qkv_kn; p.qkv_d = a.qkv_d; p.qkv_dh = a.qkv_dh;
     p.err_word = ctx->err_word;

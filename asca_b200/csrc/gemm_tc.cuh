@@ -27,6 +27,7 @@ struct Args {
     int M, N, K;              // per-group problem (GROUP_M: M ignored, GROUP_K: K ignored)
     const float* bias;        // per output column, nullable
     int accumulate;
+    const float* res;         // row-tiled kernel: the rows that accumulate adds, laid out and mapped like C's; null: C itself
     const int32_t* c_idx;     // optional logical-row -> memory-row map for C
     // grouping
     const int32_t* offsets;   // device, n_groups + 1
@@ -43,7 +44,7 @@ struct Args {
     int64_t ldc2;
     int c2_only;              // row-tiled kernel, EPI_NONE, EPI_SILU or EPI_SILU_BWD, no accumulate: the result is wanted as bf16 only (C is
                               // not written and may be null)
-    int c2_mapped;            // few-row kernel only: C2's rows go through c_idx like C's
+    int c2_mapped;            // C2's rows go through c_idx like C's
     int b_packed;             // few-row kernel only: B is a buffer made by skinny_pack (b_rows = its rows of 64)
     __nv_bfloat16 *qkv_q, *qkv_k, *qkv_v;   // EPI_QKV outputs (rows x qkv_d, bf16)
     float *qkv_qn, *qkv_kn;                 // EPI_QKV: norms (rows x qkv_d / qkv_dh)

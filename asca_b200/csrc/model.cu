@@ -383,9 +383,9 @@ bool asca_tc_enabled();  // gemm.cu
 int asca_rmsnorm_bwd_add_cast(asca_ctx* ctx, const float* x, const float* dy, const float* add, float* dx, void* dx16, int64_t rows,
                               int64_t cols, float eps);
 // moe.cu
-int asca_moe_fwd_bf16_nopre(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1, const __nv_bfloat16* w2, const float* b2,
-                            const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, float* out,
-                            __nv_bfloat16* hid_p);
+int asca_moe_fwd_bf16_residual(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1, const __nv_bfloat16* w2, const float* b2,
+                               const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, const float* res, float* out,
+                               __nv_bfloat16* out16, float* pre_p, __nv_bfloat16* hid_p);
 // moe.cu / mixed.cu: the decode-step forms on rows in expert order
 int asca_moe_fwd_sorted_residual(asca_ctx* ctx, const __nv_bfloat16* xp, const __nv_bfloat16* w1, const float* b1,
                                  const __nv_bfloat16* w2, const float* b2, const int32_t* perm, const int32_t* offsets, int64_t N,
@@ -853,6 +853,20 @@ static int materialize_zero_grads(asca_ctx* ctx, asca_model* m) {
 // recurrent state, the loss, the gradients and the master weights stay f32; what a product reads
 // is bf16 (weights from a bf16 copy of the master buffer, activations written as bf16 by the
 // kernel that produces them or by a cast pass).
+
+// out = res + o W_o + b_o in the product's epilogue; ASCA_ERR_UNSUPPORTED, nothing launched, where the row-tiled kernel does not
+// take the product (the caller then adds in a pass of its own)
+static int product_onto_bf16(asca_ctx* ctx, int64_t rows, int64_t d, const __nv_bfloat16* o, const __nv_bfloat16* w_o, const float* b_o,
+                             const float* res, float* out) {
+    gemm_tc::Args t{};
+    t.mode = ASCA_NN; t.A = o; t.lda = d; t.a_rows = rows; t.a_cols = d;
+    t.B = w_o; t.ldb = d; t.b_rows = d; t.b_cols = d;
+    t.C = out; t.ldc = d; t.M = (int)rows; t.N = (int)d; t.K = (int)d;
+    t.bias = b_o; t.accumulate = 1; t.res = res;
+    t.group_dim = gemm_tc::GROUP_NONE; t.epi = gemm_tc::EPI_NONE;
+    return asca_tc_enabled() && gemm_tc::supported(t) ? gemm_tc::launch(ctx, t) : ASCA_ERR_UNSUPPORTED;
+}
+
 static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* ids_h, const uint32_t* tg_h, int64_t B,
                                  int64_t T, float* loss_h, float* logits_h) {
     typedef __nv_bfloat16 bf16;
@@ -886,9 +900,8 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
     float* x = bf.f(N * d);
     float* qkv = nullptr;   // only where the projection's epilogue does not write q, k and v itself
     float* gate = bf.f(N * 2 * H);
-    float* y = bf.f(N * d);
-    float* mo = bf.f(N * d);
-    ASCA_REQUIRE(ctx, x && gate && y && mo, "model_forward_backward: out of memory");
+    float *y = nullptr, *mo = nullptr;   // only where a product's epilogue does not add the residual itself
+    ASCA_REQUIRE(ctx, x && gate, "model_forward_backward: out of memory");
     ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, x));
     const bool vec4 = (d & 3) == 0;
     const unsigned add_grid = (unsigned)std::min<int64_t>(ceil_div64(N * d / 4, 256), 148 * 16);
@@ -924,23 +937,37 @@ static int forward_backward_bf16(asca_ctx* ctx, asca_model* m, const uint32_t* i
             ASCA_TRY(asca_delta_prep_bf16(ctx, qkv, gate, N, H, dh, a.q, a.k, a.v, a.qn, a.kn, a.al, a.be));
         }
         ASCA_TRY(asca_delta_fwd(ctx, a.q, a.k, a.v, a.al, a.be, B, T, H, dh, CH, BF, a.o, nullptr, nullptr, a.ckpt));
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, d, d, a.o, d, W + w16.w_o, d, y, d, P + w.b_o, 0, BF));
-        ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, y, a.x_mid, a.xn, N, d, 1e-6f));
+        int rc = product_onto_bf16(ctx, N, d, a.o, W + w16.w_o, P + w.b_o, x, a.x_mid);
+        if (rc == ASCA_OK) {
+            ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, a.x_mid, nullptr, nullptr, a.xn, N, d, 1e-6f));
+        } else if (rc == ASCA_ERR_UNSUPPORTED) {
+            if (!y) y = bf.f(N * d);
+            ASCA_REQUIRE(ctx, y, "model_forward_backward: out of memory");
+            ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, d, d, a.o, d, W + w16.w_o, d, y, d, P + w.b_o, 0, BF));
+            ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, y, a.x_mid, a.xn, N, d, 1e-6f));
+        } else {
+            return rc;
+        }
         ASCA_TRY(asca_dp_before_expert_weights(ctx, m, li));
-        ASCA_TRY(asca_moe_fwd(ctx, a.xn, W + w16.w1, P + w.b1, W + w16.w2, P + w.b2, perm, offs, N, d, F, E, BF, mo, a.pre_p,
-                              a.hid_p));
-        if (li + 1 < L && vec4) {   // x_out = x_mid + moe, with the bf16 copy the next block's products read
+        // x_out = x_mid + moe, with the bf16 copy the next block's products read
+        if (li + 1 < L) {
             next_x_in = h16(N * d);
             ASCA_REQUIRE(ctx, next_x_in, "model_forward_backward: out of memory");
+        }
+        rc = asca_moe_fwd_bf16_residual(ctx, a.xn, W + w16.w1, P + w.b1, W + w16.w2, P + w.b2, perm, offs, N, d, F, E, a.x_mid, x,
+                                        li + 1 < L ? next_x_in : nullptr, a.pre_p, a.hid_p);
+        if (rc == ASCA_OK) continue;
+        if (rc != ASCA_ERR_UNSUPPORTED) return rc;
+        if (!mo) mo = bf.f(N * d);
+        ASCA_REQUIRE(ctx, mo, "model_forward_backward: out of memory");
+        ASCA_TRY(asca_moe_fwd(ctx, a.xn, W + w16.w1, P + w.b1, W + w16.w2, P + w.b2, perm, offs, N, d, F, E, BF, mo, a.pre_p,
+                              a.hid_p));
+        if (li + 1 < L && vec4) {
             add_cast4_kernel<<<add_grid, 256, 0, ctx->stream>>>(a.x_mid, mo, x, next_x_in, N * d / 4);
             ASCA_CHECK_LAUNCH(ctx);
         } else {
             ASCA_TRY(asca_residual_rmsnorm(ctx, a.x_mid, mo, x, nullptr, N, d, 1e-6f));
-            if (li + 1 < L) {
-                next_x_in = h16(N * d);
-                ASCA_REQUIRE(ctx, next_x_in, "model_forward_backward: out of memory");
-                ASCA_TRY(asca_cast_bf16(ctx, x, next_x_in, N * d));
-            }
+            if (li + 1 < L) ASCA_TRY(asca_cast_bf16(ctx, x, next_x_in, N * d));
         }
     }
     bf16* h_final = h16(N * d);
@@ -1631,14 +1658,16 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     int32_t* offs = (int32_t*)bf.f(E + 1);
     int32_t* last = (int32_t*)bf.f(ns);
     uint32_t* nxt = (uint32_t*)bf.f(ns);
-    float *x = bf.f(N * d), *gate = bf.f(N * 2 * H), *y = bf.f(N * d), *x_mid = bf.f(N * d), *mo = bf.f(N * d);
+    float *x = bf.f(N * d), *gate = bf.f(N * 2 * H);
+    // bf16 mode adds onto x in place, the attention's and mostly the experts' rows in the products' epilogues
+    float *y = bfm ? nullptr : bf.f(N * d), *x_mid = bfm ? x : bf.f(N * d), *mo = bfm ? nullptr : bf.f(N * d);
     float *qn = bf.f(N * H), *kn = bf.f(N * H), *al = bf.f(N * H), *be = bf.f(N * H), *qkv = nullptr, *pre_p = nullptr;   // (two where they are needed)
     float *xl = bf.f(ns * d), *hf = bf.f(ns * d), *logits = bf.f(ns * V);
     // activations a product reads: bf16 in bf16 mode, f32 otherwise (same element counts)
     auto act = [&](int64_t n) { return bfm ? (void*)h16(n) : (void*)bf.f(n); };
     void *x_in = bfm ? act(N * d) : nullptr, *q = act(N * d), *k = act(N * d), *v = act(N * d), *o = act(N * d), *xn = act(N * d),
          *hid_p = act(N * F), *hf_in = bfm ? act(ns * d) : nullptr;
-    ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && gate && y && x_mid && mo && qn && kn && al && be &&
+    ASCA_REQUIRE(ctx, ids && perm && offs && last && nxt && x && gate && x_mid && (bfm || (y && mo)) && qn && kn && al && be &&
                           xl && hf && logits && q && k && v && o && xn && hid_p && (!bfm || (x_in && hf_in)),
                  "model_prefill: out of memory");
     asca_stage_scope staged(ctx);
@@ -1649,12 +1678,11 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
     ASCA_TRY(asca_moe_dispatch(ctx, ids, N, E, perm, offs, nullptr));
     ASCA_TRY(asca_embed_fwd(ctx, P + m->embed, ids, N, d, x));
     const size_t st_layer = (size_t)ns * H * dh * dh;
-    const bool join = bfm && N * d % 4 == 0;   // the residual add also writes the next block's bf16 input
     for (int64_t li = 0; li < L; ++li) {
         const Lyr& w = m->lay[li];
         const Lyr& w16 = m->lay16[li];
         const void* xi = bfm ? x_in : (const void*)x;
-        if (bfm && (li == 0 || !join)) ASCA_TRY(asca_cast_bf16(ctx, x, x_in, N * d));
+        if (bfm && li == 0) ASCA_TRY(asca_cast_bf16(ctx, x, x_in, N * d));   // later blocks: written with the residual add below
         const void *Wqkv = bfm ? (const void*)(W + w16.w_qkv) : (const void*)(P + w.w_qkv), *Wg = bfm ? (const void*)(W + w16.w_gate) : (const void*)(P + w.w_gate),
                    *Wo = bfm ? (const void*)(W + w16.w_o) : (const void*)(P + w.w_o), *W1 = bfm ? (const void*)(W + w16.w1) : (const void*)(P + w.w1),
                    *W2 = bfm ? (const void*)(W + w16.w2) : (const void*)(P + w.w2);
@@ -1681,19 +1709,21 @@ int asca_model_prefill_host(asca_ctx* ctx, asca_model* m, float* state, const ui
         else ASCA_TRY(asca_delta_prep(ctx, qkv, gate, N, H, dh, (float*)q, (float*)k, (float*)v, qn, kn, al, be));
         float* st = state + (size_t)li * st_layer;
         ASCA_TRY(asca_delta_fwd(ctx, q, k, v, al, be, ns, T, H, dh, 64, DT, o, st, st, nullptr));   // (in place: a CTA's own part)
-        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, d, d, o, d, Wo, d, y, d, P + w.b_o, 0, DT));
-        if (bfm) ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, y, x_mid, xn, N, d, 1e-6f));
+        ASCA_TRY(asca_gemm(ctx, ASCA_NN, N, d, d, o, d, Wo, d, bfm ? x : y, d, P + w.b_o, bfm ? 1 : 0, DT));
+        if (bfm) ASCA_TRY(asca_residual_rmsnorm_bf16(ctx, x, nullptr, nullptr, xn, N, d, 1e-6f));
         else ASCA_TRY(asca_residual_rmsnorm(ctx, x, y, x_mid, (float*)xn, N, d, 1e-6f));
-        int rc = bfm ? asca_moe_fwd_bf16_nopre(ctx, (const bf16*)xn, (const bf16*)W1, P + w.b1, (const bf16*)W2, P + w.b2, perm, offs, N, d, F, E, mo,
-                                               (bf16*)hid_p)
+        int rc = bfm ? asca_moe_fwd_bf16_residual(ctx, (const bf16*)xn, (const bf16*)W1, P + w.b1, (const bf16*)W2, P + w.b2, perm, offs, N, d, F, E, x, x,
+                                                  (bf16*)x_in, nullptr, (bf16*)hid_p)
                      : ASCA_ERR_UNSUPPORTED;
+        if (rc == ASCA_OK) continue;
         if (rc == ASCA_ERR_UNSUPPORTED) {
             if (!pre_p) pre_p = bf.f(N * F);
-            ASCA_REQUIRE(ctx, pre_p, "model_prefill: out of memory");
+            if (!mo) mo = bf.f(N * d);
+            ASCA_REQUIRE(ctx, pre_p && mo, "model_prefill: out of memory");
             rc = asca_moe_fwd(ctx, xn, W1, P + w.b1, W2, P + w.b2, perm, offs, N, d, F, E, DT, mo, pre_p, hid_p);
         }
         ASCA_TRY(rc);
-        if (join) {
+        if (bfm) {   // (d % 4 == 0: the norm above takes no other width)
             add_cast4_kernel<<<(unsigned)std::min<int64_t>(ceil_div64(N * d / 4, 256), 148 * 8), 256, 0, ctx->stream>>>(x_mid, mo, x, (bf16*)x_in, N * d / 4);
             ASCA_CHECK_LAUNCH(ctx);
         } else {

@@ -175,9 +175,10 @@ inline bool tc_shapes_ok(int64_t d, int64_t F) { return asca_tc_enabled() && d %
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Tensor-core forward: permute xn once, then two grouped tcgen05 GEMMs. pre_p null: the pre-activations are not kept.
+// res (may be out; null: nothing) is added in the second product's epilogue and out16 (nullable) takes a bf16 copy of the sum.
 int moe_fwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1,
                const __nv_bfloat16* w2, const float* b2, const int32_t* perm, const int32_t* offsets, int64_t N,
-               int64_t d, int64_t F, int64_t E, float* out, float* pre_p, __nv_bfloat16* hid_p) {
+               int64_t d, int64_t F, int64_t E, const float* res, float* out, __nv_bfloat16* out16, float* pre_p, __nv_bfloat16* hid_p) {
     void* ws;
     ASCA_TRY(asca_workspace(ctx, align256((size_t)N * d * 2) + 256, &ws));
     __nv_bfloat16* xp = (__nv_bfloat16*)ws;
@@ -194,6 +195,8 @@ int moe_fwd_tc(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, 
     b.A = hid_p; b.lda = F; b.a_rows = N; b.a_cols = F;
     b.B = w2; b.ldb = d; b.b_rows = E * F; b.b_cols = d; b.b_goff_outer = (int)F;
     b.C = out; b.ldc = d; b.N = (int)d; b.K = (int)F; b.c_idx = perm;
+    b.accumulate = res != nullptr; b.res = res == out ? nullptr : res;
+    b.C2 = out16; b.ldc2 = d; b.c2_mapped = out16 != nullptr;
     b.bias = b2; b.bias_gstride = 0;
     b.offsets = offsets; b.n_groups = (int)E; b.group_dim = gemm_tc::GROUP_M; b.total_rows = N;
     // nothing is launched unless the gather (16-byte copies) and every product can run here: the caller falls back as a whole
@@ -317,12 +320,15 @@ int moe_fwd_simt(asca_ctx* ctx, const void* xn, const void* w1, const float* b1,
 
 }  // namespace
 
-// bf16 forward that keeps no pre-activations (no backward follows: a third of the first product's epilogue and two thirds of its
-// bytes). ASCA_ERR_UNSUPPORTED where the tensor-core products cannot run; the caller then uses asca_moe_fwd.
-int asca_moe_fwd_bf16_nopre(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1, const __nv_bfloat16* w2, const float* b2,
-                            const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, float* out, __nv_bfloat16* hid_p) {
+// bf16 forward with the residual add in the second product's epilogue: out = res + moe(xn) (out may be res), and its bf16 copy in
+// out16 (nullable). pre_p null: the pre-activations are not kept (no backward follows: a third of the first product's epilogue
+// and two thirds of its bytes). ASCA_ERR_UNSUPPORTED, nothing launched, where the tensor-core products cannot run; the caller
+// then uses asca_moe_fwd and adds.
+int asca_moe_fwd_bf16_residual(asca_ctx* ctx, const __nv_bfloat16* xn, const __nv_bfloat16* w1, const float* b1, const __nv_bfloat16* w2, const float* b2,
+                            const int32_t* perm, const int32_t* offsets, int64_t N, int64_t d, int64_t F, int64_t E, const float* res, float* out,
+                               __nv_bfloat16* out16, float* pre_p, __nv_bfloat16* hid_p) {
     if (!tc_shapes_ok(d, F)) return ASCA_ERR_UNSUPPORTED;
-    return moe_fwd_tc(ctx, xn, w1, b1, w2, b2, perm, offsets, N, d, F, E, out, nullptr, hid_p);
+    return moe_fwd_tc(ctx, xn, w1, b1, w2, b2, perm, offsets, N, d, F, E, res, out, out16, pre_p, hid_p);
 }
 
 // f32 forward with the residual add in the second product's store: out = res + moe(xn)
@@ -382,7 +388,7 @@ int asca_moe_fwd(asca_ctx* ctx, const void* xn, const void* w1, const float* b1,
     const int bf = dtype == ASCA_BF16;
     if (bf && tc_shapes_ok(d, F)) {
         const int rc = moe_fwd_tc(ctx, (const __nv_bfloat16*)xn, (const __nv_bfloat16*)w1, b1, (const __nv_bfloat16*)w2, b2,
-                            perm, offsets, N, d, F, E, out, pre_p, (__nv_bfloat16*)hid_p);
+                            perm, offsets, N, d, F, E, nullptr, out, nullptr, pre_p, (__nv_bfloat16*)hid_p);
         if (rc != ASCA_ERR_UNSUPPORTED) return rc;
     }
     return moe_fwd_simt(ctx, xn, w1, b1, w2, b2, perm, offsets, N, d, F, E, bf, nullptr, out, pre_p, hid_p);
