@@ -54,10 +54,13 @@ template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct
     // main loop, and for the fused qkv epilogue (a warp's 128 columns are one head, or two of 64). Plain dense and k-grouped
     // products are faster with four (14,448 x 768 -> 2304: 56 against 68 us).
     static constexpr int EPI_WARPS = (PAIR && EW8) ? 8 : 4;
-    static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 384 /*barriers, claims*/;   // + stages + tile table
+    // A warp of its own (the k-grouped products run in this shape or on single CTAs) clears what a ragged k-tile holds of the next
+    // group's rows as soon as the tile has landed, while the issuer is still at earlier ones: see there
+    static constexpr bool RAG_WARP = PAIR && !EW8;
+    static constexpr int THREADS = 64 + 32 * EPI_WARPS + (RAG_WARP ? 32 : 0);
+    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 392 /*barriers, claims*/;   // + stages + tile table
 };
-constexpr int MAX_GROUPS = 2048, MAX_STAGES = 8;
+constexpr int MAX_GROUPS = 2048, MAX_STAGES = 7;
 
 struct KP {
     float* C;
@@ -196,8 +199,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
     uint64_t* empty = full + MAX_STAGES;
     uint64_t* acc_full = empty + MAX_STAGES; // [2] accumulator buffer written (MMA -> epilogue)
     uint64_t* acc_empty = acc_full + 2;      // [2] accumulator buffer read out (epilogue -> MMA)
-    uint64_t* peer_full = acc_empty + 2;     // [stage] PAIR, even CTA: the odd CTA has zeroed the ragged end of its k-tile
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_full + MAX_STAGES);
+    uint64_t* rag_full = acc_empty + 2;      // [stage] PAIR: this CTA's bytes of a ragged k-tile have landed (`full` takes the others)
+    uint64_t* rag_clear = rag_full + MAX_STAGES;   // [stage] PAIR, even CTA: both CTAs have cleared the end of their ragged k-tile
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rag_clear + MAX_STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile unsigned long long* claims = reinterpret_cast<volatile unsigned long long*>(tmem_slot + 2);   // [DYN_Q] (number + 1) << 32 | tile
     int* prefix = reinterpret_cast<int*>(const_cast<unsigned long long*>(claims) + DYN_Q);             // [n_groups + 1] first tile of every group
@@ -239,7 +243,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             for (uint32_t s = 0; s < STAGES; ++s) {
                 tc::mbar_init(&full[s], 1);
                 tc::mbar_init(&empty[s], 1);
-                tc::mbar_init(&peer_full[s], 1);
+                tc::mbar_init(&rag_full[s], 1);
+                tc::mbar_init(&rag_clear[s], 2);
             }
             for (int b = 0; b < 2; ++b) {
                 tc::mbar_init(&acc_full[b], 1);
@@ -318,6 +323,14 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         }
     };
     if (dyn && blockIdx.x == 0 && threadIdx.x == 0) *p.dyn_reset = 0;   // the launch after this one starts from zero
+    // A ragged k-tile of an expert's tokens: the instructions take whole sixteens of k rows, so A's rows from `valid` to the next
+    // sixteen, which are the next expert's, are cleared by one warp (a row of k is 128 bytes in each of two boxes)
+    auto clear_rows = [&](uint32_t s, int valid) {
+        uint8_t* a_s = tiles + s * STAGE_BYTES + ((lane >> 3) & 1) * 8192 + (lane & 7) * 16;
+        for (int kr = valid + (lane >> 4); kr < ((valid + 15) & ~15); kr += 2) *reinterpret_cast<uint4*>(a_s + kr * 128) = make_uint4(0, 0, 0, 0);
+        tc::fence_proxy_async_smem();
+        __syncwarp();
+    };
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (one thread)
@@ -353,10 +366,10 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     uint8_t* a_s = tiles + s * STAGE_BYTES;
                     uint8_t* b_s = a_s + A_BYTES;
                     // A pair's stage completes on the even CTA's barrier, for both CTAs' bytes at once. A ragged k-tile is zeroed
-                    // in part by each CTA first, so each waits for its own bytes.
+                    // in part by each CTA first, so each waits for its own bytes, on a barrier of its own.
                     const bool joint = PAIR && !(p.group_dim == GROUP_K && kt + 1 == x.num_k && (x.K % BK) != 0);
-                    const uint32_t bar = tc::smem_u32(&full[s]), bar0 = joint && rank ? tc::mapa_u32(bar, 0) : bar;
-                    if (!joint) tc::mbar_expect_tx(&full[s], STAGE_BYTES);
+                    const uint32_t bar = tc::smem_u32(PAIR && !joint ? &rag_full[s] : &full[s]), bar0 = joint && rank ? tc::mapa_u32(bar, 0) : bar;
+                    if (!joint) tc::mbar_expect_tx(PAIR ? &rag_full[s] : &full[s], STAGE_BYTES);
                     else if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
                     auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1) {
                         if (PAIR) tc::tma_load_2d_pair(dst, map, c0, c1, bar0);
@@ -398,7 +411,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        // One thread runs the loop (the rest of the warp joins only to zero a ragged k-tile): wait for the
+        // One thread of the even CTA runs the loop (in single CTAs the rest of the warp joins to clear a ragged k-tile): wait for the
         // stage, four tcgen05.mma whose descriptors are the stage's base descriptor plus a constant, commit.
         // The loop's own dependent instructions are what bounds a single MMA stream, so it is kept short.
         constexpr uint32_t IDESC = tc::idesc_bf16_f32(TM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
@@ -408,9 +421,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         const uint32_t a_lo0 = ((tc::smem_u32(tiles) >> 4) & 0x3FFF) | (A_LBO << 16);
         const uint32_t b_lo0 = (((tc::smem_u32(tiles) + A_BYTES) >> 4) & 0x3FFF) | (B_LBO << 16);
         bool ok = true;
-        uint32_t s = 0, par = 0;         // ring slot and parity of the next k-tile (kept by every lane)
-        uint32_t rag_own = 0, rag_peer = 0;   // PAIR: parity of every slot's next ragged k-tile (odd CTA: full; even CTA: peer_full)
-        for (int tl = 0;; ++tl) {   // tiles done by this CTA: accumulator buffer tl & 1
+        uint32_t s = 0;                      // ring slot of the next k-tile
+        uint32_t par = 0, rag_par = 0;       // parity of every slot's next wait on `full` and on `rag_clear` (a bit each)
+        for (int tl = 0; rank == 0; ++tl) {   // tiles done by this CTA: accumulator buffer tl & 1
             int t = lane == 0 && ok ? read_tile(tl) : -1;
             t = __shfl_sync(0xffffffffu, t, 0);
             if (t < 0) break;
@@ -420,12 +433,13 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             const bool ragged = p.group_dim == GROUP_K && (x.K % BK) != 0;   // warp-uniform
             const int n_plain = ragged ? x.num_k - 1 : x.num_k;
             auto next = [&] {
-                if (++s == STAGES) s = 0, par ^= 1;
+                if (++s == STAGES) s = 0;
             };
-            auto issue = [&](int kt) {   // the even CTA's (or the only) lane 0: one k-tile's instructions, slot release, tile hand-over
+            auto issue = [&](int kt, int rows) {   // one k-tile's instructions (on the first `rows` of its k), slot release, tile hand-over
                 const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = b_lo0 + s * (STAGE_BYTES >> 4);
 #pragma unroll
                 for (int k16 = 0; k16 < BK / 16; ++k16) {
+                    if (k16 * 16 >= rows) break;
                     const uint64_t da = ((uint64_t)DESC_HI << 32) | (a_lo + k16 * A_K16), db = ((uint64_t)DESC_HI << 32) | (b_lo + k16 * B_K16);
                     if (PAIR) tc::umma_bf16_pair(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
                     else tc::umma_bf16(tmem_acc, da, db, IDESC, (kt > 0 || k16 > 0) ? 1u : 0u);
@@ -438,71 +452,77 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     if (kt == x.num_k - 1) tc::umma_commit(&acc_full[buf]);
                 }
             };
-            if (lane == 0 && rank == 0) {
+            if (lane == 0) {
                 if (tl >= 2) {   // the epilogue (of both CTAs) has read this buffer's previous tile out
                     ok = PAIR ? tc::mbar_wait_cluster(&acc_empty[buf], ((tl >> 1) - 1) & 1, abort_flag, p.err_word, 104)
                               : tc::mbar_wait(&acc_empty[buf], ((tl >> 1) - 1) & 1, abort_flag, p.err_word, 104);
                 }
                 tc::tcgen05_fence_after();
                 for (int kt = 0; kt < n_plain && ok; ++kt) {
-                    ok = tc::mbar_wait(&full[s], par, abort_flag, p.err_word, 102);
+                    ok = tc::mbar_wait(&full[s], (par >> s) & 1, abort_flag, p.err_word, 102);
                     if (!ok) break;
                     tc::tcgen05_fence_after();
-                    issue(kt);
+                    issue(kt, BK);
+                    par ^= 1u << s;
                     next();
                 }
-            }
-            if (p.group_dim == GROUP_K) {   // (the other lanes and the odd CTA need the slot for ragged k-tiles only)
-                if (rank == 1) {
-                    const uint32_t at = s + (uint32_t)n_plain;
-                    par ^= (at / STAGES) & 1;
-                    s = at % STAGES;
-                } else {
-                    s = __shfl_sync(0xffffffffu, s, 0);
-                    par = __shfl_sync(0xffffffffu, par, 0);
+                if (PAIR && ragged && ok) {
+                    ok = tc::mbar_wait_cluster(&rag_clear[s], (rag_par >> s) & 1, abort_flag, p.err_word, 106);
+                    if (ok) {
+                        tc::tcgen05_fence_after();
+                        issue(n_plain, x.K - n_plain * BK);
+                        rag_par ^= 1u << s;
+                        next();
+                    }
                 }
             }
-            if (ragged) {
-                // last k-tile of this expert: rows >= K - kt*BK belong to the next expert and are zeroed by the whole warp,
-                // in each CTA's own half; the odd CTA then reports to the issuer
-                const int kt = x.num_k - 1;
+            if (!PAIR && ragged) {
+                // last k-tile of this expert: rows past it belong to the next expert and are cleared by the whole warp
+                s = __shfl_sync(0xffffffffu, s, 0);
                 int got = 0;
-                if (lane == 0) got = ok && tc::mbar_wait(&full[s], rank == 1 ? (rag_own >> s) & 1 : par, abort_flag, p.err_word, 105) ? 1 : 0;
-                rag_own ^= 1u << s;
+                if (lane == 0) got = ok && tc::mbar_wait(&full[s], (par >> s) & 1, abort_flag, p.err_word, 105) ? 1 : 0;
                 got = __shfl_sync(0xffffffffu, got, 0);
                 ok = got != 0;
                 if (ok) {
-                    tc::tcgen05_fence_after();
-                    uint8_t* a_s = tiles + s * STAGE_BYTES;
-                    const int valid = x.K - kt * BK;
-                    const int lines = (BK - valid) * 2;  // 128-byte lines in the two A boxes
-                    for (int i = lane; i < lines * 8; i += 32) {
-                        const int line = i >> 3, chunk = i & 7;
-                        const int h = line / (BK - valid), kr = valid + line % (BK - valid);
-                        *reinterpret_cast<uint4*>(a_s + h * 8192 + kr * 128 + chunk * 16) = make_uint4(0, 0, 0, 0);
-                    }
-                    tc::fence_proxy_async_smem();
-                    __syncwarp();
+                    clear_rows(s, x.K - n_plain * BK);
                     if (lane == 0) {
-                        if (PAIR && rank == 1) {
-                            tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&peer_full[s]), 0));
-                        } else {
-                            if (PAIR) ok = tc::mbar_wait_cluster(&peer_full[s], (rag_peer >> s) & 1, abort_flag, p.err_word, 106);
-                            if (ok) {
-                                tc::tcgen05_fence_after();
-                                issue(kt);
-                            }
-                        }
+                        tc::tcgen05_fence_after();
+                        issue(n_plain, x.K - n_plain * BK);
                     }
-                    rag_peer ^= 1u << s;
                 }
+                par ^= 1u << s;
                 next();
             }
-            if (lane == 0 && ok && x.num_k == 0 && rank == 0) {   // empty expert: the epilogue stores zeros
+            if (lane == 0 && ok && x.num_k == 0) {   // empty expert: the epilogue stores zeros
                 tc::mbar_arrive(&acc_full[buf]);
                 if (PAIR) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&acc_full[buf]), 1));
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;   // lane 0's verdict; keeps the warp's tile loops in step
+        }
+    } else if (SH::RAG_WARP && warp == 2 + SH::EPI_WARPS) {
+        // ------------------------------------------------------------ ragged k-tiles of a pair (both CTAs)
+        // Clears the end of an expert's last k-tile when the tile lands, up to a ring's depth ahead of the instructions that read it.
+        // In the issuing warp, all 64 rows' ends at a time, it held the instructions of the tile and of the next one up by 3 us a
+        // tile: C = 1024 x 4096 for 64 experts of 512 tokens took 350 us where every count is a multiple of 64 and 498 where none
+        // is (1,024 tokens: 520 and 718); now 367 and 377 (527 and 590).
+        uint32_t s = 0, par = 0;   // first ring slot of the tile; parity of every slot's next ragged k-tile (a bit each)
+        bool ok = p.group_dim == GROUP_K;
+        for (int tl = 0; ok; ++tl) {
+            int t = lane == 0 ? read_tile(tl) : -1;
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t < 0) break;
+            const Tile x = locate(t);
+            if (x.K % BK) {
+                const uint32_t last = (s + (uint32_t)x.num_k - 1) % STAGES;
+                int got = 0;
+                if (lane == 0) got = tc::mbar_wait(&rag_full[last], (par >> last) & 1, abort_flag, p.err_word, 105) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, got, 0) != 0;
+                if (!ok) break;
+                clear_rows(last, x.K % BK);
+                if (lane == 0) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&rag_clear[last]), 0));
+                par ^= 1u << last;
+            }
+            s = (s + (uint32_t)x.num_k) % STAGES;
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5, EW8: 2..9)
@@ -547,7 +567,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             const float* brow = p.bias ? p.bias + (int64_t)x.g * p.bias_gstride + x.n0 : nullptr;
             // aux, or where there is none the rows to add, ahead of their use (an add of the residual here, with the bf16 copy the
             // next block reads, hides behind the next tile's instructions: a prefill of 14,448 tokens x 12 blocks took 6.06 ms with
-            // the adds in passes of their own, 5.92 with them here; a training step of 8,192 x 2048 15.95 and 15.82 ms)
+            // the adds in passes of their own, 5.92 with them here; a training step of 32,768 x 2048 15.95 and 15.82 ms)
             const float* prow = with_aux ? arow : orow;
             const bool ahead = live && (with_aux || p.old);
             const int p_w = with_aux ? aux_w : c_w;

@@ -785,3 +785,32 @@ def test_residual_in_the_products_epilogues(orc, gpu, B, T, E):
             last[s] = ref.step(int(ids[s * T + t]), st)[0]
     assert rel_err(logits, last) < 2e-2
     dev.free()
+
+
+# Weight gradients of experts whose token counts end a 64-token tile anywhere (empty experts, sixteens, one past them): nothing of a
+# neighbour's rows, 1e4 times as large, enters a sum. d_w2 from the hidden rows as they were stored, within the bound of f32 sums.
+@pytest.mark.parametrize("d,F", [(256, 512), (128, 128)])   # CTA pairs; single CTAs
+def test_ragged_token_counts_in_weight_gradients(gpu, d, F):
+    import torch
+    from asca_b200 import ops
+
+    counts = [0, 1, 64, 15, 16, 17, 0, 63, 65, 79, 80, 81, 127, 128, 129, 448, 449, 511, 512, 513, 900, 33, 48, 2, 320, 7]
+    E, N = len(counts), sum(counts)
+    g = torch.Generator(device="cuda").manual_seed(F)
+
+    def norm(*s):
+        return torch.randn(*s, generator=g, device="cuda")
+
+    offs = torch.tensor([0] + counts, device="cuda").cumsum(0).int()
+    perm = torch.randperm(N, generator=g, device="cuda").int()
+    xn, w1, w2 = norm(N, d).bfloat16(), (norm(d, E * F) * d ** -0.5).bfloat16(), norm(E * F, d).bfloat16()
+    _, pre, hid = ops.moe_fwd(gpu, xn, w1, norm(E * F), w2, norm(d), perm, offs, F, E)
+    dout = norm(N, d)
+    for e in range(0, E, 2):
+        dout[perm[offs[e]:offs[e + 1]].long()] *= 1e4
+    _, _, d_w2, _, _ = ops.moe_bwd(gpu, xn, w1, w2, pre, hid, dout, perm, offs, F, E)
+    gpu.sync()
+    for e, n in enumerate(counts):
+        h, dy = hid[offs[e]:offs[e + 1]].double(), dout[perm[offs[e]:offs[e + 1]].long()].bfloat16().double()
+        err = (d_w2[e * F:(e + 1) * F].double() - h.t() @ dy).abs()
+        assert (err <= n * 2.0 ** -22 * (h.abs().t() @ dy.abs())).all(), (e, n)
