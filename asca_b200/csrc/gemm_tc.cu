@@ -181,6 +181,28 @@ __device__ __forceinline__ void store_row(__nv_bfloat16* p, const float (&v)[32]
         if (j < n) p[j] = __float2bfloat16(v[j]);
 }
 
+// 32 columns of the rows of two neighbouring lanes: 32-byte pieces are exchanged first, so that a store instruction's lane pairs
+// write 64 consecutive bytes. even_row, odd_row: where the even and the odd lane's columns go.
+__device__ __forceinline__ void store_row_pair(float* even_row, float* odd_row, const float (&v)[32], bool odd) {
+#pragma unroll
+    for (int h = 0; h < 32; h += 16) {
+        float e[8], o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float a = v[h + j], b = v[h + 8 + j], got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+            e[j] = odd ? got : a;
+            o[j] = odd ? b : got;
+        }
+        const int at = h + (odd ? 8 : 0);
+        asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                     ::"f"(e[0]), "f"(e[1]), "f"(e[2]), "f"(e[3]), "f"(e[4]), "f"(e[5]), "f"(e[6]), "f"(e[7]), "l"(even_row + at)
+                     : "memory");
+        asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                     ::"f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3]), "f"(o[4]), "f"(o[5]), "f"(o[6]), "f"(o[7]), "l"(odd_row + at)
+                     : "memory");
+    }
+}
+
 template <int MODE, int BN, bool DEEP, bool PAIR, bool EW8>
 __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN, DEEP, PAIR, EW8>::CTAS_PER_SM) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                                                              const __grid_constant__ CUtensorMap mapB, const KP p) {
@@ -655,6 +677,13 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             }
             const bool c_out = !(p.c2_only || qkv || ce), h_out = qkv || ce || p.C2;
             const int h_w = qkv ? qkv_w : c2_w;
+            // Every 32-byte piece that a store instruction writes to a line of its own is a request to L2, and with f32 results the
+            // requests bound these epilogues; lane pairs that write 64 bytes halve them. 64 experts of about 1,024 tokens, C = 1024 x
+            // 4096: 563 -> 531 us, and of about 512 tokens, 2048 x 4096: 790 -> 700. Not with eight warps, whose bf16 second results or
+            // reads weigh as much and whose registers are full: SiLU' 727 -> 775 us, the fused qkv form 70 -> 76.
+            const bool odd = lane & 1, c_pair = PAIR && !EW8 && c_out && c_w == 8 && __all_sync(0xffffffffu, live);
+            float* const nb_row = reinterpret_cast<float*>(__shfl_xor_sync(0xffffffffu, reinterpret_cast<unsigned long long>(crow), 1));
+            float *const even_row = odd ? nb_row : crow, *const odd_row = odd ? crow : nb_row;
             // A tcgen05.ld takes about 1,000 cycles beside the next tile's instructions, so the next group's is under way while one is
             // processed. (Unrolled to the end: what it loads may not pass through a loop's register moves before the wait. The four-warp
             // form, which takes the cross-entropy alone, loads in turn.)
@@ -712,9 +741,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     for (int j = 0; j < 32; ++j) v[j] += pre[i % AHEAD][j];
                 }
                 if (ahead && i + AHEAD < C_PER_WARP) load_row(pre[i % AHEAD], prow + (c + AHEAD) * 32, n_left - 32 * AHEAD, p_w);
-                if (!live) continue;
-                if (c_out) store_row(crow + c * 32, v, n_left, c_w);
-                if (h_out) {
+                if (PAIR && !EW8 && c_pair && n_left >= 32) store_row_pair(even_row + c * 32, odd_row + c * 32, v, odd);
+                else if (c_out && live) store_row(crow + c * 32, v, n_left, c_w);
+                if (h_out && live) {
                     if (p.epi == EPI_SILU) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = silu_f(v[j]);
