@@ -680,13 +680,14 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             // Every 32-byte piece that a store instruction writes to a line of its own is a request to L2, and with f32 results the
             // requests bound these epilogues; lane pairs that write 64 bytes halve them. 64 experts of about 1,024 tokens, C = 1024 x
             // 4096: 563 -> 531 us, and of about 512 tokens, 2048 x 4096: 790 -> 700. Not with eight warps, whose bf16 second results or
-            // reads weigh as much and whose registers are full: SiLU' 727 -> 775 us, the fused qkv form 70 -> 76.
+            // reads weigh as much and whose registers are full: SiLU' 727 -> 775 us, the fused qkv form 70 -> 76. Groups of four lanes and
+            // 128 bytes cost more in exchanges than they save (734 -> 781).
             const bool odd = lane & 1, c_pair = PAIR && !EW8 && c_out && c_w == 8 && __all_sync(0xffffffffu, live);
             float* const nb_row = reinterpret_cast<float*>(__shfl_xor_sync(0xffffffffu, reinterpret_cast<unsigned long long>(crow), 1));
             float *const even_row = odd ? nb_row : crow, *const odd_row = odd ? crow : nb_row;
             // A tcgen05.ld takes about 1,000 cycles beside the next tile's instructions, so the next group's is under way while one is
             // processed. (Unrolled to the end: what it loads may not pass through a loop's register moves before the wait. The four-warp
-            // form, which takes the cross-entropy alone, loads in turn.)
+            // form loads in turn: two under way took 66 us against 51 for 14,448 x 768 x 768 with a residual.)
             constexpr bool TWO = C_PER_WARP <= 4;
             uint32_t acc[TWO ? 2 : 1][32];
             if (TWO) tc::tmem_ld_32x32(tmem_acc + (uint32_t)(c_lo * 32), acc[0]);

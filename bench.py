@@ -650,12 +650,13 @@ def run_moe(hs: Harness, args):
 
 
 # ------------------------------------------------------------------ isolated delta op
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch at B=2, H=16, T=4096, dh=128 (32 chains), divided by 32:
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch at B=4, H=16, T=4096, dh=128 (64 chains), divided by 64:
 # traffic is proportional to the number of chains (profiles/delta_tc_bf16_cfg2.md).
 NCU_TRAFFIC_PER_CHAIN = {
-    "delta_bwd_tc_kernel": (438.934784e6 + 179.197440e6) / 32,
-    "delta_fwd_tc_kernel": (151.054336e6 + 63.292160e6) / 32,
-    "delta_prep_tc_kernel": (102.092288e6 + 310.865920e6) / 32,
+    "delta_grad_tc_kernel": (614.2e6 + 238.3e6) / 64,
+    "delta_bwd_tc_kernel": (372.1e6 + 302.2e6) / 64,
+    "delta_fwd_tc_kernel": (337.7e6 + 230.9e6) / 64,
+    "delta_prep_tc_kernel": (203.5e6 + 188.3e6) / 64,
 }
 
 
@@ -701,7 +702,7 @@ def run_delta(hs: Harness, args, bf16: bool):
     top = max(table, key=lambda kk: table[kk][1])
     n_top, t_top, _ = table[top]
     top_ms = t_top / n_top
-    top_bytes = bwd_bytes if "bwd" in top else fwd_bytes
+    top_bytes = bwd_bytes if "bwd" in top or "grad" in top else fwd_bytes
     pk = hs.peaks
     achieved = top_bytes / (top_ms * 1e-3) / 1e9
     # end to end from pinned host buffers
@@ -791,7 +792,7 @@ def run_delta(hs: Harness, args, bf16: bool):
                                     "frac": (fwd_bytes + bwd_bytes) / (dev_ms * 1e-3) / 1e9 / pk["hbm"]},
                      "note": "algorithmic bytes of the op the dominant kernel belongs to (q,k,v,o + gates forward; q,k,v,dO in and "
                              "dq,dk,dv out in the activation dtype + gates backward) / that kernel's mean CUDA-event time; traffic = dram "
-                             "bytes of one ncu capture at B=2 scaled by the number of chains"},
+                             "bytes of one ncu capture at B=4 scaled by the number of chains"},
         "e2e": {"value": b * t * 1e3 / e2e_ms, "unit": "tok/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms,
                 "api": api},
         "gpu_launches": launches, "clocks": clocks, "cpu_baseline": cpu, "parity_of_timed_batch": parity,
