@@ -968,12 +968,22 @@ __global__ void __launch_bounds__(BT, DH >= 64 ? 1 : 2) delta_bwd_chain_kernel(c
     }
 }
 
-// x / n for a row's common n and its reciprocal: one Newton step on the quotient, as close as a division; the plain quotient where the step
-// is not finite (n zero or infinite, or an overflow)
-__device__ __forceinline__ float div_row(float x, float n, float inv) {
-    const float q = x * inv, e = fmaf(-n, q, x);
-    return fabsf(e) < INFINITY ? fmaf(e, inv, q) : q;
-}
+// x / n for a row's common n: one Newton step on the quotient by its reciprocal, within a rounding of a division; the plain quotient where the
+// step is not finite (n zero or infinite, or an overflow). Below 2^-128 n has no finite reciprocal, so both sides of a small n are scaled by
+// a power of two first (an x that overflows by it has an infinite quotient).
+struct RowDiv {
+    float scale, n, inv;
+    __device__ __forceinline__ explicit RowDiv(float norm) {
+        scale = fabsf(norm) < 0x1p-100f ? 0x1p100f : 1.0f;
+        n = norm * scale;
+        inv = 1.0f / n;
+    }
+    __device__ __forceinline__ float operator()(float x) const {
+        x *= scale;
+        const float q = x * inv, e = fmaf(-n, q, x);
+        return fabsf(e) < INFINITY ? fmaf(e, inv, q) : q;
+    }
+};
 
 template <int DH>
 struct GradSmem {
@@ -1111,9 +1121,9 @@ __global__ void __launch_bounds__(BT, DH == 128 ? 1 : DH == 64 ? 2 : 3) delta_bw
             const int t = m.row(i);
             const float s = m.row_sum(i, [&](int, int, float x, int j) { return x * qv[i][j]; });
             if (t < n) {
-                const float nq = nq_s[t], inv = 1.0f / nq;
+                const RowDiv by(nq_s[t]);
 #pragma unroll
-                for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + h * DH + m.col(j)] = div_row(m.acc[i][j] - qv[i][j] * s, nq, inv);
+                for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + h * DH + m.col(j)] = by(m.acc[i][j] - qv[i][j] * s);
             }
         }
     }
@@ -1194,9 +1204,9 @@ __global__ void __launch_bounds__(BT, DH == 128 ? 1 : DH == 64 ? 2 : 3) delta_bw
         const int t = dk.row(i);
         const float s = dk.row_sum(i, [&](int tt, int c, float x, int) { return x * Ks[tt * LD + c]; });
         if (t < n) {
-            const float nk = nk_s[t], inv = 1.0f / nk;
+            const RowDiv by(nk_s[t]);
 #pragma unroll
-            for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + d + h * DH + dk.col(j)] = div_row(dk.acc[i][j] - Ks[t * LD + dk.col(j)] * s, nk, inv);
+            for (int j = 0; j < MD::TN; ++j) d_qkv[(row0 + t) * 3 * d + d + h * DH + dk.col(j)] = by(dk.acc[i][j] - Ks[t * LD + dk.col(j)] * s);
         }
     }
     // gates: dg, its suffix sums (two steps a lane), sigmoid backward

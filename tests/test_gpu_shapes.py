@@ -725,6 +725,38 @@ def test_delta_f32_norm_division_at_its_edges(gpu, dh):
         assert ((a - w)[fin].abs() <= 2 ** -22 * w[fin].abs() + 2 ** -148).all()
 
 
+# The same division by norms without a finite reciprocal (below 2^-128, denormal ones among them): finite quotients, infinities and the zeros of rows
+# without a gradient as in 64 bits.
+@pytest.mark.parametrize("dh", [32, 64, 128])
+def test_delta_f32_norms_without_a_reciprocal(gpu, dh):
+    import torch
+    from asca_b200 import ops
+
+    B, T, H = 1, 70, 2
+    g = torch.Generator(device="cuda").manual_seed(dh + 1)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, H, dh, generator=g, device="cuda"), dim=-1).reshape(T, H * dh) for _ in range(2))
+    v, d_o = (torch.randn(T, H * dh, generator=g, device="cuda") for _ in range(2))
+    d_o *= 10.0 ** torch.empty(T, 1, device="cuda").uniform_(-8, 0, generator=g)
+    d_o[2:7] = 0.0    # dq of these rows is zero
+    al, be = (torch.sigmoid(torch.randn(T, H, generator=g, device="cuda")) for _ in range(2))
+    one = torch.ones(T, H, device="cuda")
+    _, _, ck = ops.delta_fwd(gpu, q, k, v, al, be, B, T, H, dh)
+    want, _ = ops.delta_bwd(gpu, q, k, v, al, be, one, one, d_o, ck, B, T, H, dh)
+    norm = (10.0 ** torch.empty(T, H, device="cuda", dtype=torch.float64).uniform_(-44, -36, generator=g)).float()
+    norm[4], norm[9], norm[68], norm[69] = 2.0 ** -149, 2.0 ** -100, 2.0 ** -128, 2.0 ** -129
+    got, _ = ops.delta_bwd(gpu, q, k, v, al, be, norm, norm, d_o, ck, B, T, H, dh)
+    gpu.sync()
+    assert (norm > 0).all()
+    for part in range(2):
+        a, w = (x.view(T, 3, H, dh)[:, part] for x in (got, want))
+        w = (w.double() / norm.double()[..., None]).float()
+        fin = torch.isfinite(w)
+        assert (fin & (w != 0)).any() and not fin.all()
+        assert torch.equal(fin, torch.isfinite(a)) and not torch.isnan(a).any() and torch.equal(a[~fin], w[~fin])
+        assert ((a - w)[fin].abs() <= 2 ** -22 * w[fin].abs()).all()   # one rounding of the quotient on each side
+    assert (got.view(T, 3, H, dh)[2:7, 0] == 0).all()
+
+
 # Expert products of a few tokens, whose k range two or four CTAs share: odd numbers of k-tiles, experts without tokens and with more than
 # one token tile (several tiles a cluster), and just past the rule; against f64 sums over the hidden rows as they were stored.
 @pytest.mark.parametrize("tokens,experts,d,F", [(1, 16, 768, 3072), (3, 16, 768, 3072), (12, 16, 768, 3072), (13, 16, 768, 3072), (70, 2, 128, 1664), (300, 6, 64, 832), (200, 40, 64, 448)])
