@@ -59,10 +59,10 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc)
             : "r"(a4[i]), "r"(b4[i]));
     return acc;
 }
-// exp(x) like __expf, in an instruction the compiler does not move under a condition
-__device__ __forceinline__ float exp_neg(float x) {
-    float y;
-    asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504f));
+// __expf, taken whatever becomes of it: the compiler does not move it under a condition
+__device__ __forceinline__ float exp_always(float x) {
+    float y = __expf(x);
+    asm volatile("" : "+f"(y));
     return y;
 }
 // 32 columns of a row, 32 bytes at a time where the rows lie on that grid
@@ -268,10 +268,10 @@ __global__ void __launch_bounds__(PRE_THREADS, DH == 64 ? 4 : 3) delta_prep_tc_k
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {   // (every one, also above the diagonal: branches around them cost more)
                 const float4 g4 = *reinterpret_cast<const float4*>(g_s + cg * 32 + 4 * j4);
-                e[4 * j4] = exp_neg(gt - g4.x);
-                e[4 * j4 + 1] = exp_neg(gt - g4.y);
-                e[4 * j4 + 2] = exp_neg(gt - g4.z);
-                e[4 * j4 + 3] = exp_neg(gt - g4.w);
+                e[4 * j4] = exp_always(gt - g4.x);
+                e[4 * j4 + 1] = exp_always(gt - g4.y);
+                e[4 * j4 + 2] = exp_always(gt - g4.z);
+                e[4 * j4 + 3] = exp_always(gt - g4.w);
             }
             tc::tmem_ld_wait();
         }
@@ -453,7 +453,7 @@ struct ChainCfg {
     static constexpr int S_BYTES = NB * DH * 128;
     static constexpr int F_STAGE = NB * 32768 + 16384, F_K = NB * 16384, F_UV = NB * 24576, F_A = NB * 32768, F_AL = F_A + 8192;   // (W^, Q from 0)
     static constexpr size_t F_SMEM = 1024 + 2 * F_STAGE + S_BYTES + 4 * 512 + 128;
-        static constexpr int B_STAGE = NB * 24576 + 24576, B_KQ = 0, B_DO = NB * 16384, B_A = NB * 24576, B_AL = B_A + 8192, B_TP = B_AL + 8192;
+    static constexpr int B_STAGE = NB * 24576 + 24576, B_KQ = 0, B_DO = NB * 16384, B_A = NB * 24576, B_AL = B_A + 8192, B_TP = B_AL + 8192;
     static constexpr int B_RS = DH == 128 ? B_AL : B_TP;   // beta gam dR, where X - I (and AL) were
     static constexpr size_t B_SMEM = 1024 + 2 * B_STAGE + S_BYTES + (DH == 128 ? 16384 : 0) /*dU then dR; at 64 where A was*/ + 2 * 512 + 128;
 };
@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             // Masked exponentials are skipped one by one at head dim 128 and all taken at 64, where the branches cost more than the
             // exponentials (64: 264 -> 228 us at 8192 chunks; 128 the other way about: 449 and 411).
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x8[e] = DH == 64 ? exp_neg(g_row - g8[e]) : 8 * j + e < lim ? __expf(g_row - g8[e]) : 0.0f;
+            for (int e = 0; e < 8; ++e) x8[e] = DH == 64 ? exp_always(g_row - g8[e]) : 8 * j + e < lim ? __expf(g_row - g8[e]) : 0.0f;
 #pragma unroll
             for (int e = 0; e < 8; ++e) x8[e] = 8 * j + e < lim ? f * x8[e] * __uint_as_float(r[8 * j + e]) : 0.0f;
             *reinterpret_cast<uint4*>(sm + (half == 0 ? Cfg::R_M : Cfg::R_P) + tc::sw128_off(row, cg * 4 + j)) = tc::pack8_bf16(x8);

@@ -98,8 +98,9 @@ struct KP {
 };
 constexpr int DYN_Q = 16;              // claims a walker's producer can be ahead of its slowest role, with room to spare
 
-// bf16 mode only (2e-2 tolerance; the results are rounded to bf16 or multiply bf16 products): the hardware's base-2 exponential
-// and reciprocal without the denormal handling around them. An epilogue is bound by its instructions.
+// 1 / (1 + 2^(-x log2 e)), in the two approximate instructions whose errors the PTX manual bounds (2^-22 relative for ex2, one unit
+// in the last place for rcp): within (|x| + 5) 2^-23 of the sigmoid, and 0 or 1 where 2^(-x log2 e) leaves the range of f32. Its
+// results are rounded to bf16 or multiply bf16 products, and an epilogue is bound by its instructions.
 __device__ __forceinline__ float sigmoid_f(float x) {
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));

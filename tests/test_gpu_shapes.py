@@ -819,6 +819,33 @@ def test_residual_in_the_products_epilogues(orc, gpu, B, T, E):
     dev.free()
 
 
+# SiLU and its derivative in the expert products' epilogues (few rows, row tiles), from large negative arguments to large positive ones, against
+# 64 bits: the bf16 rounding of the result and (|x| + 5) 2^-23 of the sigmoid inside it.
+@pytest.mark.parametrize("tokens", [8, 256])
+def test_silu_over_the_range_of_its_argument(gpu, tokens):
+    import torch
+    from asca_b200 import ops
+
+    d, F, E = 128, 512, 2
+    x = torch.cat([torch.linspace(-110, 110, F // 2), torch.linspace(-9, 9, F // 2 - 4), torch.tensor([0.0, -1.2784645, 3e4, -3e4])]).cuda()
+    xn = torch.zeros(tokens, d, device="cuda").bfloat16()
+    w1, w2 = torch.zeros(d, E * F, device="cuda").bfloat16(), torch.zeros(E * F, d, device="cuda").bfloat16()
+    w2[:, 0] = 1.0
+    perm, offs = ops.moe_dispatch(gpu, torch.arange(tokens, device="cuda", dtype=torch.int32), E)
+    _, _, hid = ops.moe_fwd(gpu, xn, w1, x.repeat(E), w2, torch.zeros(d, device="cuda"), perm, offs, F, E)
+    dout = torch.zeros(tokens, d, device="cuda")
+    dout[0, 0] = 1.0
+    _, d_b1, _, _, _ = ops.moe_bwd(gpu, xn, w1, w2, x.repeat(tokens, 1), hid, dout, perm, offs, F, E)
+    gpu.sync()
+    x64 = x.double()
+    sg = torch.sigmoid(x64)
+    want, rel = x64 * sg, 2.0 ** -9 + (x64.abs() + 6) * 2.0 ** -23
+    assert ((hid.double() - want).abs() <= rel * want.abs() + 2e-36).all()
+    want = sg * (1 + x64 * (1 - sg))
+    off = 2.0 ** -9 * want.abs() + sg * (1 + 2 * x64.abs()) * (x64.abs() + 6) * 2.0 ** -23 + 2e-36
+    assert ((d_b1.view(E, F).double().sum(0) - want).abs() <= off).all()
+
+
 # Weight gradients of experts whose token counts end a 64-token tile anywhere (empty experts, sixteens, one past them): nothing of a
 # neighbour's rows, 1e4 times as large, enters a sum. d_w2 from the hidden rows as they were stored, within the bound of f32 sums.
 @pytest.mark.parametrize("d,F", [(256, 512), (128, 128)])   # CTA pairs; single CTAs
