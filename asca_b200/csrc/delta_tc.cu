@@ -9,14 +9,14 @@
 //   delta_fwd_tc_kernel    one CTA per chain, two dependent products a chunk
 //     U = Uv - W^ S          S <- gam_C S + K^T (eg U)          o = gam (Q S) + A U      (o off the serial path)
 //   delta_bwd_tc_kernel    one CTA per chain in reverse, three dependent products a chunk
-//     dU = A^T dO + eg (K dS)    dR = X^T dU    dS <- gam_C dS + Q^T (gam dO) - K^T (beta gam dR)    dv = beta dR
+//     dU = A^T dO + eg (K dS)    dR = X^T dU    dS <- gam_C dS + Q^T (gam dO) - K^T (beta gam dR)    dv = beta dR    <S, dS>
 //   delta_grad_tc_kernel   one CTA per (chunk, chain): dq, dk and the gate gradients from S, dS, U and dR, see its header
 //
 // Row factors (gam, eg, beta) are applied in f32 to results or to the rows of a 64-row operand just before it is rounded, never
 // to copies of q, k, v: the kernels read those straight from the caller's tensors, and what travels between them per (chunk, chain) is
 // W^, Uv, A, X - I (56 KB at DH 128) and, for a backward, S, U (in the checkpoint buffer) and dS, dR. A travels as two bf16
 // tiles, value and remainder: the rounding of an entry of A meets a whole row of U or dO, an error common to 128 columns that was most of
-// what the gate gradients and o's sums over heads had.
+// what the gate gradients and o's sums over heads had. Sums over dS and dR are taken in the chain, where these are f32.
 //
 // Tiles arrive by TMA (plain loads, 128-byte swizzle); a box that runs past a sequence's end is filled with zeros. Many products have
 // 64 rows: they either run as M = 128 with whatever lies behind the operand as rows 64 - 127 (the results of those rows land
@@ -47,17 +47,6 @@ __device__ __forceinline__ void load_vec(void* dst, const float* src, uint64_t* 
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 512, [%2];"
                  ::"r"(tc::smem_u32(dst)), "l"(src), "r"(tc::smem_u32(bar))
                  : "memory");
-}
-// acc += the products of eight pairs of bf16, exact each, added one by one in f32
-__device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc) {
-    const uint32_t a4[4] = {a.x, a.y, a.z, a.w}, b4[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
-            "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
-            : "+f"(acc)
-            : "r"(a4[i]), "r"(b4[i]));
-    return acc;
 }
 // __expf, taken whatever becomes of it: the compiler does not move it under a condition
 __device__ __forceinline__ float exp_always(float x) {
@@ -455,7 +444,8 @@ struct ChainCfg {
     static constexpr size_t F_SMEM = 1024 + 2 * F_STAGE + S_BYTES + 4 * 512 + 128;
     static constexpr int B_STAGE = NB * 24576 + 24576, B_KQ = 0, B_DO = NB * 16384, B_A = NB * 24576, B_AL = B_A + 8192, B_TP = B_AL + 8192;
     static constexpr int B_RS = DH == 128 ? B_AL : B_TP;   // beta gam dR, where X - I (and AL) were
-    static constexpr size_t B_SMEM = 1024 + 2 * B_STAGE + S_BYTES + (DH == 128 ? 16384 : 0) /*dU then dR; at 64 where A was*/ + 2 * 512 + 128;
+    // behind the stages: dS and, at 128, dU (then dR) and S; at 64 these lie where A and its remainder were
+    static constexpr size_t B_SMEM = 1024 + 2 * B_STAGE + S_BYTES + (DH == 128 ? 16384 + S_BYTES : 0) + 2 * 512 + 192;
 };
 
 // What bounds it: at 128 chains HBM (145 KB per chunk with a backward to follow: 5.8 TB/s at 203 us for 64 chunks, 281 before), at few
@@ -719,7 +709,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 
 // ------------------------------------------------------------------ backward chain
 // Same threads as the forward: quarters 0 and 1 hold the 64 rows of dU and dR, quarters 2 and 3 scale the rows of dO by gam in place
-// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO. 170 KB of HBM per chunk
+// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO. 202 KB of HBM per chunk
 // (dv in f32 among them) at 3.8 TB/s: 367 us for 64 chunks of 128 chains, three products and their register passes one after another.
 // With the gradients on the same chain a chunk was nine groups of products: 914 us.
 template <int DH>
@@ -727,8 +717,9 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapDO,
     const __grid_constant__ CUtensorMap mapAA, const __grid_constant__ CUtensorMap mapAL, const __grid_constant__ CUtensorMap mapTP,
     const __grid_constant__ CUtensorMap mapDS,
-    const __grid_constant__ CUtensorMap mapDR, const __grid_constant__ CUtensorMap mapV, const float* __restrict__ GB, const __nv_bfloat16* __restrict__ v,
-    int T, int H, int n_chunks, float* __restrict__ d_qkv, float* __restrict__ VD /* [tile][NG][64]: v . dv over 32 columns */, int ahead, int* err_word) {
+    const __grid_constant__ CUtensorMap mapDR, const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapS0,
+    const float* __restrict__ GB, const __nv_bfloat16* __restrict__ v, int T, int H, int n_chunks, float* __restrict__ d_qkv,
+    float* __restrict__ VD /* [tile][NG][64]: v . dv over 32 columns */, float* __restrict__ SD /* [tile][S_WARPS]: parts of <S, dS> */, int ahead, int* err_word) {
     using Cfg = ChainCfg<DH>;
     constexpr int NB = Cfg::NB, NG = Cfg::NG;
     extern __shared__ uint8_t smem_raw[];
@@ -738,11 +729,15 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
         return DH == 128 ? S_s + Cfg::S_BYTES : base + s * Cfg::B_STAGE + Cfg::B_A;
     };
     auto Rs_s = [&](int s) { return base + s * Cfg::B_STAGE + Cfg::B_RS; };
-    float* gb_s = reinterpret_cast<float*>(S_s + Cfg::S_BYTES + (DH == 128 ? 16384 : 0));   // [2][128], with the stages
+    // S at the start of step it's chunk, which meets dS in the step before: a buffer of its own, or at head dim 64 the place that the
+    // remainder of A has left in that step's stage
+    auto S0_s = [&](int it) { return DH == 128 ? S_s + Cfg::S_BYTES + 16384 : base + ((it & 1) ^ 1) * Cfg::B_STAGE + Cfg::B_AL; };
+    float* gb_s = reinterpret_cast<float*>(S_s + Cfg::S_BYTES + (DH == 128 ? 16384 + Cfg::S_BYTES : 0));   // [2][128], with the stages
     uint64_t* bars = reinterpret_cast<uint64_t*>(gb_s + 256);
     uint64_t *full = bars, *mma0_done = bars + 2, *mma1_done = bars + 3, *mma2_done = bars + 4, *mma3_done = bars + 5 /*[2], per stage as in the forward*/,
-             *s_ready = bars + 7, *do_ready = bars + 8, *du_ready = bars + 9, *dr_ready = bars + 10, *s_stored = bars + 11, *r_stored = bars + 12;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+             *s_ready = bars + 7, *do_ready = bars + 8, *du_ready = bars + 9, *dr_ready = bars + 10, *s_stored = bars + 11, *r_stored = bars + 12,
+             *s0_full = bars + 13;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -753,7 +748,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 13; ++i) {
+        for (int i = 0; i < 14; ++i) {
             const uint64_t* w = bars + i;
             tc::mbar_init(&bars[i], w == s_ready ? Cfg::S_WARPS : w == do_ready || w == du_ready || w == dr_ready ? Cfg::ROW_WARPS : 1);
         }
@@ -830,6 +825,15 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     } else if (warp > Cfg::COMPUTE / 32) {
         // ------------------------------------------------------------ everything that moves (one thread): tiles in, dS and dR out
         if (lane == 0) {
+            auto load_al = [&](int it) {   // (counted in its stage's bytes)
+                tc::tma_load_2d(base + (it & 1) * Cfg::B_STAGE + Cfg::B_AL, &mapAL, 0, (int)(tile0 + n_chunks - 1 - it) * 64, &full[it & 1]);
+            };
+            auto load_s0 = [&](int it) {
+                tc::mbar_expect_tx(s0_full, Cfg::S_BYTES);
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
+                    tc::tma_load_2d(S0_s(it) + nb * (DH * 128), &mapS0, nb * 64, (int)(tile0 + n_chunks - 1 - it) * DH, s0_full);
+            };
             auto load = [&](int it) {
                 const int c = n_chunks - 1 - it, s = it & 1;
                 uint8_t* st = base + s * Cfg::B_STAGE;
@@ -839,7 +843,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 #pragma unroll
                 for (int kb = 0; kb < NB; ++kb) tc::tma_load_3d(st + Cfg::B_DO + kb * 8192, &mapDO, h * DH + kb * 64, c * C, b, &full[s]);
                 tc::tma_load_2d(st + Cfg::B_A, &mapAA, 0, t * 64, &full[s]);
-                tc::tma_load_2d(st + Cfg::B_AL, &mapAL, 0, t * 64, &full[s]);
+                if (DH == 128 || it == 0) load_al(it);
 #pragma unroll
                 for (int kb = 0; kb < NB; ++kb) {
                     tc::tma_load_3d(st + kb * 16384, &mapK, h * DH + kb * 64, c * C, b, &full[s]);
@@ -860,6 +864,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 tc::tma_prefetch_2d(&mapAA, 0, t * 64);
                 tc::tma_prefetch_2d(&mapAL, 0, t * 64);
                 tc::tma_prefetch_2d(&mapTP, 0, t * 64);
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb) tc::tma_prefetch_2d(&mapS0, nb * 64, t * DH);
             };
             load(0);
             if (n_chunks > 1) load(1);
@@ -870,6 +876,11 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapDS, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
                 tc::bulk_commit_group();
+                if (it + 1 < n_chunks) {   // this step's S has met dS (s_ready); at head dim 64 the remainder of A gives up its place
+                    if (DH == 64 && !tc::mbar_wait(mma0_done, par, abort_flag, err_word, 309)) break;
+                    load_s0(it + 1);
+                    if (DH == 64) load_al(it + 1);
+                }
                 tc::bulk_wait_read();
                 tc::mbar_arrive(s_stored);
                 if (!tc::mbar_wait(dr_ready, par, abort_flag, err_word, 307)) break;
@@ -987,10 +998,12 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 #pragma unroll
                 for (int j = 0; j < 4; ++j) v4[j] = c * C + row < T ? reinterpret_cast<const uint4*>(vr)[j] : make_uint4(0, 0, 0, 0);
             }
+            float sd = 0.0f;
             if (c > 0) {
                 if (!warp_wait(&full[par ^ 1], ((it + 1) >> 1) & 1, 315)) break;
-                if (s_warp) {   // dS at the start of the chunk: bf16 operand copy, and f32 scaled by the chunk before's decay
+                if (s_warp) {   // dS at the start of the chunk: bf16 operand copy, f32 scaled by the chunk before's decay, and <S, dS> for that chunk
                     const float gC = expf(gb_s[(par ^ 1) * 128 + C - 1]);
+                    if (!warp_wait(s0_full, par, 318)) break;
                     if (!warp_wait(s_stored, par, 316)) break;
                     if (!warp_wait(&mma3_done[par], (it >> 1) & 1, 317)) break;
 #pragma unroll
@@ -1004,7 +1017,12 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 #pragma unroll
                         for (int j = 0; j < 2; ++j) {
                             const int c16 = cg * 4 + 2 * i + j;
-                            *reinterpret_cast<uint4*>(S_s + (c16 >> 3) * (DH * 128) + tc::sw128_off(arow, c16 & 7)) = tc::pack8_bf16(f + 8 * j);
+                            const uint32_t off = (c16 >> 3) * (DH * 128) + tc::sw128_off(arow, c16 & 7);
+                            *reinterpret_cast<uint4*>(S_s + off) = tc::pack8_bf16(f + 8 * j);
+                            float s8[8];
+                            tc::unpack8_bf16(*reinterpret_cast<const uint4*>(S0_s(it + 1) + off), s8);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) sd = fmaf(s8[e], f[8 * j + e], sd);
                         }
 #pragma unroll
                         for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gC * f[j]);
@@ -1012,6 +1030,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                     }
                     tc::tmem_st_wait();
                     arrive(s_ready);
+                    sd = warp_sum(sd);
+                    if (lane == 0) SD[(tile0 + c - 1) * Cfg::S_WARPS + cg * (Cfg::S_WARPS / NG) + wq] = sd;
                 }
             }
             if (wq < 2) {   // dv = beta dR, and this thread's part of v . dv
@@ -1059,7 +1079,7 @@ struct GradCfg {
                          R_S = NB * R_ROWS, R_DS = R_S + SB, R_S1 = R_DS + SB, R_DS1 = R_S,
                          R_K = DH == 128 ? R_DS : R_DS + SB, R_Q = DH == 128 ? R_DR : R_K + 8192, R_END = DH == 128 ? R_S1 + SB : R_Q + 8192,
                          R_M = (NB - 1) * R_ROWS + R_DR, R_P = (NB - 1) * R_ROWS + R_DO;
-    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 /*dots*/ + 2 * 64 * 3 /*k.MK, k.Y, k.dW*/ + 64 /*v.dv*/ + 8;
+    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 /*dots*/ + 2 * 64 * 3 /*k.MK, k.Y, k.dW*/ + 64 /*v.dv*/;
     static constexpr size_t SMEM = 1024 + R_END + NVEC * 4 + 64;
 };
 
@@ -1067,7 +1087,7 @@ template <int DH>
 __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapDO,
     const __grid_constant__ CUtensorMap mapDR, const __grid_constant__ CUtensorMap mapU, const __grid_constant__ CUtensorMap mapS0,
-    const __grid_constant__ CUtensorMap mapDS, const float* __restrict__ GB, const float* __restrict__ VD, const float* __restrict__ alpha,
+    const __grid_constant__ CUtensorMap mapDS, const float* __restrict__ GB, const float* __restrict__ VD, const float* __restrict__ SD, const float* __restrict__ alpha,
     const float* __restrict__ qnorm, const float* __restrict__ knorm, int T, int H, int n_chunks,
     float* __restrict__ d_qkv, float* __restrict__ d_gate, int* err_word) {
     using Cfg = GradCfg<DH>;
@@ -1076,8 +1096,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     float* g_s = reinterpret_cast<float*>(sm + Cfg::R_END);
     float *be_s = g_s + 64, *al_s = be_s + 64, *nrm_s = al_s + 64 /*q rows, k rows*/, *dot_s = nrm_s + 128 /*[2][128]*/, *mk_s = dot_s + 256 /*[2][64]*/,
-          *ky_s = mk_s + 128, *kw_s = ky_s + 128, *vd_s = kw_s + 128, *red_s = vd_s + 64;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(red_s + 8);   // tiles: [0], [1] by half, [2] dS's second, [3] K, Q; products: [4], [5] by half, [6] second group
+          *ky_s = mk_s + 128, *kw_s = ky_s + 128, *vd_s = kw_s + 128;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(vd_s + 64);   // tiles: [0], [1] by half, [2] dS's second, [3] K, Q; products: [4], [5] by half, [6] second group
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -1122,6 +1142,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
         }
     }
     if (warp == 0) tc::tmem_alloc(tmem_slot, 256);
+    constexpr int SDN = ChainCfg<DH>::S_WARPS;
+    const float sds = warp == 0 && lane < SDN && chunk + 1 < n_chunks ? SD[tix * SDN + lane] : 0.0f;   // <S, dS>'s parts (dS = 0 at the end)
     {
         const int t = tid & 63;
         const bool live = t < n;
@@ -1162,7 +1184,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
         tc::tcgen05_fence_after();
     };
 
-    // ---- first group; <S, dS> beside it
+    // ---- first group
     constexpr uint32_t I64 = tc::idesc_bf16_f32(64, 64, 0, 0), IDH = tc::idesc_bf16_f32(64, DH, 0, 0);
     auto group1 = [&](int hv) {
         const uint32_t rows = hv * Cfg::R_ROWS, s0 = hv == 0 ? Cfg::R_S : Cfg::R_S1;
@@ -1190,23 +1212,12 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             }
         }
     };
-    float sds = 0.0f;
-    auto dot_sds = [&](uint32_t a, uint32_t d_) {   // (the tiles have one layout: element by element)
-#pragma unroll
-        for (int i = 0; i < DH * 8 / GR_THREADS; ++i)
-            sds = dot8(*reinterpret_cast<const uint4*>(sm + a + (tid + i * GR_THREADS) * 16),
-                       *reinterpret_cast<const uint4*>(sm + d_ + (tid + i * GR_THREADS) * 16), sds);
-    };
     wait_bar(0, 0);
     if (tid == 0) {
         group1(0);
         products_dw(0);
         tc::umma_commit(&bars[4]);
-    }
-    dot_sds(Cfg::R_S, Cfg::R_DS);
-    if constexpr (DH == 128) {
-        __syncthreads();   // everybody has read the first half of S and dS
-        if (tid == 0) {
+        if constexpr (DH == 128) {
             tc::mbar_wait(&bars[1], 0, abort_flag, err_word, 321);
             group1(1);
             tc::umma_commit(&bars[5]);
@@ -1294,9 +1305,6 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
         }
         tc::umma_commit(&bars[6]);
     }
-    if constexpr (DH == 128) dot_sds(Cfg::R_S1, Cfg::R_DS1);   // (while the products run)
-    sds = warp_sum(sds);
-    if (lane == 0) red_s[warp] = sds;
     wait_bar(6, 0);
     // ---- dq (half 0) and dk (half 1) before the norm's backward: back to TMEM; row sums
     const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
@@ -1377,10 +1385,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             s[i] = dot_s[t] + dot_s[128 + t] - (dot_s[64 + t] + dot_s[192 + t]) + 2.0f * w[i];
             kw += kw_s[t] + kw_s[64 + t];
         }
-        float all = 0.0f;
-#pragma unroll
-        for (int i = 0; i < GR_THREADS / 32; ++i) all += red_s[i];
-        const float extra = __expf(g_s[C - 1]) * all + warp_sum(kw);
+        const float extra = __expf(g_s[C - 1]) * warp_sum(sds) + warp_sum(kw);
         if (lane == 31) s[1] += extra;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {   // suffix sums over t = 0..63
@@ -1613,13 +1618,14 @@ static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* 
             slot = (int)i;
     }
     __nv_bfloat16 *dS, *dR;
-    float* VD;
+    float *VD, *SD;
     void* ws;
     for (int pass = 0; pass < 2; ++pass) {   // count, then carve
         Carver w{pass ? al_ptr(ws) : nullptr};
         dS = w.take<__nv_bfloat16>(n_tiles * DH * DH);
         dR = w.take<__nv_bfloat16>(n_tiles * C * DH);
         VD = w.take<float>(n_tiles * C * (DH / 32));
+        SD = w.take<float>(n_tiles * ChainCfg<DH>::S_WARPS);
         if (slot < 0) {
             carve_kept(w, n_tiles, true, &t);
             carve_rows(w, n_tiles, DH, &t);
@@ -1646,8 +1652,8 @@ static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* 
     ASCA_CUDA(ctx, cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::B_SMEM));
     {
         asca_span sp(ctx, "delta_bwd_tc_kernel");
-        chain<<<(unsigned)chains, Cfg::THREADS, Cfg::B_SMEM, ctx->stream>>>(mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, mV, t.GB, (const __nv_bfloat16*)v, (int)T,
-                                                                            (int)H, (int)n_chunks, d_qkv, VD, chains <= ctx->sm_count, ctx->err_word);
+        chain<<<(unsigned)chains, Cfg::THREADS, Cfg::B_SMEM, ctx->stream>>>(mK, mQ, mDO, mAA, mAL, mTP, mDS, mDR, mV, mS0, t.GB, (const __nv_bfloat16*)v,
+                                                                            (int)T, (int)H, (int)n_chunks, d_qkv, VD, SD, chains <= ctx->sm_count, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     auto grad = delta_grad_tc_kernel<DH>;
@@ -1655,7 +1661,7 @@ static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* 
     {
         asca_span sp(ctx, "delta_grad_tc_kernel");
         grad<<<dim3((unsigned)n_chunks, (unsigned)chains), GR_THREADS, GradCfg<DH>::SMEM, ctx->stream>>>(
-            mK, mQ, mDO, mDR, mU, mS0, mDS, t.GB, VD, alpha, qnorm, knorm, (int)T, (int)H, (int)n_chunks, d_qkv, d_gate, ctx->err_word);
+            mK, mQ, mDO, mDR, mU, mS0, mDS, t.GB, VD, SD, alpha, qnorm, knorm, (int)T, (int)H, (int)n_chunks, d_qkv, d_gate, ctx->err_word);
     }
     ASCA_CHECK_LAUNCH(ctx);
     return ASCA_OK;

@@ -697,6 +697,51 @@ def test_delta_tc_sequences_do_not_mix(gpu, B, T, H, dh):
         assert (got_.double() - ref).norm() < 8e-3 * ref.norm()
 
 
+# What the bf16 delta gradients hold in f32 between their products: inputs for which everything else is exact in bf16, one chain per
+# entry, so that a value rounded to bf16 on the way (2^-9) stands out. The bound: a dozen f32 roundings, exp and log among them.
+def _delta_tc_gates(gpu, q, k, v, al, be, d_o, s_init=None):
+    """d_gate (B, T, 2, H) of float tensors (B, T, H, dh) / (B, T, H) with unit norms."""
+    import torch
+    from asca_b200 import ops
+
+    B, T, H, dh = q.shape
+    q, k, v, d_o = (x.reshape(B * T, H * dh).bfloat16() for x in (q, k, v, d_o))
+    al, be = (x.reshape(B * T, H).contiguous() for x in (al, be))
+    one = torch.ones(B * T, H, device="cuda")
+    _, _, ck = ops.delta_fwd(gpu, q, k, v, al, be, B, T, H, dh, s_init=s_init)
+    _, d_gate = ops.delta_bwd(gpu, q, k, v, al, be, one, one, d_o, ck, B, T, H, dh)
+    gpu.sync()
+    return d_gate.view(B, T, 2, H).double()
+
+
+def _bf16_values(g, *shape):
+    import torch
+
+    return (torch.rand(*shape, generator=g, device="cuda") + 1).bfloat16().float()   # eight significant bits
+
+
+@pytest.mark.parametrize("dh", [64, 128])
+@pytest.mark.parametrize("T", [65, 128, 300])
+def test_delta_tc_state_gradient_meets_the_state_in_f32(gpu, dh, T):
+    """Nothing is written (beta 0), no output of the first chunk counts: d log alpha_0 = alpha_0 <S, Q^T dO of the chunks behind>."""
+    import torch
+
+    B, H = 2, 8
+    g = torch.Generator(device="cuda").manual_seed(T + dh)
+    q, k, v, d_o = (_bf16_values(g, B, T, H, dh) for _ in range(4))
+    d_o[:, :64] = 0.0
+    al, be = torch.ones(B, T, H, device="cuda"), torch.zeros(B, T, H, device="cuda")
+    al[:, 0] = 0.75
+    s_init = torch.zeros(B, H, dh, dh, device="cuda")
+    at = torch.randint(0, dh * dh, (B, H, 1), generator=g, device="cuda")
+    s_init.view(B, H, -1).scatter_(2, at, 1.0)
+    got = _delta_tc_gates(gpu, q, k, v, al, be, d_o, s_init)[:, 0, 0]
+    d_s = torch.einsum("bthi,bthj->bhij", q.double(), d_o.double())
+    want = 0.25 * 0.75 * d_s.reshape(B, H, -1).gather(2, at)[..., 0]
+    # (f32 sums on the tensor cores: sixteen products a step, each step within 2^-23 of the sum so far)
+    assert ((got - want).abs() <= 2.0 ** -18 * want.abs()).all()
+
+
 # f32 delta backward: a row's gradients are divided by its norm through the reciprocal; zero, infinite and tiny norms behave as a division.
 @pytest.mark.parametrize("dh", [32, 64, 128])
 def test_delta_f32_norm_division_at_its_edges(gpu, dh):
