@@ -1063,12 +1063,12 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 // and gradient at its end:
 //   dL = dR U^T,  dA = dO U^T,  X = dO S^T,  Y = dR S^T,  dW = U dS^T              one group of products, value columns 64 at a time
 //   M = -beta Gam dL (strictly lower),  P = Gam dA (lower);  X *= gam,  Y *= -beta gam   (in TMEM)
-//   dq = X + P K,   dk = Y + M^T K + P^T Q + M K + eg dW                           second group
-// and the gate gradients from row sums of these alone: with qdq_t = q_t . dq_t, kdk_t = k_t . dk_t and w_t = k_t . (M K + Y)_t
-//   d log alpha_t = sum over t' >= t of (qdq - kdk + 2 w)_t' + gam_C <S, dS> + sum over t' of eg k . dW
+//   dq = X + P K,   dk = Y + M^T K + P^T Q + M K, + eg dW                          second group, on top of X and Y
+// and the gate gradients from f32 values alone, with KK = K K^T and QK = Q K^T formed once more:
+//   w_t = rowsum(M o KK)_t + k_t . Y_t
+//   d log alpha_t = sum over t' >= t of (w + rowsum(P o QK) + q . X - colsum(M o KK + P o QK) - eg k . dW)_t'
+//                   + gam_C <S, dS> + sum over t' of eg k . dW          (<S, dS> from the chain kernel, which holds dS in f32)
 //   d beta_t = (v_t . dv_t + w_t) / beta_t
-// (Row t of dA's and dL's products with Q K^T and K K^T, which these sums otherwise need, are q_t . (P K)_t and k_t . (M K)_t; their column
-// sums are what k . dk holds beyond them. The bf16 tiles P and M enter row and column sums alike, so that what should cancel does.)
 // TMEM halves: thread (warp, lane) sees row 16 (warp & 3) + (lane & 15) of the product in half lane >> 4.
 constexpr int GR_THREADS = 256;
 template <int DH>
@@ -1079,8 +1079,9 @@ struct GradCfg {
                          R_S = NB * R_ROWS, R_DS = R_S + SB, R_S1 = R_DS + SB, R_DS1 = R_S,
                          R_K = DH == 128 ? R_DS : R_DS + SB, R_Q = DH == 128 ? R_DR : R_K + 8192, R_END = DH == 128 ? R_S1 + SB : R_Q + 8192,
                          R_M = (NB - 1) * R_ROWS + R_DR, R_P = (NB - 1) * R_ROWS + R_DO;
-    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 /*dots*/ + 2 * 64 * 3 /*k.MK, k.Y, k.dW*/ + 64 /*v.dv*/;
-    static constexpr size_t SMEM = 1024 + R_END + NVEC * 4 + 64;
+    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 * 3 /*dots, row sums, q.X and k.Y*/ + 4 * 64 /*column sums*/ +
+                                2 * 64 /*k.dW*/ + 64 /*v.dv*/;
+    static constexpr size_t SMEM = 1024 + R_END + NVEC * 4 + 96;
 };
 
 template <int DH>
@@ -1095,10 +1096,11 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     float* g_s = reinterpret_cast<float*>(sm + Cfg::R_END);
-    float *be_s = g_s + 64, *al_s = be_s + 64, *nrm_s = al_s + 64 /*q rows, k rows*/, *dot_s = nrm_s + 128 /*[2][128]*/, *mk_s = dot_s + 256 /*[2][64]*/,
-          *ky_s = mk_s + 128, *kw_s = ky_s + 128, *vd_s = kw_s + 128;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(vd_s + 64);   // tiles: [0], [1] by half, [2] dS's second, [3] K, Q; products: [4], [5] by half, [6] second group
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+    float *be_s = g_s + 64, *al_s = be_s + 64, *nrm_s = al_s + 64 /*q rows, k rows*/, *dot_s = nrm_s + 128 /*[2][128]*/,
+          *rs_s = dot_s + 256 /*[2][128]*/, *xy_s = rs_s + 256 /*[2][128]*/, *cs_s = xy_s + 256 /*[4][64]*/, *kw_s = cs_s + 256 /*[2][64]*/, *vd_s = kw_s + 128;
+    // tiles: [0], [1] by half, [2] dS's second, [3] K, Q; products: [4], [5] by half, [6] second group, [7] K K^T, Q K^T
+    uint64_t* bars = reinterpret_cast<uint64_t*>(vd_s + 64);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1127,7 +1129,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     };
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 7; ++i) tc::mbar_init(&bars[i], 1);
+        for (int i = 0; i < 8; ++i) tc::mbar_init(&bars[i], 1);
         tc::mbar_fence_init();
         tc::mbar_expect_tx(&bars[0], Cfg::R_ROWS + 2 * Cfg::SB);
         load_rows(0, &bars[0]);
@@ -1167,7 +1169,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     __syncthreads();
     tc::tcgen05_fence_after();
     const uint32_t tm = *tmem_slot;
-    const uint32_t ACC_A = tm /* X | Y, then dq | dk */, ACC_D = tm + DH /* dL | dA, then M K */, ACC_W = tm + DH + 64 /* dW */;
+    const uint32_t ACC_A = tm /* X | Y, then dq | dk */, ACC_D = tm + DH /* dL | dA, then K K^T | Q K^T */, ACC_W = tm + DH + 64 /* dW */;
     constexpr uint32_t H1 = 16u << 16;                    // lane offset of the second half
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const uint32_t sb = tc::smem_u32(sm);
@@ -1231,7 +1233,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     }
     const float g_row = g_s[row], be_row = be_s[row], gam = __expf(g_row), eg = __expf(g_s[C - 1] - g_row);
     wait_bar(3 + NB, 0);
-    // ---- M (half 0) and P (half 1): 32 columns of a row per thread, where the last dR and dO were
+    // ---- M (half 0) and P (half 1): 32 columns of a row per thread, rounded where the last dR and dO were
+    float mp[32];
     {
         uint32_t r[32];
         tc::tmem_ld_32x32(ACC_D + lane_addr + cg * 32, r);
@@ -1248,19 +1251,32 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
 #pragma unroll
             for (int e = 0; e < 8; ++e) x8[e] = DH == 64 ? exp_always(g_row - g8[e]) : 8 * j + e < lim ? __expf(g_row - g8[e]) : 0.0f;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x8[e] = 8 * j + e < lim ? f * x8[e] * __uint_as_float(r[8 * j + e]) : 0.0f;
+            for (int e = 0; e < 8; ++e) mp[8 * j + e] = x8[e] = 8 * j + e < lim ? f * x8[e] * __uint_as_float(r[8 * j + e]) : 0.0f;
             *reinterpret_cast<uint4*>(sm + (half == 0 ? Cfg::R_M : Cfg::R_P) + tc::sw128_off(row, cg * 4 + j)) = tc::pack8_bf16(x8);
         }
     }
-    if constexpr (DH == 128) {
-        wait_bar(2, 0);
-        if (tid == 0) products_dw(1);   // (finished when the second group is)
-    }
+    tc::tcgen05_fence_before();
+    __syncthreads();   // everybody has dL and dA
     wait_bar(3, 0);
-    // ---- X *= gam, Y *= -beta gam, k . Y
+    if (tid == 0) {
+#pragma unroll
+        for (int k16 = 0; k16 < DH / 16; ++k16) {
+            const uint32_t off = (k16 >> 2) * 8192;
+            tc::umma_bf16(ACC_D, kmaj(Cfg::R_K + off, k16 & 3), kmaj(Cfg::R_K + off, k16 & 3), I64, k16 > 0);
+            tc::umma_bf16(ACC_D + H1, kmaj(Cfg::R_Q + off, k16 & 3), kmaj(Cfg::R_K + off, k16 & 3), I64, k16 > 0);
+        }
+        tc::umma_commit(&bars[7]);
+        if constexpr (DH == 128) {
+            tc::mbar_wait(&bars[2], 0, abort_flag, err_word, 322);
+            products_dw(1);   // (finished when the second group is)
+        }
+    }
+    __syncwarp();
+    // ---- X *= gam, Y *= -beta gam; q . X, k . Y
+    const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
     {
         const float f = half == 0 ? gam : -be_row * gam;
-        float ky = 0.0f;
+        float xy = 0.0f;
 #pragma unroll
         for (int pc = 0; pc < CW / 16; ++pc) {
             const int col = cg * CW + pc * 16;
@@ -1269,18 +1285,18 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             tc::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                float k8[8];
-                tc::unpack8_bf16(*tile(Cfg::R_K, row, (col >> 3) + j), k8);
+                float y8[8];
+                tc::unpack8_bf16(*tile(ytile, row, (col >> 3) + j), y8);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const float x = f * __uint_as_float(r[8 * j + e]);
-                    ky = fmaf(k8[e], x, ky);
+                    xy = fmaf(y8[e], x, xy);
                     r[8 * j + e] = __float_as_uint(x);
                 }
             }
             tc::tmem_st_32x16(ACC_A + lane_addr + col, r);
         }
-        if (half == 1) ky_s[cg * 64 + row] = ky;
+        xy_s[cg * 128 + half * 64 + row] = xy;
         tc::tmem_st_wait();
     }
     tc::fence_proxy_async_smem();
@@ -1288,44 +1304,58 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     __syncthreads();
     // ---- second group
     if (tid == 0) {
-        constexpr uint32_t IKM = tc::idesc_bf16_f32(64, DH, 0, 1), IMM = tc::idesc_bf16_f32(64, DH, 1, 1), IKM64 = tc::idesc_bf16_f32(64, 64, 0, 1);
+        constexpr uint32_t IKM = tc::idesc_bf16_f32(64, DH, 0, 1), IMM = tc::idesc_bf16_f32(64, DH, 1, 1);
         tc::tcgen05_fence_after();
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16) {
-            const uint64_t kk = mnmaj(Cfg::R_K, k16), mk = kmaj(Cfg::R_M, k16);
+            const uint64_t kk = mnmaj(Cfg::R_K, k16);
             tc::umma_bf16(ACC_A, kmaj(Cfg::R_P, k16), kk, IKM, 1u);                                  // P K
             tc::umma_bf16(ACC_A + H1, mnmaj(Cfg::R_M, k16), kk, IMM, 1u);                            // M^T K
             tc::umma_bf16(ACC_A + H1, mnmaj(Cfg::R_P, k16), mnmaj(Cfg::R_Q, k16), IMM, 1u);          // P^T Q
-            if constexpr (DH == 128) {
-                tc::umma_bf16(ACC_D, mk, kk, IKM64, k16 > 0);                                        // M K, keys 0-63 | 64-127
-                tc::umma_bf16(ACC_D + H1, mk, mnmaj(Cfg::R_K + 8192, k16), IKM64, k16 > 0);
-            } else {
-                tc::umma_bf16(ACC_D + H1, mk, kk, IKM64, k16 > 0);
-            }
+            tc::umma_bf16(ACC_A + H1, kmaj(Cfg::R_M, k16), kk, IKM, 1u);                             // M K
         }
         tc::umma_commit(&bars[6]);
     }
+    // ---- row and column sums of M o K K^T and P o Q K^T, while the second group runs
+    wait_bar(7, 0);
+    {
+        uint32_t r[32];
+        tc::tmem_ld_32x32(ACC_D + lane_addr + cg * 32, r);
+        tc::tmem_ld_wait();
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            mp[j] *= __uint_as_float(r[j]);
+            s += mp[j];
+        }
+        rs_s[cg * 128 + half * 64 + row] = s;
+        // columns, over the warp's 16 rows of both: lane l ends with column l
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+            const bool up = lane & w;
+#pragma unroll
+            for (int j = 0; j < w; ++j) {
+                const float give = up ? mp[j] : mp[j + w];
+                mp[j] = (up ? mp[j + w] : mp[j]) + __shfl_xor_sync(0xffffffffu, give, w);
+            }
+        }
+        cs_s[wq * 64 + cg * 32 + lane] = mp[0];
+    }
     wait_bar(6, 0);
     // ---- dq (half 0) and dk (half 1) before the norm's backward: back to TMEM; row sums
-    const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
     {
-        float dot = 0.0f, mks = 0.0f, kws = 0.0f;
+        float dot = 0.0f, kws = 0.0f;
 #pragma unroll
         for (int pc = 0; pc < CW / 16; ++pc) {
             const int col = cg * CW + pc * 16;
-            uint32_t x[16], mk[16], w[16];
-            const uint32_t acol = DH == 128 ? pc * 16 : col;
+            uint32_t x[16], w[16];
             tc::tmem_ld_32x16(ACC_A + lane_addr + col, x);
-            tc::tmem_ld_32x16(ACC_D + lane_addr + acol, mk);
-            tc::tmem_ld_32x16(ACC_W + lane_addr + acol, w);
+            tc::tmem_ld_32x16(ACC_W + lane_addr + (DH == 128 ? pc * 16 : col), w);
             tc::tmem_ld_wait();
             if constexpr (DH == 128) {   // keys 64 cg .. of a row sit in half cg
                 const int src = (lane & 15) | (cg << 4);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    mk[j] = __shfl_sync(0xffffffffu, mk[j], src);
-                    w[j] = __shfl_sync(0xffffffffu, w[j], src);
-                }
+                for (int j = 0; j < 16; ++j) w[j] = __shfl_sync(0xffffffffu, w[j], src);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -1335,9 +1365,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
                 for (int e = 0; e < 8; ++e) {
                     float g = __uint_as_float(x[8 * j + e]);
                     if (half == 1) {
-                        const float m_ = __uint_as_float(mk[8 * j + e]), w_ = eg * __uint_as_float(w[8 * j + e]);
-                        g += m_ + w_;
-                        mks = fmaf(y8[e], m_, mks);
+                        const float w_ = eg * __uint_as_float(w[8 * j + e]);
+                        g += w_;
                         kws = fmaf(y8[e], w_, kws);
                     }
                     dot = fmaf(y8[e], g, dot);
@@ -1347,10 +1376,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             tc::tmem_st_32x16(ACC_A + lane_addr + col, x);
         }
         dot_s[cg * 128 + half * 64 + row] = dot;
-        if (half == 1) {
-            mk_s[cg * 64 + row] = mks;
-            kw_s[cg * 64 + row] = kws;
-        }
+        if (half == 1) kw_s[cg * 64 + row] = kws;
         tc::tmem_st_wait();
     }
     __syncthreads();
@@ -1381,9 +1407,10 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int t = lane + 32 * i;
-            w[i] = mk_s[t] + mk_s[64 + t] + ky_s[t] + ky_s[64 + t];
-            s[i] = dot_s[t] + dot_s[128 + t] - (dot_s[64 + t] + dot_s[192 + t]) + 2.0f * w[i];
-            kw += kw_s[t] + kw_s[64 + t];
+            const float kw_t = kw_s[t] + kw_s[64 + t];
+            w[i] = rs_s[t] + rs_s[128 + t] + xy_s[64 + t] + xy_s[192 + t];
+            s[i] = w[i] + (rs_s[64 + t] + rs_s[192 + t]) + (xy_s[t] + xy_s[128 + t]) - (cs_s[t] + cs_s[64 + t] + cs_s[128 + t] + cs_s[192 + t]) - kw_t;
+            kw += kw_t;
         }
         const float extra = __expf(g_s[C - 1]) * warp_sum(sds) + warp_sum(kw);
         if (lane == 31) s[1] += extra;

@@ -742,6 +742,29 @@ def test_delta_tc_state_gradient_meets_the_state_in_f32(gpu, dh, T):
     assert ((got - want).abs() <= 2.0 ** -18 * want.abs()).all()
 
 
+@pytest.mark.parametrize("dh", [64, 128])
+@pytest.mark.parametrize("t0,t1", [(0, 1), (2, 40), (17, 63)])
+def test_delta_tc_gate_sums_within_a_chunk_in_f32(gpu, dh, t0, t1):
+    """Token t0 writes, t1 reads (d log alpha) and overwrites (d beta): sums of (dO U^T) o (Q K^T) and (dR U^T) o (K K^T) with one entry."""
+    import torch
+
+    B, H, T = 2, 8, t1 + 1
+    g = torch.Generator(device="cuda").manual_seed(dh + t1)
+    al, be = torch.ones(B, T, H, device="cuda"), torch.zeros(B, T, H, device="cuda")
+    al[:, t1], be[:, t0] = 0.75, 1.0
+    q, k, v, d_o = (torch.zeros(B, T, H, dh, device="cuda") for _ in range(4))
+    q[:, t1, :, 1], k[:, t0, :, 1] = _bf16_values(g, B, H), 1.0
+    v[:, t0, :, dh - 3], d_o[:, t1, :, dh - 3] = _bf16_values(g, B, H), _bf16_values(g, B, H)
+    got = _delta_tc_gates(gpu, q, k, v, al, be, d_o)
+    x = (v[:, t0, :, dh - 3].double() * d_o[:, t1, :, dh - 3].double()) * 0.75
+    want = 0.25 * x * q[:, t1, :, 1].double()
+    assert ((got[:, t1, 0] - want).abs() <= 2.0 ** -19 * want).all()
+    q[:, t1, :, 1], k[:, t1, :, 1], be[:, t1] = 1.0, 1.0, 0.5
+    got = _delta_tc_gates(gpu, q, k, v, al, be, d_o)
+    want = -0.25 * x
+    assert ((got[:, t1, 1] - want).abs() <= 2.0 ** -19 * want.abs()).all()
+
+
 # f32 delta backward: a row's gradients are divided by its norm through the reciprocal; zero, infinite and tiny norms behave as a division.
 @pytest.mark.parametrize("dh", [32, 64, 128])
 def test_delta_f32_norm_division_at_its_edges(gpu, dh):
