@@ -9,7 +9,7 @@
 //   delta_fwd_tc_kernel    one CTA per chain, two dependent products a chunk
 //     U = Uv - W^ S          S <- gam_C S + K^T (eg U)          o = gam (Q S) + A U      (o off the serial path)
 //   delta_bwd_tc_kernel    one CTA per chain in reverse, three dependent products a chunk
-//     dU = A^T dO + eg (K dS)    dR = X^T dU    dS <- gam_C dS + Q^T (gam dO) - K^T (beta gam dR)    dv = beta dR    <S, dS>
+//     dU = A^T dO + eg (K dS)    dR = X^T dU    dS <- gam_C dS + Q^T (gam dO) - K^T (beta gam dR)    dv = beta dR    <S, dS>    dv . (S^T k)
 //   delta_grad_tc_kernel   one CTA per (chunk, chain): dq, dk and the gate gradients from S, dS, U and dR, see its header
 //
 // Row factors (gam, eg, beta) are applied in f32 to results or to the rows of a 64-row operand just before it is rounded, never
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 
 // ------------------------------------------------------------------ backward chain
 // Same threads as the forward: quarters 0 and 1 hold the 64 rows of dU and dR, quarters 2 and 3 scale the rows of dO by gam in place
-// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO. 202 KB of HBM per chunk
+// (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO, D3 = K S. 202 KB of HBM per chunk
 // (dv in f32 among them) at 3.8 TB/s: 367 us for 64 chunks of 128 chains, three products and their register passes one after another.
 // With the gradients on the same chain a chunk was nine groups of products: 914 us.
 template <int DH>
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     const __grid_constant__ CUtensorMap mapDS,
     const __grid_constant__ CUtensorMap mapDR, const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapS0,
     const float* __restrict__ GB, const __nv_bfloat16* __restrict__ v, int T, int H, int n_chunks, float* __restrict__ d_qkv,
-    float* __restrict__ VD /* [tile][NG][64]: v . dv over 32 columns */, float* __restrict__ SD /* [tile][S_WARPS]: parts of <S, dS> */, int ahead, int* err_word) {
+    float* __restrict__ VD /* [tile][2][NG][64]: v . dv and -gam dv . (S^T k) over 32 columns */, float* __restrict__ SD /* [tile][S_WARPS]: parts of <S, dS> */, int ahead, int* err_word) {
     using Cfg = ChainCfg<DH>;
     constexpr int NB = Cfg::NB, NG = Cfg::NG;
     extern __shared__ uint8_t smem_raw[];
@@ -736,8 +736,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
     uint64_t* bars = reinterpret_cast<uint64_t*>(gb_s + 256);
     uint64_t *full = bars, *mma0_done = bars + 2, *mma1_done = bars + 3, *mma2_done = bars + 4, *mma3_done = bars + 5 /*[2], per stage as in the forward*/,
              *s_ready = bars + 7, *do_ready = bars + 8, *du_ready = bars + 9, *dr_ready = bars + 10, *s_stored = bars + 11, *r_stored = bars + 12,
-             *s0_full = bars + 13;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+             *s0_full = bars + 13, *ks_done = bars + 14, *ks_read = bars + 15;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -748,18 +748,18 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 14; ++i) {
+        for (int i = 0; i < 16; ++i) {
             const uint64_t* w = bars + i;
-            tc::mbar_init(&bars[i], w == s_ready ? Cfg::S_WARPS : w == do_ready || w == du_ready || w == dr_ready ? Cfg::ROW_WARPS : 1);
+            tc::mbar_init(&bars[i], w == s_ready ? Cfg::S_WARPS : w == do_ready || w == du_ready || w == dr_ready || w == ks_read ? Cfg::ROW_WARPS : 1);
         }
         tc::mbar_fence_init();
     }
-    constexpr int TMEM_COLS = 4 * DH;   // 3 DH, and a power of two
+    constexpr int TMEM_COLS = 4 * DH;
     if (warp == Cfg::COMPUTE / 32) tc::tmem_alloc(tmem_slot, TMEM_COLS);
     tc::tcgen05_fence_before();
     __syncthreads();
     tc::tcgen05_fence_after();
-    const uint32_t tmem_S = *tmem_slot, tmem_D1 = tmem_S + DH, tmem_D2 = tmem_S + 2 * DH;
+    const uint32_t tmem_S = *tmem_slot, tmem_D1 = tmem_S + DH, tmem_D2 = tmem_S + 2 * DH, tmem_D3 = tmem_S + 3 * DH;
 
     if (warp == Cfg::COMPUTE / 32) {
         // ------------------------------------------------------------ MMA issuer (one thread)
@@ -783,7 +783,20 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 tc::umma_commit(mma0_done);
                 return true;
             };
-            bool ok = mma0(0);
+            // D3 = K S of step `it`, off the serial path
+            auto mma_ks = [&](int it) -> bool {
+                if (!tc::mbar_wait(s0_full, it & 1, abort_flag, err_word, 319)) return false;
+                if (it > 0 && !tc::mbar_wait(ks_read, (it - 1) & 1, abort_flag, err_word, 300)) return false;
+                const uint32_t st = tc::smem_u32(base + (it & 1) * Cfg::B_STAGE), s0 = tc::smem_u32(S0_s(it));
+                tc::tcgen05_fence_after();
+#pragma unroll
+                for (int k16 = 0; k16 < DH / 16; ++k16)
+                    tc::umma_bf16(tmem_D3, tc::smem_desc_sw128(st + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
+                                  tc::smem_desc_sw128(s0 + k16 * 2048, DH * 128, 1024), ID_KM, k16 > 0 ? 1u : 0u);
+                tc::umma_commit(ks_done);
+                return true;
+            };
+            bool ok = mma0(0) && mma_ks(0);
             for (int it = 0; ok && it < n_chunks; ++it) {
                 const int c = n_chunks - 1 - it, par = it & 1;
                 const uint32_t st = tc::smem_u32(base + par * Cfg::B_STAGE), r_addr = tc::smem_u32(R_s(par)), rs_addr = tc::smem_u32(Rs_s(par));
@@ -819,7 +832,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                     tc::umma_bf16(tmem_S, tc::smem_desc_sw128(st + k16 * 2048, 16384, 1024),
                                   tc::smem_desc_sw128(rs_addr + k16 * 2048, 8192, 1024), ID_MM_NEG, 1u);
                 tc::umma_commit(&mma3_done[par]);
-                if (!mma0(it + 1)) break;
+                if (!mma0(it + 1) || !mma_ks(it + 1)) break;
             }
         }
     } else if (warp > Cfg::COMPUTE / 32) {
@@ -868,6 +881,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 for (int nb = 0; nb < NB; ++nb) tc::tma_prefetch_2d(&mapS0, nb * 64, t * DH);
             };
             load(0);
+            load_s0(0);
             if (n_chunks > 1) load(1);
             if (ahead) prefetch(2);
             for (int it = 0; it < n_chunks; ++it) {
@@ -876,8 +890,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) tc::tma_store_2d(&mapDS, S_s + nb * (DH * 128), nb * 64, (int)(tile0 + c) * DH);
                 tc::bulk_commit_group();
-                if (it + 1 < n_chunks) {   // this step's S has met dS (s_ready); at head dim 64 the remainder of A gives up its place
-                    if (DH == 64 && !tc::mbar_wait(mma0_done, par, abort_flag, err_word, 309)) break;
+                if (it + 1 < n_chunks) {   // this step's S has met dS (s_ready) and K; at head dim 64 the remainder of A gives up its place
+                    if (!tc::mbar_wait(ks_done, par, abort_flag, err_word, 309)) break;   // (and A^T dO before it)
                     load_s0(it + 1);
                     if (DH == 64) load_al(it + 1);
                 }
@@ -997,13 +1011,25 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 const __nv_bfloat16* vr = v + ((int64_t)b * T + c * C + row) * d + h * DH + col;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) v4[j] = c * C + row < T ? reinterpret_cast<const uint4*>(vr)[j] : make_uint4(0, 0, 0, 0);
+                // -beta gam dR . (S^T k)   (K S was done before K dS)
+                float ky = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t r[16];
+                    tc::tmem_ld_32x16(tmem_D3 + lane_addr + col + 16 * i, r);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) ky = fmaf(du[16 * i + j], __uint_as_float(r[j]), ky);
+                }
+                arrive(ks_read);
+                VD[(((tile0 + c) * 2 + 1) * NG + cg) * 64 + row] = -bg * ky;
             }
             float sd = 0.0f;
             if (c > 0) {
                 if (!warp_wait(&full[par ^ 1], ((it + 1) >> 1) & 1, 315)) break;
                 if (s_warp) {   // dS at the start of the chunk: bf16 operand copy, f32 scaled by the chunk before's decay, and <S, dS> for that chunk
                     const float gC = expf(gb_s[(par ^ 1) * 128 + C - 1]);
-                    if (!warp_wait(s0_full, par, 318)) break;
+                    if (!warp_wait(s0_full, par ^ 1, 318)) break;
                     if (!warp_wait(s_stored, par, 316)) break;
                     if (!warp_wait(&mma3_done[par], (it >> 1) & 1, 317)) break;
 #pragma unroll
@@ -1046,7 +1072,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                         vd = fmaf(x8[e], du[8 * j + e], vd);
                     }
                 }
-                VD[((tile0 + c) * NG + cg) * 64 + row] = vd;
+                VD[((tile0 + c) * 2 * NG + cg) * 64 + row] = vd;
                 if (c * C + row < T) store32(d_qkv + ((int64_t)b * T + c * C + row) * 3 * d + 2 * d + h * DH + col, du, w32);
             }
         }
@@ -1067,7 +1093,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 // and the gate gradients from f32 values alone, with KK = K K^T and QK = Q K^T formed once more:
 //   w_t = rowsum(M o KK)_t + k_t . Y_t
 //   d log alpha_t = sum over t' >= t of (w + rowsum(P o QK) + q . X - colsum(M o KK + P o QK) - eg k . dW)_t'
-//                   + gam_C <S, dS> + sum over t' of eg k . dW          (<S, dS> from the chain kernel, which holds dS in f32)
+//                   + gam_C <S, dS> + sum over t' of eg k . dW          (<S, dS> and k . Y = -gam dv . (S^T k) from the chain
+//                                                                        kernel, which holds dS and dR in f32)
 //   d beta_t = (v_t . dv_t + w_t) / beta_t
 // TMEM halves: thread (warp, lane) sees row 16 (warp & 3) + (lane & 15) of the product in half lane >> 4.
 constexpr int GR_THREADS = 256;
@@ -1079,8 +1106,8 @@ struct GradCfg {
                          R_S = NB * R_ROWS, R_DS = R_S + SB, R_S1 = R_DS + SB, R_DS1 = R_S,
                          R_K = DH == 128 ? R_DS : R_DS + SB, R_Q = DH == 128 ? R_DR : R_K + 8192, R_END = DH == 128 ? R_S1 + SB : R_Q + 8192,
                          R_M = (NB - 1) * R_ROWS + R_DR, R_P = (NB - 1) * R_ROWS + R_DO;
-    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 * 3 /*dots, row sums, q.X and k.Y*/ + 4 * 64 /*column sums*/ +
-                                2 * 64 /*k.dW*/ + 64 /*v.dv*/;
+    static constexpr int NVEC = 64 /*g*/ + 64 /*beta*/ + 64 /*alpha*/ + 128 /*norms*/ + 2 * 128 * 2 /*dots, row sums*/ + 4 * 64 /*column sums*/ +
+                                2 * 64 * 2 /*q.X, k.dW*/ + 64 * 2 /*v.dv, k.Y*/;
     static constexpr size_t SMEM = 1024 + R_END + NVEC * 4 + 96;
 };
 
@@ -1097,9 +1124,10 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     float* g_s = reinterpret_cast<float*>(sm + Cfg::R_END);
     float *be_s = g_s + 64, *al_s = be_s + 64, *nrm_s = al_s + 64 /*q rows, k rows*/, *dot_s = nrm_s + 128 /*[2][128]*/,
-          *rs_s = dot_s + 256 /*[2][128]*/, *xy_s = rs_s + 256 /*[2][128]*/, *cs_s = xy_s + 256 /*[4][64]*/, *kw_s = cs_s + 256 /*[2][64]*/, *vd_s = kw_s + 128;
+          *rs_s = dot_s + 256 /*[2][128]*/, *qx_s = rs_s + 256 /*[2][64]*/, *cs_s = qx_s + 128 /*[4][64]*/, *kw_s = cs_s + 256 /*[2][64]*/, *vd_s = kw_s + 128,
+          *ky_s = vd_s + 64;
     // tiles: [0], [1] by half, [2] dS's second, [3] K, Q; products: [4], [5] by half, [6] second group, [7] K K^T, Q K^T
-    uint64_t* bars = reinterpret_cast<uint64_t*>(vd_s + 64);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ky_s + 64);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -1155,10 +1183,14 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             be_s[t] = GB[tix * 128 + 64 + t];
         } else if (tid < 128) {
             al_s[t] = alpha[r];
-            float s = 0.0f;
+            float s = 0.0f, y = 0.0f;
 #pragma unroll
-            for (int i = 0; i < DH / 32; ++i) s += VD[(tix * (DH / 32) + i) * 64 + t];
+            for (int i = 0; i < DH / 32; ++i) {
+                s += VD[(tix * 2 * (DH / 32) + i) * 64 + t];
+                y += VD[((tix * 2 + 1) * (DH / 32) + i) * 64 + t];
+            }
             vd_s[t] = s;
+            ky_s[t] = y;
         } else if (tid < 192) {
             nrm_s[t] = qnorm[r];
         } else {
@@ -1272,11 +1304,10 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
         }
     }
     __syncwarp();
-    // ---- X *= gam, Y *= -beta gam; q . X, k . Y
-    const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
+    // ---- X *= gam, Y *= -beta gam; q . X
     {
         const float f = half == 0 ? gam : -be_row * gam;
-        float xy = 0.0f;
+        float qx = 0.0f;
 #pragma unroll
         for (int pc = 0; pc < CW / 16; ++pc) {
             const int col = cg * CW + pc * 16;
@@ -1285,18 +1316,18 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
             tc::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                float y8[8];
-                tc::unpack8_bf16(*tile(ytile, row, (col >> 3) + j), y8);
+                float q8[8];
+                tc::unpack8_bf16(*tile(Cfg::R_Q, row, (col >> 3) + j), q8);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const float x = f * __uint_as_float(r[8 * j + e]);
-                    xy = fmaf(y8[e], x, xy);
+                    qx = fmaf(q8[e], x, qx);
                     r[8 * j + e] = __float_as_uint(x);
                 }
             }
             tc::tmem_st_32x16(ACC_A + lane_addr + col, r);
         }
-        xy_s[cg * 128 + half * 64 + row] = xy;
+        if (half == 0) qx_s[cg * 64 + row] = qx;
         tc::tmem_st_wait();
     }
     tc::fence_proxy_async_smem();
@@ -1343,6 +1374,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
     }
     wait_bar(6, 0);
     // ---- dq (half 0) and dk (half 1) before the norm's backward: back to TMEM; row sums
+    const uint32_t ytile = half == 0 ? Cfg::R_Q : Cfg::R_K;
     {
         float dot = 0.0f, kws = 0.0f;
 #pragma unroll
@@ -1408,8 +1440,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) delta_grad_tc_kernel(
         for (int i = 0; i < 2; ++i) {
             const int t = lane + 32 * i;
             const float kw_t = kw_s[t] + kw_s[64 + t];
-            w[i] = rs_s[t] + rs_s[128 + t] + xy_s[64 + t] + xy_s[192 + t];
-            s[i] = w[i] + (rs_s[64 + t] + rs_s[192 + t]) + (xy_s[t] + xy_s[128 + t]) - (cs_s[t] + cs_s[64 + t] + cs_s[128 + t] + cs_s[192 + t]) - kw_t;
+            w[i] = rs_s[t] + rs_s[128 + t] + ky_s[t];
+            s[i] = w[i] + (rs_s[64 + t] + rs_s[192 + t]) + (qx_s[t] + qx_s[64 + t]) - (cs_s[t] + cs_s[64 + t] + cs_s[128 + t] + cs_s[192 + t]) - kw_t;
             kw += kw_t;
         }
         const float extra = __expf(g_s[C - 1]) * warp_sum(sds) + warp_sum(kw);
@@ -1651,7 +1683,7 @@ static int backward_dh(asca_ctx* ctx, const void* q, const void* k, const void* 
         Carver w{pass ? al_ptr(ws) : nullptr};
         dS = w.take<__nv_bfloat16>(n_tiles * DH * DH);
         dR = w.take<__nv_bfloat16>(n_tiles * C * DH);
-        VD = w.take<float>(n_tiles * C * (DH / 32));
+        VD = w.take<float>(n_tiles * 2 * C * (DH / 32));
         SD = w.take<float>(n_tiles * ChainCfg<DH>::S_WARPS);
         if (slot < 0) {
             carve_kept(w, n_tiles, true, &t);

@@ -765,6 +765,24 @@ def test_delta_tc_gate_sums_within_a_chunk_in_f32(gpu, dh, t0, t1):
     assert ((got[:, t1, 1] - want).abs() <= 2.0 ** -19 * want.abs()).all()
 
 
+@pytest.mark.parametrize("dh", [64, 128])
+def test_delta_tc_value_gradient_meets_the_state_in_f32(gpu, dh):
+    """One token on a state with one entry: d beta = -dR . (S^T k), dR = (q . k) dO a product of two eight-bit numbers."""
+    import torch
+
+    B, H = 2, 8
+    g = torch.Generator(device="cuda").manual_seed(dh)
+    q, k, v, d_o = (torch.zeros(B, 1, H, dh, device="cuda") for _ in range(4))
+    q[..., 3], k[..., 3] = _bf16_values(g, B, 1, H), 1.0
+    d_o[..., dh - 2] = _bf16_values(g, B, 1, H)
+    s_init = torch.zeros(B, H, dh, dh, device="cuda")
+    s_init[..., 3, dh - 2] = 1.0
+    al, be = torch.ones(B, 1, H, device="cuda"), torch.full((B, 1, H), 0.5, device="cuda")
+    got = _delta_tc_gates(gpu, q, k, v, al, be, d_o, s_init)[:, 0, 1]
+    want = -0.25 * (q[..., 3] * d_o[..., dh - 2]).double()[:, 0]
+    assert ((got - want).abs() <= 2.0 ** -19 * want.abs()).all()
+
+
 # f32 delta backward: a row's gradients are divided by its norm through the reciprocal; zero, infinite and tiny norms behave as a division.
 @pytest.mark.parametrize("dh", [32, 64, 128])
 def test_delta_f32_norm_division_at_its_edges(gpu, dh):
