@@ -58,9 +58,11 @@ template <int BN, bool DEEP = false, bool PAIR = false, bool EW8 = false> struct
     // group's rows as soon as the tile has landed, while the issuer is still at earlier ones: see there
     static constexpr bool RAG_WARP = PAIR && !EW8;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS + (RAG_WARP ? 32 : 0);
-    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 392 /*barriers, claims*/;   // + stages + tile table
+    static constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 416 /*barriers, claims, ragged k-tiles*/;   // + stages + tile table
 };
 constexpr int MAX_GROUPS = 2048, MAX_STAGES = 7;
+constexpr int RAG_Q = 8;               // ragged k-tiles under way in a CTA at most: each holds a ring slot until it has been cleared and used
+static_assert(RAG_Q >= MAX_STAGES, "every ring slot may hold a ragged k-tile");
 
 struct KP {
     float* C;
@@ -227,7 +229,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rag_clear + MAX_STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile unsigned long long* claims = reinterpret_cast<volatile unsigned long long*>(tmem_slot + 2);   // [DYN_Q] (number + 1) << 32 | tile
-    int* prefix = reinterpret_cast<int*>(const_cast<unsigned long long*>(claims) + DYN_Q);             // [n_groups + 1] first tile of every group
+    volatile int* rag_word = reinterpret_cast<volatile int*>(claims + DYN_Q);        // [0] 2 x ragged k-tiles handed over (+ 1: no more come), [1] tiles
+    volatile uint16_t* rag_q = reinterpret_cast<volatile uint16_t*>(rag_word + 2);   // [RAG_Q] ring slot << 8 | rows of k that are the expert's
+    int* prefix = reinterpret_cast<int*>(const_cast<uint16_t*>(rag_q) + RAG_Q);      // [n_groups + 1] first tile of every group
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_n = (p.N + BN - 1) / BN;
@@ -263,6 +267,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
             prefix[n_groups] = base;
             *abort_flag = 0;
             for (int i = 0; i < DYN_Q; ++i) claims[i] = 0;
+            rag_word[0] = rag_word[1] = 0;
             for (uint32_t s = 0; s < STAGES; ++s) {
                 tc::mbar_init(&full[s], 1);
                 tc::mbar_init(&empty[s], 1);
@@ -359,6 +364,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         // ------------------------------------------------------------ TMA producer (one thread)
         if (lane == 0) {
             uint32_t s = 0, round = 0;   // ring slot of the next k-tile and how often the ring has been around
+            int n_rag = 0;
             bool ok = true;
             // The claiming thread asks for claim ci + 1 half way through claim ci's loads and publishes it after them: the
             // atomic's round trip hides behind the loads, and no other role needs the next claim before this one is used up.
@@ -413,8 +419,14 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     } else {      // memory (N rows x K)
                         load(b_s, &mapB, k0 + x.b_in, nl0 + x.b_out);
                     }
+                    if (SH::RAG_WARP && !joint) {   // to the warp that clears its end
+                        rag_q[n_rag++ % RAG_Q] = (uint16_t)(s << 8 | (uint32_t)(x.K % BK));
+                        __threadfence_block();
+                        rag_word[0] = 2 * n_rag;
+                    }
                     if (++s == STAGES) s = 0, ++round;
                 }
+                if (SH::RAG_WARP) rag_word[1] = ci + 1;
                 if (claimer) {
                     // A tile without k-tiles takes no ring slot, so nothing above holds the claims of a run of them back: each waits
                     // for the epilogue to release its accumulator buffer once more (of the tile two before it, or of one before that
@@ -431,6 +443,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
                     publish_claim(c, cur);
                 }
             }
+            if (SH::RAG_WARP) rag_word[0] = 2 * n_rag + 1;
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -528,24 +541,39 @@ __global__ void __launch_bounds__(Shape<BN, DEEP, PAIR, EW8>::THREADS, Shape<BN,
         // In the issuing warp, all 64 rows' ends at a time, it held the instructions of the tile and of the next one up by 3 us a
         // tile: C = 1024 x 4096 for 64 experts of 512 tokens took 350 us where every count is a multiple of 64 and 498 where none
         // is (1,024 tokens: 520 and 718); now 367 and 377 (527 and 590).
-        uint32_t s = 0, par = 0;   // first ring slot of the tile; parity of every slot's next ragged k-tile (a bit each)
-        bool ok = p.group_dim == GROUP_K;
-        for (int tl = 0; ok; ++tl) {
-            int t = lane == 0 ? read_tile(tl) : -1;
-            t = __shfl_sync(0xffffffffu, t, 0);
-            if (t < 0) break;
-            const Tile x = locate(t);
-            if (x.K % BK) {
-                const uint32_t last = (s + (uint32_t)x.num_k - 1) % STAGES;
-                int got = 0;
-                if (lane == 0) got = tc::mbar_wait(&rag_full[last], (par >> last) & 1, abort_flag, p.err_word, 105) ? 1 : 0;
-                ok = __shfl_sync(0xffffffffu, got, 0) != 0;
-                if (!ok) break;
-                clear_rows(last, x.K % BK);
-                if (lane == 0) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&rag_clear[last]), 0));
-                par ^= 1u << last;
+        // The producer hands the ragged k-tiles over one by one, so this warp need not follow the claims, which nothing would hold for
+        // it over a run of tiles without a ragged end.
+        uint32_t par = 0;   // parity of every slot's next ragged k-tile (a bit each)
+        if (p.group_dim == GROUP_K) {
+            for (int done = 0;; ++done) {
+                int item = -1;   // none left, or a wait gave up
+                if (lane == 0) {
+                    long long t0 = clock64();
+                    for (int beat = 0;;) {
+                        const int w = rag_word[0], tiles_done = rag_word[1];
+                        if ((w >> 1) > done) {
+                            __threadfence_block();
+                            item = rag_q[done % RAG_Q];
+                            if (!tc::mbar_wait(&rag_full[item >> 8], (par >> (item >> 8)) & 1, abort_flag, p.err_word, 105)) item = -1;
+                            break;
+                        }
+                        if ((w & 1) || *abort_flag) break;
+                        if (tiles_done != beat) beat = tiles_done, t0 = clock64();
+                        if (clock64() - t0 > tc::WAIT_LIMIT_CYCLES) {   // (no tile for as long as any wait of the producer may take)
+                            *abort_flag = 1;
+                            if (p.err_word) atomicExch(p.err_word, 109);
+                            break;
+                        }
+                        __nanosleep(100);
+                    }
+                }
+                item = __shfl_sync(0xffffffffu, item, 0);
+                if (item < 0) break;
+                const uint32_t slot = (uint32_t)item >> 8;
+                clear_rows(slot, item & 255);
+                if (lane == 0) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&rag_clear[slot]), 0));
+                par ^= 1u << slot;
             }
-            s = (s + (uint32_t)x.num_k) % STAGES;
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5, EW8: 2..9)

@@ -934,12 +934,15 @@ def test_silu_over_the_range_of_its_argument(gpu, tokens):
 
 # Weight gradients of experts whose token counts end a 64-token tile anywhere (empty experts, sixteens, one past them): nothing of a
 # neighbour's rows, 1e4 times as large, enters a sum. d_w2 from the hidden rows as they were stored, within the bound of f32 sums.
-@pytest.mark.parametrize("d,F", [(256, 512), (128, 128)])   # CTA pairs; single CTAs
-def test_ragged_token_counts_in_weight_gradients(gpu, d, F):
+# The long form: runs of tiles without a ragged end, more than a CTA's 16 claims at a time, between ragged ones.
+@pytest.mark.parametrize("d,F,long", [(256, 512, False), (128, 128, False), (1024, 2048, True)])   # CTA pairs; single CTAs; CTA pairs
+def test_ragged_token_counts_in_weight_gradients(gpu, d, F, long):
     import torch
     from asca_b200 import ops
 
     counts = [0, 1, 64, 15, 16, 17, 0, 63, 65, 79, 80, 81, 127, 128, 129, 448, 449, 511, 512, 513, 900, 33, 48, 2, 320, 7]
+    if long:
+        counts = [65, 7] + [64] * 46 + [129, 1, 0, 190] + [128, 64] * 24 + [63]
     E, N = len(counts), sum(counts)
     g = torch.Generator(device="cuda").manual_seed(F)
 
