@@ -651,7 +651,7 @@ def run_moe(hs: Harness, args):
 
 # ------------------------------------------------------------------ isolated delta op
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch at B=4, H=16, T=4096, dh=128 (64 chains), divided by 64:
-# traffic is proportional to the number of chains (profiles/delta_tc_bf16_cfg2.md).
+# traffic is proportional to the number of chains.
 NCU_TRAFFIC_PER_CHAIN = {
     "delta_grad_tc_kernel": (614.2e6 + 238.3e6) / 64,
     "delta_bwd_tc_kernel": (372.1e6 + 302.2e6) / 64,

@@ -285,7 +285,7 @@ def test_trainer_loop_matches_oracle_loss_for_loss_and_resumes(orc, gpu, tmp_pat
 
 def test_bf16_compute_train_step_head_dim_64(orc, gpu):
     """bf16 compute mode with head dim 64 (the decode configuration's head size): the delta op runs on the
-    tensor-core kernels with every head zero-padded to 128; loss and gradients stay within 2e-2 of the f32
+    tensor-core kernels in their 64-wide form; loss and gradients stay within 2e-2 of the f32
     oracle (the gate biases of these toy shapes: see _bf16_grad_tol). 1024 tokens, four chunks per chain."""
     import asca_b200
 

@@ -291,7 +291,7 @@ def test_delta_bf16_mode(orc, gpu):
 @pytest.mark.parametrize("dh", [128, 64])
 @pytest.mark.parametrize("B,T,H", [(1, 64, 1), (2, 128, 2), (2, 200, 3), (1, 1000, 2), (3, 37, 1)])
 def test_delta_bf16_tensor_core_forward(orc, gpu, B, T, H, dh):
-    """bf16 inputs at dh = 128 (and dh = 64, zero-padded to 128 inside the kernels) take the chunked WY/UT tcgen05
+    """bf16 inputs at dh = 128 (and dh = 64, in tiles of its own width) take the chunked WY/UT tcgen05
     forward: outputs, final state and every chunk checkpoint against the f32 recurrence on the same (bf16-rounded)
     inputs; ragged last chunk; continuation from an initial state."""
     import torch

@@ -697,6 +697,41 @@ def test_delta_tc_sequences_do_not_mix(gpu, B, T, H, dh):
         assert (got_.double() - ref).norm() < 8e-3 * ref.norm()
 
 
+# bf16 delta: chains over many chunks, more chains than SMs (the requests ahead into L2 switch off, heads of 64 share an SM): within a handful
+# of bf16 roundings of the f32 kernels, and bit for bit what the sequences give in smaller launches.
+@pytest.mark.parametrize("dh", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(1, 2111, 2), (20, 130, 16)])
+def test_delta_tc_many_chunks_and_many_chains(gpu, B, T, H, dh):
+    import torch
+    from asca_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(B + dh)
+    n = B * T
+
+    def norm(*s):
+        return torch.randn(*s, generator=g, device="cuda")
+
+    q, k = (torch.nn.functional.normalize(norm(n, H, dh), dim=-1).reshape(n, H * dh).bfloat16() for _ in range(2))
+    v, d_o = norm(n, H * dh).bfloat16(), norm(n, H * dh).bfloat16()
+    al, be, qn = torch.sigmoid(3 + norm(n, H)), torch.sigmoid(norm(n, H)), 1 + torch.rand(n, H, generator=g, device="cuda")
+
+    def run(b0, b1, cast):
+        part = [x[b0 * T:b1 * T].contiguous() for x in (q, k, v, d_o, al, be, qn)]
+        q_, k_, v_, do_ = (cast(x) for x in part[:4])
+        o, fin, ck = ops.delta_fwd(gpu, q_, k_, v_, *part[4:6], b1 - b0, T, H, dh, want_final=True)
+        d_qkv, d_gate = ops.delta_bwd(gpu, q_, k_, v_, *part[4:6], part[6], part[6], do_, ck, b1 - b0, T, H, dh)
+        gpu.sync()
+        return o, fin.view(b1 - b0, -1), d_qkv, d_gate
+
+    got = run(0, B, lambda x: x)
+    for a, b in zip(got, run(0, B, lambda x: x.float())):
+        assert (a.double() - b.double()).norm() < 8e-3 * b.double().norm()
+    cut = B * 9 // 20   # (9 x 16 chains: fewer than SMs)
+    if cut:
+        for a, b, c in zip(got, run(0, cut, lambda x: x), run(cut, B, lambda x: x)):
+            assert torch.equal(a, torch.cat([b, c]))
+
+
 # What the bf16 delta gradients hold in f32 between their products: inputs for which everything else is exact in bf16, one chain per
 # entry, so that a value rounded to bf16 on the way (2^-9) stands out. The bound: a dozen f32 roundings, exp and log among them.
 def _delta_tc_gates(gpu, q, k, v, al, be, d_o, s_init=None):
