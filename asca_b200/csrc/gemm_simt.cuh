@@ -116,7 +116,7 @@ __device__ __forceinline__ void stage4(float* dst, const float* p, bool vec_ok, 
     if (vec_ok) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(p), "r"(valid * 4) : "memory");
     } else {
-#pragma unroll 1
+#pragma unroll
         for (int j = 0; j < 4; ++j)
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s + 4 * j), "l"(j < valid ? p + j : p), "r"(j < valid ? 4 : 0)
                          : "memory");
