@@ -22,6 +22,7 @@
 #include "gemm_tc.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include "tc_common.cuh"
 
 namespace gemm_tc {
@@ -505,17 +506,21 @@ int sk_launch_shape(asca_ctx* ctx, const Args& a, int64_t tiles) {
     return ASCA_OK;
 }
 
-// CTAs that share a tile's k range in an expert product: as many as the SMs that would have no tile allow, each with three k-tiles at least.
-// The tiles are taken as one token tile for every group that can have a row (their number is known on the device only). 768 -> 3072 -> 768 with 16
-// experts, us a decode step of 12 blocks without and with it: 1 stream 536 / 447, 5 573 / 493, 12 672 / 641; from 24 streams on
-// the second product has its 96 tiles and nothing is shared. Measured and not taken: eight CTAs (1 stream 454, 3 streams 597 / 508
-// with four), three CTAs for two tiles (256 streams 941 / 1150: three SMs of one GPC are rarely free at once), and the dense
-// products of the same step (12 streams 641 / 646, 40 706 / 721: their time is not the stream of weights).
+// CTAs that share a tile's k range in an expert product. One product alone, us for one, two and four CTAs a tile: k = 3072, 6 tiles
+// 23.0 / 18.9 / 16.8, 30 tiles 23.1 / 19.8 / 18.9, 36 tiles 23.1 / 20.9 / 29.2 (clusters of four do not fill the last SMs of a GPC, so
+// fewer of them run at once than the SMs make), 60 tiles 25.0 / 23.1, 72 tiles 25.0 / 25.0; k = 2048, 16 tiles 18.9 / 16.8 / 15.0, 48 tiles 18.9 /
+// 18.9; k = 4096, 64 tiles 29.1 / 27.1, 80 tiles 29.3 / 37.3. Below k = 2048 the exchange costs what the shorter streams save, and more
+// (1024, 8 tiles 12.9 / 14.8 / 14.8; 768, 24 tiles 12.5 / 14.5 / 14.5). Hence 2048 on, seven eighths of the SMs at most. Measured and not taken: eight CTAs
+// (a decode step of one stream 454 us, 447 with four), three CTAs for two tiles (three SMs of one GPC are rarely free at once), and the
+// dense products of a step (12 streams 641 / 646, 40 706 / 721: their time is not the stream of weights).
+// How many token tiles there are is known on the device only; they are estimated for tokens spread over the experts by chance: the
+// experts that get any, and from sixteen tokens an expert on, half a tile beside the full ones for each.
 int sk_split(asca_ctx* ctx, const Args& a, int64_t tiles_f) {
-    const int64_t n_sm = ctx->sm_count > 0 ? ctx->sm_count : 148, tiles = std::min<int64_t>(a.n_groups, a.total_rows) * tiles_f, num_k = (a.K + BK - 1) / BK;
-    if (tiles * 4 <= n_sm && num_k >= 12) return 4;
-    if (tiles * 2 <= n_sm && num_k >= 6) return 2;
-    return 1;
+    const double E = (double)a.n_groups, rows = (double)a.total_rows;
+    const double tiles = (rows >= 16.0 * E ? rows / 32.0 + 0.5 * E : E * (1.0 - std::pow(1.0 - 1.0 / E, rows))) * (double)tiles_f;
+    const double room = 0.875 * (ctx->sm_count > 0 ? ctx->sm_count : 148);
+    if (a.K < 2048) return 1;
+    return tiles * 4 <= room ? 4 : tiles * 2 <= room ? 2 : 1;
 }
 
 }  // namespace

@@ -878,8 +878,8 @@ def test_delta_f32_norms_without_a_reciprocal(gpu, dh):
     assert (got.view(T, 3, H, dh)[2:7, 0] == 0).all()
 
 
-# Expert products of a few tokens, whose k range two or four CTAs share: odd numbers of k-tiles, experts without tokens and with more than
-# one token tile (several tiles a cluster), and just past the rule; against f64 sums over the hidden rows as they were stored.
+# Expert products of a few tokens: ones whose k range two or four CTAs share and ones past the rule (more tokens, shorter k), experts without tokens
+# and with more than one token tile; against f64 sums over the hidden rows as they were stored.
 @pytest.mark.parametrize("tokens,experts,d,F", [(1, 16, 768, 3072), (3, 16, 768, 3072), (12, 16, 768, 3072), (13, 16, 768, 3072), (70, 2, 128, 1664), (300, 6, 64, 832), (200, 40, 64, 448)])
 def test_few_tokens_per_expert_with_a_shared_k_range(gpu, tokens, experts, d, F):
     import torch
@@ -905,6 +905,34 @@ def test_few_tokens_per_expert_with_a_shared_k_range(gpu, tokens, experts, d, F)
         if len(rows):   # from the hidden rows as they were stored (bf16)
             want[perm[rows].long()] = hid[rows].double() @ w2[e * F:(e + 1) * F].double() + b2.double()
     assert (out - want).abs().max() < 4e-6 * F ** 0.5
+
+
+# The same with more tiles than clusters run at a time (148 SMs: 37 of four CTAs, 74 of two), so that some take a second tile into slots
+# and an accumulator buffer that the first one's readers have to leave; odd and even numbers of k-tiles.
+@pytest.mark.parametrize("counts,share,F", [([33] * 15 + [1] * 17, 4, 2048), ([1] * 17 + [33] * 15, 4, 2112), ([33] * 30 + [1] * 34, 2, 2048), ([1] * 34 + [33] * 30, 2, 2624)])
+def test_shared_k_range_over_several_tiles_a_cluster(gpu, counts, share, F):
+    import torch
+    from asca_b200 import ops
+
+    E, tokens, d = len(counts), sum(counts), 128
+    assert tokens == 16 * E and sum((c + 31) // 32 for c in counts) > 148 // share   # (one feature tile each)
+    g = torch.Generator(device="cuda").manual_seed(F + E)
+
+    def norm(*s, scale=1.0):
+        return torch.randn(*s, generator=g, device="cuda") * scale
+
+    xn, w1, w2 = norm(tokens, d).bfloat16(), norm(d, E * F, scale=d ** -0.5).bfloat16(), norm(E * F, d, scale=F ** -0.5).bfloat16()
+    b1, b2 = norm(E * F), norm(d)
+    offs = torch.tensor([0] + counts, device="cuda").cumsum(0).int()
+    perm = torch.randperm(tokens, generator=g, device="cuda").int()
+    out, _, hid = ops.moe_fwd(gpu, xn, w1, b1, w2, b2, perm, offs, F, E)
+    out2, _, _ = ops.moe_fwd(gpu, xn, w1, b1, w2, b2, perm, offs, F, E)
+    gpu.sync()
+    assert torch.equal(out, out2)
+    for e in range(E):
+        rows = slice(int(offs[e]), int(offs[e + 1]))
+        want = hid[rows].double() @ w2[e * F:(e + 1) * F].double() + b2.double()
+        assert (out[perm[rows].long()] - want).abs().max() < 4e-6 * F ** 0.5
 
 
 # The residual adds in the epilogues of the attention's and the experts' second product, on both sides of where the row-tiled kernel
