@@ -710,7 +710,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 // ------------------------------------------------------------------ backward chain
 // Same threads as the forward: quarters 0 and 1 hold the 64 rows of dU and dR, quarters 2 and 3 scale the rows of dO by gam in place
 // (after A^T dO has read them), dS is held like S. TMEM: dS, D1 = K dS and later (X - I)^T dU, D2 = A^T dO, D3 = K S. 202 KB of HBM per chunk
-// (dv in f32 among them) at 3.8 TB/s: 367 us for 64 chunks of 128 chains, three products and their register passes one after another.
+// (dv in f32 among them) at 3.9 TB/s: 420 us for 64 chunks of 128 chains, three products and their register passes one after another. The 32 KB of
+// S are there for two sums over f32 values, <S, dS> and dv . (S^T k): without them 371 us, of the difference most is the load.
 // With the gradients on the same chain a chunk was nine groups of products: 914 us.
 template <int DH>
 __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delta_bwd_tc_kernel(
@@ -948,7 +949,14 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
             uint8_t* st = base + par * Cfg::B_STAGE;
             const float g_row = gb_s[par * 128 + row], be_row = gb_s[par * 128 + 64 + row], gam = expf(g_row);
             float du[32];
+            // The row of v, used behind the state's update: at head dim 64 asked for before it (265 us for 128 chains of 64 chunks, 279 behind it), at
+            // 128 behind it, where the update needs the registers (438 and 420).
             uint4 v4[4];
+            auto ask_v = [&] {
+                const __nv_bfloat16* vr = v + ((int64_t)b * T + c * C + row) * d + h * DH + col;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v4[j] = c * C + row < T ? reinterpret_cast<const uint4*>(vr)[j] : make_uint4(0, 0, 0, 0);
+            };
             if (wq >= 2) {
                 if (c > 0) {   // gam dO in place, once A^T dO is done
                     if (!warp_wait(mma0_done, par, 311)) break;
@@ -1007,10 +1015,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                     }
                 }
                 arrive(dr_ready);
-                // the row of v is asked for here and used behind the state's update
-                const __nv_bfloat16* vr = v + ((int64_t)b * T + c * C + row) * d + h * DH + col;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v4[j] = c * C + row < T ? reinterpret_cast<const uint4*>(vr)[j] : make_uint4(0, 0, 0, 0);
+                if (DH == 64) ask_v();
                 // -beta gam dR . (S^T k)   (K S was done before K dS)
                 float ky = 0.0f;
 #pragma unroll
@@ -1061,6 +1066,7 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
                 }
             }
             if (wq < 2) {   // dv = beta dR, and this thread's part of v . dv
+                if (DH == 128) ask_v();
                 float vd = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -1084,8 +1090,8 @@ __global__ void __launch_bounds__(ChainCfg<DH>::THREADS, DH == 128 ? 1 : 2) delt
 }
 
 // ------------------------------------------------------------------ gradients per chunk
-// One CTA per (chunk, chain), two per SM; nothing here depends on another chunk. 209 KB of HBM a chunk: 395 us for 8192 of 64 x 128
-// (4.3 TB/s; two CTAs per SM are what 103 KB of tiles allow, and one's loads and stores hide the other's register passes). With S and dS the (bf16) state at the chunk's start
+// One CTA per (chunk, chain), two per SM; nothing here depends on another chunk. 209 KB of HBM a chunk: 410 us for 8192 of 64 x 128
+// (4.2 TB/s, 394 us with the gates' sums over the bf16 tiles M and P; two CTAs per SM are what 103 KB of tiles allow, and one's loads and stores hide the other's register passes). With S and dS the (bf16) state at the chunk's start
 // and gradient at its end:
 //   dL = dR U^T,  dA = dO U^T,  X = dO S^T,  Y = dR S^T,  dW = U dS^T              one group of products, value columns 64 at a time
 //   M = -beta Gam dL (strictly lower),  P = Gam dA (lower);  X *= gam,  Y *= -beta gam   (in TMEM)

@@ -653,10 +653,10 @@ def run_moe(hs: Harness, args):
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch at B=4, H=16, T=4096, dh=128 (64 chains), divided by 64:
 # traffic is proportional to the number of chains.
 NCU_TRAFFIC_PER_CHAIN = {
-    "delta_grad_tc_kernel": (614.2e6 + 238.3e6) / 64,
-    "delta_bwd_tc_kernel": (372.1e6 + 302.2e6) / 64,
-    "delta_fwd_tc_kernel": (337.7e6 + 230.9e6) / 64,
-    "delta_prep_tc_kernel": (203.5e6 + 188.3e6) / 64,
+    "delta_grad_tc_kernel": (617.5e6 + 235.3e6) / 64,
+    "delta_bwd_tc_kernel": (507.8e6 + 305.3e6) / 64,
+    "delta_fwd_tc_kernel": (337.7e6 + 226.3e6) / 64,
+    "delta_prep_tc_kernel": (203.5e6 + 184.0e6) / 64,
 }
 
 
